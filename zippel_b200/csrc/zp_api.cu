@@ -5,82 +5,17 @@
 #include <cstring>
 #include <mutex>
 #include <new>
-#include <vector>
 
 #include <cuda_bf16.h>
 
-#include "zp_common.cuh"
-
-// Event pairs recorded around kernel classes while timing is on.
-struct ZpTimer {
-  struct Span { int cls; cudaEvent_t a, b; int64_t launches; };
-  std::vector<Span> spans;      // pool; `used` of them hold live records
-  size_t used = 0;
-  Span *open(int cls, cudaStream_t st) {
-    if (used == spans.size()) {
-      Span s{cls, nullptr, nullptr, 0};
-      if (cudaEventCreate(&s.a) != cudaSuccess || cudaEventCreate(&s.b) != cudaSuccess) return nullptr;
-      spans.push_back(s);
-    }
-    Span *s = &spans[used++];
-    s->cls = cls;
-    s->launches = zp_launch_counter();
-    cudaEventRecord(s->a, st);
-    return s;
-  }
-  static void close(Span *s, cudaStream_t st) {
-    if (!s) return;
-    cudaEventRecord(s->b, st);
-    s->launches = zp_launch_counter() - s->launches;
-  }
-};
+#include "zp_core.cuh"
 
 namespace {
 
 thread_local char g_cuda_error[512] = "";
 thread_local int64_t g_launches = 0;
 
-// brackets one expression with a timing span when the plan has a timer
-#define ZP_TIMED(cls, expr)                                                      \
-  do {                                                                           \
-    ZpTimer::Span *span_ = plan->timer ? plan->timer->open(cls, st) : nullptr;   \
-    rc = (expr);                                                                 \
-    ZpTimer::close(span_, st);                                                   \
-    if (rc) return rc;                                                           \
-  } while (0)
-
-bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
-
-// Workspace carving; every region starts 256-byte aligned.
-//   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials
-//   backward: dy planes | dht | dh1 planes | da1 | du_src | grot | wgrad partials | scratch
-// mode 0 / 1: forward that keeps what a backward reads (1: plus the backward's own regions);
-// mode 2: forward alone with fused epilogues -- of h1 only the gate scalars exist, y does not.
-struct Workspace {
-  float *rot, *h1, *y, *dht, *da1, *du_src, *grot, *wgrad, *scratch, *scales, *head, *cont;
-  float *radial, *rad_partials;          // radial layer inside the call: its output, dW partials
-  int64_t ld_h1;
-  int32_t *block_node;
-  ZpPlanes a1, ht, dy, dh1;
-  ZpPlanes hr, rw, gr;                   // planes of the layer's input, weight, output gradient
-  uint16_t *wfold;
-  size_t bytes;
-};
-
-// slots of the device-side scale array (fp16-plane precision): raw maxima, derived scales, and
-// per weight block {max |W|, scale} from kScWeights on
-enum { kScX = 0, kScRad, kScG, kScH1, kScDht, kScA1, kScHt, kScDy, kScDh1, kScGate,
-       kScMaxNode /* an int */,
-       // the radial layer run inside the call: {max, scale} of its input and of its weight, max
-       // of conv1's input gradient, scale of the planes of grad_radial
-       kScHr, kScHrScale, kScRw, kScRwScale, kScDa1, kScGrScale,
-       kScWeights = 24,
-       kScCount = kScWeights + 4 * (ZP_MAX_L + 1) };
-
-constexpr int kMaxWgradSplits = 8;
 constexpr int kChunkK = 2048;          // contraction length of one TMEM accumulation chunk
-
-int64_t round8(int64_t x) { return (x + 7) / 8 * 8; }
 
 // The fused epilogues (gate activation in conv1, rotation back + segmented sums in conv2) need
 // one- or two-plane operands and contractions that fit one accumulation chunk.  They are opt-in
@@ -102,85 +37,6 @@ bool can_fuse(const zp_plan *p, int conv) {
   for (int m = 0; m < p->n_blocks; ++m)
     if ((conv ? p->c2_in[m] : p->c1_in[m]) > kChunkK) return false;
   return true;
-}
-
-constexpr int kRadialSplits = 8;         // K splits of the radial layer's weight gradient
-
-// ec > 0: the last layer of the radial MLP (ec -> R) runs inside the call
-Workspace carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *base, int ec = 0) {
-  const ZpTables &t = p->t;
-  Workspace w;
-  std::memset(&w, 0, sizeof(w));
-  size_t off = 0;
-  auto take = [&](size_t nbytes) {
-    char *ptr = base ? static_cast<char *>(base) + off : nullptr;
-    off += zp_align_up(nbytes, 256);
-    return ptr;
-  };
-  auto takef = [&](size_t elems) { return reinterpret_cast<float *>(take(elems * sizeof(float))); };
-  auto takep_rows = [&](int64_t rows, int64_t cols) {
-    ZpPlanes pl;
-    pl.ld = round8(cols);
-    pl.planes = p->planes;
-    pl.fp16 = p->fp16;
-    pl.scale = nullptr;
-    pl.plane_stride = (int64_t)zp_align_up((size_t)rows * pl.ld, 128);
-    pl.base = take((size_t)pl.planes * pl.plane_stride * 2);
-    return pl;
-  };
-  auto takep = [&](int64_t cols) { return takep_rows(E, cols); };
-  const size_t e = (size_t)E;
-  const bool lean = mode == 2 && can_fuse(p, 0) && can_fuse(p, 1);
-  w.rot = takef(e * t.nnz_pad);
-  w.a1 = takep((int64_t)t.Km * 2 * t.C);
-  w.ld_h1 = lean ? t.n_gate : t.w1_cols;
-  w.h1 = takef(e * w.ld_h1);
-  w.ht = takep((int64_t)t.Km * t.H);
-  if (!lean) w.y = takef(e * t.Km * t.C);
-  w.wfold = reinterpret_cast<uint16_t *>(take((size_t)p->w_elems * 2));
-  w.scales = takef(kScCount);
-  if (ec > 0) {
-    w.radial = takef(e * t.R);
-    w.hr = takep(ec);
-    w.rw = takep_rows(t.R, ec);
-  }
-  // the partial sums of the rotate-back epilogue live only inside the forward: the backward's own
-  // regions start at the same offset and reuse the space
-  const size_t off_fwd = off;
-  if (can_fuse(p, 1)) {
-    w.head = takef((size_t)N * t.nnz * t.C);
-    w.cont = takef((size_t)zp_ceil_div(E, 32) * t.nnz * t.C);
-    w.block_node = reinterpret_cast<int32_t *>(take((size_t)zp_ceil_div(E, 32) * sizeof(int32_t)));
-  }
-  const size_t end_fwd = off;
-  if (mode == 1) {
-    off = off_fwd;
-    w.dy = takep((int64_t)t.Km * t.C);
-    w.dht = takef(e * t.Km * t.H);
-    w.dh1 = takep(t.w1_cols);
-    w.da1 = takef(e * t.Km * 2 * t.C);
-    w.du_src = takef(e * 2 * t.K * t.C);
-    w.grot = takef(e * t.nnz_pad);
-    w.wgrad = takef((size_t)kMaxWgradSplits * p->g_elems);
-    // column-sum partials (bias gradients; the widest user is the radial layer's R columns)
-    w.scratch = takef((size_t)zp_ceil_div(E > 0 ? E : 1, 128) *
-                      (size_t)(ec > 0 && t.R > t.w1_cols ? t.R : t.w1_cols));
-    if (ec > 0) {
-      w.gr = takep(t.R);
-      w.rad_partials = takef((size_t)kRadialSplits * t.R * ec);
-    }
-  }
-  if (p->fp16 && base) {
-    w.a1.scale = w.scales + kScA1;
-    w.ht.scale = w.scales + kScHt;
-    w.dy.scale = w.scales + kScDy;
-    w.dh1.scale = w.scales + kScDh1;
-    w.hr.scale = w.scales + kScHrScale;
-    w.rw.scale = w.scales + kScRwScale;
-    w.gr.scale = w.scales + kScGrScale;
-  }
-  w.bytes = off > end_fwd ? off : end_fwd;
-  return w;
 }
 
 // ZP_STREAMS=0 in the environment keeps every launch on the caller's stream.
@@ -222,7 +78,7 @@ struct Lanes {
   }
 };
 
-const float *wscale(const zp_plan *p, const Workspace &w, int conv, int m) {
+const float *wscale(const zp_plan *p, const ZpWorkspace &w, int conv, int m) {
   return p->fp16 ? w.scales + kScWeights + (conv * (ZP_MAX_L + 1) + m) * 2 + 1 : nullptr;
 }
 
@@ -234,6 +90,59 @@ ZpPlanes sub(const ZpPlanes &p, int64_t col) {
 }
 
 }  // namespace
+
+ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *base, int ec,
+                     ZpFormat rad) {
+  const ZpTables &t = p->t;
+  const ZpFormat f{p->planes, p->fp16};
+  ZpWorkspace w;
+  std::memset(&w, 0, sizeof(w));
+  ZpCarver c(base);
+  const size_t e = (size_t)E;
+  const bool lean = mode == 2 && can_fuse(p, 0) && can_fuse(p, 1);
+  w.scales = c.floats(kScCount);
+  w.rot = c.floats(e * t.nnz_pad);
+  w.a1 = c.planes(E, (int64_t)t.Km * 2 * t.C, f, w.scales + kScA1);
+  w.ld_h1 = lean ? t.n_gate : t.w1_cols;
+  w.h1 = c.floats(e * w.ld_h1);
+  w.ht = c.planes(E, (int64_t)t.Km * t.H, f, w.scales + kScHt);
+  if (!lean) w.y = c.floats(e * t.Km * t.C);
+  w.wfold = reinterpret_cast<uint16_t *>(c.bytes((size_t)p->w_elems * 2));
+  if (ec > 0) {
+    w.radial = c.floats(e * t.R);
+    w.hr = c.planes(E, ec, rad, w.scales + kScHrScale);
+    w.rw = c.planes(t.R, ec, rad, w.scales + kScRwScale);
+  }
+  // the partial sums of the rotate-back epilogue live only inside the forward: the backward's own
+  // regions start at the same offset and reuse the space
+  const size_t off_fwd = c.off;
+  if (can_fuse(p, 1)) {
+    w.head = c.floats((size_t)N * t.nnz * t.C);
+    w.cont = c.floats((size_t)zp_ceil_div(E, 32) * t.nnz * t.C);
+    w.block_node = reinterpret_cast<int32_t *>(c.bytes((size_t)zp_ceil_div(E, 32) * sizeof(int32_t)));
+  }
+  const size_t end_fwd = c.off;
+  if (mode == 1) {
+    c.off = off_fwd;
+    w.dy = c.planes(E, (int64_t)t.Km * t.C, f, w.scales + kScDy);
+    w.dht = c.floats(e * t.Km * t.H);
+    w.dh1 = c.planes(E, t.w1_cols, f, w.scales + kScDh1);
+    w.da1 = c.floats(e * t.Km * 2 * t.C);
+    w.du_src = c.floats(e * 2 * t.K * t.C);
+    w.grot = c.floats(e * t.nnz_pad);
+    w.wgrad = c.floats((size_t)kZpWgradSplits * p->g_elems);
+    const size_t parts = (size_t)zp_ceil_div(E > 0 ? E : 1, kZpColRows);
+    w.col1 = c.floats(parts * p->c1_out[0]);
+    w.col2 = c.floats(parts * p->c2_out[0]);
+    if (ec > 0) {
+      w.gr = c.planes(E, t.R, rad, w.scales + kScGrScale);
+      w.col_rad = c.floats(parts * t.R);
+      w.rad_partials = c.floats((size_t)kZpRadialSplits * t.R * ((ec + 3) / 4 * 4));
+    }
+  }
+  w.bytes = c.off > end_fwd ? c.off : end_fwd;
+  return w;
+}
 
 int64_t &zp_launch_counter() { return g_launches; }
 
@@ -441,7 +350,7 @@ int zp_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in, 
   if (rows < 0 || cols < 0 || cols > ld_out || planes < 1 || planes > 3 || !in || !out || ld_out % 2)
     return ZP_ERR_INVALID_ARG;
   const ZpPlanes pl{out, plane_stride, ld_out, planes, planes == 2, nullptr};
-  return zp_launch_split_planes(rows, cols, in, ld_in, pl, (cudaStream_t)stream);
+  return zp_launch_split_planes(rows, cols, in, ld_in, pl, ZpScale{}, (cudaStream_t)stream);
 }
 
 int zp_gemm_planes(zp_plan *plan, int64_t M, int64_t N, int64_t K, int planes, const void *A,
@@ -495,10 +404,12 @@ int zp_wigner_backward(const zp_plan *plan, int64_t n_edges, const float *edge_v
 size_t zp_workspace_bytes(const zp_plan *plan, int64_t n_nodes, int64_t n_edges,
                           int with_backward) {
   if (!plan || n_nodes < 0 || n_edges < 0 || with_backward < 0 || with_backward > 2) return 0;
-  return carve(plan, n_nodes, n_edges, with_backward, nullptr).bytes;
+  return zp_carve(plan, n_nodes, n_edges, with_backward, nullptr, 0, ZpFormat{0, 0}).bytes;
 }
 
-static int check_weights(const zp_plan *p, const zp_weights *w) {
+}  // extern "C"
+
+int zp_check_weights(const zp_plan *p, const zp_weights *w) {
   if (!w || !w->c1_w0 || !w->c1_b0 || !w->c2_w0 || !w->c2_b0) return ZP_ERR_INVALID_ARG;
   if (p->n_blocks > 1 && (!w->c1_wm || !w->c2_wm)) return ZP_ERR_INVALID_ARG;
   for (int m = 1; m < p->n_blocks; ++m)
@@ -506,88 +417,34 @@ static int check_weights(const zp_plan *p, const zp_weights *w) {
   return ZP_OK;
 }
 
-// The last dense layer of the radial MLP (blocks/eso2_ref.py:169-182, rad_func[6]), when the call
-// runs it itself: radial[E, R] = h[E, ec] w[R, ec]^T + b.
-struct RadialLayer {
-  const float *h, *w, *b;
-  int ec;
-  float *grad_h, *grad_w, *grad_b;       // backward only
-};
-
-static int check_radial_layer(const zp_plan *plan, const RadialLayer *rl, int64_t E, bool backward) {
-  if (!rl->w || !rl->b || (E && !rl->h)) return ZP_ERR_INVALID_ARG;
-  if (rl->ec <= 0 || rl->ec % 8 || plan->t.R % 8) return ZP_ERR_UNSUPPORTED;
-  if (!aligned16(rl->h) || !aligned16(rl->w)) return ZP_ERR_INVALID_ARG;
-  // the layer's parameter gradients are wanted together or not at all (frozen parameters)
-  if (backward && ((!rl->grad_w != !rl->grad_b) || (E && !rl->grad_h))) return ZP_ERR_INVALID_ARG;
+int zp_core_radial(const zp_plan *plan, const ZpWorkspace &ws, int64_t E, int ec, const float *bias,
+                   cudaStream_t st) {
+  int rc;
+  const int R = plan->t.R;
+  const ZpGemmTc g{E, R, ec, ws.hr.planes, ws.hr.base, ws.hr.ld, ws.hr.plane_stride, 0,
+                   ws.rw.base, ws.rw.ld, ws.rw.plane_stride, 0, bias, ws.radial, R,
+                   plan->status_dev, 0, 1, 0, 0, ws.hr.fp16, ws.hr.scale, ws.rw.scale,
+                   plan->fp16 ? ws.scales + kScRad : nullptr};
+  ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(g, st));
   return ZP_OK;
 }
 
-// keep != 0: everything a following zp_eso2_backward reads is left in the workspace
-static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *x_node,
-                        const float *edge_vec, const float *cos_g, const float *sin_g,
-                        const float *radial, const float *env, const int32_t *src,
-                        const int32_t *dst, const int32_t *row_ptr, const zp_weights *w,
-                        float *node_out, void *workspace, size_t workspace_bytes, void *stream,
-                        int keep, const RadialLayer *rl = nullptr) {
-  if (!plan || N < 0 || E < 0) return ZP_ERR_INVALID_ARG;
-  if (N == 0) return E == 0 ? ZP_OK : ZP_ERR_INVALID_ARG;
-  if (!x_node || !row_ptr || !node_out || !workspace) return ZP_ERR_INVALID_ARG;
-  if (E && (!edge_vec || !cos_g || !sin_g || (!radial && !rl) || !env || !src || !dst))
-    return ZP_ERR_INVALID_ARG;
-  if (!aligned16(x_node) || !aligned16(node_out) || !aligned16(radial) || !aligned16(workspace))
-    return ZP_ERR_INVALID_ARG;
-  int rc = check_weights(plan, w);
-  if (rc) return rc;
-  if (rl && (rc = check_radial_layer(plan, rl, E, false))) return rc;
-  const Workspace ws = carve(plan, N, E, keep ? 0 : 2, workspace, rl ? rl->ec : 0);
-  if (workspace_bytes < ws.bytes) return ZP_ERR_WORKSPACE;
-  cudaStream_t st = (cudaStream_t)stream;
-  Lanes lanes(plan, st);
+int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c, float *node_out,
+                    int keep, cudaStream_t st) {
+  int rc;
   const ZpTables &t = plan->t;
+  Lanes lanes(plan, st);
   const bool fuse1 = can_fuse(plan, 0), fuse2 = can_fuse(plan, 1);
   const bool lean = !keep && fuse1 && fuse2;          // h1 rows and y are never written
-
-  if (rl && E > 0) {
-    // the radial layer: its input and weight as planes, its output into the workspace; the
-    // largest output magnitude (which scales the rotated message) falls out of the epilogue
-    const int ec = rl->ec;
-    if (plan->fp16) {
-      ZP_TIMED(ZP_K_FOLD, zp_launch_absmax(E, ec, rl->h, ec, ws.scales + kScHr, st));
-      ZP_TIMED(ZP_K_FOLD, zp_launch_scale(1.f, ws.scales + kScHr, nullptr, nullptr, 0.f,
-                                          ws.scales + kScHrScale, st));
-      ZP_TIMED(ZP_K_FOLD, zp_launch_absmax(t.R, ec, rl->w, ec, ws.scales + kScRw, st));
-      ZP_TIMED(ZP_K_FOLD, zp_launch_scale(1.f, ws.scales + kScRw, nullptr, nullptr, 0.f,
-                                          ws.scales + kScRwScale, st));
-      ZP_CUDA(cudaMemsetAsync(ws.scales + kScRad, 0, sizeof(float), st));
-    }
-    ZP_TIMED(ZP_K_FOLD, zp_launch_split_planes(E, ec, rl->h, ec, ws.hr, st));
-    ZP_TIMED(ZP_K_FOLD, zp_launch_split_planes(t.R, ec, rl->w, ec, ws.rw, st));
-    const ZpGemmTc g{E, t.R, ec, plan->planes, ws.hr.base, ws.hr.ld, ws.hr.plane_stride, 0,
-                     ws.rw.base, ws.rw.ld, ws.rw.plane_stride, 0, rl->b, ws.radial, t.R,
-                     plan->status_dev, 0, 1, 0, 0, plan->fp16, ws.hr.scale, ws.rw.scale,
-                     plan->fp16 ? ws.scales + kScRad : nullptr};
-    ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(g, st));
-    radial = ws.radial;
-  }
-  if (plan->fp16) {
-    // magnitude bounds -> power-of-two scales, all on the device:  |rot row . x| <= sqrt(2l+1) max|x|
-    // over every row the edges can name: a caller that asks for the rows of a node range passes
-    // that range's row count as N while its edges gather from the whole array
-    int *max_node = reinterpret_cast<int *>(ws.scales + kScMaxNode);
-    ZP_TIMED(ZP_K_FOLD, zp_launch_max_index(E, src, dst, max_node, st));
-    ZP_TIMED(ZP_K_FOLD, zp_launch_absmax_row_range(x_node, (int64_t)t.K * t.C, nullptr, max_node, N,
-                                                   ws.scales + kScX, st));
-    if (!rl || E == 0)
-      ZP_TIMED(ZP_K_FOLD, zp_launch_absmax(E, t.R, radial, t.R, ws.scales + kScRad, st));
-    ZP_TIMED(ZP_K_FOLD, zp_launch_scale(3.7f, ws.scales + kScX, ws.scales + kScRad, nullptr, 0.f,
-                                        ws.scales + kScA1, st));
-    ZP_CUDA(cudaMemsetAsync(ws.scales + kScH1, 0, sizeof(float), st));
-  }
-  ZP_TIMED(ZP_K_FOLD, zp_launch_fold_weights(plan, w, ws.wfold, ws.scales + kScWeights, st));
-  ZP_TIMED(ZP_K_WIGNER_FWD, zp_launch_wigner_fwd(plan, E, edge_vec, cos_g, sin_g, ws.rot, st));
+  ZP_TIMED(ZP_K_WIGNER_FWD,
+           zp_launch_wigner_fwd(plan, c.E, c.edge_vec, c.cos_g, c.sin_g, ws.rot, st));
+  // |rot row . x| <= sqrt(2l+1) max|x|, over the rows the edges name
   ZP_TIMED(ZP_K_ROTATE_IN,
-           zp_launch_rotate_in(plan, E, x_node, src, dst, ws.rot, radial, ws.a1, st));
+           zp_launch_rotate_in(plan, c.E, c.x_node, c.src, c.dst, ws.rot, c.radial, ws.a1,
+                               zp_scale_of(3.7f, ws.scales + kScX, ws.scales + kScA1, ws.scales + kScRad),
+                               st));
+  const int64_t N = c.N, E = c.E;
+  const zp_weights *w = c.w;
   const int P = plan->planes;
   const int64_t ldy = (int64_t)t.Km * t.C;
 
@@ -608,7 +465,6 @@ static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *
       ZP_TIMED(ZP_K_GATE_FWD, zp_launch_conv1_bound(plan, ws.scales + kScA1, ws.scales + kScWeights,
                                                     w->c1_b0, ws.scales + kScHt, st));
     float *slope = plan->fp16 ? ws.scales + kScGate : nullptr;
-    if (slope) ZP_CUDA(cudaMemsetAsync(slope, 0, sizeof(float), st));
     epi.mode = ZP_EPI_GATE;
     epi.store_c = lean ? 0 : 1;
     epi.width = t.H;
@@ -655,11 +511,10 @@ static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *
       ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(g, lanes.pick(m)));
     }
     if ((rc = lanes.join())) return rc;
-    if (plan->fp16)      // |gate(h1)| <= |h1|
-      ZP_TIMED(ZP_K_GATE_FWD, zp_launch_scale(1.f, ws.scales + kScH1, nullptr, nullptr, 0.f,
-                                              ws.scales + kScHt, st));
-    ZP_TIMED(ZP_K_GATE_FWD, zp_launch_gate_fwd(plan, E, ws.h1, ws.ht,
-                                               plan->fp16 ? ws.scales + kScGate : nullptr, st));
+    // |gate(h1)| <= |h1|
+    ZP_TIMED(ZP_K_GATE_FWD,
+             zp_launch_gate_fwd(plan, E, ws.h1, ws.ht, zp_scale_of(1.f, ws.scales + kScH1, ws.scales + kScHt),
+                                plan->fp16 ? ws.scales + kScGate : nullptr, st));
   }
 
   // ---- conv2 (+ envelope, rotation back, segmented sums) ----
@@ -668,15 +523,15 @@ static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *
     epi.store_c = lean ? 0 : 1;
     epi.width = t.C;
     epi.rot = ws.rot;
-    epi.env = env;
-    epi.row_ptr = row_ptr;
+    epi.env = c.env;
+    epi.row_ptr = c.row_ptr;
     epi.n_nodes = (int)N;
     epi.nnz = t.nnz;
     epi.nnz_pad = t.nnz_pad;
     epi.head = ws.head;
     epi.cont = ws.cont;
     epi.block_node = ws.block_node;
-    ZP_TIMED(ZP_K_ROTATE_BACK, zp_launch_block_nodes(E, N, row_ptr, ws.block_node, st));
+    ZP_TIMED(ZP_K_ROTATE_BACK, zp_launch_block_nodes(E, N, c.row_ptr, ws.block_node, st));
   }
   if ((rc = lanes.fork())) return rc;
   for (int m = 0; m < plan->n_blocks && E > 0; ++m) {
@@ -694,11 +549,82 @@ static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *
   if ((rc = lanes.join())) return rc;
   if (fuse2)
     ZP_TIMED(ZP_K_ROTATE_BACK,
-             zp_launch_node_sum(plan, N, ws.head, ws.cont, row_ptr, node_out, st));
+             zp_launch_node_sum(plan, N, ws.head, ws.cont, c.row_ptr, node_out, st));
   else
     ZP_TIMED(ZP_K_ROTATE_BACK,
-             zp_launch_rotate_back_scatter(plan, N, ws.y, env, ws.rot, row_ptr, node_out, st));
+             zp_launch_rotate_back_scatter(plan, N, ws.y, c.env, ws.rot, c.row_ptr, node_out, st));
   return ZP_OK;
+}
+
+extern "C" {
+
+static int check_radial_layer(const zp_plan *plan, const ZpRadialLayer *rl, int64_t E, bool backward) {
+  if (!rl->w || !rl->b || (E && !rl->h)) return ZP_ERR_INVALID_ARG;
+  if (rl->ec <= 0 || rl->ec % 8 || plan->t.R % 8) return ZP_ERR_UNSUPPORTED;
+  if (!zp_aligned16(rl->h) || !zp_aligned16(rl->w)) return ZP_ERR_INVALID_ARG;
+  // the layer's parameter gradients are wanted together or not at all (frozen parameters)
+  if (backward && ((!rl->grad_w != !rl->grad_b) || (E && !rl->grad_h))) return ZP_ERR_INVALID_ARG;
+  return ZP_OK;
+}
+
+// keep != 0: everything a following zp_eso2_backward reads is left in the workspace
+static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *x_node,
+                        const float *edge_vec, const float *cos_g, const float *sin_g,
+                        const float *radial, const float *env, const int32_t *src,
+                        const int32_t *dst, const int32_t *row_ptr, const zp_weights *w,
+                        float *node_out, void *workspace, size_t workspace_bytes, void *stream,
+                        int keep, const ZpRadialLayer *rl = nullptr) {
+  if (!plan || N < 0 || E < 0) return ZP_ERR_INVALID_ARG;
+  if (N == 0) return E == 0 ? ZP_OK : ZP_ERR_INVALID_ARG;
+  if (!x_node || !row_ptr || !node_out || !workspace) return ZP_ERR_INVALID_ARG;
+  if (E && (!edge_vec || !cos_g || !sin_g || (!radial && !rl) || !env || !src || !dst))
+    return ZP_ERR_INVALID_ARG;
+  if (!zp_aligned16(x_node) || !zp_aligned16(node_out) || !zp_aligned16(radial) ||
+      !zp_aligned16(workspace))
+    return ZP_ERR_INVALID_ARG;
+  int rc = zp_check_weights(plan, w);
+  if (rc) return rc;
+  if (rl && (rc = check_radial_layer(plan, rl, E, false))) return rc;
+  const ZpFormat f{plan->planes, plan->fp16};
+  const ZpWorkspace ws = zp_carve(plan, N, E, keep ? 0 : 2, workspace, rl ? rl->ec : 0, f);
+  if (workspace_bytes < ws.bytes) return ZP_ERR_WORKSPACE;
+  cudaStream_t st = (cudaStream_t)stream;
+  const ZpTables &t = plan->t;
+  const bool layer = rl && E > 0;
+
+  // magnitude bounds -> power-of-two scales, all on the device; then every weight as planes
+  ZpMaxList maxima;
+  ZpPrepList prep;
+  zp_add_so2_weights(plan, w, ws.wfold, ws.scales + kScWeights, maxima, prep);
+  if (layer)
+    prep.add(rl->w, ws.rw.base, ws.scales + kScRw, ws.rw.plane_stride, t.R, rl->ec, (int)ws.rw.ld,
+             ZP_PREP_PLAIN, f.planes, f.fp16);
+  if (plan->fp16) {
+    ZP_CUDA(cudaMemsetAsync(ws.scales, 0, sizeof(float) * kScCount, st));
+    if (layer) {
+      maxima.add(rl->h, E * rl->ec, ws.scales + kScHr);
+      maxima.add(rl->w, (int64_t)t.R * rl->ec, ws.scales + kScRw);
+    } else {
+      maxima.add(radial, E * t.R, ws.scales + kScRad);
+    }
+    ZP_TIMED(ZP_K_FOLD, zp_launch_max_list(maxima, st));
+    // over every row the edges can name: a caller that asks for the rows of a node range passes
+    // that range's row count as N while its edges gather from the whole array
+    int *max_node = reinterpret_cast<int *>(ws.scales + kScMaxNode);
+    ZP_TIMED(ZP_K_FOLD, zp_launch_max_index(E, src, dst, max_node, st));
+    ZP_TIMED(ZP_K_FOLD, zp_launch_absmax_row_range(x_node, (int64_t)t.K * t.C, nullptr, max_node, N,
+                                                   ws.scales + kScX, st));
+  }
+  ZP_TIMED(ZP_K_FOLD, zp_launch_prep_weights(prep, st));
+  ZpConv c{N, E, x_node, edge_vec, cos_g, sin_g, radial, env, src, dst, row_ptr, nullptr, nullptr, w};
+  if (layer) {
+    ZP_TIMED(ZP_K_FOLD, zp_launch_split_planes(E, rl->ec, rl->h, rl->ec, ws.hr,
+                                               zp_scale_of(1.f, ws.scales + kScHr, ws.scales + kScHrScale),
+                                               st));
+    if ((rc = zp_core_radial(plan, ws, E, rl->ec, rl->b, st))) return rc;
+    c.radial = ws.radial;
+  }
+  return zp_core_forward(plan, ws, c, node_out, keep, st);
 }
 
 int zp_eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *x_node,
@@ -720,67 +646,41 @@ int zp_eso2_forward_inference(const zp_plan *plan, int64_t N, int64_t E, const f
                       w, node_out, workspace, workspace_bytes, stream, 0);
 }
 
-static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float *grad_node_out,
-                         const float *x_node, const float *edge_vec, const float *cos_g,
-                         const float *sin_g, const float *radial, const float *env,
-                         const int32_t *src, const int32_t *dst, const int32_t *row_ptr,
-                         const int32_t *perm_src, const int32_t *row_ptr_src, const zp_weights *w,
-                         float *grad_x_node, float *grad_edge_vec, float *grad_radial,
-                         float *grad_env, const zp_weight_grads *gw, void *workspace,
-                         size_t workspace_bytes, void *stream, const RadialLayer *rl) {
-  if (!plan || N < 0 || E < 0) return ZP_ERR_INVALID_ARG;
-  if (N == 0) return E == 0 ? ZP_OK : ZP_ERR_INVALID_ARG;
-  if (!grad_node_out || !x_node || !row_ptr || !row_ptr_src || !workspace)
-    return ZP_ERR_INVALID_ARG;
+}  // extern "C"
+
+int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
+                     const float *grad_node_out, float *grad_x_node, float *grad_edge_vec,
+                     float *grad_radial, float *grad_env, const zp_weight_grads *gw,
+                     const ZpRadialLayer *rl, ZpFinalList &list, cudaStream_t st) {
+  int rc;
+  const int64_t N = c.N, E = c.E;
   // gw == NULL: the parameters are frozen (an MD / inference force evaluation): no weight-gradient
   // product, no bias column sum, no unfolding
   const bool want_w = gw != nullptr;
-  if (E && (!edge_vec || !cos_g || !sin_g || (!radial && !rl) || !env || !src || !dst || !perm_src ||
-            !grad_edge_vec || (!grad_radial && !rl) || !grad_env))
-    return ZP_ERR_INVALID_ARG;
-  if (want_w) {
-    if (!gw->c1_w0 || !gw->c1_b0 || !gw->c2_w0 || !gw->c2_b0) return ZP_ERR_INVALID_ARG;
-    for (int m = 1; m < plan->n_blocks; ++m)
-      if (!gw->c1_wm || !gw->c2_wm || !gw->c1_wm[m - 1] || !gw->c2_wm[m - 1])
-        return ZP_ERR_INVALID_ARG;
-  }
-  if (!aligned16(grad_node_out) || !aligned16(grad_x_node) || !aligned16(grad_radial) ||
-      !aligned16(workspace))   /* a null grad_radial (radial layer inside the call) is aligned */
-    return ZP_ERR_INVALID_ARG;
-  int rc = check_weights(plan, w);
-  if (rc) return rc;
-  if (rl && (rc = check_radial_layer(plan, rl, E, true))) return rc;
-  // (the node count only sizes regions that live inside the forward)
-  const Workspace ws = carve(plan, 0, E, 1, workspace, rl ? rl->ec : 0);
-  if (workspace_bytes < ws.bytes) return ZP_ERR_WORKSPACE;
-  if (rl) radial = ws.radial;            // left there by the forward
   // grad_x_node == NULL: the embeddings are an input without a gradient (E and dE/dpos of one
   // block): the per-edge contributions are neither written nor summed
   float *du_out = grad_x_node ? ws.du_src : nullptr;
-  cudaStream_t st = (cudaStream_t)stream;
   Lanes lanes(plan, st);
   const ZpTables &t = plan->t;
   const int P = plan->planes;
   const int64_t lda = (int64_t)t.Km * 2 * t.C, ldh = (int64_t)t.Km * t.H;
   int splits_c1[ZP_MAX_L + 1], splits_c2[ZP_MAX_L + 1];
-  int sms = 148;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, plan->device);
+  const float *radial = rl ? ws.radial : c.radial;      // rl: left there by the forward
 
-  if (plan->fp16) {
+  const bool scaled_gr = rl && ws.gr.fp16;               // the planes of grad_radial have a scale
+  if (plan->fp16 || scaled_gr)
+    ZP_CUDA(cudaMemsetAsync(ws.scales + kScBwd, 0, sizeof(float) * (kScBwdEnd - kScBwd), st));
+  if (plan->fp16 && E > 0) {
     // only rows dst[0] .. dst[E-1] (the edges are destination-sorted): the rows the kernels read,
     // and the only ones a caller that holds a node range's rows alone has
-    if (E > 0)
-      ZP_TIMED(ZP_K_ROTATE_GRAD_OUT,
-               zp_launch_absmax_row_range(grad_node_out, (int64_t)t.K * t.C, dst, dst + (E - 1), 0,
-                                          ws.scales + kScG, st));
-    else
-      ZP_CUDA(cudaMemsetAsync(ws.scales + kScG, 0, sizeof(float), st));
-    ZP_TIMED(ZP_K_ROTATE_GRAD_OUT, zp_launch_scale(3.7f, ws.scales + kScG, nullptr, nullptr, 0.f,
-                                                   ws.scales + kScDy, st));
+    ZP_TIMED(ZP_K_ROTATE_GRAD_OUT,
+             zp_launch_absmax_row_range(grad_node_out, (int64_t)t.K * t.C, c.dst, c.dst + (E - 1), 0,
+                                        ws.scales + kScG, st));
   }
   ZP_TIMED(ZP_K_ROTATE_GRAD_OUT,
-           zp_launch_rotate_grad_out(plan, E, grad_node_out, ws.y, env, ws.rot, dst, ws.dy,
-                                     grad_env, ws.grot, st));
+           zp_launch_rotate_grad_out(plan, E, grad_node_out, ws.y, c.env, ws.rot, c.dst, ws.dy,
+                                     zp_scale_of(3.7f, ws.scales + kScG, ws.scales + kScDy), grad_env,
+                                     ws.grot, st));
   // One conv at a time: input gradient dX = dY W_fold (K-major against the transposed planes),
   // weight gradient dW_fold = dY^T X with both operands MN-major (the contraction runs over
   // edges), bias gradient = column sums of dY.
@@ -791,15 +691,13 @@ static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float 
     const int64_t ldx = conv ? ldh : lda;
     const int cin = conv ? t.H : 2 * t.C, cout = conv ? t.C : t.H;
     if (conv == 0) {
-      if (plan->fp16 && rl) ZP_CUDA(cudaMemsetAsync(ws.scales + kScDa1, 0, sizeof(float), st));
-      if (plan->fp16)        // |dh1| <= 1.1 max|dht| max(1, rows * max sigmoid' * max|h1|)
-        ZP_TIMED(ZP_K_GATE_BWD,
-                 zp_launch_scale(1.1f, ws.scales + kScDht, nullptr, ws.scales + kScGate, 1.f,
-                                 ws.scales + kScDh1, st, ws.scales + kScH1,
-                                 (float)(2 * t.mmax + 1)));
-      ZP_TIMED(ZP_K_GATE_BWD, zp_launch_gate_bwd(plan, E, ws.h1, ws.dht, ws.dh1, st));
-    } else if (plan->fp16) {
-      ZP_CUDA(cudaMemsetAsync(ws.scales + kScDht, 0, sizeof(float), st));
+      // |dh1| <= 1.1 max|dht| max(1, rows * max sigmoid' * max|h1|)
+      ZpScale dh1_scale = zp_scale_of(1.1f, ws.scales + kScDht, ws.scales + kScDh1);
+      dh1_scale.c = ws.scales + kScGate;
+      dh1_scale.d = ws.scales + kScH1;
+      dh1_scale.offset = 1.f;
+      dh1_scale.c_factor = (float)(2 * t.mmax + 1);
+      ZP_TIMED(ZP_K_GATE_BWD, zp_launch_gate_bwd(plan, E, ws.h1, ws.dht, ws.dh1, dh1_scale, st));
     }
     // the input- and weight-gradient products of the blocks and the bias column sums only read
     // dY, X and the weights: side by side on the plan's streams
@@ -825,56 +723,94 @@ static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float 
                         plan->status_dev, 0, 1, 0, 0, plan->fp16, dYm.scale,
                         wscale(plan, ws, conv, m),
                         // max |dht|; max |da1| when the radial layer's gradient needs it
-                        !plan->fp16 ? nullptr : conv ? ws.scales + kScDht
-                                                     : rl ? ws.scales + kScDa1 : nullptr};
+                        conv ? (plan->fp16 ? ws.scales + kScDht : nullptr)
+                             : (scaled_gr ? ws.scales + kScDa1 : nullptr)};
       ZP_TIMED(ZP_K_GEMM_DGRAD, zp_launch_gemm_tc(gd, lanes.pick(want_w ? 2 * m : m)));
       if (!want_w) continue;
       ZpGemmTc gw_{out, in, E, P, dYm.base, dYm.ld, dYm.plane_stride, 1,
                    Xm.base, Xm.ld, Xm.plane_stride, 1, nullptr, G, in,
                    plan->status_dev, 0, 1, plan->g_elems, 0, plan->fp16, dYm.scale, Xm.scale,
                    nullptr};
-      gw_.ksplit = zp_gemm_tc_pick_splits(gw_, kMaxWgradSplits);
+      gw_.ksplit = zp_gemm_tc_pick_splits(gw_, kZpWgradSplits);
       nsplit = zp_gemm_tc_splits(gw_);
       ZP_TIMED(ZP_K_GEMM_WGRAD, zp_launch_gemm_tc(gw_, lanes.pick(2 * m + 1)));
     }
     if (want_w)
       ZP_TIMED(ZP_K_BIAS_GRAD,
                zp_launch_colsum(E, conv ? plan->c2_out[0] : plan->c1_out[0], dYp,
-                                conv ? gw->c2_b0 : gw->c1_b0, ws.scratch, lanes.pick(2)));
+                                conv ? gw->c2_b0 : gw->c1_b0, conv ? ws.col2 : ws.col1, list,
+                                lanes.pick(2)));
     if ((rc = lanes.join())) return rc;
   }
-  if (rl) {
-    // grad_radial leaves the kernel as operand planes for the layer's VJP; their scale comes from
-    // |grad_radial| <= 2 max|da1| max|rot . x| <= 2 * 3.7 max|da1| max|x|
-    if (plan->fp16)
-      ZP_TIMED(ZP_K_ROTATE_IN_BWD, zp_launch_scale(7.4f, ws.scales + kScDa1, ws.scales + kScX, nullptr,
-                                                   0.f, ws.scales + kScGrScale, st));
-    ZP_TIMED(ZP_K_ROTATE_IN_BWD,
-             zp_launch_rotate_in_bwd(plan, E, ws.da1, radial, x_node, src, dst, ws.rot,
-                                     nullptr, du_out, ws.grot, st, &ws.gr));
-    if (E > 0) {
-      ZP_TIMED(ZP_K_GEMM_WGRAD,
-               zp_linear_backward_planes(plan, E, rl->ec, t.R, ws.hr, ws.rw, ws.gr, rl->grad_h,
-                                         rl->grad_w, rl->grad_b, ws.rad_partials, kRadialSplits,
-                                         ws.scratch, st));
-    } else if (rl->grad_w) {
-      ZP_CUDA(cudaMemsetAsync(rl->grad_w, 0, sizeof(float) * (size_t)t.R * rl->ec, st));
-      ZP_CUDA(cudaMemsetAsync(rl->grad_b, 0, sizeof(float) * (size_t)t.R, st));
-    }
-  } else {
-    ZP_TIMED(ZP_K_ROTATE_IN_BWD,
-             zp_launch_rotate_in_bwd(plan, E, ws.da1, radial, x_node, src, dst, ws.rot,
-                                     grad_radial, du_out, ws.grot, st));
+  // With the layer inside the call grad_radial leaves the kernel as operand planes for the layer's
+  // VJP; their scale comes from |grad_radial| <= 2 max|da1| max|rot . x| <= 2 * 3.7 max|da1| max|x|
+  ZP_TIMED(ZP_K_ROTATE_IN_BWD,
+           zp_launch_rotate_in_bwd(plan, E, ws.da1, radial, c.x_node, c.src, c.dst, ws.rot,
+                                   rl ? nullptr : grad_radial, du_out, ws.grot, st,
+                                   rl ? &ws.gr : nullptr,
+                                   zp_scale_of(7.4f, ws.scales + kScDa1, ws.scales + kScGrScale,
+                                               ws.scales + kScX)));
+  if (rl && E > 0) {
+    ZP_TIMED(ZP_K_GEMM_WGRAD,
+             zp_linear_backward_planes(plan, E, rl->ec, t.R, ws.hr, ws.rw, ws.gr, rl->grad_h,
+                                       rl->grad_w, rl->grad_b, ws.rad_partials, kZpRadialSplits,
+                                       ws.col_rad, list, st, rl->grad_h_max));
+  } else if (rl && rl->grad_w) {
+    ZP_CUDA(cudaMemsetAsync(rl->grad_w, 0, sizeof(float) * (size_t)t.R * rl->ec, st));
+    ZP_CUDA(cudaMemsetAsync(rl->grad_b, 0, sizeof(float) * (size_t)t.R, st));
   }
   if (grad_x_node)
     ZP_TIMED(ZP_K_SRC_REDUCE,
-             zp_launch_node_reduce(plan, N, ws.du_src, row_ptr, perm_src, row_ptr_src,
+             zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
                                    grad_x_node, st));
   ZP_TIMED(ZP_K_WIGNER_BWD,
-           zp_launch_wigner_bwd(plan, E, edge_vec, cos_g, sin_g, ws.grot, grad_edge_vec, st));
+           zp_launch_wigner_bwd(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.grot, grad_edge_vec, st));
   if (want_w)
-    ZP_TIMED(ZP_K_FOLD, zp_launch_unfold_wgrad(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2,
-                                               gw, st));
+    zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
+  return ZP_OK;
+}
+
+extern "C" {
+
+static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float *grad_node_out,
+                         const float *x_node, const float *edge_vec, const float *cos_g,
+                         const float *sin_g, const float *radial, const float *env,
+                         const int32_t *src, const int32_t *dst, const int32_t *row_ptr,
+                         const int32_t *perm_src, const int32_t *row_ptr_src, const zp_weights *w,
+                         float *grad_x_node, float *grad_edge_vec, float *grad_radial,
+                         float *grad_env, const zp_weight_grads *gw, void *workspace,
+                         size_t workspace_bytes, void *stream, const ZpRadialLayer *rl) {
+  if (!plan || N < 0 || E < 0) return ZP_ERR_INVALID_ARG;
+  if (N == 0) return E == 0 ? ZP_OK : ZP_ERR_INVALID_ARG;
+  if (!grad_node_out || !x_node || !row_ptr || !row_ptr_src || !workspace)
+    return ZP_ERR_INVALID_ARG;
+  if (E && (!edge_vec || !cos_g || !sin_g || (!radial && !rl) || !env || !src || !dst || !perm_src ||
+            !grad_edge_vec || (!grad_radial && !rl) || !grad_env))
+    return ZP_ERR_INVALID_ARG;
+  if (gw) {
+    if (!gw->c1_w0 || !gw->c1_b0 || !gw->c2_w0 || !gw->c2_b0) return ZP_ERR_INVALID_ARG;
+    for (int m = 1; m < plan->n_blocks; ++m)
+      if (!gw->c1_wm || !gw->c2_wm || !gw->c1_wm[m - 1] || !gw->c2_wm[m - 1])
+        return ZP_ERR_INVALID_ARG;
+  }
+  if (!zp_aligned16(grad_node_out) || !zp_aligned16(grad_x_node) || !zp_aligned16(grad_radial) ||
+      !zp_aligned16(workspace))   /* a null grad_radial (radial layer inside the call) is aligned */
+    return ZP_ERR_INVALID_ARG;
+  int rc = zp_check_weights(plan, w);
+  if (rc) return rc;
+  if (rl && (rc = check_radial_layer(plan, rl, E, true))) return rc;
+  // (the node count only sizes regions that live inside the forward)
+  const ZpFormat f{plan->planes, plan->fp16};
+  const ZpWorkspace ws = zp_carve(plan, 0, E, 1, workspace, rl ? rl->ec : 0, f);
+  if (workspace_bytes < ws.bytes) return ZP_ERR_WORKSPACE;
+  cudaStream_t st = (cudaStream_t)stream;
+  const ZpConv c{N, E, x_node, edge_vec, cos_g, sin_g, radial, env, src, dst, row_ptr, perm_src,
+                 row_ptr_src, w};
+  ZpFinalList list;
+  if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, grad_edge_vec, grad_radial,
+                             grad_env, gw, rl, list, st)))
+    return rc;
+  ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, st));
   return ZP_OK;
 }
 
@@ -896,7 +832,9 @@ size_t zp_workspace_bytes_radial(const zp_plan *plan, int64_t n_nodes, int64_t n
   if (!plan || n_nodes < 0 || n_edges < 0 || with_backward < 0 || with_backward > 2 ||
       edge_channels <= 0 || edge_channels % 8)
     return 0;
-  return carve(plan, n_nodes, n_edges, with_backward, nullptr, edge_channels).bytes;
+  return zp_carve(plan, n_nodes, n_edges, with_backward, nullptr, edge_channels,
+                  ZpFormat{plan->planes, plan->fp16})
+      .bytes;
 }
 
 int zp_eso2_forward_radial(const zp_plan *plan, int64_t N, int64_t E, const float *x_node,
@@ -906,7 +844,7 @@ int zp_eso2_forward_radial(const zp_plan *plan, int64_t N, int64_t E, const floa
                            const int32_t *dst, const int32_t *row_ptr, const zp_weights *w,
                            float *node_out, void *workspace, size_t workspace_bytes,
                            int keep_for_backward, void *stream) {
-  const RadialLayer rl{h_rad, rad_w, rad_b, edge_channels, nullptr, nullptr, nullptr};
+  const ZpRadialLayer rl{h_rad, rad_w, rad_b, edge_channels, nullptr, nullptr, nullptr, nullptr};
   return eso2_forward(plan, N, E, x_node, edge_vec, cos_g, sin_g, nullptr, env, src, dst, row_ptr,
                       w, node_out, workspace, workspace_bytes, stream, keep_for_backward, &rl);
 }
@@ -921,7 +859,8 @@ int zp_eso2_backward_radial(const zp_plan *plan, int64_t N, int64_t E, const flo
                             float *grad_h_rad, float *grad_rad_w, float *grad_rad_b,
                             float *grad_env, const zp_weight_grads *gw, void *workspace,
                             size_t workspace_bytes, void *stream) {
-  const RadialLayer rl{h_rad, rad_w, rad_b, edge_channels, grad_h_rad, grad_rad_w, grad_rad_b};
+  const ZpRadialLayer rl{h_rad, rad_w, rad_b, edge_channels, grad_h_rad, grad_rad_w, grad_rad_b,
+                         nullptr};
   return eso2_backward(plan, N, E, grad_node_out, x_node, edge_vec, cos_g, sin_g, nullptr, env, src,
                        dst, row_ptr, perm_src, row_ptr_src, w, grad_x_node, grad_edge_vec, nullptr,
                        grad_env, gw, workspace, workspace_bytes, stream, &rl);

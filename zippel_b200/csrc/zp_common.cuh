@@ -107,6 +107,49 @@ int zp_ensure_smem(Kernel kernel, size_t bytes, ZpSmemOptIn &state) {
   return ZP_OK;
 }
 
+// ---- lists of small jobs that share one launch (blockIdx.y = entry) ---------------------------
+#define ZP_MAX_ITEMS 32
+struct ZpMaxList {                              // *out = max |x[0 .. count)|, out zeroed beforehand
+  int n = 0;
+  const float *x[ZP_MAX_ITEMS];
+  int64_t count[ZP_MAX_ITEMS];
+  float *out[ZP_MAX_ITEMS];
+  void add(const float *src, int64_t cnt, float *slot) {
+    x[n] = src; count[n] = cnt; out[n++] = slot;
+  }
+};
+enum { ZP_PREP_PLAIN = 0, ZP_PREP_KEPT = 1, ZP_PREP_FOLDED = 2 };
+struct ZpPrepList {                             // weight matrices to 16-bit planes
+  int n = 0;
+  const float *w[ZP_MAX_ITEMS];
+  uint16_t *dst[ZP_MAX_ITEMS];
+  float *slot[ZP_MAX_ITEMS];                    // {max |W|, scale}
+  int64_t plane_stride[ZP_MAX_ITEMS];
+  int out[ZP_MAX_ITEMS], in[ZP_MAX_ITEMS], ld[ZP_MAX_ITEMS];
+  int8_t kind[ZP_MAX_ITEMS], planes[ZP_MAX_ITEMS], fp16[ZP_MAX_ITEMS];
+  void add(const float *src, void *to, float *max_and_scale, int64_t stride, int rows, int cols,
+           int row_stride, int what, int n_planes, int is_fp16) {
+    w[n] = src; dst[n] = static_cast<uint16_t *>(to); slot[n] = max_and_scale;
+    plane_stride[n] = stride; out[n] = rows; in[n] = cols; ld[n] = row_stride;
+    kind[n] = (int8_t)what; planes[n] = (int8_t)n_planes; fp16[n++] = (int8_t)is_fp16;
+  }
+};
+enum { ZP_FIN_SUM = 0, ZP_FIN_UNFOLD = 1, ZP_FIN_COLUMN = 2 };
+struct ZpFinalList {                            // last sums of the parameter gradients
+  int n = 0;
+  const float *src[ZP_MAX_ITEMS];
+  float *dst[ZP_MAX_ITEMS];
+  int64_t stride[ZP_MAX_ITEMS];                 // elements between partials
+  int rows[ZP_MAX_ITEMS], cols[ZP_MAX_ITEMS], parts[ZP_MAX_ITEMS];
+  int ld[ZP_MAX_ITEMS];                         // row stride of a partial
+  int8_t kind[ZP_MAX_ITEMS];
+  void add(const float *partials, float *to, int64_t between, int n_rows, int n_cols, int n_parts,
+           int what, int row_stride = 0) {
+    src[n] = partials; dst[n] = to; stride[n] = between; ld[n] = row_stride ? row_stride : n_cols;
+    rows[n] = n_rows; cols[n] = n_cols; parts[n] = n_parts; kind[n++] = (int8_t)what;
+  }
+};
+
 static inline int64_t zp_ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline size_t zp_align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -130,20 +173,21 @@ int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const flo
 
 int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32_t *src,
                         const int32_t *dst, const float *rot, const float *radial,
-                        const ZpPlanes &a1, cudaStream_t st);
+                        const ZpPlanes &a1, const ZpScale &scale, cudaStream_t st);
 int zp_launch_rotate_back_scatter(const zp_plan *p, int64_t N, const float *y, const float *env,
                                   const float *rot, const int32_t *row_ptr, float *node_out,
                                   cudaStream_t st);
 int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const float *y,
                               const float *env, const float *rot, const int32_t *dst,
-                              const ZpPlanes &dy, float *grad_env, float *grad_rot,
-                              cudaStream_t st);
+                              const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
+                              float *grad_rot, cudaStream_t st);
 // du_both [E][2][K][C]: per-edge contributions to grad_x of the source (0) and destination (1)
 // grad_radial goes out as fp32 rows [E, R], or (grad_radial_planes given) as operand planes
 int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const float *radial,
                             const float *x, const int32_t *src, const int32_t *dst,
                             const float *rot, float *grad_radial, float *du_both, float *grad_rot,
-                            cudaStream_t st, const ZpPlanes *grad_radial_planes = nullptr);
+                            cudaStream_t st, const ZpPlanes *grad_radial_planes,
+                            const ZpScale &scale);
 // node_out[n, l^2 + j, c] = sum over the m' rows r of degree l, in table order, of
 //   head[n][rot_off[r] + j][c] + the continuation partials of the 32-edge blocks n's edges reach
 int zp_launch_node_sum(const zp_plan *p, int64_t N, const float *head, const float *cont,
@@ -153,10 +197,10 @@ int zp_launch_node_reduce(const zp_plan *p, int64_t N, const float *du_both,
                           const int32_t *row_ptr_src, float *grad_x, cudaStream_t st);
 
 int zp_launch_gate_fwd(const zp_plan *p, int64_t E, const float *h1, const ZpPlanes &ht,
-                       float *gate_max, cudaStream_t st);
+                       const ZpScale &scale, float *gate_max, cudaStream_t st);
 // gate_max (device scalar, may be null): largest sigmoid'(gate) seen by the forward
 int zp_launch_gate_bwd(const zp_plan *p, int64_t E, const float *h1, const float *dht,
-                       const ZpPlanes &dh1, cudaStream_t st);
+                       const ZpPlanes &dh1, const ZpScale &scale, cudaStream_t st);
 
 // Work the contraction's epilogue does on a finished 32-row x 32-column block of the result
 // while it is still on chip (staged in shared memory), besides or instead of storing it.
@@ -227,42 +271,77 @@ int zp_gemm_tc_splits(const ZpGemmTc &g);
 int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits);
 // fp32 [rows, cols] (row stride ld_in) -> planes [rows, out.ld], zero padded
 int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,
-                           const ZpPlanes &out, cudaStream_t st);
-// *out = max |in| (device scalar)
-int zp_launch_absmax(int64_t rows, int64_t cols, const float *in, int64_t ld, float *out,
-                     cudaStream_t st);
-// *out = largest node index in src / dst (device scalar)
+                           const ZpPlanes &out, const ZpScale &scale, cudaStream_t st);
+int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st);
+int zp_launch_prep_weights(const ZpPrepList &list, cudaStream_t st);
+int zp_launch_finalize(const ZpFinalList &list, cudaStream_t st);
+// *out = largest node index in src / dst (device scalar, zeroed by the caller)
 int zp_launch_max_index(int64_t E, const int32_t *src, const int32_t *dst, int *out,
                         cudaStream_t st);
 // *out = max |in| over rows [first ? *first : 0, max(min_rows, last ? *last + 1 : 0)) of a
-// contiguous [*, cols] matrix; first / last are device pointers to row numbers
+// contiguous [*, cols] matrix; first / last are device pointers to row numbers, *out was zeroed
 int zp_launch_absmax_row_range(const float *in, int64_t cols, const int32_t *first,
                                const int32_t *last, int64_t min_rows, float *out,
                                cudaStream_t st);
-// *scale = power of two mapping factor*a*b*max(offset_c, c_factor*c*d) to 2^15 (device scalars;
-// null = 1; without c the max term is left out)
-int zp_launch_scale(float factor, const float *a, const float *b, const float *c, float offset_c,
-                    float *scale, cudaStream_t st, const float *d = nullptr, float c_factor = 1.f);
 
-// Folded SO(2) weights as bf16 planes: per block W_fold [P][out][in] followed by its transpose
-// [P][in][out], at element offset c{1,2}_woff[m] of `packed`.
-// `scales`: per block (conv * (ZP_MAX_L+1) + m) two floats {max |W|, scale}; used for fp16 planes
-int zp_launch_fold_weights(const zp_plan *p, const zp_weights *w, void *packed, float *scales,
-                           cudaStream_t st);
-// partials: per split s the folded fp32 gradients at partials + s*split_stride + c{1,2}_goff[m]
-int zp_launch_unfold_wgrad(const zp_plan *p, const float *partials, int64_t split_stride,
-                           const int *splits_c1, const int *splits_c2, const zp_weight_grads *gw,
-                           cudaStream_t st);
+// The SO(2) weight blocks of both convolutions, for zp_launch_max_list (fp16 planes) and
+// zp_launch_prep_weights: per block W_fold [P][out][in] followed by its transpose [P][in][out], at
+// element offset c{1,2}_woff[m] of `packed`; `scales`: per block (conv * (ZP_MAX_L+1) + m) two
+// floats {max |W|, scale}.
+void zp_add_so2_weights(const zp_plan *p, const zp_weights *w, void *packed, float *scales,
+                        ZpMaxList &maxima, ZpPrepList &prep);
+// ... and their gradients, for zp_launch_finalize: per split s the folded fp32 gradients stand at
+// partials + s*split_stride + c{1,2}_goff[m]
+void zp_add_so2_grads(const zp_plan *p, const float *partials, int64_t split_stride,
+                      const int *splits_c1, const int *splits_c2, const zp_weight_grads *gw,
+                      ZpFinalList &list);
 // *ht_scale = fp16-plane scale of conv1's activated output from an a-priori bound:
 //   |h1| <= max_m(in_m * max|a1| * max|W1_m|) + max|b1|,  |gate_act(h1)| <= |h1|
 // (a1_scale maps the bound of a1 to 2^15; wscales: {max, scale} pairs per weight block)
 int zp_launch_conv1_bound(const zp_plan *p, const float *a1_scale, const float *wscales,
                           const float *bias, float *ht_scale, cudaStream_t st);
-// VJP of y = x W^T + b with all operands as planes; `partials`: max_splits * N * K floats,
-// `colsum_scratch`: ceil(M / 128) * N floats (only when db is wanted)
+// LayerNorm + SiLU over rows of `width` floats.  The result goes out as fp32 rows (y / dx) or, with
+// y_planes / dx_planes given, as operand planes of the next product; rstd_max: device scalar updated
+// with the largest 1/std (or null).  Backward: dgamma null = no parameter gradients; dbias = column
+// sums of dx (or null); `partial`: ZP_LN_PARTIALS * 3 * width floats.
+#define ZP_LN_PARTIALS 296
+int zp_launch_ln_silu_fwd(int64_t rows, int width, const float *x, const float *gamma,
+                          const float *beta, float eps, float *y, const ZpPlanes *y_planes,
+                          const ZpScale &scale, float *mean, float *rstd, float *rstd_max,
+                          cudaStream_t st);
+int zp_launch_ln_silu_bwd(int64_t rows, int width, const float *x, const float *gamma,
+                          const float *beta, const float *mean, const float *rstd, const float *dy,
+                          float *dx, const ZpPlanes *dx_planes, const ZpScale &scale,
+                          float *dgamma, float *dbeta, float *dbias, float *partial,
+                          ZpFinalList &list, cudaStream_t st);
+// VJP of y = x W^T + b with all operands as planes (of one format); `partials`: max_splits * N *
+// round4(K) floats, `colsum_scratch`: ceil(M / 512) * N floats.  dw and db get their last sums from `list`
+// (zp_launch_finalize); dx_absmax: device scalar updated with max |dx|, or null; dx_cols: how many
+// leading columns of dx are wanted (0: all K), ld_dx its row stride (0: K)
 int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t N,
                               const ZpPlanes &x, const ZpPlanes &w, const ZpPlanes &dy, float *dx,
                               float *dw, float *db, float *partials, int max_splits,
-                              float *colsum_scratch, cudaStream_t st);
+                              float *colsum_scratch, ZpFinalList &list, cudaStream_t st,
+                              float *dx_absmax = nullptr, int64_t dx_cols = 0);
+// column sums of `a`: partial sums into scratch (ceil(rows / 512) * cols floats), the rest by `list`
 int zp_launch_colsum(int64_t rows, int64_t cols, const ZpPlanes &a, float *out, float *scratch,
-                     cudaStream_t st);
+                     ZpFinalList &list, cudaStream_t st);
+
+// The per-edge front end.  x_planes given: the input of the radial MLP goes out as operand planes
+// (zero padded to their row stride) instead of fp32 rows.
+int zp_launch_edge_features_fwd(const zp_front_config &cfg, int64_t E, const float *pos,
+                                const float *shifts, const int64_t *atomic_numbers, const float *emb,
+                                const float *gauss_offsets, const float *cos_g, const float *sin_g,
+                                const int32_t *perm, const int32_t *src, const int32_t *dst,
+                                float *edge_vec, float *dist, float *x_edge,
+                                const ZpPlanes *x_planes, const ZpScale &scale, float *env,
+                                float *cos_sorted, float *sin_sorted, cudaStream_t st);
+// grad_x_edge [E, ldg]: all columns when grad_emb is wanted, at least the num_basis leading ones
+// otherwise; grad_pos or grad_emb may be null
+int zp_launch_edge_features_bwd(const zp_front_config &cfg, int64_t N, int64_t E,
+                                const float *edge_vec, const float *dist,
+                                const float *gauss_offsets, const int64_t *atomic_numbers,
+                                const float *grad_edge_vec, const float *grad_x_edge, int64_t ldg,
+                                const float *grad_env, const int32_t *row_ptr,
+                                const int32_t *perm_src, const int32_t *row_ptr_src,
+                                float *grad_pos, float *grad_emb, void *work, cudaStream_t st);

@@ -1,0 +1,140 @@
+// The edge convolution's workspace and the launch sequences shared by the C-ABI entry points of
+// the convolution alone (zp_api.cu) and of the whole block (zp_block.cu).
+#pragma once
+
+#include <cstring>
+#include <vector>
+
+#include "zp_common.cuh"
+
+// Event pairs recorded around kernel classes while timing is on.
+struct ZpTimer {
+  struct Span { int cls; cudaEvent_t a, b; int64_t launches; };
+  std::vector<Span> spans;      // pool; `used` of them hold live records
+  size_t used = 0;
+  Span *open(int cls, cudaStream_t st) {
+    if (used == spans.size()) {
+      Span s{cls, nullptr, nullptr, 0};
+      if (cudaEventCreate(&s.a) != cudaSuccess || cudaEventCreate(&s.b) != cudaSuccess) return nullptr;
+      spans.push_back(s);
+    }
+    Span *s = &spans[used++];
+    s->cls = cls;
+    s->launches = zp_launch_counter();
+    cudaEventRecord(s->a, st);
+    return s;
+  }
+  static void close(Span *s, cudaStream_t st) {
+    if (!s) return;
+    cudaEventRecord(s->b, st);
+    s->launches = zp_launch_counter() - s->launches;
+  }
+};
+
+// brackets one expression with a timing span when the plan has a timer
+#define ZP_TIMED(cls, expr)                                                      \
+  do {                                                                           \
+    ZpTimer::Span *span_ = plan->timer ? plan->timer->open(cls, st) : nullptr;   \
+    rc = (expr);                                                                 \
+    ZpTimer::close(span_, st);                                                   \
+    if (rc) return rc;                                                           \
+  } while (0)
+
+inline bool zp_aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline int64_t zp_round8(int64_t x) { return (x + 7) / 8 * 8; }
+
+// 16-bit operand format of a product: number of planes and element type
+struct ZpFormat {
+  int planes, fp16;
+};
+
+// Carves regions out of one buffer (or, with a null base, measures them); each starts 256-byte
+// aligned.
+struct ZpCarver {
+  char *base;
+  size_t off = 0;
+  explicit ZpCarver(void *b) : base(static_cast<char *>(b)) {}
+  char *bytes(size_t n) {
+    char *p = base ? base + off : nullptr;
+    off += zp_align_up(n, 256);
+    return p;
+  }
+  float *floats(size_t n) { return reinterpret_cast<float *>(bytes(n * sizeof(float))); }
+  ZpPlanes planes(int64_t rows, int64_t cols, ZpFormat f, const float *scale) {
+    ZpPlanes pl;
+    pl.ld = zp_round8(cols);
+    pl.planes = f.planes;
+    pl.fp16 = f.fp16;
+    pl.scale = base && f.fp16 ? scale : nullptr;
+    pl.plane_stride = (int64_t)zp_align_up((size_t)rows * pl.ld, 128);
+    pl.base = bytes((size_t)pl.planes * pl.plane_stride * 2);
+    return pl;
+  }
+};
+
+// Device-side scale array (fp16 planes): raw maxima, derived scales, and per weight block
+// {max |W|, scale} from kScWeights on.  One memset at the start of a forward clears it; a backward
+// clears the maxima it accumulates itself, kScBwd .. kScBwdEnd.
+enum { kScX = 0, kScRad, kScH1, kScA1, kScHt, kScDy, kScDh1, kScGate, kScMaxNode /* an int */,
+       // the radial layer run inside the call: {max, scale} of its input and of its weight, scale
+       // of the planes of grad_radial
+       kScHr, kScHrScale, kScRw, kScRwScale, kScGrScale,
+       kScBwd, kScG = kScBwd, kScDht, kScDa1, kScBwdEnd,
+       kScWeights = 24,
+       kScCount = kScWeights + 4 * (ZP_MAX_L + 1) };
+
+constexpr int kZpWgradSplits = 8;
+constexpr int kZpRadialSplits = 8;       // K splits of the radial layer's weight gradient
+constexpr int kZpColRows = 512;          // rows per partial column sum
+
+//   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials
+//   backward: dy planes | dht | dh1 planes | da1 | du_src | grot | wgrad partials | scratch
+// mode 0 / 1: forward that keeps what a backward reads (1: plus the backward's own regions);
+// mode 2: forward alone with fused epilogues -- of h1 only the gate scalars exist, y does not.
+struct ZpWorkspace {
+  float *rot, *h1, *y, *dht, *da1, *du_src, *grot, *wgrad, *scales, *head, *cont;
+  float *col1, *col2, *col_rad;          // partial column sums: bias gradients of conv1, conv2, radial
+  float *radial, *rad_partials;          // radial layer inside the call: its output, dW partials
+  int64_t ld_h1;
+  int32_t *block_node;
+  ZpPlanes a1, ht, dy, dh1;
+  ZpPlanes hr, rw, gr;                   // planes of the layer's input, weight, output gradient
+  uint16_t *wfold;
+  size_t bytes;
+};
+// ec > 0: the last layer of the radial MLP (ec -> R), with operands in format `rad`, runs inside
+// the call
+ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *base, int ec,
+                     ZpFormat rad);
+
+// One convolution call.  Per-edge arrays are in the sorted order.
+struct ZpConv {
+  int64_t N, E;
+  const float *x_node, *edge_vec, *cos_g, *sin_g, *radial, *env;
+  const int32_t *src, *dst, *row_ptr, *perm_src, *row_ptr_src;
+  const zp_weights *w;
+};
+// The last dense layer of the radial MLP (blocks/eso2_ref.py:169-182, rad_func[6]), when the call
+// runs it itself: radial[E, R] = h[E, ec] w[R, ec]^T + b.
+struct ZpRadialLayer {
+  const float *h, *w, *b;
+  int ec;
+  float *grad_h, *grad_w, *grad_b;       // backward only
+  float *grad_h_max;                     // device scalar updated with max |grad_h|, or null
+};
+
+int zp_check_weights(const zp_plan *p, const zp_weights *w);
+
+// radial = hr rw^T + b into ws.radial, its largest magnitude into the scale array
+int zp_core_radial(const zp_plan *plan, const ZpWorkspace &ws, int64_t E, int ec, const float *bias,
+                   cudaStream_t st);
+// Everything from the rotation matrices to node_out; the maxima of x_node and radial and the weight
+// planes are in place.  keep != 0: what a backward reads is left in the workspace.
+int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c, float *node_out,
+                    int keep, cudaStream_t st);
+// gw null: no weight gradients; grad_x_node null: no node contributions.  With rl the gradient of
+// radial stays inside.  The last sums of the parameter gradients are left to `list`.
+int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
+                     const float *grad_node_out, float *grad_x_node, float *grad_edge_vec,
+                     float *grad_radial, float *grad_env, const zp_weight_grads *gw,
+                     const ZpRadialLayer *rl, ZpFinalList &list, cudaStream_t st);

@@ -19,11 +19,13 @@ namespace {
 // fp32 matrix -> planes (bf16, or fp16 with the tensor's scale), zero padding up to ld_out.
 // threadIdx.x walks the quads of a row, threadIdx.y / blockIdx.x the rows (no division anywhere).
 __global__ void split_planes_kernel(int64_t rows, int64_t cols, const float *__restrict__ in,
-                                    int64_t ld_in, const ZpPlanes out) {
+                                    int64_t ld_in, const ZpPlanes out, const ZpScale scale) {
   const int64_t c = 4 * ((int64_t)blockIdx.y * blockDim.x + threadIdx.x);
+  const float inv =
+      zp_publish_scale(out, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 &&
+                                       threadIdx.y == 0);
   if (c >= out.ld) return;
   const bool vec = (ld_in & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && c + 3 < cols;
-  const float inv = zp_inv_scale(out);
   for (int64_t r = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; r < rows;
        r += (int64_t)gridDim.x * blockDim.y) {
     float v[4];
@@ -36,29 +38,6 @@ __global__ void split_planes_kernel(int64_t rows, int64_t cols, const float *__r
     }
     zp_store_planes<4>(out, r * out.ld + c, v, inv);
   }
-}
-
-// max |x| over a strided matrix into *out (which the caller zeroed), and the scale derived from
-// products of such maxima
-__global__ void absmax_kernel(int64_t rows, int64_t cols, const float *__restrict__ in, int64_t ld,
-                              float *out) {
-  float m = 0.f;
-  const int64_t n = rows * cols;
-  if (ld == cols && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0) {
-    const float4 *in4 = reinterpret_cast<const float4 *>(in);     // contiguous: 16-byte loads
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n / 4;
-         i += (int64_t)gridDim.x * blockDim.x) {
-      const float4 v = in4[i];
-      m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-    }
-  } else {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x)
-      m = fmaxf(m, fabsf(in[(i / cols) * ld + i % cols]));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(out, m);
 }
 
 // largest node index the edge list names (the caller zeroed *out)
@@ -95,15 +74,6 @@ __global__ void absmax_row_range_kernel(const float *__restrict__ in, int64_t co
   if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(out, m);
 }
 
-// scale[0] = power of two mapping  factor * a * b * max(offset_c, c_factor * c * d)  to 2^15;
-// null pointers count as 1, the max term is left out when c is null
-__global__ void scale_kernel(float factor, const float *a, const float *b, const float *c,
-                             const float *d, float c_factor, float offset_c, float *scale) {
-  float bound = factor * (a ? *a : 1.f) * (b ? *b : 1.f);
-  if (c) bound *= fmaxf(offset_c, c_factor * *c * (d ? *d : 1.f));
-  *scale = zp_scale_for_bound(bound);
-}
-
 // ------------------------------------------------------------------------------------------
 // gate activation (blocks/eso2_ref.py:295-301): conv1 output row h1[e] = [gate (lmax*H) | y (Km*H)]
 // ------------------------------------------------------------------------------------------
@@ -118,7 +88,7 @@ constexpr int kGateEdges = 8;
 constexpr int kGateSub = 4;            // groups of kGateEdges edges per block of gate_fwd
 __global__ void gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
                                 const float *__restrict__ h1, const ZpPlanes ht,
-                                float *gate_max) {
+                                const ZpScale scale, float *gate_max) {
   // blockIdx.x counts groups of kGateEdges edges; the items of a group are indexed with 32-bit
   // arithmetic (a 64-bit division per thread would cost more than the rest of the kernel)
   const int H4 = t.H / 4;
@@ -129,7 +99,8 @@ __global__ void gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
   const int h = (rem - rp * H4) * 4;
   float seen = 0.f;
   bool probe = false;
-  const float inv = zp_inv_scale(ht);
+  const float inv = zp_publish_scale(
+      ht, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
   // a block walks kGateSub groups of kGateEdges edges: fewer, longer-lived blocks
 #pragma unroll 2
   for (int sub = 0; sub < kGateSub; ++sub) {
@@ -178,7 +149,7 @@ __global__ void gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
 template <int LM>
 __global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
                                 const float *__restrict__ h1, const float *__restrict__ dht,
-                                const ZpPlanes dh1) {
+                                const ZpPlanes dh1, const ZpScale scale) {
   const int H4 = t.H / 4;
   const int item = blockIdx.y * blockDim.x + threadIdx.x;            // within a group of edges
   const int le = item / H4;
@@ -188,7 +159,8 @@ __global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant_
   const int h = (item - le * H4) * 4;
   const float *row = h1 + (size_t)e * t.w1_cols;
   const int64_t drow = e * dh1.ld;
-  const float inv = zp_inv_scale(dh1);
+  const float inv = zp_publish_scale(
+      dh1, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
   const float *dt = dht + (size_t)e * t.Km * t.H;
   constexpr int NL = LM > 0 ? LM : 1;        // gates: one per degree 1..lmax
   float sg[NL][4], dg[NL][4];
@@ -243,56 +215,61 @@ __global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant_
 // ------------------------------------------------------------------------------------------
 // weight folding and its transpose
 // ------------------------------------------------------------------------------------------
-// All weight blocks of both convolutions in one launch each (blockIdx.y = block).
-struct FoldDesc {
-  int n;
-  int out[2 * (ZP_MAX_L + 1)], in[2 * (ZP_MAX_L + 1)], folded[2 * (ZP_MAX_L + 1)];
-  int slot[2 * (ZP_MAX_L + 1)];                 // index of the block's {max, scale} pair
-  const float *w[2 * (ZP_MAX_L + 1)];
-  int64_t woff[2 * (ZP_MAX_L + 1)];
-};
-
-__global__ void weight_absmax_kernel(const FoldDesc d, float *scales) {
+// Maxima of up to ZP_MAX_ITEMS arrays in one launch (blockIdx.y = array; the caller zeroed the slots):
+// every weight block, and whatever else a call needs the magnitude of before its first product.
+__global__ void __launch_bounds__(256) max_list_kernel(const __grid_constant__ ZpMaxList d) {
   const int b = blockIdx.y;
-  const int64_t total = (int64_t)d.out[b] * (d.folded[b] ? d.in[b] / 2 : d.in[b]);
+  const float *x = d.x[b];
+  const int64_t n = d.count[b], step = (int64_t)gridDim.x * blockDim.x;
+  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   float m = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (int64_t)gridDim.x * blockDim.x)
-    m = fmaxf(m, fabsf(d.w[b][i]));
+  if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    for (; i < n / 4; i += step) {
+      const float4 v = x4[i];
+      m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+    }
+    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) m = fmaxf(m, fabsf(x[(n & ~3ll) + threadIdx.x]));
+  } else {
+    for (; i < n; i += step) m = fmaxf(m, fabsf(x[i]));
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(scales + 2 * d.slot[b], m);
+  if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(d.out[b], m);
 }
 
-__global__ void weight_scale_kernel(const FoldDesc d, float *scales) {
-  const int b = threadIdx.x;
-  if (b < d.n) scales[2 * d.slot[b] + 1] = zp_scale_for_bound(scales[2 * d.slot[b]]);
-}
-
-// fold: writes W_fold [out, in] and its transpose [in, out] as 16-bit planes.
-//   m = 0 (folded == 0): W_fold = W.   m > 0: W = [Wa ; Wb] (rows), W_fold = [Wa -Wb ; Wb Wa].
-__global__ void __launch_bounds__(256)
-fold_planes_kernel(const FoldDesc d, uint16_t *__restrict__ packed, int planes, int fp16,
-                   const float *__restrict__ scales) {
+// Writes every weight matrix as 16-bit planes, all of them in one launch (blockIdx.y = matrix).
+//   plain          W [out, in] -> planes [out, ld], zero padded
+//   kept / folded  W_fold [out, in] and its transpose [in, out];  m = 0 (kept): W_fold = W,
+//                  m > 0 (folded): W = [Wa ; Wb] (rows), W_fold = [Wa -Wb ; Wb Wa]
+// slot = {max |W|, scale}: the scale follows from the maximum here (fp16 planes).
+__global__ void __launch_bounds__(256) prep_weights_kernel(const __grid_constant__ ZpPrepList d) {
   // 32 x 32 tiles: the planes of W_fold go out row-major as they are formed; the transpose is
   // written from a shared copy of the tile so that both stores run along the fastest axis.
   __shared__ uint16_t tile[3][32][34];
   const int b = blockIdx.y;
-  const int out = d.out[b], in = d.in[b];
-  const int64_t total = (int64_t)out * in;
-  uint16_t *wp = packed + d.woff[b], *wtp = wp + (size_t)planes * total;
-  const float inv = fp16 ? 1.f / scales[2 * d.slot[b] + 1] : 1.f;
+  const int out = d.out[b], in = d.in[b], kind = d.kind[b], planes = d.planes[b], fp16 = d.fp16[b];
+  const int ld = d.ld[b];
+  const int64_t stride = d.plane_stride[b];
+  uint16_t *wp = d.dst[b], *wtp = wp + (size_t)planes * stride;
+  float inv = 1.f;
+  if (fp16) {
+    const float s = zp_scale_for_bound(d.slot[b][0]);
+    inv = 1.f / s;
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.slot[b][1] = s;
+  }
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;          // 32 x 8
-  const int tiles_c = (in + 31) / 32, tiles = ((out + 31) / 32) * tiles_c;
+  const int cols = kind == ZP_PREP_PLAIN ? ld : in;
+  const int tiles_c = (cols + 31) / 32, tiles = ((out + 31) / 32) * tiles_c;
   for (int tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
     const int r0 = (tl / tiles_c) * 32, c0 = (tl % tiles_c) * 32;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int row = r0 + ty + 8 * k, col = c0 + tx;
-      if (row < out && col < in) {
-        float v;
-        if (!d.folded[b]) {
-          v = d.w[b][(size_t)row * in + col];
+      if (row < out && col < cols) {
+        float v = 0.f;
+        if (kind != ZP_PREP_FOLDED) {
+          if (col < in) v = d.w[b][(size_t)row * in + col];
         } else {
           const int half = out / 2, kin = in / 2;
           const bool lower = row >= half, right = col >= kin;
@@ -312,56 +289,81 @@ fold_planes_kernel(const FoldDesc d, uint16_t *__restrict__ packed, int planes, 
             h = __bfloat16_as_ushort(q);
             v -= __bfloat162float(q);
           }
-          wp[(size_t)p * total + (size_t)row * in + col] = h;
+          wp[(size_t)p * stride + (size_t)row * ld + col] = h;
           tile[p][ty + 8 * k][tx] = h;
         }
       }
     }
+    if (kind == ZP_PREP_PLAIN) continue;         // uniform over the block
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int col = c0 + ty + 8 * k, row = r0 + tx;
       if (row < out && col < in)
         for (int p = 0; p < planes; ++p)
-          wtp[(size_t)p * total + (size_t)col * out + row] = tile[p][tx][ty + 8 * k];
+          wtp[(size_t)p * stride + (size_t)col * out + row] = tile[p][tx][ty + 8 * k];
     }
     __syncthreads();
   }
 }
 
-// Sums the `splits` partial folded gradients in order and maps them back to the reference
-// layout: m = 0 copies; m > 0: dWa = F[0,0] + F[1,1], dWb = F[1,0] - F[0,1].  All weight blocks
-// of both convolutions in one launch (blockIdx.y = block).
-struct UnfoldDesc {
-  int n;
-  int out[2 * (ZP_MAX_L + 1)], in[2 * (ZP_MAX_L + 1)], folded[2 * (ZP_MAX_L + 1)];
-  int splits[2 * (ZP_MAX_L + 1)];
-  int64_t foff[2 * (ZP_MAX_L + 1)];             // offset of the block's folded gradient
-  float *gw[2 * (ZP_MAX_L + 1)];
-};
-__global__ void unfold_kernel(const UnfoldDesc d, int64_t split_stride, const float *__restrict__ f) {
+// The last step of every parameter gradient, all of them in one launch (blockIdx.y = gradient).
+//   ZP_FIN_SUM     sum of `parts` partial matrices (K splits of a product), in order
+//   ZP_FIN_UNFOLD  the same, mapped from the folded layout back to the reference's:
+//                  dWa = F[0,0] + F[1,1], dWb = F[1,0] - F[0,1]
+//   ZP_FIN_COLUMN  sum of `parts` partial rows: 32 columns per block, eight threads per column take
+//                  every eighth row, and their sums are added in order
+__global__ void __launch_bounds__(256) finalize_kernel(const __grid_constant__ ZpFinalList d) {
+  __shared__ float red[8][33];
   const int b = blockIdx.y;
-  const int out = d.out[b], in = d.in[b], folded = d.folded[b];
-  const int kin = folded ? in / 2 : in, half = out / 2;
-  const int64_t total = (int64_t)out * kin;
+  const float *f = d.src[b];
+  float *dst = d.dst[b];
+  const int64_t stride = d.stride[b];
+  const int rows = d.rows[b], cols = d.cols[b], parts = d.parts[b], kind = d.kind[b];
+  if (kind == ZP_FIN_COLUMN) {
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    for (int c0 = blockIdx.x * 32; c0 < cols; c0 += gridDim.x * 32) {
+      const int c = c0 + tx;
+      float s = 0.f;
+      if (c < cols) {
+#pragma unroll 4
+        for (int p = ty; p < parts; p += 8) s += f[(size_t)p * stride + c];
+      }
+      red[ty][tx] = s;
+      __syncthreads();
+      if (ty == 0 && c < cols) {
+        float acc = 0.f;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) acc += red[g][tx];
+        dst[c] = acc;
+      }
+      __syncthreads();
+    }
+    return;
+  }
+  const bool folded = kind == ZP_FIN_UNFOLD;
+  const int ld = d.ld[b];
+  const int kin = folded ? cols / 2 : cols, half = rows / 2;
+  const int64_t total = (int64_t)rows * kin;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int c = (int)(idx % kin), row = (int)(idx / kin);
     float acc = 0.f;
-    for (int s = 0; s < d.splits[b]; ++s) {
-      const float *fs = f + d.foff[b] + (size_t)s * split_stride;
-      if (!folded) acc += fs[idx];
-      else if (row < half) acc += fs[(size_t)row * in + c] + fs[(size_t)(half + row) * in + kin + c];
-      else acc += fs[(size_t)row * in + c] - fs[(size_t)(row - half) * in + kin + c];
+    for (int s = 0; s < parts; ++s) {
+      const float *fs = f + (size_t)s * stride;
+      const float v = fs[(size_t)row * ld + c];
+      if (!folded) acc += v;
+      else if (row < half) acc += v + fs[(size_t)(half + row) * ld + kin + c];
+      else acc += v - fs[(size_t)(row - half) * ld + kin + c];
     }
-    d.gw[b][idx] = acc;
+    dst[idx] = acc;
   }
 }
 
 // column sums in two fixed-order stages.  Stage one: a block of 32 x 8 threads sums 128 rows of
 // 256 columns; a thread owns 8 consecutive columns (one 16-byte load per row and plane) and every
 // eighth row, the eight row groups are then added in order through shared memory.
-constexpr int kColRowsPerBlock = 512;    // scratch is sized for 128 (more partials than are used)
+constexpr int kColRowsPerBlock = 512;
 __global__ void __launch_bounds__(256)
 colsum_part_kernel(int64_t rows, int64_t cols, const ZpPlanes a, float *__restrict__ part) {
   __shared__ float red[8][32][9];
@@ -371,6 +373,7 @@ colsum_part_kernel(int64_t rows, int64_t cols, const ZpPlanes a, float *__restri
   const int64_t r1 = min(rows, r0 + kColRowsPerBlock);
   float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (c0 < cols) {
+#pragma unroll 4
     for (int64_t r = r0 + ty; r < r1; r += 8) {
       for (int pl = a.planes - 1; pl >= 0; --pl) {
         const uint4 v = *reinterpret_cast<const uint4 *>(
@@ -396,15 +399,6 @@ colsum_part_kernel(int64_t rows, int64_t cols, const ZpPlanes a, float *__restri
     }
   }
 }
-__global__ void colsum_final_kernel(int64_t nparts, int64_t cols, const float *__restrict__ part,
-                                    float *__restrict__ out) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float s = 0.f;
-  for (int64_t p = 0; p < nparts; ++p) s += part[(size_t)p * cols + c];
-  out[c] = s;
-}
-
 // scale of conv1's activated output from an a-priori bound (one block):
 //   |h1| <= max_m(in_m * A * max|W_m|) + max|b|,  A = 2^15 * a1_scale >= max|a1|
 struct BoundDesc {
@@ -446,7 +440,7 @@ int zp_launch_conv1_bound(const zp_plan *p, const float *a1_scale, const float *
 }
 
 int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,
-                           const ZpPlanes &out, cudaStream_t st) {
+                           const ZpPlanes &out, const ZpScale &scale, cudaStream_t st) {
   if (rows == 0 || out.ld == 0) return ZP_OK;
   const int quads = (int)(out.ld / 4);
   int bx = 32;
@@ -455,25 +449,52 @@ int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t 
   int64_t gx = zp_ceil_div(rows, by);
   if (gx > 148 * 32) gx = 148 * 32;
   const dim3 grid((unsigned)gx, (unsigned)zp_ceil_div(quads, bx)), block(bx, by);
-  split_planes_kernel<<<grid, block, 0, st>>>(rows, cols, in, ld_in, out);
+  split_planes_kernel<<<grid, block, 0, st>>>(rows, cols, in, ld_in, out, scale);
   ZP_LAUNCH_CHECK("split_planes_kernel");
   return ZP_OK;
 }
 
-int zp_launch_absmax(int64_t rows, int64_t cols, const float *in, int64_t ld, float *out,
-                     cudaStream_t st) {
-  ZP_CUDA(cudaMemsetAsync(out, 0, sizeof(float), st));
-  if (rows * cols == 0) return ZP_OK;
-  int64_t blocks = zp_ceil_div(rows * cols, 256 * 8);
-  if (blocks > 1184) blocks = 1184;
-  absmax_kernel<<<(unsigned)blocks, 256, 0, st>>>(rows, cols, in, ld, out);
-  ZP_LAUNCH_CHECK("absmax_kernel");
+int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st) {
+  if (list.n == 0) return ZP_OK;
+  // sixteen values per thread, so that small arrays take few blocks; the largest take two waves
+  int64_t most = 0;
+  for (int i = 0; i < list.n; ++i) most = list.count[i] > most ? list.count[i] : most;
+  int64_t gx = zp_ceil_div(most, 256 * 16);
+  if (gx > 1184) gx = 1184;
+  if (gx < 1) gx = 1;
+  max_list_kernel<<<dim3((unsigned)gx, list.n), 256, 0, st>>>(list);
+  ZP_LAUNCH_CHECK("max_list_kernel");
+  return ZP_OK;
+}
+
+int zp_launch_prep_weights(const ZpPrepList &list, cudaStream_t st) {
+  if (list.n == 0) return ZP_OK;
+  int64_t most = 1;                     // 32 x 32 tiles of the largest matrix
+  for (int i = 0; i < list.n; ++i) {
+    const int64_t t = zp_ceil_div(list.out[i], 32) * zp_ceil_div(list.ld[i], 32);
+    most = t > most ? t : most;
+  }
+  prep_weights_kernel<<<dim3((unsigned)(most > 296 ? 296 : most), list.n), 256, 0, st>>>(list);
+  ZP_LAUNCH_CHECK("prep_weights_kernel");
+  return ZP_OK;
+}
+
+int zp_launch_finalize(const ZpFinalList &list, cudaStream_t st) {
+  if (list.n == 0) return ZP_OK;
+  int64_t most = 1;
+  for (int i = 0; i < list.n; ++i) {
+    const int64_t t = list.kind[i] == ZP_FIN_COLUMN
+                          ? zp_ceil_div(list.cols[i], 32)
+                          : zp_ceil_div((int64_t)list.rows[i] * list.cols[i], 256);
+    most = t > most ? t : most;
+  }
+  finalize_kernel<<<dim3((unsigned)(most > 148 ? 148 : most), list.n), 256, 0, st>>>(list);
+  ZP_LAUNCH_CHECK("finalize_kernel");
   return ZP_OK;
 }
 
 int zp_launch_max_index(int64_t E, const int32_t *src, const int32_t *dst, int *out,
                         cudaStream_t st) {
-  ZP_CUDA(cudaMemsetAsync(out, 0, sizeof(int), st));
   if (E == 0) return ZP_OK;
   int64_t blocks = zp_ceil_div(E, 256 * 4);
   if (blocks > 592) blocks = 592;
@@ -485,38 +506,29 @@ int zp_launch_max_index(int64_t E, const int32_t *src, const int32_t *dst, int *
 int zp_launch_absmax_row_range(const float *in, int64_t cols, const int32_t *first,
                                const int32_t *last, int64_t min_rows, float *out,
                                cudaStream_t st) {
-  ZP_CUDA(cudaMemsetAsync(out, 0, sizeof(float), st));
   if (cols == 0 || (cols & 3)) return cols ? ZP_ERR_INVALID_ARG : ZP_OK;
   absmax_row_range_kernel<<<1184, 256, 0, st>>>(in, cols, first, last, min_rows, out);
   ZP_LAUNCH_CHECK("absmax_row_range_kernel");
   return ZP_OK;
 }
 
-int zp_launch_scale(float factor, const float *a, const float *b, const float *c, float offset_c,
-                    float *scale, cudaStream_t st, const float *d, float c_factor) {
-  scale_kernel<<<1, 1, 0, st>>>(factor, a, b, c, d, c_factor, offset_c, scale);
-  ZP_LAUNCH_CHECK("scale_kernel");
-  return ZP_OK;
-}
-
 int zp_launch_gate_fwd(const zp_plan *p, int64_t E, const float *h1, const ZpPlanes &ht,
-                       float *gate_max, cudaStream_t st) {
-  if (gate_max) ZP_CUDA(cudaMemsetAsync(gate_max, 0, sizeof(float), st));
+                       const ZpScale &scale, float *gate_max, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const int per_group = kGateEdges * ((p->t.Km + 1) / 2) * (p->t.H / 4);
   const dim3 grid((unsigned)zp_ceil_div(E, kGateEdges * kGateSub),
                   (unsigned)zp_ceil_div(per_group, 256));
-  gate_fwd_kernel<<<grid, 256, 0, st>>>(p->t, E, h1, ht, gate_max);
+  gate_fwd_kernel<<<grid, 256, 0, st>>>(p->t, E, h1, ht, scale, gate_max);
   ZP_LAUNCH_CHECK("gate_fwd_kernel");
   return ZP_OK;
 }
 
 int zp_launch_gate_bwd(const zp_plan *p, int64_t E, const float *h1, const float *dht,
-                       const ZpPlanes &dh1, cudaStream_t st) {
+                       const ZpPlanes &dh1, const ZpScale &scale, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const int per_group = kGateEdges * (p->t.H / 4);
   const dim3 grid((unsigned)zp_ceil_div(E, kGateEdges), (unsigned)zp_ceil_div(per_group, 128));
-#define CALL(LM) gate_bwd_kernel<LM><<<grid, 128, 0, st>>>(p->t, E, h1, dht, dh1)
+#define CALL(LM) gate_bwd_kernel<LM><<<grid, 128, 0, st>>>(p->t, E, h1, dht, dh1, scale)
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("gate_bwd_kernel");
@@ -528,57 +540,35 @@ static const float *block_weight(const zp_weights *w, int conv, int m) {
   return conv ? w->c2_wm[m - 1] : w->c1_wm[m - 1];
 }
 
-int zp_launch_fold_weights(const zp_plan *p, const zp_weights *w, void *packed, float *scales,
-                           cudaStream_t st) {
-  FoldDesc d;
-  d.n = 0;
+void zp_add_so2_weights(const zp_plan *p, const zp_weights *w, void *packed, float *scales,
+                        ZpMaxList &maxima, ZpPrepList &prep) {
   for (int conv = 0; conv < 2; ++conv)
     for (int m = 0; m < p->n_blocks; ++m) {
-      const int b = d.n++;
-      d.out[b] = conv ? p->c2_out[m] : p->c1_out[m];
-      d.in[b] = conv ? p->c2_in[m] : p->c1_in[m];
-      d.folded[b] = m > 0;
-      d.slot[b] = conv * (ZP_MAX_L + 1) + m;
-      d.w[b] = block_weight(w, conv, m);
-      d.woff[b] = conv ? p->c2_woff[m] : p->c1_woff[m];
+      const int out = conv ? p->c2_out[m] : p->c1_out[m], in = conv ? p->c2_in[m] : p->c1_in[m];
+      const float *src = block_weight(w, conv, m);
+      float *slot = scales + 2 * (conv * (ZP_MAX_L + 1) + m);
+      // one power-of-two scale per weight block from its largest magnitude
+      if (p->fp16) maxima.add(src, (int64_t)out * (m ? in / 2 : in), slot);
+      prep.add(src, static_cast<uint16_t *>(packed) + (conv ? p->c2_woff[m] : p->c1_woff[m]), slot,
+               (int64_t)out * in, out, in, in, m ? ZP_PREP_FOLDED : ZP_PREP_KEPT, p->planes, p->fp16);
     }
-  if (p->fp16) {       // one power-of-two scale per weight block from its largest magnitude
-    ZP_CUDA(cudaMemsetAsync(scales, 0, sizeof(float) * 4 * (ZP_MAX_L + 1), st));
-    weight_absmax_kernel<<<dim3(148, d.n), 256, 0, st>>>(d, scales);
-    ZP_LAUNCH_CHECK("weight_absmax_kernel");
-    weight_scale_kernel<<<1, 32, 0, st>>>(d, scales);
-    ZP_LAUNCH_CHECK("weight_scale_kernel");
-  }
-  fold_planes_kernel<<<dim3(296, d.n), 256, 0, st>>>(d, static_cast<uint16_t *>(packed), p->planes,
-                                                     p->fp16, scales);
-  ZP_LAUNCH_CHECK("fold_planes_kernel");
-  return ZP_OK;
 }
 
-int zp_launch_unfold_wgrad(const zp_plan *p, const float *partials, int64_t split_stride,
-                           const int *splits_c1, const int *splits_c2, const zp_weight_grads *gw,
-                           cudaStream_t st) {
-  UnfoldDesc d;
-  d.n = 0;
-  for (int conv = 0; conv < 2; ++conv) {
+void zp_add_so2_grads(const zp_plan *p, const float *partials, int64_t split_stride,
+                      const int *splits_c1, const int *splits_c2, const zp_weight_grads *gw,
+                      ZpFinalList &list) {
+  for (int conv = 0; conv < 2; ++conv)
     for (int m = 0; m < p->n_blocks; ++m) {
-      const int b = d.n++;
-      d.out[b] = conv ? p->c2_out[m] : p->c1_out[m];
-      d.in[b] = conv ? p->c2_in[m] : p->c1_in[m];
-      d.folded[b] = m > 0;
-      d.splits[b] = (conv ? splits_c2 : splits_c1)[m];
-      d.foff[b] = conv ? p->c2_goff[m] : p->c1_goff[m];
-      d.gw[b] = m == 0 ? (conv ? gw->c2_w0 : gw->c1_w0)
-                       : (conv ? gw->c2_wm[m - 1] : gw->c1_wm[m - 1]);
+      float *dst = m == 0 ? (conv ? gw->c2_w0 : gw->c1_w0)
+                          : (conv ? gw->c2_wm[m - 1] : gw->c1_wm[m - 1]);
+      list.add(partials + (conv ? p->c2_goff[m] : p->c1_goff[m]), dst, split_stride,
+               conv ? p->c2_out[m] : p->c1_out[m], conv ? p->c2_in[m] : p->c1_in[m],
+               (conv ? splits_c2 : splits_c1)[m], m ? ZP_FIN_UNFOLD : ZP_FIN_SUM);
     }
-  }
-  unfold_kernel<<<dim3(148, d.n), 256, 0, st>>>(d, split_stride, partials);
-  ZP_LAUNCH_CHECK("unfold_kernel");
-  return ZP_OK;
 }
 
 int zp_launch_colsum(int64_t rows, int64_t cols, const ZpPlanes &a, float *out, float *scratch,
-                     cudaStream_t st) {
+                     ZpFinalList &list, cudaStream_t st) {
   if (cols == 0) return ZP_OK;
   const int64_t nparts = rows > 0 ? zp_ceil_div(rows, kColRowsPerBlock) : 0;
   if (nparts > 0) {
@@ -586,7 +576,6 @@ int zp_launch_colsum(int64_t rows, int64_t cols, const ZpPlanes &a, float *out, 
     colsum_part_kernel<<<grid, block, 0, st>>>(rows, cols, a, scratch);
     ZP_LAUNCH_CHECK("colsum_part_kernel");
   }
-  colsum_final_kernel<<<(unsigned)zp_ceil_div(cols, 128), 128, 0, st>>>(nparts, cols, scratch, out);
-  ZP_LAUNCH_CHECK("colsum_final_kernel");
+  list.add(scratch, out, cols, 1, (int)cols, (int)nparts, ZP_FIN_COLUMN);
   return ZP_OK;
 }

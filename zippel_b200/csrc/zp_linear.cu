@@ -48,23 +48,30 @@ LinWork carve_lin(const zp_plan *p, int64_t M, int64_t K, int64_t N, void *base)
   return w;
 }
 
-__global__ void sum_partials_kernel(int64_t n, int splits, const float *__restrict__ part,
-                                    float *__restrict__ out) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float s = 0.f;
-  for (int k = 0; k < splits; ++k) s += part[(size_t)k * n + i];
-  out[i] = s;
-}
-
-int split_scaled(const zp_plan *p, int64_t rows, int64_t cols, const float *in, const ZpPlanes &pl,
-                 float *max_slot, cudaStream_t st) {
+// planes of up to three fp32 matrices, each with the scale of its own maximum (slot = {max, scale})
+struct SplitJob {
+  int64_t rows, cols;
+  const float *in;
+  const ZpPlanes *planes;
+  float *slot;
+};
+int split_scaled(const zp_plan *p, const SplitJob *jobs, int n, cudaStream_t st) {
   int rc;
   if (p->fp16) {
-    if ((rc = zp_launch_absmax(rows, cols, in, cols, max_slot, st))) return rc;
-    if ((rc = zp_launch_scale(1.f, max_slot, nullptr, nullptr, 0.f, max_slot + 1, st))) return rc;
+    ZpMaxList maxima;
+    for (int i = 0; i < n; ++i) {
+      ZP_CUDA(cudaMemsetAsync(jobs[i].slot, 0, sizeof(float), st));
+      maxima.add(jobs[i].in, jobs[i].rows * jobs[i].cols, jobs[i].slot);
+    }
+    if ((rc = zp_launch_max_list(maxima, st))) return rc;
   }
-  return zp_launch_split_planes(rows, cols, in, cols, pl, st);
+  for (int i = 0; i < n; ++i) {
+    const SplitJob &q = jobs[i];
+    if ((rc = zp_launch_split_planes(q.rows, q.cols, q.in, q.cols, *q.planes,
+                                     zp_scale_of(1.f, q.slot, q.slot + 1), st)))
+      return rc;
+  }
+  return ZP_OK;
 }
 
 }  // namespace
@@ -77,24 +84,28 @@ int split_scaled(const zp_plan *p, int64_t rows, int64_t cols, const float *in, 
 int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t N,
                               const ZpPlanes &x, const ZpPlanes &w, const ZpPlanes &dy, float *dx,
                               float *dw, float *db, float *partials, int max_splits,
-                              float *colsum_scratch, cudaStream_t st) {
+                              float *colsum_scratch, ZpFinalList &list, cudaStream_t st,
+                              float *dx_absmax, int64_t dx_cols) {
   int rc;
+  const int P = dy.planes, fp16 = dy.fp16;
   if (dx) {
-    const ZpGemmTc g{M, K, N, plan->planes, dy.base, dy.ld, dy.plane_stride, 0,
-                     w.base, w.ld, w.plane_stride, 1, nullptr, dx, K, plan->status_dev,
-                     0, 1, 0, 0, plan->fp16, dy.scale, w.scale, nullptr};
+    const int64_t cols = dx_cols > 0 ? dx_cols : K;
+    const ZpGemmTc g{M, cols, N, P, dy.base, dy.ld, dy.plane_stride, 0,
+                     w.base, w.ld, w.plane_stride, 1, nullptr, dx, (cols + 3) / 4 * 4,
+                     plan->status_dev, 0, 1, 0, 0, fp16, dy.scale, w.scale, dx_absmax};
     if ((rc = zp_launch_gemm_tc(g, st))) return rc;
   }
-  if (!dw) return db ? zp_launch_colsum(M, N, dy, db, colsum_scratch, st) : ZP_OK;
-  ZpGemmTc g{N, K, M, plan->planes, dy.base, dy.ld, dy.plane_stride, 1,
-             x.base, x.ld, x.plane_stride, 1, nullptr, partials, K, plan->status_dev,
-             0, 1, N * K, 0, plan->fp16, dy.scale, x.scale, nullptr};
-  g.ksplit = zp_gemm_tc_pick_splits(g, max_splits);
-  const int splits = zp_gemm_tc_splits(g);
-  if ((rc = zp_launch_gemm_tc(g, st))) return rc;
-  sum_partials_kernel<<<(unsigned)zp_ceil_div(N * K, 256), 256, 0, st>>>(N * K, splits, partials, dw);
-  ZP_LAUNCH_CHECK("sum_partials_kernel");
-  if (db) return zp_launch_colsum(M, N, dy, db, colsum_scratch, st);
+  if (dw) {
+    const int64_t ldk = (K + 3) / 4 * 4;         // rows of the partial sums start 16-byte aligned
+    ZpGemmTc g{N, K, M, P, dy.base, dy.ld, dy.plane_stride, 1,
+               x.base, x.ld, x.plane_stride, 1, nullptr, partials, ldk, plan->status_dev,
+               0, 1, N * ldk, 0, fp16, dy.scale, x.scale, nullptr};
+    g.ksplit = zp_gemm_tc_pick_splits(g, max_splits);
+    const int splits = zp_gemm_tc_splits(g);
+    if ((rc = zp_launch_gemm_tc(g, st))) return rc;
+    list.add(partials, dw, N * ldk, (int)N, (int)K, splits, ZP_FIN_SUM, (int)ldk);
+  }
+  if (db) return zp_launch_colsum(M, N, dy, db, colsum_scratch, list, st);
   return ZP_OK;
 }
 
@@ -125,8 +136,8 @@ int zp_linear_forward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, cons
   const LinWork lw = carve_lin(plan, M, K, N, work);
   if (work_bytes < lw.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  if ((rc = split_scaled(plan, M, K, x, lw.x, lw.scales + 0, st))) return rc;
-  if ((rc = split_scaled(plan, N, K, w, lw.w, lw.scales + 2, st))) return rc;
+  const SplitJob jobs[2] = {{M, K, x, &lw.x, lw.scales}, {N, K, w, &lw.w, lw.scales + 2}};
+  if ((rc = split_scaled(plan, jobs, 2, st))) return rc;
   const ZpGemmTc g{M, N, K, plan->planes, lw.x.base, lw.x.ld, lw.x.plane_stride, 0,
                    lw.w.base, lw.w.ld, lw.w.plane_stride, 0, bias, y, N, plan->status_dev,
                    0, 1, 0, 0, plan->fp16, lw.x.scale, lw.w.scale, nullptr};
@@ -148,11 +159,17 @@ int zp_linear_backward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, con
     return ZP_OK;
   }
   // dw == NULL: frozen parameters, only the input gradient (and db if given) is formed
-  if (dw && (rc = split_scaled(plan, M, K, x, lw.x, lw.scales + 0, st))) return rc;
-  if (dx && (rc = split_scaled(plan, N, K, w, lw.w, lw.scales + 2, st))) return rc;
-  if ((rc = split_scaled(plan, M, N, dy, lw.dy, lw.scales + 4, st))) return rc;
-  return zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
-                                   kLinSplits, lw.colsum, st);
+  SplitJob jobs[3];
+  int n = 0;
+  if (dw) jobs[n++] = {M, K, x, &lw.x, lw.scales};
+  if (dx) jobs[n++] = {N, K, w, &lw.w, lw.scales + 2};
+  jobs[n++] = {M, N, dy, &lw.dy, lw.scales + 4};
+  if ((rc = split_scaled(plan, jobs, n, st))) return rc;
+  ZpFinalList list;
+  if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
+                                      kLinSplits, lw.colsum, list, st)))
+    return rc;
+  return zp_launch_finalize(list, st);
 }
 
 int zp_linear_backward_saved(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *dy,
@@ -170,9 +187,13 @@ int zp_linear_backward_saved(const zp_plan *plan, int64_t M, int64_t K, int64_t 
     return ZP_OK;
   }
   // the planes of x and w and their scales are where zp_linear_forward left them
-  if ((rc = split_scaled(plan, M, N, dy, lw.dy, lw.scales + 4, st))) return rc;
-  return zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
-                                   kLinSplits, lw.colsum, st);
+  const SplitJob job{M, N, dy, &lw.dy, lw.scales + 4};
+  if ((rc = split_scaled(plan, &job, 1, st))) return rc;
+  ZpFinalList list;
+  if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
+                                      kLinSplits, lw.colsum, list, st)))
+    return rc;
+  return zp_launch_finalize(list, st);
 }
 
 }  // extern "C"

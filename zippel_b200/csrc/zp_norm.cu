@@ -20,7 +20,6 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr int kMaxGroups = 8;              // 128-column groups per row: width <= 1024
-constexpr int kPartialBlocks = 296;        // blocks of the backward kernel = partial rows
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -32,9 +31,11 @@ template <int G>
 __global__ void __launch_bounds__(32 * kWarps)
 ln_silu_fwd_kernel(int64_t rows, int width, const float *__restrict__ x,
                    const float *__restrict__ gamma, const float *__restrict__ beta, float eps,
-                   float *__restrict__ y, float *__restrict__ mean_out,
-                   float *__restrict__ rstd_out) {
+                   float *__restrict__ y, const ZpPlanes yp, const ZpScale scale,
+                   float *__restrict__ mean_out, float *__restrict__ rstd_out, float *rstd_max) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const float inv = yp.planes ? zp_publish_scale(yp, scale, blockIdx.x == 0 && threadIdx.x == 0) : 1.f;
+  float seen = 0.f;
   float4 g[G], b[G];
 #pragma unroll
   for (int i = 0; i < G; ++i) {
@@ -64,7 +65,7 @@ ln_silu_fwd_kernel(int64_t rows, int width, const float *__restrict__ x,
       }
     }
     const float rstd = rsqrtf(warp_sum(q) * inv_w + eps);
-    float *yr = y + (size_t)r * width;
+    seen = fmaxf(seen, rstd);
 #pragma unroll
     for (int i = 0; i < G; ++i) {
       const int c = 128 * i + 4 * lane;
@@ -75,11 +76,21 @@ ln_silu_fwd_kernel(int64_t rows, int width, const float *__restrict__ x,
         u = (v[i].y - mean) * rstd * g[i].y + b[i].y; o.y = u / (1.f + expf(-u));
         u = (v[i].z - mean) * rstd * g[i].z + b[i].z; o.z = u / (1.f + expf(-u));
         u = (v[i].w - mean) * rstd * g[i].w + b[i].w; o.w = u / (1.f + expf(-u));
-        *reinterpret_cast<float4 *>(yr + c) = o;
+        if (yp.planes) {
+          const float ov[4] = {o.x, o.y, o.z, o.w};
+          zp_store_planes<4>(yp, r * yp.ld + c, ov, inv);
+        } else {
+          *reinterpret_cast<float4 *>(y + (size_t)r * width + c) = o;
+        }
+      } else if (yp.planes && c < yp.ld) {         // zero padding up to the row stride
+        const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+        zp_store_planes<4>(yp, r * yp.ld + c, zero, 1.f);
       }
     }
     if (lane == 0) { mean_out[r] = mean; rstd_out[r] = rstd; }
   }
+  if (rstd_max && lane == 0 && seen > *reinterpret_cast<volatile float *>(rstd_max))
+    zp_atomic_absmax(rstd_max, seen);
 }
 
 __device__ __forceinline__ void bwd_elem(float xv, float mean, float rstd, float g, float b,
@@ -90,16 +101,19 @@ __device__ __forceinline__ void bwd_elem(float xv, float mean, float rstd, float
   du = dyv * s * (1.f + u * (1.f - s));
 }
 
-template <int G>
+// NP: partial rows per block, 2 = {dgamma, dbeta}, 3 = those and the column sums of dx (the bias
+// gradient of the dense layer in front), 0 = no parameter gradients
+template <int G, int NP>
 __global__ void __launch_bounds__(32 * kWarps)
 ln_silu_bwd_kernel(int64_t rows, int width, const float *__restrict__ x,
                    const float *__restrict__ gamma, const float *__restrict__ beta,
                    const float *__restrict__ mean_in, const float *__restrict__ rstd_in,
-                   const float *__restrict__ dy, float *__restrict__ dx,
-                   float *__restrict__ partial) {           // [gridDim.x][2][width]
-  extern __shared__ float red[];                              // [kWarps][2][width]
+                   const float *__restrict__ dy, float *__restrict__ dx, const ZpPlanes dxp,
+                   const ZpScale scale, float *__restrict__ partial) {   // [gridDim.x][NP][width]
+  extern __shared__ float red[];                              // [kWarps][NP][width]
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  float4 g[G], b[G], dg[G], db[G];
+  const float inv = dxp.planes ? zp_publish_scale(dxp, scale, blockIdx.x == 0 && threadIdx.x == 0) : 1.f;
+  float4 g[G], b[G], dg[G], db[G], dd[G];
 #pragma unroll
   for (int i = 0; i < G; ++i) {
     const int c = 128 * i + 4 * lane;
@@ -107,6 +121,7 @@ ln_silu_bwd_kernel(int64_t rows, int width, const float *__restrict__ x,
     b[i] = c < width ? *reinterpret_cast<const float4 *>(beta + c) : make_float4(0, 0, 0, 0);
     dg[i] = make_float4(0, 0, 0, 0);
     db[i] = make_float4(0, 0, 0, 0);
+    dd[i] = make_float4(0, 0, 0, 0);
   }
   const float inv_w = 1.f / (float)width;
   for (int64_t r = (int64_t)blockIdx.x * kWarps + warp; r < rows; r += (int64_t)gridDim.x * kWarps) {
@@ -136,7 +151,6 @@ ln_silu_bwd_kernel(int64_t rows, int width, const float *__restrict__ x,
       }
     }
     const float m1 = warp_sum(s1) * inv_w, m2 = warp_sum(s2) * inv_w;
-    float *dxr = dx + (size_t)r * width;
 #pragma unroll
     for (int i = 0; i < G; ++i) {
       const int c = 128 * i + 4 * lane;
@@ -146,36 +160,38 @@ ln_silu_bwd_kernel(int64_t rows, int width, const float *__restrict__ x,
         o.y = rstd * (dz[i].y - m1 - z[i].y * m2);
         o.z = rstd * (dz[i].z - m1 - z[i].z * m2);
         o.w = rstd * (dz[i].w - m1 - z[i].w * m2);
-        *reinterpret_cast<float4 *>(dxr + c) = o;
+        if (NP == 3) { dd[i].x += o.x; dd[i].y += o.y; dd[i].z += o.z; dd[i].w += o.w; }
+        if (dxp.planes) {
+          const float ov[4] = {o.x, o.y, o.z, o.w};
+          zp_store_planes<4>(dxp, r * dxp.ld + c, ov, inv);
+        } else {
+          *reinterpret_cast<float4 *>(dx + (size_t)r * width + c) = o;
+        }
+      } else if (dxp.planes && c < dxp.ld) {
+        const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+        zp_store_planes<4>(dxp, r * dxp.ld + c, zero, 1.f);
       }
     }
   }
+  if constexpr (NP != 0) {
   // block partial of (dgamma, dbeta): warps added in warp order
 #pragma unroll
   for (int i = 0; i < G; ++i) {
     const int c = 128 * i + 4 * lane;
     if (c < width) {
-      *reinterpret_cast<float4 *>(red + (size_t)(warp * 2 + 0) * width + c) = dg[i];
-      *reinterpret_cast<float4 *>(red + (size_t)(warp * 2 + 1) * width + c) = db[i];
+      *reinterpret_cast<float4 *>(red + (size_t)(warp * NP + 0) * width + c) = dg[i];
+      *reinterpret_cast<float4 *>(red + (size_t)(warp * NP + 1) * width + c) = db[i];
+      if (NP == 3) *reinterpret_cast<float4 *>(red + (size_t)(warp * NP + 2) * width + c) = dd[i];
     }
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * width; i += blockDim.x) {
+  for (int i = threadIdx.x; i < NP * width; i += blockDim.x) {
     float s = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) s += red[(size_t)w * 2 * width + i];
-    partial[(size_t)blockIdx.x * 2 * width + i] = s;
+    for (int w = 0; w < kWarps; ++w) s += red[(size_t)w * NP * width + i];
+    partial[(size_t)blockIdx.x * NP * width + i] = s;
   }
-}
-
-__global__ void ln_param_grad_kernel(int blocks, int width, const float *__restrict__ partial,
-                                     float *__restrict__ dgamma, float *__restrict__ dbeta) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 2 * width) return;
-  float s = 0.f;
-  for (int b = 0; b < blocks; ++b) s += partial[(size_t)b * 2 * width + i];
-  if (i < width) dgamma[i] = s;
-  else dbeta[i - width] = s;
+  }
 }
 
 int check_shape(int64_t rows, int width) {
@@ -193,10 +209,62 @@ int check_shape(int64_t rows, int width) {
 
 }  // namespace
 
+int zp_launch_ln_silu_fwd(int64_t rows, int width, const float *x, const float *gamma,
+                          const float *beta, float eps, float *y, const ZpPlanes *y_planes,
+                          const ZpScale &scale, float *mean, float *rstd, float *rstd_max,
+                          cudaStream_t st) {
+  if (rows == 0) return ZP_OK;
+  const ZpPlanes yp = y_planes ? *y_planes : ZpPlanes{nullptr, 0, 0, 0, 0, nullptr};
+  const int groups = (width + 127) / 128;
+  const unsigned grid = (unsigned)std::min<int64_t>(zp_ceil_div(rows, kWarps), 148 * 8);
+#define CALL(G)                                                                                   \
+  ln_silu_fwd_kernel<G><<<grid, 32 * kWarps, 0, st>>>(rows, width, x, gamma, beta, eps, y, yp, scale, \
+                                                      mean, rstd, rstd_max)
+  ZP_DISPATCH_GROUPS(groups, CALL);
+#undef CALL
+  ZP_LAUNCH_CHECK("ln_silu_fwd_kernel");
+  return ZP_OK;
+}
+
+int zp_launch_ln_silu_bwd(int64_t rows, int width, const float *x, const float *gamma,
+                          const float *beta, const float *mean, const float *rstd, const float *dy,
+                          float *dx, const ZpPlanes *dx_planes, const ZpScale &scale,
+                          float *dgamma, float *dbeta, float *dbias, float *partial,
+                          ZpFinalList &list, cudaStream_t st) {
+  if (rows == 0) return ZP_OK;
+  const ZpPlanes dxp = dx_planes ? *dx_planes : ZpPlanes{nullptr, 0, 0, 0, 0, nullptr};
+  const int groups = (width + 127) / 128;
+  const int blocks = (int)std::min<int64_t>(zp_ceil_div(rows, kWarps), ZP_LN_PARTIALS);
+  const int np = !dgamma ? 0 : dbias ? 3 : 2;
+  const size_t smem = sizeof(float) * kWarps * np * (size_t)width;     // <= 96 KB
+#define CALL_NP(G, NP)                                                                          \
+  do {                                                                                          \
+    static ZpSmemOptIn opt_in;                                                                  \
+    if (int rc_ = zp_ensure_smem(ln_silu_bwd_kernel<G, NP>, smem, opt_in)) return rc_;          \
+    ln_silu_bwd_kernel<G, NP><<<blocks, 32 * kWarps, smem, st>>>(                               \
+        rows, width, x, gamma, beta, mean, rstd, dy, dx, dxp, scale, partial);                  \
+  } while (0)
+#define CALL(G)                      \
+  do {                               \
+    if (np == 3) CALL_NP(G, 3);      \
+    else if (np == 2) CALL_NP(G, 2); \
+    else CALL_NP(G, 0);              \
+  } while (0)
+  ZP_DISPATCH_GROUPS(groups, CALL);
+#undef CALL
+#undef CALL_NP
+  ZP_LAUNCH_CHECK("ln_silu_bwd_kernel");
+  float *const dst[3] = {dgamma, dbeta, dbias};
+  for (int k = 0; k < np; ++k)
+    list.add(partial + (size_t)k * width, dst[k], (int64_t)np * width, 1, width, blocks,
+             ZP_FIN_COLUMN);
+  return ZP_OK;
+}
+
 extern "C" {
 
 size_t zp_layernorm_work_bytes(int width) {
-  return sizeof(float) * (size_t)kPartialBlocks * 2 * (size_t)(width > 0 ? width : 0);
+  return sizeof(float) * (size_t)ZP_LN_PARTIALS * 2 * (size_t)(width > 0 ? width : 0);
 }
 
 int zp_layernorm_silu_forward(int64_t rows, int width, const float *x, const float *gamma,
@@ -207,15 +275,8 @@ int zp_layernorm_silu_forward(int64_t rows, int width, const float *x, const flo
   if (rows == 0) return ZP_OK;
   if (!x || !gamma || !beta || !y || !mean || !rstd) return ZP_ERR_INVALID_ARG;
   cudaStream_t st = (cudaStream_t)stream;
-  const int groups = (width + 127) / 128;
-  const unsigned grid = (unsigned)std::min<int64_t>(zp_ceil_div(rows, kWarps), 148 * 8);
-#define CALL(G)                                                                              \
-  ln_silu_fwd_kernel<G><<<grid, 32 * kWarps, 0, st>>>(rows, width, x, gamma, beta, eps, y, \
-                                                      mean, rstd)
-  ZP_DISPATCH_GROUPS(groups, CALL);
-#undef CALL
-  ZP_LAUNCH_CHECK("ln_silu_fwd_kernel");
-  return ZP_OK;
+  return zp_launch_ln_silu_fwd(rows, width, x, gamma, beta, eps, y, nullptr, ZpScale{}, mean, rstd,
+                               nullptr, st);
 }
 
 int zp_layernorm_silu_backward(int64_t rows, int width, const float *x, const float *gamma,
@@ -233,24 +294,11 @@ int zp_layernorm_silu_backward(int64_t rows, int width, const float *x, const fl
   }
   if (!x || !gamma || !beta || !mean || !rstd || !dy || !dx || !work) return ZP_ERR_INVALID_ARG;
   if (work_bytes < zp_layernorm_work_bytes(width)) return ZP_ERR_WORKSPACE;
-  const int groups = (width + 127) / 128;
-  const int blocks = (int)std::min<int64_t>(zp_ceil_div(rows, kWarps), kPartialBlocks);
-  const size_t smem = sizeof(float) * kWarps * 2 * (size_t)width;     // <= 64 KB
-  float *partial = static_cast<float *>(work);
-#define CALL(G)                                                                                 \
-  do {                                                                                          \
-    static ZpSmemOptIn opt_in;                                                                  \
-    if (int rc_ = zp_ensure_smem(ln_silu_bwd_kernel<G>, 65536, opt_in)) return rc_;             \
-    ln_silu_bwd_kernel<G><<<blocks, 32 * kWarps, smem, st>>>(rows, width, x, gamma, beta, mean, \
-                                                             rstd, dy, dx, partial);           \
-  } while (0)
-  ZP_DISPATCH_GROUPS(groups, CALL);
-#undef CALL
-  ZP_LAUNCH_CHECK("ln_silu_bwd_kernel");
-  ln_param_grad_kernel<<<(unsigned)zp_ceil_div(2 * width, 128), 128, 0, st>>>(blocks, width, partial,
-                                                                              dgamma, dbeta);
-  ZP_LAUNCH_CHECK("ln_param_grad_kernel");
-  return ZP_OK;
+  ZpFinalList list;
+  if ((rc = zp_launch_ln_silu_bwd(rows, width, x, gamma, beta, mean, rstd, dy, dx, nullptr, ZpScale{},
+                                  dgamma, dbeta, nullptr, static_cast<float *>(work), list, st)))
+    return rc;
+  return zp_launch_finalize(list, st);
 }
 
 }  // extern "C"

@@ -38,6 +38,40 @@ __device__ __forceinline__ float zp_scale_for_bound(float bound) {
   return ldexpf(1.f, e - 15);
 }
 
+// How the scale of a tensor's fp16 planes follows from device scalars (maxima of the operands the
+// tensor is formed from):  bound = factor * a * b * max(offset, c_factor * c * d) + e_factor * e,
+// null a, b, d counting as 1 and the terms of null c, e as 1 and 0.  The kernel that writes the
+// planes evaluates it itself -- every thread, a few loads of one cache line -- and its first
+// thread leaves the scale in *out for the consumers; a launch of its own would cost more than
+// the whole evaluation.
+struct ZpScale {
+  float factor;
+  const float *a, *b, *c, *d;
+  float offset, c_factor;
+  const float *e;
+  float e_factor;
+  float *out;              // null: the planes' scale is already in place
+};
+
+static inline ZpScale zp_scale_of(float factor, const float *a, float *out, const float *b = nullptr) {
+  return ZpScale{factor, a, b, nullptr, nullptr, 0.f, 1.f, nullptr, 0.f, out};
+}
+
+__device__ __forceinline__ float zp_eval_scale(const ZpScale &q) {
+  float bound = q.factor * (q.a ? *q.a : 1.f) * (q.b ? *q.b : 1.f);
+  if (q.c) bound *= fmaxf(q.offset, q.c_factor * *q.c * (q.d ? *q.d : 1.f));
+  if (q.e) bound += q.e_factor * *q.e;
+  return zp_scale_for_bound(bound);
+}
+// inverse scale for the writers of a tensor; `first`: the one thread that publishes the scale
+__device__ __forceinline__ float zp_publish_scale(const ZpPlanes &p, const ZpScale &q, bool first) {
+  if (!p.fp16) return 1.f;
+  if (!q.out) return zp_inv_scale(p);
+  const float s = zp_eval_scale(q);
+  if (first) *q.out = s;
+  return 1.f / s;
+}
+
 // writes VEC (2 or 4) consecutive values at element offset `idx` of every plane;
 // `inv` = zp_inv_scale(p), read once per thread.  The format is chosen by ONE warp-uniform branch
 // around the whole conversion (a per-element choice makes the compiler issue both conversions).

@@ -109,13 +109,14 @@ __global__ void __launch_bounds__(kRotInThreads, (LMAX <= 4 ? 4 : 3))
 rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
                  const float *__restrict__ x, const int32_t *__restrict__ src,
                  const int32_t *__restrict__ dst, const float *__restrict__ rot,
-                 const float *__restrict__ radial, const ZpPlanes a1) {
+                 const float *__restrict__ radial, const ZpPlanes a1, const ZpScale scale) {
   extern __shared__ float rot_s[];                       // [epb][nnz_pad]
   const int Q = t.C / 2;                                 // channel quads of the 2C-wide message
   const int64_t e0 = (int64_t)blockIdx.x * epb;
   const int n_e = (int)min((int64_t)epb, E - e0);
   for (int i = threadIdx.x; i < n_e * t.nnz_pad; i += blockDim.x)
     rot_s[i] = rot[e0 * t.nnz_pad + i];
+  const float inv = zp_publish_scale(a1, scale, blockIdx.x == 0 && threadIdx.x == 0);
   __syncthreads();
   const int le = threadIdx.x / Q, q = threadIdx.x % Q;
   if (le >= n_e) return;
@@ -125,7 +126,7 @@ rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
   const int64_t node = second ? dst[e] : src[e];
   const float *xrow = x + (size_t)node * t.K * t.C + (second ? c2 - t.C : c2);
   RotIn<LMAX, LMAX>::run(t, xrow, rot_s + le * t.nnz_pad, radial + (size_t)e * t.R,
-                         a1, e * a1.ld, c2, zp_inv_scale(a1));
+                         a1, e * a1.ld, c2, inv);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -397,7 +398,7 @@ __global__ void __launch_bounds__(kEdgeThreads, 3)
 rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t E, int W,
                        const float *__restrict__ g_out, const float *__restrict__ y,
                        const float *__restrict__ env, const float *__restrict__ rot,
-                       const int32_t *__restrict__ dst, const ZpPlanes dy,
+                       const int32_t *__restrict__ dst, const ZpPlanes dy, const ZpScale scale,
                        float *__restrict__ grad_env, float *__restrict__ grad_rot) {
   extern __shared__ float smem[];
   const int epb = 8 / W;
@@ -409,6 +410,7 @@ rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t E, int W,
   const int64_t e0 = (int64_t)blockIdx.x * epb;
   const int n_e = (int)min((int64_t)epb, E - e0);
   for (int i = threadIdx.x; i < n_e * t.nnz_pad; i += blockDim.x) rot_s[i] = rot[e0 * t.nnz_pad + i];
+  const float inv = zp_publish_scale(dy, scale, blockIdx.x == 0 && threadIdx.x == 0);
   __syncthreads();
   const bool edge_ok = slot < n_e;
   const int64_t e = e0 + (edge_ok ? slot : 0);
@@ -419,7 +421,7 @@ rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t E, int W,
     const float *g_row = g_out + (size_t)dst[e] * t.K * t.C + c;
     GradOutE<LMAX, LMAX>::run(t, g_row, y + (size_t)e * t.Km * t.C, dy, e * dy.ld,
                               rot_s + slot * t.nnz_pad, part_all + warp * t.nnz_pad, env[e], genv,
-                              c, active, lane, zp_inv_scale(dy));
+                              c, active, lane, inv);
     genv = warp_sum(genv);
     if (lane == 0) genv_s[warp] = genv;
   }
@@ -571,6 +573,7 @@ rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int W,
                      const float *__restrict__ x, const int32_t *__restrict__ src,
                      const int32_t *__restrict__ dst, const float *__restrict__ rot,
                      float *__restrict__ grad_radial, const ZpPlanes grad_radial_planes,
+                     const ZpScale scale,
                      float *__restrict__ du_both, float *__restrict__ grad_rot) {
   extern __shared__ __align__(16) float smem[];
   const int nw = blockDim.x / 32;
@@ -590,6 +593,7 @@ rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int W,
   StageInBwd<LMAX, LMAX>::run(t, da1 + (size_t)e * t.Km * 2 * t.C, radial + (size_t)e * t.R, stage,
                               c2, lane, active);
   for (int i = threadIdx.x; i < n_e * t.nnz_pad; i += blockDim.x) rot_s[i] = rot[e0 * t.nnz_pad + i];
+  const float inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && threadIdx.x == 0);
   __syncthreads();
   if (edge_ok) {
     const int half = c2 >= t.C ? 1 : 0;
@@ -599,7 +603,7 @@ rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int W,
     float *du_row = du_both ? du_both + ((size_t)e * 2 + half) * t.K * t.C + c : nullptr;
     RotInBwdE<LMAX, LMAX>::run(t, xrow, stage, radial + (size_t)e * t.R,
                                grad_radial + (size_t)e * t.R, grad_radial_planes,
-                               e * grad_radial_planes.ld, zp_inv_scale(grad_radial_planes),
+                               e * grad_radial_planes.ld, inv,
                                rot_s + slot * t.nnz_pad, part_all + warp * t.nnz_pad, du_row, c2,
                                active, lane);
   }
@@ -687,7 +691,7 @@ int zp_launch_node_sum(const zp_plan *p, int64_t N, const float *head, const flo
 
 int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32_t *src,
                         const int32_t *dst, const float *rot, const float *radial,
-                        const ZpPlanes &a1, cudaStream_t st) {
+                        const ZpPlanes &a1, const ZpScale &scale, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const ZpTables &t = p->t;
   const int Q = t.C / 2;
@@ -697,7 +701,7 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
   const dim3 grid((unsigned)zp_ceil_div(E, epb)), block(epb * Q);
   const size_t smem = (size_t)epb * t.nnz_pad * sizeof(float);
 #define CALL(LM) \
-  rotate_in_kernel<LM><<<grid, block, smem, st>>>(t, E, epb, x, src, dst, rot, radial, a1)
+  rotate_in_kernel<LM><<<grid, block, smem, st>>>(t, E, epb, x, src, dst, rot, radial, a1, scale)
   ZP_DISPATCH_LMAX(t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("rotate_in_kernel");
@@ -734,8 +738,8 @@ static int warps_per_edge(int quads) {
 
 int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const float *y,
                               const float *env, const float *rot, const int32_t *dst,
-                              const ZpPlanes &dy, float *grad_env, float *grad_rot,
-                              cudaStream_t st) {
+                              const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
+                              float *grad_rot, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const ZpTables &t = p->t;
   const int W = warps_per_edge(t.C / 4);
@@ -745,7 +749,7 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const
   const size_t smem = ((size_t)(epb + 8) * t.nnz_pad + 8) * sizeof(float);
 #define CALL(LM)                                                                              \
   rotate_grad_out_kernel<LM><<<grid, kEdgeThreads, smem, st>>>(t, E, W, g, y, env, rot, dst, dy, \
-                                                               grad_env, grad_rot)
+                                                               scale, grad_env, grad_rot)
   ZP_DISPATCH_LMAX(t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("rotate_grad_out_kernel");
@@ -755,7 +759,8 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const
 int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const float *radial,
                             const float *x, const int32_t *src, const int32_t *dst,
                             const float *rot, float *grad_radial, float *du_both, float *grad_rot,
-                            cudaStream_t st, const ZpPlanes *grad_radial_planes) {
+                            cudaStream_t st, const ZpPlanes *grad_radial_planes,
+                            const ZpScale &scale) {
   ZpPlanes gp{nullptr, 0, 0, 0, 0, nullptr};
   if (grad_radial_planes) gp = *grad_radial_planes;
   if (E == 0) return ZP_OK;
@@ -772,7 +777,7 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                  \
     if (int rc_ = zp_ensure_smem(rotate_in_bwd_kernel<LM>, smem, opt_in)) return rc_;          \
     rotate_in_bwd_kernel<LM><<<grid, 32 * nw, smem, st>>>(t, E, W, da1, radial, x, src, dst,   \
-                                                          rot, grad_radial, gp, du_both,       \
+                                                          rot, grad_radial, gp, scale, du_both, \
                                                           grad_rot);                           \
   }
   ZP_DISPATCH_LMAX(t.lmax, CALL)
