@@ -105,6 +105,16 @@ int zp_csr_build(const int64_t *edge_index /* [2,E] int64: row 0 src, row 1 dst 
                  int32_t *perm_src, int32_t *row_ptr_src, void *work, size_t work_bytes,
                  void *stream);
 
+/* zp_csr_build that also range-checks the element numbers [n_nodes] against [0, n_elements) and
+ * copies the flags to host memory (page-locked, valid once the stream has got there) instead of
+ * being asked for them: bit 0 a node index out of range, bit 1 an element number.  A caller can
+ * so enqueue the work that follows and look at the flags afterwards, without draining the device. */
+int zp_csr_build_checked(const int64_t *edge_index, int64_t n_edges, int64_t n_nodes,
+                         const int64_t *atomic_numbers, int n_elements, int32_t *perm,
+                         int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr,
+                         int32_t *perm_src, int32_t *row_ptr_src, int32_t *flags_host, void *work,
+                         size_t work_bytes, void *stream);
+
 /* zp_csr_build for callers that must not allocate device memory.  This entry point has no
  * counterpart in the reference.  A molecular-dynamics driver typically reserves all device
  * memory when it starts and then rebuilds its neighbour list every few steps from inside the
@@ -360,6 +370,54 @@ int zp_edge_features_backward(const zp_front_config *cfg, int64_t n_nodes, int64
                               const int32_t *perm_src, const int32_t *row_ptr_src,
                               float *grad_pos, float *grad_emb, void *work, size_t work_bytes,
                               void *stream);
+
+/* The whole block in two calls (blocks/eso2_ref.py:317-349 and autograd through it): the per-edge
+ * front end, the three dense layers of the radial MLP with their LayerNorm + SiLU pairs, and the
+ * edge convolution; positions to node_out, and back to every gradient.  Same results as the entry
+ * points above run one after the other, in fewer launches and passes.
+ * Node ranges as zp_eso2_forward: node_out holds rows first_node .. first_node + n_nodes of the
+ * n_rows nodes and the edges are those into them; row_ptr and row_ptr_src cover all n_rows nodes.
+ * Per-edge inputs (shifts, cos_g, sin_g) are in the caller's order, `perm` names the position of a
+ * sorted edge in them; perm .. row_ptr_src from zp_csr_build.                                    */
+typedef struct zp_block_call {
+  int64_t n_nodes, n_edges, n_rows, first_node;
+  const float *pos;                /* [n_rows, 3]                                               */
+  const float *shifts;             /* [*, 3]                                                    */
+  const int64_t *atomic_numbers;   /* [n_rows]                                                  */
+  const float *x_node;             /* [n_rows, K, C]                                            */
+  const float *cos_g, *sin_g;      /* [*, lmax + 1]                                             */
+  const int32_t *perm, *src, *dst, *row_ptr, *perm_src, *row_ptr_src;
+} zp_block_call;
+typedef struct zp_block_params {
+  const float *emb, *gauss_offsets;
+  const float *rad_w[3], *rad_b[3];        /* Linear layers of rad_func                         */
+  const float *ln_gamma[2], *ln_beta[2];   /* LayerNorms between them                           */
+  float ln_eps;
+  zp_weights so2;
+} zp_block_params;
+/* null: not wanted; the radial parameters (rad_w .. ln_beta) and the SO(2) weights each all or none */
+typedef struct zp_block_grads {
+  float *emb;
+  float *rad_w[3], *rad_b[3];
+  float *ln_gamma[2], *ln_beta[2];
+  zp_weight_grads so2;
+} zp_block_grads;
+/* with_backward: ZP_WS_BACKWARD for a forward that keeps what a backward reads (and that backward),
+ * ZP_WS_INFERENCE for one that does not.                                                         */
+size_t zp_block_workspace_bytes(const zp_plan *plan, const zp_front_config *front, int64_t n_nodes,
+                                int64_t n_rows, int64_t n_edges, int with_backward);
+/* x_ready_event (a cudaEvent_t, or null): x_node is valid after it; the stream waits for it only
+ * where the embeddings are first read.                                                           */
+int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp_block_call *call,
+                     const zp_block_params *params, float *node_out, void *workspace,
+                     size_t workspace_bytes, int keep_for_backward, void *x_ready_event,
+                     void *stream);
+/* grad_node_out as zp_eso2_backward (indexed by dst); grad_x_node [n_rows, K, C] and
+ * grad_pos [n_rows, 3] may be null.                                                              */
+int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const zp_block_call *call,
+                      const zp_block_params *params, const float *grad_node_out,
+                      float *grad_x_node, float *grad_pos, const zp_block_grads *grads,
+                      void *workspace, size_t workspace_bytes, void *stream);
 
 /* Periodic neighbour list with the per-destination cap, on the device (the graph front end; the
  * reference builds edge lists on the host with an external package and applies no cap,

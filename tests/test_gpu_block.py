@@ -1,0 +1,80 @@
+"""The whole-block calls (zp_block_forward / zp_block_backward behind ``ESO2Block.node_output``) and
+the checked edge sort, at the sizes where their dispatch turns: widths that are and are not
+multiples of 8 (operand format of a layer, zero padding), frozen parameter groups, no edges."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+from oracle import eso2_oracle as orc
+from tests.helpers import (check_against, gpu_node_out_and_vjp, make_block, oracle_node_out_and_vjp,
+                           random_case, rel_l2)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision,tol", [("fp32", 1e-5), ("fp32_bf16x3", 1e-5), ("bf16", 2e-2)])
+@pytest.mark.parametrize("ec,nb", [(12, 5), (8, 6), (20, 8), (132, 64)])
+def test_radial_layer_widths(ec, nb, precision, tol, jd64):
+    cfg = dict(lmax=2, mmax=1, sphere_channels=16, hidden_channels=8, edge_channels=ec,
+               num_distance_basis=nb, cutoff=5.0)
+    params = orc.init_params(cfg, seed=ec)
+    case = random_case(cfg, 17, 131, seed=nb)
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    block = make_block(cfg, params, precision=precision)
+    check_against(*gpu_node_out_and_vjp(block, case, case["upstream"]), *want, tol=tol)
+    assert block.plan("cuda").device_status() == 0
+
+
+@pytest.mark.parametrize("frozen", [("elem_emb",), ("rad_func",), ("c1_", "c2_"), ("elem_emb", "rad_func")])
+def test_frozen_groups_leave_the_other_gradients_alone(frozen):
+    cfg = dict(lmax=3, mmax=2, sphere_channels=16, hidden_channels=16, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1))
+    case = {k: v.cuda().float() if v.is_floating_point() else v.cuda()
+            for k, v in random_case(cfg, 20, 150, seed=2).items()}
+
+    def grads():
+        pos, x = case["pos"].clone().requires_grad_(True), case["x_node"].clone().requires_grad_(True)
+        out = block.node_output(pos, case["atomic_numbers"], x, case["edge_index"], case["shifts"],
+                                case["cos_gamma_k"], case["sin_gamma_k"])
+        names = ["pos", "x"] + [n for n, p in block.named_parameters() if p.requires_grad]
+        wrt = [pos, x] + [p for p in block.parameters() if p.requires_grad]
+        return dict(zip(names, torch.autograd.grad(out, wrt, case["upstream"], allow_unused=True)))
+
+    full = grads()
+    for n, p in block.named_parameters():
+        p.requires_grad_(not n.startswith(frozen))
+    part = grads()
+    assert set(full) - set(part) == {n for n in full if n.startswith(frozen)}
+    for n, g in part.items():
+        assert (g is None) == (full[n] is None) and (g is None or rel_l2(g, full[n]) < 1e-6), n
+
+
+@pytest.mark.parametrize("n,degree", [(3, 31), (3, 33), (2, 64), (2, 65), (16385, 2), (40000, 3)])
+def test_sort_at_its_bucket_and_scan_edges(n, degree):
+    import numpy as np
+    from zippel_b200.graph import EdgeGraph, csr_reference
+    g = torch.Generator("cpu").manual_seed(n + degree)
+    ei = torch.stack([torch.randint(0, n, (n * degree,), generator=g),
+                      torch.arange(n).repeat_interleave(degree)])[:, torch.randperm(n * degree, generator=g)]
+    want = csr_reference(ei.numpy(), n)
+    got, check = EdgeGraph.build_checked(ei.cuda(), torch.zeros(n, dtype=torch.int64, device="cuda"), 5)
+    check()
+    for key, val in want.items():
+        assert np.array_equal(getattr(got, key).cpu().numpy(), val), key
+
+
+@pytest.mark.parametrize("what", ["edge", "element"])
+def test_bad_input_raises(what):
+    cfg = dict(lmax=1, mmax=1, sphere_channels=8, hidden_channels=8, edge_channels=8,
+               num_distance_basis=4, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1))
+    case = random_case(cfg, 6, 20, seed=2)
+    if what == "edge":
+        case["edge_index"][0, 3] = 6
+    else:
+        case["atomic_numbers"][5] = block.cfg.max_num_elements
+    with pytest.raises(IndexError):
+        gpu_node_out_and_vjp(block, case, case["upstream"])

@@ -43,6 +43,24 @@ class ZpWeights(C.Structure):
                 ("c2_w0", C.c_void_p), ("c2_b0", C.c_void_p), ("c2_wm", C.POINTER(C.c_void_p))]
 
 
+class ZpBlockCall(C.Structure):
+    _fields_ = ([(n, C.c_int64) for n in ("n_nodes", "n_edges", "n_rows", "first_node")]
+                + [(n, C.c_void_p) for n in ("pos", "shifts", "atomic_numbers", "x_node", "cos_g",
+                                             "sin_g", "perm", "src", "dst", "row_ptr", "perm_src",
+                                             "row_ptr_src")])
+
+
+class ZpBlockParams(C.Structure):
+    _fields_ = [("emb", C.c_void_p), ("gauss_offsets", C.c_void_p), ("rad_w", C.c_void_p * 3),
+                ("rad_b", C.c_void_p * 3), ("ln_gamma", C.c_void_p * 2), ("ln_beta", C.c_void_p * 2),
+                ("ln_eps", C.c_float), ("so2", ZpWeights)]
+
+
+class ZpBlockGrads(C.Structure):
+    _fields_ = [("emb", C.c_void_p), ("rad_w", C.c_void_p * 3), ("rad_b", C.c_void_p * 3),
+                ("ln_gamma", C.c_void_p * 2), ("ln_beta", C.c_void_p * 2), ("so2", ZpWeights)]
+
+
 # name -> (restype, argtypes); must list every symbol of include/zippel_b200.h
 _P, _I64, _SZ = C.c_void_p, C.c_int64, C.c_size_t
 SIGNATURES = {
@@ -55,6 +73,8 @@ SIGNATURES = {
     "zp_plan_tables": (C.c_int, [_P] + [C.POINTER(C.c_int32)] * 4),
     "zp_csr_work_bytes": (_SZ, [_I64, _I64]),
     "zp_csr_build": (C.c_int, [_P, _I64, _I64, _P, _P, _P, _P, _P, _P, _P, _SZ, _P]),
+    "zp_csr_build_checked": (C.c_int, [_P, _I64, _I64, _P, C.c_int, _P, _P, _P, _P, _P, _P, _P, _P,
+                                       _SZ, _P]),
     "zp_csr_build_static": (C.c_int, [_P, _I64, _I64, _P, _P, _P, _P, _P, _P, _P]),
     "zp_csr_status": (C.c_int, [_P, _P, C.POINTER(C.c_int)]),
     "zp_csr_static_status": (C.c_int, [_P, C.POINTER(C.c_int)]),
@@ -92,6 +112,12 @@ SIGNATURES = {
     "zp_edge_features_forward": (C.c_int, [C.POINTER(ZpFrontConfig), _I64, _I64] + [_P] * 16 + [_P]),
     "zp_edge_features_backward": (C.c_int, [C.POINTER(ZpFrontConfig), _I64, _I64] + [_P] * 14
                                   + [_SZ, _P]),
+    "zp_block_workspace_bytes": (_SZ, [_P, C.POINTER(ZpFrontConfig), _I64, _I64, _I64, C.c_int]),
+    "zp_block_forward": (C.c_int, [_P, C.POINTER(ZpFrontConfig), C.POINTER(ZpBlockCall),
+                                   C.POINTER(ZpBlockParams), _P, _P, _SZ, C.c_int, _P, _P]),
+    "zp_block_backward": (C.c_int, [_P, C.POINTER(ZpFrontConfig), C.POINTER(ZpBlockCall),
+                                    C.POINTER(ZpBlockParams), _P, _P, _P, C.POINTER(ZpBlockGrads),
+                                    _P, _SZ, _P]),
     "zp_neighbors_work_bytes": (_SZ, [_I64, C.c_double, C.c_double]),
     "zp_neighbors_count": (C.c_int, [_P, _I64, C.c_double, C.c_double, C.c_int, _P, _P, _P, _SZ, _P]),
     "zp_neighbors_fill": (C.c_int, [_P, _I64, C.c_double, C.c_double, C.c_int, _P, _I64, _P, _P, _P,

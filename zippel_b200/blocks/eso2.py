@@ -8,13 +8,13 @@ do not provide).  Unlike the reference, ``mmax < lmax`` works: the l-major -> m'
 is the rectangular ``[Km, K]`` matrix.
 
 What runs where
-    * the per-edge front end (geometry, Gaussian basis, element embeddings, envelope) is one
-      kernel each way (``EdgeFeatures``); the radial MLP runs on the contraction engine
-      (``TensorCoreLinear``) with fused LayerNorm + SiLU passes (``LayerNormSiLU``);
-    * everything per edge and per (l, m, channel) -- gather, Wigner-D rotation, both SO(2)
-      convolutions, the gate, rotation back and the scatter onto destination nodes, forward and
-      VJP -- is one call into the C ABI (``zp_eso2_forward`` / ``zp_eso2_backward``) through
-      ``EdgeConvFunction``;
+    * the block from positions to node output -- per-edge front end, radial MLP, and everything
+      per edge and per (l, m, channel): gather, Wigner-D rotation, both SO(2) convolutions, the
+      gate, rotation back and the scatter onto destination nodes -- is one call into the C ABI each
+      way (``zp_block_forward`` / ``zp_block_backward``) through ``BlockFunction``;
+    * its pieces are autograd functions of their own for callers that have radial features or other
+      inputs in hand: ``EdgeFeatures``, ``TensorCoreLinear``, ``LayerNormSiLU``, and the edge
+      convolution alone, ``EdgeConvFunction`` (``zp_eso2_forward`` / ``zp_eso2_backward``);
     * the readout head after the node output (invariants, two dense layers, sum over atoms) is
       ``Readout`` (``zp_readout_forward`` / ``zp_readout_backward``).
 There is no fallback: without the built library and a supported GPU every call raises, and
@@ -128,6 +128,11 @@ class Plan:
         sizes = _lib.ZpSizes()
         _lib.check(lib.zp_plan_sizes(handle, ctypes.byref(sizes)), "zp_plan_sizes")
         self.sizes = sizes
+        # what one more edge adds to a call that keeps what its backward reads
+        probe = 4096
+        self.bytes_per_edge = max(1.0, (lib.zp_workspace_bytes(handle, 0, probe, 1)
+                                        - lib.zp_workspace_bytes(handle, 0, 0, 1)) / probe)
+        self.total_memory = torch.cuda.get_device_properties(device).total_memory
         self.lmax, self.mmax, self.c, self.h = lmax, mmax, c, h
 
     @classmethod
@@ -192,14 +197,18 @@ MAX_EDGES_PER_CALL: int | None = None
 def _edge_budget(plan: Plan, n: int, e: int) -> int:
     if MAX_EDGES_PER_CALL is not None:
         return max(1, MAX_EDGES_PER_CALL)
-    lib = _lib.load()
-    probe = 4096
-    per_edge = (lib.zp_workspace_bytes(plan.handle, 0, probe, 1)
-                - lib.zp_workspace_bytes(plan.handle, 0, 0, 1)) / probe
     free, _total = torch.cuda.mem_get_info(plan.device)
     # memory the caching allocator holds but is not using can be re-used for the workspace
     free += torch.cuda.memory_reserved(plan.device) - torch.cuda.memory_allocated(plan.device)
-    return _quantise_budget(max(1024, int(0.5 * free / max(per_edge, 1.0))))
+    return _quantise_budget(max(1024, int(0.5 * free / plan.bytes_per_edge)))
+
+
+def _surely_fits(plan: Plan, e: int) -> bool:
+    """Whether ``e`` edges take so little of the device's memory (an eighth, gradients included)
+    that a call is made in one piece without asking how much is free, a question that costs the
+    host more than a small call's launches.  A call that runs out of memory all the same is made
+    again in pieces."""
+    return MAX_EDGES_PER_CALL is None and 16 * e * plan.bytes_per_edge <= plan.total_memory
 
 
 def _quantise_budget(budget: int) -> int:
@@ -305,7 +314,7 @@ class EdgeConvFunction(torch.autograd.Function):
         wstruct, keep = _weights_struct(mmax, w10, b10, wms[:mmax], w20, b20, wms[mmax:])
         with torch.cuda.device(x.device):
             # a node-range graph is already one piece of a chunked run: never split it again
-            chunks = ([EdgeChunk(0, e, 0, n, graph)] if rng is not None
+            chunks = ([EdgeChunk(0, e, 0, n, graph)] if rng is not None or _surely_fits(plan, e)
                       else graph.chunks(_edge_budget(plan, n, e)))
             if len(chunks) == 1:
                 ws = plan.workspace(n1 - n0, e, needs_bwd, inference=not needs_bwd, edge_channels=ec)
@@ -664,13 +673,109 @@ def radial_mlp(plan: Plan, x_edge: torch.Tensor, layers: list) -> torch.Tensor:
     return h
 
 
-def edge_conv(plan: Plan, graph: EdgeGraph, x_node, edge_vec, cos_g, sin_g, radial, env,
-              c1_m0: nn.Linear, c1_m, c2_m0: nn.Linear, c2_m, rad_w=None, rad_b=None) -> torch.Tensor:
-    """``rad_w`` / ``rad_b``: see ``EdgeConvFunction`` (``radial`` is then the last radial
-    layer's input)."""
-    return EdgeConvFunction.apply(plan, graph, x_node, edge_vec, cos_g, sin_g, radial, env,
-                                  rad_w, rad_b, c1_m0.weight, c1_m0.bias, c2_m0.weight, c2_m0.bias,
-                                  *[l.weight for l in c1_m], *[l.weight for l in c2_m])
+class BlockFunction(torch.autograd.Function):
+    """node_out = the whole block from positions and embeddings (``zp_block_forward``), with the VJP
+    of all of it (``zp_block_backward``): reference blocks/eso2_ref.py:317-349 and autograd through
+    it.  ``block`` gives the configuration, ``params`` are its parameters in registration order
+    without the readout; ``perm``: int32 positions of the graph's sorted edges in the per-edge arrays.
+    fp32, first order only."""
+
+    @staticmethod
+    def forward(ctx, block, plan: Plan, graph: EdgeGraph, perm, atomic_numbers, shifts, cos_g, sin_g,
+                x_ready, pos, x_node, *params):
+        lib, cfg, s = _lib.load(), block.cfg, plan.sizes
+        needs_bwd = any(ctx.needs_input_grad)
+        n, e = graph.n_nodes, graph.n_edges
+        n0, n1 = getattr(graph, "node_range", None) or (0, n)
+        dtypes = [t.dtype for t in (pos, x_node, *params)]
+        pos, x, shifts, cos_g, sin_g = (_as_f32(t) for t in (pos, x_node, shifts, cos_g, sin_g))
+        params = [_as_f32(t) for t in params]
+        off, z = _as_f32(block.gauss_offset), atomic_numbers
+        if z.dtype != torch.int64 or not z.is_contiguous():
+            z = z.to(torch.int64).contiguous()
+        for t in (pos, x, shifts, z, *params):
+            if not t.is_cuda:
+                raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
+        assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
+        assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.shape == (n,)
+        assert cos_g.shape[1] == cfg.lmax + 1 and sin_g.shape == cos_g.shape
+        assert min(shifts.shape[0], cos_g.shape[0]) >= e
+        out = torch.empty(n1 - n0, s.K, plan.c, dtype=torch.float32, device=x.device)
+        front = block.front_config()
+        nbytes = lib.zp_block_workspace_bytes(plan.handle, front, n1 - n0, n, e, 1 if needs_bwd else 2)
+        if nbytes == 0:
+            raise _lib.ZpError(2, "zp_block_workspace_bytes")
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+        call = _lib.ZpBlockCall(
+            n1 - n0, e, n, n0, pos.data_ptr(), shifts.data_ptr(), z.data_ptr(), x.data_ptr(),
+            cos_g.data_ptr(), sin_g.data_ptr(), perm.data_ptr(), graph.src.data_ptr(),
+            graph.dst.data_ptr(), graph.row_ptr.data_ptr(), graph.perm_src.data_ptr(),
+            graph.row_ptr_src.data_ptr())
+        p = [t.data_ptr() for t in params]
+        m = plan.mmax
+        so2, keep = _weights_ptrs(m, p[11:])
+        cparams = _lib.ZpBlockParams(p[0], off.data_ptr(), _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
+                                     _P2(p[3], p[7]), _P2(p[4], p[8]), block.rad_func[1].eps, so2)
+        with torch.cuda.device(x.device):
+            _lib.check(lib.zp_block_forward(
+                plan.handle, front, call, cparams, out.data_ptr(), ws.data_ptr(), nbytes, needs_bwd,
+                x_ready.cuda_event if x_ready is not None else None,
+                torch.cuda.current_stream().cuda_stream), "zp_block_forward")
+        if needs_bwd:
+            # the workspace goes through save_for_backward like any activation, so that activation
+            # checkpointing can drop it and recompute; of the parameters the backward reads only
+            # the LayerNorms' (the products read the planes in the workspace)
+            ctx.save_for_backward(ws, x, pos, z, off, params[3], params[4], params[7], params[8])
+            ctx.native = (plan, graph, front, call, cparams, keep)
+            ctx.shapes, ctx.dtypes = [t.shape for t in params], dtypes
+            ctx.row0 = n0
+        return out.to(dtypes[1])
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_out):
+        ws, x, pos = ctx.saved_tensors[:3]
+        plan, graph, front, call, cparams, _keep = ctx.native
+        g = _as_f32(grad_out)
+        want = ctx.needs_input_grad[9:]
+        f32 = dict(dtype=torch.float32, device=x.device)
+        gpos = torch.empty(pos.shape, **f32) if want[0] else None
+        gx = torch.empty(x.shape, **f32) if want[1] else None
+        # frozen parameters: the products behind their gradients are not run; the radial and the
+        # SO(2) parameters are each formed together
+        wp = want[2:]
+        groups = [wp[0]] + [any(wp[1:11])] * 10 + [any(wp[11:])] * (len(wp) - 11)
+        gp = [torch.empty(sh, **f32) if w else None for sh, w in zip(ctx.shapes, groups)]
+        p = [t.data_ptr() if t is not None else None for t in gp]
+        so2, keep = (_weights_ptrs(plan.mmax, p[11:]) if p[11] is not None
+                     else (_lib.ZpWeights(), None))
+        grads = _lib.ZpBlockGrads(p[0], _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
+                                  _P2(p[3], p[7]), _P2(p[4], p[8]), so2)
+        with torch.cuda.device(x.device):
+            _lib.check(_lib.load().zp_block_backward(
+                plan.handle, front, call, cparams,
+                g.data_ptr() - ctx.row0 * plan.sizes.K * plan.c * 4,
+                gx.data_ptr() if gx is not None else None,
+                gpos.data_ptr() if gpos is not None else None, grads, ws.data_ptr(), ws.numel(),
+                torch.cuda.current_stream().cuda_stream), "zp_block_backward")
+        del keep
+        out = [t if t is None or t.dtype == dt else t.to(dt)
+               for t, dt in zip([gpos, gx, *gp], ctx.dtypes)]
+        return (None,) * 9 + tuple(t if w else None for t, w in zip(out, want))
+
+
+_P2, _P3 = ctypes.c_void_p * 2, ctypes.c_void_p * 3
+
+
+def _as_f32(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dtype == torch.float32 and t.is_contiguous() else _f32(t)
+
+
+def _weights_ptrs(mmax: int, p: list):
+    """ZpWeights from addresses in parameter order: c1_w0, c1_b0, c1_wm.., c2_w0, c2_b0, c2_wm.."""
+    arr = ctypes.c_void_p * max(mmax, 1)
+    a1, a2 = arr(*p[2:2 + mmax]), arr(*p[4 + mmax:4 + 2 * mmax])
+    return _lib.ZpWeights(p[0], p[1], a1, p[2 + mmax], p[3 + mmax], a2), (a1, a2)
 
 
 # --------------------------------------------------------------------------------------------
@@ -763,31 +868,25 @@ class ESO2Block(nn.Module):
         return radial_mlp(plan, x_edge, list(self.rad_func))
 
     # -- forward --------------------------------------------------------------------------
+    def _block_params(self) -> list:
+        """Parameters of everything before the readout, in registration order."""
+        params = list(self.parameters())
+        return params[:len(params) - 4]
+
     def _edges_to_nodes(self, plan, graph, perm, pos, atomic_numbers, x_node, shifts, cos_gamma_k,
                         sin_gamma_k, x_ready=None) -> torch.Tensor:
-        """Geometry, radial features, envelope and the edge convolution for the edges of `graph`
-        (whose original positions in the caller's arrays are `perm`)."""
-        cfg = self.cfg
+        """node_out rows of the edges of `graph` (whose positions in the caller's arrays are the
+        int32 `perm`)."""
+        return BlockFunction.apply(self, plan, graph, perm, atomic_numbers, shifts, cos_gamma_k,
+                                   sin_gamma_k, x_ready, pos, x_node, *self._block_params())
 
-        def conv(*args):
-            if x_ready is not None:        # x_node is still arriving on another stream
-                torch.cuda.current_stream(pos.device).wait_event(x_ready)
-            return edge_conv(*args)
-
-        # geometry, distance basis, embeddings, envelope and the sorted copies in one pass
-        edge_vec, x_edge, env, cos_s, sin_s = EdgeFeatures.apply(
-            graph, perm.to(torch.int32).contiguous(), self.front_config(), pos, shifts,
-            atomic_numbers, self.elem_emb.weight, self.gauss_offset, cos_gamma_k, sin_gamma_k)
-        last = self.rad_func[-1]
-        if isinstance(last, nn.Linear) and last.in_features % 8 == 0 and graph.n_edges > 0:
-            # the last (widest) radial layer runs inside the edge-convolution call: its output
-            # and that output's gradient never leave the kernel path
-            h_rad = radial_mlp(plan, x_edge, list(self.rad_func)[:-1])
-            return conv(plan, graph, x_node, edge_vec, cos_s, sin_s, h_rad, env,
-                        self.c1_m0, self.c1_m, self.c2_m0, self.c2_m, last.weight, last.bias)
-        radial = self.radial_mlp(plan, x_edge)
-        return conv(plan, graph, x_node, edge_vec, cos_s, sin_s, radial, env,
-                    self.c1_m0, self.c1_m, self.c2_m0, self.c2_m)
+    def _sorted_edges(self, edge_index, atomic_numbers):
+        """The edge order of new input and the check of its indices, to be called once the work that
+        follows has been enqueued (nothing can be checked while a stream is being captured: the
+        kernels leave edges with bad indices out and clamp element numbers either way)."""
+        if torch.cuda.is_current_stream_capturing():
+            return EdgeGraph.build(edge_index, atomic_numbers.shape[0]), None
+        return EdgeGraph.build_checked(edge_index, atomic_numbers, self.cfg.max_num_elements)
 
     def node_output(self, pos, atomic_numbers, x_node, edge_index, shifts, cos_gamma_k,
                     sin_gamma_k, graph: EdgeGraph | None = None,
@@ -801,33 +900,43 @@ class ESO2Block(nn.Module):
         Graphs whose per-edge activations (radial features included) exceed the memory budget
         are processed as destination-node chunks under activation checkpointing: each chunk's
         forward is recomputed in the backward, so memory stays bounded by one chunk."""
-        n = pos.shape[0]
+        check = None
         if graph is None:
-            # new input: node indices are range-checked by the sort, element numbers here (a
-            # caller that passes a prebuilt graph has had both checked when it was built)
-            graph = EdgeGraph.build(edge_index, n)
-            if (atomic_numbers.numel() and not torch.cuda.is_current_stream_capturing()
-                    and not bool(((atomic_numbers >= 0)
-                                  & (atomic_numbers < self.cfg.max_num_elements)).all())):
-                raise IndexError(f"atomic_numbers outside [0, {self.cfg.max_num_elements})")
+            # new input: node indices and element numbers are range-checked (a caller that passes
+            # a prebuilt graph has had them checked when it was built)
+            graph, check = self._sorted_edges(edge_index, atomic_numbers)
         plan = self.plan(pos.device)
+        args = (atomic_numbers, shifts, cos_gamma_k, sin_gamma_k)
+        try:
+            out = None
+            if _surely_fits(plan, graph.n_edges):
+                try:
+                    out = self._edges_to_nodes(plan, graph, graph.perm, pos, args[0], x_node,
+                                               *args[1:], x_ready)
+                except torch.cuda.OutOfMemoryError:
+                    pass
+            if out is None:
+                out = self._node_output_in_chunks(plan, graph, pos, x_node, args, x_ready)
+        finally:
+            if check is not None:
+                check()
+        return out
+
+    def _node_output_in_chunks(self, plan, graph, pos, x_node, args, x_ready) -> torch.Tensor:
         # radial features and their gradients roughly double the per-edge footprint
-        budget = max(1024, _edge_budget(plan, n, graph.n_edges) // 2)
-        chunks = graph.chunks(budget)
-        perm = graph.perm64
+        chunks = graph.chunks(max(1024, _edge_budget(plan, pos.shape[0], graph.n_edges) // 2))
         if len(chunks) == 1:
-            return self._edges_to_nodes(plan, graph, perm, pos, atomic_numbers, x_node, shifts,
-                                        cos_gamma_k, sin_gamma_k, x_ready)
+            return self._edges_to_nodes(plan, graph, graph.perm, pos, args[0], x_node, *args[1:],
+                                        x_ready)
         if x_ready is not None:
             torch.cuda.current_stream(pos.device).wait_event(x_ready)
         from torch.utils.checkpoint import checkpoint
         outs = []
         for c in chunks:
-            sub_perm = perm[c.e0:c.e1]
+            sub_perm = graph.perm[c.e0:c.e1]
 
             def run(pos_, x_, c=c, sub_perm=sub_perm):
-                return self._edges_to_nodes(plan, c.sub, sub_perm, pos_, atomic_numbers, x_, shifts,
-                                            cos_gamma_k, sin_gamma_k)
+                return self._edges_to_nodes(plan, c.sub, sub_perm, pos_, args[0], x_, *args[1:])
 
             if torch.is_grad_enabled():
                 outs.append(checkpoint(run, pos, x_node, use_reentrant=False))
@@ -856,36 +965,33 @@ class ESO2Block(nn.Module):
         if graph is None:
             graph = EdgeGraph.build(edge_index, n)
         plan = self.plan(pos.device)
-        budget = max(1024, _edge_budget(plan, n, graph.n_edges) // 2)
-        chunks = graph.chunks(budget)
-        perm = graph.perm64
+        if _surely_fits(plan, graph.n_edges):
+            chunks = [EdgeChunk(0, graph.n_edges, 0, n, graph)]
+        else:
+            chunks = graph.chunks(max(1024, _edge_budget(plan, n, graph.n_edges) // 2))
         params = list(self.parameters())
-        gx = torch.zeros_like(x_node)
-        gpos = torch.zeros_like(pos)
-        gparams: list = [None] * len(params)
+        total = None
         outs = []
         for c in chunks:
-            if len(chunks) > 1:
-                sub_graph, sub_perm = c.sub, perm[c.e0:c.e1]
-            else:
-                sub_graph, sub_perm = graph, perm
+            sub_perm = graph.perm[c.e0:c.e1] if len(chunks) > 1 else graph.perm
             pos_ = pos.detach().requires_grad_(True)
             x_ = x_node.detach().requires_grad_(True)
             with torch.enable_grad():
-                rows = self._edges_to_nodes(plan, sub_graph, sub_perm, pos_, atomic_numbers, x_,
+                rows = self._edges_to_nodes(plan, c.sub, sub_perm, pos_, atomic_numbers, x_,
                                             shifts, cos_gamma_k, sin_gamma_k)
             g_rows = (upstream(rows.detach(), c.n0, c.n1) if callable(upstream)
                       else upstream[c.n0:c.n1])
             grads = torch.autograd.grad(rows, [x_, pos_, *params], g_rows, allow_unused=True)
-            gx += grads[0]
-            gpos += grads[1]
-            for i, g in enumerate(grads[2:]):
-                if g is not None:
-                    gparams[i] = g if gparams[i] is None else gparams[i].add_(g)
+            if total is None:
+                total = list(grads)
+            else:
+                for a, b in zip(total, grads):
+                    if a is not None:
+                        a.add_(b)
             outs.append(rows.detach())
             del rows, grads, g_rows
         node_out = outs[0] if len(outs) == 1 else torch.cat(outs, dim=0)
-        return node_out, gx, gpos, gparams
+        return node_out, total[0], total[1], total[2:]
 
     def _check_jd(self, jd) -> None:
         """The kernels hold the J matrices shipped with the package; a caller's ``jd`` (the

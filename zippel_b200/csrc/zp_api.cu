@@ -668,8 +668,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   const float *radial = rl ? ws.radial : c.radial;      // rl: left there by the forward
 
   const bool scaled_gr = rl && ws.gr.fp16;               // the planes of grad_radial have a scale
-  if (plan->fp16 || scaled_gr)
-    ZP_CUDA(cudaMemsetAsync(ws.scales + kScBwd, 0, sizeof(float) * (kScBwdEnd - kScBwd), st));
+  ZP_CUDA(cudaMemsetAsync(ws.scales + kScBwd, 0, sizeof(float) * (kScBwdEnd - kScBwd), st));
   if (plan->fp16 && E > 0) {
     // only rows dst[0] .. dst[E-1] (the edges are destination-sorted): the rows the kernels read,
     // and the only ones a caller that holds a node range's rows alone has

@@ -79,9 +79,16 @@ enum { kScX = 0, kScRad, kScH1, kScA1, kScHt, kScDy, kScDh1, kScGate, kScMaxNode
        // the radial layer run inside the call: {max, scale} of its input and of its weight, scale
        // of the planes of grad_radial
        kScHr, kScHrScale, kScRw, kScRwScale, kScGrScale,
-       kScBwd, kScG = kScBwd, kScDht, kScDa1, kScBwdEnd,
+       // maxima a backward accumulates: upstream gradient, conv2's and conv1's input gradient,
+       // gradients of the radial MLP's two hidden activations
+       kScBwd, kScG = kScBwd, kScDht, kScDa1, kScGHid1, kScGHid0, kScBwdEnd,
        kScWeights = 24,
-       kScCount = kScWeights + 4 * (ZP_MAX_L + 1) };
+       // the rest of the radial MLP (whole-block calls): maxima of the embedding table, of the
+       // LayerNorm parameters and of 1/std, {max, scale} of the two weights, scales of activations
+       // and gradients
+       kScEmb = kScWeights + 4 * (ZP_MAX_L + 1), kScGamma0, kScBeta0, kScGamma1, kScBeta1, kScRstd0,
+       kScRstd1, kScW0, kScW0Scale, kScW1, kScW1Scale, kScXe, kScHid0, kScDz1, kScDz0,
+       kScCount };
 
 constexpr int kZpWgradSplits = 8;
 constexpr int kZpRadialSplits = 8;       // K splits of the radial layer's weight gradient

@@ -15,132 +15,230 @@ static __device__ __align__(256) unsigned char g_csr_static_scratch[ZP_CSR_STATI
 
 namespace {
 
-constexpr int kScanBlock = 1024;
+constexpr int kScanThreads = 1024;
+constexpr int kScanItems = 8;                          // counters per thread and scan step
+constexpr int kScanSpan = kScanThreads * kScanItems;   // counters per block of a multi-block scan
+constexpr int64_t kScanOneBlock = 2 * kScanSpan;       // up to here one block per array does it all
+
+enum { kFlagEdges = 1, kFlagElements = 2 };
 
 // Node indices come from the caller.  One outside [0, N) is never used as an address: the edge
 // is left out, the flag word is raised, and zp_csr_status reports it (the arrays of such a call
-// are not a valid sort).
-__global__ void count_kernel(int64_t E, int64_t N, const int64_t *__restrict__ key,
-                             const int64_t *__restrict__ other, int32_t *counts, int32_t *flag) {
+// are not a valid sort).  Both views are counted in one pass; the slot that an omitted edge leaves
+// in the sorted list reads as an edge 0 -> 0, so it counts for source 0.  Element numbers, when
+// given, are only range-checked.
+__global__ void count_kernel(int64_t E, int64_t N, const int64_t *__restrict__ src,
+                             const int64_t *__restrict__ dst, const int64_t *__restrict__ z,
+                             int n_elements, int32_t *cnt_dst, int32_t *cnt_src, int32_t *flag) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (z && i < N && (uint64_t)z[i] >= (uint64_t)n_elements) atomicOr(flag, kFlagElements);
   if (i >= E) return;
-  const int64_t k = key[i];
-  if ((uint64_t)k >= (uint64_t)N || (uint64_t)other[i] >= (uint64_t)N) {
-    *flag = 1;
+  const int64_t d = dst[i], s = src[i];
+  if ((uint64_t)d >= (uint64_t)N || (uint64_t)s >= (uint64_t)N) {
+    atomicOr(flag, kFlagEdges);
+    if (N > 0) atomicAdd(&cnt_src[0], 1);
     return;
   }
-  atomicAdd(&counts[k], 1);
-}
-// keys written by rank_dst_kernel, or the 0 a slot without a valid edge was cleared to: in range
-// by construction (the test keeps a broken invariant from becoming a wild access)
-__global__ void count32_kernel(int64_t E, int64_t N, const int32_t *__restrict__ key,
-                               int32_t *counts) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < E && (uint32_t)key[i] < (uint64_t)N) atomicAdd(&counts[key[i]], 1);
+  atomicAdd(&cnt_dst[d], 1);
+  atomicAdd(&cnt_src[s], 1);
 }
 
-// exclusive scan of n ints in three steps: per-block scan, scan of block totals, add back
-__global__ void scan_block_kernel(int64_t n, const int32_t *__restrict__ in, int32_t *out,
-                                  int32_t *block_sums) {
-  __shared__ int32_t s[kScanBlock];
-  const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
-  s[threadIdx.x] = i < n ? in[i] : 0;
+// Exclusive scan of the two counter arrays (blockIdx.y), in place, the offsets also going to
+// row_ptr / row_ptr_src with the total behind them: the counters become the fill cursors of the
+// buckets.  One block walks a whole array up to kScanOneBlock counters; beyond that each block takes
+// kScanSpan of them and adds up the totals of the blocks before it (written by scan_totals_kernel).
+struct ScanArgs {
+  int32_t *cnt[2], *ptr[2];
+  int32_t *totals;                       // [2][gridDim.x], multi-block scans only
+};
+__device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t *warp_sums, int32_t &total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int32_t inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) warp_sums[warp] = inc;
   __syncthreads();
-  for (int off = 1; off < kScanBlock; off <<= 1) {
-    const int32_t v = threadIdx.x >= off ? s[threadIdx.x - off] : 0;
-    __syncthreads();
-    s[threadIdx.x] += v;
-    __syncthreads();
-  }
-  if (i < n) out[i] = s[threadIdx.x] - in[i];          // exclusive
-  if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = s[threadIdx.x];
-}
-// block_sums [nb + 1]: exclusive prefix of the block totals, the grand total in slot nb
-__global__ void scan_sums_kernel(int64_t nb, int32_t *block_sums) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int32_t run = 0;
-    for (int64_t b = 0; b < nb; ++b) {
-      const int32_t v = block_sums[b];
-      block_sums[b] = run;
-      run += v;
+  if (warp == 0) {
+    int32_t w = warp_sums[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int32_t u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
     }
-    block_sums[nb] = run;
+    warp_sums[lane] = w;
   }
+  __syncthreads();
+  total = warp_sums[31];
+  const int32_t before = warp ? warp_sums[warp - 1] : 0;
+  __syncthreads();
+  return before + inc - v;
 }
-// out[n] = the number of elements COUNTED (edges that were left out for an invalid node index are
-// not among them), so that no offset range ever covers a slot nothing was written to
-__global__ void scan_add_kernel(int64_t n, int64_t nb, int32_t *out,
-                                const int32_t *__restrict__ block_sums) {
-  const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
-  if (i < n) out[i] += block_sums[blockIdx.x];
-  if (i == n) out[n] = block_sums[nb];
+__global__ void __launch_bounds__(kScanThreads) scan_totals_kernel(int64_t n, const ScanArgs a) {
+  __shared__ int32_t sums[32];
+  const int32_t *cnt = a.cnt[blockIdx.y];
+  const int64_t base = (int64_t)blockIdx.x * kScanSpan + threadIdx.x * kScanItems;
+  int32_t v = 0, total;
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) v += base + k < n ? cnt[base + k] : 0;
+  block_exclusive_scan(v, sums, total);
+  if (threadIdx.x == 0) a.totals[blockIdx.y * gridDim.x + blockIdx.x] = total;
+}
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(int64_t n, const ScanArgs a) {
+  __shared__ int32_t sums[32];
+  int32_t *cnt = a.cnt[blockIdx.y], *ptr = a.ptr[blockIdx.y];
+  int64_t lo = 0, hi = n;
+  int32_t carry = 0, total;
+  if (gridDim.x > 1) {
+    lo = (int64_t)blockIdx.x * kScanSpan;
+    hi = min(n, lo + kScanSpan);
+    for (int b0 = 0; b0 < (int)blockIdx.x; b0 += kScanThreads) {     // totals of the blocks before
+      const int b = b0 + threadIdx.x;
+      block_exclusive_scan(b < (int)blockIdx.x ? a.totals[blockIdx.y * gridDim.x + b] : 0, sums, total);
+      carry += total;
+    }
+  }
+  for (int64_t s0 = lo; s0 < hi || s0 == lo; s0 += kScanSpan) {
+    const int64_t base = s0 + threadIdx.x * kScanItems;
+    int32_t v[kScanItems], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      v[k] = base + k < hi ? cnt[base + k] : 0;
+      sum += v[k];
+    }
+    int32_t run = carry + block_exclusive_scan(sum, sums, total);
+#pragma unroll
+    for (int k = 0; k < kScanItems; ++k) {
+      if (base + k < hi) {
+        ptr[base + k] = run;
+        cnt[base + k] = run;
+      }
+      run += v[k];
+    }
+    carry += total;
+  }
+  // ptr[n] = the number of elements COUNTED (edges left out for an invalid node index are not among
+  // them), so that no offset range ever covers a slot nothing was written to
+  if (hi == n && threadIdx.x == 0) ptr[n] = carry;
 }
 
-__global__ void bucket_kernel(int64_t E, int64_t N, const int64_t *__restrict__ key,
-                              const int64_t *__restrict__ other,
-                              const int32_t *__restrict__ row_ptr, int32_t *cursor,
-                              int32_t *tmp) {
+__global__ void bucket_kernel(int64_t E, int64_t N, const int64_t *__restrict__ src,
+                              const int64_t *__restrict__ dst, int32_t *cursor, int32_t *tmp) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= E) return;
-  const int64_t k = key[i];
-  if ((uint64_t)k >= (uint64_t)N || (uint64_t)other[i] >= (uint64_t)N) return;   // flagged above
-  tmp[row_ptr[k] + atomicAdd(&cursor[k], 1)] = (int32_t)i;
+  const int64_t k = dst[i];
+  if ((uint64_t)k >= (uint64_t)N || (uint64_t)src[i] >= (uint64_t)N) return;   // flagged above
+  tmp[atomicAdd(&cursor[k], 1)] = (int32_t)i;
 }
-__global__ void bucket32_kernel(int64_t E, int64_t N, const int32_t *__restrict__ key,
-                                const int32_t *__restrict__ row_ptr, int32_t *cursor,
-                                int32_t *tmp) {
+__global__ void bucket_src_kernel(int64_t E, int64_t N, const int32_t *__restrict__ key,
+                                  int32_t *cursor, int32_t *tmp) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= E) return;
   const int32_t k = key[i];
   if ((uint32_t)k >= (uint64_t)N) return;
-  tmp[row_ptr[k] + atomicAdd(&cursor[k], 1)] = (int32_t)i;
+  tmp[atomicAdd(&cursor[k], 1)] = (int32_t)i;
 }
 
-// One warp per destination node: order its edges by (src, original position).
+// Order of the keys of one bucket, a warp per node.  Keys are unique, so the place of a key is the
+// number of smaller ones.  A bucket of up to 64 edges (two per lane) is ranked from registers by
+// shuffles; a larger one reads the bucket again for every key.
+template <typename Load>
+__device__ __forceinline__ void rank_bucket(int beg, int end, int lane, Load load,
+                                            unsigned long long (&key)[2], int (&rank)[2]) {
+  const unsigned long long last = ~0ull;
+  const int n = end - beg;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    key[q] = lane + 32 * q < n ? load(beg + lane + 32 * q) : last;
+    rank[q] = 0;
+  }
+  const int m0 = min(n, 32), m1 = n - m0;
+  for (int j = 0; j < m0; ++j) {
+    const unsigned long long o = __shfl_sync(0xffffffffu, key[0], j);
+    rank[0] += o < key[0];
+    rank[1] += o < key[1];
+  }
+  for (int j = 0; j < m1; ++j) {
+    const unsigned long long o = __shfl_sync(0xffffffffu, key[1], j);
+    rank[0] += o < key[0];
+    rank[1] += o < key[1];
+  }
+}
+
+// One warp per destination node: order its edges by (src, original position).  The slots past the
+// kept edges read as an edge 0 -> 0 at position 0: a caller that launches per-edge kernels over all
+// E slots without looking at the flag (a recorded graph replay) still indexes inside its arrays.
 __global__ void rank_dst_kernel(int64_t N, int64_t E, const int64_t *__restrict__ src64,
                                 const int32_t *__restrict__ row_ptr,
                                 const int32_t *__restrict__ tmp, int32_t *perm,
                                 int32_t *src_sorted, int32_t *dst_sorted) {
-  const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = row_ptr[N] + tid; i < E; i += (int64_t)gridDim.x * blockDim.x)
+    perm[i] = src_sorted[i] = dst_sorted[i] = 0;
+  const int64_t n = tid / 32;
   const int lane = threadIdx.x % 32;
   if (n >= N) return;
   const int beg = row_ptr[n], end = row_ptr[n + 1];
-  for (int i = beg + lane; i < end; i += 32) {
-    // every slot of a bucket was filled by bucket_kernel with an edge id; the range test only
-    // keeps a broken invariant from turning into a wild read
+  // every slot of a bucket was filled by bucket_kernel with an edge id; the range test only keeps
+  // a broken invariant from turning into a wild read
+  auto load = [&](int i) -> unsigned long long {
     const int32_t id = tmp[i];
-    if ((uint32_t)id >= (uint64_t)E) continue;
-    const int64_t s = src64[id];
-    int rank = 0;
-    for (int j = beg; j < end; ++j) {
-      const int32_t jd = tmp[j];
-      if ((uint32_t)jd >= (uint64_t)E) continue;
-      const int64_t sj = src64[jd];
-      rank += (sj < s) || (sj == s && jd < id);
-    }
-    perm[beg + rank] = id;
-    src_sorted[beg + rank] = (int32_t)s;
+    if ((uint32_t)id >= (uint64_t)E) return ~0ull;
+    return ((unsigned long long)src64[id] << 32) | (uint32_t)id;
+  };
+  auto put = [&](unsigned long long key, int rank) {
+    if (key == ~0ull) return;
+    perm[beg + rank] = (int32_t)(uint32_t)key;
+    src_sorted[beg + rank] = (int32_t)(key >> 32);
     dst_sorted[beg + rank] = (int32_t)n;
+  };
+  if (end - beg <= 64) {
+    unsigned long long key[2];
+    int rank[2];
+    rank_bucket(beg, end, lane, load, key, rank);
+    put(key[0], rank[0]);
+    put(key[1], rank[1]);
+    return;
+  }
+  for (int i = beg + lane; i < end; i += 32) {
+    const unsigned long long key = load(i);
+    int rank = 0;
+    for (int j = beg; j < end; ++j) rank += load(j) < key;
+    put(key, rank);
   }
 }
 
 // One warp per source node: order the sorted-edge ids of its outgoing edges increasingly.
-__global__ void rank_src_kernel(int64_t N, const int32_t *__restrict__ row_ptr_src,
+__global__ void rank_src_kernel(int64_t N, int64_t E, const int32_t *__restrict__ row_ptr_src,
                                 const int32_t *__restrict__ tmp, int32_t *perm_src) {
-  const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  for (int64_t i = row_ptr_src[N] + tid; i < E; i += (int64_t)gridDim.x * blockDim.x) perm_src[i] = 0;
+  const int64_t n = tid / 32;
   const int lane = threadIdx.x % 32;
   if (n >= N) return;
   const int beg = row_ptr_src[n], end = row_ptr_src[n + 1];
+  auto load = [&](int i) -> unsigned long long { return (uint32_t)tmp[i]; };
+  if (end - beg <= 64) {
+    unsigned long long key[2];
+    int rank[2];
+    rank_bucket(beg, end, lane, load, key, rank);
+#pragma unroll
+    for (int q = 0; q < 2; ++q)
+      if (key[q] != ~0ull) perm_src[beg + rank[q]] = (int32_t)key[q];
+    return;
+  }
   for (int i = beg + lane; i < end; i += 32) {
     const int32_t id = tmp[i];
     int rank = 0;
     for (int j = beg; j < end; ++j) rank += tmp[j] < id;
-    perm_src[beg + rank] = id;          // ids are positions 0 .. E-1 written by bucket32_kernel
+    perm_src[beg + rank] = id;          // ids are positions 0 .. E-1 written by bucket_src_kernel
   }
 }
 
 struct CsrWork {
-  int32_t *flag, *counts, *cursor, *tmp, *block_sums;
+  int32_t *flag, *cnt_dst, *cnt_src, *tmp, *totals;   // flag and counters stand side by side
   size_t bytes;
 };
 
@@ -153,24 +251,12 @@ CsrWork carve_csr(int64_t E, int64_t N, void *base) {
     return p;
   };
   w.flag = take(1);
-  w.counts = take((size_t)N + 1);
-  w.cursor = take((size_t)N + 1);
+  w.cnt_dst = take((size_t)N + 1);
+  w.cnt_src = take((size_t)N + 1);
   w.tmp = take((size_t)(E > 0 ? E : 1));
-  w.block_sums = take((size_t)zp_ceil_div(N + 1, kScanBlock) + 1);
+  w.totals = take((size_t)zp_ceil_div(N + 1, 1024) + 1);   // >= two per kScanSpan counters
   w.bytes = off;
   return w;
-}
-
-int exclusive_scan(int64_t n, const int32_t *in, int32_t *out, int32_t *block_sums,
-                   cudaStream_t st) {
-  const int64_t nb = zp_ceil_div(n + 1, kScanBlock);
-  scan_block_kernel<<<(unsigned)nb, kScanBlock, 0, st>>>(n, in, out, block_sums);
-  ZP_LAUNCH_CHECK("scan_block_kernel");
-  scan_sums_kernel<<<1, 32, 0, st>>>(nb, block_sums);
-  ZP_LAUNCH_CHECK("scan_sums_kernel");
-  scan_add_kernel<<<(unsigned)nb, kScanBlock, 0, st>>>(n, nb, out, block_sums);
-  ZP_LAUNCH_CHECK("scan_add_kernel");
-  return ZP_OK;
 }
 
 }  // namespace
@@ -182,60 +268,68 @@ size_t zp_csr_work_bytes(int64_t n_edges, int64_t n_nodes) {
   return carve_csr(n_edges, n_nodes, nullptr).bytes;
 }
 
-int zp_csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *perm,
-                 int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr, int32_t *perm_src,
-                 int32_t *row_ptr_src, void *work, size_t work_bytes, void *stream) {
+static int csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *perm,
+                     int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr, int32_t *perm_src,
+                     int32_t *row_ptr_src, const int64_t *atomic_numbers, int n_elements,
+                     void *work, size_t work_bytes, cudaStream_t st) {
   if (E < 0 || N < 0 || E > INT32_MAX || N >= INT32_MAX) return ZP_ERR_INVALID_ARG;
   if (!row_ptr || !row_ptr_src || !work) return ZP_ERR_INVALID_ARG;
   if (E && (!edge_index || !perm || !src_sorted || !dst_sorted || !perm_src))
     return ZP_ERR_INVALID_ARG;
   const CsrWork w = carve_csr(E, N, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
-  cudaStream_t st = (cudaStream_t)stream;
   const int64_t *src64 = edge_index, *dst64 = edge_index + E;
   const unsigned eb = (unsigned)zp_ceil_div(E > 0 ? E : 1, 256);
   const unsigned nbw = (unsigned)zp_ceil_div((N > 0 ? N : 1) * 32, 256);
-  int rc;
 
-  // destination view
-  ZP_CUDA(cudaMemsetAsync(w.flag, 0, sizeof(int32_t), st));
-  if (E) {
-    // The slots an invalid edge leaves empty (the last ones, past row_ptr[N]) read as edges
-    // 0 -> 0 at position 0: a caller that launches per-edge kernels over all E slots without
-    // looking at the flag (a recorded graph replay) still indexes inside its arrays.
-    ZP_CUDA(cudaMemsetAsync(src_sorted, 0, sizeof(int32_t) * E, st));
-    ZP_CUDA(cudaMemsetAsync(dst_sorted, 0, sizeof(int32_t) * E, st));
-    ZP_CUDA(cudaMemsetAsync(perm, 0, sizeof(int32_t) * E, st));
-    ZP_CUDA(cudaMemsetAsync(perm_src, 0, sizeof(int32_t) * E, st));
-  }
-  ZP_CUDA(cudaMemsetAsync(w.counts, 0, sizeof(int32_t) * (N + 1), st));
-  ZP_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (N + 1), st));
-  if (E) {
-    count_kernel<<<eb, 256, 0, st>>>(E, N, dst64, src64, w.counts, w.flag);
+  ZP_CUDA(cudaMemsetAsync(w.flag, 0, (char *)w.tmp - (char *)w.flag, st));
+  if (E || atomic_numbers) {
+    const int64_t items = atomic_numbers && N > E ? N : E;
+    count_kernel<<<(unsigned)zp_ceil_div(items > 0 ? items : 1, 256), 256, 0, st>>>(
+        E, N, src64, dst64, atomic_numbers, n_elements, w.cnt_dst, w.cnt_src, w.flag);
     ZP_LAUNCH_CHECK("count_kernel");
   }
-  if ((rc = exclusive_scan(N, w.counts, row_ptr, w.block_sums, st))) return rc;
+  const ScanArgs a{{w.cnt_dst, w.cnt_src}, {row_ptr, row_ptr_src}, w.totals};
+  const unsigned sb = N <= kScanOneBlock ? 1u : (unsigned)zp_ceil_div(N, kScanSpan);
+  if (sb > 1) {
+    scan_totals_kernel<<<dim3(sb, 2), kScanThreads, 0, st>>>(N, a);
+    ZP_LAUNCH_CHECK("scan_totals_kernel");
+  }
+  scan_kernel<<<dim3(sb, 2), kScanThreads, 0, st>>>(N, a);
+  ZP_LAUNCH_CHECK("scan_kernel");
   if (E) {
-    bucket_kernel<<<eb, 256, 0, st>>>(E, N, dst64, src64, row_ptr, w.cursor, w.tmp);
+    bucket_kernel<<<eb, 256, 0, st>>>(E, N, src64, dst64, w.cnt_dst, w.tmp);
     ZP_LAUNCH_CHECK("bucket_kernel");
     rank_dst_kernel<<<nbw, 256, 0, st>>>(N, E, src64, row_ptr, w.tmp, perm, src_sorted, dst_sorted);
     ZP_LAUNCH_CHECK("rank_dst_kernel");
-  }
-
-  // source view over sorted-edge ids
-  ZP_CUDA(cudaMemsetAsync(w.counts, 0, sizeof(int32_t) * (N + 1), st));
-  ZP_CUDA(cudaMemsetAsync(w.cursor, 0, sizeof(int32_t) * (N + 1), st));
-  if (E) {
-    count32_kernel<<<eb, 256, 0, st>>>(E, N, src_sorted, w.counts);
-    ZP_LAUNCH_CHECK("count32_kernel");
-  }
-  if ((rc = exclusive_scan(N, w.counts, row_ptr_src, w.block_sums, st))) return rc;
-  if (E) {
-    bucket32_kernel<<<eb, 256, 0, st>>>(E, N, src_sorted, row_ptr_src, w.cursor, w.tmp);
-    ZP_LAUNCH_CHECK("bucket32_kernel");
-    rank_src_kernel<<<nbw, 256, 0, st>>>(N, row_ptr_src, w.tmp, perm_src);
+    // source view over sorted-edge ids
+    bucket_src_kernel<<<eb, 256, 0, st>>>(E, N, src_sorted, w.cnt_src, w.tmp);
+    ZP_LAUNCH_CHECK("bucket_src_kernel");
+    rank_src_kernel<<<nbw, 256, 0, st>>>(N, E, row_ptr_src, w.tmp, perm_src);
     ZP_LAUNCH_CHECK("rank_src_kernel");
   }
+  return ZP_OK;
+}
+
+int zp_csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *perm,
+                 int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr, int32_t *perm_src,
+                 int32_t *row_ptr_src, void *work, size_t work_bytes, void *stream) {
+  return csr_build(edge_index, E, N, perm, src_sorted, dst_sorted, row_ptr, perm_src, row_ptr_src,
+                   nullptr, 0, work, work_bytes, (cudaStream_t)stream);
+}
+
+int zp_csr_build_checked(const int64_t *edge_index, int64_t E, int64_t N,
+                         const int64_t *atomic_numbers, int n_elements, int32_t *perm,
+                         int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr,
+                         int32_t *perm_src, int32_t *row_ptr_src, int32_t *flags_host, void *work,
+                         size_t work_bytes, void *stream) {
+  if (!flags_host || (N && !atomic_numbers)) return ZP_ERR_INVALID_ARG;
+  const int rc = csr_build(edge_index, E, N, perm, src_sorted, dst_sorted, row_ptr, perm_src,
+                           row_ptr_src, atomic_numbers, n_elements, work, work_bytes,
+                           (cudaStream_t)stream);
+  if (rc) return rc;
+  ZP_CUDA(cudaMemcpyAsync(flags_host, carve_csr(E, N, work).flag, sizeof(int32_t),
+                          cudaMemcpyDeviceToHost, (cudaStream_t)stream));
   return ZP_OK;
 }
 

@@ -99,16 +99,9 @@ class EdgeGraph:
         ``IndexError`` if a node index lies outside ``[0, n_nodes)``, as indexing with it raises in
         the reference.  Skipped while the stream is being captured into a CUDA graph (no
         synchronisation is possible there; the kernels leave such edges out either way)."""
-        if not edge_index.is_cuda:
-            raise RuntimeError("EdgeGraph.build needs a CUDA edge_index; there is no CPU path")
-        lib = _lib.load()
-        ei = edge_index.to(torch.int64).contiguous()
-        e, dev = ei.shape[1], ei.device
-        i32 = dict(dtype=torch.int32, device=dev)
-        perm, src, dst, perm_src = (torch.empty(max(e, 1), **i32) for _ in range(4))
-        row_ptr, row_ptr_src = (torch.empty(n_nodes + 1, **i32) for _ in range(2))
-        nbytes = lib.zp_csr_work_bytes(e, n_nodes)
-        work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+        lib, ei, e, dev = EdgeGraph._open(edge_index)
+        perm, src, dst, perm_src, row_ptr, row_ptr_src, work = EdgeGraph._arrays(lib, e, n_nodes, dev)
+        nbytes = work.numel()
         with torch.cuda.device(dev):
             st = torch.cuda.current_stream().cuda_stream
             _lib.check(lib.zp_csr_build(ei.data_ptr(), e, n_nodes, perm.data_ptr(), src.data_ptr(),
@@ -122,6 +115,61 @@ class EdgeGraph:
                 if flag.value:
                     raise IndexError(f"edge_index names a node outside [0, {n_nodes})")
         return EdgeGraph(n_nodes, e, perm[:e], src[:e], dst[:e], row_ptr, perm_src[:e], row_ptr_src)
+
+    @staticmethod
+    def _open(edge_index: torch.Tensor):
+        if not edge_index.is_cuda:
+            raise RuntimeError("EdgeGraph.build needs a CUDA edge_index; there is no CPU path")
+        ei = edge_index.to(torch.int64).contiguous()
+        return _lib.load(), ei, ei.shape[1], ei.device
+
+    @staticmethod
+    def _arrays(lib, e: int, n_nodes: int, dev):
+        i32 = dict(dtype=torch.int32, device=dev)
+        edges = [torch.empty(max(e, 1), **i32) for _ in range(4)]
+        work = torch.empty(lib.zp_csr_work_bytes(e, n_nodes), dtype=torch.uint8, device=dev)
+        return (*edges, torch.empty(n_nodes + 1, **i32), torch.empty(n_nodes + 1, **i32), work)
+
+    @staticmethod
+    def build_checked(edge_index: torch.Tensor, atomic_numbers: torch.Tensor, n_elements: int):
+        """``build`` for a caller that goes on enqueueing work: returns ``(graph, check)``, and
+        ``check()`` raises ``IndexError`` for a node index outside ``[0, N)`` or an element number
+        outside ``[0, n_elements)``.  It waits for the sort alone, so work enqueued in between keeps
+        the device busy.  Not for use while the stream is being captured."""
+        lib, ei, e, dev = EdgeGraph._open(edge_index)
+        z = atomic_numbers.to(torch.int64).contiguous()
+        n = z.shape[0]
+        perm, src, dst, perm_src, row_ptr, row_ptr_src, work = EdgeGraph._arrays(lib, e, n, dev)
+        slots = _flag_slots.setdefault(dev.index, [])
+        try:
+            flags, done = slots.pop()
+        except IndexError:
+            flags, done = torch.empty(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
+        with torch.cuda.device(dev):
+            stream = torch.cuda.current_stream()
+            _lib.check(lib.zp_csr_build_checked(
+                ei.data_ptr(), e, n, z.data_ptr(), n_elements, perm.data_ptr(), src.data_ptr(),
+                dst.data_ptr(), row_ptr.data_ptr(), perm_src.data_ptr(), row_ptr_src.data_ptr(),
+                flags.data_ptr(), work.data_ptr(), work.numel(), stream.cuda_stream),
+                "zp_csr_build_checked")
+            done.record(stream)
+
+        def check() -> None:
+            done.synchronize()
+            bits = int(flags[0])
+            if len(slots) < 8:
+                slots.append((flags, done))
+            if bits & 1:
+                raise IndexError(f"edge_index names a node outside [0, {n})")
+            if bits & 2:
+                raise IndexError(f"atomic_numbers outside [0, {n_elements})")
+
+        return EdgeGraph(n, e, perm[:e], src[:e], dst[:e], row_ptr, perm_src[:e], row_ptr_src), check
+
+
+#: Per device, page-locked words (and the events behind them) that the flags of a sort arrive in,
+#: reused; at most eight are kept, and a slot belongs to one call from its pop to its append.
+_flag_slots: dict = {}
 
 
 @dataclasses.dataclass
