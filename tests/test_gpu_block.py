@@ -78,3 +78,40 @@ def test_bad_input_raises(what):
         case["atomic_numbers"][5] = block.cfg.max_num_elements
     with pytest.raises(IndexError):
         gpu_node_out_and_vjp(block, case, case["upstream"])
+
+
+@pytest.mark.parametrize("lmax,mmax,c,h", [(6, 3, 8, 8), (6, 6, 16, 8), (5, 4, 40, 8), (1, 0, 136, 8),
+                                           (4, 4, 256, 8)])
+def test_rotations_over_degrees_orders_and_widths(lmax, mmax, c, h, jd64):
+    """Row walks, packed sums and torques of the per-edge kernels from two degrees to seven, orders
+    up to the degree, and widths that leave a block's last warp partly idle."""
+    cfg = dict(lmax=lmax, mmax=mmax, sphere_channels=c, hidden_channels=h, edge_channels=8,
+               num_distance_basis=6, cutoff=5.0)
+    params = orc.init_params(cfg, seed=lmax)
+    case = random_case(cfg, 7, 45, seed=mmax)
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    check_against(*gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"]), *want)
+
+
+def test_edges_along_the_polar_axis(jd64):
+    """An edge whose direction is the polar axis has no proper rotation; its gradient follows the
+    construction of the matrices (clamped, large) and must not disturb the other edges."""
+    cfg = dict(lmax=3, mmax=2, sphere_channels=16, hidden_channels=8, edge_channels=8,
+               num_distance_basis=6, cutoff=8.0)
+    params = orc.init_params(cfg, seed=5)
+    case = random_case(cfg, 12, 60, seed=6)
+    case["pos"] = case["pos"].float().double()
+    case["shifts"] = torch.zeros_like(case["shifts"])
+    for e, sign in ((0, 1.0), (31, -1.0), (40, 1.0)):      # atoms that only these edges touch
+        i, j = 2 * (e % 3), 2 * (e % 3) + 1
+        case["edge_index"][:, e] = torch.tensor([i, j])
+        case["pos"][j] = case["pos"][i] + torch.tensor([0.0, sign * 1.5, 0.0])
+    for k in range(60):
+        if k not in (0, 31, 40):
+            case["edge_index"][:, k] = 6 + case["edge_index"][:, k] % 6
+            if case["edge_index"][0, k] == case["edge_index"][1, k]:
+                case["edge_index"][0, k] = 6 + (case["edge_index"][0, k] - 5) % 6
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    got = gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"])
+    assert rel_l2(got[0], want[0]) < 1e-5
+    assert rel_l2(got[2][6:], want[2][6:]) < 1e-5 and rel_l2(got[2][:6], want[2][:6]) < 1e-3

@@ -1,5 +1,6 @@
 // C ABI of zippel_b200: plan/tables, workspace carving, and the forward / backward drivers
 // that sequence the kernels on the caller's stream.
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -101,7 +102,7 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
   const size_t e = (size_t)E;
   const bool lean = mode == 2 && can_fuse(p, 0) && can_fuse(p, 1);
   w.scales = c.floats(kScCount);
-  w.rot = c.floats(e * t.nnz_pad);
+  w.rot = c.floats(e * t.rot_ld);
   w.a1 = c.planes(E, (int64_t)t.Km * 2 * t.C, f, w.scales + kScA1);
   w.ld_h1 = lean ? t.n_gate : t.w1_cols;
   w.h1 = c.floats(e * w.ld_h1);
@@ -129,7 +130,7 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
     w.dh1 = c.planes(E, t.w1_cols, f, w.scales + kScDh1);
     w.da1 = c.floats(e * t.Km * 2 * t.C);
     w.du_src = c.floats(e * 2 * t.K * t.C);
-    w.grot = c.floats(e * t.nnz_pad);
+    w.torque = c.floats(e * 4);
     w.wgrad = c.floats((size_t)kZpWgradSplits * p->g_elems);
     const size_t parts = (size_t)zp_ceil_div(E > 0 ? E : 1, kZpColRows);
     w.col1 = c.floats(parts * p->c1_out[0]);
@@ -215,6 +216,26 @@ int zp_plan_create(const zp_config *cfg, const double *jd_host, zp_plan **plan_o
   t.nnz = off;
   t.nnz_pad = (off + 3) / 4 * 4;
   t.R = rad;
+  t.rad_rows = (int16_t)(rad / (2 * C));
+  int po = 0, rows = 0, rads = 0;
+  for (int l = 0; l <= L; ++l) {
+    const int mm = MM < l ? MM : l, width = 2 * l + 2;
+    t.deg_rot[l] = (int16_t)po;
+    t.deg_row[l] = (int16_t)rows;
+    t.deg_rad[l] = (int16_t)rads;
+    for (int i = 0; i < 2 * l + 1; ++i) {
+      const int m = i - l, am = m < 0 ? -m : m, place = m > 0 ? 2 * m - 1 : 2 * am;
+      if (am <= mm) t.row_off[t.row_of[l][i]] = (int16_t)(po + place * width);
+      else if (am == MM + 1) t.ext_off[l][m > 0 ? 0 : 1] = (int16_t)(po + place * width);
+    }
+    po += (2 * mm + 1 + (l > MM ? 2 : 0)) * width;
+    rows += 2 * mm + 1;
+    rads += mm + 1;
+  }
+  t.rot_ld = (int16_t)((po + 3) / 4 * 4);
+  for (int l = 0; l <= L; ++l)
+    for (int m = 0; m < l; ++m)
+      t.couple[l][m] = (float)(m == 0 ? std::sqrt(0.5 * l * (l + 1)) : 0.5 * std::sqrt((double)(l - m) * (l + m + 1)));
   t.n_gate = L * H;
   t.w1_cols = t.n_gate + t.Km * H;
   for (int l = 0; l <= L; ++l) {
@@ -388,7 +409,7 @@ int zp_wigner_forward(const zp_plan *plan, int64_t n_edges, const float *edge_ve
                       const float *cos_g, const float *sin_g, float *rot, void *stream) {
   if (!plan || n_edges < 0) return ZP_ERR_INVALID_ARG;
   if (n_edges && (!edge_vec || !cos_g || !sin_g || !rot)) return ZP_ERR_INVALID_ARG;
-  return zp_launch_wigner_fwd(plan, n_edges, edge_vec, cos_g, sin_g, rot, (cudaStream_t)stream);
+  return zp_launch_wigner_fwd(plan, n_edges, edge_vec, cos_g, sin_g, rot, 1, (cudaStream_t)stream);
 }
 
 int zp_wigner_backward(const zp_plan *plan, int64_t n_edges, const float *edge_vec,
@@ -437,7 +458,7 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
   const bool fuse1 = can_fuse(plan, 0), fuse2 = can_fuse(plan, 1);
   const bool lean = !keep && fuse1 && fuse2;          // h1 rows and y are never written
   ZP_TIMED(ZP_K_WIGNER_FWD,
-           zp_launch_wigner_fwd(plan, c.E, c.edge_vec, c.cos_g, c.sin_g, ws.rot, st));
+           zp_launch_wigner_fwd(plan, c.E, c.edge_vec, c.cos_g, c.sin_g, ws.rot, 0, st));
   // |rot row . x| <= sqrt(2l+1) max|x|, over the rows the edges name
   ZP_TIMED(ZP_K_ROTATE_IN,
            zp_launch_rotate_in(plan, c.E, c.x_node, c.src, c.dst, ws.rot, c.radial, ws.a1,
@@ -453,6 +474,7 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
   std::memset(&epi, 0, sizeof(epi));
   std::memcpy(epi.row_l, t.row_l, sizeof(epi.row_l));
   std::memcpy(epi.rot_off, t.rot_off, sizeof(epi.rot_off));
+  std::memcpy(epi.row_off, t.row_off, sizeof(epi.row_off));
 
   // ---- conv1 (+ gate) ----
   if (fuse1 && E > 0) {
@@ -527,7 +549,7 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
     epi.row_ptr = c.row_ptr;
     epi.n_nodes = (int)N;
     epi.nnz = t.nnz;
-    epi.nnz_pad = t.nnz_pad;
+    epi.rot_ld = t.rot_ld;
     epi.head = ws.head;
     epi.cont = ws.cont;
     epi.block_node = ws.block_node;
@@ -679,7 +701,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   ZP_TIMED(ZP_K_ROTATE_GRAD_OUT,
            zp_launch_rotate_grad_out(plan, E, grad_node_out, ws.y, c.env, ws.rot, c.dst, ws.dy,
                                      zp_scale_of(3.7f, ws.scales + kScG, ws.scales + kScDy), grad_env,
-                                     ws.grot, st));
+                                     ws.torque, st));
   // One conv at a time: input gradient dX = dY W_fold (K-major against the transposed planes),
   // weight gradient dW_fold = dY^T X with both operands MN-major (the contraction runs over
   // edges), bias gradient = column sums of dY.
@@ -745,7 +767,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   // VJP; their scale comes from |grad_radial| <= 2 max|da1| max|rot . x| <= 2 * 3.7 max|da1| max|x|
   ZP_TIMED(ZP_K_ROTATE_IN_BWD,
            zp_launch_rotate_in_bwd(plan, E, ws.da1, radial, c.x_node, c.src, c.dst, ws.rot,
-                                   rl ? nullptr : grad_radial, du_out, ws.grot, st,
+                                   rl ? nullptr : grad_radial, du_out, ws.torque, st,
                                    rl ? &ws.gr : nullptr,
                                    zp_scale_of(7.4f, ws.scales + kScDa1, ws.scales + kScGrScale,
                                                ws.scales + kScX)));
@@ -763,7 +785,10 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
              zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
                                    grad_x_node, st));
   ZP_TIMED(ZP_K_WIGNER_BWD,
-           zp_launch_wigner_bwd(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.grot, grad_edge_vec, st));
+           zp_launch_edge_vec_grad(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.torque,
+                                   ZpTorqueArgs{ws.da1, radial, c.x_node, ws.y, grad_node_out, c.env,
+                                                ws.rot, c.src, c.dst},
+                                   grad_edge_vec, st));
   if (want_w)
     zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
   return ZP_OK;

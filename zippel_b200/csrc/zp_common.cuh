@@ -30,7 +30,22 @@ struct ZpTables {
   int16_t m_row0[ZP_MAX_L + 1];                 // first m' row of m-block m
   int16_t m_rows[ZP_MAX_L + 1];                 // rows in m-block m (km or 2 km)
   int32_t rad_off[ZP_MAX_L + 1];                // first radial column of m-block m
+  int16_t rad_rows;                             // R / 2C
   int16_t jd_off[ZP_MAX_L + 1];                 // offset of J_l in the packed J array
+  // Rotation as the kernels keep it between themselves (rot_ld entries per edge): degree by degree,
+  // within a degree the rows m = 0, +1, -1, +2, -2, .. up to mmax and, for l > mmax, the two rows
+  // +-(mmax + 1) the VJP needs besides (see zp_rotate_bwd.cu); every row padded to an even number of
+  // entries (two weights per 16-byte load once duplicated in shared memory).  A walk through a degree's
+  // rows is then a fixed step in all the per-edge arrays in shared memory, which have the same order.
+  int16_t deg_rot[ZP_MAX_L + 1];                // first entry of a degree
+  int16_t deg_row[ZP_MAX_L + 1];                // rows |m| <= mmax of the degrees before it
+  int16_t deg_rad[ZP_MAX_L + 1];                // ... radial gains (l, |m|)
+  int16_t row_off[ZP_MAX_KM];                   // entry offset by m'-major row
+  int16_t ext_off[ZP_MAX_L + 1][2];
+  int16_t rot_ld;
+  // generators of rotations about the axes perpendicular to the edge couple m and m + 1 of one
+  // degree with these coefficients
+  float couple[ZP_MAX_L + 1][ZP_MAX_L + 1];
 };
 
 struct ZpTimer;
@@ -166,10 +181,23 @@ static inline size_t zp_align_up(size_t x, size_t a) { return (x + a - 1) / a * 
   }
 
 // ---- kernels (each in its own translation unit) --------------------------------------------
+// rot in the packed layout [E, nnz_pad] (packed != 0) or in the kernels' own [E, rot_ld]
 int zp_launch_wigner_fwd(const zp_plan *p, int64_t E, const float *ev, const float *cg,
-                         const float *sg, float *rot, cudaStream_t st);
+                         const float *sg, float *rot, int packed, cudaStream_t st);
 int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const float *cg,
                          const float *sg, const float *grot, float *gev, cudaStream_t st);
+
+// The arrays of one edge convolution's VJP that an edge's rotation gradient comes from.
+// torque [E, 4]: for each edge the derivative of the loss under a rotation of the edge frame about
+// its own axis (entry 0) and the two axes perpendicular to it (1, 2).
+struct ZpTorqueArgs {
+  const float *da1, *radial, *x, *y, *g_out, *env, *rot;
+  const int32_t *src, *dst;
+};
+// torque -> gradient of the edge vectors
+int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const float *cg,
+                            const float *sg, const float *torque, const ZpTorqueArgs &a, float *gev,
+                            cudaStream_t st);
 
 int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32_t *src,
                         const int32_t *dst, const float *rot, const float *radial,
@@ -180,12 +208,12 @@ int zp_launch_rotate_back_scatter(const zp_plan *p, int64_t N, const float *y, c
 int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const float *y,
                               const float *env, const float *rot, const int32_t *dst,
                               const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
-                              float *grad_rot, cudaStream_t st);
+                              float *torque, cudaStream_t st);
 // du_both [E][2][K][C]: per-edge contributions to grad_x of the source (0) and destination (1)
 // grad_radial goes out as fp32 rows [E, R], or (grad_radial_planes given) as operand planes
 int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const float *radial,
                             const float *x, const int32_t *src, const int32_t *dst,
-                            const float *rot, float *grad_radial, float *du_both, float *grad_rot,
+                            const float *rot, float *grad_radial, float *du_both, float *torque,
                             cudaStream_t st, const ZpPlanes *grad_radial_planes,
                             const ZpScale &scale);
 // node_out[n, l^2 + j, c] = sum over the m' rows r of degree l, in table order, of
@@ -224,17 +252,19 @@ struct ZpEpilogue {
   int width;                                    // channels per m' row (H or C)
   int row_first;                                // m' row of column 0
   int8_t row_l[ZP_MAX_KM];                      // degree of each m' row
-  int16_t rot_off[ZP_MAX_KM];                   // offset of the row's entries in a packed rotation
+  int16_t rot_off[ZP_MAX_KM];                   // offset of the row's partial sums in a slab
   // gate
   const float *gate;                            // [M, ld_gate] raw gate scalars, block l-1 at column (l-1)*width
   int64_t ld_gate;
   ZpPlanes out;                                 // activated rows: element (e, n) at e*out.ld + n
   float *slope_max;                             // running max of sigmoid'(gate), or null
   // rotate back
-  const float *rot, *env;                       // [M, nnz_pad], [M]
+  const float *rot, *env;                       // [M, rot_ld], [M]
+  int16_t row_off[ZP_MAX_KM];                   // offset of the row's entries in `rot`
+  int rot_ld;
   const int32_t *row_ptr;                       // [n_nodes + 1] offsets of the nodes' edges
   const int32_t *block_node;                    // [ceil(M/32)] node of edge 32 b (zp_launch_block_nodes)
-  int n_nodes, nnz, nnz_pad;
+  int n_nodes, nnz;
   float *head, *cont;                           // [n_nodes][nnz][width], [ceil(M/32)][nnz][width]
 };
 

@@ -95,11 +95,11 @@ constexpr int kZpRadialSplits = 8;       // K splits of the radial layer's weigh
 constexpr int kZpColRows = 512;          // rows per partial column sum
 
 //   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials
-//   backward: dy planes | dht | dh1 planes | da1 | du_src | grot | wgrad partials | scratch
+//   backward: dy planes | dht | dh1 planes | da1 | du_src | torque | wgrad partials | scratch
 // mode 0 / 1: forward that keeps what a backward reads (1: plus the backward's own regions);
 // mode 2: forward alone with fused epilogues -- of h1 only the gate scalars exist, y does not.
 struct ZpWorkspace {
-  float *rot, *h1, *y, *dht, *da1, *du_src, *grot, *wgrad, *scales, *head, *cont;
+  float *rot, *h1, *y, *dht, *da1, *du_src, *torque, *wgrad, *scales, *head, *cont;
   float *col1, *col2, *col_rad;          // partial column sums: bias gradients of conv1, conv2, radial
   float *radial, *rad_partials;          // radial layer inside the call: its output, dW partials
   int64_t ld_h1;

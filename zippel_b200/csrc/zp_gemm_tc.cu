@@ -411,7 +411,7 @@ __device__ __forceinline__ void rotate_back_block(const ZpEpilogue &f, const uin
   if (one_row && row0 + lane < row_end) {
     const int ei = row0 + lane;
     env_l = f.env[ei];
-    const float *re = f.rot + (size_t)ei * f.nnz_pad + off;
+    const float *re = f.rot + (size_t)ei * f.rot_ld + f.row_off[r];
 #pragma unroll
     for (int j = 0; j < kMaxNj; ++j)
       if (j < nj) rot_l[j] = re[j];
@@ -448,7 +448,7 @@ __device__ __forceinline__ void rotate_back_block(const ZpEpilogue &f, const uin
         const int i = e - row0;
         const float yv = f.env[e] * *reinterpret_cast<const float *>(
                                         stage + i * 128 + (((lane >> 2) ^ (i & 7)) << 4) + ((lane & 3) << 2));
-        const float *re = f.rot + (size_t)e * f.nnz_pad + off;
+        const float *re = f.rot + (size_t)e * f.rot_ld + f.row_off[r];
 #pragma unroll
         for (int j = 0; j < kMaxNj; ++j) {
           if (j >= njmax) break;                 // warp-uniform

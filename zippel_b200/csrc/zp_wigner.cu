@@ -57,58 +57,48 @@ __device__ __forceinline__ double anti(const double *sn, int i) {
   return f > 0 ? -sn[f] : (f < 0 ? sn[-f] : 0.0);
 }
 
-template <int L, int LMAX>
-__device__ __forceinline__ void block_forward(const ZpTables &t, const double *__restrict__ J,
-                                              const Frame<LMAX> &f, const double *cg,
-                                              const double *sg, float *rot_e) {
+// Column j of the degree-L block: the rows |m| <= rows_m, written through put(i, value).
+// frame: cos/sin(k beta), cos/sin(k alpha), cos/sin(k gamma) at frame[(6 * k + which) * 32].
+template <int L, typename Put>
+__device__ __forceinline__ void block_column(const double *__restrict__ J, const double *frame, int j,
+                                             int rows_m, Put put) {
   constexpr int n = 2 * L + 1;
-  const int mm = t.mmax < L ? t.mmax : L;
-#pragma unroll 1
-  for (int j = 0; j < n; ++j) {
-    // column j of  Xb J Xc
-    const int dj = j > L ? j - L : L - j;
-    const double c1 = f.ca[dj];
-    const double s1 = j > L ? -f.sa[dj] : (j < L ? f.sa[dj] : 0.0);   // Xc[n-1-j, j]
-    double P[n], Nn[n];
+  auto fr = [&](int k, int which) { return frame[(6 * k + which) * 32]; };
+  // column j of  Xb J Xc
+  const int dj = j > L ? j - L : L - j;
+  const double c1 = fr(dj, 2);
+  const double s1 = j > L ? -fr(dj, 3) : (j < L ? fr(dj, 3) : 0.0);       // Xc[n-1-j, j]
+  double P[n], Nn[n];
 #pragma unroll
-    for (int i = 0; i < n; ++i) P[i] = J[i * n + j] * c1 + J[i * n + (n - 1 - j)] * s1;
+  for (int i = 0; i < n; ++i) P[i] = J[i * n + j] * c1 + J[i * n + (n - 1 - j)] * s1;
 #pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const int di = i > L ? i - L : L - i;
-      Nn[i] = f.cb[di] * P[i] + anti<L>(f.sb, i) * P[n - 1 - i];
+  for (int i = 0; i < n; ++i) {
+    const int di = i > L ? i - L : L - i;
+    const double sb = i < L ? -fr(di, 1) : (i > L ? fr(di, 1) : 0.0);
+    Nn[i] = fr(di, 0) * P[i] + sb * P[n - 1 - i];
+  }
+  // rows |m| <= rows_m of J (Xb J Xc), then the Xa mix of row i with its partner n-1-i
+#pragma unroll
+  for (int d = 0; d <= L; ++d) {
+    if (d > rows_m) break;
+    double mp = 0.0, mn = 0.0;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      mp += J[(L + d) * n + k] * Nn[k];
+      if (d) mn += J[(L - d) * n + k] * Nn[k];
     }
-    // rows |m| <= mm of J (Xb J Xc), then the Xa mix of row i with its partner n-1-i
-    double M[n];
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      M[i] = 0.0;
-      const int di = i > L ? i - L : L - i;
-      if (di <= mm) {
-        double acc = 0.0;
-#pragma unroll
-        for (int k = 0; k < n; ++k) acc += J[i * n + k] * Nn[k];
-        M[i] = acc;
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const int di = i > L ? i - L : L - i;
-      if (di <= mm) {
-        const double d = cg[di] * M[i] + anti<L>(sg, i) * M[n - 1 - i];
-        rot_e[t.rot_off[t.row_of[L][i]] + j] = (float)d;
-      }
+    if (d == 0) {
+      put(L, mp);
+    } else {
+      const double cg = fr(d, 4), sg = fr(d, 5);
+      put(L + d, cg * mp + sg * mn);
+      put(L - d, cg * mn - sg * mp);
     }
   }
 }
 
 template <int L, int LMAX>
 struct ForEachL {
-  static __device__ __forceinline__ void fwd(const ZpTables &t, const double *J,
-                                             const Frame<LMAX> &f, const double *cg,
-                                             const double *sg, float *rot_e) {
-    ForEachL<L - 1, LMAX>::fwd(t, J, f, cg, sg, rot_e);
-    block_forward<L, LMAX>(t, J + t.jd_off[L], f, cg, sg, rot_e);
-  }
   static __device__ __forceinline__ void bwd(const ZpTables &t, const double *J,
                                              const Frame<LMAX> &f, const double *cg,
                                              const double *sg, const float *g_e, double *dcb,
@@ -116,9 +106,6 @@ struct ForEachL {
 };
 template <int LMAX>
 struct ForEachL<-1, LMAX> {
-  static __device__ __forceinline__ void fwd(const ZpTables &, const double *,
-                                             const Frame<LMAX> &, const double *, const double *,
-                                             float *) {}
   static __device__ __forceinline__ void bwd(const ZpTables &, const double *,
                                              const Frame<LMAX> &, const double *, const double *,
                                              const float *, double *, double *, double *,
@@ -199,45 +186,96 @@ __device__ __forceinline__ void ForEachL<L, LMAX>::bwd(const ZpTables &t, const 
   block_backward<L, LMAX>(t, J + t.jd_off[L], f, cg, sg, g_e, dcb, dsb, dca, dsa);
 }
 
+template <int L, int LMAX>
+struct ColumnOf {
+  template <typename Put>
+  static __device__ __forceinline__ void run(const ZpTables &t, const double *J, const double *frame,
+                                             int l, int j, int extra, Put put) {
+    if (l == L) {
+      const int rows = t.mmax + extra < L ? t.mmax + extra : L;
+      block_column<L>(J + t.jd_off[L], frame, j, rows, put);
+    } else {
+      ColumnOf<L - 1, LMAX>::run(t, J, frame, l, j, extra, put);
+    }
+  }
+};
 template <int LMAX>
-__global__ void __launch_bounds__(128)
+struct ColumnOf<-1, LMAX> {
+  template <typename Put>
+  static __device__ __forceinline__ void run(const ZpTables &, const double *, const double *, int, int,
+                                             int, Put) {}
+};
+
+// A block turns 32 edges: one warp forms their frames, then every warp takes columns (l, j) of the
+// rotation in turn, its lanes being the edges, so all lanes read the same J entries and run the same
+// code.  The entries are collected in shared memory and leave as whole rows.  (One thread per edge
+// wrote them one by one, 32 sectors per store, and had too few warps to hide the fp64 latency:
+// 87 us for 60 000 edges at lmax 4, against x us.)  packed: the public layout, else the kernels' own
+// with the rows m = +-(mmax + 1).
+constexpr int kFwdThreads = 256;
+template <int LMAX>
+__global__ void __launch_bounds__(kFwdThreads)
 wigner_fwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
                   const float *__restrict__ ev, const float *__restrict__ cgam,
-                  const float *__restrict__ sgam, float *__restrict__ rot) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
-  Frame<LMAX> f;
-  frame_forward<LMAX>(f, ev + 3 * e);
-  double cg[LMAX + 1], sg[LMAX + 1];
+                  const float *__restrict__ sgam, float *__restrict__ rot, int packed) {
+  extern __shared__ __align__(16) double smem_d[];       // frames [LMAX + 1][6][32] | out [32][ld + 1]
+  double *frames = smem_d;
+  float *out = reinterpret_cast<float *>(smem_d + (LMAX + 1) * 6 * 32);
+  const int ld = packed ? t.nnz_pad : t.rot_ld, lds = ld | 1;
+  const int64_t e0 = (int64_t)blockIdx.x * 32;
+  const int n_e = (int)min((int64_t)32, E - e0);
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  if (warp == 0) {
+    const int64_t e = e0 + min(lane, n_e - 1);
+    Frame<LMAX> f;
+    frame_forward<LMAX>(f, ev + 3 * e);
 #pragma unroll
-  for (int k = 0; k <= LMAX; ++k) {
-    cg[k] = cgam[e * (LMAX + 1) + k];
-    sg[k] = sgam[e * (LMAX + 1) + k];
+    for (int k = 0; k <= LMAX; ++k) {
+      double *q = frames + 6 * k * 32 + lane;
+      q[0] = f.cb[k]; q[32] = f.sb[k]; q[64] = f.ca[k]; q[96] = f.sa[k];
+      q[128] = cgam[e * (LMAX + 1) + k];
+      q[160] = sgam[e * (LMAX + 1) + k];
+    }
+  } else {
+    for (int i = threadIdx.x - 32; i < 32 * lds; i += kFwdThreads - 32) out[i] = 0.f;   // padding entries
   }
-  float *rot_e = rot + e * t.nnz_pad;
-  for (int p = t.nnz; p < t.nnz_pad; ++p) rot_e[p] = 0.f;
-  ForEachL<LMAX, LMAX>::fwd(t, J, f, cg, sg, rot_e);
+  __syncthreads();
+  float *mine = out + lane * lds;
+  for (int col = warp; col < t.K; col += kFwdThreads / 32) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= col) ++l;
+    const int j = col - l * l;
+    ColumnOf<LMAX, LMAX>::run(t, J, frames + lane, l, j, packed ? 0 : 1, [&](int i, double v) {
+      const int am = i > l ? i - l : l - i;
+      int off;
+      if (am > t.mmax) off = t.ext_off[l][i > l ? 0 : 1];
+      else off = packed ? t.rot_off[t.row_of[l][i]] : t.row_off[t.row_of[l][i]];
+      mine[off + j] = (float)v;
+    });
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < n_e * ld; i += kFwdThreads) {
+    const int le = i / ld, k = i - le * ld;
+    rot[e0 * ld + i] = out[le * lds + k];
+  }
 }
 
+// VJP of one edge's rotation, step by step through the construction above.  g_e: packed layout.
 template <int LMAX>
-__global__ void __launch_bounds__(128)
-wigner_bwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
-                  const float *__restrict__ ev, const float *__restrict__ cgam,
-                  const float *__restrict__ sgam, const float *__restrict__ grot,
-                  float *__restrict__ gev) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= E) return;
+__device__ __noinline__ void chain_backward(const ZpTables &t, const double *__restrict__ J,
+                                            const float *ev, const float *cgam, const float *sgam,
+                                            const float *g_e, float *gev) {
   Frame<LMAX> f;
-  frame_forward<LMAX>(f, ev + 3 * e);
+  frame_forward<LMAX>(f, ev);
   double cg[LMAX + 1], sg[LMAX + 1];
   double dcb[LMAX + 1], dsb[LMAX + 1], dca[LMAX + 1], dsa[LMAX + 1], du[LMAX + 1];
 #pragma unroll
   for (int k = 0; k <= LMAX; ++k) {
-    cg[k] = cgam[e * (LMAX + 1) + k];
-    sg[k] = sgam[e * (LMAX + 1) + k];
+    cg[k] = cgam[k];
+    sg[k] = sgam[k];
     dcb[k] = dsb[k] = dca[k] = dsa[k] = du[k] = 0.0;
   }
-  ForEachL<LMAX, LMAX>::bwd(t, J, f, cg, sg, grot + e * t.nnz_pad, dcb, dsb, dca, dsa);
+  ForEachL<LMAX, LMAX>::bwd(t, J, f, cg, sg, g_e, dcb, dsb, dca, dsa);
 
   // sin(k beta) = r * U_{k-1}(y)
   double dr = 0.0, dy = 0.0;
@@ -274,18 +312,109 @@ wigner_bwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__
   const double dinv_norm = dx * f.v[0] + dy * f.v[1] + dz * f.v[2];
   double dn2 = -0.5 * dinv_norm * f.inv_norm / fmax(f.n2_raw, kS2Floor);
   if (!(f.n2_raw >= kS2Floor)) dn2 = 0.0;
-  gev[3 * e + 0] = (float)(dx * f.inv_norm + 2.0 * f.v[0] * dn2);
-  gev[3 * e + 1] = (float)(dy * f.inv_norm + 2.0 * f.v[1] * dn2);
-  gev[3 * e + 2] = (float)(dz * f.inv_norm + 2.0 * f.v[2] * dn2);
+  gev[0] = (float)(dx * f.inv_norm + 2.0 * f.v[0] * dn2);
+  gev[1] = (float)(dy * f.inv_norm + 2.0 * f.v[1] * dn2);
+  gev[2] = (float)(dz * f.inv_norm + 2.0 * f.v[2] * dn2);
+}
+
+template <int LMAX>
+__global__ void __launch_bounds__(128)
+wigner_bwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
+                  const float *__restrict__ ev, const float *__restrict__ cgam,
+                  const float *__restrict__ sgam, const float *__restrict__ grot,
+                  float *__restrict__ gev) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= E) return;
+  chain_backward<LMAX>(t, J, ev + 3 * e, cgam + e * (LMAX + 1), sgam + e * (LMAX + 1),
+                       grot + e * t.nnz_pad, gev + 3 * e);
+}
+
+// The rotation of an edge frame depends on the edge's direction only, so its VJP needs no more than
+// the three derivatives under rotations of the frame, which the kernels that hold the rows form on
+// the way (torque; zp_rotate.cu):  with v = |v| (sin b sin a, cos b, sin b cos a), roll angle g,
+//   dL/db = cos g T1 + sin g T2,    dL/da = sin b (sin g T1 - cos g T2) + cos b T0,
+//   grad v = ( dL/db e_b + dL/da / sin b  e_a ) / |v|.
+// An edge along the polar axis (sin^2 b below the floor of the construction) has no proper rotation
+// and goes through the construction step by step: its warp forms the gradient of every rotation
+// entry from the saved rows.  A crystal without displacements has a few such edges per atom.
+template <int LMAX>
+__global__ void __launch_bounds__(128)
+edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
+                     const float *__restrict__ ev, const float *__restrict__ cgam,
+                     const float *__restrict__ sgam, const float4 *__restrict__ torque,
+                     const ZpTorqueArgs a, float *__restrict__ gev) {
+  extern __shared__ float grads[];                      // [4 warps][nnz_pad]
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int64_t e = (int64_t)blockIdx.x * 128 + threadIdx.x;
+  bool pole = false;
+  if (e < E) {
+    const double x = ev[3 * e], y = ev[3 * e + 1], z = ev[3 * e + 2];
+    const double n2 = x * x + y * y + z * z;
+    const double inv = rsqrt(fmax(n2, kS2Floor));
+    const double xh = x * inv, yh = y * inv, zh = z * inv, s2 = xh * xh + zh * zh;
+    pole = LMAX >= 1 && !(n2 >= kS2Floor && s2 >= kS2Floor);
+    if (!pole) {
+      double gx = 0.0, gy = 0.0, gz = 0.0;
+      if constexpr (LMAX >= 1) {
+        const float4 T = torque[e];
+        const double inv_r = rsqrt(s2), r = s2 * inv_r, ca = zh * inv_r, sa = xh * inv_r;
+        const double c1 = cgam[e * (LMAX + 1) + 1], s1 = sgam[e * (LMAX + 1) + 1];
+        const double gb = c1 * T.y + s1 * T.z, ga = s1 * T.y - c1 * T.z + yh * inv_r * T.x;
+        gx = inv * (gb * yh * sa + ga * ca);
+        gy = -inv * gb * r;
+        gz = inv * (gb * yh * ca - ga * sa);
+      }
+      gev[3 * e] = (float)gx;
+      gev[3 * e + 1] = (float)gy;
+      gev[3 * e + 2] = (float)gz;
+    }
+  }
+  float *g_s = grads + warp * t.nnz_pad;
+  for (unsigned todo = __ballot_sync(0xffffffffu, pole); todo; todo &= todo - 1) {
+    const int who = __ffs(todo) - 1;
+    const int64_t q = (int64_t)blockIdx.x * 128 + warp * 32 + who;
+    const int C = t.C, C2 = 2 * t.C;
+    const float *xs = a.x + (size_t)a.src[q] * t.K * C, *xd = a.x + (size_t)a.dst[q] * t.K * C;
+    const float *g = a.g_out + (size_t)a.dst[q] * t.K * C;
+    for (int r = 0; r < t.Km; ++r) {
+      const int l = t.row_l[r], m = t.row_m[r], am = m < 0 ? -m : m;
+      const float *da = a.da1 + ((size_t)q * t.Km + r) * C2;
+      const float *rad = a.radial + (size_t)q * t.R + t.rad_off[am] + (l - am) * C2;
+      const float *yr = a.y + ((size_t)q * t.Km + r) * C;
+      for (int j = 0; j < 2 * l + 1; ++j) {
+        const size_t o = (size_t)(l * l + j) * C;
+        float in = 0.f, back = 0.f;
+        for (int c = lane; c < C; c += 32) {
+          in += da[c] * rad[c] * xs[o + c] + da[C + c] * rad[C + c] * xd[o + c];
+          back += yr[c] * g[o + c];
+        }
+        in += a.env[q] * back;
+#pragma unroll
+        for (int k = 16; k > 0; k >>= 1) in += __shfl_xor_sync(0xffffffffu, in, k);
+        if (lane == 0) g_s[t.rot_off[r] + j] = in;
+      }
+    }
+    __syncwarp();
+    if (lane == who)
+      chain_backward<LMAX>(t, J, ev + 3 * q, cgam + q * (LMAX + 1), sgam + q * (LMAX + 1), g_s, gev + 3 * q);
+    __syncwarp();
+  }
 }
 
 }  // namespace
 
 int zp_launch_wigner_fwd(const zp_plan *p, int64_t E, const float *ev, const float *cg,
-                         const float *sg, float *rot, cudaStream_t st) {
+                         const float *sg, float *rot, int packed, cudaStream_t st) {
   if (E == 0) return ZP_OK;
-  const dim3 grid((unsigned)zp_ceil_div(E, 128)), block(128);
-#define CALL(LM) wigner_fwd_kernel<LM><<<grid, block, 0, st>>>(p->t, p->jd_dev, E, ev, cg, sg, rot)
+  const unsigned grid = (unsigned)zp_ceil_div(E, 32);
+  const int ld = packed ? p->t.nnz_pad : p->t.rot_ld;
+  const size_t smem = (size_t)(p->t.lmax + 1) * 6 * 32 * sizeof(double) + (size_t)32 * (ld | 1) * sizeof(float);
+#define CALL(LM)                                                                                  \
+  {                                                                                               \
+    static ZpSmemOptIn opt_in;                                                                    \
+    if (int rc_ = zp_ensure_smem(wigner_fwd_kernel<LM>, smem, opt_in)) return rc_;                \
+    wigner_fwd_kernel<LM><<<grid, kFwdThreads, smem, st>>>(p->t, p->jd_dev, E, ev, cg, sg, rot, packed); \
+  }
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("wigner_fwd_kernel");
@@ -301,5 +430,20 @@ int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const flo
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("wigner_bwd_kernel");
+  return ZP_OK;
+}
+
+int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const float *cg,
+                            const float *sg, const float *torque, const ZpTorqueArgs &a, float *gev,
+                            cudaStream_t st) {
+  if (E == 0) return ZP_OK;
+  const dim3 grid((unsigned)zp_ceil_div(E, 128)), block(128);
+  const size_t smem = (size_t)4 * p->t.nnz_pad * sizeof(float);
+#define CALL(LM)                                                                                  \
+  edge_vec_grad_kernel<LM><<<grid, block, smem, st>>>(p->t, p->jd_dev, E, ev, cg, sg,             \
+                                                      reinterpret_cast<const float4 *>(torque), a, gev)
+  ZP_DISPATCH_LMAX(p->t.lmax, CALL)
+#undef CALL
+  ZP_LAUNCH_CHECK("edge_vec_grad_kernel");
   return ZP_OK;
 }
