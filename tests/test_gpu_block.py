@@ -115,3 +115,17 @@ def test_edges_along_the_polar_axis(jd64):
     got = gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"])
     assert rel_l2(got[0], want[0]) < 1e-5
     assert rel_l2(got[2][6:], want[2][6:]) < 1e-5 and rel_l2(got[2][:6], want[2][:6]) < 1e-3
+
+
+@pytest.mark.parametrize("e", [63, 64, 65, 2049, 24000, 24001])
+def test_products_together_and_apart(e):
+    """Around the edge counts where the products of a step stop sharing one launch, where a split of
+    the contraction over the edges has a remainder, and where it needs a second accumulation chunk:
+    the same gradients as the three-plane format, whose kernel and tiles differ."""
+    cfg = dict(lmax=1, mmax=1, sphere_channels=16, hidden_channels=24, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    params = orc.init_params(cfg, seed=e)
+    case = random_case(cfg, 50, e, seed=e)
+    a = gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"])
+    b = gpu_node_out_and_vjp(make_block(cfg, params, precision="fp32_bf16x3"), case, case["upstream"])
+    check_against(*a, *b)

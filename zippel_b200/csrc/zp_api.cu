@@ -16,6 +16,12 @@ namespace {
 thread_local char g_cuda_error[512] = "";
 thread_local int64_t g_launches = 0;
 
+// Up to this many edges the products of a step share one launch.  Beyond it each is a launch of its
+// own on the plan's streams: the fixed walk through one long list leaves CTAs idle at its end (3 % at
+// 60 000 edges), while the CTAs of a next launch start wherever an SM becomes free; below it the
+// set-up and the draining of each launch cost more (conv1 of 6 000 edges in bf16: 82 us apart, 70
+// together).
+constexpr int64_t kTogetherEdges = 24000;
 constexpr int kChunkK = 2048;          // contraction length of one TMEM accumulation chunk
 
 // The fused epilogues (gate activation in conv1, rotation back + segmented sums in conv2) need
@@ -83,6 +89,18 @@ const float *wscale(const zp_plan *p, const ZpWorkspace &w, int conv, int m) {
   return p->fp16 ? w.scales + kScWeights + (conv * (ZP_MAX_L + 1) + m) * 2 + 1 : nullptr;
 }
 
+// Independent products, in one launch or side by side (between fork and join).
+int run_products(const zp_plan *plan, Lanes &lanes, const ZpGemmTc *g, int n, int cls, cudaStream_t st) {
+  int rc;
+  if (n == 0) return ZP_OK;
+  if (n <= ZP_GEMM_GROUP && (g[0].a_mn ? g[0].K : g[0].M) <= kTogetherEdges) {
+    ZP_TIMED(cls, zp_launch_gemm_group(g, n, st));
+    return ZP_OK;
+  }
+  for (int i = 0; i < n; ++i) ZP_TIMED(cls, zp_launch_gemm_tc(g[i], lanes.pick(i)));
+  return ZP_OK;
+}
+
 // operand views of one m-block inside a plane buffer (column offset `col`)
 ZpPlanes sub(const ZpPlanes &p, int64_t col) {
   ZpPlanes q = p;
@@ -138,7 +156,7 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
     if (ec > 0) {
       w.gr = c.planes(E, t.R, rad, w.scales + kScGrScale);
       w.col_rad = c.floats(parts * t.R);
-      w.rad_partials = c.floats((size_t)kZpRadialSplits * t.R * ((ec + 3) / 4 * 4));
+      w.rad_partials = c.floats((size_t)zp_radial_splits(t.R, ec) * t.R * ((ec + 3) / 4 * 4));
     }
   }
   w.bytes = c.off > end_fwd ? c.off : end_fwd;
@@ -519,20 +537,22 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
     }
     if ((rc = lanes.join())) return rc;
   } else {
-    // the per-m products are independent: side by side on the plan's streams
-    if ((rc = lanes.fork())) return rc;
-    for (int m = 0; m < plan->n_blocks && E > 0; ++m) {
+    // the per-m products are independent
+    ZpGemmTc products[ZP_MAX_L + 1];
+    for (int m = 0; m < plan->n_blocks; ++m) {
       const int in = plan->c1_in[m], out = plan->c1_out[m];
       const ZpPlanes A = sub(ws.a1, (int64_t)t.m_row0[m] * 2 * t.C);
-      float *Cc = ws.h1 + (m == 0 ? 0 : t.n_gate + (size_t)t.m_row0[m] * t.H);
-      const ZpGemmTc g{E, out, in, P, A.base, A.ld, A.plane_stride, 0,
-                       ws.wfold + plan->c1_woff[m], in, (int64_t)out * in, 0,
-                       m == 0 ? w->c1_b0 : nullptr, Cc, t.w1_cols, plan->status_dev, 0, 1, 0, 0,
-                       plan->fp16, A.scale, wscale(plan, ws, 0, m),
-                       plan->fp16 ? ws.scales + kScH1 : nullptr, nullptr};
-      ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(g, lanes.pick(m)));
+      products[m] = ZpGemmTc{E, out, in, P, A.base, A.ld, A.plane_stride, 0,
+                             ws.wfold + plan->c1_woff[m], in, (int64_t)out * in, 0,
+                             m == 0 ? w->c1_b0 : nullptr,
+                             ws.h1 + (m == 0 ? 0 : t.n_gate + (size_t)t.m_row0[m] * t.H), t.w1_cols,
+                             plan->status_dev, 0, 1, 0, 0, plan->fp16, A.scale, wscale(plan, ws, 0, m),
+                             plan->fp16 ? ws.scales + kScH1 : nullptr, nullptr};
     }
-    if ((rc = lanes.join())) return rc;
+    const bool apart = E > kTogetherEdges;
+    if (apart && (rc = lanes.fork())) return rc;
+    if ((rc = run_products(plan, lanes, products, plan->n_blocks, ZP_K_GEMM_FWD, st))) return rc;
+    if (apart && (rc = lanes.join())) return rc;
     // |gate(h1)| <= |h1|
     ZP_TIMED(ZP_K_GATE_FWD,
              zp_launch_gate_fwd(plan, E, ws.h1, ws.ht, zp_scale_of(1.f, ws.scales + kScH1, ws.scales + kScHt),
@@ -555,20 +575,24 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
     epi.block_node = ws.block_node;
     ZP_TIMED(ZP_K_ROTATE_BACK, zp_launch_block_nodes(E, N, c.row_ptr, ws.block_node, st));
   }
-  if ((rc = lanes.fork())) return rc;
+  const bool apart = fuse2 || E > kTogetherEdges;
+  if (apart && (rc = lanes.fork())) return rc;
+  ZpGemmTc products[ZP_MAX_L + 1];
   for (int m = 0; m < plan->n_blocks && E > 0; ++m) {
     const int in = plan->c2_in[m], out = plan->c2_out[m];
     const ZpPlanes A = sub(ws.ht, (int64_t)t.m_row0[m] * t.H);
     float *Cc = lean ? ws.h1 : ws.y + (size_t)t.m_row0[m] * t.C;     // lean: never dereferenced
     epi.row_first = t.m_row0[m];
-    const ZpGemmTc g{E, out, in, P, A.base, A.ld, A.plane_stride, 0,
-                     ws.wfold + plan->c2_woff[m], in, (int64_t)out * in, 0,
-                     m == 0 ? w->c2_b0 : nullptr, Cc, ldy, plan->status_dev, 0, 1, 0, 0,
-                     plan->fp16, A.scale, wscale(plan, ws, 1, m), nullptr,
-                     fuse2 ? &epi : nullptr};
-    ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(g, lanes.pick(m)));
+    products[m] = ZpGemmTc{E, out, in, P, A.base, A.ld, A.plane_stride, 0,
+                           ws.wfold + plan->c2_woff[m], in, (int64_t)out * in, 0,
+                           m == 0 ? w->c2_b0 : nullptr, Cc, ldy, plan->status_dev, 0, 1, 0, 0,
+                           plan->fp16, A.scale, wscale(plan, ws, 1, m), nullptr,
+                           fuse2 ? &epi : nullptr};
+    if (fuse2) ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(products[m], lanes.pick(m)));
   }
-  if ((rc = lanes.join())) return rc;
+  if (!fuse2 && E > 0 && (rc = run_products(plan, lanes, products, plan->n_blocks, ZP_K_GEMM_FWD, st)))
+    return rc;
+  if (apart && (rc = lanes.join())) return rc;
   if (fuse2)
     ZP_TIMED(ZP_K_ROTATE_BACK,
              zp_launch_node_sum(plan, N, ws.head, ws.cont, c.row_ptr, node_out, st));
@@ -721,8 +745,11 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
       ZP_TIMED(ZP_K_GATE_BWD, zp_launch_gate_bwd(plan, E, ws.h1, ws.dht, ws.dh1, dh1_scale, st));
     }
     // the input- and weight-gradient products of the blocks and the bias column sums only read
-    // dY, X and the weights: side by side on the plan's streams
-    if ((rc = lanes.fork())) return rc;
+    // dY, X and the weights
+    ZpGemmTc products[2 * (ZP_MAX_L + 1)];
+    int nd = 0, nw = 0;
+    ZpGemmTc *const wgrads = products + plan->n_blocks;
+    int *const splits = conv ? splits_c2 : splits_c1;
     for (int m = 0; m < plan->n_blocks; ++m) {
       const int in = conv ? plan->c2_in[m] : plan->c1_in[m];
       const int out = conv ? plan->c2_out[m] : plan->c1_out[m];
@@ -732,29 +759,38 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
       const uint16_t *Wt = ws.wfold + (conv ? plan->c2_woff[m] : plan->c1_woff[m]) +
                                 (int64_t)P * out * in;
       float *G = ws.wgrad + (conv ? plan->c2_goff[m] : plan->c1_goff[m]);
-      int &nsplit = (conv ? splits_c2 : splits_c1)[m];
-      nsplit = 1;
+      splits[m] = 1;
       if (E == 0) {
-        if (want_w)
-          ZP_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * (size_t)out * in, lanes.pick(2 * m + 1)));
+        if (want_w) ZP_CUDA(cudaMemsetAsync(G, 0, sizeof(float) * (size_t)out * in, st));
         continue;
       }
-      const ZpGemmTc gd{E, in, out, P, dYm.base, dYm.ld, dYm.plane_stride, 0,
-                        Wt, out, (int64_t)out * in, 0, nullptr, dX + xcol, ldx,
-                        plan->status_dev, 0, 1, 0, 0, plan->fp16, dYm.scale,
-                        wscale(plan, ws, conv, m),
-                        // max |dht|; max |da1| when the radial layer's gradient needs it
-                        conv ? (plan->fp16 ? ws.scales + kScDht : nullptr)
-                             : (scaled_gr ? ws.scales + kScDa1 : nullptr)};
-      ZP_TIMED(ZP_K_GEMM_DGRAD, zp_launch_gemm_tc(gd, lanes.pick(want_w ? 2 * m : m)));
-      if (!want_w) continue;
-      ZpGemmTc gw_{out, in, E, P, dYm.base, dYm.ld, dYm.plane_stride, 1,
-                   Xm.base, Xm.ld, Xm.plane_stride, 1, nullptr, G, in,
-                   plan->status_dev, 0, 1, plan->g_elems, 0, plan->fp16, dYm.scale, Xm.scale,
-                   nullptr};
-      gw_.ksplit = zp_gemm_tc_pick_splits(gw_, kZpWgradSplits);
-      nsplit = zp_gemm_tc_splits(gw_);
-      ZP_TIMED(ZP_K_GEMM_WGRAD, zp_launch_gemm_tc(gw_, lanes.pick(2 * m + 1)));
+      products[nd++] = ZpGemmTc{E, in, out, P, dYm.base, dYm.ld, dYm.plane_stride, 0,
+                                Wt, out, (int64_t)out * in, 0, nullptr, dX + xcol, ldx,
+                                plan->status_dev, 0, 1, 0, 0, plan->fp16, dYm.scale,
+                                wscale(plan, ws, conv, m),
+                                // max |dht|; max |da1| when the radial layer's gradient needs it
+                                conv ? (plan->fp16 ? ws.scales + kScDht : nullptr)
+                                     : (scaled_gr ? ws.scales + kScDa1 : nullptr), nullptr};
+      if (want_w)
+        wgrads[nw++] = ZpGemmTc{out, in, E, P, dYm.base, dYm.ld, dYm.plane_stride, 1,
+                                Xm.base, Xm.ld, Xm.plane_stride, 1, nullptr, G, in,
+                                plan->status_dev, 0, 1, plan->g_elems, 0, plan->fp16, dYm.scale,
+                                Xm.scale, nullptr, nullptr};
+    }
+    const bool together = E <= kTogetherEdges && nd + nw <= ZP_GEMM_GROUP;
+    if (nw && together) zp_gemm_group_splits(wgrads, nw, kZpWgradSplits);
+    for (int m = 0; m < nw; ++m) {
+      if (!together) wgrads[m].ksplit = zp_gemm_tc_pick_splits(wgrads[m], kZpWgradSplits);
+      splits[m] = zp_gemm_tc_splits(wgrads[m]);
+    }
+    if ((rc = lanes.fork())) return rc;
+    if (together) {
+      if ((rc = run_products(plan, lanes, products, nd + nw, ZP_K_GEMM_DGRAD, st))) return rc;
+    } else {
+      for (int m = 0; m < nd; ++m) {
+        ZP_TIMED(ZP_K_GEMM_DGRAD, zp_launch_gemm_tc(products[m], lanes.pick(want_w ? 2 * m : m)));
+        if (nw) ZP_TIMED(ZP_K_GEMM_WGRAD, zp_launch_gemm_tc(wgrads[m], lanes.pick(2 * m + 1)));
+      }
     }
     if (want_w)
       ZP_TIMED(ZP_K_BIAS_GRAD,
@@ -774,7 +810,8 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   if (rl && E > 0) {
     ZP_TIMED(ZP_K_GEMM_WGRAD,
              zp_linear_backward_planes(plan, E, rl->ec, t.R, ws.hr, ws.rw, ws.gr, rl->grad_h,
-                                       rl->grad_w, rl->grad_b, ws.rad_partials, kZpRadialSplits,
+                                       rl->grad_w, rl->grad_b, ws.rad_partials,
+                                       zp_radial_splits(t.R, rl->ec),
                                        ws.col_rad, list, st, rl->grad_h_max));
   } else if (rl && rl->grad_w) {
     ZP_CUDA(cudaMemsetAsync(rl->grad_w, 0, sizeof(float) * (size_t)t.R * rl->ec, st));

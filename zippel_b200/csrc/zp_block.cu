@@ -76,8 +76,8 @@ BlockWs carve_block(const zp_plan *p, const zp_front_config &f, int64_t N, int64
     w.g_env = c.floats(e);
     w.dz1 = c.planes(E, ec, fm.f1, sc + kScDz1);
     w.dz0 = c.planes(E, ec, fm.f0, sc + kScDz0);
-    w.part0 = c.floats((size_t)kZpRadialSplits * ec * round4(w0));
-    w.part1 = c.floats((size_t)kZpRadialSplits * ec * round4(ec));
+    w.part0 = c.floats((size_t)zp_radial_splits(ec, w0) * ec * round4(w0));
+    w.part1 = c.floats((size_t)zp_radial_splits(ec, ec) * ec * round4(ec));
     w.ln_part = c.floats((size_t)2 * ZP_LN_PARTIALS * 3 * ec);
     w.front = c.bytes(zp_edge_features_work_bytes(&f, rows, E));
   }
@@ -292,7 +292,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                                     grads->ln_gamma[1], grads->ln_beta[1], grads->rad_b[1], ln1, list, st)))
       return rc;
     if ((rc = zp_linear_backward_planes(plan, E, ec, ec, b.hid0, b.w1, b.dz1, b.g_hid0,
-                                        grads->rad_w[1], nullptr, b.part1, kZpRadialSplits, nullptr,
+                                        grads->rad_w[1], nullptr, b.part1, zp_radial_splits(ec, ec), nullptr,
                                         list, st, fm.f0.fp16 ? sc + kScGHid0 : nullptr)))
       return rc;
     if ((rc = zp_launch_ln_silu_bwd(E, ec, b.h0, params->ln_gamma[0], params->ln_beta[0], mean0, rstd0,
@@ -305,7 +305,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
     const int64_t cols = grads->emb ? w0 : front->num_basis;
     const bool want_in = grad_pos || grads->emb;
     if ((rc = zp_linear_backward_planes(plan, E, w0, ec, b.xe, b.w0, b.dz0, want_in ? b.g_xe : nullptr,
-                                        grads->rad_w[0], nullptr, b.part0, kZpRadialSplits, nullptr,
+                                        grads->rad_w[0], nullptr, b.part0, zp_radial_splits(ec, w0), nullptr,
                                         list, st, nullptr, cols)))
       return rc;
     if (want_in &&

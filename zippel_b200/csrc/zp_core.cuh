@@ -91,7 +91,13 @@ enum { kScX = 0, kScRad, kScH1, kScA1, kScHt, kScDy, kScDh1, kScGate, kScMaxNode
        kScCount };
 
 constexpr int kZpWgradSplits = 8;
-constexpr int kZpRadialSplits = 8;       // K splits of the radial layer's weight gradient
+// K splits of a radial layer's weight gradient [N, K], whose contraction runs over the edges: as many
+// as it takes to give every SM a share of the few tiles (eight left 140 SMs idle for 100 us at
+// 60 000 edges and 128 x 128), eight at least
+inline int zp_radial_splits(int64_t N, int64_t K) {
+  const int64_t tiles = zp_ceil_div(N, 128) * zp_ceil_div(K, 256), s = 148 / tiles;
+  return (int)(s < 8 ? 8 : s > 64 ? 64 : s);
+}
 constexpr int kZpColRows = 512;          // rows per partial column sum
 
 //   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials

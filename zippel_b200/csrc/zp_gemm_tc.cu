@@ -38,6 +38,7 @@
 // Shared-memory tiles use the 128-byte (BK = 64) or 64-byte (BK = 32) swizzle that TMA writes
 // and the matrix descriptors name.  Every mbarrier wait is bounded: after ~2 s it records
 // ZP_ERR_DEVICE_TIMEOUT in the status word, raises the CTA's abort flag and the CTA drains.
+#include <atomic>
 #include <cstdlib>
 #include <mutex>
 
@@ -156,18 +157,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
       : "r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-        "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -175,6 +164,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
         "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
         "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
       : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_ld_wait() {
@@ -196,23 +191,30 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes
   return d;
 }
 
-struct GemmParams {
-  int M, N, K;
+// One product of a launch.
+struct GemmProb {
+  CUtensorMap map_a, map_b, map_c;
+  int M, N;
   int BN;                 // tile width, multiple of 16, <= 256
-  int num_m, num_n, num_k;
+  int num_n, num_k;
   int ksplit, kb_per_split, kc;   // CTAs-level split of K; k-blocks per TMEM accumulation chunk
   int a_mn, b_mn;         // operand is MN-major
-  int fp16;               // operand planes are fp16 (else bf16)
+  int start;              // first work item
   const float *scale_a, *scale_b;   // device scalars multiplying the result (null = 1)
   float *absmax_out;      // device scalar: running max |C| of what this launch stores (or null)
   const float *bias;
-  float *C;
-  int64_t ldc, split_stride;
-  int tma_store;          // epilogue goes through TMA stores (map_c is valid)
+};
+// The products of one launch.  Independent products (the orders m of a convolution, input and weight
+// gradients) share a launch when each alone would leave the device's last wave half empty: their
+// tiles form one list that the persistent CTAs walk.
+struct GemmGroup {
+  GemmProb p[ZP_GEMM_GROUP];
+  int n, total;           // products, work items of all of them
+  int fp16;               // operand planes are fp16 (else bf16)
   int *status;
   uint64_t wait_limit_ns; // bound of every mbarrier wait
   int unarmed;            // self-test: the producers load nothing, so the first wait runs out
-  ZpEpilogue epi;         // work of the fused epilogues (mode 0: none)
+  ZpEpilogue epi;         // work of the fused epilogues (mode 0: none; one product only)
 };
 
 // plane pairs; for three planes pair 0 is the leading product, pairs 1..5 the small ones
@@ -239,8 +241,8 @@ template <> struct Pairs<3> {
 // epilogue of a 128 x 256 tile costs ~8 000 store wavefronts.  Instead each epilogue warp writes
 // 32 x 32 blocks into its own 4 KB of shared memory (128-byte rows under the 128-byte swizzle, the
 // layout the tensor map names) and one lane hands the block to the TMA unit, which writes full
-// lines and clips rows / columns beyond the matrix.  Later K chunks of a tile use the reducing
-// store (add) after the previous store of that tile has completed.
+// lines and clips rows / columns beyond the matrix.  The accumulation chunks of a long contraction
+// are added up in the epilogue's registers, so a tile is stored once.
 constexpr int kEpiBlockBytes = 32 * 32 * 4;
 constexpr int kEpiBytes = 8 * kEpiBlockBytes;                 // eight epilogue warps
 
@@ -250,14 +252,6 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void 
                :
                : "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
                : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap *map, const void *src, int c0,
-                                                  int c1, int c2) {
-  asm volatile(
-      "cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-      :
-      : "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
 }
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() {            // shared source may be overwritten
@@ -275,17 +269,13 @@ __device__ __forceinline__ void bulk_wait_all() {             // the writes them
 // out of shared memory while the next block is staged (products with a short contraction are
 // bound by their output stores, and one 4 KB block per warp in flight does not cover the latency).
 template <int EB>
-__device__ __forceinline__ void epilogue_store_tma(const GemmParams &p, const CUtensorMap *map_c,
-                                                   float (&v)[4][32], uint8_t *stage0, int lane,
-                                                   int row0, int n0, int col_lo, int col_hi,
-                                                   int split, const float *bias, bool first,
-                                                   float &seen_max, uint32_t &blocks_done) {
+__device__ __forceinline__ void epilogue_store_tma(const GemmProb &p, float (&v)[4][32],
+                                                   uint8_t *stage0, int lane, int row0, int n0,
+                                                   int col_lo, int col_hi, int split,
+                                                   const float *bias, float &seen_max,
+                                                   uint32_t &blocks_done) {
   if (row0 >= p.M) return;                        // warp-uniform: nothing of this slice exists
   const bool row_ok = row0 + lane < p.M;
-  if (!first) {                                   // the tile's previous store must have landed
-    if (lane == 0) bulk_wait_all();
-    __syncwarp();
-  }
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int cc = col_lo + 32 * b;
@@ -302,7 +292,7 @@ __device__ __forceinline__ void epilogue_store_tma(const GemmParams &p, const CU
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       float4 o = make_float4(v[b][4 * k], v[b][4 * k + 1], v[b][4 * k + 2], v[b][4 * k + 3]);
-      if (first && bias) {
+      if (bias) {
         const int c = n + 4 * k;
         o.x += c < p.N ? bias[c] : 0.f;
         o.y += c + 1 < p.N ? bias[c + 1] : 0.f;
@@ -323,8 +313,7 @@ __device__ __forceinline__ void epilogue_store_tma(const GemmParams &p, const CU
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) {
-      if (first) tma_store_3d(map_c, stage, n, row0, split);
-      else tma_reduce_add_3d(map_c, stage, n, row0, split);
+      tma_store_3d(&p.map_c, stage, n, row0, split);
       bulk_commit();
     }
   }
@@ -468,21 +457,21 @@ __device__ __forceinline__ void rotate_back_block(const ZpEpilogue &f, const uin
 
 // v[b][j]: value at row `row0 + lane`, column `n0 + col_lo + 32 b + j` (scaled, no bias yet).
 template <int EPI>
-__device__ __forceinline__ void epilogue_fused(const GemmParams &p, const CUtensorMap *map_c,
+__device__ __forceinline__ void epilogue_fused(const GemmProb &p, const ZpEpilogue &epi,
                                                float (&v)[4][32], uint8_t *stage, int lane, int row0,
                                                int n0, int col_lo, int col_hi, const float *bias,
                                                float &seen_max, float &slope_max, int node,
                                                int rp_l) {
   if (row0 >= p.M) return;
   const bool row_ok = row0 + lane < p.M;
-  const float inv = EPI == ZP_EPI_GATE ? zp_inv_scale(p.epi.out) : 1.f;
+  const float inv = EPI == ZP_EPI_GATE ? zp_inv_scale(epi.out) : 1.f;
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int cc = col_lo + 32 * b;
     if (cc >= col_hi) continue;                   // warp-uniform
     const int n = n0 + cc;
     if (n >= p.N) continue;
-    if (p.epi.store_c && lane == 0) bulk_wait_read();   // the TMA store of the previous block
+    if (epi.store_c && lane == 0) bulk_wait_read();   // the TMA store of the previous block
     __syncwarp();                                 // ... and every lane's reads of it are done
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -503,18 +492,18 @@ __device__ __forceinline__ void epilogue_fused(const GemmParams &p, const CUtens
       }
       *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) = o;
     }
-    if (p.epi.store_c) {
+    if (epi.store_c) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) {
-        tma_store_3d(map_c, stage, n, row0, 0);
+        tma_store_3d(&p.map_c, stage, n, row0, 0);
         bulk_commit();
       }
     } else {
       __syncwarp();
     }
-    if (EPI == ZP_EPI_GATE) gate_block(p.epi, stage, lane, row0, n, p.M, p.N, inv, slope_max);
-    else rotate_back_block(p.epi, stage, lane, row0, n, p.M, p.N, node, node, rp_l);
+    if (EPI == ZP_EPI_GATE) gate_block(epi, stage, lane, row0, n, p.M, p.N, inv, slope_max);
+    else rotate_back_block(epi, stage, lane, row0, n, p.M, p.N, node, node, rp_l);
   }
 }
 
@@ -526,32 +515,121 @@ struct SmemLayout {
   static constexpr int kStage = P * (kATile + kBTile);
   static constexpr int kTiles = STAGES * kStage;
   static constexpr int kBars = 8 * (2 * STAGES + 4);
-  // barriers, TMEM slot and abort flag live in the first KB after the tiles; the epilogue's
-  // store blocks (when the CTA's budget allows them) follow, 1 KB aligned; + 1 KB alignment slack
+  // barriers, TMEM slot and abort flag live in the first KB after the tiles; the epilogue's store
+  // blocks follow, 1 KB aligned; + 1 KB alignment slack
   static_assert(kBars + 16 <= 1024, "control words fit in one KB");
-  static constexpr bool kTmaEpilogue = kTiles + 1024 + kEpiBytes + 1024 <= 232448;
   static constexpr int kEpiOffset = kTiles + 1024;
-  static constexpr int kTotal = kTiles + 1024 + (kTmaEpilogue ? kEpiBytes : 0) + 1024;
+  static constexpr int kTotal = kTiles + 1024 + kEpiBytes + 1024;
 };
 
-// One unit of work of a CTA: an output tile, a K split, and its k-block range.
+// One unit of work of a CTA (or CTA pair): a product, an output tile of it, a K split and its
+// k-block range.
 struct Work {
-  int m0, n0, split, kb0, kb1;
+  int prob, m0, n0, split, kb0, kb1;
 };
-__device__ __forceinline__ Work decode_work(const GemmParams &p, int w) {
+template <int TM>
+__device__ __forceinline__ Work decode_work(const GemmGroup &g, int w) {
   Work x;
+  x.prob = 0;
+  while (x.prob + 1 < g.n && w >= g.p[x.prob + 1].start) ++x.prob;
+  const GemmProb &p = g.p[x.prob];
+  w -= p.start;
   x.split = w % p.ksplit;
   const int tile = w / p.ksplit;
-  x.m0 = (tile / p.num_n) * BM;
+  x.m0 = (tile / p.num_n) * TM;
   x.n0 = (tile % p.num_n) * p.BN;
   x.kb0 = x.split * p.kb_per_split;
   x.kb1 = min(p.num_k, x.kb0 + p.kb_per_split);
   return x;
 }
+__device__ __forceinline__ void prefetch_maps(const GemmGroup &g) {
+  for (int i = 0; i < g.n; ++i) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.p[i].map_a)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.p[i].map_b)) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.p[i].map_c)) : "memory");
+  }
+}
+// instruction descriptor: fp32 accumulators, operand format and majorness, tile shape
+__device__ __forceinline__ uint32_t instr_desc(const GemmGroup &g, const GemmProb &p, int tile_m) {
+  const uint32_t fmt = g.fp16 ? 0u : 1u;      // operand format field: 0 = f16, 1 = bf16
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
+         ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(p.BN >> 3) << 17) | ((uint32_t)(tile_m >> 4) << 24);
+}
+
+// What an epilogue warp carries from tile to tile: the largest magnitude it stored of the current
+// product, handed over when the product changes.
+struct MaxTracker {
+  float *out = nullptr;
+  float seen = 0.f;
+  __device__ __forceinline__ void flush(int lane) {
+    if (out) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) seen = fmaxf(seen, __shfl_xor_sync(0xffffffffu, seen, o));
+      if (lane == 0 && seen > 0.f) zp_atomic_absmax(out, seen);
+    }
+    seen = 0.f;
+  }
+  __device__ __forceinline__ void follow(float *next, int lane) {
+    if (next != out) {
+      flush(lane);
+      out = next;
+    }
+  }
+};
+
+// The accumulator slice of a tile's first chunk (this warp's 32 rows, columns col_lo .. col_hi) into
+// v.  Sixteen columns at a time: the slice itself (128 values per thread) leaves little room for
+// staging registers; both accumulators' loads are in flight before one wait.
+template <int P>
+__device__ __forceinline__ void read_accumulator(float (&v)[4][32], uint32_t t_row, int col_lo,
+                                                 int col_hi, float out_scale) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const int cc = col_lo + 32 * b;
+    if (cc < col_hi) {                    // warp-uniform
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t r[16], r2[16];
+        tmem_ld16(t_row + cc + 16 * h, r);
+        if (P != 1) tmem_ld16(t_row + kTmemBuf + cc + 16 * h, r2);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          float a = __uint_as_float(r[j]);
+          if (P != 1) a += __uint_as_float(r2[j]);
+          v[b][16 * h + j] = a * out_scale;
+        }
+      }
+    }
+  }
+}
+// ... and of a later chunk, added to it (all of v is live here: eight columns at a time)
+template <int P>
+__device__ __forceinline__ void add_accumulator(float (&v)[4][32], uint32_t t_row, int col_lo,
+                                                int col_hi, float out_scale) {
+#pragma unroll
+  for (int b = 0; b < 4; ++b) {
+    const int cc = col_lo + 32 * b;
+    if (cc < col_hi) {
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        uint32_t r[8], r2[8];
+        tmem_ld8(t_row + cc + 8 * h, r);
+        if (P != 1) tmem_ld8(t_row + kTmemBuf + cc + 8 * h, r2);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float a = __uint_as_float(r[j]);
+          if (P != 1) a += __uint_as_float(r2[j]);
+          v[b][8 * h + j] = fmaf(a, out_scale, v[b][8 * h + j]);
+        }
+      }
+    }
+  }
+}
 
 template <int P, int BK, int STAGES, int BN_CAP, int EPI, int EB = 1>
-__device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
-                                             const CUtensorMap &map_c, const GemmParams &p) {
+__device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
   using L = SmemLayout<P, BK, STAGES, BN_CAP, EB>;
   constexpr int kAccBufs = P == 1 ? 2 : 1;      // accumulation units in flight in TMEM
   extern __shared__ uint8_t smem_raw[];
@@ -565,9 +643,10 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int num_work = p.num_m * p.num_n * p.ksplit;
+  const int num_work = g.total;
 
   if (threadIdx.x == 0) {
+    prefetch_maps(g);
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 8); }
     *abort_flag = 0;
@@ -587,18 +666,19 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
   const uint32_t tmem_base = *tmem_slot;
 
   const uint32_t a_bytes = BM * BK * 2;
-  const uint32_t b_bytes = (uint32_t)p.BN * BK * 2;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (!p.unarmed && elect_one()) {
+    if (!g.unarmed && elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-        const Work x = decode_work(p, w);
+        const Work x = decode_work<BM>(g, w);
+        const GemmProb &p = g.p[x.prob];
+        const uint32_t b_bytes = (uint32_t)p.BN * BK * 2;
         for (int kb = x.kb0; kb < x.kb1 && ok; ++kb, ++it) {
           const int s = it % STAGES;
-          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, p.status, p.wait_limit_ns);
+          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           uint8_t *st = smem + (size_t)s * L::kStage;
           mbar_expect_tx(&full[s], P * (a_bytes + b_bytes));
@@ -607,16 +687,16 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
           for (int pl = 0; pl < P; ++pl) {
             uint8_t *ta = st + pl * L::kATile, *tb = st + P * L::kATile + pl * L::kBTile;
             if (!p.a_mn) {
-              tma_load_3d(ta, &map_a, &full[s], k0, x.m0, pl);
+              tma_load_3d(ta, &p.map_a, &full[s], k0, x.m0, pl);
             } else {                      // two 64-wide column blocks of [BK][64]
-              tma_load_3d(ta, &map_a, &full[s], x.m0, k0, pl);
-              tma_load_3d(ta + BK * 128, &map_a, &full[s], x.m0 + 64, k0, pl);
+              tma_load_3d(ta, &p.map_a, &full[s], x.m0, k0, pl);
+              tma_load_3d(ta + BK * 128, &p.map_a, &full[s], x.m0 + 64, k0, pl);
             }
             if (!p.b_mn) {
-              tma_load_3d(tb, &map_b, &full[s], k0, x.n0, pl);
+              tma_load_3d(tb, &p.map_b, &full[s], k0, x.n0, pl);
             } else {
               for (int nb = 0; nb < p.BN; nb += 64)
-                tma_load_3d(tb + (nb / 64) * BK * 128, &map_b, &full[s], x.n0 + nb, k0, pl);
+                tma_load_3d(tb + (nb / 64) * BK * 128, &p.map_b, &full[s], x.n0 + nb, k0, pl);
             }
           }
         }
@@ -625,19 +705,17 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     if (elect_one()) {
-      const uint32_t fmt = p.fp16 ? 0u : 1u;    // operand format field: 0 = f16, 1 = bf16
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
-                             ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(p.BN >> 3) << 17) |
-                             ((uint32_t)(BM >> 4) << 24);
       constexpr uint32_t kLayout = BK == 64 ? 2u : 4u;
       uint32_t it = 0, unit = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-        const Work x = decode_work(p, w);
+        const Work x = decode_work<BM>(g, w);
+        const GemmProb &p = g.p[x.prob];
+        const uint32_t idesc = instr_desc(g, p, BM);
         for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
           const int c1 = min(x.kb1, c0 + p.kc);
           const int buf = unit % kAccBufs;
-          ok = mbar_wait(&tmem_empty[buf], ((unit / kAccBufs) & 1) ^ 1, abort_flag, p.status, p.wait_limit_ns);
+          ok = mbar_wait(&tmem_empty[buf], ((unit / kAccBufs) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           tcgen05_fence_after();
           // one plane: accumulator `buf`; three planes: leading product at column 0, small at 256
@@ -645,7 +723,7 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
           const uint32_t d_small = tmem_base + kTmemBuf;
           for (int kb = c0; kb < c1 && ok; ++kb, ++it) {
             const int s = it % STAGES;
-            ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, p.status, p.wait_limit_ns);
+            ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, g.status, g.wait_limit_ns);
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t sa = smem_u32(smem + (size_t)s * L::kStage);
@@ -683,112 +761,52 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
     uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes * EB;
     uint32_t unit = 0, blocks_done = 0;
     bool ok = true;
-    const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
-    float seen_max = 0.f, slope_max = 0.f;
-    const int col_lo = half * 128, col_hi = min(p.BN, col_lo + 128);
+    float slope_max = 0.f;
+    MaxTracker maxima;
+    const int col_lo = half * 128;
     for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-      const Work x = decode_work(p, w);
+      const Work x = decode_work<BM>(g, w);
+      const GemmProb &p = g.p[x.prob];
       const int row0 = x.m0 + q * 32;
-      const int row = row0 + lane;
-      float *crow = p.C + (size_t)x.split * p.split_stride + (size_t)row * p.ldc;
+      const int col_hi = min(p.BN, col_lo + 128);
       const float *bias = x.split == 0 ? p.bias : nullptr;
+      const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
+      maxima.follow(p.absmax_out, lane);
+      // the node of the warp's first edge and the offsets of the 32 nodes from there on, fetched
+      // while the tile is still being formed
+      int node = 0, rp_l = 0;
+      if (EPI == ZP_EPI_ROTATE_BACK && row0 < p.M) {
+        node = g.epi.block_node[row0 >> 5];
+        rp_l = g.epi.row_ptr[min(node + lane, g.epi.n_nodes)];
+      }
+      float v[4][32];
       for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
         const int buf = unit % kAccBufs;
-        const bool first = c0 == x.kb0;         // first chunk stores, later chunks add
-        // the node of the warp's first edge and the offsets of the 32 nodes from there on,
-        // fetched while the tile is still being formed
-        int node = 0, rp_l = 0;
-        if (EPI == ZP_EPI_ROTATE_BACK && row0 < p.M) {
-          node = p.epi.block_node[row0 >> 5];
-          rp_l = p.epi.row_ptr[min(node + lane, p.epi.n_nodes)];
-        }
-        ok = mbar_wait(&tmem_full[buf], (unit / kAccBufs) & 1, abort_flag, p.status, p.wait_limit_ns);
+        ok = mbar_wait(&tmem_full[buf], (unit / kAccBufs) & 1, abort_flag, g.status, g.wait_limit_ns);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) +
-                               (P == 1 ? (uint32_t)buf * kTmemBuf : 0u);
-        float v[4][32];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int cc = col_lo + 32 * b;
-          if (cc < col_hi) {                    // warp-uniform
-            // 16 columns at a time, the small-product accumulator added in place: the slice
-            // itself (128 values per thread) leaves little room for staging registers
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              // both accumulators' loads are in flight together: one wait per 16 columns
-              uint32_t r[16], r2[16];
-              tmem_ld16(t_row + cc + 16 * h, r);
-              if (P != 1) tmem_ld16(t_row + kTmemBuf + cc + 16 * h, r2);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                float a = __uint_as_float(r[j]);
-                if (P != 1) a += __uint_as_float(r2[j]);
-                v[b][16 * h + j] = a * out_scale;
-              }
-            }
-          }
-        }
+        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (P == 1 ? (uint32_t)buf * kTmemBuf : 0u);
+        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&tmem_empty[buf]);      // TMEM slice is in registers now
-
-        if (EPI != ZP_EPI_NONE) {
-          if (L::kTmaEpilogue)
-            epilogue_fused<EPI>(p, &map_c, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias,
-                                seen_max, slope_max, node, rp_l);
-        } else if (L::kTmaEpilogue && p.tma_store) {
-          epilogue_store_tma<EB>(p, &map_c, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split,
-                                 bias, first, seen_max, blocks_done);
-        } else if (row < p.M) {
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int cc = col_lo + 32 * b;
-            if (cc >= col_hi) continue;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const int n = x.n0 + cc + j;
-              if (cc + j < p.BN && n + 3 < p.N) {
-                float4 o = make_float4(v[b][j], v[b][j + 1], v[b][j + 2], v[b][j + 3]);
-                if (first) {
-                  if (bias) {
-                    const float4 bv = *reinterpret_cast<const float4 *>(bias + n);
-                    o.x += bv.x; o.y += bv.y; o.z += bv.z; o.w += bv.w;
-                  }
-                } else {
-                  const float4 old = *reinterpret_cast<const float4 *>(crow + n);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4 *>(crow + n) = o;
-                seen_max = fmaxf(seen_max, fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)),
-                                                 fmaxf(fabsf(o.z), fabsf(o.w))));
-              } else if (cc + j < p.BN) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                  if (n + u < p.N) {
-                    const float base = first ? (bias ? bias[n + u] : 0.f) : crow[n + u];
-                    const float o = v[b][j + u] + base;
-                    crow[n + u] = o;
-                    seen_max = fmaxf(seen_max, fabsf(o));
-                  }
-              }
-            }
-          }
-        }
       }
+      if (!ok) break;
+      if constexpr (EPI != ZP_EPI_NONE)
+        epilogue_fused<EPI>(p, g.epi, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias, maxima.seen,
+                            slope_max, node, rp_l);
+      else
+        epilogue_store_tma<EB>(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias,
+                               maxima.seen, blocks_done);
     }
-    if (L::kTmaEpilogue && p.tma_store && lane == 0) bulk_wait_all();   // this warp's stores are done
-    if (p.absmax_out) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) seen_max = fmaxf(seen_max, __shfl_xor_sync(0xffffffffu, seen_max, o));
-      if (lane == 0 && seen_max > 0.f) zp_atomic_absmax(p.absmax_out, seen_max);
-    }
-    if (EPI == ZP_EPI_GATE && p.epi.slope_max) {
+    if (lane == 0) bulk_wait_all();                        // this warp's stores are done
+    maxima.flush(lane);
+    if (EPI == ZP_EPI_GATE && g.epi.slope_max) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) slope_max = fmaxf(slope_max, __shfl_xor_sync(0xffffffffu, slope_max, o));
-      if (lane == 0 && slope_max > 0.f) zp_atomic_absmax(p.epi.slope_max, slope_max);
+      if (lane == 0 && slope_max > 0.f) zp_atomic_absmax(g.epi.slope_max, slope_max);
     }
   }
 
@@ -802,19 +820,13 @@ __device__ __forceinline__ void gemm_tc_body(const CUtensorMap &map_a, const CUt
 }
 
 template <int P, int BK, int STAGES, int BN_CAP, int EB = 1>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_c, const __grid_constant__ GemmParams p) {
-  gemm_tc_body<P, BK, STAGES, BN_CAP, ZP_EPI_NONE, EB>(map_a, map_b, map_c, p);
+__global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmGroup g) {
+  gemm_tc_body<P, BK, STAGES, BN_CAP, ZP_EPI_NONE, EB>(g);
 }
 // the same contraction with a fused epilogue (the epilogue warps hold more live values)
 template <int P, int BK, int STAGES, int BN_CAP, int EPI>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_fused_kernel(const __grid_constant__ CUtensorMap map_a,
-                     const __grid_constant__ CUtensorMap map_b,
-                     const __grid_constant__ CUtensorMap map_c,
-                     const __grid_constant__ GemmParams p) {
-  gemm_tc_body<P, BK, STAGES, BN_CAP, EPI>(map_a, map_b, map_c, p);
+__global__ void __launch_bounds__(kThreads, 1) gemm_tc_fused_kernel(const __grid_constant__ GemmGroup g) {
+  gemm_tc_body<P, BK, STAGES, BN_CAP, EPI>(g);
 }
 
 // ---- CTA-pair variant ---------------------------------------------------------------------
@@ -895,25 +907,12 @@ struct SmemLayoutPair {
   static constexpr int kTiles = STAGES * kStage;
   static constexpr int kBars = 8 * (2 * STAGES + 4);
   static_assert(kBars + 16 <= 1024, "control words fit in one KB");
-  static constexpr bool kTmaEpilogue = kTiles + 1024 + kEpiBytes + 1024 <= 232448;
   static constexpr int kEpiOffset = kTiles + 1024;
-  static constexpr int kTotal = kTiles + 1024 + (kTmaEpilogue ? kEpiBytes : 0) + 1024;
+  static constexpr int kTotal = kTiles + 1024 + kEpiBytes + 1024;
 };
 
-__device__ __forceinline__ Work decode_work_pair(const GemmParams &p, int w) {
-  Work x;
-  x.split = w % p.ksplit;
-  const int tile = w / p.ksplit;
-  x.m0 = (tile / p.num_n) * BM2;
-  x.n0 = (tile % p.num_n) * p.BN;
-  x.kb0 = x.split * p.kb_per_split;
-  x.kb1 = min(p.num_k, x.kb0 + p.kb_per_split);
-  return x;
-}
-
 template <int P, int BK, int STAGES, int EPI>
-__device__ __forceinline__ void gemm_tc_pair_body(const CUtensorMap &map_a, const CUtensorMap &map_b,
-                                                  const CUtensorMap &map_c, const GemmParams &p) {
+__device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
   using L = SmemLayoutPair<P, BK, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared window starts at the same offset in both CTAs, so does everything below
@@ -929,10 +928,10 @@ __device__ __forceinline__ void gemm_tc_pair_body(const CUtensorMap &map_a, cons
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t rank = cluster_ctarank();          // 0 = leader
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int num_work = p.num_m * p.num_n * p.ksplit;
-  const int half_n = p.BN >> 1;
+  const int num_work = g.total;
 
   if (threadIdx.x == 0) {
+    prefetch_maps(g);
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 16); }
     *abort_flag = 0;
@@ -955,19 +954,21 @@ __device__ __forceinline__ void gemm_tc_pair_body(const CUtensorMap &map_a, cons
   const uint32_t tmem_base = *tmem_slot;
 
   const uint32_t a_bytes = BM * BK * 2;
-  const uint32_t b_bytes = (uint32_t)half_n * BK * 2;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer (both CTAs)
-    if (!p.unarmed && elect_one()) {
+    if (!g.unarmed && elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int w = pair; w < num_work && ok; w += num_pairs) {
-        const Work x = decode_work_pair(p, w);
+        const Work x = decode_work<BM2>(g, w);
+        const GemmProb &p = g.p[x.prob];
+        const int half_n = p.BN >> 1;
+        const uint32_t b_bytes = (uint32_t)half_n * BK * 2;
         const int m0 = x.m0 + (int)rank * BM, n0 = x.n0 + (int)rank * half_n;
         for (int kb = x.kb0; kb < x.kb1 && ok; ++kb, ++it) {
           const int s = it % STAGES;
-          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, p.status, p.wait_limit_ns);
+          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           uint8_t *st = smem + (size_t)s * L::kStage;
           if (rank == 0) mbar_expect_tx(&full[s], 2 * P * (a_bytes + b_bytes));
@@ -977,50 +978,48 @@ __device__ __forceinline__ void gemm_tc_pair_body(const CUtensorMap &map_a, cons
           for (int pl = 0; pl < P; ++pl) {
             uint8_t *ta = st + pl * L::kATile, *tb = st + P * L::kATile + pl * L::kBTile;
             if (!p.a_mn) {
-              tma_load_3d_pair(ta, &map_a, bar, k0, m0, pl);
+              tma_load_3d_pair(ta, &p.map_a, bar, k0, m0, pl);
             } else {
-              tma_load_3d_pair(ta, &map_a, bar, m0, k0, pl);
-              tma_load_3d_pair(ta + BK * 128, &map_a, bar, m0 + 64, k0, pl);
+              tma_load_3d_pair(ta, &p.map_a, bar, m0, k0, pl);
+              tma_load_3d_pair(ta + BK * 128, &p.map_a, bar, m0 + 64, k0, pl);
             }
             if (!p.b_mn) {
-              tma_load_3d_pair(tb, &map_b, bar, k0, n0, pl);
+              tma_load_3d_pair(tb, &p.map_b, bar, k0, n0, pl);
             } else {
               for (int nb = 0; nb < half_n; nb += 64)
-                tma_load_3d_pair(tb + (nb / 64) * BK * 128, &map_b, bar, n0 + nb, k0, pl);
+                tma_load_3d_pair(tb + (nb / 64) * BK * 128, &p.map_b, bar, n0 + nb, k0, pl);
             }
           }
         }
       }
       // the leader's last stage releases must have landed here before this CTA may exit
       for (int j = 0; j < STAGES && ok; ++j, ++it)
-        ok = mbar_wait(&empty[it % STAGES], ((it / STAGES) & 1) ^ 1, abort_flag, p.status, p.wait_limit_ns);
+        ok = mbar_wait(&empty[it % STAGES], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer (leader only)
     if (rank == 0 && elect_one()) {
-      const uint32_t fmt = p.fp16 ? 0u : 1u;
-      const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.a_mn ? 1 : 0) << 15) |
-                             ((uint32_t)(p.b_mn ? 1 : 0) << 16) | ((uint32_t)(p.BN >> 3) << 17) |
-                             ((uint32_t)(BM2 >> 4) << 24);
       constexpr uint32_t kLayout = BK == 64 ? 2u : 4u;
       uint32_t it = 0, unit = 0;
       bool ok = true;
       for (int w = pair; w < num_work && ok; w += num_pairs) {
-        const Work x = decode_work_pair(p, w);
+        const Work x = decode_work<BM2>(g, w);
+        const GemmProb &p = g.p[x.prob];
+        const uint32_t idesc = instr_desc(g, p, BM2);
         for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
           const int c1 = min(x.kb1, c0 + p.kc);
           // one plane: the two accumulator buffers alternate, so the next tile's MMAs run
           // while the epilogue drains this one
           const int buf = P == 1 ? (int)(unit & 1) : 0;
           const uint32_t round = P == 1 ? (unit >> 1) : unit;
-          ok = mbar_wait(&tmem_empty[buf], (round & 1) ^ 1, abort_flag, p.status, p.wait_limit_ns);
+          ok = mbar_wait(&tmem_empty[buf], (round & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           tcgen05_fence_after();
           const uint32_t d_main = tmem_base + (uint32_t)buf * kTmemBuf;
           const uint32_t d_small = tmem_base + kTmemBuf;
           for (int kb = c0; kb < c1 && ok; ++kb, ++it) {
             const int s = it % STAGES;
-            ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, p.status, p.wait_limit_ns);
+            ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, g.status, g.wait_limit_ns);
             if (!ok) break;
             tcgen05_fence_after();
             const uint32_t sa = smem_u32(smem + (size_t)s * L::kStage);
@@ -1053,114 +1052,55 @@ __device__ __forceinline__ void gemm_tc_pair_body(const CUtensorMap &map_a, cons
     uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes;
     uint32_t unit = 0, blocks_done = 0;
     bool ok = true;
-    const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
-    float seen_max = 0.f, slope_max = 0.f;
-    const int col_lo = half * 128, col_hi = min(p.BN, col_lo + 128);
+    float slope_max = 0.f;
+    MaxTracker maxima;
+    const int col_lo = half * 128;
     const uint32_t release_bar0 = map_to_cta(smem_u32(&tmem_empty[0]), 0);
     const uint32_t release_bar1 = map_to_cta(smem_u32(&tmem_empty[1]), 0);
     for (int w = pair; w < num_work && ok; w += num_pairs) {
-      const Work x = decode_work_pair(p, w);
+      const Work x = decode_work<BM2>(g, w);
+      const GemmProb &p = g.p[x.prob];
       const int row0 = x.m0 + (int)rank * BM + q * 32;
-      const int row = row0 + lane;
-      float *crow = p.C + (size_t)x.split * p.split_stride + (size_t)row * p.ldc;
+      const int col_hi = min(p.BN, col_lo + 128);
       const float *bias = x.split == 0 ? p.bias : nullptr;
+      const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
+      maxima.follow(p.absmax_out, lane);
+      // the node of the warp's first edge and the offsets of the 32 nodes from there on, fetched
+      // while the tile is still being formed
+      int node = 0, rp_l = 0;
+      if (EPI == ZP_EPI_ROTATE_BACK && row0 < p.M) {
+        node = g.epi.block_node[row0 >> 5];
+        rp_l = g.epi.row_ptr[min(node + lane, g.epi.n_nodes)];
+      }
+      float v[4][32];
       for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
-        const bool first = c0 == x.kb0;
         const int buf = P == 1 ? (int)(unit & 1) : 0;
         const uint32_t round = P == 1 ? (unit >> 1) : unit;
-        // the node of the warp's first edge and the offsets of the 32 nodes from there on,
-        // fetched while the tile is still being formed
-        int node = 0, rp_l = 0;
-        if (EPI == ZP_EPI_ROTATE_BACK && row0 < p.M) {
-          node = p.epi.block_node[row0 >> 5];
-          rp_l = p.epi.row_ptr[min(node + lane, p.epi.n_nodes)];
-        }
-        ok = mbar_wait(&tmem_full[buf], round & 1, abort_flag, p.status, p.wait_limit_ns);
+        ok = mbar_wait(&tmem_full[buf], round & 1, abort_flag, g.status, g.wait_limit_ns);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tcgen05_fence_after();
         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * kTmemBuf;
-        float v[4][32];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const int cc = col_lo + 32 * b;
-          if (cc < col_hi) {
-            // 16 columns at a time, the small-product accumulator added in place: the slice
-            // itself (128 values per thread) leaves little room for staging registers
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              // both accumulators' loads are in flight together: one wait per 16 columns
-              uint32_t r[16], r2[16];
-              tmem_ld16(t_row + cc + 16 * h, r);
-              if (P != 1) tmem_ld16(t_row + kTmemBuf + cc + 16 * h, r2);
-              tmem_ld_wait();
-#pragma unroll
-              for (int j = 0; j < 16; ++j) {
-                float a = __uint_as_float(r[j]);
-                if (P != 1) a += __uint_as_float(r2[j]);
-                v[b][16 * h + j] = a * out_scale;
-              }
-            }
-          }
-        }
+        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(buf ? release_bar1 : release_bar0);
-
-        if (EPI != ZP_EPI_NONE) {
-          if (L::kTmaEpilogue)
-            epilogue_fused<EPI>(p, &map_c, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias,
-                                seen_max, slope_max, node, rp_l);
-        } else if (L::kTmaEpilogue && p.tma_store) {
-          epilogue_store_tma<1>(p, &map_c, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split,
-                                bias, first, seen_max, blocks_done);
-        } else if (row < p.M) {
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int cc = col_lo + 32 * b;
-            if (cc >= col_hi) continue;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const int n = x.n0 + cc + j;
-              if (cc + j < p.BN && n + 3 < p.N) {
-                float4 o = make_float4(v[b][j], v[b][j + 1], v[b][j + 2], v[b][j + 3]);
-                if (first) {
-                  if (bias) {
-                    const float4 bv = *reinterpret_cast<const float4 *>(bias + n);
-                    o.x += bv.x; o.y += bv.y; o.z += bv.z; o.w += bv.w;
-                  }
-                } else {
-                  const float4 old = *reinterpret_cast<const float4 *>(crow + n);
-                  o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-                }
-                *reinterpret_cast<float4 *>(crow + n) = o;
-                seen_max = fmaxf(seen_max, fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)),
-                                                 fmaxf(fabsf(o.z), fabsf(o.w))));
-              } else if (cc + j < p.BN) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                  if (n + u < p.N) {
-                    const float base = first ? (bias ? bias[n + u] : 0.f) : crow[n + u];
-                    const float o = v[b][j + u] + base;
-                    crow[n + u] = o;
-                    seen_max = fmaxf(seen_max, fabsf(o));
-                  }
-              }
-            }
-          }
-        }
       }
+      if (!ok) break;
+      if constexpr (EPI != ZP_EPI_NONE)
+        epilogue_fused<EPI>(p, g.epi, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias, maxima.seen,
+                            slope_max, node, rp_l);
+      else
+        epilogue_store_tma<1>(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias,
+                              maxima.seen, blocks_done);
     }
-    if (L::kTmaEpilogue && p.tma_store && lane == 0) bulk_wait_all();   // this warp's stores are done
-    if (p.absmax_out) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) seen_max = fmaxf(seen_max, __shfl_xor_sync(0xffffffffu, seen_max, o));
-      if (lane == 0 && seen_max > 0.f) zp_atomic_absmax(p.absmax_out, seen_max);
-    }
-    if (EPI == ZP_EPI_GATE && p.epi.slope_max) {
+    if (lane == 0) bulk_wait_all();                        // this warp's stores are done
+    maxima.flush(lane);
+    if (EPI == ZP_EPI_GATE && g.epi.slope_max) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) slope_max = fmaxf(slope_max, __shfl_xor_sync(0xffffffffu, slope_max, o));
-      if (lane == 0 && slope_max > 0.f) zp_atomic_absmax(p.epi.slope_max, slope_max);
+      if (lane == 0 && slope_max > 0.f) zp_atomic_absmax(g.epi.slope_max, slope_max);
     }
   }
 
@@ -1176,20 +1116,13 @@ __device__ __forceinline__ void gemm_tc_pair_body(const CUtensorMap &map_a, cons
 }
 
 template <int P, int BK, int STAGES>
-__global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_a,
-                    const __grid_constant__ CUtensorMap map_b,
-                    const __grid_constant__ CUtensorMap map_c,
-                    const __grid_constant__ GemmParams p) {
-  gemm_tc_pair_body<P, BK, STAGES, ZP_EPI_NONE>(map_a, map_b, map_c, p);
+__global__ void __launch_bounds__(kThreads, 1) gemm_tc_pair_kernel(const __grid_constant__ GemmGroup g) {
+  gemm_tc_pair_body<P, BK, STAGES, ZP_EPI_NONE>(g);
 }
 template <int P, int BK, int STAGES, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_tc_pair_fused_kernel(const __grid_constant__ CUtensorMap map_a,
-                          const __grid_constant__ CUtensorMap map_b,
-                          const __grid_constant__ CUtensorMap map_c,
-                          const __grid_constant__ GemmParams p) {
-  gemm_tc_pair_body<P, BK, STAGES, EPI>(map_a, map_b, map_c, p);
+gemm_tc_pair_fused_kernel(const __grid_constant__ GemmGroup g) {
+  gemm_tc_pair_body<P, BK, STAGES, EPI>(g);
 }
 
 // block_node[b] = the last node n with row_ptr[n] <= 32 b: the node of the first edge of 32-edge
@@ -1290,10 +1223,16 @@ bool pair_enabled() {
   }
   return on == 1;
 }
+// whole 32-column store blocks; each CTA's share of an MN-major B tile comes in 64-wide blocks
+int bn_step(const ZpGemmTc &g, int halves) { return g.b_mn ? 64 * halves : 32; }
 int device_sms() {
+  static std::atomic<int> known[64];               // asked for several times per launch
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 64 && known[dev].load(std::memory_order_relaxed))
+    return known[dev].load(std::memory_order_relaxed);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (dev >= 0 && dev < 64) known[dev].store(sms, std::memory_order_relaxed);
   return sms;
 }
 // Expected utilisation of the tensor pipes for one kernel choice and K split: padded-tile waste
@@ -1308,7 +1247,7 @@ double launch_score(const ZpGemmTc &g, bool pair, int splits) {
   const double wave = (double)items / (double)(zp_ceil_div(items, units) * units);
   // one plane (one MMA pass per k-block) leans on the operand feed harder than two planes do
   const double feed = !pair ? 1.0 : g.planes == 1 ? 1.25 : 1.12;
-  return pad * wave * feed - 0.004 * splits;
+  return pad * wave * feed * (1.0 - 0.004 * splits);
 }
 bool use_pair(const ZpGemmTc &g) {
   if (g.planes != 2 && g.planes != 1) return false;
@@ -1326,12 +1265,15 @@ int block_k(const ZpGemmTc &g) {
   return ((g.planes == 3 && g.variant != 1) || g.planes == 2) ? 32 : 64;
 }
 
+// Split of the contraction in whole 64-deep steps, so that it does not depend on the kernel's k-block
 void split_plan(const ZpGemmTc &g, int bk, int *ksplit, int *kbs, int *num_k) {
-  *num_k = (int)zp_ceil_div(g.K, bk);
+  const int steps = (int)zp_ceil_div(g.K, 64);
   int req = g.ksplit < 1 ? 1 : g.ksplit;
-  if (req > *num_k) req = *num_k;
-  *kbs = (int)zp_ceil_div(*num_k, req);
-  *ksplit = (int)zp_ceil_div(*num_k, *kbs);
+  if (req > steps) req = steps;
+  const int per = (int)zp_ceil_div(steps, req);
+  *ksplit = (int)zp_ceil_div(steps, per);
+  *kbs = per * (64 / bk);
+  *num_k = (int)zp_ceil_div(g.K, bk);
 }
 
 // One-time set-up of a kernel is per device (the raised dynamic shared-memory limit is an
@@ -1355,89 +1297,93 @@ bool fused_mode_ok(const ZpGemmTc &g, int bk) {
   return ksplit == 1 && kbs <= kc && (g.epi->width % 4) == 0;
 }
 
-void fill_params(GemmParams &p, const ZpGemmTc &g, int bk) {
-  p.M = (int)g.M; p.N = (int)g.N; p.K = (int)g.K;
-  split_plan(g, bk, &p.ksplit, &p.kb_per_split, &p.num_k);
-  const int kc_elems = g.kc_elems > 0 ? g.kc_elems : 2048;
-  p.kc = kc_elems / bk < 1 ? 1 : kc_elems / bk;
-  p.a_mn = g.a_mn; p.b_mn = g.b_mn;
-  p.fp16 = g.fp16; p.scale_a = g.scale_a; p.scale_b = g.scale_b; p.absmax_out = g.absmax_out;
-  p.bias = g.bias; p.C = g.C; p.ldc = g.ldc; p.split_stride = g.split_stride; p.status = g.status;
-  p.wait_limit_ns = g.wait_limit_ns > 0 ? (uint64_t)g.wait_limit_ns : kWaitLimitNs;
-  p.unarmed = g.unarmed;
-  if (g.epi) p.epi = *g.epi;
-  else p.epi.mode = ZP_EPI_NONE;
+// Describes the products of one launch: tile shapes, work items, tensor maps.  Products whose items
+// take longest come first, so that what is left for the last round is short.
+// tile_m: rows of a tile; box_m: rows of A one CTA loads; halves: CTAs that share a B tile
+int fill_group(GemmGroup &grp, const ZpGemmTc *const *g, int n, int P, int bk, int tile_m, int halves,
+               int bn_cap) {
+  if (n < 1 || n > ZP_GEMM_GROUP) return ZP_ERR_INVALID_ARG;
+  grp.n = n;
+  grp.fp16 = g[0]->fp16;
+  grp.status = g[0]->status;
+  grp.wait_limit_ns = g[0]->wait_limit_ns > 0 ? (uint64_t)g[0]->wait_limit_ns : kWaitLimitNs;
+  grp.unarmed = g[0]->unarmed;
+  const ZpEpilogue *epi = g[0]->epi;
+  if (epi) grp.epi = *epi;
+  else grp.epi.mode = ZP_EPI_NONE;
+  int order[ZP_GEMM_GROUP];
+  int64_t cost[ZP_GEMM_GROUP];
+  for (int i = 0; i < n; ++i) {
+    int ksplit, kbs, num_k;
+    split_plan(*g[i], bk, &ksplit, &kbs, &num_k);
+    cost[i] = (int64_t)kbs * pick_bn(g[i]->N, bn_cap, bn_step(*g[i], halves));
+    int k = i;
+    for (; k > 0 && cost[order[k - 1]] < cost[i]; --k) order[k] = order[k - 1];
+    order[k] = i;
+  }
+  const CUtensorMapSwizzle kswz = bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+  grp.total = 0;
+  for (int k = 0; k < n; ++k) {
+    const ZpGemmTc &q = *g[order[k]];
+    GemmProb &p = grp.p[k];
+    p.M = (int)q.M; p.N = (int)q.N;
+    split_plan(q, bk, &p.ksplit, &p.kb_per_split, &p.num_k);
+    const int kc_elems = q.kc_elems > 0 ? q.kc_elems : 2048;
+    p.kc = kc_elems / bk < 1 ? 1 : kc_elems / bk;
+    p.a_mn = q.a_mn; p.b_mn = q.b_mn;
+    p.scale_a = q.scale_a; p.scale_b = q.scale_b; p.absmax_out = q.absmax_out; p.bias = q.bias;
+    p.BN = pick_bn(q.N, bn_cap, bn_step(q, halves));
+    p.num_n = (int)zp_ceil_div(q.N, p.BN);
+    p.start = grp.total;
+    grp.total += (int)zp_ceil_div(q.M, tile_m) * p.num_n * p.ksplit;
+    int rc;
+    if (!q.a_mn) rc = make_map(&p.map_a, q.A, q.K, q.M, P, q.lda, q.a_plane, bk, BM, kswz, q.fp16);
+    else rc = make_map(&p.map_a, q.A, q.M, q.K, P, q.lda, q.a_plane, 64, bk, CU_TENSOR_MAP_SWIZZLE_128B, q.fp16);
+    if (rc) return rc;
+    if (!q.b_mn) rc = make_map(&p.map_b, q.B, q.K, q.N, P, q.ldb, q.b_plane, bk, p.BN / halves, kswz, q.fp16);
+    else rc = make_map(&p.map_b, q.B, q.N, q.K, P, q.ldb, q.b_plane, 64, bk, CU_TENSOR_MAP_SWIZZLE_128B, q.fp16);
+    if (rc) return rc;
+    if (epi && epi->mode != ZP_EPI_NONE && !epi->store_c) p.map_c = p.map_a;      // never used
+    else if ((rc = make_map_c(&p.map_c, q.C, q.N, q.M, p.ksplit, q.ldc, q.split_stride))) return rc;
+  }
+  return ZP_OK;
 }
 
 template <int P, int BK, int STAGES, int BN_CAP, int EPI, int EB = 1>
-int launch_e(const ZpGemmTc &g, cudaStream_t st) {
+int launch_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
   using L = SmemLayout<P, BK, STAGES, BN_CAP, EB>;
   static_assert(EB == 1 || EPI == ZP_EPI_NONE, "two store buffers only in the plain epilogue");
   static_assert(L::kTotal <= 232448, "shared memory budget of one CTA");
-  static_assert(EPI == ZP_EPI_NONE || L::kTmaEpilogue, "fused epilogues need the store stage");
   auto kernel = [] {
     if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_kernel<P, BK, STAGES, BN_CAP, EB>;
     else return gemm_tc_fused_kernel<P, BK, STAGES, BN_CAP, EPI>;
   }();
-  int dev = 0, sms = 148;
-  ZP_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kMaxDevices) return ZP_ERR_UNSUPPORTED;
-  static PerDevice configured;
-  {
-    std::lock_guard<std::mutex> hold(configured.lock);
-    if (!configured.done[dev]) {
-      ZP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-      configured.done[dev] = true;
-    }
-  }
-  GemmParams p;
-  fill_params(p, g, BK);
-  // whole 32-column store blocks; MN-major B tiles come in 64-wide blocks
-  p.BN = pick_bn(g.N, BN_CAP, g.b_mn ? 64 : 32);
-  p.num_m = (int)zp_ceil_div(g.M, BM);
-  p.num_n = (int)zp_ceil_div(g.N, p.BN);
-  const CUtensorMapSwizzle kswz = BK == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-  CUtensorMap ma, mb;
+  static ZpSmemOptIn opt_in;
   int rc;
-  if (!g.a_mn) rc = make_map(&ma, g.A, g.K, g.M, P, g.lda, g.a_plane, BK, BM, kswz, g.fp16);
-  else rc = make_map(&ma, g.A, g.M, g.K, P, g.lda, g.a_plane, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B, g.fp16);
-  if (rc) return rc;
-  if (!g.b_mn) rc = make_map(&mb, g.B, g.K, g.N, P, g.ldb, g.b_plane, BK, p.BN, kswz, g.fp16);
-  else rc = make_map(&mb, g.B, g.N, g.K, P, g.ldb, g.b_plane, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B, g.fp16);
-  if (rc) return rc;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  CUtensorMap mc;
-  const int chunks = (int)zp_ceil_div(p.kb_per_split, p.kc);
-  p.tma_store = EPI == ZP_EPI_NONE ? (L::kTmaEpilogue && !(g.absmax_out && chunks > 1))
-                                   : p.epi.store_c;
-  if (p.tma_store) {
-    if ((rc = make_map_c(&mc, g.C, g.N, g.M, p.ksplit, g.ldc, g.split_stride))) return rc;
-  } else {
-    mc = ma;                                      // never read
-  }
-  const int work = p.num_m * p.num_n * p.ksplit;
-  const int grid = work < sms ? work : sms;
-  kernel<<<grid, kThreads, L::kTotal, st>>>(ma, mb, mc, p);
+  if ((rc = zp_ensure_smem(kernel, (size_t)L::kTotal, opt_in))) return rc;
+  GemmGroup grp;
+  if ((rc = fill_group(grp, g, n, P, BK, BM, 1, BN_CAP))) return rc;
+  const int sms = device_sms(), grid = grp.total < sms ? grp.total : sms;
+  kernel<<<grid, kThreads, L::kTotal, st>>>(grp);
   ZP_LAUNCH_CHECK("gemm_tc_kernel");
   return ZP_OK;
 }
 
 template <int P, int BK, int STAGES, int BN_CAP>
-int launch(const ZpGemmTc &g, cudaStream_t st) {
-  const int mode = g.epi ? g.epi->mode : ZP_EPI_NONE;
-  if constexpr (SmemLayout<P, BK, STAGES, BN_CAP>::kTmaEpilogue && (P == 1 || P == 2)) {
-    if (mode == ZP_EPI_GATE) return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_GATE>(g, st);
-    if (mode == ZP_EPI_ROTATE_BACK) return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_ROTATE_BACK>(g, st);
+int launch(const ZpGemmTc *const *g, int n, cudaStream_t st) {
+  const int mode = g[0]->epi ? g[0]->epi->mode : ZP_EPI_NONE;
+  if constexpr (P == 1 || P == 2) {
+    if (mode == ZP_EPI_GATE) return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_GATE>(g, n, st);
+    if (mode == ZP_EPI_ROTATE_BACK) return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_ROTATE_BACK>(g, n, st);
   }
   if (mode != ZP_EPI_NONE) return ZP_ERR_UNSUPPORTED;
-  return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_NONE>(g, st);
+  return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_NONE>(g, n, st);
 }
 
 template <int P, int BK, int STAGES, int EPI>
-int launch_pair_e(const ZpGemmTc &g, cudaStream_t st) {
+int launch_pair_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
   using L = SmemLayoutPair<P, BK, STAGES>;
   static_assert(L::kTotal <= 232448, "shared memory budget of one CTA");
-  static_assert(EPI == ZP_EPI_NONE || L::kTmaEpilogue, "fused epilogues need the store stage");
   auto kernel = [] {
     if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_pair_kernel<P, BK, STAGES>;
     else return gemm_tc_pair_fused_kernel<P, BK, STAGES, EPI>;
@@ -1457,53 +1403,65 @@ int launch_pair_e(const ZpGemmTc &g, cudaStream_t st) {
     std::lock_guard<std::mutex> hold(pairs.lock);
     if (!pairs.done[dev]) {
       ZP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-      int sms = 148, n = 0;
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+      const int sms = device_sms();
+      int fit = 0;
       cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
-      ZP_CUDA(cudaOccupancyMaxActiveClusters(&n, kernel, &cfg));
-      pairs.value[dev] = n < sms / 2 ? n : sms / 2;
+      ZP_CUDA(cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg));
+      pairs.value[dev] = fit < sms / 2 ? fit : sms / 2;
       pairs.done[dev] = true;
     }
     max_pairs = pairs.value[dev];
   }
   if (max_pairs < 1) return ZP_ERR_UNSUPPORTED;
-  GemmParams p;
-  fill_params(p, g, BK);
-  // whole 32-column store blocks; each CTA's half of an MN-major tile comes in 64-wide blocks
-  p.BN = pick_bn(g.N, 256, g.b_mn ? 128 : 32);
-  p.num_m = (int)zp_ceil_div(g.M, BM2);
-  p.num_n = (int)zp_ceil_div(g.N, p.BN);
-  const CUtensorMapSwizzle kswz = BK == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
-  CUtensorMap ma, mb;
-  int rc;
-  if (!g.a_mn) rc = make_map(&ma, g.A, g.K, g.M, P, g.lda, g.a_plane, BK, BM, kswz, g.fp16);
-  else rc = make_map(&ma, g.A, g.M, g.K, P, g.lda, g.a_plane, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B, g.fp16);
-  if (rc) return rc;
-  if (!g.b_mn) rc = make_map(&mb, g.B, g.K, g.N, P, g.ldb, g.b_plane, BK, p.BN / 2, kswz, g.fp16);
-  else rc = make_map(&mb, g.B, g.N, g.K, P, g.ldb, g.b_plane, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B, g.fp16);
-  if (rc) return rc;
-  CUtensorMap mc;
-  const int chunks = (int)zp_ceil_div(p.kb_per_split, p.kc);
-  p.tma_store = EPI == ZP_EPI_NONE ? (L::kTmaEpilogue && !(g.absmax_out && chunks > 1))
-                                   : p.epi.store_c;
-  if (p.tma_store) {
-    if ((rc = make_map_c(&mc, g.C, g.N, g.M, p.ksplit, g.ldc, g.split_stride))) return rc;
-  } else {
-    mc = ma;                                      // never read
-  }
-  const int work = p.num_m * p.num_n * p.ksplit;
-  cfg.gridDim = dim3((unsigned)(2 * (work < max_pairs ? work : max_pairs)));
-  ZP_CUDA(cudaLaunchKernelEx(&cfg, kernel, ma, mb, mc, p));
+  GemmGroup grp;
+  if (const int rc = fill_group(grp, g, n, P, BK, BM2, 2, 256)) return rc;
+  cfg.gridDim = dim3((unsigned)(2 * (grp.total < max_pairs ? grp.total : max_pairs)));
+  ZP_CUDA(cudaLaunchKernelEx(&cfg, kernel, grp));
   ZP_LAUNCH_CHECK("gemm_tc_pair_kernel");
   return ZP_OK;
 }
 
 template <int P, int BK, int STAGES>
-int launch_pair(const ZpGemmTc &g, cudaStream_t st) {
-  const int mode = g.epi ? g.epi->mode : ZP_EPI_NONE;
-  if (mode == ZP_EPI_GATE) return launch_pair_e<P, BK, STAGES, ZP_EPI_GATE>(g, st);
-  if (mode == ZP_EPI_ROTATE_BACK) return launch_pair_e<P, BK, STAGES, ZP_EPI_ROTATE_BACK>(g, st);
-  return launch_pair_e<P, BK, STAGES, ZP_EPI_NONE>(g, st);
+int launch_pair(const ZpGemmTc *const *g, int n, cudaStream_t st) {
+  const int mode = g[0]->epi ? g[0]->epi->mode : ZP_EPI_NONE;
+  if (mode == ZP_EPI_GATE) return launch_pair_e<P, BK, STAGES, ZP_EPI_GATE>(g, n, st);
+  if (mode == ZP_EPI_ROTATE_BACK) return launch_pair_e<P, BK, STAGES, ZP_EPI_ROTATE_BACK>(g, n, st);
+  return launch_pair_e<P, BK, STAGES, ZP_EPI_NONE>(g, n, st);
+}
+
+int check_product(const ZpGemmTc &g) {
+  if (g.K <= 0) return ZP_ERR_INVALID_ARG;
+  if (g.fp16 != (g.planes == 2)) return ZP_ERR_UNSUPPORTED;   // fp16 planes come in pairs
+  if (!fused_mode_ok(g, block_k(g))) return ZP_ERR_UNSUPPORTED;
+  if ((g.lda % 8) || (g.ldb % 8) || (g.a_plane % 8) || (g.b_plane % 8) || (g.ldc % 4) ||
+      (g.split_stride % 4))
+    return ZP_ERR_INVALID_ARG;
+  if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B) |
+       reinterpret_cast<uintptr_t>(g.C)) & 15)
+    return ZP_ERR_INVALID_ARG;
+  return ZP_OK;
+}
+
+// the launch for products of one format that all go the same way
+int dispatch(const ZpGemmTc *const *g, int n, bool pair, cudaStream_t st) {
+  const int planes = g[0]->planes;
+  if (pair) return planes == 2 ? launch_pair<2, 64, 3>(g, n, st) : launch_pair<1, 64, 6>(g, n, st);
+  // a contraction of at most four k-blocks is bound by its output stores: fewer operand stages,
+  // two store buffers per epilogue warp
+  const bool store_bound = n == 1 && !g[0]->a_mn && !g[0]->b_mn && !(g[0]->epi && g[0]->epi->mode) &&
+                           g[0]->ksplit <= 1;
+  if (planes == 2) {
+    if (store_bound && g[0]->K <= 128) return launch_e<2, 32, 2, 256, ZP_EPI_NONE, 2>(g, n, st);
+    return launch<2, 32, 4, 256>(g, n, st);
+  }
+  if (planes == 1) {
+    if (store_bound && g[0]->K <= 256) return launch_e<1, 64, 2, 256, ZP_EPI_NONE, 2>(g, n, st);
+    return launch<1, 64, 4, 256>(g, n, st);
+  }
+  // three planes: two stages of six MMA passes each leave room for the store blocks
+  if (planes == 3)
+    return g[0]->variant == 1 ? launch<3, 64, 2, 128>(g, n, st) : launch<3, 32, 2, 256>(g, n, st);
+  return ZP_ERR_UNSUPPORTED;
 }
 
 }  // namespace
@@ -1511,7 +1469,7 @@ int launch_pair(const ZpGemmTc &g, cudaStream_t st) {
 int zp_gemm_tc_splits(const ZpGemmTc &g) {
   if (g.K <= 0) return 1;
   int ksplit, kbs, num_k;
-  split_plan(g, block_k(g), &ksplit, &kbs, &num_k);
+  split_plan(g, 64, &ksplit, &kbs, &num_k);
   return ksplit;
 }
 
@@ -1525,6 +1483,23 @@ int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits) {
     if (score > best_score) { best_score = score; best = s; }
   }
   return best;
+}
+
+// One K split for all products of a group (their contraction is the same): the one whose rounds of
+// work items leave the least of the device idle.
+void zp_gemm_group_splits(ZpGemmTc *g, int n, int max_splits) {
+  const bool pair = use_pair(g[0]);
+  const int64_t units = pair ? device_sms() / 2 : device_sms();
+  int64_t tiles = 0;
+  for (int i = 0; i < n; ++i)
+    tiles += zp_ceil_div(g[i].M, pair ? BM2 : BM) * zp_ceil_div(g[i].N, pick_bn(g[i].N, 256, bn_step(g[i], pair ? 2 : 1)));
+  int best = 1;
+  double best_cost = 1e30;
+  for (int s = 1; s <= max_splits; ++s) {
+    const double cost = (double)zp_ceil_div(tiles * s, units) / s + 0.004 * s;
+    if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  for (int i = 0; i < n; ++i) g[i].ksplit = best;
 }
 
 int zp_launch_block_nodes(int64_t E, int64_t N, const int32_t *row_ptr, int32_t *block_node,
@@ -1543,37 +1518,25 @@ bool zp_gemm_tc_fusable(const ZpGemmTc &g) {
 
 int zp_launch_gemm_tc(const ZpGemmTc &g, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0) return ZP_OK;
-  if (g.K <= 0) return ZP_ERR_INVALID_ARG;
-  if (g.fp16 != (g.planes == 2)) return ZP_ERR_UNSUPPORTED;   // fp16 planes come in pairs
-  if (!fused_mode_ok(g, block_k(g))) return ZP_ERR_UNSUPPORTED;
-  if ((g.lda % 8) || (g.ldb % 8) || (g.a_plane % 8) || (g.b_plane % 8) || (g.ldc % 4) ||
-      (g.split_stride % 4))
-    return ZP_ERR_INVALID_ARG;
-  if ((reinterpret_cast<uintptr_t>(g.A) | reinterpret_cast<uintptr_t>(g.B) |
-       reinterpret_cast<uintptr_t>(g.C)) & 15)
-    return ZP_ERR_INVALID_ARG;
-  if (use_pair(g))
-    return g.planes == 2 ? launch_pair<2, 64, 3>(g, st) : launch_pair<1, 64, 6>(g, st);
-  if (g.a_mn || g.b_mn) {
-    // MN-major tiles are [BK][64] blocks under the 128-byte swizzle
-    if (g.planes == 3)
-      return g.variant == 1 ? launch<3, 64, 2, 128>(g, st) : launch<3, 32, 3, 256>(g, st);
-    if (g.planes == 2) return launch<2, 32, 4, 256>(g, st);
-    if (g.planes == 1) return launch<1, 64, 4, 256>(g, st);
-    return ZP_ERR_UNSUPPORTED;
+  if (const int rc = check_product(g)) return rc;
+  const ZpGemmTc *one = &g;
+  return dispatch(&one, 1, use_pair(g), st);
+}
+
+// Several independent products of one format in one launch.  The CTA-pair kernel takes them when
+// it would take most of the work on its own.
+int zp_launch_gemm_group(const ZpGemmTc *g, int n, cudaStream_t st) {
+  const ZpGemmTc *live[ZP_GEMM_GROUP];
+  int k = 0;
+  double pair_work = 0.0, work = 0.0;
+  for (int i = 0; i < n; ++i) {
+    if (g[i].M <= 0 || g[i].N <= 0) continue;
+    if (const int rc = check_product(g[i])) return rc;
+    if (k == ZP_GEMM_GROUP || (g[i].epi && g[i].epi->mode) || g[i].planes != g[0].planes) return ZP_ERR_INVALID_ARG;
+    const double w = (double)g[i].M * (double)g[i].N * (double)g[i].K;
+    work += w;
+    if (use_pair(g[i])) pair_work += w;
+    live[k++] = &g[i];
   }
-  // a contraction of at most four k-blocks is bound by its output stores: fewer operand stages,
-  // two store buffers per epilogue warp
-  const bool store_bound = !(g.epi && g.epi->mode) && g.ksplit <= 1;
-  if (g.planes == 2) {
-    if (store_bound && g.K <= 128) return launch_e<2, 32, 2, 256, ZP_EPI_NONE, 2>(g, st);
-    return launch<2, 32, 4, 256>(g, st);
-  }
-  if (g.planes == 3)
-    return g.variant == 1 ? launch<3, 64, 2, 128>(g, st) : launch<3, 32, 3, 256>(g, st);
-  if (g.planes == 1) {
-    if (store_bound && g.K <= 256) return launch_e<1, 64, 2, 256, ZP_EPI_NONE, 2>(g, st);
-    return launch<1, 64, 4, 256>(g, st);
-  }
-  return ZP_ERR_UNSUPPORTED;
+  return k ? dispatch(live, k, pair_work > 0.5 * work, st) : ZP_OK;
 }
