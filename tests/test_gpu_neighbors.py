@@ -108,3 +108,17 @@ def test_rejections():
         neighbor_list(torch.rand(10, 3, dtype=torch.float64).cuda(), 10.0, 5.0, 1000)
     with pytest.raises(_lib.ZpError):
         neighbor_list(torch.rand(10, 3, dtype=torch.float64).cuda(), 0.1, 5.0, 30)   # reach > 8
+
+
+@pytest.mark.parametrize("jitter", [0.0, 1e-3])
+@pytest.mark.parametrize("atoms", [2, 33, 128, 129, 130, 216])
+@pytest.mark.parametrize("cap", [None, 1, 31, 127, 128])
+def test_selection_at_its_edges(atoms, cap, jitter):
+    """Every atom has atoms - 1 neighbours: around the 128 hits that fit a warp's registers, with
+    equal distances at the cap (a lattice) and without."""
+    g = np.random.default_rng(3)
+    site = np.stack(np.meshgrid(*[np.arange(6)] * 3, indexing="ij"), -1).reshape(-1, 3)
+    pos = 9.0 + 0.5 * g.permutation(site)[:atoms] + jitter * g.standard_normal((atoms, 3))
+    from oracle import neighbors_oracle as no
+    for a, b in zip(run(pos, 20.0, 6.0, cap), no.neighbor_list(pos, 20.0, 6.0, cap)):
+        assert a.shape == b.shape and np.array_equal(a, b)

@@ -239,8 +239,8 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
     smallest by (d2, src, shift) kept.
     ``pos``: CUDA tensor [N, 3] (computed in float64).  Returns (edge_index [2, E] int64,
     shifts [E, 3] float64, row_ptr [N + 1] int32) in (dst, src, shift) order, which is already the
-    destination-sorted form the kernels consume.  One host read (the edge count) in between the
-    two passes."""
+    destination-sorted form the kernels consume.  One host read (edge count and flags) in between
+    the two passes, one of the flags at the end."""
     if not pos.is_cuda:
         raise RuntimeError("neighbor_list needs a CUDA tensor: there is no CPU path")
     lib = _lib.load()
@@ -252,14 +252,14 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
         raise _lib.ZpError(1, "zp_neighbors_work_bytes")
     dev = p.device
     work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    row_ptr = torch.empty(n + 1, dtype=torch.int32, device=dev)
-    flags = torch.zeros(1, dtype=torch.int32, device=dev)
+    out = torch.empty(n + 2, dtype=torch.int32, device=dev)       # row_ptr and, read with its end, flags
+    row_ptr, flags = out[:n + 1], out[n + 1:]
     with torch.cuda.device(dev):
         st = torch.cuda.current_stream().cuda_stream
         _lib.check(lib.zp_neighbors_count(p.data_ptr(), n, float(box), float(cutoff), cap,
                                           row_ptr.data_ptr(), flags.data_ptr(), work.data_ptr(),
                                           nbytes, st), "zp_neighbors_count")
-        e, fl = int(row_ptr[n].item()), int(flags.item())
+        e, fl = out[n:].tolist()
         if fl & 1:
             raise ValueError("neighbor_list: positions must be finite")
         if fl & 2:
@@ -271,8 +271,9 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
                                          row_ptr.data_ptr(), e, edge_index.data_ptr(),
                                          shifts.data_ptr(), flags.data_ptr(), work.data_ptr(),
                                          nbytes, st), "zp_neighbors_fill")
-        if int(flags.item()):
-            raise RuntimeError(f"zp_neighbors_fill: device flags {int(flags.item())}")
+        fl = int(flags.item())
+        if fl:
+            raise RuntimeError(f"zp_neighbors_fill: device flags {fl}")
     return edge_index, shifts, row_ptr
 
 
