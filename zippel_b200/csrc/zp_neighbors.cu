@@ -13,16 +13,17 @@
 // and of total orders without ties, so the arrays are reproducible bit for bit and equal to the
 // host statement of the same rule.
 //
-// Method: uniform cells of edge >= cutoff / w (w = 1 unless the box is smaller than the cutoff);
-// one warp per destination walks the (2w+1)^3 cells around it in unwrapped cell coordinates; the
+// Method: uniform cells of edge >= cutoff / w (w = 2, or 1 where atoms are sparse, or more where
+// the box is smaller than the cutoff); one warp per destination walks the (2w+1)^2 columns of cells
+// around it in unwrapped cell coordinates, each cut to the stretch that the cutoff can reach; the
 // unwrapped coordinate gives both the wrapped cell and the periodic image, so every
-// (source, image) pair is visited exactly once.  The atoms are copied in cell order with their own
-// image numbers, so the walk reads them with whole-line loads and divides nothing, and the cells
-// of a walk are laid end to end so that no lane waits at a cell's end.  Pass 1 counts, a scan gives
-// row_ptr, pass 2 collects the hits and, when the cap binds, selects the nearest: up to 128 hits
-// in registers by bisecting the distance until it parts off exactly `cap` of them (ranking all
-// when equal distances stand in the way), more by a bitonic sort on (d2, src, image) in shared
-// memory.  The survivors are placed by counting the smaller (src, image) keys.
+// (source, image) pair is visited at most once.  The atoms are copied in cell order with their own
+// image numbers, so the walk reads them with whole-line loads and divides nothing, and the
+// columns of a walk are laid end to end so that no lane waits at a column's end.  Pass 1 counts
+// (up to the cap), a scan gives row_ptr, pass 2 collects the hits and, when the cap binds, selects
+// the nearest: up to 128 hits by closing in on a distance that parts off exactly `cap` of them
+// (ranking all when equal distances stand in the way), more by a bitonic sort on (d2, src, image) in
+// shared memory.  The survivors are placed by counting the smaller (src, image) keys.
 #include <algorithm>
 #include <cmath>
 
@@ -41,6 +42,7 @@ struct Grid {
   int nc;          // cells per dimension
   int w;           // search half-width in cells
   int reach;       // largest |image| component that can occur
+  float reach2;    // (cutoff / cell)^2 and a margin for working in fp32
 };
 
 struct Hit {
@@ -56,10 +58,12 @@ __device__ __forceinline__ bool hit_less(const Hit &a, const Hit &b) {
 // p - o * box its wrapped coordinate, used only to pick the cell.  Distances are always taken
 // between the positions as given.
 __device__ __forceinline__ int own_image(double p, const Grid &g) { return (int)floor(p / g.box); }
-__device__ __forceinline__ int cell_coord(double p, const Grid &g) {
-  const double pw = p - floor(p / g.box) * g.box;
-  int c = (int)floor(pw / g.cell);
+__device__ __forceinline__ int clamp_cell(double p, const Grid &g) {
+  const int c = (int)floor(p);
   return c < 0 ? 0 : (c >= g.nc ? g.nc - 1 : c);
+}
+__device__ __forceinline__ int cell_coord(double p, const Grid &g) {
+  return clamp_cell((p - floor(p / g.box) * g.box) / g.cell, g);
 }
 
 __device__ __forceinline__ int floor_div(int a, int n) {
@@ -78,8 +82,8 @@ __device__ __forceinline__ unsigned image_code(int nkx, int nky, int nkz, int re
 }
 
 __global__ void cell_count_kernel(int64_t N, const double *__restrict__ pos, Grid g,
-                                  int32_t *__restrict__ atom_cell, int32_t *cell_count,
-                                  int32_t *flags) {
+                                  int32_t *__restrict__ atom_cell, int4 *__restrict__ own,
+                                  int32_t *cell_count, int32_t *flags) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
@@ -88,6 +92,7 @@ __global__ void cell_count_kernel(int64_t N, const double *__restrict__ pos, Gri
     atomicOr(flags, 1);                               // not finite, or absurdly far from the box
   const int c = (cell_coord(x, g) * g.nc + cell_coord(y, g)) * g.nc + cell_coord(z, g);
   atom_cell[i] = c;
+  own[i] = make_int4(own_image(x, g), own_image(y, g), own_image(z, g), (int)i);
   atomicAdd(&cell_count[c], 1);
 }
 
@@ -98,17 +103,16 @@ struct Sorted {
 };
 __global__ void cell_fill_kernel(int64_t N, const double *__restrict__ pos, Grid g,
                                  const int32_t *__restrict__ atom_cell,
-                                 const int32_t *__restrict__ cell_start, int32_t *cell_cursor,
+                                 const int4 *__restrict__ own, const int32_t *__restrict__ cell_start, int32_t *cell_cursor,
                                  const Sorted out) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const int c = atom_cell[i];
   const int at = cell_start[c] + atomicAdd(&cell_cursor[c], 1);
-  const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
-  out.x[at] = x;
-  out.y[at] = y;
-  out.z[at] = z;
-  out.who[at] = make_int4(own_image(x, g), own_image(y, g), own_image(z, g), (int)i);
+  out.x[at] = pos[3 * i];
+  out.y[at] = pos[3 * i + 1];
+  out.z[at] = pos[3 * i + 2];
+  out.who[at] = own[i];
 }
 
 // exclusive scan of n ints (n + 1 outputs, the last is the total): block scans, serial scan of
@@ -158,86 +162,100 @@ int exclusive_scan(int64_t n, const int32_t *in, int32_t *out, int32_t *block_su
 
 // Calls f(hit, src, -kx, -ky, -kz, d2) on all 32 lanes together for every batch of candidate
 // (source, image) pairs around destination j; `hit` marks the lanes whose candidate lies within
-// the cutoff, k is its image in wrapped coordinates.
+// the cutoff, k is its image in wrapped coordinates.  The walk goes on while f returns true (the
+// same on all lanes).
 template <typename F>
-__device__ __forceinline__ void for_each_hit(const Grid &g, const double *__restrict__ pos,
-                                             const int32_t *__restrict__ cell_start,
-                                             const Sorted &atoms, int64_t j, int lane, F &&f) {
-  const double xj = pos[3 * j], yj = pos[3 * j + 1], zj = pos[3 * j + 2];
-  const int cx = cell_coord(xj, g), cy = cell_coord(yj, g), cz = cell_coord(zj, g);
-  const int ojx = own_image(xj, g), ojy = own_image(yj, g), ojz = own_image(zj, g);
-  const int side = 2 * g.w + 1, cells = side * side * side;
-  for (int q0 = 0; q0 < cells; q0 += 32) {
-    // a lane per cell: where its atoms stand, and its image
+__device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__restrict__ cell_start,
+                                             const Sorted &atoms, int64_t at, int lane, F &&f) {
+  const double xj = atoms.x[at], yj = atoms.y[at], zj = atoms.z[at];
+  const int4 own = atoms.who[at];
+  // cell, and where in it (in cells)
+  const double wx = (xj - own.x * g.box) / g.cell, wy = (yj - own.y * g.box) / g.cell,
+               wz = (zj - own.z * g.box) / g.cell;
+  const int cx = clamp_cell(wx, g), cy = clamp_cell(wy, g), cz = clamp_cell(wz, g);
+  const float fx = (float)(wx - cx), fy = (float)(wy - cy), fz = (float)(wz - cz);
+  const int side = 2 * g.w + 1, columns = side * side;
+  const int kz1 = floor_div(cz + g.w, g.nc);
+  for (int q0 = 0; q0 < columns; q0 += 32) {
+    // a lane per column of cells along z, cut to what the cutoff can reach
     const int q = q0 + lane;
-    int off = 0, len = 0, image = 0;
-    if (q < cells) {
-      const int ux = cx - g.w + q / (side * side), uy = cy - g.w + q / side % side, uz = cz - g.w + q % side;
-      const int kx = floor_div(ux, g.nc), ky = floor_div(uy, g.nc), kz = floor_div(uz, g.nc);
-      const int c = ((ux - kx * g.nc) * g.nc + (uy - ky * g.nc)) * g.nc + (uz - kz * g.nc);
-      off = cell_start[c];
-      len = cell_start[c + 1] - off;
-      image = (kx + 512) | (ky + 512) << 10 | (kz + 512) << 20;
-    }
-    int upto = len;                              // candidates of the cells up to this one
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto += u;
-    }
-    const int total = __shfl_sync(0xffffffffu, upto, 31);
-    off -= upto - len;
-    for (int t0 = 0; t0 < total; t0 += 32) {
-      const int t = t0 + lane;
-      int cell = 0;                              // the cell candidate t belongs to
-#pragma unroll
-      for (int b = 16; b > 0; b >>= 1) {
-        const int v = __shfl_sync(0xffffffffu, upto, cell + b - 1);
-        if (v <= t) cell += b;
+    const int ox = q / side - g.w, oy = q % side - g.w;
+    const float ax = ox > 0 ? ox - fx : ox < 0 ? fx - (ox + 1) : 0.f;
+    const float ay = oy > 0 ? oy - fy : oy < 0 ? fy - (oy + 1) : 0.f;
+    const float r2 = g.reach2 - (ax * ax + ay * ay);
+    const bool in = q < columns && r2 > 0.f;
+    const float r = in ? sqrtf(r2) : 0.f;
+    const int u0 = max(cz - g.w, cz + (int)floorf(fz - r)), u1 = min(cz + g.w, cz + (int)floorf(fz + r));
+    const int kx = floor_div(cx + ox, g.nc), ky = floor_div(cy + oy, g.nc);
+    const int column = ((cx + ox - kx * g.nc) * g.nc + (cy + oy - ky * g.nc)) * g.nc;
+    for (int kz = floor_div(cz - g.w, g.nc); kz <= kz1; ++kz) {
+      const int z0 = max(u0 - kz * g.nc, 0), z1 = min(u1 - kz * g.nc, g.nc - 1);
+      int off = 0, len = 0;
+      const int image = (kx + 512) | (ky + 512) << 10 | (kz + 512) << 20;
+      if (in && z0 <= z1) {
+        off = cell_start[column + z0];
+        len = cell_start[column + z1 + 1] - off;
       }
-      const int a = __shfl_sync(0xffffffffu, off, cell) + t;
-      const int im = __shfl_sync(0xffffffffu, image, cell);
-      bool hit = false;
-      int i = 0, nkx = 0, nky = 0, nkz = 0;
-      double d2 = 0.0;
-      if (t < total) {
-        const int4 who = atoms.who[a];
-        i = who.w;
-        nkx = 512 - (im & 1023);
-        nky = 512 - (im >> 10 & 1023);
-        nkz = 512 - (im >> 20 & 1023);
-        // the source's wrapped copy sits k boxes away in wrapped coordinates:
-        // pos[j] - (pos[i] - o_i box + k box) stays as (pos[j] - pos[i]) + (o_i - o_j - k) box
-        // once the destination's own offset o_j is taken out of the search origin
-        const int mx = who.x - ojx + nkx, my = who.y - ojy + nky, mz = who.z - ojz + nkz;
-        const double dx = __dadd_rn(__dsub_rn(xj, atoms.x[a]), __dmul_rn((double)mx, g.box));
-        const double dy = __dadd_rn(__dsub_rn(yj, atoms.y[a]), __dmul_rn((double)my, g.box));
-        const double dz = __dadd_rn(__dsub_rn(zj, atoms.z[a]), __dmul_rn((double)mz, g.box));
-        d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-        hit = d2 < g.cutoff2 && !(i == j && mx == 0 && my == 0 && mz == 0);
+      int upto = len;                              // candidates of the columns up to this one
+  #pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += u;
       }
-      f(hit, i, nkx, nky, nkz, d2);
+      const int total = __shfl_sync(0xffffffffu, upto, 31);
+      off -= upto - len;
+      for (int t0 = 0; t0 < total; t0 += 32) {
+        const int t = t0 + lane;
+        int cell = 0;                              // the column candidate t belongs to
+  #pragma unroll
+        for (int b = 16; b > 0; b >>= 1) {
+          const int v = __shfl_sync(0xffffffffu, upto, cell + b - 1);
+          if (v <= t) cell += b;
+        }
+        const int a = __shfl_sync(0xffffffffu, off, cell) + t;
+        const int im = __shfl_sync(0xffffffffu, image, cell);
+        bool hit = false;
+        int i = 0, nkx = 0, nky = 0, nkz = 0;
+        double d2 = 0.0;
+        if (t < total) {
+          const int4 who = atoms.who[a];
+          i = who.w;
+          nkx = 512 - (im & 1023);
+          nky = 512 - (im >> 10 & 1023);
+          nkz = 512 - (im >> 20 & 1023);
+          // the source's wrapped copy sits k boxes away in wrapped coordinates:
+          // pos[j] - (pos[i] - o_i box + k box) stays as (pos[j] - pos[i]) + (o_i - o_j - k) box
+          // once the destination's own offset o_j is taken out of the search origin
+          const int mx = who.x - own.x + nkx, my = who.y - own.y + nky, mz = who.z - own.z + nkz;
+          const double dx = __dadd_rn(__dsub_rn(xj, atoms.x[a]), __dmul_rn((double)mx, g.box));
+          const double dy = __dadd_rn(__dsub_rn(yj, atoms.y[a]), __dmul_rn((double)my, g.box));
+          const double dz = __dadd_rn(__dsub_rn(zj, atoms.z[a]), __dmul_rn((double)mz, g.box));
+          d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+          hit = d2 < g.cutoff2 && !(i == own.w && mx == 0 && my == 0 && mz == 0);
+        }
+        if (!f(hit, i, nkx, nky, nkz, d2)) return;
+      }
     }
   }
 }
 
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-count_kernel(int64_t N, const double *__restrict__ pos, Grid g,
+count_kernel(int64_t N, Grid g,
              const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
-             int32_t *__restrict__ counts, int32_t *flags, int32_t *__restrict__ crowded) {
+             int32_t *__restrict__ counts, int32_t *flags) {
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t at = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
   if (at >= N) return;
   const int64_t j = atoms.who[at].w;           // in cell order: neighbours read the same cells
   int n = 0;
-  for_each_hit(g, pos, cell_start, atoms, j, lane,
+  for_each_hit(g, cell_start, atoms, at, lane,
                [&](bool hit, int, int, int, int, double) {
                  n += __popc(__ballot_sync(0xffffffffu, hit));
+                 return cap <= 0 || n < cap;             // past the cap the count is known
                });
   if (lane == 0) {
     if (cap <= 0 && n > kHitCap) atomicOr(flags, 2);       // uncapped list too long for pass 2
     counts[j] = cap > 0 && n > cap ? cap : n;
-    if (n > kFewHits) crowded[1 + atomicAdd(&crowded[0], 1)] = (int32_t)j;
   }
 }
 
@@ -267,39 +285,36 @@ __device__ __forceinline__ int pow2_at_least(int n) {
 
 // Writes the edges of destination j: survivor `tie` at place `rank` of its list.
 struct Writer {
-  const double *pos;
+  const int4 *own;
   const Grid &g;
   int64_t E, j, base;
   int64_t *edge_index;
   double *shifts;
-  int ojx, ojy, ojz;
-  __device__ Writer(const double *p, const Grid &grid, int64_t n_edges, int64_t dst, int64_t first,
-                    int64_t *edges, double *sh)
-      : pos(p), g(grid), E(n_edges), j(dst), base(first), edge_index(edges), shifts(sh),
-        ojx(own_image(p[3 * dst], grid)), ojy(own_image(p[3 * dst + 1], grid)),
-        ojz(own_image(p[3 * dst + 2], grid)) {}
   __device__ __forceinline__ void put(unsigned long long tie, int rank) const {
     const unsigned s = 2u * g.reach + 1u;
     const unsigned code = (unsigned)(tie & 0xffffffffu);
     const int64_t i = (int64_t)(tie >> 32);
     const int nkz = (int)(code % s) - g.reach, nky = (int)((code / s) % s) - g.reach,
               nkx = (int)(code / (s * s)) - g.reach;
+    const int4 a = own[i], b = own[j];
     edge_index[base + rank] = i;
     edge_index[E + base + rank] = j;
-    shifts[3 * (base + rank)] = (double)(own_image(pos[3 * i], g) - ojx + nkx) * g.box;
-    shifts[3 * (base + rank) + 1] = (double)(own_image(pos[3 * i + 1], g) - ojy + nky) * g.box;
-    shifts[3 * (base + rank) + 2] = (double)(own_image(pos[3 * i + 2], g) - ojz + nkz) * g.box;
+    shifts[3 * (base + rank)] = (double)(a.x - b.x + nkx) * g.box;
+    shifts[3 * (base + rank) + 1] = (double)(a.y - b.y + nky) * g.box;
+    shifts[3 * (base + rank) + 2] = (double)(a.z - b.z + nkz) * g.box;
   }
 };
 
-// Destinations with at most kFewHits hits.  The hits are compacted through 2 KB of shared memory per
-// warp and then live in registers, four per lane.
+// Destinations with at most kFewHits hits, compacted in 2 KB of shared memory per warp so that an
+// SM holds its full count of warps; the others go on the list `crowded`.  Bound by instruction issue
+// (a third of it the walk); 100 000 atoms, 90 hits, cap 30: 240 us, where two bitonic sorts in 64 KB
+// of shared memory per four warps took 3400.
 constexpr int kFillWarps = 8;
 __global__ void __launch_bounds__(32 * kFillWarps)
-fill_few_kernel(int64_t N, const double *__restrict__ pos, Grid g,
+fill_few_kernel(int64_t N, const int4 *__restrict__ own, Grid g,
                 const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
                 const int32_t *__restrict__ row_ptr, int64_t E, int64_t *__restrict__ edge_index,
-                double *__restrict__ shifts, int32_t *flags) {
+                double *__restrict__ shifts, int32_t *flags, int32_t *__restrict__ crowded) {
   __shared__ Hit hits[kFillWarps][kFewHits];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t at = (int64_t)blockIdx.x * kFillWarps + warp;
@@ -307,7 +322,7 @@ fill_few_kernel(int64_t N, const double *__restrict__ pos, Grid g,
   const int64_t j = atoms.who[at].w;
   Hit *h = hits[warp];
   int n = 0;                      // hits seen (warp-uniform)
-  for_each_hit(g, pos, cell_start, atoms, j, lane,
+  for_each_hit(g, cell_start, atoms, at, lane,
                [&](bool hit, int i, int nkx, int nky, int nkz, double d2) {
                  const unsigned m = __ballot_sync(0xffffffffu, hit);
                  const int slot = n + __popc(m & ((1u << lane) - 1u));
@@ -316,81 +331,80 @@ fill_few_kernel(int64_t N, const double *__restrict__ pos, Grid g,
                    h[slot].tie = ((unsigned long long)(unsigned)i << 32) | image_code(nkx, nky, nkz, g.reach);
                  }
                  n += __popc(m);
+                 return n <= kFewHits;
                });
-  if (n > kFewHits) return;       // left to fill_many_kernel
-  __syncwarp();
-  constexpr int R = kFewHits / 32;
-  double d2[R];
-  unsigned long long tie[R];
-  unsigned alive = 0;             // which of this lane's hits survive
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    const int t = lane + 32 * k;
-    d2[k] = t < n ? h[t].d2 : INFINITY;
-    tie[k] = t < n ? h[t].tie : ~0ull;
-    if (t < n) alive |= 1u << k;
+  if (n > kFewHits) {             // left to fill_many_kernel
+    if (lane == 0) crowded[1 + atomicAdd(&crowded[0], 1)] = (int32_t)at;
+    return;
   }
+  __syncwarp();
   if (cap > 0 && n > cap) {
-    // bisect the distance; every step counts the hits up to the middle
-    double lo = 0.0, hi = g.cutoff2;
+    constexpr int R = kFewHits / 32;
+    float near[R];                // rounding to fp32 keeps the order, or makes equals
+#pragma unroll
+    for (int k = 0; k < R; ++k) near[k] = lane + 32 * k < n ? (float)h[lane + 32 * k].d2 : INFINITY;
+    // close in on a distance that exactly `cap` hits do not exceed: by interpolation and by halves
+    float lo = 0.f, hi = (float)g.cutoff2;
+    int below_lo = 0, below_hi = n;
+    unsigned alive[R];            // survivors, a bit per lane
     bool found = false;
-    for (int step = 0; step < 40 && !found; ++step) {
-      const double mid = 0.5 * (lo + hi);
+    for (int step = 0; step < 32 && !found; ++step) {
+      const float part = step & 1 ? 0.5f : (cap - below_lo) / (float)(below_hi - below_lo);
+      const float mid = lo + (hi - lo) * part;
       int below = 0;
 #pragma unroll
-      for (int k = 0; k < R; ++k) below += __popc(__ballot_sync(0xffffffffu, d2[k] <= mid));
-      if (below == cap) {
-        found = true;
-#pragma unroll
-        for (int k = 0; k < R; ++k)
-          if (!(d2[k] <= mid)) alive &= ~(1u << k);
-      } else if (below < cap) {
+      for (int k = 0; k < R; ++k) {
+        alive[k] = __ballot_sync(0xffffffffu, near[k] <= mid);
+        below += __popc(alive[k]);
+      }
+      found = below == cap;
+      if (below < cap) {
         lo = mid;
+        below_lo = below;
       } else {
         hi = mid;
+        below_hi = below;
       }
     }
     if (!found) {                 // equal distances at the cap: rank by (d2, src, image)
-      int rank[R];
-#pragma unroll
-      for (int k = 0; k < R; ++k) rank[k] = 0;
-      for (int t = 0; t < n; ++t) {
-        const Hit o = h[t];
-#pragma unroll
-        for (int k = 0; k < R; ++k) rank[k] += o.d2 < d2[k] || (o.d2 == d2[k] && o.tie < tie[k]);
+      for (int k = 0; k < R; ++k) {
+        const int own_t = lane + 32 * k;
+        const Hit mine = h[own_t < n ? own_t : 0];
+        int rank = 0;
+        for (int t = 0; t < n; ++t) rank += hit_less(h[t], mine);
+        alive[k] = __ballot_sync(0xffffffffu, own_t < n && rank < cap);
       }
-#pragma unroll
-      for (int k = 0; k < R; ++k)
-        if (rank[k] >= cap) alive &= ~(1u << k);
     }
+    // survivors to the front
+    unsigned long long tie[R];
+#pragma unroll
+    for (int k = 0; k < R; ++k) tie[k] = h[lane + 32 * k].tie;
+    __syncwarp();
+    int slot = 0;
+#pragma unroll
+    for (int k = 0; k < R; ++k) {
+      if (alive[k] >> lane & 1) h[slot + __popc(alive[k] & ((1u << lane) - 1u))].tie = tie[k];
+      slot += __popc(alive[k]);
+    }
+    __syncwarp();
     n = cap;
-  }
-  // place of a survivor = number of survivors with a smaller (src, image)
-  int rank[R];
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    rank[k] = 0;
-    if (!(alive >> k & 1)) tie[k] = ~0ull;
-  }
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    for (unsigned m = __ballot_sync(0xffffffffu, alive >> k & 1); m; m &= m - 1) {
-      const unsigned long long o = __shfl_sync(0xffffffffu, tie[k], __ffs(m) - 1);
-#pragma unroll
-      for (int q = 0; q < R; ++q) rank[q] += o < tie[q];
-    }
   }
   const int64_t base = row_ptr[j];
   if (lane == 0 && row_ptr[j + 1] - base != n) atomicOr(flags, 4);     // passes disagree
-  const Writer out(pos, g, E, j, base, edge_index, shifts);
-#pragma unroll
-  for (int k = 0; k < R; ++k)
-    if (alive >> k & 1) out.put(tie[k], rank[k]);
+  const Writer out{own, g, E, j, base, edge_index, shifts};
+  // place of a survivor = number of survivors with a smaller (src, image)
+  for (int t = lane; t < n; t += 32) {
+    const unsigned long long mine = h[t].tie;
+    int rank = 0;
+#pragma unroll 4
+    for (int q = 0; q < n; ++q) rank += h[q].tie < mine;
+    out.put(mine, rank);
+  }
 }
 
 // The destinations listed in `crowded` (more than kFewHits hits).
 __global__ void __launch_bounds__(32 * kWarpsPerBlock)
-fill_many_kernel(const int32_t *__restrict__ crowded, const double *__restrict__ pos, Grid g,
+fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ own, Grid g,
                  const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
                  const int32_t *__restrict__ row_ptr, int64_t E, int64_t *__restrict__ edge_index,
                  double *__restrict__ shifts, int32_t *flags) {
@@ -398,11 +412,11 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const double *__restrict__
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   Hit *h = reinterpret_cast<Hit *>(smem_raw) + (size_t)warp * kHitCap;
   for (int c = blockIdx.x * kWarpsPerBlock + warp; c < crowded[0]; c += gridDim.x * kWarpsPerBlock) {
-    const int64_t j = crowded[1 + c];
+    const int64_t at = crowded[1 + c], j = atoms.who[at].w;
     const Hit inf{INFINITY, ~0ull};
     int n = 0;                      // hits held (warp-uniform)
     bool overflow = false;
-    for_each_hit(g, pos, cell_start, atoms, j, lane,
+    for_each_hit(g, cell_start, atoms, at, lane,
                  [&](bool hit, int i, int nkx, int nky, int nkz, double d2) {
                    const unsigned m = __ballot_sync(0xffffffffu, hit);
                    const int add = __popc(m);
@@ -425,6 +439,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const double *__restrict__
                    }
                    if (!overflow) n += add;
                    __syncwarp();
+                   return !overflow;
                  });
     if (overflow) {
       if (lane == 0) atomicOr(flags, 2);
@@ -446,7 +461,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const double *__restrict__
     }
     const int64_t base = row_ptr[j];
     if (lane == 0 && row_ptr[j + 1] - base != n) atomicOr(flags, 4);     // passes disagree
-    const Writer out(pos, g, E, j, base, edge_index, shifts);
+    const Writer out{own, g, E, j, base, edge_index, shifts};
     for (int t = lane; t < n; t += 32) out.put(h[t].tie, t);
     __syncwarp();
   }
@@ -455,23 +470,29 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const double *__restrict__
 struct NbWork {
   int32_t *flags, *cell_count, *cell_start, *cell_cursor, *atom_cell, *counts, *crowded,
       *block_sums;
+  int4 *own;       // own image and index of each atom
   Sorted atoms;
   size_t bytes;
 };
 
-int make_grid(double box, double cutoff, Grid *g) {
+int make_grid(int64_t N, double box, double cutoff, Grid *g) {
   if (!(box > 0.0) || !(cutoff > 0.0) || !std::isfinite(box) || !std::isfinite(cutoff))
     return ZP_ERR_INVALID_ARG;
-  // cells a hair wider than the cutoff, so that a last-bit rounding of a cell coordinate can
-  // never put a pair within the cutoff more than w cells apart
-  int nc = (int)std::floor(box / (cutoff * (1.0 + 1e-9)));
+  // Cells a hair wider than the cutoff, so that a last-bit rounding of a cell coordinate can
+  // never put a pair within the cutoff more than w cells apart.  Half-cutoff cells leave 2.4 times
+  // as few candidates outside the sphere and still give a warp one column per lane (25); they
+  // are taken when they are no more than the atoms, so that clearing and scanning them is cheap.
+  const double wide = cutoff * (1.0 + 1e-9);
+  int nc = (int)std::floor(box / (0.5 * wide));
+  if (nc < 1 || nc > 256 || (int64_t)nc * nc * nc > N) nc = (int)std::floor(box / wide);
   if (nc < 1) nc = 1;
   if (nc > 256) nc = 256;
   g->box = box;
   g->nc = nc;
   g->cell = box / nc;
   g->cutoff2 = cutoff * cutoff;
-  g->w = (int)std::ceil(cutoff * (1.0 + 1e-9) / g->cell);
+  g->reach2 = (float)(1.0001 * (cutoff / g->cell) * (cutoff / g->cell));
+  g->w = (int)std::ceil(wide / g->cell);
   if (g->w < 1) g->w = 1;
   g->reach = (int)std::ceil(cutoff / box);
   if (g->reach < 1) g->reach = 1;
@@ -490,11 +511,12 @@ NbWork carve_nb(int64_t N, const Grid &g, void *base) {
   };
   const size_t cells = (size_t)g.nc * g.nc * g.nc;
   w.flags = take((size_t)N + 4);
-  w.crowded = w.flags + 3;                 // how many, then which: cleared with the flags
+  w.crowded = w.flags + 3;                 // how many, then which
   w.cell_count = take(cells + 1);
   w.cell_cursor = take(cells + 1);
   w.cell_start = take(cells + 1);
   w.atom_cell = take((size_t)N);
+  w.own = reinterpret_cast<int4 *>(take((size_t)4 * N));
   w.atoms.x = reinterpret_cast<double *>(take((size_t)2 * N));
   w.atoms.y = reinterpret_cast<double *>(take((size_t)2 * N));
   w.atoms.z = reinterpret_cast<double *>(take((size_t)2 * N));
@@ -511,7 +533,7 @@ extern "C" {
 
 size_t zp_neighbors_work_bytes(int64_t n_atoms, double box, double cutoff) {
   Grid g;
-  if (n_atoms < 0 || make_grid(box, cutoff, &g)) return 0;
+  if (n_atoms < 0 || make_grid(n_atoms, box, cutoff, &g)) return 0;
   return carve_nb(n_atoms, g, nullptr).bytes;
 }
 
@@ -519,7 +541,7 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
                        int32_t *row_ptr, int32_t *flags_out, void *work, size_t work_bytes,
                        void *stream) {
   Grid g;
-  int rc = make_grid(box, cutoff, &g);
+  int rc = make_grid(N, box, cutoff, &g);
   if (rc) return rc;
   if (N < 0 || N > 2000000000ll || !row_ptr || !flags_out || !work || (N && !pos))
     return ZP_ERR_INVALID_ARG;
@@ -531,17 +553,17 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
   ZP_CUDA(cudaMemsetAsync(w.flags, 0, 4 * sizeof(int32_t), st));
   ZP_CUDA(cudaMemsetAsync(w.cell_count, 0, (w.cell_start - w.cell_count) * sizeof(int32_t), st));
   if (N > 0) {
-    cell_count_kernel<<<(unsigned)zp_ceil_div(N, 256), 256, 0, st>>>(N, pos, g, w.atom_cell,
+    cell_count_kernel<<<(unsigned)zp_ceil_div(N, 256), 256, 0, st>>>(N, pos, g, w.atom_cell, w.own,
                                                                      w.cell_count, w.flags);
     ZP_LAUNCH_CHECK("cell_count_kernel");
   }
   if ((rc = exclusive_scan((int64_t)cells, w.cell_count, w.cell_start, w.block_sums, st))) return rc;
   if (N > 0) {
-    cell_fill_kernel<<<(unsigned)zp_ceil_div(N, 256), 256, 0, st>>>(N, pos, g, w.atom_cell,
+    cell_fill_kernel<<<(unsigned)zp_ceil_div(N, 256), 256, 0, st>>>(N, pos, g, w.atom_cell, w.own,
                                                                     w.cell_start, w.cell_cursor, w.atoms);
     ZP_LAUNCH_CHECK("cell_fill_kernel");
     count_kernel<<<(unsigned)zp_ceil_div(N, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st>>>(
-        N, pos, g, w.cell_start, w.atoms, max_neighbors, w.counts, w.flags, w.crowded);
+        N, g, w.cell_start, w.atoms, max_neighbors, w.counts, w.flags);
     ZP_LAUNCH_CHECK("count_kernel");
   }
   if ((rc = exclusive_scan(N, w.counts, row_ptr, w.block_sums, st))) return rc;
@@ -553,7 +575,7 @@ int zp_neighbors_fill(const double *pos, int64_t N, double box, double cutoff, i
                       const int32_t *row_ptr, int64_t E, int64_t *edge_index, double *shifts,
                       int32_t *flags_out, void *work, size_t work_bytes, void *stream) {
   Grid g;
-  int rc = make_grid(box, cutoff, &g);
+  int rc = make_grid(N, box, cutoff, &g);
   if (rc) return rc;
   if (N < 0 || E < 0 || !row_ptr || !flags_out || !work || (N && !pos) ||
       (E && (!edge_index || !shifts)))
@@ -562,15 +584,17 @@ int zp_neighbors_fill(const double *pos, int64_t N, double box, double cutoff, i
   const NbWork w = carve_nb(N, g, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
+  ZP_CUDA(cudaMemsetAsync(w.crowded, 0, sizeof(int32_t), st));
   if (N > 0) {
     fill_few_kernel<<<(unsigned)zp_ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st>>>(
-        N, pos, g, w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags);
+        N, w.own, g, w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags,
+        w.crowded);
     ZP_LAUNCH_CHECK("fill_few_kernel");
     const size_t smem = sizeof(Hit) * kHitCap * kWarpsPerBlock;
     static ZpSmemOptIn opt_in;
     if (int rc_ = zp_ensure_smem(fill_many_kernel, smem, opt_in)) return rc_;
     const unsigned blocks = (unsigned)std::min<int64_t>(zp_ceil_div(N, kWarpsPerBlock), 148 * 3);
-    fill_many_kernel<<<blocks, 32 * kWarpsPerBlock, smem, st>>>(w.crowded, pos, g, w.cell_start, w.atoms,
+    fill_many_kernel<<<blocks, 32 * kWarpsPerBlock, smem, st>>>(w.crowded, w.own, g, w.cell_start, w.atoms,
                                                                 max_neighbors, row_ptr, E, edge_index,
                                                                 shifts, w.flags);
     ZP_LAUNCH_CHECK("fill_many_kernel");
