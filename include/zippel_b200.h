@@ -107,13 +107,14 @@ int zp_csr_build(const int64_t *edge_index /* [2,E] int64: row 0 src, row 1 dst 
 
 /* zp_csr_build that also range-checks the element numbers [n_nodes] against [0, n_elements) and
  * copies the flags to host memory (page-locked, valid once the stream has got there) instead of
- * being asked for them: bit 0 a node index out of range, bit 1 an element number.  A caller can
- * so enqueue the work that follows and look at the flags afterwards, without draining the device. */
+ * being asked for them: bit 0 a node index out of range, bit 1 an element number.  `done` (a
+ * cudaEvent_t, or NULL) is recorded behind the copy.  A caller can so enqueue the work that follows
+ * and look at the flags afterwards, without draining the device.                                */
 int zp_csr_build_checked(const int64_t *edge_index, int64_t n_edges, int64_t n_nodes,
                          const int64_t *atomic_numbers, int n_elements, int32_t *perm,
                          int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr,
-                         int32_t *perm_src, int32_t *row_ptr_src, int32_t *flags_host, void *work,
-                         size_t work_bytes, void *stream);
+                         int32_t *perm_src, int32_t *row_ptr_src, int32_t *flags_host, void *done,
+                         void *work, size_t work_bytes, void *stream);
 
 /* zp_csr_build for callers that must not allocate device memory.  This entry point has no
  * counterpart in the reference.  A molecular-dynamics driver typically reserves all device
@@ -326,7 +327,8 @@ int zp_layernorm_silu_backward(int64_t rows, int width, const float *x, const fl
  * grad_node_out [N, K, C], which is the upstream gradient zp_eso2_backward wants in a force
  * pass.  The hidden layer runs on the contraction engine in the plan's operand format; all sums
  * over nodes have a fixed order.  `work`: zp_readout_work_bytes() bytes; the backward reads what
- * the forward left there, so both get the same buffer.                                          */
+ * the forward left there, so both get the same buffer.  The four parameter gradients are given
+ * together, or all NULL for frozen parameters.                                                  */
 size_t zp_readout_work_bytes(const zp_plan *plan, int64_t n_nodes);
 int zp_readout_forward(const zp_plan *plan, int64_t n_nodes, const float *node_out, const float *w0,
                        const float *b0, const float *w1, const float *b1, float *energy, void *work,

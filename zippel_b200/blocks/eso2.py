@@ -594,43 +594,42 @@ class Readout(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, plan: Plan, node_out, w0, b0, w1, b1):
-        lib = _lib.load()
         if not node_out.is_cuda:
             raise RuntimeError("Readout needs CUDA tensors: there is no CPU path")
-        x, w0f, b0f, w1f, b1f = (_f32(t) for t in (node_out, w0, b0, w1.reshape(-1), b1))
-        n = x.shape[0]
-        nbytes = lib.zp_readout_work_bytes(plan.handle, n)
-        work = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=x.device)
-        energy = torch.empty(1, dtype=torch.float32, device=x.device)
-        with torch.cuda.device(x.device):
-            st = torch.cuda.current_stream().cuda_stream
-            _lib.check(lib.zp_readout_forward(plan.handle, n, x.data_ptr(), w0f.data_ptr(),
-                                              b0f.data_ptr(), w1f.data_ptr(), b1f.data_ptr(),
-                                              energy.data_ptr(), work.data_ptr(), work.numel(), st),
-                       "zp_readout_forward")
-        ctx.plan = plan
-        ctx.shapes = (w1.shape, [t.dtype for t in (node_out, w0, b0, w1, b1)])
-        ctx.save_for_backward(x, w0f, b0f, w1f, b1f, work)
-        return energy.reshape(()).to(node_out.dtype)
+        x, head = _as_f32(node_out), [_as_f32(t) for t in (w0, b0, w1, b1)]
+        energy, work = _readout(plan, x, head)
+        ctx.plan, ctx.dtypes = plan, [t.dtype for t in (node_out, w0, b0, w1, b1)]
+        ctx.save_for_backward(x, *head, work)
+        return energy.to(node_out.dtype)
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_e):
-        lib = _lib.load()
-        x, w0f, b0f, w1f, b1f, work = ctx.saved_tensors
-        n = x.shape[0]
-        ge = _f32(grad_e).reshape(1)
-        gx, gw0, gb0, gw1, gb1 = (torch.empty_like(t) for t in (x, w0f, b0f, w1f, b1f))
-        with torch.cuda.device(x.device):
-            st = torch.cuda.current_stream().cuda_stream
-            _lib.check(lib.zp_readout_backward(
-                ctx.plan.handle, n, x.data_ptr(), w0f.data_ptr(), b0f.data_ptr(), w1f.data_ptr(),
-                b1f.data_ptr(), ge.data_ptr(), gx.data_ptr(), gw0.data_ptr(), gb0.data_ptr(),
-                gw1.data_ptr(), gb1.data_ptr(), work.data_ptr(), work.numel(), st),
-                "zp_readout_backward")
-        w1_shape, dts = ctx.shapes
-        return (None, gx.to(dts[0]), gw0.to(dts[1]), gb0.to(dts[2]),
-                gw1.reshape(w1_shape).to(dts[3]), gb1.to(dts[4]))
+        x, *head, work = ctx.saved_tensors
+        gx = torch.empty_like(x)
+        grads = [gx, *_readout_vjp(ctx.plan, x, head, grad_e, gx, work, any(ctx.needs_input_grad[2:]))]
+        return None, *(t if t is None or t.dtype == dt else t.to(dt) for t, dt in zip(grads, ctx.dtypes))
+
+
+def _readout(plan: Plan, x, head):
+    """Energy (0-dim) of node rows ``x`` under the head's parameters, and the buffer its VJP reads."""
+    n = x.shape[0]
+    nbytes = max(_lib.load().zp_readout_work_bytes(plan.handle, n), 16)
+    work = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    energy = torch.empty((), dtype=torch.float32, device=x.device)
+    _lib.run(x.device, "zp_readout_forward", plan.handle, n, x.data_ptr(), *[t.data_ptr() for t in head],
+             energy.data_ptr(), work.data_ptr(), nbytes)
+    return energy, work
+
+
+def _readout_vjp(plan: Plan, x, head, grad_e, gx, work, trainable: bool):
+    """Writes the gradient of ``x`` to ``gx``; returns those of the head (None when frozen)."""
+    ge = _as_f32(grad_e)
+    grads = [torch.empty_like(t) if trainable else None for t in head]
+    _lib.run(x.device, "zp_readout_backward", plan.handle, x.shape[0], x.data_ptr(),
+             *[t.data_ptr() for t in head], ge.data_ptr(), gx.data_ptr(),
+             *[t.data_ptr() if t is not None else None for t in grads], work.data_ptr(), work.numel())
+    return grads
 
 
 def tensor_core_linear(plan: Plan, x: torch.Tensor, weight: torch.Tensor, bias) -> torch.Tensor:
@@ -683,85 +682,120 @@ class BlockFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, block, plan: Plan, graph: EdgeGraph, perm, atomic_numbers, shifts, cos_g, sin_g,
                 x_ready, pos, x_node, *params):
-        lib, cfg, s = _lib.load(), block.cfg, plan.sizes
-        needs_bwd = any(ctx.needs_input_grad)
-        n, e = graph.n_nodes, graph.n_edges
-        n0, n1 = getattr(graph, "node_range", None) or (0, n)
-        dtypes = [t.dtype for t in (pos, x_node, *params)]
-        pos, x, shifts, cos_g, sin_g = (_as_f32(t) for t in (pos, x_node, shifts, cos_g, sin_g))
-        params = [_as_f32(t) for t in params]
-        off, z = _as_f32(block.gauss_offset), atomic_numbers
-        if z.dtype != torch.int64 or not z.is_contiguous():
-            z = z.to(torch.int64).contiguous()
-        for t in (pos, x, shifts, z, *params):
-            if not t.is_cuda:
-                raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
-        assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
-        assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.shape == (n,)
-        assert cos_g.shape[1] == cfg.lmax + 1 and sin_g.shape == cos_g.shape
-        assert min(shifts.shape[0], cos_g.shape[0]) >= e
-        out = torch.empty(n1 - n0, s.K, plan.c, dtype=torch.float32, device=x.device)
-        front = block.front_config()
-        nbytes = lib.zp_block_workspace_bytes(plan.handle, front, n1 - n0, n, e, 1 if needs_bwd else 2)
-        if nbytes == 0:
-            raise _lib.ZpError(2, "zp_block_workspace_bytes")
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
-        call = _lib.ZpBlockCall(
-            n1 - n0, e, n, n0, pos.data_ptr(), shifts.data_ptr(), z.data_ptr(), x.data_ptr(),
-            cos_g.data_ptr(), sin_g.data_ptr(), perm.data_ptr(), graph.src.data_ptr(),
-            graph.dst.data_ptr(), graph.row_ptr.data_ptr(), graph.perm_src.data_ptr(),
-            graph.row_ptr_src.data_ptr())
-        p = [t.data_ptr() for t in params]
-        m = plan.mmax
-        so2, keep = _weights_ptrs(m, p[11:])
-        cparams = _lib.ZpBlockParams(p[0], off.data_ptr(), _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
-                                     _P2(p[3], p[7]), _P2(p[4], p[8]), block.rad_func[1].eps, so2)
-        with torch.cuda.device(x.device):
-            _lib.check(lib.zp_block_forward(
-                plan.handle, front, call, cparams, out.data_ptr(), ws.data_ptr(), nbytes, needs_bwd,
-                x_ready.cuda_event if x_ready is not None else None,
-                torch.cuda.current_stream().cuda_stream), "zp_block_forward")
-        if needs_bwd:
-            # the workspace goes through save_for_backward like any activation, so that activation
-            # checkpointing can drop it and recompute; of the parameters the backward reads only
-            # the LayerNorms' (the products read the planes in the workspace)
-            ctx.save_for_backward(ws, x, pos, z, off, params[3], params[4], params[7], params[8])
-            ctx.native = (plan, graph, front, call, cparams, keep)
-            ctx.shapes, ctx.dtypes = [t.shape for t in params], dtypes
-            ctx.row0 = n0
-        return out.to(dtypes[1])
+        out, saved = _block(ctx, block, plan, graph, perm, atomic_numbers, shifts, cos_g, sin_g,
+                            x_ready, pos, x_node, params)
+        ctx.save_for_backward(*saved)
+        return out if out.dtype == x_node.dtype else out.to(x_node.dtype)
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
-        ws, x, pos = ctx.saved_tensors[:3]
-        plan, graph, front, call, cparams, _keep = ctx.native
-        g = _as_f32(grad_out)
-        want = ctx.needs_input_grad[9:]
-        f32 = dict(dtype=torch.float32, device=x.device)
-        gpos = torch.empty(pos.shape, **f32) if want[0] else None
-        gx = torch.empty(x.shape, **f32) if want[1] else None
-        # frozen parameters: the products behind their gradients are not run; the radial and the
-        # SO(2) parameters are each formed together
-        wp = want[2:]
-        groups = [wp[0]] + [any(wp[1:11])] * 10 + [any(wp[11:])] * (len(wp) - 11)
-        gp = [torch.empty(sh, **f32) if w else None for sh, w in zip(ctx.shapes, groups)]
-        p = [t.data_ptr() if t is not None else None for t in gp]
-        so2, keep = (_weights_ptrs(plan.mmax, p[11:]) if p[11] is not None
-                     else (_lib.ZpWeights(), None))
-        grads = _lib.ZpBlockGrads(p[0], _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
-                                  _P2(p[3], p[7]), _P2(p[4], p[8]), so2)
-        with torch.cuda.device(x.device):
-            _lib.check(_lib.load().zp_block_backward(
-                plan.handle, front, call, cparams,
-                g.data_ptr() - ctx.row0 * plan.sizes.K * plan.c * 4,
-                gx.data_ptr() if gx is not None else None,
-                gpos.data_ptr() if gpos is not None else None, grads, ws.data_ptr(), ws.numel(),
-                torch.cuda.current_stream().cuda_stream), "zp_block_backward")
-        del keep
-        out = [t if t is None or t.dtype == dt else t.to(dt)
-               for t, dt in zip([gpos, gx, *gp], ctx.dtypes)]
-        return (None,) * 9 + tuple(t if w else None for t, w in zip(out, want))
+        return (None,) * 9 + _block_vjp(ctx, ctx.saved_tensors, grad_out, ctx.needs_input_grad[9:])
+
+
+class EnergyFunction(torch.autograd.Function):
+    """``BlockFunction`` and ``Readout`` as one: the energy of a call made in one piece.  ``params`` are
+    all of the block's.  One function, not two, because in a force evaluation of some tens of atoms
+    the autograd machinery of the second costs a tenth of the whole call."""
+
+    @staticmethod
+    def forward(ctx, block, plan: Plan, graph: EdgeGraph, perm, atomic_numbers, shifts, cos_g, sin_g,
+                x_ready, pos, x_node, *params):
+        out, saved = _block(ctx, block, plan, graph, perm, atomic_numbers, shifts, cos_g, sin_g,
+                            x_ready, pos, x_node, params[:-4])
+        head = [_as_f32(t) for t in params[-4:]]
+        energy, work = _readout(plan, out, head)
+        ctx.head_dtypes = [t.dtype for t in params[-4:]]
+        ctx.save_for_backward(*saved, out, *head, work)
+        return energy if energy.dtype == x_node.dtype else energy.to(x_node.dtype)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad_e):
+        out, *head, work = ctx.saved_tensors[-6:]
+        want, plan = ctx.needs_input_grad[9:], ctx.native[0]
+        g = torch.empty_like(out)
+        ghead = _readout_vjp(plan, out, head, grad_e, g, work, any(want[-4:]))
+        ghead = [t if w else None for t, w in zip(ghead, want[-4:])]
+        grads = ((None,) * len(want[:-4]) if not any(want[:-4]) else
+                 _block_vjp(ctx, ctx.saved_tensors[:-6], g, want[:-4]))
+        return (None,) * 9 + grads + tuple(t if t is None or t.dtype == dt else t.to(dt)
+                                           for t, dt in zip(ghead, ctx.head_dtypes))
+
+
+def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin_g, x_ready, pos,
+           x_node, params):
+    """node_out in fp32 and, if a backward can follow, the tensors it reads (the rest goes to ``ctx``)."""
+    cfg, s = block.cfg, plan.sizes
+    needs_bwd = any(ctx.needs_input_grad)
+    n, e = graph.n_nodes, graph.n_edges
+    n0, n1 = getattr(graph, "node_range", None) or (0, n)
+    dtypes = [t.dtype for t in (pos, x_node, *params)]
+    pos, x, shifts, cos_g, sin_g = (_as_f32(t) for t in (pos, x_node, shifts, cos_g, sin_g))
+    params = [_as_f32(t) for t in params]
+    off = _as_f32(block.gauss_offset)
+    if z.dtype != torch.int64 or not z.is_contiguous():
+        z = z.to(torch.int64).contiguous()
+    for t in (pos, x, shifts, z, *params):
+        if not t.is_cuda:
+            raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
+    assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
+    assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.shape == (n,)
+    assert cos_g.shape[1] == cfg.lmax + 1 and sin_g.shape == cos_g.shape
+    assert min(shifts.shape[0], cos_g.shape[0]) >= e
+    out = torch.empty(n1 - n0, s.K, plan.c, dtype=torch.float32, device=x.device)
+    front = block.front_config()
+    nbytes = _lib.load().zp_block_workspace_bytes(plan.handle, front, n1 - n0, n, e,
+                                                  1 if needs_bwd else 2)
+    if nbytes == 0:
+        raise _lib.ZpError(2, "zp_block_workspace_bytes")
+    ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    call = _lib.ZpBlockCall(
+        n1 - n0, e, n, n0, pos.data_ptr(), shifts.data_ptr(), z.data_ptr(), x.data_ptr(),
+        cos_g.data_ptr(), sin_g.data_ptr(), perm.data_ptr(), graph.src.data_ptr(),
+        graph.dst.data_ptr(), graph.row_ptr.data_ptr(), graph.perm_src.data_ptr(),
+        graph.row_ptr_src.data_ptr())
+    p = [t.data_ptr() for t in params]
+    so2, keep = _weights_ptrs(plan.mmax, p[11:])
+    cparams = _lib.ZpBlockParams(p[0], off.data_ptr(), _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
+                                 _P2(p[3], p[7]), _P2(p[4], p[8]), block.rad_func[1].eps, so2)
+    _lib.run(x.device, "zp_block_forward", plan.handle, front, call, cparams, out.data_ptr(),
+             ws.data_ptr(), nbytes, needs_bwd, x_ready.cuda_event if x_ready is not None else None)
+    if not needs_bwd:
+        return out, ()
+    # the workspace goes through save_for_backward like any activation, so that activation
+    # checkpointing can drop it and recompute; of the parameters the backward reads only
+    # the LayerNorms' (the products read the planes in the workspace)
+    ctx.native = (plan, graph, front, call, cparams, keep)
+    ctx.shapes, ctx.dtypes, ctx.row0 = [t.shape for t in params], dtypes, n0
+    return out, (ws, x, pos, z, off, params[3], params[4], params[7], params[8])
+
+
+def _block_vjp(ctx, saved, grad_out, want):
+    """Gradients of (pos, x_node, *params), None where ``want`` is false."""
+    ws, x, pos = saved[:3]
+    plan, graph, front, call, cparams, _keep = ctx.native
+    g = _as_f32(grad_out)
+    f32 = dict(dtype=torch.float32, device=x.device)
+    gpos = torch.empty(pos.shape, **f32) if want[0] else None
+    gx = torch.empty(x.shape, **f32) if want[1] else None
+    # frozen parameters: the products behind their gradients are not run; the radial and the
+    # SO(2) parameters are each formed together
+    wp = want[2:]
+    groups = [wp[0]] + [any(wp[1:11])] * 10 + [any(wp[11:])] * (len(wp) - 11)
+    gp = [torch.empty(sh, **f32) if w else None for sh, w in zip(ctx.shapes, groups)]
+    p = [t.data_ptr() if t is not None else None for t in gp]
+    so2, keep = (_weights_ptrs(plan.mmax, p[11:]) if p[11] is not None
+                 else (_lib.ZpWeights(), None))
+    grads = _lib.ZpBlockGrads(p[0], _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
+                              _P2(p[3], p[7]), _P2(p[4], p[8]), so2)
+    _lib.run(x.device, "zp_block_backward", plan.handle, front, call, cparams,
+             g.data_ptr() - ctx.row0 * plan.sizes.K * plan.c * 4,
+             gx.data_ptr() if gx is not None else None,
+             gpos.data_ptr() if gpos is not None else None, grads, ws.data_ptr(), ws.numel())
+    del keep
+    return tuple(None if t is None or not w else t if t.dtype == dt else t.to(dt)
+                 for t, w, dt in zip([gpos, gx, *gp], want, ctx.dtypes))
 
 
 _P2, _P3 = ctypes.c_void_p * 2, ctypes.c_void_p * 3
@@ -868,10 +902,18 @@ class ESO2Block(nn.Module):
         return radial_mlp(plan, x_edge, list(self.rad_func))
 
     # -- forward --------------------------------------------------------------------------
+    def _all_params(self) -> list:
+        """``list(self.parameters())`` without the names and the search for repetitions."""
+        found, todo = [], [self]
+        while todo:
+            module = todo.pop()
+            found += [p for p in module._parameters.values() if p is not None]
+            todo += reversed(module._modules.values())
+        return found
+
     def _block_params(self) -> list:
         """Parameters of everything before the readout, in registration order."""
-        params = list(self.parameters())
-        return params[:len(params) - 4]
+        return self._all_params()[:-4]
 
     def _edges_to_nodes(self, plan, graph, perm, pos, atomic_numbers, x_node, shifts, cos_gamma_k,
                         sin_gamma_k, x_ready=None) -> torch.Tensor:
@@ -900,23 +942,32 @@ class ESO2Block(nn.Module):
         Graphs whose per-edge activations (radial features included) exceed the memory budget
         are processed as destination-node chunks under activation checkpointing: each chunk's
         forward is recomputed in the backward, so memory stays bounded by one chunk."""
+        return self._evaluate(BlockFunction, pos, atomic_numbers, x_node, edge_index, shifts,
+                              cos_gamma_k, sin_gamma_k, graph, x_ready)
+
+    def _evaluate(self, function, pos, atomic_numbers, x_node, edge_index, shifts, cos_gamma_k,
+                  sin_gamma_k, graph, x_ready=None) -> torch.Tensor:
+        """``function`` (node_out or energy) of a call, in one piece if it surely fits."""
         check = None
         if graph is None:
             # new input: node indices and element numbers are range-checked (a caller that passes
             # a prebuilt graph has had them checked when it was built)
             graph, check = self._sorted_edges(edge_index, atomic_numbers)
         plan = self.plan(pos.device)
-        args = (atomic_numbers, shifts, cos_gamma_k, sin_gamma_k)
+        energy = function is EnergyFunction
         try:
             out = None
             if _surely_fits(plan, graph.n_edges):
                 try:
-                    out = self._edges_to_nodes(plan, graph, graph.perm, pos, args[0], x_node,
-                                               *args[1:], x_ready)
+                    out = function.apply(self, plan, graph, graph.perm, atomic_numbers, shifts,
+                                         cos_gamma_k, sin_gamma_k, x_ready, pos, x_node,
+                                         *(self._all_params() if energy else self._block_params()))
                 except torch.cuda.OutOfMemoryError:
                     pass
             if out is None:
+                args = (atomic_numbers, shifts, cos_gamma_k, sin_gamma_k)
                 out = self._node_output_in_chunks(plan, graph, pos, x_node, args, x_ready)
+                out = self.energy(out) if energy else out
         finally:
             if check is not None:
                 check()
@@ -1013,9 +1064,8 @@ class ESO2Block(nn.Module):
         """Scalar E.  ``jd`` (the reference's argument) is verified against the J matrices the
         kernels use; anything else raises ``ValueError``."""
         self._check_jd(jd)
-        node_out = self.node_output(pos, atomic_numbers, x_node, edge_index, shifts,
-                                    cos_gamma_k, sin_gamma_k, graph)
-        return self.energy(node_out)
+        return self._evaluate(EnergyFunction, pos, atomic_numbers, x_node, edge_index, shifts,
+                              cos_gamma_k, sin_gamma_k, graph)
 
     def energy(self, node_out: torch.Tensor) -> torch.Tensor:
         """The readout head on the library's kernels (``Readout``): invariants, two dense layers,

@@ -133,6 +133,17 @@ struct ZpMaxList {                              // *out = max |x[0 .. count)|, o
     x[n] = src; count[n] = cnt; out[n++] = slot;
   }
 };
+struct ZpSplitList {                            // fp32 matrices to 16-bit planes
+  int n = 0;
+  int64_t rows[3], cols[3], ld_in[3];
+  const float *in[3];
+  ZpPlanes out[3];
+  ZpScale scale[3];
+  void add(int64_t n_rows, int64_t n_cols, const float *src, int64_t ld, const ZpPlanes &to,
+           const ZpScale &q) {
+    rows[n] = n_rows; cols[n] = n_cols; ld_in[n] = ld; in[n] = src; out[n] = to; scale[n++] = q;
+  }
+};
 enum { ZP_PREP_PLAIN = 0, ZP_PREP_KEPT = 1, ZP_PREP_FOLDED = 2 };
 struct ZpPrepList {                             // weight matrices to 16-bit planes
   int n = 0;
@@ -305,6 +316,7 @@ int zp_gemm_tc_splits(const ZpGemmTc &g);
 // K split (<= max_splits) that fills the device's CTAs (or CTA pairs) most evenly for this problem
 int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits);
 // fp32 [rows, cols] (row stride ld_in) -> planes [rows, out.ld], zero padded
+int zp_launch_split_list(const ZpSplitList &list, cudaStream_t st);
 int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,
                            const ZpPlanes &out, const ZpScale &scale, cudaStream_t st);
 int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st);
@@ -353,6 +365,15 @@ int zp_launch_ln_silu_bwd(int64_t rows, int width, const float *x, const float *
 // round4(K) floats, `colsum_scratch`: ceil(M / 512) * N floats.  dw and db get their last sums from `list`
 // (zp_launch_finalize); dx_absmax: device scalar updated with max |dx|, or null; dx_cols: how many
 // leading columns of dx are wanted (0: all K), ld_dx its row stride (0: K)
+// zp_linear_forward / zp_linear_backward_saved for a caller whose own kernels found the maxima.
+// `slots` (the start of the work buffer): {max x, scale, max w, scale, max dy, scale, and two words
+// for the caller's use}; with fp16 planes the maxima stand there when these are called.
+constexpr int kLinSlotX = 0, kLinSlotW = 2, kLinSlotDy = 4, kLinSlotFree = 6, kLinSlots = 8;
+int zp_linear_forward_maxima(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *x,
+                             const float *w, const float *bias, float *y, void *work,
+                             cudaStream_t st);
+int zp_linear_backward_maxima(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *dy,
+                              float *dx, float *dw, float *db, void *work, cudaStream_t st);
 int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t N,
                               const ZpPlanes &x, const ZpPlanes &w, const ZpPlanes &dy, float *dx,
                               float *dw, float *db, float *partials, int max_splits,

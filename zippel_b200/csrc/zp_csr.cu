@@ -321,8 +321,8 @@ int zp_csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *perm,
 int zp_csr_build_checked(const int64_t *edge_index, int64_t E, int64_t N,
                          const int64_t *atomic_numbers, int n_elements, int32_t *perm,
                          int32_t *src_sorted, int32_t *dst_sorted, int32_t *row_ptr,
-                         int32_t *perm_src, int32_t *row_ptr_src, int32_t *flags_host, void *work,
-                         size_t work_bytes, void *stream) {
+                         int32_t *perm_src, int32_t *row_ptr_src, int32_t *flags_host, void *done,
+                         void *work, size_t work_bytes, void *stream) {
   if (!flags_host || (N && !atomic_numbers)) return ZP_ERR_INVALID_ARG;
   const int rc = csr_build(edge_index, E, N, perm, src_sorted, dst_sorted, row_ptr, perm_src,
                            row_ptr_src, atomic_numbers, n_elements, work, work_bytes,
@@ -330,6 +330,7 @@ int zp_csr_build_checked(const int64_t *edge_index, int64_t E, int64_t N,
   if (rc) return rc;
   ZP_CUDA(cudaMemcpyAsync(flags_host, carve_csr(E, N, work).flag, sizeof(int32_t),
                           cudaMemcpyDeviceToHost, (cudaStream_t)stream));
+  if (done) ZP_CUDA(cudaEventRecord((cudaEvent_t)done, (cudaStream_t)stream));
   return ZP_OK;
 }
 

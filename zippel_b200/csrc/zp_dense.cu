@@ -16,14 +16,17 @@
 
 namespace {
 
-// fp32 matrix -> planes (bf16, or fp16 with the tensor's scale), zero padding up to ld_out.
+// fp32 matrices (blockIdx.z) -> planes (bf16, or fp16 with the tensor's scale), zero padding up to ld_out.
 // threadIdx.x walks the quads of a row, threadIdx.y / blockIdx.x the rows (no division anywhere).
-__global__ void split_planes_kernel(int64_t rows, int64_t cols, const float *__restrict__ in,
-                                    int64_t ld_in, const ZpPlanes out, const ZpScale scale) {
+__global__ void split_planes_kernel(const __grid_constant__ ZpSplitList d) {
+  const int b = blockIdx.z;
+  const float *__restrict__ in = d.in[b];
+  const int64_t rows = d.rows[b], cols = d.cols[b], ld_in = d.ld_in[b];
+  const ZpPlanes out = d.out[b];
   const int64_t c = 4 * ((int64_t)blockIdx.y * blockDim.x + threadIdx.x);
   const float inv =
-      zp_publish_scale(out, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 &&
-                                       threadIdx.y == 0);
+      zp_publish_scale(out, d.scale[b], blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 &&
+                                            threadIdx.y == 0);
   if (c >= out.ld) return;
   const bool vec = (ld_in & 3) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 && c + 3 < cols;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.y + threadIdx.y; r < rows;
@@ -439,19 +442,29 @@ int zp_launch_conv1_bound(const zp_plan *p, const float *a1_scale, const float *
   return ZP_OK;
 }
 
-int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,
-                           const ZpPlanes &out, const ZpScale &scale, cudaStream_t st) {
-  if (rows == 0 || out.ld == 0) return ZP_OK;
-  const int quads = (int)(out.ld / 4);
+int zp_launch_split_list(const ZpSplitList &list, cudaStream_t st) {
+  int64_t rows = 0, quads = 0;
+  for (int i = 0; i < list.n; ++i) {
+    rows = list.rows[i] > rows ? list.rows[i] : rows;
+    quads = list.out[i].ld / 4 > quads ? list.out[i].ld / 4 : quads;
+  }
+  if (rows == 0 || quads == 0) return ZP_OK;
   int bx = 32;
   while (bx < quads && bx < 256) bx <<= 1;
   const int by = 256 / bx;
   int64_t gx = zp_ceil_div(rows, by);
   if (gx > 148 * 32) gx = 148 * 32;
-  const dim3 grid((unsigned)gx, (unsigned)zp_ceil_div(quads, bx)), block(bx, by);
-  split_planes_kernel<<<grid, block, 0, st>>>(rows, cols, in, ld_in, out, scale);
+  split_planes_kernel<<<dim3((unsigned)gx, (unsigned)zp_ceil_div(quads, bx), list.n), dim3(bx, by), 0,
+                        st>>>(list);
   ZP_LAUNCH_CHECK("split_planes_kernel");
   return ZP_OK;
+}
+
+int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,
+                           const ZpPlanes &out, const ZpScale &scale, cudaStream_t st) {
+  ZpSplitList list;
+  list.add(rows, cols, in, ld_in, out, scale);
+  return zp_launch_split_list(list, st);
 }
 
 int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st) {

@@ -11,7 +11,7 @@
 namespace {
 
 struct LinWork {
-  float *scales;          // {max x, s_x, max w, s_w, max dy, s_dy}
+  float *scales;          // kLinSlots
   ZpPlanes x, w, dy;
   float *partials;        // weight-gradient partial sums [splits][N*K]
   float *colsum;          // bias-gradient partials
@@ -38,10 +38,10 @@ LinWork carve_lin(const zp_plan *p, int64_t M, int64_t K, int64_t N, void *base)
     pl.base = take((size_t)pl.planes * pl.plane_stride * 2);
     return pl;
   };
-  w.scales = reinterpret_cast<float *>(take(8 * sizeof(float)));
-  w.x = planes(M, K, w.scales + 1);
-  w.w = planes(N, K, w.scales + 3);
-  w.dy = planes(M, N, w.scales + 5);
+  w.scales = reinterpret_cast<float *>(take(kLinSlots * sizeof(float)));
+  w.x = planes(M, K, w.scales + kLinSlotX + 1);
+  w.w = planes(N, K, w.scales + kLinSlotW + 1);
+  w.dy = planes(M, N, w.scales + kLinSlotDy + 1);
   w.partials = reinterpret_cast<float *>(take(sizeof(float) * kLinSplits * N * K));
   w.colsum = reinterpret_cast<float *>(take(sizeof(float) * (size_t)zp_ceil_div(M > 0 ? M : 1, 128) * N));
   w.bytes = off;
@@ -55,23 +55,22 @@ struct SplitJob {
   const ZpPlanes *planes;
   float *slot;
 };
-int split_scaled(const zp_plan *p, const SplitJob *jobs, int n, cudaStream_t st) {
+int split_scaled(const zp_plan *p, const SplitJob *jobs, int n, cudaStream_t st,
+                 bool maxima_known = false) {
   int rc;
-  if (p->fp16) {
+  if (p->fp16 && !maxima_known) {
     ZpMaxList maxima;
-    for (int i = 0; i < n; ++i) {
-      ZP_CUDA(cudaMemsetAsync(jobs[i].slot, 0, sizeof(float), st));
-      maxima.add(jobs[i].in, jobs[i].rows * jobs[i].cols, jobs[i].slot);
-    }
+    float *last = jobs[n - 1].slot;                       // slots in ascending order
+    ZP_CUDA(cudaMemsetAsync(jobs[0].slot, 0, (last + 1 - jobs[0].slot) * sizeof(float), st));
+    for (int i = 0; i < n; ++i) maxima.add(jobs[i].in, jobs[i].rows * jobs[i].cols, jobs[i].slot);
     if ((rc = zp_launch_max_list(maxima, st))) return rc;
   }
+  ZpSplitList list;
   for (int i = 0; i < n; ++i) {
     const SplitJob &q = jobs[i];
-    if ((rc = zp_launch_split_planes(q.rows, q.cols, q.in, q.cols, *q.planes,
-                                     zp_scale_of(1.f, q.slot, q.slot + 1), st)))
-      return rc;
+    list.add(q.rows, q.cols, q.in, q.cols, *q.planes, zp_scale_of(1.f, q.slot, q.slot + 1));
   }
-  return ZP_OK;
+  return zp_launch_split_list(list, st);
 }
 
 }  // namespace
@@ -117,6 +116,30 @@ int check(const zp_plan *p, int64_t M, int64_t K, int64_t N) {
   return ZP_OK;
 }
 
+int forward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *x, const float *w,
+            const float *bias, float *y, const LinWork &lw, bool maxima_known, cudaStream_t st) {
+  const SplitJob jobs[2] = {{M, K, x, &lw.x, lw.scales + kLinSlotX},
+                            {N, K, w, &lw.w, lw.scales + kLinSlotW}};
+  if (int rc = split_scaled(plan, jobs, 2, st, maxima_known)) return rc;
+  const ZpGemmTc g{M, N, K, plan->planes, lw.x.base, lw.x.ld, lw.x.plane_stride, 0,
+                   lw.w.base, lw.w.ld, lw.w.plane_stride, 0, bias, y, N, plan->status_dev,
+                   0, 1, 0, 0, plan->fp16, lw.x.scale, lw.w.scale, nullptr};
+  return zp_launch_gemm_tc(g, st);
+}
+
+// the planes of x and w and their scales are where the forward left them
+int backward_saved(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *dy, float *dx,
+                   float *dw, float *db, const LinWork &lw, bool maximum_known, cudaStream_t st) {
+  const SplitJob job{M, N, dy, &lw.dy, lw.scales + kLinSlotDy};
+  int rc = split_scaled(plan, &job, 1, st, maximum_known);
+  if (rc) return rc;
+  ZpFinalList list;
+  if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
+                                      kLinSplits, lw.colsum, list, st)))
+    return rc;
+  return zp_launch_finalize(list, st);
+}
+
 }  // namespace
 
 extern "C" {
@@ -135,13 +158,7 @@ int zp_linear_forward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, cons
   if (!x || !w || !y || !work) return ZP_ERR_INVALID_ARG;
   const LinWork lw = carve_lin(plan, M, K, N, work);
   if (work_bytes < lw.bytes) return ZP_ERR_WORKSPACE;
-  cudaStream_t st = (cudaStream_t)stream;
-  const SplitJob jobs[2] = {{M, K, x, &lw.x, lw.scales}, {N, K, w, &lw.w, lw.scales + 2}};
-  if ((rc = split_scaled(plan, jobs, 2, st))) return rc;
-  const ZpGemmTc g{M, N, K, plan->planes, lw.x.base, lw.x.ld, lw.x.plane_stride, 0,
-                   lw.w.base, lw.w.ld, lw.w.plane_stride, 0, bias, y, N, plan->status_dev,
-                   0, 1, 0, 0, plan->fp16, lw.x.scale, lw.w.scale, nullptr};
-  return zp_launch_gemm_tc(g, st);
+  return forward(plan, M, K, N, x, w, bias, y, lw, false, (cudaStream_t)stream);
 }
 
 int zp_linear_backward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *x,
@@ -162,8 +179,8 @@ int zp_linear_backward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, con
   SplitJob jobs[3];
   int n = 0;
   if (dw) jobs[n++] = {M, K, x, &lw.x, lw.scales};
-  if (dx) jobs[n++] = {N, K, w, &lw.w, lw.scales + 2};
-  jobs[n++] = {M, N, dy, &lw.dy, lw.scales + 4};
+  if (dx) jobs[n++] = {N, K, w, &lw.w, lw.scales + kLinSlotW};
+  jobs[n++] = {M, N, dy, &lw.dy, lw.scales + kLinSlotDy};
   if ((rc = split_scaled(plan, jobs, n, st))) return rc;
   ZpFinalList list;
   if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
@@ -186,14 +203,18 @@ int zp_linear_backward_saved(const zp_plan *plan, int64_t M, int64_t K, int64_t 
     if (db) ZP_CUDA(cudaMemsetAsync(db, 0, sizeof(float) * N, st));
     return ZP_OK;
   }
-  // the planes of x and w and their scales are where zp_linear_forward left them
-  const SplitJob job{M, N, dy, &lw.dy, lw.scales + 4};
-  if ((rc = split_scaled(plan, &job, 1, st))) return rc;
-  ZpFinalList list;
-  if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
-                                      kLinSplits, lw.colsum, list, st)))
-    return rc;
-  return zp_launch_finalize(list, st);
+  return backward_saved(plan, M, K, N, dy, dx, dw, db, lw, false, st);
 }
 
 }  // extern "C"
+
+int zp_linear_forward_maxima(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *x,
+                             const float *w, const float *bias, float *y, void *work,
+                             cudaStream_t st) {
+  return forward(plan, M, K, N, x, w, bias, y, carve_lin(plan, M, K, N, work), true, st);
+}
+
+int zp_linear_backward_maxima(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *dy,
+                              float *dx, float *dw, float *db, void *work, cudaStream_t st) {
+  return backward_saved(plan, M, K, N, dy, dx, dw, db, carve_lin(plan, M, K, N, work), true, st);
+}

@@ -6,9 +6,12 @@
 //
 // and, given dE:  the gradients of W0, b0, W1, b1 and of node_out -- the upstream gradient of the
 // edge convolution's backward in the force pass.  The hidden layer runs on the tensor-core
-// contraction engine (zp_linear_forward / zp_linear_backward); everything else is streaming
-// kernels.  Every sum over nodes has a fixed order (strided partial sums, then one ordered pass),
-// so E and the parameter gradients repeat bit for bit.
+// contraction engine; everything else is streaming kernels, and since the head's arrays are small
+// (2 MB for 1000 atoms) what counts is how few launches it takes: the kernels that stream an
+// operand of the hidden layer also find its maximum, the energies are summed by the last block of
+// the kernel that forms them, and frozen parameters cost nothing.  Force evaluation of 64 atoms: 10
+// launches, where a pass for each step took 19.  Every sum over nodes has a fixed order (strided
+// partial sums, then one ordered pass), so E and the parameter gradients repeat bit for bit.
 #include "zp_common.cuh"
 #include "zippel_b200.h"
 
@@ -18,13 +21,32 @@ constexpr int kSumBlocks = 64;           // partial sums over nodes: node n goes
 
 __device__ __forceinline__ float sigmoid_fast(float x) { return 1.f / (1.f + __expf(-x)); }
 
+// *out = max(*out, max of m over the block) (blockDim.x a multiple of 32)
+__device__ __forceinline__ void block_absmax(float m, float *out) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(out, m);
+}
+
+// A block per node, and kWeightBlocks more that look for max |w0| (slots: kLinSlots of the hidden
+// layer, null when its operand format needs no maxima).
+constexpr int kWeightBlocks = 16;
 __global__ void __launch_bounds__(128)
 node_invariants_kernel(const __grid_constant__ ZpTables t, int64_t N,
-                       const float *__restrict__ node_out, float *__restrict__ inv) {
+                       const float *__restrict__ node_out, float *__restrict__ inv,
+                       const float *__restrict__ w0, float *slots) {
   const int64_t n = blockIdx.x;
+  const int W = (t.lmax + 1) * t.C;
+  float most = 0.f;
+  if (n >= N) {
+    for (int64_t i = (n - N) * 128 + threadIdx.x; i < (int64_t)W * t.C; i += kWeightBlocks * 128)
+      most = fmaxf(most, fabsf(w0[i]));
+    block_absmax(most, slots + kLinSlotW);
+    return;
+  }
   const float *row = node_out + (size_t)n * t.K * t.C;
-  float *out = inv + (size_t)n * (t.lmax + 1) * t.C;
-  for (int i = threadIdx.x; i < (t.lmax + 1) * t.C; i += blockDim.x) {
+  float *out = inv + (size_t)n * W;
+  for (int i = threadIdx.x; i < W; i += blockDim.x) {
     const int l = i / t.C, c = i - l * t.C;
     float s;
     if (l == 0) {
@@ -37,7 +59,9 @@ node_invariants_kernel(const __grid_constant__ ZpTables t, int64_t N,
       }
     }
     out[i] = s;
+    most = fmaxf(most, fabsf(s));
   }
+  if (slots) block_absmax(most, slots + kLinSlotX);
 }
 
 // grad_node_out from the gradient of the invariants
@@ -57,46 +81,55 @@ node_invariants_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N,
   }
 }
 
-// one warp per node: e_n = b1 + sum_c W1[c] silu(hid[n, c])
+// One warp per node: e_n = b1 + sum_c W1[c] silu(hid[n, c]).  The last block to finish (`done` counts
+// them) adds the e_n up in a fixed order: partial sum i takes e_i, e_(i + 1024), ...; the 1024 partial
+// sums are then added pairwise in a fixed tree.
 __global__ void __launch_bounds__(256)
 head_fwd_kernel(int64_t N, int C, const float *__restrict__ hid, const float *__restrict__ w1,
-                const float *__restrict__ b1, float *__restrict__ e_node) {
+                const float *__restrict__ b1, float *e_node, float *__restrict__ energy,
+                unsigned *done) {
+  __shared__ float part[1024];
+  __shared__ bool last;
   const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
   const int lane = threadIdx.x % 32;
-  if (n >= N) return;
-  float s = 0.f;
-  for (int c = lane; c < C; c += 32) {
-    const float h = hid[(size_t)n * C + c];
-    s = fmaf(w1[c], h * sigmoid_fast(h), s);
-  }
+  if (n < N) {
+    float s = 0.f;
+    for (int c = lane; c < C; c += 32) {
+      const float h = hid[(size_t)n * C + c];
+      s = fmaf(w1[c], h * sigmoid_fast(h), s);
+    }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) e_node[n] = s + b1[0];
-}
-
-// out[0] = sum of v[0..n) in a fixed order: thread i adds v[i], v[i + 1024], ...; the 1024
-// partial sums are then added pairwise in a fixed tree
-__global__ void __launch_bounds__(1024) ordered_sum_kernel(int64_t n, const float *__restrict__ v,
-                                                           float *__restrict__ out) {
-  __shared__ float part[1024];
-  float s = 0.f;
-  for (int64_t i = threadIdx.x; i < n; i += 1024) s += v[i];
-  part[threadIdx.x] = s;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) __stcg(&e_node[n], s + b1[0]);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float s = 0.f;
+    for (int64_t i = threadIdx.x + 256 * q; i < N; i += 1024) s += __ldcg(&e_node[i]);
+    part[threadIdx.x + 256 * q] = s;
+  }
   __syncthreads();
   for (int o = 512; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) part[threadIdx.x] += part[threadIdx.x + o];
+    for (int i = threadIdx.x; i < o; i += 256) part[i] += part[i + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[0] = part[0];
+  if (threadIdx.x == 0) energy[0] = part[0];
 }
 
-// g_hid[n, c] = dE * W1[c] * silu'(hid[n, c]);  block b also sums silu(hid[n, c]) over its nodes
-// n = b, b + 64, ... (in that order) into partial[b][c]
+// g_hid[n, c] = dE * W1[c] * silu'(hid[n, c]), and its maximum (slots as above);  block b also sums
+// silu(hid[n, c]) over its nodes n = b, b + 64, ... (in that order) into partial[b][c], unless null
 __global__ void __launch_bounds__(128)
 head_bwd_kernel(int64_t N, int C, const float *__restrict__ hid, const float *__restrict__ w1,
                 const float *__restrict__ grad_e, float *__restrict__ g_hid,
-                float *__restrict__ partial) {
+                float *__restrict__ partial, float *slots) {
   const float ge = grad_e[0];
+  float most = 0.f;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
     const float w = w1[c];
     float acc = 0.f;
@@ -104,10 +137,13 @@ head_bwd_kernel(int64_t N, int C, const float *__restrict__ hid, const float *__
       const float h = hid[(size_t)n * C + c];
       const float s = sigmoid_fast(h);
       acc += h * s;
-      g_hid[(size_t)n * C + c] = ge * w * (s + h * s * (1.f - s));
+      const float g = ge * w * (s + h * s * (1.f - s));
+      g_hid[(size_t)n * C + c] = g;
+      most = fmaxf(most, fabsf(g));
     }
-    partial[(size_t)blockIdx.x * C + c] = acc;
+    if (partial) partial[(size_t)blockIdx.x * C + c] = acc;
   }
+  if (slots) block_absmax(most, slots + kLinSlotDy);
 }
 
 __global__ void head_param_grad_kernel(int64_t N, int C, const float *__restrict__ partial,
@@ -172,15 +208,17 @@ int zp_readout_forward(const zp_plan *plan, int64_t N, const float *node_out, co
     ZP_CUDA(cudaMemsetAsync(energy, 0, sizeof(float), st));
     return ZP_OK;
   }
-  node_invariants_kernel<<<(unsigned)N, 128, 0, st>>>(t, N, node_out, rw.inv);
+  float *slots = static_cast<float *>(rw.linear);
+  ZP_CUDA(cudaMemsetAsync(slots, 0, kLinSlots * sizeof(float), st));
+  node_invariants_kernel<<<(unsigned)(N + (plan->fp16 ? kWeightBlocks : 0)), 128, 0, st>>>(
+      t, N, node_out, rw.inv, w0, plan->fp16 ? slots : nullptr);
   ZP_LAUNCH_CHECK("node_invariants_kernel");
-  int rc = zp_linear_forward(plan, N, (int64_t)(t.lmax + 1) * t.C, t.C, rw.inv, w0, b0, rw.hid,
-                             rw.linear, rw.linear_bytes, stream);
+  int rc = zp_linear_forward_maxima(plan, N, (int64_t)(t.lmax + 1) * t.C, t.C, rw.inv, w0, b0, rw.hid,
+                                    rw.linear, st);
   if (rc) return rc;
-  head_fwd_kernel<<<(unsigned)zp_ceil_div(N * 32, 256), 256, 0, st>>>(N, t.C, rw.hid, w1, b1, rw.e_node);
+  head_fwd_kernel<<<(unsigned)zp_ceil_div(N * 32, 256), 256, 0, st>>>(
+      N, t.C, rw.hid, w1, b1, rw.e_node, energy, reinterpret_cast<unsigned *>(slots + kLinSlotFree));
   ZP_LAUNCH_CHECK("head_fwd_kernel");
-  ordered_sum_kernel<<<1, 1024, 0, st>>>(N, rw.e_node, energy);
-  ZP_LAUNCH_CHECK("ordered_sum_kernel");
   return ZP_OK;
 }
 
@@ -189,14 +227,17 @@ int zp_readout_backward(const zp_plan *plan, int64_t N, const float *node_out, c
                         float *grad_node_out, float *grad_w0, float *grad_b0, float *grad_w1,
                         float *grad_b1, void *work, size_t work_bytes, void *stream) {
   (void)b0; (void)b1;
-  if (!plan || N < 0 || !grad_energy || !work || !w0 || !w1 || !grad_w0 || !grad_b0 || !grad_w1 ||
-      !grad_b1 || (N && (!node_out || !grad_node_out)))
+  const bool frozen = !grad_w0 && !grad_b0 && !grad_w1 && !grad_b1;
+  if (!plan || N < 0 || !grad_energy || !work || !w0 || !w1 ||
+      (!frozen && (!grad_w0 || !grad_b0 || !grad_w1 || !grad_b1)) ||
+      (N && (!node_out || !grad_node_out)))
     return ZP_ERR_INVALID_ARG;
   const ReadoutWork rw = carve_readout(plan, N, work);
   if (work_bytes < rw.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const ZpTables &t = plan->t;
   const int64_t W = (int64_t)(t.lmax + 1) * t.C;
+  if (N == 0 && frozen) return ZP_OK;
   if (N == 0) {
     ZP_CUDA(cudaMemsetAsync(grad_w0, 0, sizeof(float) * W * t.C, st));
     ZP_CUDA(cudaMemsetAsync(grad_b0, 0, sizeof(float) * t.C, st));
@@ -204,14 +245,19 @@ int zp_readout_backward(const zp_plan *plan, int64_t N, const float *node_out, c
     ZP_CUDA(cudaMemsetAsync(grad_b1, 0, sizeof(float), st));
     return ZP_OK;
   }
-  head_bwd_kernel<<<kSumBlocks, 128, 0, st>>>(N, t.C, rw.hid, w1, grad_energy, rw.g_hid, rw.partial);
+  float *slots = plan->fp16 ? static_cast<float *>(rw.linear) : nullptr;
+  if (slots) ZP_CUDA(cudaMemsetAsync(slots + kLinSlotDy, 0, sizeof(float), st));
+  head_bwd_kernel<<<kSumBlocks, 128, 0, st>>>(N, t.C, rw.hid, w1, grad_energy, rw.g_hid,
+                                              frozen ? nullptr : rw.partial, slots);
   ZP_LAUNCH_CHECK("head_bwd_kernel");
-  head_param_grad_kernel<<<(unsigned)zp_ceil_div(t.C, 128), 128, 0, st>>>(N, t.C, rw.partial,
-                                                                          grad_energy, grad_w1, grad_b1);
-  ZP_LAUNCH_CHECK("head_param_grad_kernel");
+  if (!frozen) {
+    head_param_grad_kernel<<<(unsigned)zp_ceil_div(t.C, 128), 128, 0, st>>>(
+        N, t.C, rw.partial, grad_energy, grad_w1, grad_b1);
+    ZP_LAUNCH_CHECK("head_param_grad_kernel");
+  }
   // the hidden layer's operand planes are still in the work buffer the forward used
-  int rc = zp_linear_backward_saved(plan, N, W, t.C, rw.g_hid, rw.g_inv, grad_w0, grad_b0,
-                                    rw.linear, rw.linear_bytes, stream);
+  int rc = zp_linear_backward_maxima(plan, N, W, t.C, rw.g_hid, rw.g_inv, grad_w0, grad_b0,
+                                     rw.linear, st);
   if (rc) return rc;
   node_invariants_bwd_kernel<<<(unsigned)N, 128, 0, st>>>(t, N, node_out, rw.g_inv, grad_node_out);
   ZP_LAUNCH_CHECK("node_invariants_bwd_kernel");

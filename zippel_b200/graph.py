@@ -145,14 +145,11 @@ class EdgeGraph:
             flags, done = slots.pop()
         except IndexError:
             flags, done = torch.empty(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
-        with torch.cuda.device(dev):
-            stream = torch.cuda.current_stream()
-            _lib.check(lib.zp_csr_build_checked(
-                ei.data_ptr(), e, n, z.data_ptr(), n_elements, perm.data_ptr(), src.data_ptr(),
-                dst.data_ptr(), row_ptr.data_ptr(), perm_src.data_ptr(), row_ptr_src.data_ptr(),
-                flags.data_ptr(), work.data_ptr(), work.numel(), stream.cuda_stream),
-                "zp_csr_build_checked")
-            done.record(stream)
+            done.record(torch.cuda.current_stream(dev))        # gives the event its handle
+        _lib.run(dev, "zp_csr_build_checked", ei.data_ptr(), e, n, z.data_ptr(), n_elements,
+                 perm.data_ptr(), src.data_ptr(), dst.data_ptr(), row_ptr.data_ptr(),
+                 perm_src.data_ptr(), row_ptr_src.data_ptr(), flags.data_ptr(), done.cuda_event,
+                 work.data_ptr(), work.numel())
 
         def check() -> None:
             done.synchronize()
