@@ -46,51 +46,12 @@ bool can_fuse(const zp_plan *p, int conv) {
   return true;
 }
 
-// ZP_STREAMS=0 in the environment keeps every launch on the caller's stream.
-bool lanes_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char *e = getenv("ZP_STREAMS");
-    on = (e && e[0] == '0') ? 0 : 1;
-  }
-  return on == 1;
-}
-
-// The caller's stream plus the plan's two side streams for one forward / backward call.
-struct Lanes {
-  const zp_plan *p;
-  cudaStream_t main;
-  bool on;
-  std::unique_lock<std::mutex> hold;
-  Lanes(const zp_plan *plan, cudaStream_t st)
-      : p(plan), main(st), on(lanes_enabled() && !plan->timer && plan->aux_stream[0]) {
-    if (on) hold = std::unique_lock<std::mutex>(*static_cast<std::mutex *>(plan->lane_lock));
-  }
-  cudaStream_t pick(int i) const { return (!on || i % 3 == 0) ? main : p->aux_stream[i % 3 - 1]; }
-  // side streams continue from what the caller's stream has been given so far
-  int fork() {
-    if (!on) return ZP_OK;
-    ZP_CUDA(cudaEventRecord(p->ev_fork, main));
-    for (int i = 0; i < 2; ++i) ZP_CUDA(cudaStreamWaitEvent(p->aux_stream[i], p->ev_fork, 0));
-    return ZP_OK;
-  }
-  // the caller's stream continues after everything the side streams have been given
-  int join() {
-    if (!on) return ZP_OK;
-    for (int i = 0; i < 2; ++i) {
-      ZP_CUDA(cudaEventRecord(p->ev_join[i], p->aux_stream[i]));
-      ZP_CUDA(cudaStreamWaitEvent(main, p->ev_join[i], 0));
-    }
-    return ZP_OK;
-  }
-};
-
 const float *wscale(const zp_plan *p, const ZpWorkspace &w, int conv, int m) {
   return p->fp16 ? w.scales + kScWeights + (conv * (ZP_MAX_L + 1) + m) * 2 + 1 : nullptr;
 }
 
 // Independent products, in one launch or side by side (between fork and join).
-int run_products(const zp_plan *plan, Lanes &lanes, const ZpGemmTc *g, int n, int cls, cudaStream_t st) {
+int run_products(const zp_plan *plan, ZpLanes &lanes, const ZpGemmTc *g, int n, int cls, cudaStream_t st) {
   int rc;
   if (n == 0) return ZP_OK;
   if (n <= ZP_GEMM_GROUP && (g[0].a_mn ? g[0].K : g[0].M) <= kTogetherEdges) {
@@ -109,6 +70,16 @@ ZpPlanes sub(const ZpPlanes &p, int64_t col) {
 }
 
 }  // namespace
+
+// ZP_STREAMS=0 in the environment keeps every launch on the caller's stream.
+bool zp_lanes_enabled() {
+  static int on = -1;
+  if (on < 0) {
+    const char *e = getenv("ZP_STREAMS");
+    on = (e && e[0] == '0') ? 0 : 1;
+  }
+  return on == 1;
+}
 
 ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *base, int ec,
                      ZpFormat rad) {
@@ -150,12 +121,12 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
     w.du_src = c.floats(e * 2 * t.K * t.C);
     w.torque = c.floats(e * 4);
     w.wgrad = c.floats((size_t)kZpWgradSplits * p->g_elems);
-    const size_t parts = (size_t)zp_ceil_div(E > 0 ? E : 1, kZpColRows);
-    w.col1 = c.floats(parts * p->c1_out[0]);
-    w.col2 = c.floats(parts * p->c2_out[0]);
+    auto column_parts = [&](int64_t cols) { return c.floats((size_t)(zp_colsum_parts(E, cols) * cols)); };
+    w.col1 = column_parts(p->c1_out[0]);
+    w.col2 = column_parts(p->c2_out[0]);
     if (ec > 0) {
       w.gr = c.planes(E, t.R, rad, w.scales + kScGrScale);
-      w.col_rad = c.floats(parts * t.R);
+      w.col_rad = column_parts(t.R);
       w.rad_partials = c.floats((size_t)zp_radial_splits(t.R, ec) * t.R * ((ec + 3) / 4 * 4));
     }
   }
@@ -469,14 +440,12 @@ int zp_core_radial(const zp_plan *plan, const ZpWorkspace &ws, int64_t E, int ec
 }
 
 int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c, float *node_out,
-                    int keep, cudaStream_t st) {
+                    int keep, ZpLanes &lanes) {
   int rc;
   const ZpTables &t = plan->t;
-  Lanes lanes(plan, st);
+  cudaStream_t st = lanes.main;
   const bool fuse1 = can_fuse(plan, 0), fuse2 = can_fuse(plan, 1);
   const bool lean = !keep && fuse1 && fuse2;          // h1 rows and y are never written
-  ZP_TIMED(ZP_K_WIGNER_FWD,
-           zp_launch_wigner_fwd(plan, c.E, c.edge_vec, c.cos_g, c.sin_g, ws.rot, 0, st));
   // |rot row . x| <= sqrt(2l+1) max|x|, over the rows the edges name
   ZP_TIMED(ZP_K_ROTATE_IN,
            zp_launch_rotate_in(plan, c.E, c.x_node, c.src, c.dst, ws.rot, c.radial, ws.a1,
@@ -641,7 +610,7 @@ static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *
   // magnitude bounds -> power-of-two scales, all on the device; then every weight as planes
   ZpMaxList maxima;
   ZpPrepList prep;
-  zp_add_so2_weights(plan, w, ws.wfold, ws.scales + kScWeights, maxima, prep);
+  zp_add_so2_weights(plan, w, ws.wfold, ws.scales + kScWeights, maxima, prep, keep != 0);
   if (layer)
     prep.add(rl->w, ws.rw.base, ws.scales + kScRw, ws.rw.plane_stride, t.R, rl->ec, (int)ws.rw.ld,
              ZP_PREP_PLAIN, f.planes, f.fp16);
@@ -670,7 +639,9 @@ static int eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *
     if ((rc = zp_core_radial(plan, ws, E, rl->ec, rl->b, st))) return rc;
     c.radial = ws.radial;
   }
-  return zp_core_forward(plan, ws, c, node_out, keep, st);
+  ZP_TIMED(ZP_K_WIGNER_FWD, zp_launch_wigner_fwd(plan, E, edge_vec, cos_g, sin_g, ws.rot, 0, st));
+  ZpLanes lanes(plan, E, st);
+  return zp_core_forward(plan, ws, c, node_out, keep, lanes);
 }
 
 int zp_eso2_forward(const zp_plan *plan, int64_t N, int64_t E, const float *x_node,
@@ -697,8 +668,10 @@ int zp_eso2_forward_inference(const zp_plan *plan, int64_t N, int64_t E, const f
 int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
                      const float *grad_node_out, float *grad_x_node, float *grad_edge_vec,
                      float *grad_radial, float *grad_env, const zp_weight_grads *gw,
-                     const ZpRadialLayer *rl, ZpFinalList &list, cudaStream_t st) {
+                     const ZpRadialLayer *rl, ZpFinalList &radial_list, ZpLanes &lanes) {
   int rc;
+  cudaStream_t st = lanes.main;
+  ZpFinalList list;
   const int64_t N = c.N, E = c.E;
   // gw == NULL: the parameters are frozen (an MD / inference force evaluation): no weight-gradient
   // product, no bias column sum, no unfolding
@@ -706,7 +679,6 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   // grad_x_node == NULL: the embeddings are an input without a gradient (E and dE/dpos of one
   // block): the per-edge contributions are neither written nor summed
   float *du_out = grad_x_node ? ws.du_src : nullptr;
-  Lanes lanes(plan, st);
   const ZpTables &t = plan->t;
   const int P = plan->planes;
   const int64_t lda = (int64_t)t.Km * 2 * t.C, ldh = (int64_t)t.Km * t.H;
@@ -807,27 +779,33 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                    rl ? &ws.gr : nullptr,
                                    zp_scale_of(7.4f, ws.scales + kScDa1, ws.scales + kScGrScale,
                                                ws.scales + kScX)));
+  // What is left are short kernels, most of them waiting on one another: the node sums and the last
+  // sums of the convolutions' parameter gradients on the first side stream, the radial layer's
+  // parameter gradients on the second, the way to the positions on the caller's.
+  if ((rc = lanes.fork())) return rc;
+  if (grad_x_node)
+    ZP_TIMED(ZP_K_SRC_REDUCE,
+             zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
+                                   grad_x_node, lanes.pick(1)));
+  if (want_w) {
+    zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
+    ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, lanes.pick(1)));
+  }
   if (rl && E > 0) {
     ZP_TIMED(ZP_K_GEMM_WGRAD,
              zp_linear_backward_planes(plan, E, rl->ec, t.R, ws.hr, ws.rw, ws.gr, rl->grad_h,
                                        rl->grad_w, rl->grad_b, ws.rad_partials,
-                                       zp_radial_splits(t.R, rl->ec),
-                                       ws.col_rad, list, st, rl->grad_h_max));
+                                       zp_radial_splits(t.R, rl->ec), ws.col_rad, radial_list, st,
+                                       lanes.pick(2), rl->grad_h_max));
   } else if (rl && rl->grad_w) {
     ZP_CUDA(cudaMemsetAsync(rl->grad_w, 0, sizeof(float) * (size_t)t.R * rl->ec, st));
     ZP_CUDA(cudaMemsetAsync(rl->grad_b, 0, sizeof(float) * (size_t)t.R, st));
   }
-  if (grad_x_node)
-    ZP_TIMED(ZP_K_SRC_REDUCE,
-             zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
-                                   grad_x_node, st));
   ZP_TIMED(ZP_K_WIGNER_BWD,
            zp_launch_edge_vec_grad(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.torque,
                                    ZpTorqueArgs{ws.da1, radial, c.x_node, ws.y, grad_node_out, c.env,
                                                 ws.rot, c.src, c.dst},
                                    grad_edge_vec, st));
-  if (want_w)
-    zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
   return ZP_OK;
 }
 
@@ -868,9 +846,11 @@ static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float 
   const ZpConv c{N, E, x_node, edge_vec, cos_g, sin_g, radial, env, src, dst, row_ptr, perm_src,
                  row_ptr_src, w};
   ZpFinalList list;
+  ZpLanes lanes(plan, E, st);
   if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, grad_edge_vec, grad_radial,
-                             grad_env, gw, rl, list, st)))
+                             grad_env, gw, rl, list, lanes)))
     return rc;
+  if ((rc = lanes.join())) return rc;
   ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, st));
   return ZP_OK;
 }

@@ -153,9 +153,16 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
   float *sc = ws.scales;
   const bool x_scale = plan->fp16 || fm.f2.fp16;
 
-  ZpMaxList maxima;
-  ZpPrepList prep;
-  zp_add_so2_weights(plan, &params->so2, ws.wfold, sc + kScWeights, maxima, prep);
+  // The convolutions' weights and the embeddings are first read after the radial MLP: their maxima
+  // and planes are formed beside it, on a side stream, unless there are none (the two calls then
+  // share their launches).
+  ZpLanes lanes(plan, E, st);
+  ZpMaxList maxima, late_maxima_;
+  ZpPrepList prep, late_prep_;
+  ZpMaxList &late_maxima = lanes.on ? late_maxima_ : maxima;
+  ZpPrepList &late_prep = lanes.on ? late_prep_ : prep;
+  zp_add_so2_weights(plan, &params->so2, ws.wfold, sc + kScWeights, late_maxima, late_prep,
+                     keep_for_backward);
   if (E > 0) {
     prep.add(params->rad_w[0], b.w0.base, sc + kScW0, b.w0.plane_stride, ec, w0, (int)b.w0.ld,
              ZP_PREP_PLAIN, fm.f0.planes, fm.f0.fp16);
@@ -174,12 +181,15 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
     if (g0) maxima.add(params->ln_beta[0], ec, sc + kScBeta0);
     if (g1) maxima.add(params->ln_gamma[1], ec, sc + kScGamma1);
     if (g1) maxima.add(params->ln_beta[1], ec, sc + kScBeta1);
-    if (x_scale && !x_ready_event) maxima.add(call->x_node, call->n_rows * t.K * t.C, sc + kScX);
+    if (x_scale && !x_ready_event) late_maxima.add(call->x_node, call->n_rows * t.K * t.C, sc + kScX);
   }
-  if (maxima.n) {
-    ZP_CUDA(cudaMemsetAsync(sc, 0, sizeof(float) * kScCount, st));
-    ZP_TIMED(ZP_K_FOLD, zp_launch_max_list(maxima, st));
+  if (maxima.n || late_maxima.n) ZP_CUDA(cudaMemsetAsync(sc, 0, sizeof(float) * kScCount, st));
+  if (lanes.on) {
+    if ((rc = lanes.fork(1))) return rc;
+    ZP_TIMED(ZP_K_FOLD, zp_launch_max_list(late_maxima, lanes.pick(1)));
+    ZP_TIMED(ZP_K_FOLD, zp_launch_prep_weights(late_prep, lanes.pick(1)));
   }
+  ZP_TIMED(ZP_K_FOLD, zp_launch_max_list(maxima, st));
   ZP_TIMED(ZP_K_FOLD, zp_launch_prep_weights(prep, st));
   if (E > 0) {
     float *mean0 = b.stats, *rstd0 = b.stats + E, *mean1 = b.stats + 2 * E, *rstd1 = b.stats + 3 * E;
@@ -192,6 +202,9 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
                                           b.dist, nullptr, &b.xe, xe_scale, b.env, b.cos_s, b.sin_s,
                                           st)))
       return rc;
+    if ((rc = lanes.fork(1))) return rc;
+    ZP_TIMED(ZP_K_WIGNER_FWD, zp_launch_wigner_fwd(plan, E, b.edge_vec, b.cos_s, b.sin_s, ws.rot, 0,
+                                                   lanes.pick(1)));
     const ZpGemmTc g0{E, ec, w0, b.xe.planes, b.xe.base, b.xe.ld, b.xe.plane_stride, 0,
                       b.w0.base, b.w0.ld, b.w0.plane_stride, 0, params->rad_b[0], b.h0, ec,
                       plan->status_dev, 0, 1, 0, 0, b.xe.fp16, b.xe.scale, b.w0.scale, nullptr};
@@ -212,6 +225,7 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
       return rc;
     if ((rc = zp_core_radial(plan, ws, E, ec, params->rad_b[2], st))) return rc;
   }
+  if ((rc = lanes.join(1))) return rc;
   if (x_ready_event) {                   // x_node is first read from here on
     ZP_CUDA(cudaStreamWaitEvent(st, (cudaEvent_t)x_ready_event, 0));
     if (x_scale && E > 0) {
@@ -222,7 +236,7 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
   }
   const ZpConv c{N, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
                  call->dst, call->row_ptr + call->first_node, nullptr, nullptr, &params->so2};
-  return zp_core_forward(plan, ws, c, node_out, keep_for_backward, st);
+  return zp_core_forward(plan, ws, c, node_out, keep_for_backward, lanes);
 }
 
 int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const zp_block_call *call,
@@ -264,8 +278,9 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                    grads->rad_w[2], grads->rad_b[2], fm.f1.fp16 ? sc + kScGHid1 : nullptr};
   const ZpConv c{rows, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
                  call->dst, call->row_ptr, call->perm_src, call->row_ptr_src, &params->so2};
+  ZpLanes lanes(plan, E, st);
   if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, b.g_vec_rot, nullptr, b.g_env,
-                             want_so2 ? &grads->so2 : nullptr, &rl, list, st)))
+                             want_so2 ? &grads->so2 : nullptr, &rl, list, lanes)))
     return rc;
   if (E == 0) {
     auto zero = [&](float *p, size_t n) { return p ? cudaMemsetAsync(p, 0, n * sizeof(float), st) : cudaSuccess; };
@@ -291,9 +306,10 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                                                   sc + kScDz1),
                                     grads->ln_gamma[1], grads->ln_beta[1], grads->rad_b[1], ln1, list, st)))
       return rc;
+    if (want_rad && (rc = lanes.fork(2))) return rc;       // their weight gradients on the side
     if ((rc = zp_linear_backward_planes(plan, E, ec, ec, b.hid0, b.w1, b.dz1, b.g_hid0,
                                         grads->rad_w[1], nullptr, b.part1, zp_radial_splits(ec, ec), nullptr,
-                                        list, st, fm.f0.fp16 ? sc + kScGHid0 : nullptr)))
+                                        list, st, lanes.pick(2), fm.f0.fp16 ? sc + kScGHid0 : nullptr)))
       return rc;
     if ((rc = zp_launch_ln_silu_bwd(E, ec, b.h0, params->ln_gamma[0], params->ln_beta[0], mean0, rstd0,
                                     b.g_hid0, nullptr, &b.dz0,
@@ -304,9 +320,10 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
     // without an embedding gradient only the distance basis' columns of the input gradient are used
     const int64_t cols = grads->emb ? w0 : front->num_basis;
     const bool want_in = grad_pos || grads->emb;
+    if (want_rad && (rc = lanes.fork(2))) return rc;
     if ((rc = zp_linear_backward_planes(plan, E, w0, ec, b.xe, b.w0, b.dz0, want_in ? b.g_xe : nullptr,
                                         grads->rad_w[0], nullptr, b.part0, zp_radial_splits(ec, w0), nullptr,
-                                        list, st, nullptr, cols)))
+                                        list, st, lanes.pick(2), nullptr, cols)))
       return rc;
     if (want_in &&
         (rc = zp_launch_edge_features_bwd(*front, rows, E, b.edge_vec, b.dist, params->gauss_offsets,
@@ -315,6 +332,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                                           grad_pos, grads->emb, b.front, st)))
       return rc;
   }
+  if ((rc = lanes.join())) return rc;
   ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, st));
   return ZP_OK;
 }

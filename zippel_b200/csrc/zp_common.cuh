@@ -122,8 +122,22 @@ int zp_ensure_smem(Kernel kernel, size_t bytes, ZpSmemOptIn &state) {
   return ZP_OK;
 }
 
-// ---- lists of small jobs that share one launch (blockIdx.y = entry) ---------------------------
+// ---- lists of small jobs that share one launch ------------------------------------------------
+// The tiles of all entries stand in one row, entry i's from first[i] on, and blocks walk the row: a
+// block column for each entry, as long as the largest needs, started 18 000 blocks to find most of
+// them without work.
 #define ZP_MAX_ITEMS 32
+struct ZpTileRow {
+  int n = 0;
+  int first[ZP_MAX_ITEMS + 1] = {0};
+  void add(int64_t tiles) { first[n + 1] = first[n] + (int)tiles; ++n; }
+  int total() const { return first[n]; }
+  // entry that tile `t` belongs to, not before entry `from`
+  __device__ __forceinline__ int entry(int t, int from = 0) const {
+    while (t >= first[from + 1]) ++from;
+    return from;
+  }
+};
 struct ZpMaxList {                              // *out = max |x[0 .. count)|, out zeroed beforehand
   int n = 0;
   const float *x[ZP_MAX_ITEMS];
@@ -153,6 +167,7 @@ struct ZpPrepList {                             // weight matrices to 16-bit pla
   int64_t plane_stride[ZP_MAX_ITEMS];
   int out[ZP_MAX_ITEMS], in[ZP_MAX_ITEMS], ld[ZP_MAX_ITEMS];
   int8_t kind[ZP_MAX_ITEMS], planes[ZP_MAX_ITEMS], fp16[ZP_MAX_ITEMS];
+  bool transposes = true;                       // of kept and folded matrices
   void add(const float *src, void *to, float *max_and_scale, int64_t stride, int rows, int cols,
            int row_stride, int what, int n_planes, int is_fp16) {
     w[n] = src; dst[n] = static_cast<uint16_t *>(to); slot[n] = max_and_scale;
@@ -168,7 +183,7 @@ struct ZpFinalList {                            // last sums of the parameter gr
   int64_t stride[ZP_MAX_ITEMS];                 // elements between partials
   int rows[ZP_MAX_ITEMS], cols[ZP_MAX_ITEMS], parts[ZP_MAX_ITEMS];
   int ld[ZP_MAX_ITEMS];                         // row stride of a partial
-  int8_t kind[ZP_MAX_ITEMS];
+  int8_t kind[ZP_MAX_ITEMS], quads[ZP_MAX_ITEMS];   // quads: set by the launch
   void add(const float *partials, float *to, int64_t between, int n_rows, int n_cols, int n_parts,
            int what, int row_stride = 0) {
     src[n] = partials; dst[n] = to; stride[n] = between; ld[n] = row_stride ? row_stride : n_cols;
@@ -321,7 +336,7 @@ int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t 
                            const ZpPlanes &out, const ZpScale &scale, cudaStream_t st);
 int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st);
 int zp_launch_prep_weights(const ZpPrepList &list, cudaStream_t st);
-int zp_launch_finalize(const ZpFinalList &list, cudaStream_t st);
+int zp_launch_finalize(ZpFinalList &list, cudaStream_t st);
 // *out = largest node index in src / dst (device scalar, zeroed by the caller)
 int zp_launch_max_index(int64_t E, const int32_t *src, const int32_t *dst, int *out,
                         cudaStream_t st);
@@ -335,8 +350,9 @@ int zp_launch_absmax_row_range(const float *in, int64_t cols, const int32_t *fir
 // zp_launch_prep_weights: per block W_fold [P][out][in] followed by its transpose [P][in][out], at
 // element offset c{1,2}_woff[m] of `packed`; `scales`: per block (conv * (ZP_MAX_L+1) + m) two
 // floats {max |W|, scale}.
+// (the transpose only if a backward follows: `transposes`)
 void zp_add_so2_weights(const zp_plan *p, const zp_weights *w, void *packed, float *scales,
-                        ZpMaxList &maxima, ZpPrepList &prep);
+                        ZpMaxList &maxima, ZpPrepList &prep, bool transposes);
 // ... and their gradients, for zp_launch_finalize: per split s the folded fp32 gradients stand at
 // partials + s*split_stride + c{1,2}_goff[m]
 void zp_add_so2_grads(const zp_plan *p, const float *partials, int64_t split_stride,
@@ -362,9 +378,14 @@ int zp_launch_ln_silu_bwd(int64_t rows, int width, const float *x, const float *
                           float *dgamma, float *dbeta, float *dbias, float *partial,
                           ZpFinalList &list, cudaStream_t st);
 // VJP of y = x W^T + b with all operands as planes (of one format); `partials`: max_splits * N *
-// round4(K) floats, `colsum_scratch`: ceil(M / 512) * N floats.  dw and db get their last sums from `list`
-// (zp_launch_finalize); dx_absmax: device scalar updated with max |dx|, or null; dx_cols: how many
-// leading columns of dx are wanted (0: all K), ld_dx its row stride (0: K)
+// round4(K) floats, `colsum_scratch`: zp_colsum_parts(M, N) * N floats.  dw and db, formed on
+// `side`, get their last sums from `list` (zp_launch_finalize); dx_absmax: device scalar updated with
+// max |dx|, or null; dx_cols: how many leading columns of dx are wanted (0: all K)
+int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t N,
+                              const ZpPlanes &x, const ZpPlanes &w, const ZpPlanes &dy, float *dx,
+                              float *dw, float *db, float *partials, int max_splits,
+                              float *colsum_scratch, ZpFinalList &list, cudaStream_t st,
+                              cudaStream_t side, float *dx_absmax = nullptr, int64_t dx_cols = 0);
 // zp_linear_forward / zp_linear_backward_saved for a caller whose own kernels found the maxima.
 // `slots` (the start of the work buffer): {max x, scale, max w, scale, max dy, scale, and two words
 // for the caller's use}; with fp16 planes the maxima stand there when these are called.
@@ -374,12 +395,15 @@ int zp_linear_forward_maxima(const zp_plan *plan, int64_t M, int64_t K, int64_t 
                              cudaStream_t st);
 int zp_linear_backward_maxima(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const float *dy,
                               float *dx, float *dw, float *db, void *work, cudaStream_t st);
-int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t N,
-                              const ZpPlanes &x, const ZpPlanes &w, const ZpPlanes &dy, float *dx,
-                              float *dw, float *db, float *partials, int max_splits,
-                              float *colsum_scratch, ZpFinalList &list, cudaStream_t st,
-                              float *dx_absmax = nullptr, int64_t dx_cols = 0);
-// column sums of `a`: partial sums into scratch (ceil(rows / 512) * cols floats), the rest by `list`
+// column sums of `a`: partial sums into scratch (zp_colsum_parts(rows, cols) * cols floats), the rest by
+// `list`.  A part has 512 rows, or fewer (64 at least) where that leaves less than eight blocks per SM.
+inline int64_t zp_colsum_rows(int64_t rows, int64_t cols) {
+  const int64_t each = zp_ceil_div(rows * zp_ceil_div(cols, 256), 148 * 8);
+  return each <= 64 ? 64 : each >= 512 ? 512 : zp_ceil_div(each, 8) * 8;
+}
+inline int64_t zp_colsum_parts(int64_t rows, int64_t cols) {
+  return rows > 0 ? zp_ceil_div(rows, zp_colsum_rows(rows, cols)) : 0;
+}
 int zp_launch_colsum(int64_t rows, int64_t cols, const ZpPlanes &a, float *out, float *scratch,
                      ZpFinalList &list, cudaStream_t st);
 

@@ -3,6 +3,7 @@
 #pragma once
 
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "zp_common.cuh"
@@ -98,7 +99,6 @@ inline int zp_radial_splits(int64_t N, int64_t K) {
   const int64_t tiles = zp_ceil_div(N, 128) * zp_ceil_div(K, 256), s = 148 / tiles;
   return (int)(s < 8 ? 8 : s > 64 ? 64 : s);
 }
-constexpr int kZpColRows = 512;          // rows per partial column sum
 
 //   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials
 //   backward: dy planes | dht | dh1 planes | da1 | du_src | torque | wgrad partials | scratch
@@ -121,6 +121,43 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
                      ZpFormat rad);
 
 // One convolution call.  Per-edge arrays are in the sorted order.
+// The caller's stream plus the plan's two side streams for one forward / backward call.  Up to
+// kZpLaneEdges edges everything stays on the caller's: the kernels are then shorter than the host
+// takes to launch them, and every event makes it take longer.
+constexpr int64_t kZpLaneEdges = 4096;
+bool zp_lanes_enabled();
+struct ZpLanes {
+  const zp_plan *p;
+  cudaStream_t main;
+  bool on;
+  std::unique_lock<std::mutex> hold;
+  ZpLanes(const zp_plan *plan, int64_t edges, cudaStream_t st)
+      : p(plan), main(st),
+        on(edges > kZpLaneEdges && zp_lanes_enabled() && !plan->timer && plan->aux_stream[0]) {
+    if (on) hold = std::unique_lock<std::mutex>(*static_cast<std::mutex *>(plan->lane_lock));
+  }
+  cudaStream_t pick(int i) const { return (!on || i % 3 == 0) ? main : p->aux_stream[i % 3 - 1]; }
+  // side streams (`which`: bit 0 the first, bit 1 the second) continue from what the caller's
+  // stream has been given so far
+  int fork(int which = 3) {
+    if (!on) return ZP_OK;
+    ZP_CUDA(cudaEventRecord(p->ev_fork, main));
+    for (int i = 0; i < 2; ++i)
+      if (which >> i & 1) ZP_CUDA(cudaStreamWaitEvent(p->aux_stream[i], p->ev_fork, 0));
+    return ZP_OK;
+  }
+  // the caller's stream continues after everything the side streams have been given
+  int join(int which = 3) {
+    if (!on) return ZP_OK;
+    for (int i = 0; i < 2; ++i) {
+      if (!(which >> i & 1)) continue;
+      ZP_CUDA(cudaEventRecord(p->ev_join[i], p->aux_stream[i]));
+      ZP_CUDA(cudaStreamWaitEvent(main, p->ev_join[i], 0));
+    }
+    return ZP_OK;
+  }
+};
+
 struct ZpConv {
   int64_t N, E;
   const float *x_node, *edge_vec, *cos_g, *sin_g, *radial, *env;
@@ -141,13 +178,15 @@ int zp_check_weights(const zp_plan *p, const zp_weights *w);
 // radial = hr rw^T + b into ws.radial, its largest magnitude into the scale array
 int zp_core_radial(const zp_plan *plan, const ZpWorkspace &ws, int64_t E, int ec, const float *bias,
                    cudaStream_t st);
-// Everything from the rotation matrices to node_out; the maxima of x_node and radial and the weight
-// planes are in place.  keep != 0: what a backward reads is left in the workspace.
+// Everything from the rotation into the edge frame to node_out; the rotation matrices, the maxima of
+// x_node and radial and the weight planes are in place.  keep != 0: what a backward reads is left in
+// the workspace.
 int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c, float *node_out,
-                    int keep, cudaStream_t st);
+                    int keep, ZpLanes &lanes);
 // gw null: no weight gradients; grad_x_node null: no node contributions.  With rl the gradient of
-// radial stays inside.  The last sums of the parameter gradients are left to `list`.
+// radial stays inside.  The last sums of the radial layer's parameter gradients are left to `list`;
+// both side streams are still to be joined.
 int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
                      const float *grad_node_out, float *grad_x_node, float *grad_edge_vec,
                      float *grad_radial, float *grad_env, const zp_weight_grads *gw,
-                     const ZpRadialLayer *rl, ZpFinalList &list, cudaStream_t st);
+                     const ZpRadialLayer *rl, ZpFinalList &list, ZpLanes &lanes);

@@ -12,6 +12,8 @@
 // Every m-block of conv1 and conv2 is therefore a plain  Y[E, out] = X[E, in] W_fold^T.
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "zp_common.cuh"
 
 namespace {
@@ -218,27 +220,38 @@ __global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant_
 // ------------------------------------------------------------------------------------------
 // weight folding and its transpose
 // ------------------------------------------------------------------------------------------
-// Maxima of up to ZP_MAX_ITEMS arrays in one launch (blockIdx.y = array; the caller zeroed the slots):
-// every weight block, and whatever else a call needs the magnitude of before its first product.
-__global__ void __launch_bounds__(256) max_list_kernel(const __grid_constant__ ZpMaxList d) {
-  const int b = blockIdx.y;
-  const float *x = d.x[b];
-  const int64_t n = d.count[b], step = (int64_t)gridDim.x * blockDim.x;
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float m = 0.f;
-  if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
-    const float4 *x4 = reinterpret_cast<const float4 *>(x);
-    for (; i < n / 4; i += step) {
-      const float4 v = x4[i];
-      m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+// Maxima of up to ZP_MAX_ITEMS arrays in one launch (the caller zeroed the slots): every weight block,
+// and whatever else a call needs the magnitude of before its first product.  A block takes a stretch
+// of neighbouring tiles of 4096 values and leaves one atomic per warp and array.
+constexpr int kMaxTile = 4096;
+__global__ void __launch_bounds__(256)
+max_list_kernel(const __grid_constant__ ZpMaxList d, const __grid_constant__ ZpTileRow row) {
+  const int total = row.first[row.n];
+  int t = (int)((int64_t)total * blockIdx.x / gridDim.x);
+  const int end = (int)((int64_t)total * (blockIdx.x + 1) / gridDim.x);
+  for (int b = 0; t < end;) {
+    b = row.entry(t, b);
+    const float *x = d.x[b];
+    const int last = min(end, row.first[b + 1]);
+    const int64_t i0 = (int64_t)(t - row.first[b]) * kMaxTile;
+    const int64_t i1 = min(d.count[b], (int64_t)(last - row.first[b]) * kMaxTile);
+    float m = 0.f;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+      const float4 *x4 = reinterpret_cast<const float4 *>(x);
+#pragma unroll 4
+      for (int64_t i = i0 / 4 + threadIdx.x; i < i1 / 4; i += 256) {
+        const float4 v = x4[i];
+        m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+      }
+      if ((int)threadIdx.x < (int)(i1 & 3)) m = fmaxf(m, fabsf(x[(i1 & ~3ll) + threadIdx.x]));
+    } else {
+      for (int64_t i = i0 + threadIdx.x; i < i1; i += 256) m = fmaxf(m, fabsf(x[i]));
     }
-    if (blockIdx.x == 0 && threadIdx.x < (n & 3)) m = fmaxf(m, fabsf(x[(n & ~3ll) + threadIdx.x]));
-  } else {
-    for (; i < n; i += step) m = fmaxf(m, fabsf(x[i]));
-  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(d.out[b], m);
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0.f) zp_atomic_absmax(d.out[b], m);
+    t = last;
+  }
 }
 
 // Writes every weight matrix as 16-bit planes, all of them in one launch (blockIdx.y = matrix).
@@ -246,58 +259,67 @@ __global__ void __launch_bounds__(256) max_list_kernel(const __grid_constant__ Z
 //   kept / folded  W_fold [out, in] and its transpose [in, out];  m = 0 (kept): W_fold = W,
 //                  m > 0 (folded): W = [Wa ; Wb] (rows), W_fold = [Wa -Wb ; Wb Wa]
 // slot = {max |W|, scale}: the scale follows from the maximum here (fp16 planes).
-__global__ void __launch_bounds__(256) prep_weights_kernel(const __grid_constant__ ZpPrepList d) {
+__global__ void __launch_bounds__(256)
+prep_weights_kernel(const __grid_constant__ ZpPrepList d, const __grid_constant__ ZpTileRow tiles) {
   // 32 x 32 tiles: the planes of W_fold go out row-major as they are formed; the transpose is
   // written from a shared copy of the tile so that both stores run along the fastest axis.
   __shared__ uint16_t tile[3][32][34];
-  const int b = blockIdx.y;
-  const int out = d.out[b], in = d.in[b], kind = d.kind[b], planes = d.planes[b], fp16 = d.fp16[b];
-  const int ld = d.ld[b];
-  const int64_t stride = d.plane_stride[b];
-  uint16_t *wp = d.dst[b], *wtp = wp + (size_t)planes * stride;
-  float inv = 1.f;
-  if (fp16) {
-    const float s = zp_scale_for_bound(d.slot[b][0]);
-    inv = 1.f / s;
-    if (blockIdx.x == 0 && threadIdx.x == 0) d.slot[b][1] = s;
-  }
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;          // 32 x 8
-  const int cols = kind == ZP_PREP_PLAIN ? ld : in;
-  const int tiles_c = (cols + 31) / 32, tiles = ((out + 31) / 32) * tiles_c;
-  for (int tl = blockIdx.x; tl < tiles; tl += gridDim.x) {
+  int b = 0;
+  for (int t = blockIdx.x; t < tiles.first[tiles.n]; t += gridDim.x) {
+    b = tiles.entry(t, b);
+    const int out = d.out[b], in = d.in[b], kind = d.kind[b], planes = d.planes[b], fp16 = d.fp16[b];
+    const int ld = d.ld[b], tl = t - tiles.first[b];
+    const float *__restrict__ w = d.w[b];
+    const int64_t stride = d.plane_stride[b];
+    uint16_t *wp = d.dst[b], *wtp = wp + (size_t)planes * stride;
+    float inv = 1.f;
+    if (fp16) {
+      const float s = zp_scale_for_bound(d.slot[b][0]);
+      inv = 1.f / s;
+      if (tl == 0 && threadIdx.x == 0) d.slot[b][1] = s;
+    }
+    const int cols = kind == ZP_PREP_PLAIN ? ld : in;
+    const int tiles_c = (cols + 31) / 32;
     const int r0 = (tl / tiles_c) * 32, c0 = (tl % tiles_c) * 32;
+    const int half = out / 2, kin = in / 2;
+    float v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const int row = r0 + ty + 8 * k, col = c0 + tx;
-      if (row < out && col < cols) {
-        float v = 0.f;
+      v[k] = 0.f;
+      if (row < out && col < in) {
         if (kind != ZP_PREP_FOLDED) {
-          if (col < in) v = d.w[b][(size_t)row * in + col];
+          v[k] = w[(size_t)row * in + col];
         } else {
-          const int half = out / 2, kin = in / 2;
           const bool lower = row >= half, right = col >= kin;
           const int o = lower ? row - half : row, c = right ? col - kin : col;
-          v = d.w[b][(size_t)((lower != right) ? half + o : o) * kin + c];
-          if (!lower && right) v = -v;
-        }
-        v *= inv;
-        for (int p = 0; p < planes; ++p) {
-          uint16_t h;
-          if (fp16) {
-            const __half q = __float2half_rn(v);
-            h = __half_as_ushort(q);
-            v -= __half2float(q);
-          } else {
-            const __nv_bfloat16 q = __float2bfloat16_rn(v);
-            h = __bfloat16_as_ushort(q);
-            v -= __bfloat162float(q);
-          }
-          wp[(size_t)p * stride + (size_t)row * ld + col] = h;
-          tile[p][ty + 8 * k][tx] = h;
+          v[k] = w[(size_t)((lower != right) ? half + o : o) * kin + c];
+          if (!lower && right) v[k] = -v[k];
         }
       }
     }
-    if (kind == ZP_PREP_PLAIN) continue;         // uniform over the block
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = r0 + ty + 8 * k, col = c0 + tx;
+      if (row >= out || col >= cols) continue;
+      float x = v[k] * inv;
+      for (int p = 0; p < planes; ++p) {
+        uint16_t h;
+        if (fp16) {
+          const __half q = __float2half_rn(x);
+          h = __half_as_ushort(q);
+          x -= __half2float(q);
+        } else {
+          const __nv_bfloat16 q = __float2bfloat16_rn(x);
+          h = __bfloat16_as_ushort(q);
+          x -= __bfloat162float(q);
+        }
+        wp[(size_t)p * stride + (size_t)row * ld + col] = h;
+        tile[p][ty + 8 * k][tx] = h;
+      }
+    }
+    if (kind == ZP_PREP_PLAIN || !d.transposes) continue;         // uniform over the block
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -310,70 +332,96 @@ __global__ void __launch_bounds__(256) prep_weights_kernel(const __grid_constant
   }
 }
 
-// The last step of every parameter gradient, all of them in one launch (blockIdx.y = gradient).
+// The last step of every parameter gradient, all of them in one launch.
 //   ZP_FIN_SUM     sum of `parts` partial matrices (K splits of a product), in order
 //   ZP_FIN_UNFOLD  the same, mapped from the folded layout back to the reference's:
 //                  dWa = F[0,0] + F[1,1], dWb = F[1,0] - F[0,1]
-//   ZP_FIN_COLUMN  sum of `parts` partial rows: 32 columns per block, eight threads per column take
+//   ZP_FIN_COLUMN  sum of `parts` partial rows: 32 columns per tile, eight threads per column take
 //                  every eighth row, and their sums are added in order
-__global__ void __launch_bounds__(256) finalize_kernel(const __grid_constant__ ZpFinalList d) {
-  __shared__ float red[8][33];
-  const int b = blockIdx.y;
-  const float *f = d.src[b];
-  float *dst = d.dst[b];
-  const int64_t stride = d.stride[b];
-  const int rows = d.rows[b], cols = d.cols[b], parts = d.parts[b], kind = d.kind[b];
-  if (kind == ZP_FIN_COLUMN) {
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int c0 = blockIdx.x * 32; c0 < cols; c0 += gridDim.x * 32) {
-      const int c = c0 + tx;
-      float s = 0.f;
-      if (c < cols) {
-#pragma unroll 4
-        for (int p = ty; p < parts; p += 8) s += f[(size_t)p * stride + c];
-      }
-      red[ty][tx] = s;
-      __syncthreads();
-      if (ty == 0 && c < cols) {
-        float acc = 0.f;
-#pragma unroll
-        for (int g = 0; g < 8; ++g) acc += red[g][tx];
-        dst[c] = acc;
-      }
-      __syncthreads();
-    }
-    return;
-  }
-  const bool folded = kind == ZP_FIN_UNFOLD;
-  const int ld = d.ld[b];
+// Bound by the partials it reads.  A tile of the matrices has 256 groups of V neighbouring entries.
+template <int V>
+__device__ __forceinline__ void finalize_entries(const float *__restrict__ f, float *__restrict__ dst,
+                                                 int64_t stride, int rows, int cols, int parts, int ld,
+                                                 bool folded, int64_t tile) {
   const int kin = folded ? cols / 2 : cols, half = rows / 2;
-  const int64_t total = (int64_t)rows * kin;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(idx % kin), row = (int)(idx / kin);
-    float acc = 0.f;
-    for (int s = 0; s < parts; ++s) {
-      const float *fs = f + (size_t)s * stride;
-      const float v = fs[(size_t)row * ld + c];
-      if (!folded) acc += v;
-      else if (row < half) acc += v + fs[(size_t)(half + row) * ld + kin + c];
-      else acc += v - fs[(size_t)(row - half) * ld + kin + c];
+  const int64_t idx = (tile * 256 + threadIdx.x) * V;
+  if (idx >= (int64_t)rows * kin) return;
+  const int c = (int)(idx % kin), row = (int)(idx / kin);
+  const bool upper = row < half;
+  const float *p = f + (size_t)row * ld + c;
+  const float *q = f + (size_t)(upper ? half + row : row - half) * ld + kin + c;
+  const float sign = upper ? 1.f : -1.f;
+  float acc[V], v[V], u[V];
+#pragma unroll
+  for (int k = 0; k < V; ++k) acc[k] = 0.f;
+  auto load = [](const float *from, float (&to)[V]) {
+    if (V == 4) {
+      const float4 x = *reinterpret_cast<const float4 *>(from);
+      to[0] = x.x; to[V / 4] = x.y; to[V / 2] = x.z; to[V - 1] = x.w;
+    } else {
+      to[0] = *from;
     }
-    dst[idx] = acc;
+  };
+#pragma unroll 4
+  for (int s = 0; s < parts; ++s) {
+    load(p + (size_t)s * stride, v);
+    if (folded) {
+      load(q + (size_t)s * stride, u);
+#pragma unroll
+      for (int k = 0; k < V; ++k) v[k] += sign * u[k];
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k) acc[k] += v[k];
+  }
+  if (V == 4) *reinterpret_cast<float4 *>(dst + idx) = make_float4(acc[0], acc[V / 4], acc[V / 2], acc[V - 1]);
+  else dst[idx] = acc[0];
+}
+__global__ void __launch_bounds__(256)
+finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ ZpTileRow tiles) {
+  __shared__ float red[8][33];
+  int b = 0;
+  for (int t = blockIdx.x; t < tiles.first[tiles.n]; t += gridDim.x) {
+    b = tiles.entry(t, b);
+    const float *f = d.src[b];
+    float *dst = d.dst[b];
+    const int64_t stride = d.stride[b];
+    const int cols = d.cols[b], parts = d.parts[b], kind = d.kind[b], tile = t - tiles.first[b];
+    if (kind != ZP_FIN_COLUMN) {
+      const bool folded = kind == ZP_FIN_UNFOLD;
+      if (d.quads[b]) finalize_entries<4>(f, dst, stride, d.rows[b], cols, parts, d.ld[b], folded, tile);
+      else finalize_entries<1>(f, dst, stride, d.rows[b], cols, parts, d.ld[b], folded, tile);
+      continue;
+    }
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    const int c = tile * 32 + tx;
+    float s = 0.f;
+    if (c < cols) {
+#pragma unroll 4
+      for (int p = ty; p < parts; p += 8) s += f[(size_t)p * stride + c];
+    }
+    red[ty][tx] = s;
+    __syncthreads();
+    if (ty == 0 && c < cols) {
+      float acc = 0.f;
+#pragma unroll
+      for (int g = 0; g < 8; ++g) acc += red[g][tx];
+      dst[c] = acc;
+    }
+    __syncthreads();
   }
 }
 
-// column sums in two fixed-order stages.  Stage one: a block of 32 x 8 threads sums 128 rows of
+// column sums in two fixed-order stages.  Stage one: a block of 32 x 8 threads sums `per_block` rows of
 // 256 columns; a thread owns 8 consecutive columns (one 16-byte load per row and plane) and every
 // eighth row, the eight row groups are then added in order through shared memory.
-constexpr int kColRowsPerBlock = 512;
 __global__ void __launch_bounds__(256)
-colsum_part_kernel(int64_t rows, int64_t cols, const ZpPlanes a, float *__restrict__ part) {
+colsum_part_kernel(int64_t rows, int64_t cols, int64_t per_block, const ZpPlanes a,
+                   float *__restrict__ part) {
   __shared__ float red[8][32][9];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int64_t c0 = ((int64_t)blockIdx.x * 32 + tx) * 8;
-  const int64_t r0 = (int64_t)blockIdx.y * kColRowsPerBlock;
-  const int64_t r1 = min(rows, r0 + kColRowsPerBlock);
+  const int64_t r0 = (int64_t)blockIdx.y * per_block;
+  const int64_t r1 = min(rows, r0 + per_block);
   float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   if (c0 < cols) {
 #pragma unroll 4
@@ -469,39 +517,35 @@ int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t 
 
 int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st) {
   if (list.n == 0) return ZP_OK;
-  // sixteen values per thread, so that small arrays take few blocks; the largest take two waves
-  int64_t most = 0;
-  for (int i = 0; i < list.n; ++i) most = list.count[i] > most ? list.count[i] : most;
-  int64_t gx = zp_ceil_div(most, 256 * 16);
-  if (gx > 1184) gx = 1184;
-  if (gx < 1) gx = 1;
-  max_list_kernel<<<dim3((unsigned)gx, list.n), 256, 0, st>>>(list);
+  ZpTileRow row;
+  for (int i = 0; i < list.n; ++i) row.add(zp_ceil_div(list.count[i], kMaxTile));
+  if (row.total() == 0) return ZP_OK;
+  max_list_kernel<<<(unsigned)std::min(row.total(), 148 * 8), 256, 0, st>>>(list, row);
   ZP_LAUNCH_CHECK("max_list_kernel");
   return ZP_OK;
 }
 
 int zp_launch_prep_weights(const ZpPrepList &list, cudaStream_t st) {
-  if (list.n == 0) return ZP_OK;
-  int64_t most = 1;                     // 32 x 32 tiles of the largest matrix
-  for (int i = 0; i < list.n; ++i) {
-    const int64_t t = zp_ceil_div(list.out[i], 32) * zp_ceil_div(list.ld[i], 32);
-    most = t > most ? t : most;
-  }
-  prep_weights_kernel<<<dim3((unsigned)(most > 296 ? 296 : most), list.n), 256, 0, st>>>(list);
+  ZpTileRow row;
+  for (int i = 0; i < list.n; ++i)
+    row.add(zp_ceil_div(list.out[i], 32) *
+            zp_ceil_div(list.kind[i] == ZP_PREP_PLAIN ? list.ld[i] : list.in[i], 32));
+  if (row.total() == 0) return ZP_OK;
+  prep_weights_kernel<<<(unsigned)std::min(row.total(), 148 * 16), 256, 0, st>>>(list, row);
   ZP_LAUNCH_CHECK("prep_weights_kernel");
   return ZP_OK;
 }
 
-int zp_launch_finalize(const ZpFinalList &list, cudaStream_t st) {
-  if (list.n == 0) return ZP_OK;
-  int64_t most = 1;
+int zp_launch_finalize(ZpFinalList &list, cudaStream_t st) {
+  ZpTileRow row;
   for (int i = 0; i < list.n; ++i) {
-    const int64_t t = list.kind[i] == ZP_FIN_COLUMN
-                          ? zp_ceil_div(list.cols[i], 32)
-                          : zp_ceil_div((int64_t)list.rows[i] * list.cols[i], 256);
-    most = t > most ? t : most;
+    const int kin = list.kind[i] == ZP_FIN_UNFOLD ? list.cols[i] / 2 : list.cols[i];
+    list.quads[i] = (kin | list.ld[i] | (int)(list.stride[i] & 3)) % 4 == 0 && ((uintptr_t)list.src[i] | (uintptr_t)list.dst[i]) % 16 == 0;
+    row.add(list.kind[i] == ZP_FIN_COLUMN ? zp_ceil_div(list.cols[i], 32)
+                                          : zp_ceil_div((int64_t)list.rows[i] * kin, list.quads[i] ? 1024 : 256));
   }
-  finalize_kernel<<<dim3((unsigned)(most > 148 ? 148 : most), list.n), 256, 0, st>>>(list);
+  if (row.total() == 0) return ZP_OK;
+  finalize_kernel<<<(unsigned)std::min(row.total(), 148 * 16), 256, 0, st>>>(list, row);
   ZP_LAUNCH_CHECK("finalize_kernel");
   return ZP_OK;
 }
@@ -554,7 +598,8 @@ static const float *block_weight(const zp_weights *w, int conv, int m) {
 }
 
 void zp_add_so2_weights(const zp_plan *p, const zp_weights *w, void *packed, float *scales,
-                        ZpMaxList &maxima, ZpPrepList &prep) {
+                        ZpMaxList &maxima, ZpPrepList &prep, bool transposes) {
+  prep.transposes = transposes;
   for (int conv = 0; conv < 2; ++conv)
     for (int m = 0; m < p->n_blocks; ++m) {
       const int out = conv ? p->c2_out[m] : p->c1_out[m], in = conv ? p->c2_in[m] : p->c1_in[m];
@@ -583,10 +628,10 @@ void zp_add_so2_grads(const zp_plan *p, const float *partials, int64_t split_str
 int zp_launch_colsum(int64_t rows, int64_t cols, const ZpPlanes &a, float *out, float *scratch,
                      ZpFinalList &list, cudaStream_t st) {
   if (cols == 0) return ZP_OK;
-  const int64_t nparts = rows > 0 ? zp_ceil_div(rows, kColRowsPerBlock) : 0;
+  const int64_t nparts = zp_colsum_parts(rows, cols);
   if (nparts > 0) {
     const dim3 grid((unsigned)zp_ceil_div(cols, 256), (unsigned)nparts), block(32, 8);
-    colsum_part_kernel<<<grid, block, 0, st>>>(rows, cols, a, scratch);
+    colsum_part_kernel<<<grid, block, 0, st>>>(rows, cols, zp_colsum_rows(rows, cols), a, scratch);
     ZP_LAUNCH_CHECK("colsum_part_kernel");
   }
   list.add(scratch, out, cols, 1, (int)cols, (int)nparts, ZP_FIN_COLUMN);

@@ -43,7 +43,7 @@ LinWork carve_lin(const zp_plan *p, int64_t M, int64_t K, int64_t N, void *base)
   w.w = planes(N, K, w.scales + kLinSlotW + 1);
   w.dy = planes(M, N, w.scales + kLinSlotDy + 1);
   w.partials = reinterpret_cast<float *>(take(sizeof(float) * kLinSplits * N * K));
-  w.colsum = reinterpret_cast<float *>(take(sizeof(float) * (size_t)zp_ceil_div(M > 0 ? M : 1, 128) * N));
+  w.colsum = reinterpret_cast<float *>(take(sizeof(float) * (size_t)(zp_colsum_parts(M, N) * N)));
   w.bytes = off;
   return w;
 }
@@ -84,7 +84,7 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
                               const ZpPlanes &x, const ZpPlanes &w, const ZpPlanes &dy, float *dx,
                               float *dw, float *db, float *partials, int max_splits,
                               float *colsum_scratch, ZpFinalList &list, cudaStream_t st,
-                              float *dx_absmax, int64_t dx_cols) {
+                              cudaStream_t side, float *dx_absmax, int64_t dx_cols) {
   int rc;
   const int P = dy.planes, fp16 = dy.fp16;
   if (dx) {
@@ -101,10 +101,10 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
                0, 1, N * ldk, 0, fp16, dy.scale, x.scale, nullptr};
     g.ksplit = zp_gemm_tc_pick_splits(g, max_splits);
     const int splits = zp_gemm_tc_splits(g);
-    if ((rc = zp_launch_gemm_tc(g, st))) return rc;
+    if ((rc = zp_launch_gemm_tc(g, side))) return rc;
     list.add(partials, dw, N * ldk, (int)N, (int)K, splits, ZP_FIN_SUM, (int)ldk);
   }
-  if (db) return zp_launch_colsum(M, N, dy, db, colsum_scratch, list, st);
+  if (db) return zp_launch_colsum(M, N, dy, db, colsum_scratch, list, side);
   return ZP_OK;
 }
 
@@ -135,7 +135,7 @@ int backward_saved(const zp_plan *plan, int64_t M, int64_t K, int64_t N, const f
   if (rc) return rc;
   ZpFinalList list;
   if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
-                                      kLinSplits, lw.colsum, list, st)))
+                                      kLinSplits, lw.colsum, list, st, st)))
     return rc;
   return zp_launch_finalize(list, st);
 }
@@ -184,7 +184,7 @@ int zp_linear_backward(const zp_plan *plan, int64_t M, int64_t K, int64_t N, con
   if ((rc = split_scaled(plan, jobs, n, st))) return rc;
   ZpFinalList list;
   if ((rc = zp_linear_backward_planes(plan, M, K, N, lw.x, lw.w, lw.dy, dx, dw, db, lw.partials,
-                                      kLinSplits, lw.colsum, list, st)))
+                                      kLinSplits, lw.colsum, list, st, st)))
     return rc;
   return zp_launch_finalize(list, st);
 }
