@@ -174,3 +174,11 @@ def test_bounded_wait_runs_out_and_the_library_keeps_working():
     assert (c - want).abs().max().item() < 1e-3 * want.abs().max().item()
     assert plan.device_status() == 0
     assert lib.zp_selftest_bounded_wait(plan.handle, scratch.data_ptr(), 16, 1000, st) == 3   # workspace
+
+
+@pytest.mark.parametrize("planes,K", [(1, 8), (1, 200), (1, 256), (2, 36), (2, 64), (2, 128)])
+@pytest.mark.parametrize("M,N", [(1, 4), (128, 96), (129, 160), (40000, 40), (9000, 400)])
+def test_short_contractions(M, N, K, planes):
+    """The resident column block: widths that are no multiple of it, one to many columns per CTA."""
+    err_p, err_f = run_gemm(M, N, K, planes, False, False)
+    assert (err_p if planes == 1 else err_f) < 4e-6

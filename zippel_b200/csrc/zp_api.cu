@@ -668,7 +668,7 @@ int zp_eso2_forward_inference(const zp_plan *plan, int64_t N, int64_t E, const f
 int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
                      const float *grad_node_out, float *grad_x_node, float *grad_edge_vec,
                      float *grad_radial, float *grad_env, const zp_weight_grads *gw,
-                     const ZpRadialLayer *rl, ZpFinalList &radial_list, ZpLanes &lanes) {
+                     const ZpRadialLayer *rl, ZpLanes &lanes) {
   int rc;
   cudaStream_t st = lanes.main;
   ZpFinalList list;
@@ -779,28 +779,31 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                    rl ? &ws.gr : nullptr,
                                    zp_scale_of(7.4f, ws.scales + kScDa1, ws.scales + kScGrScale,
                                                ws.scales + kScX)));
-  // What is left are short kernels, most of them waiting on one another: the node sums and the last
-  // sums of the convolutions' parameter gradients on the first side stream, the radial layer's
-  // parameter gradients on the second, the way to the positions on the caller's.
+  // What is left are short kernels, most of them waiting on one another.  On the caller's stream
+  // the way to the positions, first of all its product: a product takes whole SMs and waits for all
+  // that was there before it.  On the second side stream the radial layer's parameter gradients,
+  // on the first the last sums of the convolutions' and the node sums.
   if ((rc = lanes.fork())) return rc;
-  if (grad_x_node)
-    ZP_TIMED(ZP_K_SRC_REDUCE,
-             zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
-                                   grad_x_node, lanes.pick(1)));
-  if (want_w) {
-    zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
-    ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, lanes.pick(1)));
-  }
   if (rl && E > 0) {
+    ZpFinalList radial_list;
     ZP_TIMED(ZP_K_GEMM_WGRAD,
              zp_linear_backward_planes(plan, E, rl->ec, t.R, ws.hr, ws.rw, ws.gr, rl->grad_h,
                                        rl->grad_w, rl->grad_b, ws.rad_partials,
                                        zp_radial_splits(t.R, rl->ec), ws.col_rad, radial_list, st,
                                        lanes.pick(2), rl->grad_h_max));
+    ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(radial_list, lanes.pick(2)));
   } else if (rl && rl->grad_w) {
     ZP_CUDA(cudaMemsetAsync(rl->grad_w, 0, sizeof(float) * (size_t)t.R * rl->ec, st));
     ZP_CUDA(cudaMemsetAsync(rl->grad_b, 0, sizeof(float) * (size_t)t.R, st));
   }
+  if (want_w) {
+    zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
+    ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, lanes.pick(1)));
+  }
+  if (grad_x_node)
+    ZP_TIMED(ZP_K_SRC_REDUCE,
+             zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
+                                   grad_x_node, lanes.pick(1)));
   ZP_TIMED(ZP_K_WIGNER_BWD,
            zp_launch_edge_vec_grad(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.torque,
                                    ZpTorqueArgs{ws.da1, radial, c.x_node, ws.y, grad_node_out, c.env,
@@ -845,14 +848,11 @@ static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float 
   cudaStream_t st = (cudaStream_t)stream;
   const ZpConv c{N, E, x_node, edge_vec, cos_g, sin_g, radial, env, src, dst, row_ptr, perm_src,
                  row_ptr_src, w};
-  ZpFinalList list;
   ZpLanes lanes(plan, E, st);
   if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, grad_edge_vec, grad_radial,
-                             grad_env, gw, rl, list, lanes)))
+                             grad_env, gw, rl, lanes)))
     return rc;
-  if ((rc = lanes.join())) return rc;
-  ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, st));
-  return ZP_OK;
+  return lanes.join();
 }
 
 int zp_eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float *grad_node_out,

@@ -280,7 +280,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                  call->dst, call->row_ptr, call->perm_src, call->row_ptr_src, &params->so2};
   ZpLanes lanes(plan, E, st);
   if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, b.g_vec_rot, nullptr, b.g_env,
-                             want_so2 ? &grads->so2 : nullptr, &rl, list, lanes)))
+                             want_so2 ? &grads->so2 : nullptr, &rl, lanes)))
     return rc;
   if (E == 0) {
     auto zero = [&](float *p, size_t n) { return p ? cudaMemsetAsync(p, 0, n * sizeof(float), st) : cudaSuccess; };

@@ -167,6 +167,7 @@ struct ZpPrepList {                             // weight matrices to 16-bit pla
   int64_t plane_stride[ZP_MAX_ITEMS];
   int out[ZP_MAX_ITEMS], in[ZP_MAX_ITEMS], ld[ZP_MAX_ITEMS];
   int8_t kind[ZP_MAX_ITEMS], planes[ZP_MAX_ITEMS], fp16[ZP_MAX_ITEMS];
+  int8_t quads[ZP_MAX_ITEMS];                   // set by the launch
   bool transposes = true;                       // of kept and folded matrices
   void add(const float *src, void *to, float *max_and_scale, int64_t stride, int rows, int cols,
            int row_stride, int what, int n_planes, int is_fp16) {
@@ -335,7 +336,7 @@ int zp_launch_split_list(const ZpSplitList &list, cudaStream_t st);
 int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,
                            const ZpPlanes &out, const ZpScale &scale, cudaStream_t st);
 int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st);
-int zp_launch_prep_weights(const ZpPrepList &list, cudaStream_t st);
+int zp_launch_prep_weights(ZpPrepList &list, cudaStream_t st);
 int zp_launch_finalize(ZpFinalList &list, cudaStream_t st);
 // *out = largest node index in src / dst (device scalar, zeroed by the caller)
 int zp_launch_max_index(int64_t E, const int32_t *src, const int32_t *dst, int *out,

@@ -184,9 +184,8 @@ int zp_core_radial(const zp_plan *plan, const ZpWorkspace &ws, int64_t E, int ec
 int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c, float *node_out,
                     int keep, ZpLanes &lanes);
 // gw null: no weight gradients; grad_x_node null: no node contributions.  With rl the gradient of
-// radial stays inside.  The last sums of the radial layer's parameter gradients are left to `list`;
-// both side streams are still to be joined.
+// radial stays inside.  Both side streams are still to be joined.
 int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
                      const float *grad_node_out, float *grad_x_node, float *grad_edge_vec,
                      float *grad_radial, float *grad_env, const zp_weight_grads *gw,
-                     const ZpRadialLayer *rl, ZpFinalList &list, ZpLanes &lanes);
+                     const ZpRadialLayer *rl, ZpLanes &lanes);

@@ -259,76 +259,112 @@ max_list_kernel(const __grid_constant__ ZpMaxList d, const __grid_constant__ ZpT
 //   kept / folded  W_fold [out, in] and its transpose [in, out];  m = 0 (kept): W_fold = W,
 //                  m > 0 (folded): W = [Wa ; Wb] (rows), W_fold = [Wa -Wb ; Wb Wa]
 // slot = {max |W|, scale}: the scale follows from the maximum here (fp16 planes).
+// Bound by instruction issue, so a thread takes V = 4 neighbouring columns where the widths allow (every
+// width in use): a value at a time took 115 instructions per value (38 us for the weights of lmax 4 /
+// mmax 2 / C 128 as one plane; now PREPUS).  Tiles of 32 rows and 32 V columns; the planes of W_fold go
+// out row-major as they are formed, the transpose from a shared copy of the tile so that both
+// stores run along the fastest axis.
+constexpr int kPrepPitch = 130;
+template <int V>
+__device__ __forceinline__ void prep_tile(const ZpPrepList &d, int b, int tl, uint16_t (*tile)[kPrepPitch]) {
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;          // 32 x 8
+  const int out = d.out[b], in = d.in[b], kind = d.kind[b], planes = d.planes[b], ld = d.ld[b];
+  const bool fp16 = d.fp16[b];
+  const int64_t stride = d.plane_stride[b];
+  float inv = 1.f;
+  if (fp16) {
+    const float s = zp_scale_for_bound(d.slot[b][0]);
+    inv = 1.f / s;
+    if (tl == 0 && threadIdx.x == 0) d.slot[b][1] = s;
+  }
+  const int cols = kind == ZP_PREP_PLAIN ? ld : in;
+  const int tiles_c = (cols + 32 * V - 1) / (32 * V);
+  const int r0 = (tl / tiles_c) * 32, c0 = (tl % tiles_c) * 32 * V, c = c0 + tx * V;
+  const int half = out / 2, kin = in / 2;
+  const bool right = kind == ZP_PREP_FOLDED && c >= kin;
+  const float *__restrict__ w = d.w[b] + (right ? c - kin : c);
+  const int ld_w = kind == ZP_PREP_FOLDED ? kin : in;
+  float v[4][V];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int row = r0 + ty + 8 * k;
+#pragma unroll
+    for (int q = 0; q < V; ++q) v[k][q] = 0.f;
+    if (row >= out || c >= in) continue;
+    // the upper right quarter is -Wb, the lower right Wa
+    const int o = !right ? row : row < half ? row + half : row - half;
+    const float *from = w + (size_t)o * ld_w;
+    if (V == 4) {
+      const float4 x = *reinterpret_cast<const float4 *>(from);
+      v[k][0] = x.x; v[k][V / 4] = x.y; v[k][V / 2] = x.z; v[k][V - 1] = x.w;
+    } else {
+      v[k][0] = *from;
+    }
+    const float f = right && row < half ? -inv : inv;
+#pragma unroll
+    for (int q = 0; q < V; ++q) v[k][q] *= f;
+  }
+  const bool transpose = kind != ZP_PREP_PLAIN && d.transposes;
+  uint16_t *wp = d.dst[b], *wtp = wp + (size_t)planes * stride;
+  for (int p = 0; p < planes; ++p) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int row = r0 + ty + 8 * k;
+      uint16_t h[V];
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        if (fp16) {
+          const __half x = __float2half_rn(v[k][q]);
+          h[q] = __half_as_ushort(x);
+          v[k][q] -= __half2float(x);
+        } else {
+          const __nv_bfloat16 x = __float2bfloat16_rn(v[k][q]);
+          h[q] = __bfloat16_as_ushort(x);
+          v[k][q] -= __bfloat162float(x);
+        }
+      }
+      uint16_t *to = wp + (size_t)p * stride + (size_t)row * ld + c;
+      const bool inside = row < out && c < cols;
+      if (V == 4) {
+        const uint2 x = make_uint2(h[0] | (uint32_t)h[V / 4] << 16, h[V / 2] | (uint32_t)h[V - 1] << 16);
+        if (inside) *reinterpret_cast<uint2 *>(to) = x;
+        uint32_t *copy = reinterpret_cast<uint32_t *>(&tile[ty + 8 * k][tx * V]);
+        if (transpose) copy[0] = x.x, copy[1] = x.y;
+      } else {
+        if (inside) *to = h[0];
+        if (transpose) tile[ty + 8 * k][tx] = h[0];
+      }
+    }
+    if (!transpose) continue;                    // uniform over the block
+    __syncthreads();
+    uint16_t *wt = wtp + (size_t)p * stride;
+    if (V == 4) {                                // two rows per lane: the height is even
+      const int rr = 2 * (threadIdx.x & 15), row = r0 + rr;
+#pragma unroll
+      for (int q = 0; q < 2 * V; ++q) {
+        const int cc = (threadIdx.x >> 4) + 16 * q, col = c0 + cc;
+        if (row < out && col < in)
+          *reinterpret_cast<uint32_t *>(wt + (size_t)col * out + row) =
+              tile[rr][cc] | (uint32_t)tile[rr + 1][cc] << 16;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int col = c0 + ty + 8 * k, row = r0 + tx;
+        if (row < out && col < in) wt[(size_t)col * out + row] = tile[tx][ty + 8 * k];
+      }
+    }
+    __syncthreads();
+  }
+}
 __global__ void __launch_bounds__(256)
 prep_weights_kernel(const __grid_constant__ ZpPrepList d, const __grid_constant__ ZpTileRow tiles) {
-  // 32 x 32 tiles: the planes of W_fold go out row-major as they are formed; the transpose is
-  // written from a shared copy of the tile so that both stores run along the fastest axis.
-  __shared__ uint16_t tile[3][32][34];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;          // 32 x 8
+  __shared__ __align__(16) uint16_t tile[32][kPrepPitch];
   int b = 0;
   for (int t = blockIdx.x; t < tiles.first[tiles.n]; t += gridDim.x) {
     b = tiles.entry(t, b);
-    const int out = d.out[b], in = d.in[b], kind = d.kind[b], planes = d.planes[b], fp16 = d.fp16[b];
-    const int ld = d.ld[b], tl = t - tiles.first[b];
-    const float *__restrict__ w = d.w[b];
-    const int64_t stride = d.plane_stride[b];
-    uint16_t *wp = d.dst[b], *wtp = wp + (size_t)planes * stride;
-    float inv = 1.f;
-    if (fp16) {
-      const float s = zp_scale_for_bound(d.slot[b][0]);
-      inv = 1.f / s;
-      if (tl == 0 && threadIdx.x == 0) d.slot[b][1] = s;
-    }
-    const int cols = kind == ZP_PREP_PLAIN ? ld : in;
-    const int tiles_c = (cols + 31) / 32;
-    const int r0 = (tl / tiles_c) * 32, c0 = (tl % tiles_c) * 32;
-    const int half = out / 2, kin = in / 2;
-    float v[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int row = r0 + ty + 8 * k, col = c0 + tx;
-      v[k] = 0.f;
-      if (row < out && col < in) {
-        if (kind != ZP_PREP_FOLDED) {
-          v[k] = w[(size_t)row * in + col];
-        } else {
-          const bool lower = row >= half, right = col >= kin;
-          const int o = lower ? row - half : row, c = right ? col - kin : col;
-          v[k] = w[(size_t)((lower != right) ? half + o : o) * kin + c];
-          if (!lower && right) v[k] = -v[k];
-        }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int row = r0 + ty + 8 * k, col = c0 + tx;
-      if (row >= out || col >= cols) continue;
-      float x = v[k] * inv;
-      for (int p = 0; p < planes; ++p) {
-        uint16_t h;
-        if (fp16) {
-          const __half q = __float2half_rn(x);
-          h = __half_as_ushort(q);
-          x -= __half2float(q);
-        } else {
-          const __nv_bfloat16 q = __float2bfloat16_rn(x);
-          h = __bfloat16_as_ushort(q);
-          x -= __bfloat162float(q);
-        }
-        wp[(size_t)p * stride + (size_t)row * ld + col] = h;
-        tile[p][ty + 8 * k][tx] = h;
-      }
-    }
-    if (kind == ZP_PREP_PLAIN || !d.transposes) continue;         // uniform over the block
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int col = c0 + ty + 8 * k, row = r0 + tx;
-      if (row < out && col < in)
-        for (int p = 0; p < planes; ++p)
-          wtp[(size_t)p * stride + (size_t)col * out + row] = tile[p][tx][ty + 8 * k];
-    }
-    __syncthreads();
+    if (d.quads[b]) prep_tile<4>(d, b, t - tiles.first[b], tile);
+    else prep_tile<1>(d, b, t - tiles.first[b], tile);
   }
 }
 
@@ -525,11 +561,15 @@ int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st) {
   return ZP_OK;
 }
 
-int zp_launch_prep_weights(const ZpPrepList &list, cudaStream_t st) {
+int zp_launch_prep_weights(ZpPrepList &list, cudaStream_t st) {
   ZpTileRow row;
-  for (int i = 0; i < list.n; ++i)
+  for (int i = 0; i < list.n; ++i) {
+    const bool plain = list.kind[i] == ZP_PREP_PLAIN;
+    list.quads[i] = list.in[i] % (plain ? 4 : 8) == 0 && (plain || list.out[i] % 2 == 0) &&
+                    list.plane_stride[i] % 4 == 0 && (uintptr_t)list.w[i] % 16 == 0;
     row.add(zp_ceil_div(list.out[i], 32) *
-            zp_ceil_div(list.kind[i] == ZP_PREP_PLAIN ? list.ld[i] : list.in[i], 32));
+            zp_ceil_div(plain ? list.ld[i] : list.in[i], list.quads[i] ? 128 : 32));
+  }
   if (row.total() == 0) return ZP_OK;
   prep_weights_kernel<<<(unsigned)std::min(row.total(), 148 * 16), 256, 0, st>>>(list, row);
   ZP_LAUNCH_CHECK("prep_weights_kernel");

@@ -265,15 +265,10 @@ __device__ __forceinline__ void bulk_wait_all() {             // the writes them
 }
 
 // v[b][j]: value at row `row0 + lane`, column `n0 + col_lo + 32 b + j` (scaled, no bias yet).
-// EB = 2: the warp alternates between two block buffers, so one block's store is still being read
-// out of shared memory while the next block is staged (products with a short contraction are
-// bound by their output stores, and one 4 KB block per warp in flight does not cover the latency).
-template <int EB>
 __device__ __forceinline__ void epilogue_store_tma(const GemmProb &p, float (&v)[4][32],
-                                                   uint8_t *stage0, int lane, int row0, int n0,
+                                                   uint8_t *stage, int lane, int row0, int n0,
                                                    int col_lo, int col_hi, int split,
-                                                   const float *bias, float &seen_max,
-                                                   uint32_t &blocks_done) {
+                                                   const float *bias, float &seen_max) {
   if (row0 >= p.M) return;                        // warp-uniform: nothing of this slice exists
   const bool row_ok = row0 + lane < p.M;
 #pragma unroll
@@ -282,12 +277,7 @@ __device__ __forceinline__ void epilogue_store_tma(const GemmProb &p, float (&v)
     if (cc >= col_hi) continue;                   // warp-uniform
     const int n = n0 + cc;
     if (n >= p.N) continue;
-    uint8_t *stage = stage0 + (EB == 2 ? (blocks_done & 1) * kEpiBlockBytes : 0);
-    ++blocks_done;
-    if (lane == 0) {                              // the block buffer is free again
-      if (EB == 2) bulk_wait_read_but_one();
-      else bulk_wait_read();
-    }
+    if (lane == 0) bulk_wait_read();              // the block buffer is free again
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -507,9 +497,8 @@ __device__ __forceinline__ void epilogue_fused(const GemmProb &p, const ZpEpilog
   }
 }
 
-template <int P, int BK, int STAGES, int BN_CAP, int EB = 1>
+template <int P, int BK, int STAGES, int BN_CAP>
 struct SmemLayout {
-  static constexpr int kEpiBytes = EB * ::kEpiBytes;
   static constexpr int kATile = BM * BK * 2;
   static constexpr int kBTile = BN_CAP * BK * 2;
   static constexpr int kStage = P * (kATile + kBTile);
@@ -628,9 +617,9 @@ __device__ __forceinline__ void add_accumulator(float (&v)[4][32], uint32_t t_ro
   }
 }
 
-template <int P, int BK, int STAGES, int BN_CAP, int EPI, int EB = 1>
+template <int P, int BK, int STAGES, int BN_CAP, int EPI>
 __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
-  using L = SmemLayout<P, BK, STAGES, BN_CAP, EB>;
+  using L = SmemLayout<P, BK, STAGES, BN_CAP>;
   constexpr int kAccBufs = P == 1 ? 2 : 1;      // accumulation units in flight in TMEM
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -758,8 +747,8 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
     // registers and releases TMEM, so the next tile's MMAs start while it scales and stores.
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
-    uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes * EB;
-    uint32_t unit = 0, blocks_done = 0;
+    uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes;
+    uint32_t unit = 0;
     bool ok = true;
     float slope_max = 0.f;
     MaxTracker maxima;
@@ -798,8 +787,7 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
         epilogue_fused<EPI>(p, g.epi, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias, maxima.seen,
                             slope_max, node, rp_l);
       else
-        epilogue_store_tma<EB>(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias,
-                               maxima.seen, blocks_done);
+        epilogue_store_tma(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias, maxima.seen);
     }
     if (lane == 0) bulk_wait_all();                        // this warp's stores are done
     maxima.flush(lane);
@@ -819,14 +807,237 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
   }
 }
 
-template <int P, int BK, int STAGES, int BN_CAP, int EB = 1>
+template <int P, int BK, int STAGES, int BN_CAP>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmGroup g) {
-  gemm_tc_body<P, BK, STAGES, BN_CAP, ZP_EPI_NONE, EB>(g);
+  gemm_tc_body<P, BK, STAGES, BN_CAP, ZP_EPI_NONE>(g);
 }
 // the same contraction with a fused epilogue (the epilogue warps hold more live values)
 template <int P, int BK, int STAGES, int BN_CAP, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_fused_kernel(const __grid_constant__ GemmGroup g) {
   gemm_tc_body<P, BK, STAGES, BN_CAP, EPI>(g);
+}
+
+// ---- short contractions -------------------------------------------------------------------
+//
+// With at most 256 / P operand columns a product is bound by its output stores (the last layer of the
+// radial MLP writes 12 KB per edge and reads 0.5), and a tile's main loop is over before a pipeline
+// of k-blocks has filled.  Here a CTA keeps the whole K x 128 block of B in shared memory and
+// walks the row tiles under it: only A streams (1.5 tiles ahead), two accumulators alternate in
+// TMEM, and two 4 KB blocks per epilogue warp are on their way out.  The (column, row) tiles are dealt
+// out in contiguous stretches, columns slowest, so a CTA changes its B once or twice.
+// 60 000 x 128 -> 3072, two fp16 planes: SHORTNEW us, 302 with both operands streamed in 128 x 256 tiles.
+constexpr int kShortBN = 128, kShortBK = 64;
+template <int P>
+struct ShortLayout {
+  static constexpr int kTile = 128 * kShortBK * 2;             // one plane of a k-block of A or B
+  static constexpr int kMaxBlocks = 4 / P;                     // k-blocks of B that fit
+  static constexpr int kStages = 6 / P;
+  static constexpr int kB = 0, kA = kMaxBlocks * P * kTile;
+  static constexpr int kControl = kA + kStages * P * kTile;
+  static constexpr int kEpiOffset = kControl + 1024;
+  static constexpr int kTotal = kEpiOffset + 2 * kEpiBytes + 1024;
+};
+
+template <int P>
+__global__ void __launch_bounds__(kThreads, 1) gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
+  using L = ShortLayout<P>;
+  constexpr int STAGES = L::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                              ~(uintptr_t)1023);
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::kControl);
+  uint64_t *empty = full + STAGES;
+  uint64_t *b_full = empty + STAGES, *b_empty = b_full + 1;
+  uint64_t *tmem_full = b_empty + 1, *tmem_empty = tmem_full + 2;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
+  volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const GemmProb &p = g.p[0];
+  const int num_m = (p.M + BM - 1) / BM, num_k = p.num_k;
+  const int w0 = (int)((int64_t)g.total * blockIdx.x / gridDim.x);
+  const int w1 = (int)((int64_t)g.total * (blockIdx.x + 1) / gridDim.x);
+
+  if (threadIdx.x == 0) {
+    prefetch_maps(g);
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    mbar_init(b_full, 1);
+    mbar_init(b_empty, 1);
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 8); }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(tmem_slot)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- TMA producer
+    if (!g.unarmed && elect_one()) {
+      const uint32_t b_bytes = (uint32_t)p.BN * kShortBK * 2;
+      uint32_t it = 0, columns = 0;
+      int col = -1;
+      bool ok = true;
+      for (int w = w0; w < w1 && ok; ++w) {
+        if (w / num_m != col) {
+          col = w / num_m;
+          ok = mbar_wait(b_empty, (columns & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+          if (!ok) break;
+          ++columns;
+          mbar_expect_tx(b_full, (uint32_t)(num_k * P) * b_bytes);
+          for (int kb = 0; kb < num_k; ++kb)
+#pragma unroll
+            for (int pl = 0; pl < P; ++pl)
+              tma_load_3d(smem + L::kB + (kb * P + pl) * L::kTile, &p.map_b, b_full, kb * kShortBK,
+                          col * p.BN, pl);
+        }
+        const int m0 = (w - col * num_m) * BM;
+        for (int kb = 0; kb < num_k; ++kb, ++it) {
+          const int s = it % STAGES;
+          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+          if (!ok) break;
+          mbar_expect_tx(&full[s], P * L::kTile);
+#pragma unroll
+          for (int pl = 0; pl < P; ++pl)
+            tma_load_3d(smem + L::kA + (s * P + pl) * L::kTile, &p.map_a, &full[s], kb * kShortBK, m0, pl);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer
+    if (elect_one()) {
+      const uint32_t idesc = instr_desc(g, p, BM);
+      uint32_t it = 0, columns = 0;
+      int col = -1;
+      bool ok = true;
+      for (int w = w0; w < w1 && ok; ++w) {
+        if (w / num_m != col) {
+          col = w / num_m;
+          ok = mbar_wait(b_full, columns & 1, abort_flag, g.status, g.wait_limit_ns);
+          if (!ok) break;
+          ++columns;
+        }
+        const uint32_t unit = w - w0, buf = unit & 1;
+        ok = mbar_wait(&tmem_empty[buf], ((unit / 2) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+        if (!ok) break;
+        tcgen05_fence_after();
+        const uint32_t d_main = tmem_base + buf * 256u, d_small = d_main + 128u;
+        for (int kb = 0; kb < num_k; ++kb, ++it) {
+          const int s = it % STAGES;
+          ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, g.status, g.wait_limit_ns);
+          if (!ok) break;
+          tcgen05_fence_after();
+          const uint32_t sa = smem_u32(smem + L::kA + s * P * L::kTile);
+          const uint32_t sb = smem_u32(smem + L::kB + kb * P * L::kTile);
+#pragma unroll
+          for (int ks = 0; ks < kShortBK / 16; ++ks) {
+#pragma unroll
+            for (int q = 0; q < Pairs<P>::n; ++q) {
+              const uint64_t da = make_desc(sa + Pairs<P>::a(q) * L::kTile + ks * 32, 16, 1024, 2u);
+              const uint64_t db = make_desc(sb + Pairs<P>::b(q) * L::kTile + ks * 32, 16, 1024, 2u);
+              const bool first_step = kb == 0 && ks == 0;
+              if (q == 0) umma_bf16(d_main, da, db, idesc, first_step ? 0u : 1u);
+              else umma_bf16(d_small, da, db, idesc, (first_step && q == 1) ? 0u : 1u);
+            }
+          }
+          tcgen05_commit(&empty[s]);
+        }
+        if (!ok) break;
+        if (w + 1 < w1 && (w + 1) / num_m != col) tcgen05_commit(b_empty);    // B has been read
+        tcgen05_commit(&tmem_full[buf]);
+      }
+    }
+  } else {
+    // ---------------------------------------------------------------- epilogue (warps 2..9)
+    // warp w: TMEM lane quarter w % 4, column half (w - 2) / 4
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes * 2;
+    const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
+    uint32_t blocks_done = 0;
+    float bias[2] = {0.f, 0.f};          // of columns lane and lane + 32 of the warp's half
+    MaxTracker maxima;
+    maxima.follow(p.absmax_out, lane);
+    int col = -1;
+    for (int w = w0; w < w1; ++w) {
+      if (w / num_m != col) {
+        col = w / num_m;
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+          const int c = col * p.BN + half * 64 + 32 * b + lane;
+          bias[b] = p.bias && c < p.N ? p.bias[c] : 0.f;
+        }
+      }
+      const uint32_t unit = w - w0, buf = unit & 1;
+      bool ok = mbar_wait(&tmem_full[buf], (unit / 2) & 1, abort_flag, g.status, g.wait_limit_ns);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tcgen05_fence_after();
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u + half * 64;
+      float v[2][32];
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        uint32_t r[16], r2[16];
+        tmem_ld16(t_row + 16 * h, r);
+        if (P != 1) tmem_ld16(t_row + 128 + 16 * h, r2);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          float a = __uint_as_float(r[j]);
+          if (P != 1) a += __uint_as_float(r2[j]);
+          v[h / 2][16 * (h & 1) + j] = a * out_scale;
+        }
+      }
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+      const int row0 = (w - col * num_m) * BM + q * 32;
+      const bool row_ok = row0 + lane < p.M;
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        const int n = col * p.BN + half * 64 + 32 * b;
+        if (row0 >= p.M || half * 64 + 32 * b >= p.BN || n >= p.N) continue;      // warp-uniform
+        uint8_t *stage = epi_stage + (blocks_done++ & 1) * kEpiBlockBytes;
+        if (lane == 0) bulk_wait_read_but_one();          // the block buffer is free again
+        __syncwarp();
+        float most = 0.f;                                 // columns past N are zero, bias and all
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          v[b][j] += __shfl_sync(0xffffffffu, bias[b], j);
+          most = fmaxf(most, fabsf(v[b][j]));
+        }
+        if (row_ok) maxima.seen = fmaxf(maxima.seen, most);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) =
+              make_float4(v[b][4 * k], v[b][4 * k + 1], v[b][4 * k + 2], v[b][4 * k + 3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_3d(&p.map_c, stage, n, row0, 0);
+          bulk_commit();
+        }
+      }
+    }
+    if (lane == 0) bulk_wait_all();
+    maxima.flush(lane);
+  }
+
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u)
+                 : "memory");
+  }
 }
 
 // ---- CTA-pair variant ---------------------------------------------------------------------
@@ -1050,7 +1261,7 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
     uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes;
-    uint32_t unit = 0, blocks_done = 0;
+    uint32_t unit = 0;
     bool ok = true;
     float slope_max = 0.f;
     MaxTracker maxima;
@@ -1092,8 +1303,7 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
         epilogue_fused<EPI>(p, g.epi, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias, maxima.seen,
                             slope_max, node, rp_l);
       else
-        epilogue_store_tma<1>(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias,
-                              maxima.seen, blocks_done);
+        epilogue_store_tma(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias, maxima.seen);
     }
     if (lane == 0) bulk_wait_all();                        // this warp's stores are done
     maxima.flush(lane);
@@ -1349,13 +1559,12 @@ int fill_group(GemmGroup &grp, const ZpGemmTc *const *g, int n, int P, int bk, i
   return ZP_OK;
 }
 
-template <int P, int BK, int STAGES, int BN_CAP, int EPI, int EB = 1>
+template <int P, int BK, int STAGES, int BN_CAP, int EPI>
 int launch_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
-  using L = SmemLayout<P, BK, STAGES, BN_CAP, EB>;
-  static_assert(EB == 1 || EPI == ZP_EPI_NONE, "two store buffers only in the plain epilogue");
+  using L = SmemLayout<P, BK, STAGES, BN_CAP>;
   static_assert(L::kTotal <= 232448, "shared memory budget of one CTA");
   auto kernel = [] {
-    if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_kernel<P, BK, STAGES, BN_CAP, EB>;
+    if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_kernel<P, BK, STAGES, BN_CAP>;
     else return gemm_tc_fused_kernel<P, BK, STAGES, BN_CAP, EPI>;
   }();
   static ZpSmemOptIn opt_in;
@@ -1366,6 +1575,22 @@ int launch_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
   const int sms = device_sms(), grid = grp.total < sms ? grp.total : sms;
   kernel<<<grid, kThreads, L::kTotal, st>>>(grp);
   ZP_LAUNCH_CHECK("gemm_tc_kernel");
+  return ZP_OK;
+}
+
+template <int P>
+int launch_short(const ZpGemmTc &g, cudaStream_t st) {
+  using L = ShortLayout<P>;
+  static_assert(L::kTotal <= 232448, "shared memory budget of one CTA");
+  static ZpSmemOptIn opt_in;
+  int rc;
+  if ((rc = zp_ensure_smem(gemm_tc_short_kernel<P>, (size_t)L::kTotal, opt_in))) return rc;
+  GemmGroup grp;
+  const ZpGemmTc *one = &g;
+  if ((rc = fill_group(grp, &one, 1, P, kShortBK, BM, 1, kShortBN))) return rc;
+  const int sms = device_sms(), grid = grp.total < sms ? grp.total : sms;
+  gemm_tc_short_kernel<P><<<grid, kThreads, L::kTotal, st>>>(grp);
+  ZP_LAUNCH_CHECK("gemm_tc_short_kernel");
   return ZP_OK;
 }
 
@@ -1446,18 +1671,10 @@ int check_product(const ZpGemmTc &g) {
 int dispatch(const ZpGemmTc *const *g, int n, bool pair, cudaStream_t st) {
   const int planes = g[0]->planes;
   if (pair) return planes == 2 ? launch_pair<2, 64, 3>(g, n, st) : launch_pair<1, 64, 6>(g, n, st);
-  // a contraction of at most four k-blocks is bound by its output stores: fewer operand stages,
-  // two store buffers per epilogue warp
-  const bool store_bound = n == 1 && !g[0]->a_mn && !g[0]->b_mn && !(g[0]->epi && g[0]->epi->mode) &&
-                           g[0]->ksplit <= 1;
-  if (planes == 2) {
-    if (store_bound && g[0]->K <= 128) return launch_e<2, 32, 2, 256, ZP_EPI_NONE, 2>(g, n, st);
-    return launch<2, 32, 4, 256>(g, n, st);
-  }
-  if (planes == 1) {
-    if (store_bound && g[0]->K <= 256) return launch_e<1, 64, 2, 256, ZP_EPI_NONE, 2>(g, n, st);
-    return launch<1, 64, 4, 256>(g, n, st);
-  }
+  const bool is_short = n == 1 && !g[0]->a_mn && !g[0]->b_mn && !(g[0]->epi && g[0]->epi->mode) &&
+                        g[0]->ksplit <= 1 && g[0]->variant == 0 && g[0]->K * planes <= 256;
+  if (planes == 2) return is_short ? launch_short<2>(*g[0], st) : launch<2, 32, 4, 256>(g, n, st);
+  if (planes == 1) return is_short ? launch_short<1>(*g[0], st) : launch<1, 64, 4, 256>(g, n, st);
   // three planes: two stages of six MMA passes each leave room for the store blocks
   if (planes == 3)
     return g[0]->variant == 1 ? launch<3, 64, 2, 128>(g, n, st) : launch<3, 32, 2, 256>(g, n, st);
