@@ -261,7 +261,7 @@ max_list_kernel(const __grid_constant__ ZpMaxList d, const __grid_constant__ ZpT
 // slot = {max |W|, scale}: the scale follows from the maximum here (fp16 planes).
 // Bound by instruction issue, so a thread takes V = 4 neighbouring columns where the widths allow (every
 // width in use): a value at a time took 115 instructions per value (38 us for the weights of lmax 4 /
-// mmax 2 / C 128 as one plane; now PREPUS).  Tiles of 32 rows and 32 V columns; the planes of W_fold go
+// mmax 2 / C 128 as one plane; now 12).  Tiles of 32 rows and 32 V columns; the planes of W_fold go
 // out row-major as they are formed, the transpose from a shared copy of the tile so that both
 // stores run along the fastest axis.
 constexpr int kPrepPitch = 130;
@@ -372,8 +372,8 @@ prep_weights_kernel(const __grid_constant__ ZpPrepList d, const __grid_constant_
 //   ZP_FIN_SUM     sum of `parts` partial matrices (K splits of a product), in order
 //   ZP_FIN_UNFOLD  the same, mapped from the folded layout back to the reference's:
 //                  dWa = F[0,0] + F[1,1], dWb = F[1,0] - F[0,1]
-//   ZP_FIN_COLUMN  sum of `parts` partial rows: 32 columns per tile, eight threads per column take
-//                  every eighth row, and their sums are added in order
+//   ZP_FIN_COLUMN  sum of `parts` partial rows: eight columns per tile, 32 threads per column take
+//                  every 32nd row, and their sums are added in order
 // Bound by the partials it reads.  A tile of the matrices has 256 groups of V neighbouring entries.
 template <int V>
 __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, float *__restrict__ dst,
@@ -414,7 +414,7 @@ __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, fl
 }
 __global__ void __launch_bounds__(256)
 finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ ZpTileRow tiles) {
-  __shared__ float red[8][33];
+  __shared__ float red[32][9];
   int b = 0;
   for (int t = blockIdx.x; t < tiles.first[tiles.n]; t += gridDim.x) {
     b = tiles.entry(t, b);
@@ -428,19 +428,19 @@ finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ Z
       else finalize_entries<1>(f, dst, stride, d.rows[b], cols, parts, d.ld[b], folded, tile);
       continue;
     }
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int c = tile * 32 + tx;
+    const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
+    const int c = tile * 8 + tx;
     float s = 0.f;
     if (c < cols) {
-#pragma unroll 4
-      for (int p = ty; p < parts; p += 8) s += f[(size_t)p * stride + c];
+#pragma unroll 8
+      for (int p = ty; p < parts; p += 32) s += f[(size_t)p * stride + c];
     }
     red[ty][tx] = s;
     __syncthreads();
     if (ty == 0 && c < cols) {
       float acc = 0.f;
 #pragma unroll
-      for (int g = 0; g < 8; ++g) acc += red[g][tx];
+      for (int g = 0; g < 32; ++g) acc += red[g][tx];
       dst[c] = acc;
     }
     __syncthreads();
@@ -581,7 +581,7 @@ int zp_launch_finalize(ZpFinalList &list, cudaStream_t st) {
   for (int i = 0; i < list.n; ++i) {
     const int kin = list.kind[i] == ZP_FIN_UNFOLD ? list.cols[i] / 2 : list.cols[i];
     list.quads[i] = (kin | list.ld[i] | (int)(list.stride[i] & 3)) % 4 == 0 && ((uintptr_t)list.src[i] | (uintptr_t)list.dst[i]) % 16 == 0;
-    row.add(list.kind[i] == ZP_FIN_COLUMN ? zp_ceil_div(list.cols[i], 32)
+    row.add(list.kind[i] == ZP_FIN_COLUMN ? zp_ceil_div(list.cols[i], 8)
                                           : zp_ceil_div((int64_t)list.rows[i] * kin, list.quads[i] ? 1024 : 256));
   }
   if (row.total() == 0) return ZP_OK;

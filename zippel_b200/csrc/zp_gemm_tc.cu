@@ -38,6 +38,7 @@
 // Shared-memory tiles use the 128-byte (BK = 64) or 64-byte (BK = 32) swizzle that TMA writes
 // and the matrix descriptors name.  Every mbarrier wait is bounded: after ~2 s it records
 // ZP_ERR_DEVICE_TIMEOUT in the status word, raises the CTA's abort flag and the CTA drains.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -214,6 +215,7 @@ struct GemmGroup {
   int *status;
   uint64_t wait_limit_ns; // bound of every mbarrier wait
   int unarmed;            // self-test: the producers load nothing, so the first wait runs out
+  int rows_apart;         // short contractions: row tiles between two of a CTA (0: stretches)
   ZpEpilogue epi;         // work of the fused epilogues (mode 0: none; one product only)
 };
 
@@ -256,9 +258,6 @@ __device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void 
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void bulk_wait_read() {            // shared source may be overwritten
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_wait_read_but_one() {    // all but the newest group were read
-  asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
 __device__ __forceinline__ void bulk_wait_all() {             // the writes themselves are done
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
@@ -823,10 +822,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_fused_kernel(const __grid
 // radial MLP writes 12 KB per edge and reads 0.5), and a tile's main loop is over before a pipeline
 // of k-blocks has filled.  Here a CTA keeps the whole K x 128 block of B in shared memory and
 // walks the row tiles under it: only A streams (1.5 tiles ahead), two accumulators alternate in
-// TMEM, and two 4 KB blocks per epilogue warp are on their way out.  The (column, row) tiles are dealt
-// out in contiguous stretches, columns slowest, so a CTA changes its B once or twice.
+// TMEM, and sixteen epilogue warps take one 32 x 32 block of a tile each (eight with two blocks
+// took 6 % longer: the way through TMEM, registers and shared memory is a chain of latencies).
+// All columns of the same rows are walked at the same time, by CTAs that keep to one column, so
+// that whole rows of C leave L2 together; where that would leave more than a tenth of the SMs out, CTAs
+// take contiguous stretches of the (column, row) tiles, columns slowest, and change their B on the way.
 // 60 000 x 128 -> 3072, two fp16 planes: SHORTNEW us, 302 with both operands streamed in 128 x 256 tiles.
 constexpr int kShortBN = 128, kShortBK = 64;
+constexpr int kShortEpiWarps = 16, kShortThreads = 64 + 32 * kShortEpiWarps;
 template <int P>
 struct ShortLayout {
   static constexpr int kTile = 128 * kShortBK * 2;             // one plane of a k-block of A or B
@@ -835,11 +838,12 @@ struct ShortLayout {
   static constexpr int kB = 0, kA = kMaxBlocks * P * kTile;
   static constexpr int kControl = kA + kStages * P * kTile;
   static constexpr int kEpiOffset = kControl + 1024;
-  static constexpr int kTotal = kEpiOffset + 2 * kEpiBytes + 1024;
+  static constexpr int kTotal = kEpiOffset + kShortEpiWarps * kEpiBlockBytes + 1024;
 };
 
 template <int P>
-__global__ void __launch_bounds__(kThreads, 1) gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
+__global__ void __launch_bounds__(kShortThreads, 1)
+gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
   using L = ShortLayout<P>;
   constexpr int STAGES = L::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -855,15 +859,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_short_kernel(const __grid
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const GemmProb &p = g.p[0];
   const int num_m = (p.M + BM - 1) / BM, num_k = p.num_k;
-  const int w0 = (int)((int64_t)g.total * blockIdx.x / gridDim.x);
-  const int w1 = (int)((int64_t)g.total * (blockIdx.x + 1) / gridDim.x);
+  const int step = g.rows_apart ? g.rows_apart : 1;
+  int w0 = (int)((int64_t)g.total * blockIdx.x / gridDim.x);
+  int w1 = (int)((int64_t)g.total * (blockIdx.x + 1) / gridDim.x);
+  if (g.rows_apart) {
+    const int first = blockIdx.x % p.num_n * num_m;
+    w0 = first + blockIdx.x / p.num_n;
+    w1 = first + num_m;
+  }
 
   if (threadIdx.x == 0) {
     prefetch_maps(g);
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     mbar_init(b_full, 1);
     mbar_init(b_empty, 1);
-    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 8); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], kShortEpiWarps); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -887,7 +897,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_short_kernel(const __grid
       uint32_t it = 0, columns = 0;
       int col = -1;
       bool ok = true;
-      for (int w = w0; w < w1 && ok; ++w) {
+      for (int w = w0; w < w1 && ok; w += step) {
         if (w / num_m != col) {
           col = w / num_m;
           ok = mbar_wait(b_empty, (columns & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
@@ -916,17 +926,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_short_kernel(const __grid
     // ---------------------------------------------------------------- MMA issuer
     if (elect_one()) {
       const uint32_t idesc = instr_desc(g, p, BM);
-      uint32_t it = 0, columns = 0;
+      uint32_t it = 0, columns = 0, unit = 0;
       int col = -1;
       bool ok = true;
-      for (int w = w0; w < w1 && ok; ++w) {
+      for (int w = w0; w < w1 && ok; w += step, ++unit) {
         if (w / num_m != col) {
           col = w / num_m;
           ok = mbar_wait(b_full, columns & 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           ++columns;
         }
-        const uint32_t unit = w - w0, buf = unit & 1;
+        const uint32_t buf = unit & 1;
         ok = mbar_wait(&tmem_empty[buf], ((unit / 2) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
         if (!ok) break;
         tcgen05_fence_after();
@@ -952,79 +962,72 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_short_kernel(const __grid
           tcgen05_commit(&empty[s]);
         }
         if (!ok) break;
-        if (w + 1 < w1 && (w + 1) / num_m != col) tcgen05_commit(b_empty);    // B has been read
+        if (w + step < w1 && (w + step) / num_m != col) tcgen05_commit(b_empty);    // B has been read
         tcgen05_commit(&tmem_full[buf]);
       }
     }
   } else {
-    // ---------------------------------------------------------------- epilogue (warps 2..9)
-    // warp w: TMEM lane quarter w % 4, column half (w - 2) / 4
-    const int q = warp & 3, half = (warp - 2) >> 2;
-    uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes * 2;
+    // ---------------------------------------------------------------- epilogue (warps 2..17)
+    // warp w: TMEM lane quarter w % 4, columns 32 ((w - 2) / 4) and on
+    const int q = warp & 3, first = (warp - 2) / 4 * 32;
+    uint8_t *stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes;
     const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
-    uint32_t blocks_done = 0;
-    float bias[2] = {0.f, 0.f};          // of columns lane and lane + 32 of the warp's half
+    float bias = 0.f;                    // of column `lane` of the block
     MaxTracker maxima;
     maxima.follow(p.absmax_out, lane);
+    uint32_t unit = 0;
     int col = -1;
-    for (int w = w0; w < w1; ++w) {
+    for (int w = w0; w < w1; w += step, ++unit) {
       if (w / num_m != col) {
         col = w / num_m;
-#pragma unroll
-        for (int b = 0; b < 2; ++b) {
-          const int c = col * p.BN + half * 64 + 32 * b + lane;
-          bias[b] = p.bias && c < p.N ? p.bias[c] : 0.f;
-        }
+        const int c = col * p.BN + first + lane;
+        bias = p.bias && c < p.N ? p.bias[c] : 0.f;
       }
-      const uint32_t unit = w - w0, buf = unit & 1;
+      const uint32_t buf = unit & 1;
       bool ok = mbar_wait(&tmem_full[buf], (unit / 2) & 1, abort_flag, g.status, g.wait_limit_ns);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tcgen05_fence_after();
-      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u + half * 64;
-      float v[2][32];
+      const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256u + first;
+      float v[32];
+      {
+        uint32_t r[2][16], r2[2][16];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        uint32_t r[16], r2[16];
-        tmem_ld16(t_row + 16 * h, r);
-        if (P != 1) tmem_ld16(t_row + 128 + 16 * h, r2);
+        for (int h = 0; h < 2; ++h) {
+          tmem_ld16(t_row + 16 * h, r[h]);
+          if (P != 1) tmem_ld16(t_row + 128 + 16 * h, r2[h]);
+        }
         tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          float a = __uint_as_float(r[j]);
-          if (P != 1) a += __uint_as_float(r2[j]);
-          v[h / 2][16 * (h & 1) + j] = a * out_scale;
+        for (int j = 0; j < 32; ++j) {
+          float a = __uint_as_float(r[j / 16][j % 16]);
+          if (P != 1) a += __uint_as_float(r2[j / 16][j % 16]);
+          v[j] = a * out_scale;
         }
       }
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-      const int row0 = (w - col * num_m) * BM + q * 32;
-      const bool row_ok = row0 + lane < p.M;
+      const int row0 = (w - col * num_m) * BM + q * 32, n = col * p.BN + first;
+      if (row0 >= p.M || first >= p.BN || n >= p.N) continue;               // warp-uniform
+      float most = 0.f;                                   // columns past N are zero, bias and all
 #pragma unroll
-      for (int b = 0; b < 2; ++b) {
-        const int n = col * p.BN + half * 64 + 32 * b;
-        if (row0 >= p.M || half * 64 + 32 * b >= p.BN || n >= p.N) continue;      // warp-uniform
-        uint8_t *stage = epi_stage + (blocks_done++ & 1) * kEpiBlockBytes;
-        if (lane == 0) bulk_wait_read_but_one();          // the block buffer is free again
-        __syncwarp();
-        float most = 0.f;                                 // columns past N are zero, bias and all
+      for (int j = 0; j < 32; ++j) {
+        v[j] += __shfl_sync(0xffffffffu, bias, j);
+        most = fmaxf(most, fabsf(v[j]));
+      }
+      if (row0 + lane < p.M) maxima.seen = fmaxf(maxima.seen, most);
+      if (lane == 0) bulk_wait_read();                    // the block buffer is free again
+      __syncwarp();
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          v[b][j] += __shfl_sync(0xffffffffu, bias[b], j);
-          most = fmaxf(most, fabsf(v[b][j]));
-        }
-        if (row_ok) maxima.seen = fmaxf(maxima.seen, most);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) =
-              make_float4(v[b][4 * k], v[b][4 * k + 1], v[b][4 * k + 2], v[b][4 * k + 3]);
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) {
-          tma_store_3d(&p.map_c, stage, n, row0, 0);
-          bulk_commit();
-        }
+      for (int k = 0; k < 8; ++k)
+        *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) =
+            make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        tma_store_3d(&p.map_c, stage, n, row0, 0);
+        bulk_commit();
       }
     }
     if (lane == 0) bulk_wait_all();
@@ -1588,8 +1591,11 @@ int launch_short(const ZpGemmTc &g, cudaStream_t st) {
   GemmGroup grp;
   const ZpGemmTc *one = &g;
   if ((rc = fill_group(grp, &one, 1, P, kShortBK, BM, 1, kShortBN))) return rc;
-  const int sms = device_sms(), grid = grp.total < sms ? grp.total : sms;
-  gemm_tc_short_kernel<P><<<grid, kThreads, L::kTotal, st>>>(grp);
+  const int sms = device_sms(), columns = grp.p[0].num_n, rows = grp.total / columns;
+  grp.rows_apart = columns <= sms ? std::min(sms / columns, rows) : 0;
+  if (grp.rows_apart < rows && columns * grp.rows_apart * 10 < sms * 9) grp.rows_apart = 0;
+  const int grid = grp.rows_apart ? columns * grp.rows_apart : std::min(grp.total, sms);
+  gemm_tc_short_kernel<P><<<grid, kShortThreads, L::kTotal, st>>>(grp);
   ZP_LAUNCH_CHECK("gemm_tc_short_kernel");
   return ZP_OK;
 }
