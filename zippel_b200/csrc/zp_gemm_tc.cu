@@ -263,51 +263,37 @@ __device__ __forceinline__ void bulk_wait_all() {             // the writes them
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-// v[b][j]: value at row `row0 + lane`, column `n0 + col_lo + 32 b + j` (scaled, no bias yet).
-__device__ __forceinline__ void epilogue_store_tma(const GemmProb &p, float (&v)[4][32],
-                                                   uint8_t *stage, int lane, int row0, int n0,
-                                                   int col_lo, int col_hi, int split,
-                                                   const float *bias, float &seen_max) {
-  if (row0 >= p.M) return;                        // warp-uniform: nothing of this slice exists
-  const bool row_ok = row0 + lane < p.M;
+// One 32 x 32 block of the result on its way out.  v[j]: value at row `row0 + lane`, column n + j (scaled,
+// no bias yet); `bias`: of column n + lane.  Columns past N are zero, since the operand rows they
+// come from were filled with zeros; the TMA unit leaves them out, and rows past M.
+__device__ __forceinline__ void store_block(const GemmProb &p, float (&v)[32], uint8_t *stage, int lane,
+                                            int row0, int n, int split, bool has_bias, float bias,
+                                            float &seen_max) {
+  if (row0 >= p.M || n >= p.N) return;            // warp-uniform
+  if (has_bias) {
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int cc = col_lo + 32 * b;
-    if (cc >= col_hi) continue;                   // warp-uniform
-    const int n = n0 + cc;
-    if (n >= p.N) continue;
-    if (lane == 0) bulk_wait_read();              // the block buffer is free again
-    __syncwarp();
+    for (int j = 0; j < 32; ++j) v[j] += __shfl_sync(0xffffffffu, bias, j);
+  }
+  if (p.absmax_out && row0 + lane < p.M) {
+    float m[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float4 o = make_float4(v[b][4 * k], v[b][4 * k + 1], v[b][4 * k + 2], v[b][4 * k + 3]);
-      if (bias) {
-        const int c = n + 4 * k;
-        o.x += c < p.N ? bias[c] : 0.f;
-        o.y += c + 1 < p.N ? bias[c + 1] : 0.f;
-        o.z += c + 2 < p.N ? bias[c + 2] : 0.f;
-        o.w += c + 3 < p.N ? bias[c + 3] : 0.f;
-      }
-      if (row_ok) {
-        const int c = n + 4 * k;
-        float m = c < p.N ? fabsf(o.x) : 0.f;
-        m = fmaxf(m, c + 1 < p.N ? fabsf(o.y) : 0.f);
-        m = fmaxf(m, c + 2 < p.N ? fabsf(o.z) : 0.f);
-        m = fmaxf(m, c + 3 < p.N ? fabsf(o.w) : 0.f);
-        seen_max = fmaxf(seen_max, m);
-      }
-      // 128-byte swizzle: 16-byte chunk k of row r sits at chunk k ^ (r & 7)
-      *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) = o;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane == 0) {
-      tma_store_3d(&p.map_c, stage, n, row0, split);
-      bulk_commit();
-    }
+    for (int j = 0; j < 32; ++j) m[j & 3] = fmaxf(m[j & 3], fabsf(v[j]));
+    seen_max = fmaxf(seen_max, fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3])));
+  }
+  if (lane == 0) bulk_wait_read();                // the block buffer is free again
+  __syncwarp();
+  // 128-byte swizzle: 16-byte chunk k of row r sits at chunk k ^ (r & 7)
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) =
+        make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  __syncwarp();
+  if (lane == 0) {
+    tma_store_3d(&p.map_c, stage, n, row0, split);
+    bulk_commit();
   }
 }
-
 
 // ---- fused epilogues ------------------------------------------------------------------------
 // A finished 32 x 32 block of the result sits in the warp's shared-memory stage in the layout
@@ -565,31 +551,32 @@ struct MaxTracker {
   }
 };
 
-// The accumulator slice of a tile's first chunk (this warp's 32 rows, columns col_lo .. col_hi) into
-// v.  Sixteen columns at a time: the slice itself (128 values per thread) leaves little room for
-// staging registers; both accumulators' loads are in flight before one wait.
+// 32 columns of the accumulator(s) at `taddr` into v: sixteen of them at a time (a slice of 128 values
+// per thread leaves little room), both accumulators' loads in flight before one wait
+template <int P>
+__device__ __forceinline__ void read_block(float (&v)[32], uint32_t taddr, float out_scale) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t r[16], r2[16];
+    tmem_ld16(taddr + 16 * h, r);
+    if (P != 1) tmem_ld16(taddr + kTmemBuf + 16 * h, r2);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      float a = __uint_as_float(r[j]);
+      if (P != 1) a += __uint_as_float(r2[j]);
+      v[16 * h + j] = a * out_scale;
+    }
+  }
+}
+// The accumulator slice of a tile's first chunk (this warp's 32 rows, columns col_lo .. col_hi) into v
 template <int P>
 __device__ __forceinline__ void read_accumulator(float (&v)[4][32], uint32_t t_row, int col_lo,
                                                  int col_hi, float out_scale) {
 #pragma unroll
-  for (int b = 0; b < 4; ++b) {
-    const int cc = col_lo + 32 * b;
-    if (cc < col_hi) {                    // warp-uniform
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t r[16], r2[16];
-        tmem_ld16(t_row + cc + 16 * h, r);
-        if (P != 1) tmem_ld16(t_row + kTmemBuf + cc + 16 * h, r2);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          float a = __uint_as_float(r[j]);
-          if (P != 1) a += __uint_as_float(r2[j]);
-          v[b][16 * h + j] = a * out_scale;
-        }
-      }
-    }
-  }
+  for (int b = 0; b < 4; ++b)
+    if (col_lo + 32 * b < col_hi)         // warp-uniform
+      read_block<P>(v[b], t_row + col_lo + 32 * b, out_scale);
 }
 // ... and of a later chunk, added to it (all of v is live here: eight columns at a time)
 template <int P>
@@ -767,26 +754,67 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
         node = g.epi.block_node[row0 >> 5];
         rp_l = g.epi.row_ptr[min(node + lane, g.epi.n_nodes)];
       }
-      float v[4][32];
-      for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
-        const int buf = unit % kAccBufs;
+      float bias_l[4];
+      if constexpr (EPI == ZP_EPI_NONE) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int c = x.n0 + col_lo + 32 * b + lane;
+          bias_l[b] = bias && c < p.N ? bias[c] : 0.f;
+        }
+      }
+      // wait for accumulation unit `unit`; where its columns stand
+      auto finished = [&](int buf) {
         ok = mbar_wait(&tmem_full[buf], (unit / kAccBufs) & 1, abort_flag, g.status, g.wait_limit_ns);
         ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (P == 1 ? (uint32_t)buf * kTmemBuf : 0u);
-        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
-        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        return tmem_base + ((uint32_t)(q * 32) << 16) + (P == 1 ? (uint32_t)buf * kTmemBuf : 0u);
+      };
+      auto release = [&](int buf) {
         tcgen05_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[buf]);      // TMEM slice is in registers now
+        if (lane == 0) mbar_arrive(&tmem_empty[buf]);
+        ++unit;
+      };
+      float v[4][32];
+      if constexpr (EPI == ZP_EPI_NONE && P == 1) {
+        // One plane: the next tile has the other buffer, so the slice leaves block by block.  This is what
+        // bounds the short contractions (256 x 256 tiles of K = 1024: 9.0 us, of them 5.8 MMAs; 10.2
+        // with the whole slice read first and every column checked against N).
+        if (x.kb1 - x.kb0 <= p.kc) {
+          const int buf = unit % kAccBufs;
+          const uint32_t t_row = finished(buf);
+          if (!ok) break;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const int cc = col_lo + 32 * b;
+            if (cc < col_hi) read_block<P>(v[0], t_row + cc, out_scale);
+            if (b == 3) release(buf);
+            if (cc < col_hi)
+              store_block(p, v[0], epi_stage, lane, row0, x.n0 + cc, x.split, bias != nullptr, bias_l[b],
+                          maxima.seen);
+          }
+          continue;
+        }
+      }
+      for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc) {
+        const int buf = unit % kAccBufs;
+        const uint32_t t_row = finished(buf);
+        if (!ok) break;
+        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        release(buf);                       // the slice is in registers now
       }
       if (!ok) break;
-      if constexpr (EPI != ZP_EPI_NONE)
+      if constexpr (EPI != ZP_EPI_NONE) {
         epilogue_fused<EPI>(p, g.epi, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias, maxima.seen,
                             slope_max, node, rp_l);
-      else
-        epilogue_store_tma(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias, maxima.seen);
+      } else {
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (col_lo + 32 * b < col_hi)
+            store_block(p, v[b], epi_stage, lane, row0, x.n0 + col_lo + 32 * b, x.split, bias != nullptr,
+                        bias_l[b], maxima.seen);
+      }
     }
     if (lane == 0) bulk_wait_all();                        // this warp's stores are done
     maxima.flush(lane);
@@ -827,7 +855,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_fused_kernel(const __grid
 // All columns of the same rows are walked at the same time, by CTAs that keep to one column, so
 // that whole rows of C leave L2 together; where that would leave more than a tenth of the SMs out, CTAs
 // take contiguous stretches of the (column, row) tiles, columns slowest, and change their B on the way.
-// 60 000 x 128 -> 3072, two fp16 planes: SHORTNEW us, 302 with both operands streamed in 128 x 256 tiles.
+// 60 000 x 128 -> 3072, two fp16 planes: 183 us, 302 with both operands streamed in 128 x 256 tiles.
 constexpr int kShortBN = 128, kShortBK = 64;
 constexpr int kShortEpiWarps = 16, kShortThreads = 64 + 32 * kShortEpiWarps;
 template <int P>
@@ -1008,27 +1036,9 @@ gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tmem_empty[buf]);
-      const int row0 = (w - col * num_m) * BM + q * 32, n = col * p.BN + first;
-      if (row0 >= p.M || first >= p.BN || n >= p.N) continue;               // warp-uniform
-      float most = 0.f;                                   // columns past N are zero, bias and all
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        v[j] += __shfl_sync(0xffffffffu, bias, j);
-        most = fmaxf(most, fabsf(v[j]));
-      }
-      if (row0 + lane < p.M) maxima.seen = fmaxf(maxima.seen, most);
-      if (lane == 0) bulk_wait_read();                    // the block buffer is free again
-      __syncwarp();
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        *reinterpret_cast<float4 *>(stage + lane * 128 + ((k ^ (lane & 7)) << 4)) =
-            make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) {
-        tma_store_3d(&p.map_c, stage, n, row0, 0);
-        bulk_commit();
-      }
+      if (first < p.BN)                                   // warp-uniform
+        store_block(p, v, stage, lane, (w - col * num_m) * BM + q * 32, col * p.BN + first, 0,
+                    p.bias != nullptr, bias, maxima.seen);
     }
     if (lane == 0) bulk_wait_all();
     maxima.flush(lane);
@@ -1286,27 +1296,67 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
         node = g.epi.block_node[row0 >> 5];
         rp_l = g.epi.row_ptr[min(node + lane, g.epi.n_nodes)];
       }
-      float v[4][32];
-      for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
-        const int buf = P == 1 ? (int)(unit & 1) : 0;
-        const uint32_t round = P == 1 ? (unit >> 1) : unit;
-        ok = mbar_wait(&tmem_full[buf], round & 1, abort_flag, g.status, g.wait_limit_ns);
+      float bias_l[4];
+      if constexpr (EPI == ZP_EPI_NONE) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int c = x.n0 + col_lo + 32 * b + lane;
+          bias_l[b] = bias && c < p.N ? bias[c] : 0.f;
+        }
+      }
+      // wait for accumulation unit `unit`; where its columns stand
+      auto finished = [&](int buf) {
+        ok = mbar_wait(&tmem_full[buf], (P == 1 ? unit >> 1 : unit) & 1, abort_flag, g.status, g.wait_limit_ns);
         ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
         tcgen05_fence_after();
-        const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * kTmemBuf;
-        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
-        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        return tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * kTmemBuf;
+      };
+      auto release = [&](int buf) {
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(buf ? release_bar1 : release_bar0);
+        ++unit;
+      };
+      float v[4][32];
+      if constexpr (EPI == ZP_EPI_NONE && P == 1) {
+        // One plane: the next tile has the other buffer, so the slice leaves block by block.  This is what
+        // bounds the short contractions (256 x 256 tiles of K = 1024: 9.0 us, of them 5.8 MMAs; 10.2
+        // with the whole slice read first and every column checked against N).
+        if (x.kb1 - x.kb0 <= p.kc) {
+          const int buf = P == 1 ? (int)(unit & 1) : 0;
+          const uint32_t t_row = finished(buf);
+          if (!ok) break;
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            const int cc = col_lo + 32 * b;
+            if (cc < col_hi) read_block<P>(v[0], t_row + cc, out_scale);
+            if (b == 3) release(buf);
+            if (cc < col_hi)
+              store_block(p, v[0], epi_stage, lane, row0, x.n0 + cc, x.split, bias != nullptr, bias_l[b],
+                          maxima.seen);
+          }
+          continue;
+        }
+      }
+      for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc) {
+        const int buf = P == 1 ? (int)(unit & 1) : 0;
+        const uint32_t t_row = finished(buf);
+        if (!ok) break;
+        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        release(buf);                       // the slice is in registers now
       }
       if (!ok) break;
-      if constexpr (EPI != ZP_EPI_NONE)
+      if constexpr (EPI != ZP_EPI_NONE) {
         epilogue_fused<EPI>(p, g.epi, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, bias, maxima.seen,
                             slope_max, node, rp_l);
-      else
-        epilogue_store_tma(p, v, epi_stage, lane, row0, x.n0, col_lo, col_hi, x.split, bias, maxima.seen);
+      } else {
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (col_lo + 32 * b < col_hi)
+            store_block(p, v[b], epi_stage, lane, row0, x.n0 + col_lo + 32 * b, x.split, bias != nullptr,
+                        bias_l[b], maxima.seen);
+      }
     }
     if (lane == 0) bulk_wait_all();                        // this warp's stores are done
     maxima.flush(lane);
