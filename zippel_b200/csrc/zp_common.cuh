@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include <mutex>
+#include <utility>
 
 #include "zippel_b200.h"
 #include "zp_planes.cuh"
@@ -100,6 +101,25 @@ int64_t &zp_launch_counter();
       return ZP_ERR_CUDA;                               \
     }                                                   \
   } while (0)
+
+// Every kernel is launched so that it may be put in place while its predecessor on the stream still runs
+// (two to three microseconds of every launch, a tenth of a step of some hundred atoms), and begins by
+// waiting for all of that predecessor's work.  A kernel started by zp_launch has to call
+// zp_after_previous before it touches global memory.
+__device__ __forceinline__ void zp_after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... P, typename... A>
+void zp_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A &&...args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, P(std::forward<A>(args))...);      // errors: ZP_LAUNCH_CHECK
+}
 
 // A kernel's raised dynamic shared-memory limit is an attribute of the function ON a device, so
 // "already raised" is remembered per device ordinal (one ZpSmemOptIn per call site, under a lock:

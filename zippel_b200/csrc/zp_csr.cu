@@ -30,6 +30,7 @@ enum { kFlagEdges = 1, kFlagElements = 2 };
 __global__ void count_kernel(int64_t E, int64_t N, const int64_t *__restrict__ src,
                              const int64_t *__restrict__ dst, const int64_t *__restrict__ z,
                              int n_elements, int32_t *cnt_dst, int32_t *cnt_src, int32_t *flag) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (z && i < N && (uint64_t)z[i] >= (uint64_t)n_elements) atomicOr(flag, kFlagElements);
   if (i >= E) return;
@@ -77,6 +78,7 @@ __device__ __forceinline__ int32_t block_exclusive_scan(int32_t v, int32_t *warp
   return before + inc - v;
 }
 __global__ void __launch_bounds__(kScanThreads) scan_totals_kernel(int64_t n, const ScanArgs a) {
+  zp_after_previous();
   __shared__ int32_t sums[32];
   const int32_t *cnt = a.cnt[blockIdx.y];
   const int64_t base = (int64_t)blockIdx.x * kScanSpan + threadIdx.x * kScanItems;
@@ -87,6 +89,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_totals_kernel(int64_t n, co
   if (threadIdx.x == 0) a.totals[blockIdx.y * gridDim.x + blockIdx.x] = total;
 }
 __global__ void __launch_bounds__(kScanThreads) scan_kernel(int64_t n, const ScanArgs a) {
+  zp_after_previous();
   __shared__ int32_t sums[32];
   int32_t *cnt = a.cnt[blockIdx.y], *ptr = a.ptr[blockIdx.y];
   int64_t lo = 0, hi = n;
@@ -126,6 +129,7 @@ __global__ void __launch_bounds__(kScanThreads) scan_kernel(int64_t n, const Sca
 
 __global__ void bucket_kernel(int64_t E, int64_t N, const int64_t *__restrict__ src,
                               const int64_t *__restrict__ dst, int32_t *cursor, int32_t *tmp) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= E) return;
   const int64_t k = dst[i];
@@ -134,6 +138,7 @@ __global__ void bucket_kernel(int64_t E, int64_t N, const int64_t *__restrict__ 
 }
 __global__ void bucket_src_kernel(int64_t E, int64_t N, const int32_t *__restrict__ key,
                                   int32_t *cursor, int32_t *tmp) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= E) return;
   const int32_t k = key[i];
@@ -174,6 +179,7 @@ __global__ void rank_dst_kernel(int64_t N, int64_t E, const int64_t *__restrict_
                                 const int32_t *__restrict__ row_ptr,
                                 const int32_t *__restrict__ tmp, int32_t *perm,
                                 int32_t *src_sorted, int32_t *dst_sorted) {
+  zp_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (int64_t i = row_ptr[N] + tid; i < E; i += (int64_t)gridDim.x * blockDim.x)
     perm[i] = src_sorted[i] = dst_sorted[i] = 0;
@@ -213,6 +219,7 @@ __global__ void rank_dst_kernel(int64_t N, int64_t E, const int64_t *__restrict_
 // One warp per source node: order the sorted-edge ids of its outgoing edges increasingly.
 __global__ void rank_src_kernel(int64_t N, int64_t E, const int32_t *__restrict__ row_ptr_src,
                                 const int32_t *__restrict__ tmp, int32_t *perm_src) {
+  zp_after_previous();
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   for (int64_t i = row_ptr_src[N] + tid; i < E; i += (int64_t)gridDim.x * blockDim.x) perm_src[i] = 0;
   const int64_t n = tid / 32;
@@ -285,27 +292,28 @@ static int csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *p
   ZP_CUDA(cudaMemsetAsync(w.flag, 0, (char *)w.tmp - (char *)w.flag, st));
   if (E || atomic_numbers) {
     const int64_t items = atomic_numbers && N > E ? N : E;
-    count_kernel<<<(unsigned)zp_ceil_div(items > 0 ? items : 1, 256), 256, 0, st>>>(
-        E, N, src64, dst64, atomic_numbers, n_elements, w.cnt_dst, w.cnt_src, w.flag);
+    zp_launch(count_kernel, (unsigned)zp_ceil_div(items > 0 ? items : 1, 256), 256, 0, st, E, N, src64,
+              dst64, atomic_numbers, n_elements, w.cnt_dst, w.cnt_src, w.flag);
     ZP_LAUNCH_CHECK("count_kernel");
   }
   const ScanArgs a{{w.cnt_dst, w.cnt_src}, {row_ptr, row_ptr_src}, w.totals};
   const unsigned sb = N <= kScanOneBlock ? 1u : (unsigned)zp_ceil_div(N, kScanSpan);
   if (sb > 1) {
-    scan_totals_kernel<<<dim3(sb, 2), kScanThreads, 0, st>>>(N, a);
+    zp_launch(scan_totals_kernel, dim3(sb, 2), kScanThreads, 0, st, N, a);
     ZP_LAUNCH_CHECK("scan_totals_kernel");
   }
-  scan_kernel<<<dim3(sb, 2), kScanThreads, 0, st>>>(N, a);
+  zp_launch(scan_kernel, dim3(sb, 2), kScanThreads, 0, st, N, a);
   ZP_LAUNCH_CHECK("scan_kernel");
   if (E) {
-    bucket_kernel<<<eb, 256, 0, st>>>(E, N, src64, dst64, w.cnt_dst, w.tmp);
+    zp_launch(bucket_kernel, eb, 256, 0, st, E, N, src64, dst64, w.cnt_dst, w.tmp);
     ZP_LAUNCH_CHECK("bucket_kernel");
-    rank_dst_kernel<<<nbw, 256, 0, st>>>(N, E, src64, row_ptr, w.tmp, perm, src_sorted, dst_sorted);
+    zp_launch(rank_dst_kernel, nbw, 256, 0, st, N, E, src64, row_ptr, w.tmp, perm, src_sorted,
+              dst_sorted);
     ZP_LAUNCH_CHECK("rank_dst_kernel");
     // source view over sorted-edge ids
-    bucket_src_kernel<<<eb, 256, 0, st>>>(E, N, src_sorted, w.cnt_src, w.tmp);
+    zp_launch(bucket_src_kernel, eb, 256, 0, st, E, N, src_sorted, w.cnt_src, w.tmp);
     ZP_LAUNCH_CHECK("bucket_src_kernel");
-    rank_src_kernel<<<nbw, 256, 0, st>>>(N, E, row_ptr_src, w.tmp, perm_src);
+    zp_launch(rank_src_kernel, nbw, 256, 0, st, N, E, row_ptr_src, w.tmp, perm_src);
     ZP_LAUNCH_CHECK("rank_src_kernel");
   }
   return ZP_OK;

@@ -21,6 +21,7 @@ namespace {
 // fp32 matrices (blockIdx.z) -> planes (bf16, or fp16 with the tensor's scale), zero padding up to ld_out.
 // threadIdx.x walks the quads of a row, threadIdx.y / blockIdx.x the rows (no division anywhere).
 __global__ void split_planes_kernel(const __grid_constant__ ZpSplitList d) {
+  zp_after_previous();
   const int b = blockIdx.z;
   const float *__restrict__ in = d.in[b];
   const int64_t rows = d.rows[b], cols = d.cols[b], ld_in = d.ld_in[b];
@@ -48,6 +49,7 @@ __global__ void split_planes_kernel(const __grid_constant__ ZpSplitList d) {
 // largest node index the edge list names (the caller zeroed *out)
 __global__ void max_index_kernel(int64_t E, const int32_t *__restrict__ src,
                                  const int32_t *__restrict__ dst, int *out) {
+  zp_after_previous();
   int m = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < E;
        i += (int64_t)gridDim.x * blockDim.x)
@@ -63,6 +65,7 @@ __global__ void max_index_kernel(int64_t E, const int32_t *__restrict__ src,
 __global__ void absmax_row_range_kernel(const float *__restrict__ in, int64_t cols,
                                         const int32_t *first, const int32_t *last,
                                         int64_t min_rows, float *out) {
+  zp_after_previous();
   const int64_t r0 = first ? *first : 0;
   int64_t r1 = last ? (int64_t)*last + 1 : 0;
   if (r1 < min_rows) r1 = min_rows;
@@ -94,6 +97,7 @@ constexpr int kGateSub = 4;            // groups of kGateEdges edges per block o
 __global__ void gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
                                 const float *__restrict__ h1, const ZpPlanes ht,
                                 const ZpScale scale, float *gate_max) {
+  zp_after_previous();
   // blockIdx.x counts groups of kGateEdges edges; the items of a group are indexed with 32-bit
   // arithmetic (a 64-bit division per thread would cost more than the rest of the kernel)
   const int H4 = t.H / 4;
@@ -155,6 +159,7 @@ template <int LM>
 __global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
                                 const float *__restrict__ h1, const float *__restrict__ dht,
                                 const ZpPlanes dh1, const ZpScale scale) {
+  zp_after_previous();
   const int H4 = t.H / 4;
   const int item = blockIdx.y * blockDim.x + threadIdx.x;            // within a group of edges
   const int le = item / H4;
@@ -226,6 +231,7 @@ __global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant_
 constexpr int kMaxTile = 4096;
 __global__ void __launch_bounds__(256)
 max_list_kernel(const __grid_constant__ ZpMaxList d, const __grid_constant__ ZpTileRow row) {
+  zp_after_previous();
   const int total = row.first[row.n];
   int t = (int)((int64_t)total * blockIdx.x / gridDim.x);
   const int end = (int)((int64_t)total * (blockIdx.x + 1) / gridDim.x);
@@ -359,6 +365,7 @@ __device__ __forceinline__ void prep_tile(const ZpPrepList &d, int b, int tl, ui
 }
 __global__ void __launch_bounds__(256)
 prep_weights_kernel(const __grid_constant__ ZpPrepList d, const __grid_constant__ ZpTileRow tiles) {
+  zp_after_previous();
   __shared__ __align__(16) uint16_t tile[32][kPrepPitch];
   int b = 0;
   for (int t = blockIdx.x; t < tiles.first[tiles.n]; t += gridDim.x) {
@@ -414,6 +421,7 @@ __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, fl
 }
 __global__ void __launch_bounds__(256)
 finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ ZpTileRow tiles) {
+  zp_after_previous();
   __shared__ float red[32][9];
   int b = 0;
   for (int t = blockIdx.x; t < tiles.first[tiles.n]; t += gridDim.x) {
@@ -453,6 +461,7 @@ finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ Z
 __global__ void __launch_bounds__(256)
 colsum_part_kernel(int64_t rows, int64_t cols, int64_t per_block, const ZpPlanes a,
                    float *__restrict__ part) {
+  zp_after_previous();
   __shared__ float red[8][32][9];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int64_t c0 = ((int64_t)blockIdx.x * 32 + tx) * 8;
@@ -496,6 +505,7 @@ struct BoundDesc {
 __global__ void __launch_bounds__(256)
 conv1_bound_kernel(const BoundDesc d, const float *a1_scale, const float *wscales,
                    const float *__restrict__ bias, float *ht_scale) {
+  zp_after_previous();
   __shared__ float red[8];
   float m = 0.f;
   for (int i = threadIdx.x; i < d.n_bias; i += blockDim.x) m = fmaxf(m, fabsf(bias[i]));
@@ -521,7 +531,7 @@ int zp_launch_conv1_bound(const zp_plan *p, const float *a1_scale, const float *
   d.n = p->n_blocks;
   for (int m = 0; m < p->n_blocks; ++m) d.in[m] = p->c1_in[m];
   d.n_bias = p->c1_out[0];
-  conv1_bound_kernel<<<1, 256, 0, st>>>(d, a1_scale, wscales, bias, ht_scale);
+  zp_launch(conv1_bound_kernel, 1, 256, 0, st, d, a1_scale, wscales, bias, ht_scale);
   ZP_LAUNCH_CHECK("conv1_bound_kernel");
   return ZP_OK;
 }
@@ -538,8 +548,8 @@ int zp_launch_split_list(const ZpSplitList &list, cudaStream_t st) {
   const int by = 256 / bx;
   int64_t gx = zp_ceil_div(rows, by);
   if (gx > 148 * 32) gx = 148 * 32;
-  split_planes_kernel<<<dim3((unsigned)gx, (unsigned)zp_ceil_div(quads, bx), list.n), dim3(bx, by), 0,
-                        st>>>(list);
+  zp_launch(split_planes_kernel, dim3((unsigned)gx, (unsigned)zp_ceil_div(quads, bx), list.n),
+            dim3(bx, by), 0, st, list);
   ZP_LAUNCH_CHECK("split_planes_kernel");
   return ZP_OK;
 }
@@ -556,7 +566,7 @@ int zp_launch_max_list(const ZpMaxList &list, cudaStream_t st) {
   ZpTileRow row;
   for (int i = 0; i < list.n; ++i) row.add(zp_ceil_div(list.count[i], kMaxTile));
   if (row.total() == 0) return ZP_OK;
-  max_list_kernel<<<(unsigned)std::min(row.total(), 148 * 8), 256, 0, st>>>(list, row);
+  zp_launch(max_list_kernel, (unsigned)std::min(row.total(), 148 * 8), 256, 0, st, list, row);
   ZP_LAUNCH_CHECK("max_list_kernel");
   return ZP_OK;
 }
@@ -571,7 +581,7 @@ int zp_launch_prep_weights(ZpPrepList &list, cudaStream_t st) {
             zp_ceil_div(plain ? list.ld[i] : list.in[i], list.quads[i] ? 128 : 32));
   }
   if (row.total() == 0) return ZP_OK;
-  prep_weights_kernel<<<(unsigned)std::min(row.total(), 148 * 16), 256, 0, st>>>(list, row);
+  zp_launch(prep_weights_kernel, (unsigned)std::min(row.total(), 148 * 16), 256, 0, st, list, row);
   ZP_LAUNCH_CHECK("prep_weights_kernel");
   return ZP_OK;
 }
@@ -585,7 +595,7 @@ int zp_launch_finalize(ZpFinalList &list, cudaStream_t st) {
                                           : zp_ceil_div((int64_t)list.rows[i] * kin, list.quads[i] ? 1024 : 256));
   }
   if (row.total() == 0) return ZP_OK;
-  finalize_kernel<<<(unsigned)std::min(row.total(), 148 * 16), 256, 0, st>>>(list, row);
+  zp_launch(finalize_kernel, (unsigned)std::min(row.total(), 148 * 16), 256, 0, st, list, row);
   ZP_LAUNCH_CHECK("finalize_kernel");
   return ZP_OK;
 }
@@ -595,7 +605,7 @@ int zp_launch_max_index(int64_t E, const int32_t *src, const int32_t *dst, int *
   if (E == 0) return ZP_OK;
   int64_t blocks = zp_ceil_div(E, 256 * 4);
   if (blocks > 592) blocks = 592;
-  max_index_kernel<<<(unsigned)blocks, 256, 0, st>>>(E, src, dst, out);
+  zp_launch(max_index_kernel, (unsigned)blocks, 256, 0, st, E, src, dst, out);
   ZP_LAUNCH_CHECK("max_index_kernel");
   return ZP_OK;
 }
@@ -604,7 +614,7 @@ int zp_launch_absmax_row_range(const float *in, int64_t cols, const int32_t *fir
                                const int32_t *last, int64_t min_rows, float *out,
                                cudaStream_t st) {
   if (cols == 0 || (cols & 3)) return cols ? ZP_ERR_INVALID_ARG : ZP_OK;
-  absmax_row_range_kernel<<<1184, 256, 0, st>>>(in, cols, first, last, min_rows, out);
+  zp_launch(absmax_row_range_kernel, 1184, 256, 0, st, in, cols, first, last, min_rows, out);
   ZP_LAUNCH_CHECK("absmax_row_range_kernel");
   return ZP_OK;
 }
@@ -615,7 +625,7 @@ int zp_launch_gate_fwd(const zp_plan *p, int64_t E, const float *h1, const ZpPla
   const int per_group = kGateEdges * ((p->t.Km + 1) / 2) * (p->t.H / 4);
   const dim3 grid((unsigned)zp_ceil_div(E, kGateEdges * kGateSub),
                   (unsigned)zp_ceil_div(per_group, 256));
-  gate_fwd_kernel<<<grid, 256, 0, st>>>(p->t, E, h1, ht, scale, gate_max);
+  zp_launch(gate_fwd_kernel, grid, 256, 0, st, p->t, E, h1, ht, scale, gate_max);
   ZP_LAUNCH_CHECK("gate_fwd_kernel");
   return ZP_OK;
 }
@@ -625,7 +635,7 @@ int zp_launch_gate_bwd(const zp_plan *p, int64_t E, const float *h1, const float
   if (E == 0) return ZP_OK;
   const int per_group = kGateEdges * (p->t.H / 4);
   const dim3 grid((unsigned)zp_ceil_div(E, kGateEdges), (unsigned)zp_ceil_div(per_group, 128));
-#define CALL(LM) gate_bwd_kernel<LM><<<grid, 128, 0, st>>>(p->t, E, h1, dht, dh1, scale)
+#define CALL(LM) zp_launch(gate_bwd_kernel<LM>, grid, 128, 0, st, p->t, E, h1, dht, dh1, scale)
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("gate_bwd_kernel");
@@ -671,7 +681,8 @@ int zp_launch_colsum(int64_t rows, int64_t cols, const ZpPlanes &a, float *out, 
   const int64_t nparts = zp_colsum_parts(rows, cols);
   if (nparts > 0) {
     const dim3 grid((unsigned)zp_ceil_div(cols, 256), (unsigned)nparts), block(32, 8);
-    colsum_part_kernel<<<grid, block, 0, st>>>(rows, cols, zp_colsum_rows(rows, cols), a, scratch);
+    zp_launch(colsum_part_kernel, grid, block, 0, st, rows, cols, zp_colsum_rows(rows, cols), a,
+              scratch);
     ZP_LAUNCH_CHECK("colsum_part_kernel");
   }
   list.add(scratch, out, cols, 1, (int)cols, (int)nparts, ZP_FIN_COLUMN);

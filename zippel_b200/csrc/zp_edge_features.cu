@@ -58,6 +58,7 @@ edge_features_fwd_kernel(int64_t E, zp_front_config cfg, const float *__restrict
                          float *__restrict__ dist_out, float *__restrict__ x_edge,
                          const ZpPlanes xp, const ZpScale scale, float *__restrict__ env_out, float *__restrict__ cos_s,
                          float *__restrict__ sin_s) {
+  zp_after_previous();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t e = (int64_t)blockIdx.x * kWarps + warp;
   const float inv = xp.planes ? zp_publish_scale(xp, scale, blockIdx.x == 0 && threadIdx.x == 0) : 1.f;
@@ -132,6 +133,7 @@ edge_features_bwd_edge_kernel(int64_t E, zp_front_config cfg, const float *__res
                               const float *__restrict__ gx, int64_t ldg,
                               const float *__restrict__ g_env, const float *__restrict__ g_vec_in,
                               float *__restrict__ g_vec) {
+  zp_after_previous();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t e = (int64_t)blockIdx.x * kWarps + warp;
   if (e >= E) return;
@@ -172,6 +174,7 @@ edge_features_bwd_node_kernel(int64_t N, zp_front_config cfg, const float *__res
                               const int32_t *__restrict__ perm_src,
                               const int32_t *__restrict__ row_ptr_src, float *__restrict__ g_pos,
                               float *__restrict__ node_emb) {
+  zp_after_previous();
   const int64_t n = blockIdx.x;
   const int beg = row_ptr[n], end = row_ptr[n + 1];
   const int sbeg = row_ptr_src[n], send = row_ptr_src[n + 1];
@@ -202,6 +205,7 @@ constexpr int kElemSlices = 8;           // the rows of one element are a serial
 __global__ void __launch_bounds__(128)
 edge_features_bwd_elem_kernel(int64_t N, int EC, const int64_t *__restrict__ z,
                               const float *__restrict__ node_emb, float *__restrict__ partial) {
+  zp_after_previous();
   __shared__ unsigned char mine[128];
   __shared__ int any;
   const int64_t elem = blockIdx.x;
@@ -241,6 +245,7 @@ edge_features_bwd_elem_kernel(int64_t N, int EC, const int64_t *__restrict__ z,
 
 __global__ void edge_features_elem_sum_kernel(int64_t total, const float *__restrict__ partial,
                                              float *__restrict__ g_emb) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   float s = 0.f;
@@ -268,9 +273,9 @@ int zp_launch_edge_features_fwd(const zp_front_config &cfg, int64_t E, const flo
                                 float *cos_sorted, float *sin_sorted, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const ZpPlanes xp = x_planes ? *x_planes : ZpPlanes{nullptr, 0, 0, 0, 0, nullptr};
-  edge_features_fwd_kernel<<<(unsigned)zp_ceil_div(E, kWarps), 32 * kWarps, 0, st>>>(
-      E, cfg, pos, shifts, atomic_numbers, emb, gauss_offsets, cos_g, sin_g, perm, src, dst,
-      edge_vec, dist, x_edge, xp, scale, env, cos_sorted, sin_sorted);
+  zp_launch(edge_features_fwd_kernel, (unsigned)zp_ceil_div(E, kWarps), 32 * kWarps, 0, st, E, cfg,
+            pos, shifts, atomic_numbers, emb, gauss_offsets, cos_g, sin_g, perm, src, dst, edge_vec,
+            dist, x_edge, xp, scale, env, cos_sorted, sin_sorted);
   ZP_LAUNCH_CHECK("edge_features_fwd_kernel");
   return ZP_OK;
 }
@@ -286,24 +291,23 @@ int zp_launch_edge_features_bwd(const zp_front_config &cfg, int64_t N, int64_t E
   float *node_emb = reinterpret_cast<float *>(static_cast<unsigned char *>(work) +
                                               zp_align_up(sizeof(float) * 3 * (size_t)E, 256));
   if (E && grad_pos) {
-    edge_features_bwd_edge_kernel<<<(unsigned)zp_ceil_div(E, kWarps), 32 * kWarps, 0, st>>>(
-        E, cfg, edge_vec, dist, gauss_offsets, grad_x_edge, ldg, grad_env, grad_edge_vec, g_vec);
+    zp_launch(edge_features_bwd_edge_kernel, (unsigned)zp_ceil_div(E, kWarps), 32 * kWarps, 0, st, E,
+              cfg, edge_vec, dist, gauss_offsets, grad_x_edge, ldg, grad_env, grad_edge_vec, g_vec);
     ZP_LAUNCH_CHECK("edge_features_bwd_edge_kernel");
   }
-  edge_features_bwd_node_kernel<<<(unsigned)N, 128, 0, st>>>(
-      N, cfg, g_vec, grad_x_edge, ldg, row_ptr, perm_src, row_ptr_src, grad_pos,
-      grad_emb ? node_emb : nullptr);
+  zp_launch(edge_features_bwd_node_kernel, (unsigned)N, 128, 0, st, N, cfg, g_vec, grad_x_edge, ldg,
+            row_ptr, perm_src, row_ptr_src, grad_pos, grad_emb ? node_emb : nullptr);
   ZP_LAUNCH_CHECK("edge_features_bwd_node_kernel");
   if (grad_emb) {
     float *partial = reinterpret_cast<float *>(
         reinterpret_cast<unsigned char *>(node_emb) +
         zp_align_up(sizeof(float) * (size_t)N * cfg.edge_channels, 256));
     const int64_t total = (int64_t)cfg.n_elements * cfg.edge_channels;
-    edge_features_bwd_elem_kernel<<<dim3((unsigned)cfg.n_elements, kElemSlices), 128, 0, st>>>(
-        N, cfg.edge_channels, atomic_numbers, node_emb, partial);
+    zp_launch(edge_features_bwd_elem_kernel, dim3((unsigned)cfg.n_elements, kElemSlices), 128, 0, st,
+              N, cfg.edge_channels, atomic_numbers, node_emb, partial);
     ZP_LAUNCH_CHECK("edge_features_bwd_elem_kernel");
-    edge_features_elem_sum_kernel<<<(unsigned)zp_ceil_div(total, 256), 256, 0, st>>>(total, partial,
-                                                                                  grad_emb);
+    zp_launch(edge_features_elem_sum_kernel, (unsigned)zp_ceil_div(total, 256), 256, 0, st, total,
+              partial, grad_emb);
     ZP_LAUNCH_CHECK("edge_features_elem_sum_kernel");
   }
   return ZP_OK;

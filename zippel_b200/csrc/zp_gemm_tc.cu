@@ -836,11 +836,13 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
 
 template <int P, int BK, int STAGES, int BN_CAP>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmGroup g) {
+  zp_after_previous();
   gemm_tc_body<P, BK, STAGES, BN_CAP, ZP_EPI_NONE>(g);
 }
 // the same contraction with a fused epilogue (the epilogue warps hold more live values)
 template <int P, int BK, int STAGES, int BN_CAP, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_fused_kernel(const __grid_constant__ GemmGroup g) {
+  zp_after_previous();
   gemm_tc_body<P, BK, STAGES, BN_CAP, EPI>(g);
 }
 
@@ -872,6 +874,7 @@ struct ShortLayout {
 template <int P>
 __global__ void __launch_bounds__(kShortThreads, 1)
 gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
+  zp_after_previous();
   using L = ShortLayout<P>;
   constexpr int STAGES = L::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -1380,11 +1383,13 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
 
 template <int P, int BK, int STAGES>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_pair_kernel(const __grid_constant__ GemmGroup g) {
+  zp_after_previous();
   gemm_tc_pair_body<P, BK, STAGES, ZP_EPI_NONE>(g);
 }
 template <int P, int BK, int STAGES, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_fused_kernel(const __grid_constant__ GemmGroup g) {
+  zp_after_previous();
   gemm_tc_pair_body<P, BK, STAGES, EPI>(g);
 }
 
@@ -1392,6 +1397,7 @@ gemm_tc_pair_fused_kernel(const __grid_constant__ GemmGroup g) {
 // block b (row_ptr[0] = 0 and row_ptr[n_nodes] = E > 32 b)
 __global__ void block_node_kernel(int64_t n_blocks, int n_nodes, const int32_t *__restrict__ row_ptr,
                                   int32_t *__restrict__ block_node) {
+  zp_after_previous();
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n_blocks) return;
   const int e = (int)(b * 32);
@@ -1626,7 +1632,7 @@ int launch_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
   GemmGroup grp;
   if ((rc = fill_group(grp, g, n, P, BK, BM, 1, BN_CAP))) return rc;
   const int sms = device_sms(), grid = grp.total < sms ? grp.total : sms;
-  kernel<<<grid, kThreads, L::kTotal, st>>>(grp);
+  zp_launch(kernel, grid, kThreads, L::kTotal, st, grp);
   ZP_LAUNCH_CHECK("gemm_tc_kernel");
   return ZP_OK;
 }
@@ -1645,7 +1651,7 @@ int launch_short(const ZpGemmTc &g, cudaStream_t st) {
   grp.rows_apart = columns <= sms ? std::min(sms / columns, rows) : 0;
   if (grp.rows_apart < rows && columns * grp.rows_apart * 10 < sms * 9) grp.rows_apart = 0;
   const int grid = grp.rows_apart ? columns * grp.rows_apart : std::min(grp.total, sms);
-  gemm_tc_short_kernel<P><<<grid, kShortThreads, L::kTotal, st>>>(grp);
+  zp_launch(gemm_tc_short_kernel<P>, grid, kShortThreads, L::kTotal, st, grp);
   ZP_LAUNCH_CHECK("gemm_tc_short_kernel");
   return ZP_OK;
 }
@@ -1669,7 +1675,9 @@ int launch_pair_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
     if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_pair_kernel<P, BK, STAGES>;
     else return gemm_tc_pair_fused_kernel<P, BK, STAGES, EPI>;
   }();
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
@@ -1697,6 +1705,7 @@ int launch_pair_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
   GemmGroup grp;
   if (const int rc = fill_group(grp, g, n, P, BK, BM2, 2, 256)) return rc;
   cfg.gridDim = dim3((unsigned)(2 * (grp.total < max_pairs ? grp.total : max_pairs)));
+  cfg.numAttrs = 2;
   ZP_CUDA(cudaLaunchKernelEx(&cfg, kernel, grp));
   ZP_LAUNCH_CHECK("gemm_tc_pair_kernel");
   return ZP_OK;
@@ -1779,7 +1788,8 @@ int zp_launch_block_nodes(int64_t E, int64_t N, const int32_t *row_ptr, int32_t 
                           cudaStream_t st) {
   const int64_t nb = zp_ceil_div(E, 32);
   if (nb == 0 || N == 0) return ZP_OK;
-  block_node_kernel<<<(unsigned)zp_ceil_div(nb, 256), 256, 0, st>>>(nb, (int)N, row_ptr, block_node);
+  zp_launch(block_node_kernel, (unsigned)zp_ceil_div(nb, 256), 256, 0, st, nb, (int)N, row_ptr,
+            block_node);
   ZP_LAUNCH_CHECK("block_node_kernel");
   return ZP_OK;
 }

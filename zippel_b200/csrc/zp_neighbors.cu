@@ -84,6 +84,7 @@ __device__ __forceinline__ unsigned image_code(int nkx, int nky, int nkz, int re
 __global__ void cell_count_kernel(int64_t N, const double *__restrict__ pos, Grid g,
                                   int32_t *__restrict__ atom_cell, int4 *__restrict__ own,
                                   int32_t *cell_count, int32_t *flags) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const double x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
@@ -105,6 +106,7 @@ __global__ void cell_fill_kernel(int64_t N, const double *__restrict__ pos, Grid
                                  const int32_t *__restrict__ atom_cell,
                                  const int4 *__restrict__ own, const int32_t *__restrict__ cell_start, int32_t *cell_cursor,
                                  const Sorted out) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   const int c = atom_cell[i];
@@ -119,6 +121,7 @@ __global__ void cell_fill_kernel(int64_t N, const double *__restrict__ pos, Grid
 // the block totals, add back
 __global__ void scan_block_kernel(int64_t n, const int32_t *__restrict__ in, int32_t *out,
                                   int32_t *block_sums) {
+  zp_after_previous();
   __shared__ int32_t s[kScanBlock];
   const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
   const int32_t mine = i < n ? in[i] : 0;
@@ -134,6 +137,7 @@ __global__ void scan_block_kernel(int64_t n, const int32_t *__restrict__ in, int
   if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = s[threadIdx.x];
 }
 __global__ void scan_sums_kernel(int64_t nb, int32_t *block_sums) {
+  zp_after_previous();
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     int32_t run = 0;
     for (int64_t b = 0; b < nb; ++b) {
@@ -144,6 +148,7 @@ __global__ void scan_sums_kernel(int64_t nb, int32_t *block_sums) {
   }
 }
 __global__ void scan_add_kernel(int64_t n, int32_t *out, const int32_t *__restrict__ block_sums) {
+  zp_after_previous();
   const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
   if (i <= n) out[i] += block_sums[blockIdx.x];
 }
@@ -151,11 +156,11 @@ __global__ void scan_add_kernel(int64_t n, int32_t *out, const int32_t *__restri
 int exclusive_scan(int64_t n, const int32_t *in, int32_t *out, int32_t *block_sums,
                    cudaStream_t st) {
   const int64_t nb = zp_ceil_div(n + 1, kScanBlock);
-  scan_block_kernel<<<(unsigned)nb, kScanBlock, 0, st>>>(n, in, out, block_sums);
+  zp_launch(scan_block_kernel, (unsigned)nb, kScanBlock, 0, st, n, in, out, block_sums);
   ZP_LAUNCH_CHECK("scan_block_kernel");
-  scan_sums_kernel<<<1, 32, 0, st>>>(nb, block_sums);
+  zp_launch(scan_sums_kernel, 1, 32, 0, st, nb, block_sums);
   ZP_LAUNCH_CHECK("scan_sums_kernel");
-  scan_add_kernel<<<(unsigned)nb, kScanBlock, 0, st>>>(n, out, block_sums);
+  zp_launch(scan_add_kernel, (unsigned)nb, kScanBlock, 0, st, n, out, block_sums);
   ZP_LAUNCH_CHECK("scan_add_kernel");
   return ZP_OK;
 }
@@ -243,6 +248,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock)
 count_kernel(int64_t N, Grid g,
              const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
              int32_t *__restrict__ counts, int32_t *flags) {
+  zp_after_previous();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t at = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
   if (at >= N) return;
@@ -315,6 +321,7 @@ fill_few_kernel(int64_t N, const int4 *__restrict__ own, Grid g,
                 const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
                 const int32_t *__restrict__ row_ptr, int64_t E, int64_t *__restrict__ edge_index,
                 double *__restrict__ shifts, int32_t *flags, int32_t *__restrict__ crowded) {
+  zp_after_previous();
   __shared__ Hit hits[kFillWarps][kFewHits];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t at = (int64_t)blockIdx.x * kFillWarps + warp;
@@ -408,6 +415,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ o
                  const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
                  const int32_t *__restrict__ row_ptr, int64_t E, int64_t *__restrict__ edge_index,
                  double *__restrict__ shifts, int32_t *flags) {
+  zp_after_previous();
   extern __shared__ unsigned char smem_raw[];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   Hit *h = reinterpret_cast<Hit *>(smem_raw) + (size_t)warp * kHitCap;
@@ -553,17 +561,17 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
   ZP_CUDA(cudaMemsetAsync(w.flags, 0, 4 * sizeof(int32_t), st));
   ZP_CUDA(cudaMemsetAsync(w.cell_count, 0, (w.cell_start - w.cell_count) * sizeof(int32_t), st));
   if (N > 0) {
-    cell_count_kernel<<<(unsigned)zp_ceil_div(N, 256), 256, 0, st>>>(N, pos, g, w.atom_cell, w.own,
-                                                                     w.cell_count, w.flags);
+    zp_launch(cell_count_kernel, (unsigned)zp_ceil_div(N, 256), 256, 0, st, N, pos, g, w.atom_cell,
+              w.own, w.cell_count, w.flags);
     ZP_LAUNCH_CHECK("cell_count_kernel");
   }
   if ((rc = exclusive_scan((int64_t)cells, w.cell_count, w.cell_start, w.block_sums, st))) return rc;
   if (N > 0) {
-    cell_fill_kernel<<<(unsigned)zp_ceil_div(N, 256), 256, 0, st>>>(N, pos, g, w.atom_cell, w.own,
-                                                                    w.cell_start, w.cell_cursor, w.atoms);
+    zp_launch(cell_fill_kernel, (unsigned)zp_ceil_div(N, 256), 256, 0, st, N, pos, g, w.atom_cell,
+              w.own, w.cell_start, w.cell_cursor, w.atoms);
     ZP_LAUNCH_CHECK("cell_fill_kernel");
-    count_kernel<<<(unsigned)zp_ceil_div(N, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st>>>(
-        N, g, w.cell_start, w.atoms, max_neighbors, w.counts, w.flags);
+    zp_launch(count_kernel, (unsigned)zp_ceil_div(N, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st, N, g,
+              w.cell_start, w.atoms, max_neighbors, w.counts, w.flags);
     ZP_LAUNCH_CHECK("count_kernel");
   }
   if ((rc = exclusive_scan(N, w.counts, row_ptr, w.block_sums, st))) return rc;
@@ -586,17 +594,16 @@ int zp_neighbors_fill(const double *pos, int64_t N, double box, double cutoff, i
   cudaStream_t st = (cudaStream_t)stream;
   ZP_CUDA(cudaMemsetAsync(w.crowded, 0, sizeof(int32_t), st));
   if (N > 0) {
-    fill_few_kernel<<<(unsigned)zp_ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st>>>(
-        N, w.own, g, w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags,
-        w.crowded);
+    zp_launch(fill_few_kernel, (unsigned)zp_ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st, N, w.own,
+              g, w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags,
+              w.crowded);
     ZP_LAUNCH_CHECK("fill_few_kernel");
     const size_t smem = sizeof(Hit) * kHitCap * kWarpsPerBlock;
     static ZpSmemOptIn opt_in;
     if (int rc_ = zp_ensure_smem(fill_many_kernel, smem, opt_in)) return rc_;
     const unsigned blocks = (unsigned)std::min<int64_t>(zp_ceil_div(N, kWarpsPerBlock), 148 * 3);
-    fill_many_kernel<<<blocks, 32 * kWarpsPerBlock, smem, st>>>(w.crowded, w.own, g, w.cell_start, w.atoms,
-                                                                max_neighbors, row_ptr, E, edge_index,
-                                                                shifts, w.flags);
+    zp_launch(fill_many_kernel, blocks, 32 * kWarpsPerBlock, smem, st, w.crowded, w.own, g,
+              w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags);
     ZP_LAUNCH_CHECK("fill_many_kernel");
   }
   ZP_CUDA(cudaMemcpyAsync(flags_out, w.flags, sizeof(int32_t), cudaMemcpyDeviceToDevice, st));

@@ -33,6 +33,7 @@ ln_silu_fwd_kernel(int64_t rows, int width, const float *__restrict__ x,
                    const float *__restrict__ gamma, const float *__restrict__ beta, float eps,
                    float *__restrict__ y, const ZpPlanes yp, const ZpScale scale,
                    float *__restrict__ mean_out, float *__restrict__ rstd_out, float *rstd_max) {
+  zp_after_previous();
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const float inv = yp.planes ? zp_publish_scale(yp, scale, blockIdx.x == 0 && threadIdx.x == 0) : 1.f;
   float seen = 0.f;
@@ -109,7 +110,8 @@ ln_silu_bwd_kernel(int64_t rows, int width, const float *__restrict__ x,
                    const float *__restrict__ gamma, const float *__restrict__ beta,
                    const float *__restrict__ mean_in, const float *__restrict__ rstd_in,
                    const float *__restrict__ dy, float *__restrict__ dx, const ZpPlanes dxp,
-                   const ZpScale scale, float *__restrict__ partial) {   // [gridDim.x][NP][width]
+                   const ZpScale scale, float *__restrict__ partial) {
+  zp_after_previous();   // [gridDim.x][NP][width]
   extern __shared__ float red[];                              // [kWarps][NP][width]
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const float inv = dxp.planes ? zp_publish_scale(dxp, scale, blockIdx.x == 0 && threadIdx.x == 0) : 1.f;
@@ -218,7 +220,7 @@ int zp_launch_ln_silu_fwd(int64_t rows, int width, const float *x, const float *
   const int groups = (width + 127) / 128;
   const unsigned grid = (unsigned)std::min<int64_t>(zp_ceil_div(rows, kWarps), 148 * 8);
 #define CALL(G)                                                                                   \
-  ln_silu_fwd_kernel<G><<<grid, 32 * kWarps, 0, st>>>(rows, width, x, gamma, beta, eps, y, yp, scale, \
+  zp_launch(ln_silu_fwd_kernel<G>, grid, 32 * kWarps, 0, st, rows, width, x, gamma, beta, eps, y, yp, scale, \
                                                       mean, rstd, rstd_max)
   ZP_DISPATCH_GROUPS(groups, CALL);
 #undef CALL
@@ -241,7 +243,7 @@ int zp_launch_ln_silu_bwd(int64_t rows, int width, const float *x, const float *
   do {                                                                                          \
     static ZpSmemOptIn opt_in;                                                                  \
     if (int rc_ = zp_ensure_smem(ln_silu_bwd_kernel<G, NP>, smem, opt_in)) return rc_;          \
-    ln_silu_bwd_kernel<G, NP><<<blocks, 32 * kWarps, smem, st>>>(                               \
+    zp_launch(ln_silu_bwd_kernel<G, NP>, blocks, 32 * kWarps, smem, st, \
         rows, width, x, gamma, beta, mean, rstd, dy, dx, dxp, scale, partial);                  \
   } while (0)
 #define CALL(G)                      \

@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(128)
 node_invariants_kernel(const __grid_constant__ ZpTables t, int64_t N,
                        const float *__restrict__ node_out, float *__restrict__ inv,
                        const float *__restrict__ w0, float *slots) {
+  zp_after_previous();
   const int64_t n = blockIdx.x;
   const int W = (t.lmax + 1) * t.C;
   float most = 0.f;
@@ -69,6 +70,7 @@ __global__ void __launch_bounds__(128)
 node_invariants_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N,
                            const float *__restrict__ node_out, const float *__restrict__ g_inv,
                            float *__restrict__ grad_node_out) {
+  zp_after_previous();
   const int64_t n = blockIdx.x;
   const float *row = node_out + (size_t)n * t.K * t.C;
   const float *gi = g_inv + (size_t)n * (t.lmax + 1) * t.C;
@@ -88,6 +90,7 @@ __global__ void __launch_bounds__(256)
 head_fwd_kernel(int64_t N, int C, const float *__restrict__ hid, const float *__restrict__ w1,
                 const float *__restrict__ b1, float *e_node, float *__restrict__ energy,
                 unsigned *done) {
+  zp_after_previous();
   __shared__ float part[1024];
   __shared__ bool last;
   const int64_t n = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
@@ -128,6 +131,7 @@ __global__ void __launch_bounds__(128)
 head_bwd_kernel(int64_t N, int C, const float *__restrict__ hid, const float *__restrict__ w1,
                 const float *__restrict__ grad_e, float *__restrict__ g_hid,
                 float *__restrict__ partial, float *slots) {
+  zp_after_previous();
   const float ge = grad_e[0];
   float most = 0.f;
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -149,6 +153,7 @@ head_bwd_kernel(int64_t N, int C, const float *__restrict__ hid, const float *__
 __global__ void head_param_grad_kernel(int64_t N, int C, const float *__restrict__ partial,
                                        const float *__restrict__ grad_e, float *__restrict__ grad_w1,
                                        float *__restrict__ grad_b1) {
+  zp_after_previous();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const float ge = grad_e[0];
   if (c < C) {
@@ -210,14 +215,14 @@ int zp_readout_forward(const zp_plan *plan, int64_t N, const float *node_out, co
   }
   float *slots = static_cast<float *>(rw.linear);
   ZP_CUDA(cudaMemsetAsync(slots, 0, kLinSlots * sizeof(float), st));
-  node_invariants_kernel<<<(unsigned)(N + (plan->fp16 ? kWeightBlocks : 0)), 128, 0, st>>>(
-      t, N, node_out, rw.inv, w0, plan->fp16 ? slots : nullptr);
+  zp_launch(node_invariants_kernel, (unsigned)(N + (plan->fp16 ? kWeightBlocks : 0)), 128, 0, st, t, N,
+            node_out, rw.inv, w0, plan->fp16 ? slots : nullptr);
   ZP_LAUNCH_CHECK("node_invariants_kernel");
   int rc = zp_linear_forward_maxima(plan, N, (int64_t)(t.lmax + 1) * t.C, t.C, rw.inv, w0, b0, rw.hid,
                                     rw.linear, st);
   if (rc) return rc;
-  head_fwd_kernel<<<(unsigned)zp_ceil_div(N * 32, 256), 256, 0, st>>>(
-      N, t.C, rw.hid, w1, b1, rw.e_node, energy, reinterpret_cast<unsigned *>(slots + kLinSlotFree));
+  zp_launch(head_fwd_kernel, (unsigned)zp_ceil_div(N * 32, 256), 256, 0, st, N, t.C, rw.hid, w1, b1,
+            rw.e_node, energy, reinterpret_cast<unsigned *>(slots + kLinSlotFree));
   ZP_LAUNCH_CHECK("head_fwd_kernel");
   return ZP_OK;
 }
@@ -247,19 +252,20 @@ int zp_readout_backward(const zp_plan *plan, int64_t N, const float *node_out, c
   }
   float *slots = plan->fp16 ? static_cast<float *>(rw.linear) : nullptr;
   if (slots) ZP_CUDA(cudaMemsetAsync(slots + kLinSlotDy, 0, sizeof(float), st));
-  head_bwd_kernel<<<kSumBlocks, 128, 0, st>>>(N, t.C, rw.hid, w1, grad_energy, rw.g_hid,
-                                              frozen ? nullptr : rw.partial, slots);
+  zp_launch(head_bwd_kernel, kSumBlocks, 128, 0, st, N, t.C, rw.hid, w1, grad_energy, rw.g_hid,
+            frozen ? nullptr : rw.partial, slots);
   ZP_LAUNCH_CHECK("head_bwd_kernel");
   if (!frozen) {
-    head_param_grad_kernel<<<(unsigned)zp_ceil_div(t.C, 128), 128, 0, st>>>(
-        N, t.C, rw.partial, grad_energy, grad_w1, grad_b1);
+    zp_launch(head_param_grad_kernel, (unsigned)zp_ceil_div(t.C, 128), 128, 0, st, N, t.C, rw.partial,
+              grad_energy, grad_w1, grad_b1);
     ZP_LAUNCH_CHECK("head_param_grad_kernel");
   }
   // the hidden layer's operand planes are still in the work buffer the forward used
   int rc = zp_linear_backward_maxima(plan, N, W, t.C, rw.g_hid, rw.g_inv, grad_w0, grad_b0,
                                      rw.linear, st);
   if (rc) return rc;
-  node_invariants_bwd_kernel<<<(unsigned)N, 128, 0, st>>>(t, N, node_out, rw.g_inv, grad_node_out);
+  zp_launch(node_invariants_bwd_kernel, (unsigned)N, 128, 0, st, t, N, node_out, rw.g_inv,
+            grad_node_out);
   ZP_LAUNCH_CHECK("node_invariants_bwd_kernel");
   return ZP_OK;
 }

@@ -79,6 +79,7 @@ rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
                  const float *__restrict__ x, const int32_t *__restrict__ src,
                  const int32_t *__restrict__ dst, const float *__restrict__ rot,
                  const float *__restrict__ radial, const ZpPlanes a1, const ZpScale scale) {
+  zp_after_previous();
   extern __shared__ __align__(16) float rot_in_s[];  // radial [rad_rows][blockDim] x 4 | rot [epb][rot_ld] dup.
   const int ls = 4 * blockDim.x;
   float *rad_s = rot_in_s + 4 * threadIdx.x;
@@ -160,6 +161,7 @@ rotate_back_scatter_kernel(const __grid_constant__ ZpTables t, int64_t N,
                            const float *__restrict__ y, const float *__restrict__ env,
                            const float *__restrict__ rot, const int32_t *__restrict__ row_ptr,
                            float *__restrict__ node_out) {
+  zp_after_previous();
   constexpr int K = (LMAX + 1) * (LMAX + 1);
   constexpr int W = 32 * VEC;              // channels of this block
   constexpr int P = VEC / 2;
@@ -244,6 +246,7 @@ __global__ void __launch_bounds__(128)
 node_reduce_kernel(int64_t N, int KC4, const float4 *__restrict__ du_both,
                    const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ perm_src,
                    const int32_t *__restrict__ row_ptr_src, float4 *__restrict__ grad_x) {
+  zp_after_previous();
   const int64_t n = blockIdx.x;
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (n >= N || i >= KC4) return;
@@ -275,6 +278,7 @@ __global__ void __launch_bounds__(128)
 node_sum_kernel(const __grid_constant__ ZpTables t, int64_t N, const float *__restrict__ head,
                 const float *__restrict__ cont, const int32_t *__restrict__ row_ptr,
                 float *__restrict__ node_out) {
+  zp_after_previous();
   const int64_t n = blockIdx.x;
   const int C4 = t.C / 4;
   const int beg = row_ptr[n], end = row_ptr[n + 1];
@@ -308,7 +312,7 @@ node_sum_kernel(const __grid_constant__ ZpTables t, int64_t N, const float *__re
 int zp_launch_node_sum(const zp_plan *p, int64_t N, const float *head, const float *cont,
                        const int32_t *row_ptr, float *node_out, cudaStream_t st) {
   if (N == 0) return ZP_OK;
-  node_sum_kernel<<<(unsigned)N, 128, 0, st>>>(p->t, N, head, cont, row_ptr, node_out);
+  zp_launch(node_sum_kernel, (unsigned)N, 128, 0, st, p->t, N, head, cont, row_ptr, node_out);
   ZP_LAUNCH_CHECK("node_sum_kernel");
   return ZP_OK;
 }
@@ -328,7 +332,8 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(rotate_in_kernel<LM, FMT>, smem, opt_in)) return rc_;            \
-    rotate_in_kernel<LM, FMT><<<grid, block, smem, st>>>(t, E, epb, x, src, dst, rot, radial, a1, scale); \
+    zp_launch(rotate_in_kernel<LM, FMT>, grid, block, smem, st, t, E, epb, x, src, dst, rot,      \
+              radial, a1, scale);                                                                 \
     break;                                                                                        \
   }
 #define CALL(LM)                                               \
@@ -358,7 +363,7 @@ int zp_launch_rotate_back_scatter(const zp_plan *p, int64_t N, const float *y, c
     auto kern = vec == 4 ? rotate_back_scatter_kernel<LM, 4> : rotate_back_scatter_kernel<LM, 2>; \
     static ZpSmemOptIn opt_in;             /* per instantiation and device */                    \
     if (int rc_ = zp_ensure_smem(kern, smem, opt_in)) return rc_;                              \
-    kern<<<grid, 32 * kBackWarps, smem, st>>>(t, N, y, env, rot, row_ptr, node_out);           \
+    zp_launch(kern, grid, 32 * kBackWarps, smem, st, t, N, y, env, rot, row_ptr, node_out);           \
   }
   ZP_DISPATCH_LMAX(t.lmax, CALL)
 #undef CALL
@@ -372,8 +377,8 @@ int zp_launch_node_reduce(const zp_plan *p, int64_t N, const float *du_both,
   if (N == 0) return ZP_OK;
   const int KC4 = p->t.K * p->t.C / 4;
   const dim3 grid((unsigned)N, (unsigned)zp_ceil_div(KC4, 128));
-  node_reduce_kernel<<<grid, 128, 0, st>>>(N, KC4, (const float4 *)du_both, row_ptr, perm_src,
-                                           row_ptr_src, (float4 *)grad_x);
+  zp_launch(node_reduce_kernel, grid, 128, 0, st, N, KC4, (const float4 *)du_both, row_ptr, perm_src,
+            row_ptr_src, (float4 *)grad_x);
   ZP_LAUNCH_CHECK("node_reduce_kernel");
   return ZP_OK;
 }

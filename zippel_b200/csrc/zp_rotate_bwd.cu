@@ -136,6 +136,7 @@ rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
                        const float *__restrict__ env, const float *__restrict__ rot,
                        const int32_t *__restrict__ dst, const ZpPlanes dy, const ZpScale scale,
                        float *__restrict__ grad_env, float4 *__restrict__ torque) {
+  zp_after_previous();
   extern __shared__ __align__(16) float4 edge_s[];
   float *y_s = reinterpret_cast<float *>(edge_s + blockDim.x) + 4 * threadIdx.x;
   const int ls = 4 * blockDim.x;
@@ -261,6 +262,7 @@ rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
                      const int32_t *__restrict__ dst, const float *__restrict__ rot,
                      float *__restrict__ grad_radial, const ZpPlanes grad_radial_planes,
                      const ZpScale scale, float *__restrict__ du_both, float4 *__restrict__ torque) {
+  zp_after_previous();
   extern __shared__ __align__(16) float4 edge_s[];
   const int ls = 4 * blockDim.x;
   float *da_s = reinterpret_cast<float *>(edge_s + blockDim.x) + 4 * threadIdx.x;
@@ -319,7 +321,7 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(rotate_grad_out_kernel<LM, FMT>, smem, opt_in)) return rc_;      \
-    rotate_grad_out_kernel<LM, FMT><<<grid, threads, smem, st>>>(                                 \
+    zp_launch(rotate_grad_out_kernel<LM, FMT>, grid, threads, smem, st,                           \
         t, E, epb, g, y, env, rot, dst, dy, scale, grad_env, reinterpret_cast<float4 *>(torque)); \
     break;                                                                                        \
   }
@@ -354,7 +356,7 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(rotate_in_bwd_kernel<LM, FMT>, smem, opt_in)) return rc_;        \
-    rotate_in_bwd_kernel<LM, FMT><<<grid, threads, smem, st>>>(                                   \
+    zp_launch(rotate_in_bwd_kernel<LM, FMT>, grid, threads, smem, st,                             \
         t, E, epb, da1, radial, x, src, dst, rot, grad_radial, gp, scale, du_both,                \
         reinterpret_cast<float4 *>(torque));                                                      \
     break;                                                                                        \

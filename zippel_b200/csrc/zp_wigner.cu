@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(kFwdThreads)
 wigner_fwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
                   const float *__restrict__ ev, const float *__restrict__ cgam,
                   const float *__restrict__ sgam, float *__restrict__ rot, int packed) {
+  zp_after_previous();
   extern __shared__ __align__(16) double smem_d[];       // frames [LMAX + 1][6][32] | out [32][ld + 1]
   double *frames = smem_d;
   float *out = reinterpret_cast<float *>(smem_d + (LMAX + 1) * 6 * 32);
@@ -323,6 +324,7 @@ wigner_bwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__
                   const float *__restrict__ ev, const float *__restrict__ cgam,
                   const float *__restrict__ sgam, const float *__restrict__ grot,
                   float *__restrict__ gev) {
+  zp_after_previous();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= E) return;
   chain_backward<LMAX>(t, J, ev + 3 * e, cgam + e * (LMAX + 1), sgam + e * (LMAX + 1),
@@ -343,6 +345,7 @@ edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restric
                      const float *__restrict__ ev, const float *__restrict__ cgam,
                      const float *__restrict__ sgam, const float4 *__restrict__ torque,
                      const ZpTorqueArgs a, float *__restrict__ gev) {
+  zp_after_previous();
   extern __shared__ float grads[];                      // [4 warps][nnz_pad]
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int64_t e = (int64_t)blockIdx.x * 128 + threadIdx.x;
@@ -413,7 +416,8 @@ int zp_launch_wigner_fwd(const zp_plan *p, int64_t E, const float *ev, const flo
   {                                                                                               \
     static ZpSmemOptIn opt_in;                                                                    \
     if (int rc_ = zp_ensure_smem(wigner_fwd_kernel<LM>, smem, opt_in)) return rc_;                \
-    wigner_fwd_kernel<LM><<<grid, kFwdThreads, smem, st>>>(p->t, p->jd_dev, E, ev, cg, sg, rot, packed); \
+    zp_launch(wigner_fwd_kernel<LM>, grid, kFwdThreads, smem, st, p->t, p->jd_dev, E, ev, cg, sg, rot,
+              packed); \
   }
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
@@ -426,7 +430,7 @@ int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const flo
   if (E == 0) return ZP_OK;
   const dim3 grid((unsigned)zp_ceil_div(E, 128)), block(128);
 #define CALL(LM) \
-  wigner_bwd_kernel<LM><<<grid, block, 0, st>>>(p->t, p->jd_dev, E, ev, cg, sg, grot, gev)
+  zp_launch(wigner_bwd_kernel<LM>, grid, block, 0, st, p->t, p->jd_dev, E, ev, cg, sg, grot, gev);
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("wigner_bwd_kernel");
@@ -440,7 +444,7 @@ int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const 
   const dim3 grid((unsigned)zp_ceil_div(E, 128)), block(128);
   const size_t smem = (size_t)4 * p->t.nnz_pad * sizeof(float);
 #define CALL(LM)                                                                                  \
-  edge_vec_grad_kernel<LM><<<grid, block, smem, st>>>(p->t, p->jd_dev, E, ev, cg, sg,             \
+  zp_launch(edge_vec_grad_kernel<LM>, grid, block, smem, st, p->t, p->jd_dev, E, ev, cg, sg,             \
                                                       reinterpret_cast<const float4 *>(torque), a, gev)
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
