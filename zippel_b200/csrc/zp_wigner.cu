@@ -416,8 +416,8 @@ int zp_launch_wigner_fwd(const zp_plan *p, int64_t E, const float *ev, const flo
   {                                                                                               \
     static ZpSmemOptIn opt_in;                                                                    \
     if (int rc_ = zp_ensure_smem(wigner_fwd_kernel<LM>, smem, opt_in)) return rc_;                \
-    zp_launch(wigner_fwd_kernel<LM>, grid, kFwdThreads, smem, st, p->t, p->jd_dev, E, ev, cg, sg, rot,
-              packed); \
+    zp_launch(wigner_fwd_kernel<LM>, grid, kFwdThreads, smem, st, p->t,                             \
+              p->jd_dev, E, ev, cg, sg, rot, packed);                                               \
   }
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
