@@ -394,7 +394,8 @@ __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, fl
   const float *p = f + (size_t)row * ld + c;
   const float *q = f + (size_t)(upper ? half + row : row - half) * ld + kin + c;
   const float sign = upper ? 1.f : -1.f;
-  float acc[V], v[V], u[V];
+  constexpr int kBatch = 8;
+  float acc[V], v[kBatch][V], u[kBatch][V];
 #pragma unroll
   for (int k = 0; k < V; ++k) acc[k] = 0.f;
   auto load = [](const float *from, float (&to)[V]) {
@@ -405,16 +406,19 @@ __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, fl
       to[0] = *from;
     }
   };
-#pragma unroll 4
-  for (int s = 0; s < parts; ++s) {
-    load(p + (size_t)s * stride, v);
-    if (folded) {
-      load(q + (size_t)s * stride, u);
+  for (int s0 = 0; s0 < parts; s0 += kBatch) {     // a batch on its way at a time
 #pragma unroll
-      for (int k = 0; k < V; ++k) v[k] += sign * u[k];
-    }
+    for (int b = 0; b < kBatch; ++b)
+      if (s0 + b < parts) {
+        load(p + (size_t)(s0 + b) * stride, v[b]);
+        if (folded) load(q + (size_t)(s0 + b) * stride, u[b]);
+      }
 #pragma unroll
-    for (int k = 0; k < V; ++k) acc[k] += v[k];
+    for (int b = 0; b < kBatch; ++b)
+      if (s0 + b < parts) {
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[k] += folded ? v[b][k] + sign * u[b][k] : v[b][k];
+      }
   }
   if (V == 4) *reinterpret_cast<float4 *>(dst + idx) = make_float4(acc[0], acc[V / 4], acc[V / 2], acc[V - 1]);
   else dst[idx] = acc[0];
@@ -439,10 +443,14 @@ finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ Z
     const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
     const int c = tile * 8 + tx;
     float s = 0.f;
-    if (c < cols) {
-#pragma unroll 8
-      for (int p = ty; p < parts; p += 32) s += f[(size_t)p * stride + c];
-    }
+    if (c < cols)
+      for (int p0 = ty; p0 < parts; p0 += 32 * 8) {
+        float v[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) v[b] = p0 + 32 * b < parts ? f[(size_t)(p0 + 32 * b) * stride + c] : 0.f;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) s += v[b];
+      }
     red[ty][tx] = s;
     __syncthreads();
     if (ty == 0 && c < cols) {
