@@ -676,7 +676,8 @@ class BlockFunction(torch.autograd.Function):
     """node_out = the whole block from positions and embeddings (``zp_block_forward``), with the VJP
     of all of it (``zp_block_backward``): reference blocks/eso2_ref.py:317-349 and autograd through
     it.  ``block`` gives the configuration, ``params`` are its parameters in registration order
-    without the readout; ``perm``: int32 positions of the graph's sorted edges in the per-edge arrays.
+    without the readout; ``perm``: int32 positions of the graph's sorted edges in the per-edge arrays
+    (None: the graph's own).
     fp32, first order only."""
 
     @staticmethod
@@ -750,11 +751,10 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
     if nbytes == 0:
         raise _lib.ZpError(2, "zp_block_workspace_bytes")
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
+    order = graph.addresses()
     call = _lib.ZpBlockCall(
         n1 - n0, e, n, n0, pos.data_ptr(), shifts.data_ptr(), z.data_ptr(), x.data_ptr(),
-        cos_g.data_ptr(), sin_g.data_ptr(), perm.data_ptr(), graph.src.data_ptr(),
-        graph.dst.data_ptr(), graph.row_ptr.data_ptr(), graph.perm_src.data_ptr(),
-        graph.row_ptr_src.data_ptr())
+        cos_g.data_ptr(), sin_g.data_ptr(), order[0] if perm is None else perm.data_ptr(), *order[1:])
     p = [t.data_ptr() for t in params]
     so2, keep = _weights_ptrs(plan.mmax, p[11:])
     cparams = _lib.ZpBlockParams(p[0], off.data_ptr(), _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
@@ -959,7 +959,7 @@ class ESO2Block(nn.Module):
             out = None
             if _surely_fits(plan, graph.n_edges):
                 try:
-                    out = function.apply(self, plan, graph, graph.perm, atomic_numbers, shifts,
+                    out = function.apply(self, plan, graph, None, atomic_numbers, shifts,
                                          cos_gamma_k, sin_gamma_k, x_ready, pos, x_node,
                                          *(self._all_params() if energy else self._block_params()))
                 except torch.cuda.OutOfMemoryError:

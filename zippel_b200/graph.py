@@ -139,17 +139,27 @@ class EdgeGraph:
         lib, ei, e, dev = EdgeGraph._open(edge_index)
         z = atomic_numbers.to(torch.int64).contiguous()
         n = z.shape[0]
-        perm, src, dst, perm_src, row_ptr, row_ptr_src, work = EdgeGraph._arrays(lib, e, n, dev)
+        graph = EdgeGraph.__new__(EdgeGraph)
+        graph.n_nodes, graph.n_edges = n, e
+        # all arrays and the scratch in one allocation; they become tensors when asked for
+        sizes = (e, e, e, n + 1, e, n + 1)
+        at, offsets = 0, []
+        for size in sizes:
+            offsets.append(at)
+            at += (max(size, 1) + 63) // 64 * 64
+        nbytes = lib.zp_csr_work_bytes(e, n)
+        graph.packed = torch.empty(at + (nbytes + 3) // 4, dtype=torch.int32, device=dev)
+        graph.where = dict(zip(_ARRAYS, zip(offsets, sizes)))
+        perm, src, dst, row_ptr, perm_src, row_ptr_src = graph.addresses()
         slots = _flag_slots.setdefault(dev.index, [])
         try:
             flags, done = slots.pop()
         except IndexError:
             flags, done = torch.empty(1, dtype=torch.int32, pin_memory=True), torch.cuda.Event()
             done.record(torch.cuda.current_stream(dev))        # gives the event its handle
-        _lib.run(dev, "zp_csr_build_checked", ei.data_ptr(), e, n, z.data_ptr(), n_elements,
-                 perm.data_ptr(), src.data_ptr(), dst.data_ptr(), row_ptr.data_ptr(),
-                 perm_src.data_ptr(), row_ptr_src.data_ptr(), flags.data_ptr(), done.cuda_event,
-                 work.data_ptr(), work.numel())
+        _lib.run(dev, "zp_csr_build_checked", ei.data_ptr(), e, n, z.data_ptr(), n_elements, perm, src,
+                 dst, row_ptr, perm_src, row_ptr_src, flags.data_ptr(), done.cuda_event,
+                 graph.packed.data_ptr() + 4 * at, nbytes)
 
         def check() -> None:
             done.synchronize()
@@ -161,8 +171,27 @@ class EdgeGraph:
             if bits & 2:
                 raise IndexError(f"atomic_numbers outside [0, {n_elements})")
 
-        return EdgeGraph(n, e, perm[:e], src[:e], dst[:e], row_ptr, perm_src[:e], row_ptr_src), check
+        return graph, check
 
+    def __getattr__(self, name):
+        # an array of a packed graph that is not a tensor yet
+        where = self.__dict__.get("where", {}).get(name)
+        if where is None:
+            raise AttributeError(name)
+        value = self.packed[where[0]:where[0] + where[1]]
+        setattr(self, name, value)
+        return value
+
+    def addresses(self) -> tuple:
+        """Device addresses of perm, src, dst, row_ptr, perm_src, row_ptr_src."""
+        packed = self.__dict__.get("packed")
+        if packed is None:
+            return tuple(getattr(self, name).data_ptr() for name in _ARRAYS)
+        base = packed.data_ptr()
+        return tuple(base + 4 * self.where[name][0] for name in _ARRAYS)
+
+
+_ARRAYS = ("perm", "src", "dst", "row_ptr", "perm_src", "row_ptr_src")
 
 #: Per device, page-locked words (and the events behind them) that the flags of a sort arrive in,
 #: reused; at most eight are kept, and a slot belongs to one call from its pop to its append.
