@@ -382,10 +382,10 @@ prep_weights_kernel(const __grid_constant__ ZpPrepList d, const __grid_constant_
 //   ZP_FIN_COLUMN  sum of `parts` partial rows: eight columns per tile, 32 threads per column take
 //                  every 32nd row, and their sums are added in order
 // Bound by the partials it reads.  A tile of the matrices has 256 groups of V neighbouring entries.
-template <int V>
+template <int V, bool folded>
 __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, float *__restrict__ dst,
                                                  int64_t stride, int rows, int cols, int parts, int ld,
-                                                 bool folded, int64_t tile) {
+                                                 int64_t tile) {
   const int kin = folded ? cols / 2 : cols, half = rows / 2;
   const int64_t idx = (tile * 256 + threadIdx.x) * V;
   if (idx >= (int64_t)rows * kin) return;
@@ -394,7 +394,7 @@ __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, fl
   const float *p = f + (size_t)row * ld + c;
   const float *q = f + (size_t)(upper ? half + row : row - half) * ld + kin + c;
   const float sign = upper ? 1.f : -1.f;
-  constexpr int kBatch = 8;
+  constexpr int kBatch = folded ? 4 : 8;           // loads of eight groups on their way at a time
   float acc[V], v[kBatch][V], u[kBatch][V];
 #pragma unroll
   for (int k = 0; k < V; ++k) acc[k] = 0.f;
@@ -406,7 +406,7 @@ __device__ __forceinline__ void finalize_entries(const float *__restrict__ f, fl
       to[0] = *from;
     }
   };
-  for (int s0 = 0; s0 < parts; s0 += kBatch) {     // a batch on its way at a time
+  for (int s0 = 0; s0 < parts; s0 += kBatch) {
 #pragma unroll
     for (int b = 0; b < kBatch; ++b)
       if (s0 + b < parts) {
@@ -435,9 +435,15 @@ finalize_kernel(const __grid_constant__ ZpFinalList d, const __grid_constant__ Z
     const int64_t stride = d.stride[b];
     const int cols = d.cols[b], parts = d.parts[b], kind = d.kind[b], tile = t - tiles.first[b];
     if (kind != ZP_FIN_COLUMN) {
-      const bool folded = kind == ZP_FIN_UNFOLD;
-      if (d.quads[b]) finalize_entries<4>(f, dst, stride, d.rows[b], cols, parts, d.ld[b], folded, tile);
-      else finalize_entries<1>(f, dst, stride, d.rows[b], cols, parts, d.ld[b], folded, tile);
+      const bool quads = d.quads[b];
+      const int rows = d.rows[b], ld = d.ld[b];
+      if (kind == ZP_FIN_UNFOLD) {
+        if (quads) finalize_entries<4, true>(f, dst, stride, rows, cols, parts, ld, tile);
+        else finalize_entries<1, true>(f, dst, stride, rows, cols, parts, ld, tile);
+      } else {
+        if (quads) finalize_entries<4, false>(f, dst, stride, rows, cols, parts, ld, tile);
+        else finalize_entries<1, false>(f, dst, stride, rows, cols, parts, ld, tile);
+      }
       continue;
     }
     const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3;
