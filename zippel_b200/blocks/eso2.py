@@ -677,12 +677,14 @@ class BlockFunction(torch.autograd.Function):
     of all of it (``zp_block_backward``): reference blocks/eso2_ref.py:317-349 and autograd through
     it.  ``block`` gives the configuration, ``params`` are its parameters in registration order
     without the readout; ``perm``: int32 positions of the graph's sorted edges in the per-edge arrays
-    (None: the graph's own).
+    (None: the graph's own).  Parameters none of which wants a gradient may come as one list: the
+    autograd machinery looks at every argument, which for thirty of them is as dear as three launches.
     fp32, first order only."""
 
     @staticmethod
     def forward(ctx, block, plan: Plan, graph: EdgeGraph, perm, atomic_numbers, shifts, cos_g, sin_g,
                 x_ready, pos, x_node, *params):
+        params = _listed(ctx, params)
         out, saved = _block(ctx, block, plan, graph, perm, atomic_numbers, shifts, cos_g, sin_g,
                             x_ready, pos, x_node, params)
         ctx.save_for_backward(*saved)
@@ -691,7 +693,8 @@ class BlockFunction(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
-        return (None,) * 9 + _block_vjp(ctx, ctx.saved_tensors, grad_out, ctx.needs_input_grad[9:])
+        want = _wanted(ctx, len(ctx.shapes))
+        return _returned(ctx, _block_vjp(ctx, ctx.saved_tensors, grad_out, want))
 
 
 class EnergyFunction(torch.autograd.Function):
@@ -702,6 +705,7 @@ class EnergyFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, block, plan: Plan, graph: EdgeGraph, perm, atomic_numbers, shifts, cos_g, sin_g,
                 x_ready, pos, x_node, *params):
+        params = _listed(ctx, params)
         out, saved = _block(ctx, block, plan, graph, perm, atomic_numbers, shifts, cos_g, sin_g,
                             x_ready, pos, x_node, params[:-4])
         head = [_as_f32(t) for t in params[-4:]]
@@ -714,14 +718,28 @@ class EnergyFunction(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_e):
         out, *head, work = ctx.saved_tensors[-6:]
-        want, plan = ctx.needs_input_grad[9:], ctx.native[0]
+        want, plan = _wanted(ctx, len(ctx.shapes) + 4), ctx.native[0]
         g = torch.empty_like(out)
         ghead = _readout_vjp(plan, out, head, grad_e, g, work, any(want[-4:]))
         ghead = [t if w else None for t, w in zip(ghead, want[-4:])]
         grads = ((None,) * len(want[:-4]) if not any(want[:-4]) else
                  _block_vjp(ctx, ctx.saved_tensors[:-6], g, want[:-4]))
-        return (None,) * 9 + grads + tuple(t if t is None or t.dtype == dt else t.to(dt)
-                                           for t, dt in zip(ghead, ctx.head_dtypes))
+        return _returned(ctx, grads + tuple(t if t is None or t.dtype == dt else t.to(dt)
+                                            for t, dt in zip(ghead, ctx.head_dtypes)))
+
+
+def _listed(ctx, params):
+    ctx.listed = len(params) == 1 and isinstance(params[0], list)
+    return params[0] if ctx.listed else params
+
+
+def _wanted(ctx, n_params: int) -> tuple:
+    want = ctx.needs_input_grad[9:]
+    return (*want[:2], *(False,) * n_params) if ctx.listed else want
+
+
+def _returned(ctx, grads: tuple) -> tuple:
+    return (None,) * 9 + ((*grads[:2], None) if ctx.listed else grads)
 
 
 def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin_g, x_ready, pos,
@@ -955,13 +973,15 @@ class ESO2Block(nn.Module):
             graph, check = self._sorted_edges(edge_index, atomic_numbers)
         plan = self.plan(pos.device)
         energy = function is EnergyFunction
+        params = self._all_params() if energy else self._block_params()
+        if not (torch.is_grad_enabled() and any([p.requires_grad for p in params])):
+            params = [params]
         try:
             out = None
             if _surely_fits(plan, graph.n_edges):
                 try:
                     out = function.apply(self, plan, graph, None, atomic_numbers, shifts,
-                                         cos_gamma_k, sin_gamma_k, x_ready, pos, x_node,
-                                         *(self._all_params() if energy else self._block_params()))
+                                         cos_gamma_k, sin_gamma_k, x_ready, pos, x_node, *params)
                 except torch.cuda.OutOfMemoryError:
                     pass
             if out is None:
