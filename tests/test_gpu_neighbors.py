@@ -122,3 +122,18 @@ def test_selection_at_its_edges(atoms, cap, jitter):
     from oracle import neighbors_oracle as no
     for a, b in zip(run(pos, 20.0, 6.0, cap), no.neighbor_list(pos, 20.0, 6.0, cap)):
         assert a.shape == b.shape and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("outside", [False, True])
+@pytest.mark.parametrize("atoms", [130, 192, 193, 194])
+@pytest.mark.parametrize("cap", [None, 30, 128, 129, 191, 192, 193])
+def test_long_lists(atoms, cap, outside):
+    """Around the 192 hits that are selected in registers and the 128 edges that are kept between the
+    passes, the atoms inside the box and outside it."""
+    g = np.random.default_rng(5)
+    pos = 9.0 + 1.7 * g.random((atoms, 3))
+    if outside:
+        pos += 20.0 * g.integers(-2, 3, pos.shape)
+    from oracle import neighbors_oracle as no
+    for a, b in zip(run(pos, 20.0, 6.0, cap), no.neighbor_list(pos, 20.0, 6.0, cap)):
+        assert a.shape == b.shape and np.array_equal(a, b)

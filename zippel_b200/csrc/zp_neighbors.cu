@@ -19,11 +19,13 @@
 // unwrapped coordinate gives both the wrapped cell and the periodic image, so every
 // (source, image) pair is visited at most once.  The atoms are copied in cell order with their own
 // image numbers, so the walk reads them with whole-line loads and divides nothing, and the
-// columns of a walk are laid end to end so that no lane waits at a column's end.  Pass 1 counts
-// (up to the cap), a scan gives row_ptr, pass 2 collects the hits and, when the cap binds, selects
-// the nearest: up to 128 hits by closing in on a distance that parts off exactly `cap` of them
-// (ranking all when equal distances stand in the way), more by a bitonic sort on (d2, src, image) in
-// shared memory.  The survivors are placed by counting the smaller (src, image) keys.
+// columns of a walk are laid end to end so that no lane waits at a column's end.  Pass 1 collects the
+// hits of an atom and, when the cap binds, selects the nearest by closing in on a distance that
+// parts off exactly `cap` of them (ranking all when equal distances stand in the way); the survivors
+// are placed by counting the smaller (src, image) keys and kept in the workspace.  A scan of their
+// numbers gives row_ptr, and pass 2 writes the edges out.  Atoms of more than 192 hits are only counted
+// in pass 1 (up to the cap); pass 2 walks them again and selects by a bitonic sort on (d2, src, image)
+// in shared memory.
 #include <algorithm>
 #include <cmath>
 
@@ -34,16 +36,20 @@ namespace {
 
 constexpr int kWarpsPerBlock = 4;
 constexpr int kHitCap = ZP_NEIGHBORS_MAX_HITS;     // hits held per destination in shared memory
-constexpr int kFewHits = 128;                      // ... in registers, four per lane
+constexpr int kFewHits = 192;                      // ... in registers, six per lane
+constexpr int kKept = 128;                         // edges per destination kept from pass 1 to 2
 constexpr int kScanBlock = 1024;
 
 struct Grid {
-  double box, cell, cutoff2;
+  double box, per_cell, cutoff2;   // per_cell: cells per unit of length
   int nc;          // cells per dimension
   int w;           // search half-width in cells
   int reach;       // largest |image| component that can occur
   float reach2;    // (cutoff / cell)^2 and a margin for working in fp32
 };
+
+// words of the workspace's head: error bits, whether an atom lies outside the box, crowded atoms
+enum { kFlagBits = 0, kUnwrapped = 1, kCrowdedList = 3 };
 
 struct Hit {
   double d2;
@@ -63,13 +69,17 @@ __device__ __forceinline__ int clamp_cell(double p, const Grid &g) {
   return c < 0 ? 0 : (c >= g.nc ? g.nc - 1 : c);
 }
 __device__ __forceinline__ int cell_coord(double p, const Grid &g) {
-  return clamp_cell((p - floor(p / g.box) * g.box) / g.cell, g);
+  return clamp_cell((p - floor(p / g.box) * g.box) * g.per_cell, g);
 }
 
 __device__ __forceinline__ int floor_div(int a, int n) {
   int q = a / n;
   if ((a % n) < 0) --q;
   return q;
+}
+// image that the unwrapped cell coordinate a, at most w outside [0, nc), lies in
+__device__ __forceinline__ int cell_image(int a, const Grid &g) {
+  return g.w > g.nc ? floor_div(a, g.nc) : a < 0 ? -1 : a >= g.nc;
 }
 
 // Image code.  The shift of a hit is (o_src - o_dst - k) * box with k the image found in wrapped
@@ -93,7 +103,9 @@ __global__ void cell_count_kernel(int64_t N, const double *__restrict__ pos, Gri
     atomicOr(flags, 1);                               // not finite, or absurdly far from the box
   const int c = (cell_coord(x, g) * g.nc + cell_coord(y, g)) * g.nc + cell_coord(z, g);
   atom_cell[i] = c;
-  own[i] = make_int4(own_image(x, g), own_image(y, g), own_image(z, g), (int)i);
+  const int4 mine = make_int4(own_image(x, g), own_image(y, g), own_image(z, g), (int)i);
+  own[i] = mine;
+  if (mine.x | mine.y | mine.z) flags[kUnwrapped] = 1;
   atomicAdd(&cell_count[c], 1);
 }
 
@@ -117,8 +129,8 @@ __global__ void cell_fill_kernel(int64_t N, const double *__restrict__ pos, Grid
   out.who[at] = own[i];
 }
 
-// exclusive scan of n ints (n + 1 outputs, the last is the total): block scans, serial scan of
-// the block totals, add back
+// exclusive scan of n ints (n + 1 outputs, the last is the total): block scans, then each
+// block adds the totals of those before it
 __global__ void scan_block_kernel(int64_t n, const int32_t *__restrict__ in, int32_t *out,
                                   int32_t *block_sums) {
   zp_after_previous();
@@ -136,21 +148,19 @@ __global__ void scan_block_kernel(int64_t n, const int32_t *__restrict__ in, int
   if (i <= n) out[i] = s[threadIdx.x] - mine;
   if (threadIdx.x == kScanBlock - 1) block_sums[blockIdx.x] = s[threadIdx.x];
 }
-__global__ void scan_sums_kernel(int64_t nb, int32_t *block_sums) {
+__global__ void __launch_bounds__(kScanBlock)
+scan_add_kernel(int64_t n, int32_t *out, const int32_t *__restrict__ block_sums) {
   zp_after_previous();
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    int32_t run = 0;
-    for (int64_t b = 0; b < nb; ++b) {
-      const int32_t v = block_sums[b];
-      block_sums[b] = run;
-      run += v;
-    }
-  }
-}
-__global__ void scan_add_kernel(int64_t n, int32_t *out, const int32_t *__restrict__ block_sums) {
-  zp_after_previous();
+  __shared__ int32_t before;             // totals of the blocks before this one
+  if (threadIdx.x == 0) before = 0;
+  __syncthreads();
+  int32_t sum = 0;
+  for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanBlock) sum += block_sums[b];
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (threadIdx.x % 32 == 0 && sum) atomicAdd(&before, sum);
+  __syncthreads();
   const int64_t i = (int64_t)blockIdx.x * kScanBlock + threadIdx.x;
-  if (i <= n) out[i] += block_sums[blockIdx.x];
+  if (i <= n) out[i] += before;
 }
 
 int exclusive_scan(int64_t n, const int32_t *in, int32_t *out, int32_t *block_sums,
@@ -158,29 +168,29 @@ int exclusive_scan(int64_t n, const int32_t *in, int32_t *out, int32_t *block_su
   const int64_t nb = zp_ceil_div(n + 1, kScanBlock);
   zp_launch(scan_block_kernel, (unsigned)nb, kScanBlock, 0, st, n, in, out, block_sums);
   ZP_LAUNCH_CHECK("scan_block_kernel");
-  zp_launch(scan_sums_kernel, 1, 32, 0, st, nb, block_sums);
-  ZP_LAUNCH_CHECK("scan_sums_kernel");
   zp_launch(scan_add_kernel, (unsigned)nb, kScanBlock, 0, st, n, out, block_sums);
   ZP_LAUNCH_CHECK("scan_add_kernel");
   return ZP_OK;
 }
 
-// Calls f(hit, src, -kx, -ky, -kz, d2) on all 32 lanes together for every batch of candidate
+// Calls f(hit, src, image code, d2) on all 32 lanes together for every batch of candidate
 // (source, image) pairs around destination j; `hit` marks the lanes whose candidate lies within
-// the cutoff, k is its image in wrapped coordinates.  The walk goes on while f returns true (the
-// same on all lanes).
+// the cutoff.  The walk goes on while f returns true (the same on all lanes).  Bound by instruction
+// issue: what hangs on images alone is formed once per column, and the conversions and products
+// of a shift are left out where it is zero (in a large cell, for most atoms).
+constexpr int kNoImage = 512 | 512 << 10 | 512 << 20;
 template <typename F>
 __device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__restrict__ cell_start,
                                              const Sorted &atoms, int64_t at, int lane, F &&f) {
   const double xj = atoms.x[at], yj = atoms.y[at], zj = atoms.z[at];
   const int4 own = atoms.who[at];
   // cell, and where in it (in cells)
-  const double wx = (xj - own.x * g.box) / g.cell, wy = (yj - own.y * g.box) / g.cell,
-               wz = (zj - own.z * g.box) / g.cell;
+  const double wx = (xj - own.x * g.box) * g.per_cell, wy = (yj - own.y * g.box) * g.per_cell,
+               wz = (zj - own.z * g.box) * g.per_cell;
   const int cx = clamp_cell(wx, g), cy = clamp_cell(wy, g), cz = clamp_cell(wz, g);
   const float fx = (float)(wx - cx), fy = (float)(wy - cy), fz = (float)(wz - cz);
   const int side = 2 * g.w + 1, columns = side * side;
-  const int kz1 = floor_div(cz + g.w, g.nc);
+  const int kz1 = cell_image(cz + g.w, g);
   for (int q0 = 0; q0 < columns; q0 += 32) {
     // a lane per column of cells along z, cut to what the cutoff can reach
     const int q = q0 + lane;
@@ -191,12 +201,13 @@ __device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__res
     const bool in = q < columns && r2 > 0.f;
     const float r = in ? sqrtf(r2) : 0.f;
     const int u0 = max(cz - g.w, cz + (int)floorf(fz - r)), u1 = min(cz + g.w, cz + (int)floorf(fz + r));
-    const int kx = floor_div(cx + ox, g.nc), ky = floor_div(cy + oy, g.nc);
+    const int kx = cell_image(cx + ox, g), ky = cell_image(cy + oy, g);
     const int column = ((cx + ox - kx * g.nc) * g.nc + (cy + oy - ky * g.nc)) * g.nc;
-    for (int kz = floor_div(cz - g.w, g.nc); kz <= kz1; ++kz) {
+    for (int kz = cell_image(cz - g.w, g); kz <= kz1; ++kz) {
       const int z0 = max(u0 - kz * g.nc, 0), z1 = min(u1 - kz * g.nc, g.nc - 1);
       int off = 0, len = 0;
-      const int image = (kx + 512) | (ky + 512) << 10 | (kz + 512) << 20;
+      const int image = (512 - kx) | (512 - ky) << 10 | (512 - kz) << 20;
+      const unsigned image_place = image_code(-kx, -ky, -kz, g.reach);
       if (in && z0 <= z1) {
         off = cell_start[column + z0];
         len = cell_start[column + z1 + 1] - off;
@@ -219,49 +230,34 @@ __device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__res
         }
         const int a = __shfl_sync(0xffffffffu, off, cell) + t;
         const int im = __shfl_sync(0xffffffffu, image, cell);
+        const unsigned code = __shfl_sync(0xffffffffu, image_place, cell);
         bool hit = false;
-        int i = 0, nkx = 0, nky = 0, nkz = 0;
+        int i = 0;
         double d2 = 0.0;
         if (t < total) {
           const int4 who = atoms.who[a];
           i = who.w;
-          nkx = 512 - (im & 1023);
-          nky = 512 - (im >> 10 & 1023);
-          nkz = 512 - (im >> 20 & 1023);
           // the source's wrapped copy sits k boxes away in wrapped coordinates:
           // pos[j] - (pos[i] - o_i box + k box) stays as (pos[j] - pos[i]) + (o_i - o_j - k) box
           // once the destination's own offset o_j is taken out of the search origin
-          const int mx = who.x - own.x + nkx, my = who.y - own.y + nky, mz = who.z - own.z + nkz;
-          const double dx = __dadd_rn(__dsub_rn(xj, atoms.x[a]), __dmul_rn((double)mx, g.box));
-          const double dy = __dadd_rn(__dsub_rn(yj, atoms.y[a]), __dmul_rn((double)my, g.box));
-          const double dz = __dadd_rn(__dsub_rn(zj, atoms.z[a]), __dmul_rn((double)mz, g.box));
+          double dx = __dsub_rn(xj, atoms.x[a]), dy = __dsub_rn(yj, atoms.y[a]),
+                 dz = __dsub_rn(zj, atoms.z[a]);
+          const bool shifted = im != kNoImage || who.x != own.x || who.y != own.y || who.z != own.z;
+          bool self = i == own.w;
+          if (shifted) {
+            const int mx = who.x - own.x + (im & 1023) - 512, my = who.y - own.y + (im >> 10 & 1023) - 512,
+                      mz = who.z - own.z + (im >> 20 & 1023) - 512;
+            dx = __dadd_rn(dx, __dmul_rn((double)mx, g.box));
+            dy = __dadd_rn(dy, __dmul_rn((double)my, g.box));
+            dz = __dadd_rn(dz, __dmul_rn((double)mz, g.box));
+            self = self && mx == 0 && my == 0 && mz == 0;
+          }
           d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-          hit = d2 < g.cutoff2 && !(i == own.w && mx == 0 && my == 0 && mz == 0);
+          hit = d2 < g.cutoff2 && !self;
         }
-        if (!f(hit, i, nkx, nky, nkz, d2)) return;
+        if (!f(hit, i, code, d2)) return;
       }
     }
-  }
-}
-
-__global__ void __launch_bounds__(32 * kWarpsPerBlock)
-count_kernel(int64_t N, Grid g,
-             const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
-             int32_t *__restrict__ counts, int32_t *flags) {
-  zp_after_previous();
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int64_t at = (int64_t)blockIdx.x * kWarpsPerBlock + warp;
-  if (at >= N) return;
-  const int64_t j = atoms.who[at].w;           // in cell order: neighbours read the same cells
-  int n = 0;
-  for_each_hit(g, cell_start, atoms, at, lane,
-               [&](bool hit, int, int, int, int, double) {
-                 n += __popc(__ballot_sync(0xffffffffu, hit));
-                 return cap <= 0 || n < cap;             // past the cap the count is known
-               });
-  if (lane == 0) {
-    if (cap <= 0 && n > kHitCap) atomicOr(flags, 2);       // uncapped list too long for pass 2
-    counts[j] = cap > 0 && n > cap ? cap : n;
   }
 }
 
@@ -289,124 +285,169 @@ __device__ __forceinline__ int pow2_at_least(int n) {
   return p;
 }
 
-// Writes the edges of destination j: survivor `tie` at place `rank` of its list.
+// Writes edge `place` of destination j, whose source and image are in `tie`.
 struct Writer {
   const int4 *own;
   const Grid &g;
+  bool unwrapped;          // atoms have images of their own
   int64_t E, j, base;
   int64_t *edge_index;
   double *shifts;
-  __device__ __forceinline__ void put(unsigned long long tie, int rank) const {
-    const unsigned s = 2u * g.reach + 1u;
+  __device__ __forceinline__ void put_pair(unsigned long long tie, int place) const {
+    edge_index[base + place] = (int64_t)(tie >> 32);
+    edge_index[E + base + place] = j;
+  }
+  // component `v % 3` of the shift of edge `v / 3`
+  __device__ __forceinline__ void put_shift(unsigned long long tie, int v) const {
     const unsigned code = (unsigned)(tie & 0xffffffffu);
-    const int64_t i = (int64_t)(tie >> 32);
-    const int nkz = (int)(code % s) - g.reach, nky = (int)((code / s) % s) - g.reach,
-              nkx = (int)(code / (s * s)) - g.reach;
-    const int4 a = own[i], b = own[j];
-    edge_index[base + rank] = i;
-    edge_index[E + base + rank] = j;
-    shifts[3 * (base + rank)] = (double)(a.x - b.x + nkx) * g.box;
-    shifts[3 * (base + rank) + 1] = (double)(a.y - b.y + nky) * g.box;
-    shifts[3 * (base + rank) + 2] = (double)(a.z - b.z + nkz) * g.box;
+    double shift = 0.0;
+    if (unwrapped || code != image_code(0, 0, 0, g.reach)) {
+      const unsigned s = 2u * g.reach + 1u, axis = v % 3;
+      int m = (int)((axis == 0 ? code / (s * s) : axis == 1 ? code / s : code) % s) - g.reach;
+      if (unwrapped) {
+        const int *image = reinterpret_cast<const int *>(own);
+        m += image[4 * (int64_t)(tie >> 32) + axis] - image[4 * j + axis];
+      }
+      shift = (double)m * g.box;
+    }
+    shifts[3 * base + v] = shift;
   }
 };
 
-// Destinations with at most kFewHits hits, compacted in 2 KB of shared memory per warp so that an
-// SM holds its full count of warps; the others go on the list `crowded`.  Bound by instruction issue
-// (a third of it the walk); 100 000 atoms, 90 hits, cap 30: 240 us, where two bitonic sorts in 64 KB
-// of shared memory per four warps took 3400.
-constexpr int kFillWarps = 8;
-__global__ void __launch_bounds__(32 * kFillWarps)
-fill_few_kernel(int64_t N, const int4 *__restrict__ own, Grid g,
-                const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
-                const int32_t *__restrict__ row_ptr, int64_t E, int64_t *__restrict__ edge_index,
-                double *__restrict__ shifts, int32_t *flags, int32_t *__restrict__ crowded) {
+// Moves the ties of the `cap` nearest of the n <= 32 R hits to the front, n > cap > 0.
+template <int R>
+__device__ __forceinline__ void keep_nearest(Hit *h, int n, int cap, float cutoff2, int lane) {
+      float near[R];                // rounding to fp32 keeps the order, or makes equals
+#pragma unroll
+      for (int k = 0; k < R; ++k) near[k] = lane + 32 * k < n ? (float)h[lane + 32 * k].d2 : INFINITY;
+      // close in on a distance that exactly `cap` hits do not exceed: by interpolation and by halves
+      float lo = 0.f, hi = cutoff2;
+      int below_lo = 0, below_hi = n;
+      unsigned alive[R];            // survivors, a bit per lane
+      bool found = false;
+      for (int step = 0; step < 32 && !found; ++step) {
+        const float part = step & 1 ? 0.5f : (cap - below_lo) / (float)(below_hi - below_lo);
+        const float mid = lo + (hi - lo) * part;
+        int below = 0;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+          alive[k] = __ballot_sync(0xffffffffu, near[k] <= mid);
+          below += __popc(alive[k]);
+        }
+        found = below == cap;
+        if (below < cap) {
+          lo = mid;
+          below_lo = below;
+        } else {
+          hi = mid;
+          below_hi = below;
+        }
+      }
+      if (!found) {                 // equal distances at the cap: rank by (d2, src, image)
+        for (int k = 0; k < R; ++k) {
+          const int own_t = lane + 32 * k;
+          const Hit mine = h[own_t < n ? own_t : 0];
+          int rank = 0;
+          for (int t = 0; t < n; ++t) rank += hit_less(h[t], mine);
+          alive[k] = __ballot_sync(0xffffffffu, own_t < n && rank < cap);
+        }
+      }
+      // survivors to the front
+      unsigned long long tie[R];
+#pragma unroll
+      for (int k = 0; k < R; ++k) tie[k] = h[lane + 32 * k].tie;
+      __syncwarp();
+      int slot = 0;
+#pragma unroll
+      for (int k = 0; k < R; ++k) {
+        if (alive[k] >> lane & 1) h[slot + __popc(alive[k] & ((1u << lane) - 1u))].tie = tie[k];
+        slot += __popc(alive[k]);
+      }
+      __syncwarp();
+}
+
+// Pass 1, a warp per destination, its hits compacted in 3 KB of shared memory so that an SM holds its
+// full count of warps: the survivors of destination j go to kept[j][0 ...] in their final order.  One
+// with more than kFewHits hits or kKept survivors goes on the list `crowded` instead, its row of
+// `kept` marked: 192 hits because a warp walking again alone costs as much as a third of all others
+// (57 us for the few atoms in 100 000 that have more than 128 where the mean is 90).  Bound by
+// instruction issue: 186 us for 100 000 atoms, 90 hits each, cap 30, where a count of 90 us came before 235 us of this.
+constexpr int kSelectWarps = 8;
+constexpr unsigned long long kCrowded = ~0ull;
+__global__ void __launch_bounds__(32 * kSelectWarps)
+select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
+              int32_t *__restrict__ counts, unsigned long long *__restrict__ kept, int32_t *flags,
+              int32_t *__restrict__ crowded) {
   zp_after_previous();
-  __shared__ Hit hits[kFillWarps][kFewHits];
+  __shared__ Hit hits[kSelectWarps][kFewHits];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int64_t at = (int64_t)blockIdx.x * kFillWarps + warp;
+  const int64_t at = (int64_t)blockIdx.x * kSelectWarps + warp;
   if (at >= N) return;
-  const int64_t j = atoms.who[at].w;
+  const int64_t j = atoms.who[at].w;           // in cell order: neighbours read the same cells
   Hit *h = hits[warp];
   int n = 0;                      // hits seen (warp-uniform)
   for_each_hit(g, cell_start, atoms, at, lane,
-               [&](bool hit, int i, int nkx, int nky, int nkz, double d2) {
+               [&](bool hit, int i, unsigned code, double d2) {
                  const unsigned m = __ballot_sync(0xffffffffu, hit);
                  const int slot = n + __popc(m & ((1u << lane) - 1u));
                  if (hit && slot < kFewHits) {
                    h[slot].d2 = d2;
-                   h[slot].tie = ((unsigned long long)(unsigned)i << 32) | image_code(nkx, nky, nkz, g.reach);
+                   h[slot].tie = ((unsigned long long)(unsigned)i << 32) | code;
                  }
                  n += __popc(m);
-                 return n <= kFewHits;
+                 return n <= kFewHits || cap <= 0 || n < cap;    // past both the count is known
                });
-  if (n > kFewHits) {             // left to fill_many_kernel
-    if (lane == 0) crowded[1 + atomicAdd(&crowded[0], 1)] = (int32_t)at;
+  kept += j * kKept;
+  if (n > kFewHits || (n > kKept && (cap <= 0 || cap > kKept))) {             // left to fill_many_kernel
+    if (lane == 0) {
+      if (cap <= 0 && n > kHitCap) atomicOr(flags, 2);     // uncapped list too long for it
+      counts[j] = cap > 0 && n > cap ? cap : n;
+      kept[0] = kCrowded;
+      crowded[1 + atomicAdd(&crowded[0], 1)] = (int32_t)at;
+    }
     return;
   }
   __syncwarp();
   if (cap > 0 && n > cap) {
-    constexpr int R = kFewHits / 32;
-    float near[R];                // rounding to fp32 keeps the order, or makes equals
-#pragma unroll
-    for (int k = 0; k < R; ++k) near[k] = lane + 32 * k < n ? (float)h[lane + 32 * k].d2 : INFINITY;
-    // close in on a distance that exactly `cap` hits do not exceed: by interpolation and by halves
-    float lo = 0.f, hi = (float)g.cutoff2;
-    int below_lo = 0, below_hi = n;
-    unsigned alive[R];            // survivors, a bit per lane
-    bool found = false;
-    for (int step = 0; step < 32 && !found; ++step) {
-      const float part = step & 1 ? 0.5f : (cap - below_lo) / (float)(below_hi - below_lo);
-      const float mid = lo + (hi - lo) * part;
-      int below = 0;
-#pragma unroll
-      for (int k = 0; k < R; ++k) {
-        alive[k] = __ballot_sync(0xffffffffu, near[k] <= mid);
-        below += __popc(alive[k]);
-      }
-      found = below == cap;
-      if (below < cap) {
-        lo = mid;
-        below_lo = below;
-      } else {
-        hi = mid;
-        below_hi = below;
-      }
-    }
-    if (!found) {                 // equal distances at the cap: rank by (d2, src, image)
-      for (int k = 0; k < R; ++k) {
-        const int own_t = lane + 32 * k;
-        const Hit mine = h[own_t < n ? own_t : 0];
-        int rank = 0;
-        for (int t = 0; t < n; ++t) rank += hit_less(h[t], mine);
-        alive[k] = __ballot_sync(0xffffffffu, own_t < n && rank < cap);
-      }
-    }
-    // survivors to the front
-    unsigned long long tie[R];
-#pragma unroll
-    for (int k = 0; k < R; ++k) tie[k] = h[lane + 32 * k].tie;
-    __syncwarp();
-    int slot = 0;
-#pragma unroll
-    for (int k = 0; k < R; ++k) {
-      if (alive[k] >> lane & 1) h[slot + __popc(alive[k] & ((1u << lane) - 1u))].tie = tie[k];
-      slot += __popc(alive[k]);
-    }
-    __syncwarp();
+    if (n <= 128)
+      keep_nearest<4>(h, n, cap, (float)g.cutoff2, lane);
+    else
+      keep_nearest<kFewHits / 32>(h, n, cap, (float)g.cutoff2, lane);
     n = cap;
   }
-  const int64_t base = row_ptr[j];
-  if (lane == 0 && row_ptr[j + 1] - base != n) atomicOr(flags, 4);     // passes disagree
-  const Writer out{own, g, E, j, base, edge_index, shifts};
+  if (lane == 0) counts[j] = n;
   // place of a survivor = number of survivors with a smaller (src, image)
   for (int t = lane; t < n; t += 32) {
     const unsigned long long mine = h[t].tie;
     int rank = 0;
 #pragma unroll 4
     for (int q = 0; q < n; ++q) rank += h[q].tie < mine;
-    out.put(mine, rank);
+    kept[rank] = mine;
   }
+}
+
+// Pass 2, a warp per destination: the survivors of pass 1 to their edges.  Bound by the 40 bytes that an
+// edge is written in; a lane takes one component of a shift, so that stores are whole lines, and an edge
+// inside the box needs neither a division nor its atoms' images.  Two passes that each walked the cells,
+// and a read of flags behind them, took 760 us with the edge sort that follows them, this 440 (100 000
+// atoms, 3 M edges).
+constexpr int kFillWarps = 8;
+__global__ void __launch_bounds__(32 * kFillWarps)
+fill_kernel(int64_t N, const int4 *__restrict__ own, Grid g,
+            const unsigned long long *__restrict__ kept, const int32_t *__restrict__ row_ptr,
+            int64_t E, int64_t *__restrict__ edge_index, double *__restrict__ shifts,
+            const int32_t *__restrict__ flags) {
+  zp_after_previous();
+  const int lane = threadIdx.x % 32;
+  const int64_t j = (int64_t)blockIdx.x * kFillWarps + threadIdx.x / 32;
+  if (j >= N) return;
+  const int64_t base = row_ptr[j];
+  const int n = (int)(row_ptr[j + 1] - base);
+  kept += j * kKept;
+  if (n <= 0 || kept[0] == kCrowded) return;
+  const Writer out{own, g, flags[kUnwrapped] != 0, E, j, base, edge_index, shifts};
+  for (int t = lane; t < n; t += 32) out.put_pair(kept[t], t);
+  for (int v = lane; v < 3 * n; v += 32) out.put_shift(kept[v / 3], v);
 }
 
 // The destinations listed in `crowded` (more than kFewHits hits).
@@ -425,7 +466,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ o
     int n = 0;                      // hits held (warp-uniform)
     bool overflow = false;
     for_each_hit(g, cell_start, atoms, at, lane,
-                 [&](bool hit, int i, int nkx, int nky, int nkz, double d2) {
+                 [&](bool hit, int i, unsigned code, double d2) {
                    const unsigned m = __ballot_sync(0xffffffffu, hit);
                    const int add = __popc(m);
                    if (n + add > kHitCap) {
@@ -442,8 +483,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ o
                    if (hit && !overflow) {
                      const int slot = n + __popc(m & ((1u << lane) - 1u));
                      h[slot].d2 = d2;
-                     h[slot].tie = ((unsigned long long)(unsigned)i << 32) |
-                                   image_code(nkx, nky, nkz, g.reach);
+                     h[slot].tie = ((unsigned long long)(unsigned)i << 32) | code;
                    }
                    if (!overflow) n += add;
                    __syncwarp();
@@ -468,9 +508,13 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ o
       warp_bitonic(h, n2, lane, [](const Hit &a, const Hit &b) { return a.tie < b.tie; });
     }
     const int64_t base = row_ptr[j];
-    if (lane == 0 && row_ptr[j + 1] - base != n) atomicOr(flags, 4);     // passes disagree
-    const Writer out{own, g, E, j, base, edge_index, shifts};
-    for (int t = lane; t < n; t += 32) out.put(h[t].tie, t);
+    if (row_ptr[j + 1] - base != n) {          // passes disagree: nothing is written past the row
+      if (lane == 0) atomicOr(flags, 4);
+      n = min(n, (int)(row_ptr[j + 1] - base));
+    }
+    const Writer out{own, g, flags[kUnwrapped] != 0, E, j, base, edge_index, shifts};
+    for (int t = lane; t < n; t += 32) out.put_pair(h[t].tie, t);
+    for (int v = lane; v < 3 * n; v += 32) out.put_shift(h[v / 3].tie, v);
     __syncwarp();
   }
 }
@@ -479,6 +523,7 @@ struct NbWork {
   int32_t *flags, *cell_count, *cell_start, *cell_cursor, *atom_cell, *counts, *crowded,
       *block_sums;
   int4 *own;       // own image and index of each atom
+  unsigned long long *kept;     // [N][kKept] survivors of pass 1
   Sorted atoms;
   size_t bytes;
 };
@@ -497,10 +542,11 @@ int make_grid(int64_t N, double box, double cutoff, Grid *g) {
   if (nc > 256) nc = 256;
   g->box = box;
   g->nc = nc;
-  g->cell = box / nc;
+  const double cell = box / nc;
+  g->per_cell = nc / box;
   g->cutoff2 = cutoff * cutoff;
-  g->reach2 = (float)(1.0001 * (cutoff / g->cell) * (cutoff / g->cell));
-  g->w = (int)std::ceil(wide / g->cell);
+  g->reach2 = (float)(1.0001 * (cutoff / cell) * (cutoff / cell));
+  g->w = (int)std::ceil(wide / cell);
   if (g->w < 1) g->w = 1;
   g->reach = (int)std::ceil(cutoff / box);
   if (g->reach < 1) g->reach = 1;
@@ -519,7 +565,7 @@ NbWork carve_nb(int64_t N, const Grid &g, void *base) {
   };
   const size_t cells = (size_t)g.nc * g.nc * g.nc;
   w.flags = take((size_t)N + 4);
-  w.crowded = w.flags + 3;                 // how many, then which
+  w.crowded = w.flags + kCrowdedList;      // how many, then which
   w.cell_count = take(cells + 1);
   w.cell_cursor = take(cells + 1);
   w.cell_start = take(cells + 1);
@@ -529,6 +575,7 @@ NbWork carve_nb(int64_t N, const Grid &g, void *base) {
   w.atoms.y = reinterpret_cast<double *>(take((size_t)2 * N));
   w.atoms.z = reinterpret_cast<double *>(take((size_t)2 * N));
   w.atoms.who = reinterpret_cast<int4 *>(take((size_t)4 * N));
+  w.kept = reinterpret_cast<unsigned long long *>(take((size_t)2 * kKept * N));
   w.counts = take((size_t)N + 1);
   w.block_sums = take((size_t)zp_ceil_div((int64_t)std::max<size_t>(cells, (size_t)N) + 2, kScanBlock) + 1);
   w.bytes = off;
@@ -570,9 +617,9 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
     zp_launch(cell_fill_kernel, (unsigned)zp_ceil_div(N, 256), 256, 0, st, N, pos, g, w.atom_cell,
               w.own, w.cell_start, w.cell_cursor, w.atoms);
     ZP_LAUNCH_CHECK("cell_fill_kernel");
-    zp_launch(count_kernel, (unsigned)zp_ceil_div(N, kWarpsPerBlock), 32 * kWarpsPerBlock, 0, st, N, g,
-              w.cell_start, w.atoms, max_neighbors, w.counts, w.flags);
-    ZP_LAUNCH_CHECK("count_kernel");
+    zp_launch(select_kernel, (unsigned)zp_ceil_div(N, kSelectWarps), 32 * kSelectWarps, 0, st, N, g,
+              w.cell_start, w.atoms, max_neighbors, w.counts, w.kept, w.flags, w.crowded);
+    ZP_LAUNCH_CHECK("select_kernel");
   }
   if ((rc = exclusive_scan(N, w.counts, row_ptr, w.block_sums, st))) return rc;
   ZP_CUDA(cudaMemcpyAsync(flags_out, w.flags, sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
@@ -592,16 +639,14 @@ int zp_neighbors_fill(const double *pos, int64_t N, double box, double cutoff, i
   const NbWork w = carve_nb(N, g, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  ZP_CUDA(cudaMemsetAsync(w.crowded, 0, sizeof(int32_t), st));
   if (N > 0) {
-    zp_launch(fill_few_kernel, (unsigned)zp_ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st, N, w.own,
-              g, w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags,
-              w.crowded);
-    ZP_LAUNCH_CHECK("fill_few_kernel");
+    zp_launch(fill_kernel, (unsigned)zp_ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st, N, w.own, g,
+              w.kept, row_ptr, E, edge_index, shifts, w.flags);
+    ZP_LAUNCH_CHECK("fill_kernel");
     const size_t smem = sizeof(Hit) * kHitCap * kWarpsPerBlock;
     static ZpSmemOptIn opt_in;
     if (int rc_ = zp_ensure_smem(fill_many_kernel, smem, opt_in)) return rc_;
-    const unsigned blocks = (unsigned)std::min<int64_t>(zp_ceil_div(N, kWarpsPerBlock), 148 * 3);
+    const unsigned blocks = (unsigned)std::min<int64_t>(zp_ceil_div(N, kWarpsPerBlock), 148);
     zp_launch(fill_many_kernel, blocks, 32 * kWarpsPerBlock, smem, st, w.crowded, w.own, g,
               w.cell_start, w.atoms, max_neighbors, row_ptr, E, edge_index, shifts, w.flags);
     ZP_LAUNCH_CHECK("fill_many_kernel");

@@ -266,7 +266,8 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
     ``pos``: CUDA tensor [N, 3] (computed in float64).  Returns (edge_index [2, E] int64,
     shifts [E, 3] float64, row_ptr [N + 1] int32) in (dst, src, shift) order, which is already the
     destination-sorted form the kernels consume.  One host read (edge count and flags) in between
-    the two passes, one of the flags at the end."""
+    the two passes; the second one only writes out what the first has selected or counted, so what
+    the caller enqueues next need not wait for it."""
     if not pos.is_cuda:
         raise RuntimeError("neighbor_list needs a CUDA tensor: there is no CPU path")
     lib = _lib.load()
@@ -297,9 +298,6 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
                                          row_ptr.data_ptr(), e, edge_index.data_ptr(),
                                          shifts.data_ptr(), flags.data_ptr(), work.data_ptr(),
                                          nbytes, st), "zp_neighbors_fill")
-        fl = int(flags.item())
-        if fl:
-            raise RuntimeError(f"zp_neighbors_fill: device flags {fl}")
     return edge_index, shifts, row_ptr
 
 
