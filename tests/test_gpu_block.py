@@ -129,3 +129,18 @@ def test_products_together_and_apart(e):
     a = gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"])
     b = gpu_node_out_and_vjp(make_block(cfg, params, precision="fp32_bf16x3"), case, case["upstream"])
     check_against(*a, *b)
+
+
+@pytest.mark.parametrize("e,ec,nb", [(37887, 12, 64), (37888, 12, 5), (37889, 12, 33), (37895, 132, 64),
+                                     (37896, 260, 70), (40001, 128, 130)])
+def test_front_end_of_many_edges(e, ec, nb, jd64):
+    """From 37 888 edges on a warp of the front end takes eight: the last warp full and not, basis
+    widths that end inside a quad of columns, that leave lanes over and that take several turns;
+    LayerNorm rows of up to 128, 256 and 512 columns, more than its blocks hold at a time."""
+    cfg = dict(lmax=1, mmax=1, sphere_channels=8, hidden_channels=8, edge_channels=ec,
+               num_distance_basis=nb, cutoff=5.0)
+    params = orc.init_params(cfg, seed=ec)
+    case = random_case(cfg, 400, e, seed=nb)
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    block = make_block(cfg, params)
+    check_against(*gpu_node_out_and_vjp(block, case, case["upstream"]), *want, tol=1e-5)

@@ -371,7 +371,8 @@ __device__ __forceinline__ void keep_nearest(Hit *h, int n, int cap, float cutof
 // with more than kFewHits hits or kKept survivors goes on the list `crowded` instead, its row of
 // `kept` marked: 192 hits because a warp walking again alone costs as much as a third of all others
 // (57 us for the few atoms in 100 000 that have more than 128 where the mean is 90).  Bound by
-// instruction issue: 186 us for 100 000 atoms, 90 hits each, cap 30, where a count of 90 us came before 235 us of this.
+// instruction issue: 186 us for 100 000 atoms, 90 hits each, cap 30, where a count of 90 us came before
+// 235 us of this.
 constexpr int kSelectWarps = 8;
 constexpr unsigned long long kCrowded = ~0ull;
 __global__ void __launch_bounds__(32 * kSelectWarps)
