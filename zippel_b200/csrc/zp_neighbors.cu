@@ -372,10 +372,10 @@ __device__ __forceinline__ void keep_nearest(Hit *h, int n, int cap, float cutof
 // `kept` marked: 192 hits because a warp walking again alone costs as much as a third of all others
 // (57 us for the few atoms in 100 000 that have more than 128 where the mean is 90).  Bound by
 // instruction issue: 186 us for 100 000 atoms, 90 hits each, cap 30, where a count of 90 us came before
-// 235 us of this.
+// 235 us of this.  Five blocks per SM (48 registers, no spills) instead of four: 12 us of the 186.
 constexpr int kSelectWarps = 8;
 constexpr unsigned long long kCrowded = ~0ull;
-__global__ void __launch_bounds__(32 * kSelectWarps)
+__global__ void __launch_bounds__(32 * kSelectWarps, 5)
 select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
               int32_t *__restrict__ counts, unsigned long long *__restrict__ kept, int32_t *flags,
               int32_t *__restrict__ crowded) {
