@@ -437,7 +437,10 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
  * ZP_NEIGHBORS_MAX_HITS neighbours of one atom in an uncapped list, bit 2: the passes disagree.  */
 #define ZP_NEIGHBORS_MAX_HITS 1024
 #define ZP_NEIGHBORS_MAX_CAP 256
+/* Work for any max_neighbors, and for one (less where it is below 128): the first call keeps each
+ * atom's edges there for the second.  */
 size_t zp_neighbors_work_bytes(int64_t n_atoms, double box, double cutoff);
+size_t zp_neighbors_work_bytes_capped(int64_t n_atoms, double box, double cutoff, int max_neighbors);
 int zp_neighbors_count(const double *pos, int64_t n_atoms, double box, double cutoff,
                        int max_neighbors, int32_t *row_ptr, int32_t *flags_out, void *work,
                        size_t work_bytes, void *stream);

@@ -119,6 +119,7 @@ SIGNATURES = {
                                     C.POINTER(ZpBlockParams), _P, _P, _P, C.POINTER(ZpBlockGrads),
                                     _P, _SZ, _P]),
     "zp_neighbors_work_bytes": (_SZ, [_I64, C.c_double, C.c_double]),
+    "zp_neighbors_work_bytes_capped": (_SZ, [_I64, C.c_double, C.c_double, C.c_int]),
     "zp_neighbors_count": (C.c_int, [_P, _I64, C.c_double, C.c_double, C.c_int, _P, _P, _P, _SZ, _P]),
     "zp_neighbors_fill": (C.c_int, [_P, _I64, C.c_double, C.c_double, C.c_int, _P, _I64, _P, _P, _P,
                                     _P, _SZ, _P]),

@@ -377,7 +377,7 @@ constexpr int kSelectWarps = 8;
 constexpr unsigned long long kCrowded = ~0ull;
 __global__ void __launch_bounds__(32 * kSelectWarps, 5)
 select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const Sorted atoms, int cap,
-              int32_t *__restrict__ counts, unsigned long long *__restrict__ kept, int32_t *flags,
+              int32_t *__restrict__ counts, unsigned long long *__restrict__ kept, int stride, int32_t *flags,
               int32_t *__restrict__ crowded) {
   zp_after_previous();
   __shared__ Hit hits[kSelectWarps][kFewHits];
@@ -398,7 +398,7 @@ select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const S
                  n += __popc(m);
                  return n <= kFewHits || cap <= 0 || n < cap;    // past both the count is known
                });
-  kept += j * kKept;
+  kept += j * stride;
   if (n > kFewHits || (n > kKept && (cap <= 0 || cap > kKept))) {             // left to fill_many_kernel
     if (lane == 0) {
       if (cap <= 0 && n > kHitCap) atomicOr(flags, 2);     // uncapped list too long for it
@@ -435,7 +435,8 @@ select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const S
 constexpr int kFillWarps = 8;
 __global__ void __launch_bounds__(32 * kFillWarps)
 fill_kernel(int64_t N, const int4 *__restrict__ own, Grid g,
-            const unsigned long long *__restrict__ kept, const int32_t *__restrict__ row_ptr,
+            const unsigned long long *__restrict__ kept, int stride,
+            const int32_t *__restrict__ row_ptr,
             int64_t E, int64_t *__restrict__ edge_index, double *__restrict__ shifts,
             const int32_t *__restrict__ flags) {
   zp_after_previous();
@@ -444,7 +445,7 @@ fill_kernel(int64_t N, const int4 *__restrict__ own, Grid g,
   if (j >= N) return;
   const int64_t base = row_ptr[j];
   const int n = (int)(row_ptr[j + 1] - base);
-  kept += j * kKept;
+  kept += j * stride;
   if (n <= 0 || kept[0] == kCrowded) return;
   const Writer out{own, g, flags[kUnwrapped] != 0, E, j, base, edge_index, shifts};
   for (int t = lane; t < n; t += 32) out.put_pair(kept[t], t);
@@ -524,7 +525,7 @@ struct NbWork {
   int32_t *flags, *cell_count, *cell_start, *cell_cursor, *atom_cell, *counts, *crowded,
       *block_sums;
   int4 *own;       // own image and index of each atom
-  unsigned long long *kept;     // [N][kKept] survivors of pass 1
+  unsigned long long *kept;     // [N][kept_stride] survivors of pass 1
   Sorted atoms;
   size_t bytes;
 };
@@ -555,7 +556,10 @@ int make_grid(int64_t N, double box, double cutoff, Grid *g) {
   return ZP_OK;
 }
 
-NbWork carve_nb(int64_t N, const Grid &g, void *base) {
+// edges per destination kept from pass 1 to pass 2
+int kept_stride(int cap) { return cap > 0 && cap < kKept ? cap : kKept; }
+
+NbWork carve_nb(int64_t N, const Grid &g, int cap, void *base) {
   NbWork w;
   size_t off = 0;
   auto take = [&](size_t n) {
@@ -576,7 +580,7 @@ NbWork carve_nb(int64_t N, const Grid &g, void *base) {
   w.atoms.y = reinterpret_cast<double *>(take((size_t)2 * N));
   w.atoms.z = reinterpret_cast<double *>(take((size_t)2 * N));
   w.atoms.who = reinterpret_cast<int4 *>(take((size_t)4 * N));
-  w.kept = reinterpret_cast<unsigned long long *>(take((size_t)2 * kKept * N));
+  w.kept = reinterpret_cast<unsigned long long *>(take((size_t)2 * kept_stride(cap) * N));
   w.counts = take((size_t)N + 1);
   w.block_sums = take((size_t)zp_ceil_div((int64_t)std::max<size_t>(cells, (size_t)N) + 2, kScanBlock) + 1);
   w.bytes = off;
@@ -588,9 +592,13 @@ NbWork carve_nb(int64_t N, const Grid &g, void *base) {
 extern "C" {
 
 size_t zp_neighbors_work_bytes(int64_t n_atoms, double box, double cutoff) {
+  return zp_neighbors_work_bytes_capped(n_atoms, box, cutoff, 0);
+}
+
+size_t zp_neighbors_work_bytes_capped(int64_t n_atoms, double box, double cutoff, int max_neighbors) {
   Grid g;
   if (n_atoms < 0 || make_grid(n_atoms, box, cutoff, &g)) return 0;
-  return carve_nb(n_atoms, g, nullptr).bytes;
+  return carve_nb(n_atoms, g, max_neighbors, nullptr).bytes;
 }
 
 int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, int max_neighbors,
@@ -602,7 +610,7 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
   if (N < 0 || N > 2000000000ll || !row_ptr || !flags_out || !work || (N && !pos))
     return ZP_ERR_INVALID_ARG;
   if (max_neighbors > ZP_NEIGHBORS_MAX_CAP) return ZP_ERR_TOO_LARGE;
-  const NbWork w = carve_nb(N, g, work);
+  const NbWork w = carve_nb(N, g, max_neighbors, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const size_t cells = (size_t)g.nc * g.nc * g.nc;
@@ -619,7 +627,8 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
               w.own, w.cell_start, w.cell_cursor, w.atoms);
     ZP_LAUNCH_CHECK("cell_fill_kernel");
     zp_launch(select_kernel, (unsigned)zp_ceil_div(N, kSelectWarps), 32 * kSelectWarps, 0, st, N, g,
-              w.cell_start, w.atoms, max_neighbors, w.counts, w.kept, w.flags, w.crowded);
+              w.cell_start, w.atoms, max_neighbors, w.counts, w.kept, kept_stride(max_neighbors),
+              w.flags, w.crowded);
     ZP_LAUNCH_CHECK("select_kernel");
   }
   if ((rc = exclusive_scan(N, w.counts, row_ptr, w.block_sums, st))) return rc;
@@ -637,12 +646,12 @@ int zp_neighbors_fill(const double *pos, int64_t N, double box, double cutoff, i
       (E && (!edge_index || !shifts)))
     return ZP_ERR_INVALID_ARG;
   if (max_neighbors > ZP_NEIGHBORS_MAX_CAP) return ZP_ERR_TOO_LARGE;
-  const NbWork w = carve_nb(N, g, work);
+  const NbWork w = carve_nb(N, g, max_neighbors, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   if (N > 0) {
     zp_launch(fill_kernel, (unsigned)zp_ceil_div(N, kFillWarps), 32 * kFillWarps, 0, st, N, w.own, g,
-              w.kept, row_ptr, E, edge_index, shifts, w.flags);
+              w.kept, kept_stride(max_neighbors), row_ptr, E, edge_index, shifts, w.flags);
     ZP_LAUNCH_CHECK("fill_kernel");
     const size_t smem = sizeof(Hit) * kHitCap * kWarpsPerBlock;
     static ZpSmemOptIn opt_in;

@@ -274,9 +274,9 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
     p = pos.detach().to(torch.float64).contiguous()
     n = p.shape[0]
     cap = int(max_neighbors) if max_neighbors else 0
-    nbytes = lib.zp_neighbors_work_bytes(n, float(box), float(cutoff))
+    nbytes = lib.zp_neighbors_work_bytes_capped(n, float(box), float(cutoff), cap)
     if nbytes == 0:
-        raise _lib.ZpError(1, "zp_neighbors_work_bytes")
+        raise _lib.ZpError(1, "zp_neighbors_work_bytes_capped")
     dev = p.device
     work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     out = torch.empty(n + 2, dtype=torch.int32, device=dev)       # row_ptr and, read with its end, flags
