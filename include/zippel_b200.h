@@ -415,7 +415,10 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
                      size_t workspace_bytes, int keep_for_backward, void *x_ready_event,
                      void *stream);
 /* grad_node_out as zp_eso2_backward (indexed by dst); grad_x_node [n_rows, K, C] and
- * grad_pos [n_rows, 3] may be null.                                                              */
+ * grad_pos [n_rows, 3] may be null.  Everything else the backward needs it finds in the workspace, so of
+ * `call` it reads the sizes, atomic_numbers, x_node, src, dst, row_ptr, perm_src and row_ptr_src, of
+ * `params` gauss_offsets, ln_gamma and ln_beta; these may lie elsewhere than in the forward, with the
+ * same values, and so may the workspace.  The other pointers may be null.                        */
 int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const zp_block_call *call,
                       const zp_block_params *params, const float *grad_node_out,
                       float *grad_x_node, float *grad_pos, const zp_block_grads *grads,

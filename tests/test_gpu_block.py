@@ -144,3 +144,47 @@ def test_front_end_of_many_edges(e, ec, nb, jd64):
     want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
     block = make_block(cfg, params)
     check_against(*gpu_node_out_and_vjp(block, case, case["upstream"]), *want, tol=1e-5)
+
+
+@pytest.mark.parametrize("how", ["checkpoint", "offload", "chunks"])
+def test_gradients_when_saved_tensors_come_back_elsewhere(how, monkeypatch):
+    """Checkpointed or with its saved tensors on the host, as one layer of a network whose embeddings are
+    an intermediate; and in chunks, which checkpoint by themselves, with inputs that every chunk
+    converts: the same gradients as the plain call, to the last bit where the sums are the same."""
+    from torch.autograd.graph import save_on_cpu
+    from torch.utils.checkpoint import checkpoint
+    from zippel_b200.blocks import eso2
+
+    cfg = dict(lmax=3, mmax=2, sphere_channels=32, hidden_channels=16, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=3))
+    case = {k: v.cuda() for k, v in random_case(cfg, 60, 6000, seed=4).items()}
+    f = {k: v.float() if v.is_floating_point() and k != "x_node" else v for k, v in case.items()}
+    z = f["atomic_numbers"].int()
+
+    def gradients(how):
+        pos, a = f["pos"].clone().requires_grad_(True), f["x_node"].clone().requires_grad_(True)
+
+        def layer(pos, a):
+            return block.node_output(pos, z, torch.tanh(a), f["edge_index"], f["shifts"],
+                                     f["cos_gamma_k"], f["sin_gamma_k"])
+
+        if how == "offload":
+            with save_on_cpu():
+                out = layer(pos, a)
+        elif how == "checkpoint":
+            out = checkpoint(layer, pos, a, use_reentrant=False)
+        else:
+            out = layer(pos, a)
+        junk = [torch.full_like(a, 1e3) for _ in range(40)]       # over whatever has been given back
+        grads = torch.autograd.grad(out, [pos, a, *block.parameters()], f["upstream"].to(out.dtype),
+                                    allow_unused=True)
+        del junk
+        return [out, *grads]
+
+    want = gradients("plain")
+    if how == "chunks":
+        monkeypatch.setattr(eso2, "MAX_EDGES_PER_CALL", 4096)
+    for got, ref in zip(gradients(how), want):
+        if ref is not None:
+            assert torch.equal(got, ref) if how != "chunks" else rel_l2(got, ref) < 2e-6

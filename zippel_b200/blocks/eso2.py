@@ -755,9 +755,7 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
     off = _as_f32(block.gauss_offset)
     if z.dtype != torch.int64 or not z.is_contiguous():
         z = z.to(torch.int64).contiguous()
-    for t in (pos, x, shifts, z, *params):
-        if not t.is_cuda:
-            raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
+    _need_cuda(pos, x, shifts, z, *params)
     assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
     assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.shape == (n,)
     assert cos_g.shape[1] == cfg.lmax + 1 and sin_g.shape == cos_g.shape
@@ -774,26 +772,33 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
         n1 - n0, e, n, n0, pos.data_ptr(), shifts.data_ptr(), z.data_ptr(), x.data_ptr(),
         cos_g.data_ptr(), sin_g.data_ptr(), order[0] if perm is None else perm.data_ptr(), *order[1:])
     p = [t.data_ptr() for t in params]
-    so2, keep = _weights_ptrs(plan.mmax, p[11:])
+    so2, _keep = _weights_ptrs(plan.mmax, p[11:])
     cparams = _lib.ZpBlockParams(p[0], off.data_ptr(), _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
                                  _P2(p[3], p[7]), _P2(p[4], p[8]), block.rad_func[1].eps, so2)
     _lib.run(x.device, "zp_block_forward", plan.handle, front, call, cparams, out.data_ptr(),
              ws.data_ptr(), nbytes, needs_bwd, x_ready.cuda_event if x_ready is not None else None)
     if not needs_bwd:
         return out, ()
-    # the workspace goes through save_for_backward like any activation, so that activation
-    # checkpointing can drop it and recompute; of the parameters the backward reads only
-    # the LayerNorms' (the products read the planes in the workspace)
-    ctx.native = (plan, graph, front, call, cparams, keep)
-    ctx.shapes, ctx.dtypes, ctx.row0 = [t.shape for t in params], dtypes, n0
+    # The workspace goes through save_for_backward like any activation, so that activation
+    # checkpointing and saved-tensor hooks can drop it and bring it back.  They bring it, and every
+    # other tensor, back at another address: no address outlives this call, and what the backward
+    # reads is all saved (of the parameters only the LayerNorms', the products read the planes in
+    # the workspace).
+    ctx.native = (plan, graph, front, (n1 - n0, e, n, n0))
+    ctx.shapes, ctx.dtypes = [t.shape for t in params], dtypes
     return out, (ws, x, pos, z, off, params[3], params[4], params[7], params[8])
 
 
 def _block_vjp(ctx, saved, grad_out, want):
     """Gradients of (pos, x_node, *params), None where ``want`` is false."""
-    ws, x, pos = saved[:3]
-    plan, graph, front, call, cparams, _keep = ctx.native
-    g = _as_f32(grad_out)
+    ws, x, pos, z, off, *norms = saved
+    plan, graph, front, sizes = ctx.native
+    g, x, off, *norms = (_as_f32(t) for t in (grad_out, x, off, *norms))
+    ln = [t.data_ptr() for t in norms]
+    order = graph.addresses()
+    call = _lib.ZpBlockCall(*sizes, None, None, z.data_ptr(), x.data_ptr(), None, None, None, *order[1:])
+    cparams = _lib.ZpBlockParams(None, off.data_ptr(), _P3(), _P3(), _P2(ln[0], ln[2]),
+                                 _P2(ln[1], ln[3]), 0.0, _lib.ZpWeights())
     f32 = dict(dtype=torch.float32, device=x.device)
     gpos = torch.empty(pos.shape, **f32) if want[0] else None
     gx = torch.empty(x.shape, **f32) if want[1] else None
@@ -808,7 +813,7 @@ def _block_vjp(ctx, saved, grad_out, want):
     grads = _lib.ZpBlockGrads(p[0], _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
                               _P2(p[3], p[7]), _P2(p[4], p[8]), so2)
     _lib.run(x.device, "zp_block_backward", plan.handle, front, call, cparams,
-             g.data_ptr() - ctx.row0 * plan.sizes.K * plan.c * 4,
+             g.data_ptr() - sizes[3] * plan.sizes.K * plan.c * 4,
              gx.data_ptr() if gx is not None else None,
              gpos.data_ptr() if gpos is not None else None, grads, ws.data_ptr(), ws.numel())
     del keep
@@ -817,6 +822,12 @@ def _block_vjp(ctx, saved, grad_out, want):
 
 
 _P2, _P3 = ctypes.c_void_p * 2, ctypes.c_void_p * 3
+
+
+def _need_cuda(*tensors: torch.Tensor) -> None:
+    for t in tensors:
+        if not t.is_cuda:
+            raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
 
 
 def _as_f32(t: torch.Tensor) -> torch.Tensor:

@@ -85,8 +85,9 @@ BlockWs carve_block(const zp_plan *p, const zp_front_config &f, int64_t N, int64
   return w;
 }
 
-int check_call(const zp_plan *plan, const zp_front_config *f, const zp_block_call *c,
-               const zp_block_params *p) {
+// what both directions read
+int check_common(const zp_plan *plan, const zp_front_config *f, const zp_block_call *c,
+                 const zp_block_params *p) {
   if (!plan || !f || !c || !p) return ZP_ERR_INVALID_ARG;
   if (f->lmax != plan->t.lmax || f->edge_channels < 4 || f->edge_channels % 4 ||
       f->edge_channels > 1024 || plan->t.R % 8)
@@ -94,15 +95,22 @@ int check_call(const zp_plan *plan, const zp_front_config *f, const zp_block_cal
   if (c->n_nodes < 0 || c->n_edges < 0 || c->n_rows < c->n_nodes) return ZP_ERR_INVALID_ARG;
   if (c->n_nodes == 0) return c->n_edges == 0 ? ZP_OK : ZP_ERR_INVALID_ARG;
   if (!c->x_node || !c->row_ptr || !zp_aligned16(c->x_node)) return ZP_ERR_INVALID_ARG;
-  if (c->n_edges && (!c->pos || !c->shifts || !c->atomic_numbers || !c->cos_g || !c->sin_g ||
-                     !c->perm || !c->src || !c->dst))
-    return ZP_ERR_INVALID_ARG;
-  if (!p->emb || !p->gauss_offsets || !zp_aligned16(p->emb)) return ZP_ERR_INVALID_ARG;
-  for (int i = 0; i < 3; ++i)
-    if (!p->rad_w[i] || !p->rad_b[i]) return ZP_ERR_INVALID_ARG;
+  if (c->n_edges && (!c->atomic_numbers || !c->src || !c->dst)) return ZP_ERR_INVALID_ARG;
+  if (!p->gauss_offsets) return ZP_ERR_INVALID_ARG;
   for (int i = 0; i < 2; ++i)
     if (!p->ln_gamma[i] || !p->ln_beta[i] || !zp_aligned16(p->ln_gamma[i]) || !zp_aligned16(p->ln_beta[i]))
       return ZP_ERR_INVALID_ARG;
+  return ZP_OK;
+}
+int check_forward(const zp_plan *plan, const zp_front_config *f, const zp_block_call *c,
+                  const zp_block_params *p) {
+  if (const int rc = check_common(plan, f, c, p)) return rc;
+  if (c->n_nodes == 0) return ZP_OK;
+  if (c->n_edges && (!c->pos || !c->shifts || !c->cos_g || !c->sin_g || !c->perm))
+    return ZP_ERR_INVALID_ARG;
+  if (!p->emb || !zp_aligned16(p->emb)) return ZP_ERR_INVALID_ARG;
+  for (int i = 0; i < 3; ++i)
+    if (!p->rad_w[i] || !p->rad_b[i]) return ZP_ERR_INVALID_ARG;
   return zp_check_weights(plan, &p->so2);
 }
 
@@ -137,7 +145,7 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
                      const zp_block_params *params, float *node_out, void *workspace,
                      size_t workspace_bytes, int keep_for_backward, void *x_ready_event,
                      void *stream) {
-  int rc = check_call(plan, front, call, params);
+  int rc = check_forward(plan, front, call, params);
   if (rc) return rc;
   const int64_t N = call->n_nodes, E = call->n_edges;
   if (N == 0) return ZP_OK;
@@ -243,7 +251,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                       const zp_block_params *params, const float *grad_node_out,
                       float *grad_x_node, float *grad_pos, const zp_block_grads *grads,
                       void *workspace, size_t workspace_bytes, void *stream) {
-  int rc = check_call(plan, front, call, params);
+  int rc = check_common(plan, front, call, params);
   if (rc) return rc;
   const int64_t N = call->n_nodes, E = call->n_edges, rows = call->n_rows;
   if (N == 0) return ZP_OK;
