@@ -66,7 +66,7 @@ def backward_addresses(lib):
 
 
 @pytest.mark.parametrize("what,entry", [("hooks", "node_output"), ("hooks", "energy"),
-                                        ("checkpoint", "node_output")])
+                                        ("checkpoint", "node_output"), ("checkpoint", "energy")])
 def test_the_backward_reads_the_tensors_that_were_brought_back(fake, what, entry, monkeypatch):
     lib, block, case, graph = fake
     alive = []

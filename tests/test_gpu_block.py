@@ -188,3 +188,24 @@ def test_gradients_when_saved_tensors_come_back_elsewhere(how, monkeypatch):
     for got, ref in zip(gradients(how), want):
         if ref is not None:
             assert torch.equal(got, ref) if how != "chunks" else rel_l2(got, ref) < 2e-6
+
+
+@pytest.mark.parametrize("frozen", [False, True])
+def test_checkpointed_energy(frozen):
+    from torch.utils.checkpoint import checkpoint
+    cfg = dict(lmax=2, mmax=1, sphere_channels=16, hidden_channels=16, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1)).requires_grad_(not frozen)
+    case = {k: v.cuda().float() if v.is_floating_point() else v.cuda()
+            for k, v in random_case(cfg, 20, 150, seed=2).items()}
+
+    def energy(pos):
+        return block(pos, case["atomic_numbers"], case["x_node"], case["edge_index"], case["shifts"],
+                     case["cos_gamma_k"], case["sin_gamma_k"])
+
+    pos = case["pos"].clone().requires_grad_(True)
+    wrt = [pos] if frozen else [pos, *block.parameters()]
+    want = torch.autograd.grad(energy(pos), wrt)
+    got = torch.autograd.grad(checkpoint(energy, pos, use_reentrant=False), wrt)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)

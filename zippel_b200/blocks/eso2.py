@@ -717,13 +717,15 @@ class EnergyFunction(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_e):
-        out, *head, work = ctx.saved_tensors[-6:]
+        # asked for once: checkpointing brings a tensor back a single time
+        saved = ctx.saved_tensors
+        out, *head, work = saved[-6:]
         want, plan = _wanted(ctx, len(ctx.shapes) + 4), ctx.native[0]
         g = torch.empty_like(out)
         ghead = _readout_vjp(plan, out, head, grad_e, g, work, any(want[-4:]))
         ghead = [t if w else None for t, w in zip(ghead, want[-4:])]
         grads = ((None,) * len(want[:-4]) if not any(want[:-4]) else
-                 _block_vjp(ctx, ctx.saved_tensors[:-6], g, want[:-4]))
+                 _block_vjp(ctx, saved[:-6], g, want[:-4]))
         return _returned(ctx, grads + tuple(t if t is None or t.dtype == dt else t.to(dt)
                                             for t, dt in zip(ghead, ctx.head_dtypes)))
 
