@@ -7,6 +7,9 @@ import types
 
 import pytest
 import torch
+import torch.nn.utils.parametrizations
+import torch.nn.utils.parametrize
+import torch.nn.utils.prune
 from torch.autograd.graph import saved_tensors_hooks
 from torch.utils.checkpoint import checkpoint
 
@@ -92,3 +95,67 @@ def test_the_backward_reads_the_tensors_that_were_brought_back(fake, what, entry
                             lambda ctx, saved, *rest: (alive.extend(saved), vjp(ctx, saved, *rest))[1])
         checkpoint(layer, a, use_reentrant=False).sum().backward()
     assert backward_addresses(lib) <= {t.data_ptr() for t in alive}
+
+
+def test_parameters_are_listed_in_registration_order():
+    for lmax, mmax in ((0, 0), (2, 0), (3, 3), (6, 2)):
+        block = eso2.ESO2Block(eso2.BlockConfig(**{**CFG, "lmax": lmax, "mmax": mmax, "hidden_channels": 16}))
+        listed = block._call_params(True)
+        assert [id(p) for p in listed] == [id(p) for p in block.parameters()]
+        assert [id(p) for p in block._call_params(False)] == [id(p) for p in listed[:-4]]
+
+
+@pytest.mark.parametrize("what", ["pruned", "weight_norm", "parametrized", "more parameters"])
+def test_layers_that_form_their_weights_are_asked_for_them(fake, what):
+    """The addresses the library gets are those of the weights the layers form, in their places."""
+    lib, block, case, graph = fake
+    torch.manual_seed(0)
+    if what == "pruned":
+        torch.nn.utils.prune.l1_unstructured(block.rad_func[0], "weight", 0.5)
+        torch.nn.utils.prune.l1_unstructured(block.c1_m0, "weight", 0.5)
+    elif what == "weight_norm":
+        torch.nn.utils.parametrizations.weight_norm(block.rad_func[3])
+        torch.nn.utils.parametrizations.weight_norm(block.c2_m[0])
+    elif what == "parametrized":
+        class Twice(torch.nn.Module):
+            def forward(self, w):
+                return 2 * w
+        torch.nn.utils.parametrize.register_parametrization(block.elem_emb, "weight", Twice())
+        torch.nn.utils.parametrize.register_parametrization(block.c2_m0, "bias", Twice())
+    else:
+        block.scale = torch.nn.Parameter(torch.ones(3))
+        block.head2 = torch.nn.Linear(4, 4)
+    want = [block.elem_emb.weight, *[t for i in (0, 1, 3, 4, 6) for t in (block.rad_func[i].weight, block.rad_func[i].bias)],
+            block.c1_m0.weight, block.c1_m0.bias, block.c1_m[0].weight,
+            block.c2_m0.weight, block.c2_m0.bias, block.c2_m[0].weight]
+    got = []
+    apply = eso2._block
+    eso2._block = lambda *args: (got.extend(args[-1]), apply(*args))[1]
+    try:
+        node_output(block, case, graph, case["pos"].requires_grad_(True), case["x_node"]).sum().backward()
+    finally:
+        eso2._block = apply
+    assert len(got) == len(want)
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and torch.equal(a, b)
+    named = dict(block.named_parameters())
+    for name, p in named.items():
+        unused = name.startswith(("readout", "scale", "head2"))
+        assert (p.grad is None) == unused, name
+        assert unused or p.grad.shape == p.shape
+
+
+@pytest.mark.parametrize("what", ["eps", "bias", "layers"])
+def test_radial_mlps_that_the_one_call_does_not_run(fake, what, monkeypatch):
+    lib, block, case, graph = fake
+    if what == "eps":
+        block.rad_func[4].eps = 1e-3
+    elif what == "bias":
+        block.rad_func[3].bias = None
+    else:
+        block.rad_func = torch.nn.Sequential(block.rad_func[0], *block.rad_func[1:3], block.rad_func[6])
+    taken = []
+    monkeypatch.setattr(eso2, "_edge_budget", lambda *args: 1 << 20)
+    monkeypatch.setattr(block, "_edges_to_nodes_in_parts", lambda *args: taken.append(args) or case["x_node"])
+    node_output(block, case, graph, case["pos"], case["x_node"])
+    assert len(taken) == 1 and not lib.calls

@@ -209,3 +209,54 @@ def test_checkpointed_energy(frozen):
     got = torch.autograd.grad(checkpoint(energy, pos, use_reentrant=False), wrt)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("what", ["eps", "deeper", "pruned", "parametrized"])
+def test_blocks_with_layers_of_their_own(what, jd64, monkeypatch):
+    """Two LayerNorms of different eps and a radial MLP of another depth run layer by layer; pruned and
+    parametrized layers run in one call with the weights they form."""
+    import torch.nn.utils.parametrize
+    import torch.nn.utils.prune
+    cfg = dict(lmax=2, mmax=1, sphere_channels=16, hidden_channels=8, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    params = orc.init_params(cfg, seed=9)
+    case = random_case(cfg, 17, 131, seed=8)
+    block = make_block(cfg, params)
+    used, eps = {k: v.double() for k, v in params.items()}, [1e-5, 1e-5]
+    deeper = None
+    if what == "eps":
+        eps[1] = block.rad_func[4].eps = 0.3
+    elif what == "deeper":
+        torch.manual_seed(3)
+        deeper = torch.nn.Linear(16, 16).cuda()
+        block.rad_func.insert(6, deeper)
+    elif what == "pruned":
+        torch.nn.utils.prune.l1_unstructured(block.rad_func[3], "weight", 0.4)
+        torch.nn.utils.prune.l1_unstructured(block.c1_m[0], "weight", 0.4)
+        used["rad_func.3.weight"] = block.rad_func[3].weight.detach().cpu().double()
+        used["c1_m.0.weight"] = block.c1_m[0].weight.detach().cpu().double()
+    else:
+        class Twice(torch.nn.Module):
+            def forward(self, w):
+                return 2 * w
+        torch.nn.utils.parametrize.register_parametrization(block.c2_m0, "weight", Twice())
+        used["c2_m0.weight"] = 2 * used["c2_m0.weight"]
+
+    def radial_mlp(p, h):
+        f = torch.nn.functional
+        for lin, ln, e in ((0, 1, eps[0]), (3, 4, eps[1])):
+            h = f.linear(h, p[f"rad_func.{lin}.weight"], p[f"rad_func.{lin}.bias"])
+            h = f.silu(f.layer_norm(h, h.shape[-1:], p[f"rad_func.{ln}.weight"], p[f"rad_func.{ln}.bias"], e))
+        if deeper is not None:
+            h = f.linear(h, deeper.weight.detach().cpu().double(), deeper.bias.detach().cpu().double())
+        return f.linear(h, p["rad_func.6.weight"], p["rad_func.6.bias"])
+
+    monkeypatch.setattr(orc, "radial_mlp", radial_mlp)
+    want = oracle_node_out_and_vjp(cfg, used, case, case["upstream"], jd64)
+    out, gx, gpos, pg = gpu_node_out_and_vjp(block, case, case["upstream"])
+    assert rel_l2(out, want[0]) < 1e-5 and rel_l2(gx, want[1]) < 1e-5 and rel_l2(gpos, want[2]) < 1e-5
+    for name, ref in want[3].items():
+        if name in pg and ref is not None and ref.abs().max() > 0 and not (deeper is not None and name.startswith("rad_func.6")):
+            assert rel_l2(pg[name], ref) < 1e-5, name
+    if deeper is not None:
+        assert rel_l2(pg["rad_func.7.weight"], want[3]["rad_func.6.weight"]) < 1e-5

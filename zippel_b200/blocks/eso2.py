@@ -25,6 +25,7 @@ when the block is built.
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from dataclasses import dataclass
 
@@ -183,6 +184,15 @@ def _weights_struct(mmax, c1_w0, c1_b0, c1_wm, c2_w0, c2_b0, c2_wm):
     return w, (a1, a2)
 
 
+def _so2_shapes(lmax: int, mmax: int, c: int, h: int) -> list[tuple]:
+    """Shapes of c1_w0, c1_b0, c2_w0, c2_b0, c1_wm.., c2_wm.."""
+    k = lmax + 1
+    orders = range(1, mmax + 1)
+    return [(k * h + lmax * h, 2 * k * c), (k * h + lmax * h,), (k * c, k * h), (k * c,),
+            *[(2 * (k - m) * h, 2 * (k - m) * c) for m in orders],
+            *[(2 * (k - m) * c, (k - m) * h) for m in orders]]
+
+
 def _f32(t: torch.Tensor) -> torch.Tensor:
     return t.detach().to(torch.float32).contiguous()
 
@@ -304,6 +314,7 @@ class EdgeConvFunction(torch.autograd.Function):
         assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
         assert rad.shape == ((e, ec) if has_layer else (e, s.R)) and ev.shape == (e, 3)
         assert not has_layer or (rw.shape == (s.R, ec) and rb.shape == (s.R,))
+        assert [t.shape for t in tens[8:]] == _so2_shapes(plan.lmax, mmax, plan.c, plan.h)
         assert en.shape == (e,) and cg.shape == (e, plan.lmax + 1) and sg.shape == cg.shape
         needs_bwd = any(ctx.needs_input_grad)
         # a graph may carry `node_range = (n0, n1)`: all its edges end in those nodes and only
@@ -537,6 +548,9 @@ class EdgeFeatures(torch.autograd.Function):
         posf, shf, embf, off = _f32(pos), _f32(shifts), _f32(emb), _f32(gauss_offset)
         cgf, sgf = _f32(cos_g), _f32(sin_g)
         zi = atomic_numbers.to(torch.int64).contiguous()
+        if emb.shape[0] < front.n_elements or emb.shape[1] != front.edge_channels:
+            raise ValueError(f"the element embedding has shape {tuple(emb.shape)}, the block needs "
+                             f"({front.n_elements}, {front.edge_channels})")
         f32 = dict(dtype=torch.float32, device=dev)
         width = front.num_basis + 2 * front.edge_channels
         edge_vec, dist = torch.empty(e, 3, **f32), torch.empty(e, **f32)
@@ -567,7 +581,8 @@ class EdgeFeatures(torch.autograd.Function):
         dev = edge_vec.device
         g_pos = torch.empty(n, 3, dtype=torch.float32, device=dev)
         need_emb = ctx.needs_input_grad[6]
-        g_emb = torch.empty(ctx.n_elem, front.edge_channels, dtype=torch.float32,
+        # (rows past the block's elements are not written)
+        g_emb = torch.zeros(ctx.n_elem, front.edge_channels, dtype=torch.float32,
                             device=dev) if need_emb else None
         ptr = lambda t: None if t is None else _f32(t)            # noqa: E731
         gev, gxe, gen = ptr(g_edge_vec), ptr(g_x_edge), ptr(g_env)
@@ -824,6 +839,27 @@ def _block_vjp(ctx, saved, grad_out, want):
 
 
 _P2, _P3 = ctypes.c_void_p * 2, ctypes.c_void_p * 3
+#: the radial MLP that the block runs in one call
+_RADIAL_LAYERS = (nn.Linear, nn.LayerNorm, nn.SiLU, nn.Linear, nn.LayerNorm, nn.SiLU, nn.Linear)
+
+
+@functools.cache
+def _param_shapes(cfg: BlockConfig, head: bool) -> list[tuple]:
+    """Shapes of a block's parameters in registration order, with or without the readout's."""
+    widths = [*cfg.edge_channels_list, 2 * cfg.sphere_channels * sum(Layout.make(cfg.lmax, cfg.mmax).m_size)]
+    out = [(cfg.max_num_elements, cfg.edge_channels)]
+    for i, (w_in, w_out) in enumerate(zip(widths, widths[1:])):
+        out += [(w_out, w_in), (w_out,)] + ([(w_out,), (w_out,)] if i < 2 else [])
+    c, m = cfg.sphere_channels, cfg.mmax
+    w10, b10, w20, b20, *wm = _so2_shapes(cfg.lmax, m, c, cfg.hidden_channels)
+    out += [w10, b10, *wm[:m], w20, b20, *wm[m:]]
+    return out + ([(c, c * (cfg.lmax + 1)), (c,), (1, c), (1,)] if head else [])
+
+
+def _param(module: nn.Module, name: str):
+    """``module.name``, without the search through the module where it is a plain parameter."""
+    p = module._parameters.get(name)
+    return getattr(module, name) if p is None else p
 
 
 def _need_cuda(*tensors: torch.Tensor) -> None:
@@ -933,25 +969,60 @@ class ESO2Block(nn.Module):
         return radial_mlp(plan, x_edge, list(self.rad_func))
 
     # -- forward --------------------------------------------------------------------------
-    def _all_params(self) -> list:
-        """``list(self.parameters())`` without the names and the search for repetitions."""
-        found, todo = [], [self]
-        while todo:
-            module = todo.pop()
-            found += [p for p in module._parameters.values() if p is not None]
-            todo += reversed(module._modules.values())
-        return found
-
-    def _block_params(self) -> list:
-        """Parameters of everything before the readout, in registration order."""
-        return self._all_params()[:-4]
+    def _call_params(self, head: bool) -> list | None:
+        """The parameters of everything before the readout (and with ``head`` those of the readout)
+        in the order the one-call functions list them, each by its name in the module: a pruned or
+        parametrized layer forms its weight when asked for it.  None for a block whose layers have
+        been replaced by others than the native call runs (it has one eps for both LayerNorms)."""
+        m = self._modules
+        rad = tuple(m["rad_func"]._modules.values())
+        if (len(rad) != 7 or not all(map(isinstance, rad, _RADIAL_LAYERS)) or rad[1].eps != rad[4].eps):
+            return None
+        c1, c2 = m["c1_m0"], m["c2_m0"]
+        out = [_param(m["elem_emb"], "weight")]
+        for layer in (rad[0], rad[1], rad[3], rad[4], rad[6]):
+            out += (_param(layer, "weight"), _param(layer, "bias"))
+        out += (_param(c1, "weight"), _param(c1, "bias"))
+        out += [_param(layer, "weight") for layer in m["c1_m"]._modules.values()]
+        out += (_param(c2, "weight"), _param(c2, "bias"))
+        out += [_param(layer, "weight") for layer in m["c2_m"]._modules.values()]
+        if head:
+            lin0, lin1 = self.readout[0], self.readout[2]
+            out += (_param(lin0, "weight"), _param(lin0, "bias"), _param(lin1, "weight"), _param(lin1, "bias"))
+        shapes = _param_shapes(self.cfg, head)
+        return out if [None if p is None else p.shape for p in out] == shapes else None
 
     def _edges_to_nodes(self, plan, graph, perm, pos, atomic_numbers, x_node, shifts, cos_gamma_k,
                         sin_gamma_k, x_ready=None) -> torch.Tensor:
         """node_out rows of the edges of `graph` (whose positions in the caller's arrays are the
         int32 `perm`)."""
+        params = self._call_params(False)
+        if params is None:
+            return self._edges_to_nodes_in_parts(plan, graph, perm, pos, atomic_numbers, x_node, shifts,
+                                                 cos_gamma_k, sin_gamma_k, x_ready)
         return BlockFunction.apply(self, plan, graph, perm, atomic_numbers, shifts, cos_gamma_k,
-                                   sin_gamma_k, x_ready, pos, x_node, *self._block_params())
+                                   sin_gamma_k, x_ready, pos, x_node, *params)
+
+    def _edges_to_nodes_in_parts(self, plan, graph, perm, pos, atomic_numbers, x_node, shifts,
+                                 cos_gamma_k, sin_gamma_k, x_ready) -> torch.Tensor:
+        """The same with the front end, every radial layer and the edge convolution as functions of
+        their own, for a radial MLP that the one call does not run."""
+        edge_vec, x_edge, env, cos_s, sin_s = EdgeFeatures.apply(
+            graph, perm, self.front_config(), pos, shifts, atomic_numbers, self.elem_emb.weight,
+            self.gauss_offset, cos_gamma_k, sin_gamma_k)
+        last, rad_w, rad_b = self.rad_func[-1], None, None
+        if isinstance(last, nn.Linear) and last.in_features % 8 == 0 and graph.n_edges > 0:
+            # the last (widest) radial layer runs inside the edge-convolution call
+            radial = radial_mlp(plan, x_edge, list(self.rad_func)[:-1])
+            rad_w, rad_b = last.weight, last.bias
+        else:
+            radial = self.radial_mlp(plan, x_edge)
+        if x_ready is not None:
+            torch.cuda.current_stream(pos.device).wait_event(x_ready)
+        return EdgeConvFunction.apply(plan, graph, x_node, edge_vec, cos_s, sin_s, radial, env, rad_w, rad_b,
+                                      self.c1_m0.weight, self.c1_m0.bias, self.c2_m0.weight,
+                                      self.c2_m0.bias, *[layer.weight for layer in self.c1_m],
+                                      *[layer.weight for layer in self.c2_m])
 
     def _sorted_edges(self, edge_index, atomic_numbers):
         """The edge order of new input and the check of its indices, to be called once the work that
@@ -986,12 +1057,12 @@ class ESO2Block(nn.Module):
             graph, check = self._sorted_edges(edge_index, atomic_numbers)
         plan = self.plan(pos.device)
         energy = function is EnergyFunction
-        params = self._all_params() if energy else self._block_params()
-        if not (torch.is_grad_enabled() and any([p.requires_grad for p in params])):
+        params = self._call_params(energy)
+        if params is not None and not (torch.is_grad_enabled() and any([p.requires_grad for p in params])):
             params = [params]
         try:
             out = None
-            if _surely_fits(plan, graph.n_edges):
+            if params is not None and _surely_fits(plan, graph.n_edges):
                 try:
                     out = function.apply(self, plan, graph, None, atomic_numbers, shifts,
                                          cos_gamma_k, sin_gamma_k, x_ready, pos, x_node, *params)
