@@ -159,3 +159,20 @@ def test_radial_mlps_that_the_one_call_does_not_run(fake, what, monkeypatch):
     monkeypatch.setattr(block, "_edges_to_nodes_in_parts", lambda *args: taken.append(args) or case["x_node"])
     node_output(block, case, graph, case["pos"], case["x_node"])
     assert len(taken) == 1 and not lib.calls
+
+
+@pytest.mark.parametrize("entry", ["node_output", "energy"])
+def test_tangents_of_frozen_parameters_are_refused(fake, entry):
+    """There is no forward mode: as on a tensor argument, a tangent on a parameter raises and is not lost."""
+    import torch.autograd.forward_ad as fwad
+    lib, block, case, graph = fake
+    block.requires_grad_(False)
+    args = (case["pos"], case["atomic_numbers"], case["x_node"], case["edge_index"], case["shifts"],
+            case["cos_gamma_k"], case["sin_gamma_k"])
+    call = block.node_output if entry == "node_output" else block
+    with fwad.dual_level():
+        w = fwad.make_dual(block.c1_m0.weight.detach(), torch.ones_like(block.c1_m0.weight))
+        del block.c1_m0._parameters["weight"]
+        block.c1_m0.weight = w
+        with pytest.raises(RuntimeError, match="forward"):
+            call(*args, graph=graph)

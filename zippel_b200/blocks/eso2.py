@@ -32,6 +32,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 import torch.nn as nn
+from torch.autograd import forward_ad
 
 from .. import _lib
 from ..graph import EdgeChunk, EdgeGraph
@@ -745,6 +746,13 @@ class EnergyFunction(torch.autograd.Function):
                                             for t, dt in zip(ghead, ctx.head_dtypes)))
 
 
+def _differentiated(params: list) -> bool:
+    """Whether autograd has to see each of ``params``: for a gradient, or to refuse tangents
+    (forward mode), which on a tensor inside a list it would not notice."""
+    return (forward_ad._current_level >= 0
+            or torch.is_grad_enabled() and any([p.requires_grad for p in params]))
+
+
 def _listed(ctx, params):
     ctx.listed = len(params) == 1 and isinstance(params[0], list)
     return params[0] if ctx.listed else params
@@ -1058,7 +1066,7 @@ class ESO2Block(nn.Module):
         plan = self.plan(pos.device)
         energy = function is EnergyFunction
         params = self._call_params(energy)
-        if params is not None and not (torch.is_grad_enabled() and any([p.requires_grad for p in params])):
+        if params is not None and not _differentiated(params):
             params = [params]
         try:
             out = None
