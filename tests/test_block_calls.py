@@ -176,3 +176,27 @@ def test_tangents_of_frozen_parameters_are_refused(fake, entry):
         block.c1_m0.weight = w
         with pytest.raises(RuntimeError, match="forward"):
             call(*args, graph=graph)
+
+
+@pytest.mark.parametrize("what", ["nothing", "energy", "node_output", "instance"])
+def test_the_energy_goes_through_overridden_methods(fake, what, monkeypatch):
+    lib, block, case, graph = fake
+    seen = []
+
+    def energy(self, out):
+        seen.append("energy")
+        return out.sum()
+
+    def node_output(self, *args):
+        seen.append("node_output")
+        return eso2.ESO2Block.node_output(self, *args)
+
+    monkeypatch.setattr(eso2, "Readout", types.SimpleNamespace(apply=lambda plan, out, *params: out.sum()))
+    if what == "instance":
+        block.energy = lambda out: energy(block, out)
+    elif what != "nothing":
+        block.__class__ = type("Own", (eso2.ESO2Block,), {what: {"energy": energy, "node_output": node_output}[what]})
+    with torch.no_grad():
+        block(case["pos"], case["atomic_numbers"], case["x_node"], case["edge_index"], case["shifts"],
+              case["cos_gamma_k"], case["sin_gamma_k"], graph=graph)
+    assert seen == {"nothing": [], "instance": ["energy"]}.get(what, [what])

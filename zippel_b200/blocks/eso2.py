@@ -1176,6 +1176,10 @@ class ESO2Block(nn.Module):
         """Scalar E.  ``jd`` (the reference's argument) is verified against the J matrices the
         kernels use; anything else raises ``ValueError``."""
         self._check_jd(jd)
+        for name in ("node_output", "energy"):      # a subclass' own, or one set on the instance
+            if getattr(type(self), name) is not getattr(ESO2Block, name) or name in self.__dict__:
+                return self.energy(self.node_output(pos, atomic_numbers, x_node, edge_index, shifts,
+                                                    cos_gamma_k, sin_gamma_k, graph))
         return self._evaluate(EnergyFunction, pos, atomic_numbers, x_node, edge_index, shifts,
                               cos_gamma_k, sin_gamma_k, graph)
 
