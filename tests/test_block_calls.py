@@ -48,7 +48,7 @@ def fake(monkeypatch):
     k = (CFG["lmax"] + 1) ** 2
     plan = types.SimpleNamespace(handle=None, c=8, h=8, lmax=CFG["lmax"], mmax=CFG["mmax"],
                                  sizes=types.SimpleNamespace(K=k), precision=2,
-                                 device=torch.device("cpu"), bytes_per_edge=1.0, total_memory=1 << 40)
+                                 device=torch.device("cpu"), bytes_per_edge=1.0, total_memory=1 << 40, foreign=0)
     monkeypatch.setattr(block, "plan", lambda device: plan)
     case = {key: v.float() if v.is_floating_point() else v for key, v in random_case(CFG, 9, 40, seed=1).items()}
     csr = csr_reference(case["edge_index"].numpy(), 9)
@@ -200,3 +200,23 @@ def test_the_energy_goes_through_overridden_methods(fake, what, monkeypatch):
         block(case["pos"], case["atomic_numbers"], case["x_node"], case["edge_index"], case["shifts"],
               case["cos_gamma_k"], case["sin_gamma_k"], graph=graph)
     assert seen == {"nothing": [], "instance": ["energy"]}.get(what, [what])
+
+
+def test_when_a_call_is_made_in_one_piece(monkeypatch):
+    gib = 1 << 30
+    plan = types.SimpleNamespace(device=torch.device("cuda", 0), bytes_per_edge=2.0 ** 17, total_memory=160 * gib,
+                                 foreign=8 * gib)
+    held = [0]
+    monkeypatch.setattr(eso2, "_allocated", lambda device: held[0])
+    edges = lambda g: int(g * gib / plan.bytes_per_edge)                             # noqa: E731
+    assert eso2._one_piece(plan, edges(10), True, 4) and eso2._one_piece(plan, edges(10), False, 4)
+    assert not eso2._one_piece(plan, edges(10.1), True, 4) and not eso2._one_piece(plan, edges(10.1), False, 4)
+    # layers that keep their activations stop short of filling the device, in the end layer by layer
+    held[0] = 112 * gib
+    assert eso2._one_piece(plan, edges(10), True, 4) and not eso2._one_piece(plan, edges(10) + 1, True, 4)
+    held[0] = 113 * gib
+    assert not eso2._one_piece(plan, edges(10), True, 4) and eso2._one_piece(plan, edges(10), True, 2)
+    plan.foreign = 100 * gib
+    assert not eso2._one_piece(plan, edges(10), True, 2) and eso2._one_piece(plan, edges(10), False, 2)
+    monkeypatch.setattr(eso2, "MAX_EDGES_PER_CALL", 64)
+    assert not eso2._one_piece(plan, 8, False, 4)

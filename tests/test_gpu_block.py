@@ -260,3 +260,56 @@ def test_blocks_with_layers_of_their_own(what, jd64, monkeypatch):
             assert rel_l2(pg[name], ref) < 1e-5, name
     if deeper is not None:
         assert rel_l2(pg["rad_func.7.weight"], want[3]["rad_func.6.weight"]) < 1e-5
+
+
+@pytest.mark.parametrize("entry", ["node_output", "energy", "vjp", "edge_conv"])
+def test_out_of_memory_in_one_piece_goes_on_in_chunks(entry, monkeypatch):
+    """The first allocation of a workspace fails: the call is made in chunks, with the same results."""
+    from zippel_b200.blocks import eso2
+    from zippel_b200.graph import EdgeGraph
+
+    cfg = dict(lmax=2, mmax=1, sphere_channels=16, hidden_channels=16, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=3))
+    case = {k: v.cuda().float() if v.is_floating_point() else v.cuda()
+            for k, v in random_case(cfg, 60, 6000, seed=4).items()}
+    graph = EdgeGraph.build(case["edge_index"], 60)
+    args = [case[k] for k in ("atomic_numbers", "x_node", "edge_index", "shifts", "cos_gamma_k", "sin_gamma_k")]
+    plan, params = block.plan("cuda"), [p for n, p in block.named_parameters() if not n.startswith("readout")]
+
+    def run():
+        pos = case["pos"].clone().requires_grad_(True)
+        if entry == "node_output":
+            out = block.node_output(pos, *args, graph=graph)
+            return [out, *torch.autograd.grad(out, [pos, *params], case["upstream"])]
+        if entry == "energy":
+            out = block(pos, *args, graph=graph)
+            return [out, *torch.autograd.grad(out, [pos, *params])]
+        if entry == "vjp":
+            out, gx, gpos, gp = block.node_output_vjp(case["pos"], *args, case["upstream"], graph=graph)
+            return [out, gx, gpos, *[g for g in gp if g is not None]]
+        return [block._edges_to_nodes_in_parts(plan, graph, graph.perm, pos, *args[:2], *args[3:], None)]
+
+    want = run()
+    failed = []
+
+    def failing(inner, nth):
+        def call(*a, **k):
+            if not failed:
+                failed.append(nth)
+                raise torch.cuda.OutOfMemoryError("for the test")
+            return inner(*a, **k)
+        return call
+
+    monkeypatch.setattr(eso2, "_edge_budget", lambda *a: 4096)
+    if entry == "edge_conv":
+        monkeypatch.setattr(plan, "workspace", failing(plan.workspace, 1))
+    else:
+        monkeypatch.setattr(eso2, "_block", failing(eso2._block, 1))
+    calls = []
+    run_call = eso2._abi_forward if entry == "edge_conv" else eso2._block_vjp
+    monkeypatch.setattr(eso2, run_call.__name__, lambda *a, **k: (calls.append(1), run_call(*a, **k))[1])
+    got = run()
+    assert failed and len(calls) == (2 if entry == "edge_conv" else 3)
+    for a, b in zip(got, want):
+        assert rel_l2(a, b) < 2e-6

@@ -134,7 +134,10 @@ class Plan:
         probe = 4096
         self.bytes_per_edge = max(1.0, (lib.zp_workspace_bytes(handle, 0, probe, 1)
                                         - lib.zp_workspace_bytes(handle, 0, 0, 1)) / probe)
-        self.total_memory = torch.cuda.get_device_properties(device).total_memory
+        # memory of the device, and what of it others than this process' allocator hold (as of the last
+        # time the driver was asked)
+        free, self.total_memory = torch.cuda.mem_get_info(device)
+        self.foreign = self.total_memory - free - torch.cuda.memory_reserved(device)
         self.lmax, self.mmax, self.c, self.h = lmax, mmax, c, h
 
     @classmethod
@@ -208,18 +211,32 @@ MAX_EDGES_PER_CALL: int | None = None
 def _edge_budget(plan: Plan, n: int, e: int) -> int:
     if MAX_EDGES_PER_CALL is not None:
         return max(1, MAX_EDGES_PER_CALL)
-    free, _total = torch.cuda.mem_get_info(plan.device)
+    free, total = torch.cuda.mem_get_info(plan.device)
+    plan.foreign = total - free - torch.cuda.memory_reserved(plan.device)
     # memory the caching allocator holds but is not using can be re-used for the workspace
-    free += torch.cuda.memory_reserved(plan.device) - torch.cuda.memory_allocated(plan.device)
+    free += torch.cuda.memory_reserved(plan.device) - _allocated(plan.device)
     return _quantise_budget(max(1024, int(0.5 * free / plan.bytes_per_edge)))
 
 
-def _surely_fits(plan: Plan, e: int) -> bool:
-    """Whether ``e`` edges take so little of the device's memory (an eighth, gradients included)
-    that a call is made in one piece without asking how much is free, a question that costs the
-    host more than a small call's launches.  A call that runs out of memory all the same is made
-    again in pieces."""
-    return MAX_EDGES_PER_CALL is None and 16 * e * plan.bytes_per_edge <= plan.total_memory
+def _allocated(device: torch.device) -> int:
+    """``torch.cuda.memory_allocated`` at a seventh of its time (8 us)."""
+    return torch._C._cuda_memoryStats(device.index)["allocated_bytes"]["all"]["current"]
+
+
+def _one_piece(plan: Plan, e: int, kept: bool, share: int) -> bool:
+    """Whether ``e`` edges are made one call without asking the driver how much memory is free, which
+    costs one to five milliseconds.  A call that leaves nothing behind (``kept`` false) is if it takes
+    a sixteenth of the device's memory at most, gradients included: should that not be there, the
+    allocation fails and the caller goes on in pieces.  One whose activations stay until its backward
+    has to leave memory to what follows: like ``_edge_budget``'s, its share (with ``share`` = 2 a half)
+    is of what this process has not allocated of the device, less what others held when the driver
+    was last asked.  Below a 512th of the device's memory that is not looked up either."""
+    need = e * plan.bytes_per_edge
+    if MAX_EDGES_PER_CALL is not None or 16 * need > plan.total_memory:
+        return False
+    if not kept or 512 * need <= plan.total_memory:
+        return True
+    return share * need <= plan.total_memory - plan.foreign - _allocated(plan.device)
 
 
 def _quantise_budget(budget: int) -> int:
@@ -326,10 +343,16 @@ class EdgeConvFunction(torch.autograd.Function):
         wstruct, keep = _weights_struct(mmax, w10, b10, wms[:mmax], w20, b20, wms[mmax:])
         with torch.cuda.device(x.device):
             # a node-range graph is already one piece of a chunked run: never split it again
-            chunks = ([EdgeChunk(0, e, 0, n, graph)] if rng is not None or _surely_fits(plan, e)
+            chunks = ([EdgeChunk(0, e, 0, n, graph)] if rng is not None or _one_piece(plan, e, needs_bwd, 2)
                       else graph.chunks(_edge_budget(plan, n, e)))
             if len(chunks) == 1:
-                ws = plan.workspace(n1 - n0, e, needs_bwd, inference=not needs_bwd, edge_channels=ec)
+                try:
+                    ws = plan.workspace(n1 - n0, e, needs_bwd, inference=not needs_bwd, edge_channels=ec)
+                except torch.cuda.OutOfMemoryError:
+                    chunks = [] if rng is not None else graph.chunks(_edge_budget(plan, n, e))
+                    if len(chunks) < 2:
+                        raise
+            if len(chunks) == 1:
                 _abi_forward(plan, n1 - n0, e, x, ev, cg, sg, rad, en, graph.src, graph.dst,
                              graph.row_ptr[n0:], wstruct, out, ws, inference=not needs_bwd,
                              layer=layer)
@@ -1057,7 +1080,7 @@ class ESO2Block(nn.Module):
 
     def _evaluate(self, function, pos, atomic_numbers, x_node, edge_index, shifts, cos_gamma_k,
                   sin_gamma_k, graph, x_ready=None) -> torch.Tensor:
-        """``function`` (node_out or energy) of a call, in one piece if it surely fits."""
+        """``function`` (node_out or energy) of a call, in one piece if it fits."""
         check = None
         if graph is None:
             # new input: node indices and element numbers are range-checked (a caller that passes
@@ -1070,7 +1093,7 @@ class ESO2Block(nn.Module):
             params = [params]
         try:
             out = None
-            if params is not None and _surely_fits(plan, graph.n_edges):
+            if params is not None and _one_piece(plan, graph.n_edges, torch.is_grad_enabled(), 4):
                 try:
                     out = function.apply(self, plan, graph, None, atomic_numbers, shifts,
                                          cos_gamma_k, sin_gamma_k, x_ready, pos, x_node, *params)
@@ -1128,10 +1151,16 @@ class ESO2Block(nn.Module):
         if graph is None:
             graph = EdgeGraph.build(edge_index, n)
         plan = self.plan(pos.device)
-        if _surely_fits(plan, graph.n_edges):
-            chunks = [EdgeChunk(0, graph.n_edges, 0, n, graph)]
-        else:
-            chunks = graph.chunks(max(1024, _edge_budget(plan, n, graph.n_edges) // 2))
+        args = (graph, plan, pos, x_node, (atomic_numbers, shifts, cos_gamma_k, sin_gamma_k), upstream)
+        if _one_piece(plan, graph.n_edges, False, 4):
+            try:                               # (out of memory: all of it again, ``upstream`` too)
+                return self._vjp_sweep([EdgeChunk(0, graph.n_edges, 0, n, graph)], *args)
+            except torch.cuda.OutOfMemoryError:
+                pass
+        return self._vjp_sweep(graph.chunks(max(1024, _edge_budget(plan, n, graph.n_edges) // 2)), *args)
+
+    def _vjp_sweep(self, chunks, graph, plan, pos, x_node, args, upstream):
+        atomic_numbers, *per_edge = args
         params = list(self.parameters())
         total = None
         outs = []
@@ -1140,8 +1169,7 @@ class ESO2Block(nn.Module):
             pos_ = pos.detach().requires_grad_(True)
             x_ = x_node.detach().requires_grad_(True)
             with torch.enable_grad():
-                rows = self._edges_to_nodes(plan, c.sub, sub_perm, pos_, atomic_numbers, x_,
-                                            shifts, cos_gamma_k, sin_gamma_k)
+                rows = self._edges_to_nodes(plan, c.sub, sub_perm, pos_, atomic_numbers, x_, *per_edge)
             g_rows = (upstream(rows.detach(), c.n0, c.n1) if callable(upstream)
                       else upstream[c.n0:c.n1])
             grads = torch.autograd.grad(rows, [x_, pos_, *params], g_rows, allow_unused=True)
