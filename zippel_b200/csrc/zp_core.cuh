@@ -120,16 +120,17 @@ struct ZpWorkspace {
 ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *base, int ec,
                      ZpFormat rad);
 
-// One convolution call.  Per-edge arrays are in the sorted order.
 // The caller's stream plus the plan's two side streams for one forward / backward call.  Up to
 // kZpLaneEdges edges everything stays on the caller's: the kernels are then shorter than the host
-// takes to launch them, and every event makes it take longer.
+// takes to launch them, and every event makes it take longer.  However a call ends, the caller's stream
+// goes on behind whatever the side streams have been given: they work in the caller's memory.
 constexpr int64_t kZpLaneEdges = 4096;
 bool zp_lanes_enabled();
 struct ZpLanes {
   const zp_plan *p;
   cudaStream_t main;
   bool on;
+  int open = 0;                          // side streams forked and not joined yet, a bit each
   std::unique_lock<std::mutex> hold;
   ZpLanes(const zp_plan *plan, int64_t edges, cudaStream_t st)
       : p(plan), main(st),
@@ -143,7 +144,10 @@ struct ZpLanes {
     if (!on) return ZP_OK;
     ZP_CUDA(cudaEventRecord(p->ev_fork, main));
     for (int i = 0; i < 2; ++i)
-      if (which >> i & 1) ZP_CUDA(cudaStreamWaitEvent(p->aux_stream[i], p->ev_fork, 0));
+      if (which >> i & 1) {
+        open |= 1 << i;
+        ZP_CUDA(cudaStreamWaitEvent(p->aux_stream[i], p->ev_fork, 0));
+      }
     return ZP_OK;
   }
   // the caller's stream continues after everything the side streams have been given
@@ -153,11 +157,19 @@ struct ZpLanes {
       if (!(which >> i & 1)) continue;
       ZP_CUDA(cudaEventRecord(p->ev_join[i], p->aux_stream[i]));
       ZP_CUDA(cudaStreamWaitEvent(main, p->ev_join[i], 0));
+      open &= ~(1 << i);
     }
     return ZP_OK;
   }
+  ~ZpLanes() {                           // an error left the call between fork and join
+    for (int i = 0; i < 2; ++i)
+      if ((open >> i & 1) && (cudaEventRecord(p->ev_join[i], p->aux_stream[i]) != cudaSuccess ||
+                              cudaStreamWaitEvent(main, p->ev_join[i], 0) != cudaSuccess))
+        cudaGetLastError();              // the error that is reported is the first one
+  }
 };
 
+// One convolution call.  Per-edge arrays are in the sorted order.
 struct ZpConv {
   int64_t N, E;
   const float *x_node, *edge_vec, *cos_g, *sin_g, *radial, *env;
