@@ -313,3 +313,52 @@ def test_out_of_memory_in_one_piece_goes_on_in_chunks(entry, monkeypatch):
     assert failed and len(calls) == (2 if entry == "edge_conv" else 3)
     for a, b in zip(got, want):
         assert rel_l2(a, b) < 2e-6
+
+
+@pytest.mark.parametrize("lmax,mmax,e", [(2, 1, 130), (3, 3, 300), (4, 2, 129), (6, 6, 140), (6, 1, 60)])
+@pytest.mark.parametrize("what", ["bf16", "some", "unused", "scaled"])
+def test_roll_angle_harmonics_are_taken_as_they_are(what, lmax, mmax, e, jd64):
+    """Harmonics that are not cos(k g), sin(k g) of one angle (rounded to 16 bits, or a few edges' not of
+    one angle at all, or scaled), and orders above mmax that the forward never reads: the gradient is
+    that of the forward with the arrays as given."""
+    cfg = dict(lmax=lmax, mmax=mmax, sphere_channels=40, hidden_channels=8, edge_channels=8,
+               num_distance_basis=6, cutoff=8.0)
+    params = orc.init_params(cfg, seed=lmax)
+    case = random_case(cfg, 11, e, seed=mmax)
+    for key in ("cos_gamma_k", "sin_gamma_k"):
+        g = torch.Generator("cpu").manual_seed(len(key))
+        h = case[key]
+        if what == "bf16":
+            h = h.bfloat16().double()
+        elif what == "some":
+            h[::7, 1:] = torch.randn(h[::7, 1:].shape, generator=g).float().double()
+        elif what == "unused":
+            h[:, mmax + 1:] = 0.0
+        else:
+            h[:, 1:] *= 1.01
+        case[key] = h.float().double()
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    check_against(*gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"]), *want)
+
+
+@pytest.mark.parametrize("lmax,mmax", [(6, 6), (2, 2)])
+def test_whole_blocks_of_polar_edges(lmax, mmax, jd64):
+    """More edges along the polar axis than a block forms the entries of at a time, next to others."""
+    cfg = dict(lmax=lmax, mmax=mmax, sphere_channels=16, hidden_channels=8, edge_channels=8,
+               num_distance_basis=6, cutoff=8.0)
+    params = orc.init_params(cfg, seed=5)
+    n = 60
+    case = random_case(cfg, n, 200, seed=6)
+    case["pos"], case["shifts"] = case["pos"].float().double(), torch.zeros_like(case["shifts"])
+    for e in range(90):                                   # pairs of atoms that only these edges touch
+        i = e % 15 * 2
+        case["edge_index"][:, e] = torch.tensor([i, i + 1])
+        case["pos"][i + 1] = case["pos"][i] + torch.tensor([0.0, 1.0 + 0.03125 * i, 0.0])
+    for e in range(90, 200):
+        i, j = case["edge_index"][:, e].tolist()
+        i, j = 30 + i % 30, 30 + j % 30
+        case["edge_index"][:, e] = torch.tensor([i, j if j != i else 30 + (i - 29) % 30])
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    got = gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"])
+    assert rel_l2(got[0], want[0]) < 1e-5
+    assert rel_l2(got[2][30:], want[2][30:]) < 1e-5 and rel_l2(got[2][:30], want[2][:30]) < 1e-3

@@ -120,6 +120,7 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
     w.da1 = c.floats(e * t.Km * 2 * t.C);
     w.du_src = c.floats(e * 2 * t.K * t.C);
     w.torque = c.floats(e * 4);
+    w.rot_grad = t.Km * t.H >= t.nnz_pad ? w.dht : c.floats(e * t.nnz_pad);
     w.wgrad = c.floats((size_t)kZpWgradSplits * p->g_elems);
     auto column_parts = [&](int64_t cols) { return c.floats((size_t)(zp_colsum_parts(E, cols) * cols)); };
     w.col1 = column_parts(p->c1_out[0]);
@@ -807,7 +808,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   ZP_TIMED(ZP_K_WIGNER_BWD,
            zp_launch_edge_vec_grad(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.torque,
                                    ZpTorqueArgs{ws.da1, radial, c.x_node, ws.y, grad_node_out, c.env,
-                                                ws.rot, c.src, c.dst},
+                                                c.src, c.dst, ws.rot_grad},
                                    grad_edge_vec, st));
   return ZP_OK;
 }

@@ -238,8 +238,9 @@ int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const flo
 // torque [E, 4]: for each edge the derivative of the loss under a rotation of the edge frame about
 // its own axis (entry 0) and the two axes perpendicular to it (1, 2).
 struct ZpTorqueArgs {
-  const float *da1, *radial, *x, *y, *g_out, *env, *rot;
+  const float *da1, *radial, *x, *y, *g_out, *env;
   const int32_t *src, *dst;
+  float *entries;                        // [E, nnz_pad] scratch: gradient of the rotation entries
 };
 // torque -> gradient of the edge vectors
 int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const float *cg,

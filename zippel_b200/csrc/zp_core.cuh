@@ -106,6 +106,7 @@ inline int zp_radial_splits(int64_t N, int64_t K) {
 // mode 2: forward alone with fused epilogues -- of h1 only the gate scalars exist, y does not.
 struct ZpWorkspace {
   float *rot, *h1, *y, *dht, *da1, *du_src, *torque, *wgrad, *scales, *head, *cont;
+  float *rot_grad;                       // [E, nnz_pad], in dht's place where it fits: that is read by then
   float *col1, *col2, *col_rad;          // partial column sums: bias gradients of conv1, conv2, radial
   float *radial, *rad_partials;          // radial layer inside the call: its output, dW partials
   int64_t ld_h1;

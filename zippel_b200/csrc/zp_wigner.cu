@@ -112,68 +112,65 @@ struct ForEachL<-1, LMAX> {
                                              double *) {}
 };
 
-// Reverse of block_forward: accumulates the cotangents of cos/sin(k beta), cos/sin(k alpha).
+// Reverse of block_column: adds column j's cotangents of cos/sin(k beta), cos/sin(k alpha).
 template <int L, int LMAX>
-__device__ __forceinline__ void block_backward(const ZpTables &t, const double *__restrict__ J,
+__device__ __forceinline__ void column_backward(const ZpTables &t, const double *__restrict__ J,
                                                const Frame<LMAX> &f, const double *cg,
-                                               const double *sg, const float *g_e, double *dcb,
-                                               double *dsb, double *dca, double *dsa) {
+                                               const double *sg, const float *g_e, int j,
+                                                double *dcb, double *dsb, double *dca, double *dsa) {
   constexpr int n = 2 * L + 1;
   const int mm = t.mmax < L ? t.mmax : L;
-#pragma unroll 1
-  for (int j = 0; j < n; ++j) {
-    const int dj = j > L ? j - L : L - j;
-    const double c1 = f.ca[dj];
-    const double s1 = j > L ? -f.sa[dj] : (j < L ? f.sa[dj] : 0.0);
-    double P[n];
+  const int dj = j > L ? j - L : L - j;
+  const double c1 = f.ca[dj];
+  const double s1 = j > L ? -f.sa[dj] : (j < L ? f.sa[dj] : 0.0);
+  double P[n];
 #pragma unroll
-    for (int i = 0; i < n; ++i) P[i] = J[i * n + j] * c1 + J[i * n + (n - 1 - j)] * s1;
-    // G = dL/dD column j (zero outside the kept rows);  dM = Xa^T G
-    double G[n], dM[n];
+  for (int i = 0; i < n; ++i) P[i] = J[i * n + j] * c1 + J[i * n + (n - 1 - j)] * s1;
+  // G = dL/dD column j (zero outside the kept rows);  dM = Xa^T G
+  double G[n], dM[n];
 #pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const int di = i > L ? i - L : L - i;
-      G[i] = di <= mm ? (double)g_e[t.rot_off[t.row_of[L][i]] + j] : 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < n; ++k) {
-      const int dk = k > L ? k - L : L - k;
-      // Xa[n-1-k, k] is the anti-diagonal entry of row n-1-k
-      dM[k] = dk <= mm ? cg[dk] * G[k] + anti<L>(sg, n - 1 - k) * G[n - 1 - k] : 0.0;
-    }
-    // dN = J^T dM (J symmetric in exact arithmetic; transpose written out regardless)
-    double dN[n];
-#pragma unroll
-    for (int k = 0; k < n; ++k) {
-      double acc = 0.0;
-#pragma unroll
-      for (int i = 0; i < n; ++i) {
-        const int di = i > L ? i - L : L - i;
-        if (di <= mm) acc += J[i * n + k] * dM[i];
-      }
-      dN[k] = acc;
-    }
-    // N = Xb P:  cotangents of the beta harmonics, and dP = Xb^T dN
-    double dP[n];
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      const int di = i > L ? i - L : L - i;
-      dcb[di] += dN[i] * P[i];
-      if (i < L) dsb[di] -= dN[i] * P[n - 1 - i];
-      if (i > L) dsb[di] += dN[i] * P[n - 1 - i];
-      dP[i] = f.cb[di] * dN[i] + anti<L>(f.sb, n - 1 - i) * dN[n - 1 - i];
-    }
-    // P = J Xc:  column j of Xc holds cos at row j and the signed sin at row n-1-j
-    double acc_c = 0.0, acc_s = 0.0;
-#pragma unroll
-    for (int i = 0; i < n; ++i) {
-      acc_c += J[i * n + j] * dP[i];
-      acc_s += J[i * n + (n - 1 - j)] * dP[i];
-    }
-    dca[dj] += acc_c;
-    if (j > L) dsa[dj] -= acc_s;
-    if (j < L) dsa[dj] += acc_s;
+  for (int i = 0; i < n; ++i) {
+    const int di = i > L ? i - L : L - i;
+    G[i] = di <= mm ? (double)g_e[t.rot_off[t.row_of[L][i]] + j] : 0.0;
   }
+#pragma unroll
+  for (int k = 0; k < n; ++k) {
+    const int dk = k > L ? k - L : L - k;
+    // Xa[n-1-k, k] is the anti-diagonal entry of row n-1-k
+    dM[k] = dk <= mm ? cg[dk] * G[k] + anti<L>(sg, n - 1 - k) * G[n - 1 - k] : 0.0;
+  }
+  // dN = J^T dM (J symmetric in exact arithmetic; transpose written out regardless)
+  double dN[n];
+#pragma unroll
+  for (int k = 0; k < n; ++k) {
+    double acc = 0.0;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const int di = i > L ? i - L : L - i;
+      if (di <= mm) acc += J[i * n + k] * dM[i];
+    }
+    dN[k] = acc;
+  }
+  // N = Xb P:  cotangents of the beta harmonics, and dP = Xb^T dN
+  double dP[n];
+#pragma unroll
+  for (int i = 0; i < n; ++i) {
+    const int di = i > L ? i - L : L - i;
+    dcb[di] += dN[i] * P[i];
+    if (i < L) dsb[di] -= dN[i] * P[n - 1 - i];
+    if (i > L) dsb[di] += dN[i] * P[n - 1 - i];
+    dP[i] = f.cb[di] * dN[i] + anti<L>(f.sb, n - 1 - i) * dN[n - 1 - i];
+  }
+  // P = J Xc:  column j of Xc holds cos at row j and the signed sin at row n-1-j
+  double acc_c = 0.0, acc_s = 0.0;
+#pragma unroll
+  for (int i = 0; i < n; ++i) {
+    acc_c += J[i * n + j] * dP[i];
+    acc_s += J[i * n + (n - 1 - j)] * dP[i];
+  }
+  dca[dj] += acc_c;
+  if (j > L) dsa[dj] -= acc_s;
+  if (j < L) dsa[dj] += acc_s;
 }
 
 template <int L, int LMAX>
@@ -183,7 +180,9 @@ __device__ __forceinline__ void ForEachL<L, LMAX>::bwd(const ZpTables &t, const 
                                                        double *dcb, double *dsb, double *dca,
                                                        double *dsa) {
   ForEachL<L - 1, LMAX>::bwd(t, J, f, cg, sg, g_e, dcb, dsb, dca, dsa);
-  block_backward<L, LMAX>(t, J + t.jd_off[L], f, cg, sg, g_e, dcb, dsb, dca, dsa);
+#pragma unroll 1
+  for (int j = 0; j < 2 * L + 1; ++j)
+    column_backward<L, LMAX>(t, J + t.jd_off[L], f, cg, sg, g_e, j, dcb, dsb, dca, dsa);
 }
 
 template <int L, int LMAX>
@@ -261,23 +260,13 @@ wigner_fwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__
   }
 }
 
-// VJP of one edge's rotation, step by step through the construction above.  g_e: packed layout.
+// What an edge's cotangents of the harmonics add up to in its vector.
 template <int LMAX>
-__device__ __noinline__ void chain_backward(const ZpTables &t, const double *__restrict__ J,
-                                            const float *ev, const float *cgam, const float *sgam,
-                                            const float *g_e, float *gev) {
-  Frame<LMAX> f;
-  frame_forward<LMAX>(f, ev);
-  double cg[LMAX + 1], sg[LMAX + 1];
-  double dcb[LMAX + 1], dsb[LMAX + 1], dca[LMAX + 1], dsa[LMAX + 1], du[LMAX + 1];
+__device__ __forceinline__ void frame_backward(const Frame<LMAX> &f, double *dcb, const double *dsb,
+                                               double *dca, double *dsa, float *gev) {
+  double du[LMAX + 1];
 #pragma unroll
-  for (int k = 0; k <= LMAX; ++k) {
-    cg[k] = cgam[k];
-    sg[k] = sgam[k];
-    dcb[k] = dsb[k] = dca[k] = dsa[k] = du[k] = 0.0;
-  }
-  ForEachL<LMAX, LMAX>::bwd(t, J, f, cg, sg, g_e, dcb, dsb, dca, dsa);
-
+  for (int k = 0; k <= LMAX; ++k) du[k] = 0.0;
   // sin(k beta) = r * U_{k-1}(y)
   double dr = 0.0, dy = 0.0;
 #pragma unroll
@@ -318,6 +307,74 @@ __device__ __noinline__ void chain_backward(const ZpTables &t, const double *__r
   gev[2] = (float)(dz * f.inv_norm + 2.0 * f.v[2] * dn2);
 }
 
+// VJP of one edge's rotation, step by step through the construction above.  g_e: packed layout.
+template <int LMAX>
+__device__ __noinline__ void chain_backward(const ZpTables &t, const double *__restrict__ J,
+                                            const float *ev, const float *cgam, const float *sgam,
+                                            const float *g_e, float *gev) {
+  Frame<LMAX> f;
+  frame_forward<LMAX>(f, ev);
+  double cg[LMAX + 1], sg[LMAX + 1];
+  double dcb[LMAX + 1], dsb[LMAX + 1], dca[LMAX + 1], dsa[LMAX + 1];
+#pragma unroll
+  for (int k = 0; k <= LMAX; ++k) {
+    cg[k] = cgam[k];
+    sg[k] = sgam[k];
+    dcb[k] = dsb[k] = dca[k] = dsa[k] = 0.0;
+  }
+  ForEachL<LMAX, LMAX>::bwd(t, J, f, cg, sg, g_e, dcb, dsb, dca, dsa);
+  frame_backward<LMAX>(f, dcb, dsb, dca, dsa, gev);
+}
+// The same by a warp, its lanes taking the columns (l, j).
+template <int L, int LMAX>
+struct ColumnBackward {
+  static __device__ __forceinline__ void run(const ZpTables &t, const double *J, const Frame<LMAX> &f,
+                                             const double *cg, const double *sg, const float *g_e, int l,
+                                             int j, double *dcb, double *dsb, double *dca, double *dsa) {
+    if (l == L) column_backward<L, LMAX>(t, J + t.jd_off[L], f, cg, sg, g_e, j, dcb, dsb, dca, dsa);
+    else ColumnBackward<L - 1, LMAX>::run(t, J, f, cg, sg, g_e, l, j, dcb, dsb, dca, dsa);
+  }
+};
+template <int LMAX>
+struct ColumnBackward<-1, LMAX> {
+  static __device__ __forceinline__ void run(const ZpTables &, const double *, const Frame<LMAX> &,
+                                             const double *, const double *, const float *, int, int,
+                                             double *, double *, double *, double *) {}
+};
+template <int LMAX>
+__device__ __noinline__ void chain_backward_warp(const ZpTables &t, const double *__restrict__ J,
+                                                 const float *ev, const float *cgam, const float *sgam,
+                                                 const float *g_e, float *gev) {
+  const int lane = threadIdx.x % 32;
+  Frame<LMAX> f;
+  frame_forward<LMAX>(f, ev);
+  double cg[LMAX + 1], sg[LMAX + 1];
+  double dcb[LMAX + 1], dsb[LMAX + 1], dca[LMAX + 1], dsa[LMAX + 1];
+#pragma unroll
+  for (int k = 0; k <= LMAX; ++k) {
+    cg[k] = cgam[k];
+    sg[k] = sgam[k];
+    dcb[k] = dsb[k] = dca[k] = dsa[k] = 0.0;
+  }
+#pragma unroll 1
+  for (int col = lane; col < t.K; col += 32) {
+    int l = 0;
+    while ((l + 1) * (l + 1) <= col) ++l;
+    ColumnBackward<LMAX, LMAX>::run(t, J, f, cg, sg, g_e, l, col - l * l, dcb, dsb, dca, dsa);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k <= LMAX; ++k)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      dcb[k] += __shfl_xor_sync(0xffffffffu, dcb[k], o);
+      dsb[k] += __shfl_xor_sync(0xffffffffu, dsb[k], o);
+      dca[k] += __shfl_xor_sync(0xffffffffu, dca[k], o);
+      dsa[k] += __shfl_xor_sync(0xffffffffu, dsa[k], o);
+    }
+  if (lane == 0) frame_backward<LMAX>(f, dcb, dsb, dca, dsa, gev);
+}
+
 template <int LMAX>
 __global__ void __launch_bounds__(128)
 wigner_bwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
@@ -333,12 +390,78 @@ wigner_bwd_kernel(const __grid_constant__ ZpTables t, const double *__restrict__
 
 // The rotation of an edge frame depends on the edge's direction only, so its VJP needs no more than
 // the three derivatives under rotations of the frame, which the kernels that hold the rows form on
-// the way (torque; zp_rotate.cu):  with v = |v| (sin b sin a, cos b, sin b cos a), roll angle g,
+// the way (torque; zp_rotate_bwd.cu):  with v = |v| (sin b sin a, cos b, sin b cos a), roll angle g,
 //   dL/db = cos g T1 + sin g T2,    dL/da = sin b (sin g T1 - cos g T2) + cos b T0,
 //   grad v = ( dL/db e_b + dL/da / sin b  e_a ) / |v|.
-// An edge along the polar axis (sin^2 b below the floor of the construction) has no proper rotation
-// and goes through the construction step by step: its warp forms the gradient of every rotation
-// entry from the saved rows.  A crystal without displacements has a few such edges per atom.
+// Two kinds of edges have no proper rotation and go through the construction step by step, from the
+// gradient of every rotation entry: those along the polar axis (sin^2 b below the floor of the
+// construction; a few per atom in a crystal without displacements) and those whose roll-angle
+// harmonics are not cos(k g), sin(k g) of one angle, k up to mmax + 1 (rounded to 16 bits, say).
+// A block lists its own such edges and its warps form the entries of one each, row by row.  A few of them
+// then run the construction by a warp, its lanes taking the columns; from kFewSteps on by a thread each, all
+// at the same time.  Forces of 256 fcc atoms (19 968 edges, lmax 4, 2.40 ms): undisplaced 2.49 ms (2.60
+// with one lane taking one edge after the other), every edge's harmonics rounded 3.98 (4.70 with a warp
+// per edge throughout).
+constexpr int kFewSteps = 8;
+constexpr double kHarmonicSlack = 4e-6;      // 32 units in the last place of 1: fp32 recurrences pass
+template <int LMAX>
+__device__ __forceinline__ bool one_angle(const float *cgam, const float *sgam, int top) {
+  if constexpr (LMAX == 0) return true;
+  const double c1 = cgam[1], s1 = sgam[1];
+  double worst = fabs(c1 * c1 + s1 * s1 - 1.0), c = c1, s = s1;
+#pragma unroll
+  for (int k = 2; k <= LMAX; ++k) {
+    const double cn = c1 * c - s1 * s;
+    s = s1 * c + c1 * s;
+    c = cn;
+    if (k <= top) worst = fmax(worst, fmax(fabs(cgam[k] - c), fabs(sgam[k] - s)));
+  }
+  return worst <= kHarmonicSlack;
+}
+// The gradient of the 2l + 1 entries of one row, by a warp: unrolled per degree, so that the rows of the
+// nodes are requested together.
+template <int L>
+struct RowEntries {
+  static __device__ __forceinline__ void run(int l, int C, int lane, float env, const float *da,
+                                             const float *rad, const float *y, const float *xs,
+                                             const float *xd, const float *g, float *out) {
+    if (l != L) return RowEntries<L - 1>::run(l, C, lane, env, da, rad, y, xs, xd, g, out);
+    constexpr int n = 2 * L + 1;
+    float in[n];
+#pragma unroll
+    for (int j = 0; j < n; ++j) in[j] = 0.f;
+    for (int c = 4 * lane; c < C; c += 128) {            // channel counts are multiples of 8
+      auto at = [&](const float *p) { return *reinterpret_cast<const float4 *>(p + c); };
+      auto mul = [](const float4 &u, const float4 &v) { return make_float4(u.x * v.x, u.y * v.y, u.z * v.z, u.w * v.w); };
+      auto dot = [](const float4 &u, const float4 &v) { return (u.x * v.x + u.y * v.y) + (u.z * v.z + u.w * v.w); };
+      const float4 ps = mul(at(da), at(rad)), pd = mul(at(da + C), at(rad + C));
+      const float4 py = mul(at(y), make_float4(env, env, env, env));
+      float4 u[n];
+      const float4 *const p[3] = {&ps, &pd, &py};
+      const float *const rows[3] = {xs, xd, g};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int j = 0; j < n; ++j) u[j] = at(rows[k] + (L * L + j) * C);
+#pragma unroll
+        for (int j = 0; j < n; ++j) in[j] += dot(*p[k], u[j]);
+      }
+    }
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1)
+#pragma unroll
+      for (int j = 0; j < n; ++j) in[j] += __shfl_xor_sync(0xffffffffu, in[j], k);
+    if (lane == 0) {
+#pragma unroll
+      for (int j = 0; j < n; ++j) out[j] = in[j];
+    }
+  }
+};
+template <>
+struct RowEntries<-1> {
+  static __device__ __forceinline__ void run(int, int, int, float, const float *, const float *, const float *,
+                                             const float *, const float *, const float *, float *) {}
+};
 template <int LMAX>
 __global__ void __launch_bounds__(128)
 edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
@@ -346,17 +469,19 @@ edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restric
                      const float *__restrict__ sgam, const float4 *__restrict__ torque,
                      const ZpTorqueArgs a, float *__restrict__ gev) {
   zp_after_previous();
-  extern __shared__ float grads[];                      // [4 warps][nnz_pad]
+  __shared__ int steps[128], found[4];
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int64_t e = (int64_t)blockIdx.x * 128 + threadIdx.x;
-  bool pole = false;
+  const int64_t e0 = (int64_t)blockIdx.x * 128, e = e0 + threadIdx.x;
+  bool step = false;
   if (e < E) {
     const double x = ev[3 * e], y = ev[3 * e + 1], z = ev[3 * e + 2];
     const double n2 = x * x + y * y + z * z;
     const double inv = rsqrt(fmax(n2, kS2Floor));
     const double xh = x * inv, yh = y * inv, zh = z * inv, s2 = xh * xh + zh * zh;
-    pole = LMAX >= 1 && !(n2 >= kS2Floor && s2 >= kS2Floor);
-    if (!pole) {
+    const int top = t.mmax + 1;
+    step = LMAX >= 1 && !(n2 >= kS2Floor && s2 >= kS2Floor &&
+                          one_angle<LMAX>(cgam + e * (LMAX + 1), sgam + e * (LMAX + 1), top));
+    if (!step) {
       double gx = 0.0, gy = 0.0, gz = 0.0;
       if constexpr (LMAX >= 1) {
         const float4 T = torque[e];
@@ -372,36 +497,38 @@ edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restric
       gev[3 * e + 2] = (float)gz;
     }
   }
-  float *g_s = grads + warp * t.nnz_pad;
-  for (unsigned todo = __ballot_sync(0xffffffffu, pole); todo; todo &= todo - 1) {
-    const int who = __ffs(todo) - 1;
-    const int64_t q = (int64_t)blockIdx.x * 128 + warp * 32 + who;
-    const int C = t.C, C2 = 2 * t.C;
-    const float *xs = a.x + (size_t)a.src[q] * t.K * C, *xd = a.x + (size_t)a.dst[q] * t.K * C;
-    const float *g = a.g_out + (size_t)a.dst[q] * t.K * C;
+  const int total = __syncthreads_count(step);
+  if (total == 0) return;
+  const unsigned mine = __ballot_sync(0xffffffffu, step);
+  if (lane == 0) found[warp] = __popc(mine);
+  __syncthreads();
+  int before = __popc(mine & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) before += found[w];
+  if (step) steps[before] = threadIdx.x;
+  __syncthreads();
+  const int C = t.C, C2 = 2 * t.C;
+  for (int q = warp; q < total; q += 4) {
+    const int64_t i = e0 + steps[q];
+    const float *xs = a.x + (size_t)a.src[i] * t.K * C, *xd = a.x + (size_t)a.dst[i] * t.K * C;
+    const float *g = a.g_out + (size_t)a.dst[i] * t.K * C;
+    float *entries = a.entries + (size_t)i * t.nnz_pad;
+    const float env = a.env[i];
     for (int r = 0; r < t.Km; ++r) {
       const int l = t.row_l[r], m = t.row_m[r], am = m < 0 ? -m : m;
-      const float *da = a.da1 + ((size_t)q * t.Km + r) * C2;
-      const float *rad = a.radial + (size_t)q * t.R + t.rad_off[am] + (l - am) * C2;
-      const float *yr = a.y + ((size_t)q * t.Km + r) * C;
-      for (int j = 0; j < 2 * l + 1; ++j) {
-        const size_t o = (size_t)(l * l + j) * C;
-        float in = 0.f, back = 0.f;
-        for (int c = lane; c < C; c += 32) {
-          in += da[c] * rad[c] * xs[o + c] + da[C + c] * rad[C + c] * xd[o + c];
-          back += yr[c] * g[o + c];
-        }
-        in += a.env[q] * back;
-#pragma unroll
-        for (int k = 16; k > 0; k >>= 1) in += __shfl_xor_sync(0xffffffffu, in, k);
-        if (lane == 0) g_s[t.rot_off[r] + j] = in;
-      }
+      RowEntries<LMAX>::run(l, C, lane, env, a.da1 + ((size_t)i * t.Km + r) * C2,
+                            a.radial + (size_t)i * t.R + t.rad_off[am] + (l - am) * C2,
+                            a.y + ((size_t)i * t.Km + r) * C, xs, xd, g, entries + t.rot_off[r]);
     }
-    __syncwarp();
-    if (lane == who)
-      chain_backward<LMAX>(t, J, ev + 3 * q, cgam + q * (LMAX + 1), sgam + q * (LMAX + 1), g_s, gev + 3 * q);
-    __syncwarp();
+    if (total <= kFewSteps) {
+      __syncwarp();
+      chain_backward_warp<LMAX>(t, J, ev + 3 * i, cgam + i * (LMAX + 1), sgam + i * (LMAX + 1), entries, gev + 3 * i);
+    }
   }
+  if (total <= kFewSteps) return;
+  __syncthreads();
+  if (step)
+    chain_backward<LMAX>(t, J, ev + 3 * e, cgam + e * (LMAX + 1), sgam + e * (LMAX + 1),
+                         a.entries + (size_t)e * t.nnz_pad, gev + 3 * e);
 }
 
 }  // namespace
@@ -442,9 +569,8 @@ int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const 
                             cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const dim3 grid((unsigned)zp_ceil_div(E, 128)), block(128);
-  const size_t smem = (size_t)4 * p->t.nnz_pad * sizeof(float);
 #define CALL(LM)                                                                                  \
-  zp_launch(edge_vec_grad_kernel<LM>, grid, block, smem, st, p->t, p->jd_dev, E, ev, cg, sg,             \
+  zp_launch(edge_vec_grad_kernel<LM>, grid, block, 0, st, p->t, p->jd_dev, E, ev, cg, sg,             \
                                                       reinterpret_cast<const float4 *>(torque), a, gev)
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
