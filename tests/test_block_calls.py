@@ -220,3 +220,34 @@ def test_when_a_call_is_made_in_one_piece(monkeypatch):
     assert not eso2._one_piece(plan, edges(10), True, 2) and eso2._one_piece(plan, edges(10), False, 2)
     monkeypatch.setattr(eso2, "MAX_EDGES_PER_CALL", 64)
     assert not eso2._one_piece(plan, 8, False, 4)
+
+
+def test_the_flags_of_a_sort_are_waited_for_whatever_happens(fake, monkeypatch):
+    lib, block, case, graph = fake
+    checked = []
+    monkeypatch.setattr(block, "_sorted_edges", lambda *args: (graph, lambda: checked.append(1)))
+    for what in ("plan", "_call_params"):
+        with monkeypatch.context() as m:
+            m.setattr(block, what, lambda *args: 1 / 0)
+            with pytest.raises(ZeroDivisionError):
+                node_output(block, case, None, case["pos"], case["x_node"])
+    assert len(checked) == 2
+
+
+def test_host_tensors_are_refused_before_their_addresses_are_taken(monkeypatch):
+    """Each argument in turn is the only one not on the device (here: the only one said not to be)."""
+    block = eso2.ESO2Block(eso2.BlockConfig(**CFG))
+    seen = []
+    monkeypatch.setattr(eso2, "_need_cuda", lambda *tensors: seen.extend(tensors) or 1 / 0)
+    case = {key: v.float() if v.is_floating_point() else v for key, v in random_case(CFG, 9, 40, seed=1).items()}
+    csr = csr_reference(case["edge_index"].numpy(), 9)
+    graph = EdgeGraph(9, 40, **{key: torch.from_numpy(v) for key, v in csr.items()})
+    plan = types.SimpleNamespace(sizes=types.SimpleNamespace(K=9), c=8)
+    ctx = types.SimpleNamespace(needs_input_grad=(False,))
+    with pytest.raises(ZeroDivisionError):
+        eso2._block(ctx, block, plan, graph, None, case["atomic_numbers"], case["shifts"], case["cos_gamma_k"],
+                    case["sin_gamma_k"], None, case["pos"], case["x_node"], block._call_params(False))
+    at = {t.data_ptr() for t in seen}
+    assert {case[k].data_ptr() for k in ("pos", "x_node", "shifts", "atomic_numbers", "cos_gamma_k",
+                                         "sin_gamma_k")} <= at
+    assert block.gauss_offset.data_ptr() in at and {p.data_ptr() for p in block._call_params(False)} <= at

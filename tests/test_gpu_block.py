@@ -362,3 +362,10 @@ def test_whole_blocks_of_polar_edges(lmax, mmax, jd64):
     got = gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"])
     assert rel_l2(got[0], want[0]) < 1e-5
     assert rel_l2(got[2][30:], want[2][30:]) < 1e-5 and rel_l2(got[2][:30], want[2][:30]) < 1e-3
+
+
+def test_element_numbers_on_the_host_raise():
+    from zippel_b200.graph import EdgeGraph
+    with pytest.raises(RuntimeError):
+        EdgeGraph.build_checked(torch.zeros(2, 3, dtype=torch.int64, device="cuda"),
+                                torch.zeros(4, dtype=torch.int64), 5)

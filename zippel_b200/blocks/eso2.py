@@ -803,7 +803,7 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
     off = _as_f32(block.gauss_offset)
     if z.dtype != torch.int64 or not z.is_contiguous():
         z = z.to(torch.int64).contiguous()
-    _need_cuda(pos, x, shifts, z, *params)
+    _need_cuda(pos, x, shifts, z, cos_g, sin_g, off, *params)
     assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
     assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.shape == (n,)
     assert cos_g.shape[1] == cfg.lmax + 1 and sin_g.shape == cos_g.shape
@@ -1086,12 +1086,12 @@ class ESO2Block(nn.Module):
             # new input: node indices and element numbers are range-checked (a caller that passes
             # a prebuilt graph has had them checked when it was built)
             graph, check = self._sorted_edges(edge_index, atomic_numbers)
-        plan = self.plan(pos.device)
-        energy = function is EnergyFunction
-        params = self._call_params(energy)
-        if params is not None and not _differentiated(params):
-            params = [params]
         try:
+            plan = self.plan(pos.device)
+            energy = function is EnergyFunction
+            params = self._call_params(energy)
+            if params is not None and not _differentiated(params):
+                params = [params]
             out = None
             if params is not None and _one_piece(plan, graph.n_edges, torch.is_grad_enabled(), 4):
                 try:

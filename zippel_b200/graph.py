@@ -135,8 +135,11 @@ class EdgeGraph:
         """``build`` for a caller that goes on enqueueing work: returns ``(graph, check)``, and
         ``check()`` raises ``IndexError`` for a node index outside ``[0, N)`` or an element number
         outside ``[0, n_elements)``.  It waits for the sort alone, so work enqueued in between keeps
-        the device busy.  Not for use while the stream is being captured."""
+        the device busy.  To be called in any case, errors in between included: the flags arrive in
+        memory that it holds.  Not for use while the stream is being captured."""
         lib, ei, e, dev = EdgeGraph._open(edge_index)
+        if atomic_numbers.device != dev:
+            raise RuntimeError(f"atomic_numbers on {atomic_numbers.device}, edge_index on {dev}")
         z = atomic_numbers.to(torch.int64).contiguous()
         n = z.shape[0]
         graph = EdgeGraph.__new__(EdgeGraph)
