@@ -251,3 +251,13 @@ def test_host_tensors_are_refused_before_their_addresses_are_taken(monkeypatch):
     assert {case[k].data_ptr() for k in ("pos", "x_node", "shifts", "atomic_numbers", "cos_gamma_k",
                                          "sin_gamma_k")} <= at
     assert block.gauss_offset.data_ptr() in at and {p.data_ptr() for p in block._call_params(False)} <= at
+
+
+def test_element_numbers_as_a_column(fake):
+    """[N, 1], and more entries than atoms: the kernels read the first N."""
+    lib, block, case, graph = fake
+    for z in (case["atomic_numbers"][:, None], torch.cat([case["atomic_numbers"]] * 2)):
+        assert node_output(block, case, graph, case["pos"], case["x_node"], z).shape == case["x_node"].shape
+        assert lib.calls[-1][1][2].atomic_numbers == z.data_ptr()
+    with pytest.raises(AssertionError):
+        node_output(block, case, graph, case["pos"], case["x_node"], case["atomic_numbers"][:-1])

@@ -369,3 +369,19 @@ def test_element_numbers_on_the_host_raise():
     with pytest.raises(RuntimeError):
         EdgeGraph.build_checked(torch.zeros(2, 3, dtype=torch.int64, device="cuda"),
                                 torch.zeros(4, dtype=torch.int64), 5)
+
+
+def test_element_numbers_as_a_column():
+    cfg = dict(lmax=1, mmax=1, sphere_channels=8, hidden_channels=8, edge_channels=8,
+               num_distance_basis=4, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1))
+    case = random_case(cfg, 6, 20, seed=2)
+    want = gpu_node_out_and_vjp(block, case, case["upstream"])
+    column = dict(case, atomic_numbers=case["atomic_numbers"][:, None])
+    got = gpu_node_out_and_vjp(block, column, case["upstream"])
+    for a, b in zip((*got[:3], *got[3].values()), (*want[:3], *want[3].values())):
+        assert (a is None and b is None) or torch.equal(a, b)
+    column["atomic_numbers"] = column["atomic_numbers"].clone()
+    column["atomic_numbers"][2, 0] = block.cfg.max_num_elements
+    with pytest.raises(IndexError):
+        gpu_node_out_and_vjp(block, column, case["upstream"])

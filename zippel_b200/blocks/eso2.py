@@ -572,6 +572,8 @@ class EdgeFeatures(torch.autograd.Function):
         posf, shf, embf, off = _f32(pos), _f32(shifts), _f32(emb), _f32(gauss_offset)
         cgf, sgf = _f32(cos_g), _f32(sin_g)
         zi = atomic_numbers.to(torch.int64).contiguous()
+        if zi.numel() < n:
+            raise ValueError(f"{zi.numel()} element numbers for {n} atoms")
         if emb.shape[0] < front.n_elements or emb.shape[1] != front.edge_channels:
             raise ValueError(f"the element embedding has shape {tuple(emb.shape)}, the block needs "
                              f"({front.n_elements}, {front.edge_channels})")
@@ -805,7 +807,7 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
         z = z.to(torch.int64).contiguous()
     _need_cuda(pos, x, shifts, z, cos_g, sin_g, off, *params)
     assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
-    assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.shape == (n,)
+    assert pos.shape == (n, 3) and shifts.shape[1] == 3 and z.numel() >= n
     assert cos_g.shape[1] == cfg.lmax + 1 and sin_g.shape == cos_g.shape
     assert min(shifts.shape[0], cos_g.shape[0]) >= e
     out = torch.empty(n1 - n0, s.K, plan.c, dtype=torch.float32, device=x.device)
@@ -1055,13 +1057,20 @@ class ESO2Block(nn.Module):
                                       self.c2_m0.bias, *[layer.weight for layer in self.c1_m],
                                       *[layer.weight for layer in self.c2_m])
 
-    def _sorted_edges(self, edge_index, atomic_numbers):
+    def _sorted_edges(self, edge_index, atomic_numbers, n: int):
         """The edge order of new input and the check of its indices, to be called once the work that
         follows has been enqueued (nothing can be checked while a stream is being captured: the
         kernels leave edges with bad indices out and clamp element numbers either way)."""
         if torch.cuda.is_current_stream_capturing():
-            return EdgeGraph.build(edge_index, atomic_numbers.shape[0]), None
-        return EdgeGraph.build_checked(edge_index, atomic_numbers, self.cfg.max_num_elements)
+            return EdgeGraph.build(edge_index, n), None
+        limit = self.cfg.max_num_elements
+        if atomic_numbers.shape == (n,):
+            return EdgeGraph.build_checked(edge_index, atomic_numbers, limit)
+        # [N, 1], or more entries than there are atoms: looked through one by one
+        graph = EdgeGraph.build(edge_index, n)
+        if not bool(((atomic_numbers >= 0) & (atomic_numbers < limit)).all()):
+            raise IndexError(f"atomic_numbers outside [0, {limit})")
+        return graph, None
 
     def node_output(self, pos, atomic_numbers, x_node, edge_index, shifts, cos_gamma_k,
                     sin_gamma_k, graph: EdgeGraph | None = None,
@@ -1085,7 +1094,7 @@ class ESO2Block(nn.Module):
         if graph is None:
             # new input: node indices and element numbers are range-checked (a caller that passes
             # a prebuilt graph has had them checked when it was built)
-            graph, check = self._sorted_edges(edge_index, atomic_numbers)
+            graph, check = self._sorted_edges(edge_index, atomic_numbers, pos.shape[0])
         try:
             plan = self.plan(pos.device)
             energy = function is EnergyFunction
