@@ -261,3 +261,27 @@ def test_element_numbers_as_a_column(fake):
         assert lib.calls[-1][1][2].atomic_numbers == z.data_ptr()
     with pytest.raises(AssertionError):
         node_output(block, case, graph, case["pos"], case["x_node"], case["atomic_numbers"][:-1])
+
+
+@pytest.mark.parametrize("parts", [False, True])
+@pytest.mark.parametrize("form", ["int64", "strided"])
+def test_a_graph_whose_order_is_of_another_type(fake, form, parts, monkeypatch):
+    """The order of a graph made by hand, as int64 or a column of a table: the library gets int32."""
+    import ctypes
+    lib, block, case, graph = fake
+    monkeypatch.setattr(eso2, "_edge_budget", lambda *args: 1 << 20)
+    want, got = graph.perm.tolist(), []
+    graph.perm = graph.perm.long() if form == "int64" else torch.stack([graph.perm, graph.perm], 1)[:, 0]
+    if parts:
+        block.rad_func[1].eps = 1e-3
+        monkeypatch.setattr(eso2, "EdgeFeatures",
+                            types.SimpleNamespace(apply=lambda g, perm, *rest: got.extend(
+                                (perm.dtype, perm.is_contiguous(), *perm.tolist())) or 1 / 0))
+        with pytest.raises(ZeroDivisionError):
+            node_output(block, case, graph, case["pos"], case["x_node"])
+        assert got == [torch.int32, True, *want]
+    else:
+        monkeypatch.setattr(lib, "run", lambda device, name, *args: got.extend(
+            (ctypes.c_int32 * 40).from_address(args[2].perm)))
+        node_output(block, case, graph, case["pos"], case["x_node"])
+        assert got == want

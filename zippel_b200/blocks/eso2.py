@@ -818,6 +818,9 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
         raise _lib.ZpError(2, "zp_block_workspace_bytes")
     ws = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     order = graph.addresses()
+    perm = graph.given_perm() if perm is None else perm
+    if perm is not None and (perm.dtype != torch.int32 or not perm.is_contiguous()):
+        perm = perm.to(torch.int32).contiguous()
     call = _lib.ZpBlockCall(
         n1 - n0, e, n, n0, pos.data_ptr(), shifts.data_ptr(), z.data_ptr(), x.data_ptr(),
         cos_g.data_ptr(), sin_g.data_ptr(), order[0] if perm is None else perm.data_ptr(), *order[1:])
@@ -1041,8 +1044,8 @@ class ESO2Block(nn.Module):
         """The same with the front end, every radial layer and the edge convolution as functions of
         their own, for a radial MLP that the one call does not run."""
         edge_vec, x_edge, env, cos_s, sin_s = EdgeFeatures.apply(
-            graph, perm, self.front_config(), pos, shifts, atomic_numbers, self.elem_emb.weight,
-            self.gauss_offset, cos_gamma_k, sin_gamma_k)
+            graph, perm.to(torch.int32).contiguous(), self.front_config(), pos, shifts, atomic_numbers,
+            self.elem_emb.weight, self.gauss_offset, cos_gamma_k, sin_gamma_k)
         last, rad_w, rad_b = self.rad_func[-1], None, None
         if isinstance(last, nn.Linear) and last.in_features % 8 == 0 and graph.n_edges > 0:
             # the last (widest) radial layer runs inside the edge-convolution call

@@ -185,6 +185,11 @@ class EdgeGraph:
         setattr(self, name, value)
         return value
 
+    def given_perm(self) -> torch.Tensor | None:
+        """``perm`` of a graph whose arrays somebody gave it (``perm`` alone may be of another integer
+        type), None for those of a sort."""
+        return self.perm if "packed" not in self.__dict__ else None
+
     def addresses(self) -> tuple:
         """Device addresses of perm, src, dst, row_ptr, perm_src, row_ptr_src."""
         packed = self.__dict__.get("packed")
