@@ -285,3 +285,16 @@ def test_a_graph_whose_order_is_of_another_type(fake, form, parts, monkeypatch):
             (ctypes.c_int32 * 40).from_address(args[2].perm)))
         node_output(block, case, graph, case["pos"], case["x_node"])
         assert got == want
+
+
+def test_no_atoms_have_zero_parameter_gradients(fake, monkeypatch):
+    lib, block, case, graph = fake
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: torch.full(*a, 7.0, **k) if k.get("dtype") is torch.float32
+                        else torch.zeros(*a, **k))                   # what uninitialised memory may hold
+    i32 = lambda n: torch.zeros(n, dtype=torch.int32)                                # noqa: E731
+    none = EdgeGraph(0, 0, i32(0), i32(0), i32(0), i32(1), i32(0), i32(1))
+    case = {k: v[:0] for k, v in case.items()}
+    x, pos = case["x_node"].requires_grad_(True), case["pos"].requires_grad_(True)
+    out = node_output(block, case, none, pos, x)
+    grads = torch.autograd.grad(out, [pos, x, *block._call_params(False)], torch.zeros_like(out))
+    assert all(g.abs().sum() == 0 for g in grads)

@@ -859,7 +859,9 @@ def _block_vjp(ctx, saved, grad_out, want):
     # SO(2) parameters are each formed together
     wp = want[2:]
     groups = [wp[0]] + [any(wp[1:11])] * 10 + [any(wp[11:])] * (len(wp) - 11)
-    gp = [torch.empty(sh, **f32) if w else None for sh, w in zip(ctx.shapes, groups)]
+    # (without rows the library has nothing to do, and writes nothing)
+    new = torch.empty if sizes[0] else torch.zeros
+    gp = [new(sh, **f32) if w else None for sh, w in zip(ctx.shapes, groups)]
     p = [t.data_ptr() if t is not None else None for t in gp]
     so2, keep = (_weights_ptrs(plan.mmax, p[11:]) if p[11] is not None
                  else (_lib.ZpWeights(), None))
