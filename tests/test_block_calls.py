@@ -289,8 +289,8 @@ def test_a_graph_whose_order_is_of_another_type(fake, form, parts, monkeypatch):
 
 def test_no_atoms_have_zero_parameter_gradients(fake, monkeypatch):
     lib, block, case, graph = fake
-    monkeypatch.setattr(torch, "empty", lambda *a, **k: torch.full(*a, 7.0, **k) if k.get("dtype") is torch.float32
-                        else torch.zeros(*a, **k))                   # what uninitialised memory may hold
+    monkeypatch.setattr(torch, "empty",                              # what fresh memory may hold
+                        lambda *a, **k: torch.zeros(*a, **k) + (7 if k.get("dtype") is torch.float32 else 0))
     i32 = lambda n: torch.zeros(n, dtype=torch.int32)                                # noqa: E731
     none = EdgeGraph(0, 0, i32(0), i32(0), i32(0), i32(1), i32(0), i32(1))
     case = {k: v[:0] for k, v in case.items()}
