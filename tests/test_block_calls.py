@@ -298,3 +298,14 @@ def test_no_atoms_have_zero_parameter_gradients(fake, monkeypatch):
     out = node_output(block, case, none, pos, x)
     grads = torch.autograd.grad(out, [pos, x, *block._call_params(False)], torch.zeros_like(out))
     assert all(g.abs().sum() == 0 for g in grads)
+
+
+def test_edge_conv_lists_the_weights_of_its_layers(fake, monkeypatch):
+    _, block, case, graph = fake
+    got = []
+    monkeypatch.setattr(eso2, "EdgeConvFunction", types.SimpleNamespace(apply=lambda *args: got.extend(args)))
+    rest = [object() for _ in range(8)]
+    eso2.edge_conv(*rest, block.c1_m0, block.c1_m, block.c2_m0, block.c2_m)
+    assert got[:8] == rest and got[8:10] == [None, None]
+    assert [t.shape for t in got[10:]] == eso2._so2_shapes(2, 1, 8, 8)
+    assert got[14] is block.c1_m[0].weight and got[15] is block.c2_m[0].weight

@@ -713,6 +713,14 @@ def radial_mlp(plan: Plan, x_edge: torch.Tensor, layers: list) -> torch.Tensor:
     return h
 
 
+def edge_conv(plan: Plan, graph: EdgeGraph, x_node, edge_vec, cos_g, sin_g, radial, env,
+              c1_m0: nn.Linear, c1_m, c2_m0: nn.Linear, c2_m, rad_w=None, rad_b=None) -> torch.Tensor:
+    """``EdgeConvFunction`` with the weights of these layers; ``rad_w`` / ``rad_b``: see there."""
+    return EdgeConvFunction.apply(plan, graph, x_node, edge_vec, cos_g, sin_g, radial, env, rad_w, rad_b,
+                                  c1_m0.weight, c1_m0.bias, c2_m0.weight, c2_m0.bias,
+                                  *[m.weight for m in c1_m], *[m.weight for m in c2_m])
+
+
 class BlockFunction(torch.autograd.Function):
     """node_out = the whole block from positions and embeddings (``zp_block_forward``), with the VJP
     of all of it (``zp_block_backward``): reference blocks/eso2_ref.py:317-349 and autograd through
@@ -1057,10 +1065,8 @@ class ESO2Block(nn.Module):
             radial = self.radial_mlp(plan, x_edge)
         if x_ready is not None:
             torch.cuda.current_stream(pos.device).wait_event(x_ready)
-        return EdgeConvFunction.apply(plan, graph, x_node, edge_vec, cos_s, sin_s, radial, env, rad_w, rad_b,
-                                      self.c1_m0.weight, self.c1_m0.bias, self.c2_m0.weight,
-                                      self.c2_m0.bias, *[layer.weight for layer in self.c1_m],
-                                      *[layer.weight for layer in self.c2_m])
+        return edge_conv(plan, graph, x_node, edge_vec, cos_s, sin_s, radial, env, self.c1_m0, self.c1_m,
+                         self.c2_m0, self.c2_m, rad_w, rad_b)
 
     def _sorted_edges(self, edge_index, atomic_numbers, n: int):
         """The edge order of new input and the check of its indices, to be called once the work that
