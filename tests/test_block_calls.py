@@ -309,3 +309,16 @@ def test_edge_conv_lists_the_weights_of_its_layers(fake, monkeypatch):
     assert got[:8] == rest and got[8:10] == [None, None]
     assert [t.shape for t in got[10:]] == eso2._so2_shapes(2, 1, 8, 8)
     assert got[14] is block.c1_m[0].weight and got[15] is block.c2_m[0].weight
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_a_readout_of_other_widths_is_refused(fake, which):
+    lib, block, case, graph = fake
+    eso2._readout(block.plan("cpu"), case["x_node"], block._call_params(True)[-4:])
+    if which:
+        block.readout[2] = torch.nn.Linear(8, 2)
+    else:
+        block.readout[0] = torch.nn.Linear(24, 4)
+    head = [block.readout[0].weight, block.readout[0].bias, block.readout[2].weight, block.readout[2].bias]
+    with pytest.raises(ValueError, match="readout"):
+        eso2._readout(block.plan("cpu"), case["x_node"], head)

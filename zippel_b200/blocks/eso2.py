@@ -654,7 +654,11 @@ class Readout(torch.autograd.Function):
 
 def _readout(plan: Plan, x, head):
     """Energy (0-dim) of node rows ``x`` under the head's parameters, and the buffer its VJP reads."""
-    n = x.shape[0]
+    n, c = x.shape[0], plan.c
+    sizes = [t.numel() for t in head]
+    if sizes != [c * c * (plan.lmax + 1), c, c, 1]:
+        raise ValueError(f"the readout's parameters have {sizes} elements; it runs Linear({c * (plan.lmax + 1)}, "
+                         f"{c}), SiLU, Linear({c}, 1)")
     nbytes = max(_lib.load().zp_readout_work_bytes(plan.handle, n), 16)
     work = torch.empty(nbytes, dtype=torch.uint8, device=x.device)
     energy = torch.empty((), dtype=torch.float32, device=x.device)
