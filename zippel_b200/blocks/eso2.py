@@ -230,11 +230,11 @@ def _one_piece(plan: Plan, e: int, kept: bool, share: int) -> bool:
     allocation fails and the caller goes on in pieces.  One whose activations stay until its backward
     has to leave memory to what follows: like ``_edge_budget``'s, its share (with ``share`` = 2 a half)
     is of what this process has not allocated of the device, less what others held when the driver
-    was last asked.  Below a 512th of the device's memory that is not looked up either."""
+    was last asked.  Below a 256th of the device's memory that is not looked up either."""
     need = e * plan.bytes_per_edge
     if MAX_EDGES_PER_CALL is not None or 16 * need > plan.total_memory:
         return False
-    if not kept or 512 * need <= plan.total_memory:
+    if not kept or 256 * need <= plan.total_memory:
         return True
     return share * need <= plan.total_memory - plan.foreign - _allocated(plan.device)
 
@@ -746,7 +746,7 @@ class BlockFunction(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad_out):
-        want = _wanted(ctx, len(ctx.shapes))
+        want = _wanted(ctx, ctx.n_params)
         return _returned(ctx, _block_vjp(ctx, ctx.saved_tensors, grad_out, want))
 
 
@@ -773,7 +773,7 @@ class EnergyFunction(torch.autograd.Function):
         # asked for once: checkpointing brings a tensor back a single time
         saved = ctx.saved_tensors
         out, *head, work = saved[-6:]
-        want, plan = _wanted(ctx, len(ctx.shapes) + 4), ctx.native[0]
+        want, plan = _wanted(ctx, ctx.n_params + 4), ctx.native[0]
         g = torch.empty_like(out)
         ghead = _readout_vjp(plan, out, head, grad_e, g, work, any(want[-4:]))
         ghead = [t if w else None for t, w in zip(ghead, want[-4:])]
@@ -811,10 +811,10 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
     needs_bwd = any(ctx.needs_input_grad)
     n, e = graph.n_nodes, graph.n_edges
     n0, n1 = getattr(graph, "node_range", None) or (0, n)
-    dtypes = [t.dtype for t in (pos, x_node, *params)]
-    pos, x, shifts, cos_g, sin_g = (_as_f32(t) for t in (pos, x_node, shifts, cos_g, sin_g))
-    params = [_as_f32(t) for t in params]
-    off = _as_f32(block.gauss_offset)
+    given = [pos, x_node, *params]
+    pos, x, *params, shifts, cos_g, sin_g, off = [
+        t if t.dtype is torch.float32 and t.is_contiguous() else _f32(t)
+        for t in (*given, shifts, cos_g, sin_g, block.gauss_offset)]
     if z.dtype != torch.int64 or not z.is_contiguous():
         z = z.to(torch.int64).contiguous()
     _need_cuda(pos, x, shifts, z, cos_g, sin_g, off, *params)
@@ -850,7 +850,7 @@ def _block(ctx, block, plan: Plan, graph: EdgeGraph, perm, z, shifts, cos_g, sin
     # reads is all saved (of the parameters only the LayerNorms', the products read the planes in
     # the workspace).
     ctx.native = (plan, graph, front, (n1 - n0, e, n, n0))
-    ctx.shapes, ctx.dtypes = [t.shape for t in params], dtypes
+    ctx.cfg, ctx.n_params, ctx.dtypes = cfg, len(params), [t.dtype for t in given]
     return out, (ws, x, pos, z, off, params[3], params[4], params[7], params[8])
 
 
@@ -858,37 +858,43 @@ def _block_vjp(ctx, saved, grad_out, want):
     """Gradients of (pos, x_node, *params), None where ``want`` is false."""
     ws, x, pos, z, off, *norms = saved
     plan, graph, front, sizes = ctx.native
-    g, x, off, *norms = (_as_f32(t) for t in (grad_out, x, off, *norms))
+    g, x, off, *norms = [t if t.dtype is torch.float32 and t.is_contiguous() else _f32(t)
+                         for t in (grad_out, x, off, *norms)]
     ln = [t.data_ptr() for t in norms]
-    order = graph.addresses()
-    call = _lib.ZpBlockCall(*sizes, None, None, z.data_ptr(), x.data_ptr(), None, None, None, *order[1:])
-    cparams = _lib.ZpBlockParams(None, off.data_ptr(), _P3(), _P3(), _P2(ln[0], ln[2]),
-                                 _P2(ln[1], ln[3]), 0.0, _lib.ZpWeights())
+    _, src, dst, row_ptr, perm_src, row_ptr_src = graph.addresses()
+    call = _lib.ZpBlockCall(*sizes, None, None, z.data_ptr(), x.data_ptr(), None, None, None, src, dst,
+                            row_ptr, perm_src, row_ptr_src)
+    cparams = _lib.ZpBlockParams(None, off.data_ptr(), _NONE3, _NONE3, _P2(ln[0], ln[2]), _P2(ln[1], ln[3]))
     f32 = dict(dtype=torch.float32, device=x.device)
     gpos = torch.empty(pos.shape, **f32) if want[0] else None
     gx = torch.empty(x.shape, **f32) if want[1] else None
     # frozen parameters: the products behind their gradients are not run; the radial and the
     # SO(2) parameters are each formed together
-    wp = want[2:]
-    groups = [wp[0]] + [any(wp[1:11])] * 10 + [any(wp[11:])] * (len(wp) - 11)
-    # (without rows the library has nothing to do, and writes nothing)
-    new = torch.empty if sizes[0] else torch.zeros
-    gp = [new(sh, **f32) if w else None for sh, w in zip(ctx.shapes, groups)]
-    p = [t.data_ptr() if t is not None else None for t in gp]
-    so2, keep = (_weights_ptrs(plan.mmax, p[11:]) if p[11] is not None
-                 else (_lib.ZpWeights(), None))
-    grads = _lib.ZpBlockGrads(p[0], _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
-                              _P2(p[3], p[7]), _P2(p[4], p[8]), so2)
+    wp, keep = want[2:], None
+    if any(wp):
+        groups = [wp[0]] + [any(wp[1:11])] * 10 + [any(wp[11:])] * (len(wp) - 11)
+        # (without rows the library has nothing to do, and writes nothing)
+        new = torch.empty if sizes[0] else torch.zeros
+        gp = [new(sh, **f32) if w else None for sh, w in zip(_param_shapes(ctx.cfg, False), groups)]
+        p = [t.data_ptr() if t is not None else None for t in gp]
+        so2, keep = (_weights_ptrs(plan.mmax, p[11:]) if p[11] is not None
+                     else (_lib.ZpWeights(), None))
+        grads = _lib.ZpBlockGrads(p[0], _P3(p[1], p[5], p[9]), _P3(p[2], p[6], p[10]),
+                                  _P2(p[3], p[7]), _P2(p[4], p[8]), so2)
+    else:
+        gp, grads = [], _lib.ZpBlockGrads()
     _lib.run(x.device, "zp_block_backward", plan.handle, front, call, cparams,
              g.data_ptr() - sizes[3] * plan.sizes.K * plan.c * 4,
              gx.data_ptr() if gx is not None else None,
              gpos.data_ptr() if gpos is not None else None, grads, ws.data_ptr(), ws.numel())
     del keep
-    return tuple(None if t is None or not w else t if t.dtype == dt else t.to(dt)
-                 for t, w, dt in zip([gpos, gx, *gp], want, ctx.dtypes))
+    out = [None if t is None or not w else t if t.dtype == dt else t.to(dt)
+           for t, w, dt in zip((gpos, gx, *gp), want, ctx.dtypes)]
+    return (*out, *(None,) * (len(want) - len(out)))
 
 
 _P2, _P3 = ctypes.c_void_p * 2, ctypes.c_void_p * 3
+_NONE3 = _P3()
 #: the radial MLP that the block runs in one call
 _RADIAL_LAYERS = (nn.Linear, nn.LayerNorm, nn.SiLU, nn.Linear, nn.LayerNorm, nn.SiLU, nn.Linear)
 
@@ -906,16 +912,9 @@ def _param_shapes(cfg: BlockConfig, head: bool) -> list[tuple]:
     return out + ([(c, c * (cfg.lmax + 1)), (c,), (1, c), (1,)] if head else [])
 
 
-def _param(module: nn.Module, name: str):
-    """``module.name``, without the search through the module where it is a plain parameter."""
-    p = module._parameters.get(name)
-    return getattr(module, name) if p is None else p
-
-
 def _need_cuda(*tensors: torch.Tensor) -> None:
-    for t in tensors:
-        if not t.is_cuda:
-            raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
+    if not all([t.is_cuda for t in tensors]):
+        raise RuntimeError("the block needs CUDA tensors: there is no CPU path")
 
 
 def _as_f32(t: torch.Tensor) -> torch.Tensor:
@@ -1028,19 +1027,26 @@ class ESO2Block(nn.Module):
         rad = tuple(m["rad_func"]._modules.values())
         if (len(rad) != 7 or not all(map(isinstance, rad, _RADIAL_LAYERS)) or rad[1].eps != rad[4].eps):
             return None
-        c1, c2 = m["c1_m0"], m["c2_m0"]
-        out = [_param(m["elem_emb"], "weight")]
-        for layer in (rad[0], rad[1], rad[3], rad[4], rad[6]):
-            out += (_param(layer, "weight"), _param(layer, "bias"))
-        out += (_param(c1, "weight"), _param(c1, "bias"))
-        out += [_param(layer, "weight") for layer in m["c1_m"]._modules.values()]
-        out += (_param(c2, "weight"), _param(c2, "bias"))
-        out += [_param(layer, "weight") for layer in m["c2_m"]._modules.values()]
+        both = [rad[0], rad[1], rad[3], rad[4], rad[6], m["c1_m0"], m["c2_m0"]]
         if head:
-            lin0, lin1 = self.readout[0], self.readout[2]
-            out += (_param(lin0, "weight"), _param(lin0, "bias"), _param(lin1, "weight"), _param(lin1, "bias"))
-        shapes = _param_shapes(self.cfg, head)
-        return out if [None if p is None else p.shape for p in out] == shapes else None
+            both += (self.readout[0], self.readout[2])
+        c1, c2 = m["c1_m"]._modules.values(), m["c2_m"]._modules.values()
+        try:                                   # plain parameters, without the search through a module
+            out = [m["elem_emb"]._parameters["weight"]]
+            pairs = [p[name] for p in [layer._parameters for layer in both] for name in ("weight", "bias")]
+            wm1 = [layer._parameters["weight"] for layer in c1]
+            wm2 = [layer._parameters["weight"] for layer in c2]
+        except KeyError:
+            out = [m["elem_emb"].weight]
+            pairs = [p for layer in both for p in (layer.weight, layer.bias)]
+            wm1, wm2 = [layer.weight for layer in c1], [layer.weight for layer in c2]
+        out += pairs[:12]
+        out += wm1
+        out += pairs[12:14]
+        out += wm2
+        out += pairs[14:]
+        shapes = [None if p is None else p.shape for p in out]
+        return out if shapes == _param_shapes(self.cfg, head) else None
 
     def _edges_to_nodes(self, plan, graph, perm, pos, atomic_numbers, x_node, shifts, cos_gamma_k,
                         sin_gamma_k, x_ready=None) -> torch.Tensor:
@@ -1228,10 +1234,11 @@ class ESO2Block(nn.Module):
         """Scalar E.  ``jd`` (the reference's argument) is verified against the J matrices the
         kernels use; anything else raises ``ValueError``."""
         self._check_jd(jd)
-        for name in ("node_output", "energy"):      # a subclass' own, or one set on the instance
-            if getattr(type(self), name) is not getattr(ESO2Block, name) or name in self.__dict__:
-                return self.energy(self.node_output(pos, atomic_numbers, x_node, edge_index, shifts,
-                                                    cos_gamma_k, sin_gamma_k, graph))
+        cls, own = type(self), self.__dict__
+        if ("energy" in own or "node_output" in own or cls is not ESO2Block and
+                (cls.energy is not ESO2Block.energy or cls.node_output is not ESO2Block.node_output)):
+            return self.energy(self.node_output(pos, atomic_numbers, x_node, edge_index, shifts,
+                                                cos_gamma_k, sin_gamma_k, graph))
         return self._evaluate(EnergyFunction, pos, atomic_numbers, x_node, edge_index, shifts,
                               cos_gamma_k, sin_gamma_k, graph)
 

@@ -138,8 +138,8 @@ class EdgeGraph:
         the device busy.  To be called in any case, errors in between included: the flags arrive in
         memory that it holds.  Not for use while the stream is being captured."""
         lib, ei, e, dev = EdgeGraph._open(edge_index)
-        if atomic_numbers.device != dev:
-            raise RuntimeError(f"atomic_numbers on {atomic_numbers.device}, edge_index on {dev}")
+        if not atomic_numbers.is_cuda:
+            raise RuntimeError("EdgeGraph.build_checked needs CUDA atomic_numbers; there is no CPU path")
         z = atomic_numbers.to(torch.int64).contiguous()
         n = z.shape[0]
         graph = EdgeGraph.__new__(EdgeGraph)
