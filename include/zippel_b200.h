@@ -437,7 +437,8 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
  *   zp_neighbors_fill   (same pos/box/cutoff/max_neighbors/work) writes edge_index [2,E] int64
  *                       (row 0 = src, row 1 = dst) and shifts [E,3] fp64.
  * *flags_out (device int) is 0 on success; bit 0: a position that is not finite, bit 1: more than
- * ZP_NEIGHBORS_MAX_HITS neighbours of one atom in an uncapped list, bit 2: the passes disagree.  */
+ * ZP_NEIGHBORS_MAX_HITS neighbours of one atom in an uncapped list, bit 2: the second
+ * call found another number of edges than the first (not seen: both read the same copies).       */
 #define ZP_NEIGHBORS_MAX_HITS 1024
 #define ZP_NEIGHBORS_MAX_CAP 256
 /* Work for any max_neighbors, and for one (less where it is below 128): the first call keeps each

@@ -17,10 +17,13 @@ thread_local char g_cuda_error[512] = "";
 thread_local int64_t g_launches = 0;
 
 // Up to this many edges the products of a step share one launch.  Beyond it each is a launch of its
-// own on the plan's streams: the fixed walk through one long list leaves CTAs idle at its end (3 % at
-// 60 000 edges), while the CTAs of a next launch start wherever an SM becomes free; below it the
-// set-up and the draining of each launch cost more (conv1 of 6 000 edges in bf16: 82 us apart, 70
-// together).
+// own on the plan's streams: the fixed walk through one long list leaves CTAs idle at its end (3 % of the
+// products at lmax 4, C 128 and 60 000 edges), while the CTAs of a next launch start wherever an SM becomes
+// free; below it the set-up and the draining of each launch cost more (conv1 of 6 000 edges in bf16: 82 us
+// apart, 70 together).  What decides is tiles per SM, and the line is drawn for wide blocks.  A whole
+// training step, apart / together: lmax 4, C 128 within 2 % of each other from 12 000 to 84 000 edges, fp32
+// and bf16; lmax 2, C 128 at 24 000 / 60 000 / 84 000 edges 1.79 / 3.93 / 5.38 ms against 1.64 / 3.71 /
+// 5.16; lmax 2, C 64 1.14 / 2.10 / 2.75 against 1.04 / 1.95 / 2.57: narrow ones would gain from a higher one.
 constexpr int64_t kTogetherEdges = 24000;
 constexpr int kChunkK = 2048;          // contraction length of one TMEM accumulation chunk
 

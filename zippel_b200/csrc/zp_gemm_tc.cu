@@ -16,8 +16,8 @@
 // that below the fp32 budget: (1) the leading product A0B0 has its own TMEM accumulator and the
 // five small products share a second one, whose truncation is 2^-8 smaller in absolute terms;
 // (2) the contraction is cut into chunks of at most `kc` k-blocks, each accumulated in TMEM
-// from zero and then added to C in fp32 by the epilogue (first chunk stores, later chunks
-// add), so the bias never grows beyond one chunk's length.  Long contractions (the weight
+// from zero and then added up in fp32 in the epilogue's registers (a tile is stored once), so
+// the bias never grows beyond one chunk's length.  Long contractions (the weight
 // gradients, which run over all edges) can also be split over CTAs: split s writes its own
 // partial matrix C + s * split_stride, reduced afterwards in a fixed order.
 //
@@ -1326,7 +1326,7 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
         // bounds the short contractions (256 x 256 tiles of K = 1024: 9.0 us, of them 5.8 MMAs; 10.2
         // with the whole slice read first and every column checked against N).
         if (x.kb1 - x.kb0 <= p.kc) {
-          const int buf = P == 1 ? (int)(unit & 1) : 0;
+          const int buf = (int)(unit & 1);
           const uint32_t t_row = finished(buf);
           if (!ok) break;
 #pragma unroll
@@ -1449,8 +1449,6 @@ int make_map(CUtensorMap *map, const void *base, uint64_t inner, uint64_t outer,
   return ZP_OK;
 }
 
-// Tile width: the multiple of `step` in [cap/2, cap] that wastes the fewest padded columns
-// (ties: the widest); problems narrower than cap/2 get one tile.
 // 3-d map over (column, row, split) of the fp32 output, 32 x 32 boxes under the 128-byte swizzle
 int make_map_c(CUtensorMap *map, float *C, uint64_t N, uint64_t M, uint64_t splits, uint64_t ldc,
                uint64_t split_stride) {
@@ -1470,6 +1468,8 @@ int make_map_c(CUtensorMap *map, float *C, uint64_t N, uint64_t M, uint64_t spli
   return ZP_OK;
 }
 
+// Tile width: the multiple of `step` in [cap/2, cap] that wastes the fewest padded columns
+// (ties: the widest); problems narrower than cap/2 get one tile.
 int pick_bn(int64_t N, int cap, int step = 16) {
   if (N <= cap / 2) return (int)(zp_ceil_div(N, step) * step);
   int best = cap;

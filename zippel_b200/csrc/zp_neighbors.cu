@@ -371,8 +371,8 @@ __device__ __forceinline__ void keep_nearest(Hit *h, int n, int cap, float cutof
 // with more than kFewHits hits or kKept survivors goes on the list `crowded` instead, its row of
 // `kept` marked: 192 hits because a warp walking again alone costs as much as a third of all others
 // (57 us for the few atoms in 100 000 that have more than 128 where the mean is 90).  Bound by
-// instruction issue: 186 us for 100 000 atoms, 90 hits each, cap 30, where a count of 90 us came before
-// 235 us of this.  Five blocks per SM (48 registers, no spills) instead of four: 12 us of the 186.
+// instruction issue: 175 us for 100 000 atoms, 90 hits each, cap 30, where a count of 90 us came before
+// 235 us of this; 186 with four blocks per SM instead of five (48 registers, no spills).
 constexpr int kSelectWarps = 8;
 constexpr unsigned long long kCrowded = ~0ull;
 __global__ void __launch_bounds__(32 * kSelectWarps, 5)
@@ -510,7 +510,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ o
       warp_bitonic(h, n2, lane, [](const Hit &a, const Hit &b) { return a.tie < b.tie; });
     }
     const int64_t base = row_ptr[j];
-    if (row_ptr[j + 1] - base != n) {          // passes disagree: nothing is written past the row
+    if (row_ptr[j + 1] - base != n) {          // not seen: both read the same copies; nothing is written past the row
       if (lane == 0) atomicOr(flags, 4);
       n = min(n, (int)(row_ptr[j + 1] - base));
     }

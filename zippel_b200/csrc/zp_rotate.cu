@@ -8,8 +8,8 @@
 // :269-271, :284-285 applied while the row is in registers) and :343-349 (envelope, rotate
 // back, index_add_).  The rotation is block diagonal in the degree l, so each thread keeps
 // one degree's 2l+1 input rows of its channel group in registers and forms only the rows with
-// |m| <= mmax.  Channels are the fastest axis everywhere: a thread owns VEC consecutive
-// channels and moves them with one vector load/store.  No atomics: every output element is
+// |m| <= mmax.  Channels are the fastest axis everywhere: a thread owns four consecutive
+// channels (two in rotate_back_scatter at lmax 5 and 6) and moves them with one vector load/store.  No atomics: every output element is
 // produced by exactly one thread, in an order fixed by the CSR offsets.
 #include <algorithm>
 

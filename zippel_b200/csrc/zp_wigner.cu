@@ -8,9 +8,10 @@
 // rows with |m| <= mmax are formed and they are written straight into the packed m'-major
 // layout (the reference's `to_m @ wigner`, blocks/eso2_ref.py:330-331).
 //
-// One thread per edge, arithmetic in fp64 (a few thousand flops per edge, far below the cost
-// of the SO(2) contraction), result rounded once to fp32.  The sparse X factors are applied
-// as two-term updates; only the product with J in the middle is dense.
+// Arithmetic in fp64 (a few thousand flops per edge, far below the cost of the SO(2) contraction),
+// result rounded once to fp32.  The sparse X factors are applied as two-term updates; only the product
+// with J in the middle is dense.  Forward: a block per 32 edges, its warps taking columns.  VJP: a thread
+// per edge from the gradient of the entries (zp_wigner_backward), or, in the block, from three torques.
 #include "zp_common.cuh"
 
 namespace {
