@@ -385,3 +385,25 @@ def test_element_numbers_as_a_column():
     column["atomic_numbers"][2, 0] = block.cfg.max_num_elements
     with pytest.raises(IndexError):
         gpu_node_out_and_vjp(block, column, case["upstream"])
+
+
+def test_weights_of_the_edge_convolution_by_size():
+    """Another arrangement of as many values is taken as it lies in memory; another size is refused."""
+    from zippel_b200.blocks import eso2
+    from zippel_b200.graph import EdgeGraph
+    cfg = dict(lmax=1, mmax=1, sphere_channels=8, hidden_channels=8, edge_channels=8,
+               num_distance_basis=4, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1))
+    plan, g = block.plan("cuda"), torch.Generator("cuda").manual_seed(0)
+    graph = EdgeGraph.build(torch.randint(0, 6, (2, 20), device="cuda", generator=g), 6)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g)            # noqa: E731
+    gamma = torch.rand(20, 1, device="cuda", generator=g) * torch.arange(2, device="cuda")
+    ins = (rand(6, 4, 8), rand(20, 3), gamma.cos(), gamma.sin(), rand(20, plan.sizes.R), rand(20), None, None)
+    w = [block.c1_m0.weight, block.c1_m0.bias, block.c2_m0.weight, block.c2_m0.bias, block.c1_m[0].weight,
+         block.c2_m[0].weight]
+    with torch.no_grad():
+        want = eso2.EdgeConvFunction.apply(plan, graph, *ins, *w)
+        flat = [w[0], w[1].reshape(-1, 8), w[2].flatten(), w[3].reshape(2, -1), *w[4:]]
+        assert torch.equal(want, eso2.EdgeConvFunction.apply(plan, graph, *ins, *flat))
+        with pytest.raises(AssertionError):
+            eso2.EdgeConvFunction.apply(plan, graph, *ins, w[0][:-1], *w[1:])

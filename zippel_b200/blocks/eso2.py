@@ -332,7 +332,7 @@ class EdgeConvFunction(torch.autograd.Function):
         assert x.shape == (n, s.K, plan.c), (x.shape, (n, s.K, plan.c))
         assert rad.shape == ((e, ec) if has_layer else (e, s.R)) and ev.shape == (e, 3)
         assert not has_layer or (rw.shape == (s.R, ec) and rb.shape == (s.R,))
-        assert [t.shape for t in tens[8:]] == _so2_shapes(plan.lmax, mmax, plan.c, plan.h)
+        assert [t.numel() for t in tens[8:]] == [math.prod(q) for q in _so2_shapes(plan.lmax, mmax, plan.c, plan.h)]
         assert en.shape == (e,) and cg.shape == (e, plan.lmax + 1) and sg.shape == cg.shape
         needs_bwd = any(ctx.needs_input_grad)
         # a graph may carry `node_range = (n0, n1)`: all its edges end in those nodes and only
