@@ -182,3 +182,19 @@ def test_short_contractions(M, N, K, planes):
     """The resident column block: widths that are no multiple of it, one to many columns per CTA."""
     err_p, err_f = run_gemm(M, N, K, planes, False, False)
     assert (err_p if planes == 1 else err_f) < 4e-6
+
+
+@pytest.mark.parametrize("M,N,K", [(129, 20, 24), (700, 1152, 1280), (513, 48, 72), (3000, 280, 576), (300, 256, 5000)])
+def test_three_planes_pair_kernel(M, N, K):
+    assert run_gemm(M, N, K, 3, False, False, variant=3)[1] < 4e-6
+    assert run_gemm(M, N, K, 3, True, True, variant=3)[1] < 4e-6
+
+
+@pytest.mark.parametrize("planes,variant", [(1, 2), (1, 3), (2, 2), (2, 3), (3, 2), (3, 3)])
+@pytest.mark.parametrize("M,N,K", [(256, 512, 2048), (130, 1024, 640), (300, 160, 9000), (1000, 96, 4100)])
+def test_few_tiles_are_cut_narrower(M, N, K, planes, variant):
+    """Tiles of at most 128 columns, whose accumulators alternate also with two and three planes, over one
+    accumulation chunk and several."""
+    for mn in (False, True):
+        err_p, err_f = run_gemm(M, N, K, planes, mn, mn, variant=variant)
+        assert (err_p if planes == 1 else err_f) < 4e-6

@@ -754,7 +754,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                 Xm.scale, nullptr, nullptr};
     }
     const bool together = E <= kTogetherEdges && nd + nw <= ZP_GEMM_GROUP;
-    if (nw && together) zp_gemm_group_splits(wgrads, nw, kZpWgradSplits);
+    if (nw && together) zp_gemm_group_splits(products, nd + nw, nw, kZpWgradSplits);
     for (int m = 0; m < nw; ++m) {
       if (!together) wgrads[m].ksplit = zp_gemm_tc_pick_splits(wgrads[m], kZpWgradSplits);
       splits[m] = zp_gemm_tc_splits(wgrads[m]);

@@ -341,8 +341,8 @@ int zp_launch_gemm_tc(const ZpGemmTc &g, cudaStream_t st);
 // up to ZP_GEMM_GROUP independent products of one format in one launch
 #define ZP_GEMM_GROUP 8
 int zp_launch_gemm_group(const ZpGemmTc *g, int n, cudaStream_t st);
-// sets the K split (<= max_splits) of products with one contraction that will share a launch
-void zp_gemm_group_splits(ZpGemmTc *g, int n, int max_splits);
+// sets the K split (<= max_splits) of the last nw of n products that will share a launch
+void zp_gemm_group_splits(ZpGemmTc *g, int n, int nw, int max_splits);
 // block_node[b] = node of the first edge of 32-edge block b, for ZpEpilogue::block_node
 int zp_launch_block_nodes(int64_t E, int64_t N, const int32_t *row_ptr, int32_t *block_node,
                           cudaStream_t st);

@@ -47,6 +47,7 @@
 #include <cuda_bf16.h>
 
 #include "zp_common.cuh"
+#include "zp_share.cuh"
 
 namespace {
 
@@ -200,7 +201,6 @@ struct GemmProb {
   int num_n, num_k;
   int ksplit, kb_per_split, kc;   // CTAs-level split of K; k-blocks per TMEM accumulation chunk
   int a_mn, b_mn;         // operand is MN-major
-  int start;              // first work item
   const float *scale_a, *scale_b;   // device scalars multiplying the result (null = 1)
   float *absmax_out;      // device scalar: running max |C| of what this launch stores (or null)
   const float *bias;
@@ -208,9 +208,20 @@ struct GemmProb {
 // The products of one launch.  Independent products (the orders m of a convolution, input and weight
 // gradients) share a launch when each alone would leave the device's last wave half empty: their
 // tiles form one list that the persistent CTAs walk.
+//
+// Which units (CTAs, or CTA pairs) take which tiles is laid down by the host (share_out): units of one
+// class, consecutive ones, take the same number of tiles of each product, side by side through the
+// product's list.
 struct GemmGroup {
   GemmProb p[ZP_GEMM_GROUP];
   int n, total;           // products, work items of all of them
+  int classes;
+  int unit0[kMaxClasses + 1];                  // first unit of each class, and the number of units
+  int first[kMaxClasses][ZP_GEMM_GROUP];       // first tile of the class in the product's list
+  int16_t count[kMaxClasses][ZP_GEMM_GROUP];   // tiles per unit
+  int stages, stage_bytes;                     // ring of operand stages
+  int b_tile;                                  // bytes of one plane of B in a stage
+  int acc_bufs, small_off;                     // accumulators in flight; TMEM columns to the small one
   int fp16;               // operand planes are fp16 (else bf16)
   int *status;
   uint64_t wait_limit_ns; // bound of every mbarrier wait
@@ -482,18 +493,30 @@ __device__ __forceinline__ void epilogue_fused(const GemmProb &p, const ZpEpilog
   }
 }
 
-template <int P, int BK, int STAGES, int BN_CAP>
-struct SmemLayout {
-  static constexpr int kATile = BM * BK * 2;
-  static constexpr int kBTile = BN_CAP * BK * 2;
-  static constexpr int kStage = P * (kATile + kBTile);
-  static constexpr int kTiles = STAGES * kStage;
-  static constexpr int kBars = 8 * (2 * STAGES + 4);
-  // barriers, TMEM slot and abort flag live in the first KB after the tiles; the epilogue's store
-  // blocks follow, 1 KB aligned; + 1 KB alignment slack
-  static_assert(kBars + 16 <= 1024, "control words fit in one KB");
-  static constexpr int kEpiOffset = kTiles + 1024;
-  static constexpr int kTotal = kTiles + 1024 + kEpiBytes + 1024;
+// Shared memory of the general kernels: operand stages, control words (barriers, TMEM slot, abort
+// flag), store blocks of the epilogue, and 1 KB of alignment slack.  A launch cuts the operand space into
+// as many stages as its widest tile leaves room for: 160-wide tiles of three planes have three instead of the
+// two that 256-wide ones have.
+constexpr int kMaxStages = 8;
+constexpr int kSmemTotal = 232448;
+constexpr int kTileBytes = kSmemTotal - 2048 - kEpiBytes;
+constexpr int kEpiOffset = kTileBytes + 1024;
+static_assert(kTileBytes % 1024 == 0 && 8 * (2 * kMaxStages + 4) + 16 <= 1024, "control words fit in one KB");
+
+// place in the ring of stages
+struct Ring {
+  int s = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next(int stages) {
+    if (++s == stages) { s = 0; phase ^= 1; }
+  }
+};
+
+// Accumulation unit `n` of a CTA: which of the accumulators it has, and the parity of its round.
+struct AccUnit {
+  int buf;
+  uint32_t parity;
+  __device__ __forceinline__ AccUnit(uint32_t n, bool two) : buf(two ? n & 1 : 0), parity((two ? n >> 1 : n) & 1) {}
 };
 
 // One unit of work of a CTA (or CTA pair): a product, an output tile of it, a K split and its
@@ -501,21 +524,35 @@ struct SmemLayout {
 struct Work {
   int prob, m0, n0, split, kb0, kb1;
 };
-template <int TM>
-__device__ __forceinline__ Work decode_work(const GemmGroup &g, int w) {
-  Work x;
-  x.prob = 0;
-  while (x.prob + 1 < g.n && w >= g.p[x.prob + 1].start) ++x.prob;
-  const GemmProb &p = g.p[x.prob];
-  w -= p.start;
-  x.split = w % p.ksplit;
-  const int tile = w / p.ksplit;
-  x.m0 = (tile / p.num_n) * TM;
-  x.n0 = (tile % p.num_n) * p.BN;
-  x.kb0 = x.split * p.kb_per_split;
-  x.kb1 = min(p.num_k, x.kb0 + p.kb_per_split);
-  return x;
-}
+// A unit's way through its share of the tiles.
+struct Walk {
+  int cls = 0, prob = 0, j = -1, unit;
+  __device__ __forceinline__ Walk(const GemmGroup &g, int u) {
+    while (cls + 1 < g.classes && u >= g.unit0[cls + 1]) ++cls;
+    unit = u - g.unit0[cls];
+  }
+  __device__ __forceinline__ bool next(const GemmGroup &g) {
+    ++j;
+    while (prob < g.n && j >= g.count[cls][prob]) { ++prob; j = 0; }
+    return prob < g.n;
+  }
+  template <int TM>
+  __device__ __forceinline__ Work tile(const GemmGroup &g) const {
+    Work x;
+    x.prob = prob;
+    const GemmProb &p = g.p[prob];
+    const int w = g.first[cls][prob] + j * (g.unit0[cls + 1] - g.unit0[cls]) + unit;
+    x.split = w % p.ksplit;
+    const int tile = w / p.ksplit;
+    x.m0 = (tile / p.num_n) * TM;
+    x.n0 = (tile % p.num_n) * p.BN;
+    x.kb0 = x.split * p.kb_per_split;
+    x.kb1 = min(p.num_k, x.kb0 + p.kb_per_split);
+    return x;
+  }
+};
+// Columns of a tile that an epilogue warp drains: the tile's 32-column blocks are dealt to two warps
+__device__ __forceinline__ int half_columns(int BN) { return (BN / 2 + 31) & ~31; }
 __device__ __forceinline__ void prefetch_maps(const GemmGroup &g) {
   for (int i = 0; i < g.n; ++i) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.p[i].map_a)) : "memory");
@@ -554,12 +591,12 @@ struct MaxTracker {
 // 32 columns of the accumulator(s) at `taddr` into v: sixteen of them at a time (a slice of 128 values
 // per thread leaves little room), both accumulators' loads in flight before one wait
 template <int P>
-__device__ __forceinline__ void read_block(float (&v)[32], uint32_t taddr, float out_scale) {
+__device__ __forceinline__ void read_block(float (&v)[32], uint32_t taddr, int small_off, float out_scale) {
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     uint32_t r[16], r2[16];
     tmem_ld16(taddr + 16 * h, r);
-    if (P != 1) tmem_ld16(taddr + kTmemBuf + 16 * h, r2);
+    if (P != 1) tmem_ld16(taddr + small_off + 16 * h, r2);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -571,17 +608,17 @@ __device__ __forceinline__ void read_block(float (&v)[32], uint32_t taddr, float
 }
 // The accumulator slice of a tile's first chunk (this warp's 32 rows, columns col_lo .. col_hi) into v
 template <int P>
-__device__ __forceinline__ void read_accumulator(float (&v)[4][32], uint32_t t_row, int col_lo,
-                                                 int col_hi, float out_scale) {
+__device__ __forceinline__ void read_accumulator(float (&v)[4][32], uint32_t t_row, int small_off,
+                                                 int col_lo, int col_hi, float out_scale) {
 #pragma unroll
   for (int b = 0; b < 4; ++b)
     if (col_lo + 32 * b < col_hi)         // warp-uniform
-      read_block<P>(v[b], t_row + col_lo + 32 * b, out_scale);
+      read_block<P>(v[b], t_row + col_lo + 32 * b, small_off, out_scale);
 }
 // ... and of a later chunk, added to it (all of v is live here: eight columns at a time)
 template <int P>
-__device__ __forceinline__ void add_accumulator(float (&v)[4][32], uint32_t t_row, int col_lo,
-                                                int col_hi, float out_scale) {
+__device__ __forceinline__ void add_accumulator(float (&v)[4][32], uint32_t t_row, int small_off,
+                                                int col_lo, int col_hi, float out_scale) {
 #pragma unroll
   for (int b = 0; b < 4; ++b) {
     const int cc = col_lo + 32 * b;
@@ -590,7 +627,7 @@ __device__ __forceinline__ void add_accumulator(float (&v)[4][32], uint32_t t_ro
       for (int h = 0; h < 4; ++h) {
         uint32_t r[8], r2[8];
         tmem_ld8(t_row + cc + 8 * h, r);
-        if (P != 1) tmem_ld8(t_row + kTmemBuf + cc + 8 * h, r2);
+        if (P != 1) tmem_ld8(t_row + small_off + cc + 8 * h, r2);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -603,26 +640,24 @@ __device__ __forceinline__ void add_accumulator(float (&v)[4][32], uint32_t t_ro
   }
 }
 
-template <int P, int BK, int STAGES, int BN_CAP, int EPI>
+template <int P, int BK, int EPI>
 __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
-  using L = SmemLayout<P, BK, STAGES, BN_CAP>;
-  constexpr int kAccBufs = P == 1 ? 2 : 1;      // accumulation units in flight in TMEM
+  constexpr int kATile = BM * BK * 2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                               ~(uintptr_t)1023);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::kTiles);
-  uint64_t *empty = full + STAGES;
-  uint64_t *tmem_full = empty + STAGES;
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + kTileBytes);
+  uint64_t *empty = full + kMaxStages;
+  uint64_t *tmem_full = empty + kMaxStages;
   uint64_t *tmem_empty = tmem_full + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const int num_work = g.total;
 
   if (threadIdx.x == 0) {
     prefetch_maps(g);
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < g.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 8); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -639,28 +674,29 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-
-  const uint32_t a_bytes = BM * BK * 2;
+  zp_after_previous();                  // all of the above ran beside the kernel before
+  const int stages = g.stages;
+  const bool two_accs = P == 1 || g.acc_bufs == 2;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (!g.unarmed && elect_one()) {
-      uint32_t it = 0;
+      Ring ring;
       bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-        const Work x = decode_work<BM>(g, w);
+      for (Walk walk(g, blockIdx.x); ok && walk.next(g);) {
+        const Work x = walk.tile<BM>(g);
         const GemmProb &p = g.p[x.prob];
         const uint32_t b_bytes = (uint32_t)p.BN * BK * 2;
-        for (int kb = x.kb0; kb < x.kb1 && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+        for (int kb = x.kb0; kb < x.kb1 && ok; ++kb, ring.next(stages)) {
+          const int s = ring.s;
+          ok = mbar_wait(&empty[s], ring.phase ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
-          uint8_t *st = smem + (size_t)s * L::kStage;
-          mbar_expect_tx(&full[s], P * (a_bytes + b_bytes));
+          uint8_t *st = smem + (size_t)s * g.stage_bytes;
+          mbar_expect_tx(&full[s], P * (kATile + b_bytes));
           const int k0 = kb * BK;
 #pragma unroll
           for (int pl = 0; pl < P; ++pl) {
-            uint8_t *ta = st + pl * L::kATile, *tb = st + P * L::kATile + pl * L::kBTile;
+            uint8_t *ta = st + pl * kATile, *tb = st + P * kATile + pl * g.b_tile;
             if (!p.a_mn) {
               tma_load_3d(ta, &p.map_a, &full[s], k0, x.m0, pl);
             } else {                      // two 64-wide column blocks of [BK][64]
@@ -681,34 +717,36 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
     // ---------------------------------------------------------------- MMA issuer
     if (elect_one()) {
       constexpr uint32_t kLayout = BK == 64 ? 2u : 4u;
-      uint32_t it = 0, unit = 0;
+      const int b_tile = g.b_tile;
+      uint32_t unit = 0;
+      Ring ring;
       bool ok = true;
-      for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-        const Work x = decode_work<BM>(g, w);
+      for (Walk walk(g, blockIdx.x); ok && walk.next(g);) {
+        const Work x = walk.tile<BM>(g);
         const GemmProb &p = g.p[x.prob];
         const uint32_t idesc = instr_desc(g, p, BM);
         for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
           const int c1 = min(x.kb1, c0 + p.kc);
-          const int buf = unit % kAccBufs;
-          ok = mbar_wait(&tmem_empty[buf], ((unit / kAccBufs) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+          const AccUnit acc(unit, two_accs);
+          const int buf = acc.buf;
+          ok = mbar_wait(&tmem_empty[buf], acc.parity ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           tcgen05_fence_after();
-          // one plane: accumulator `buf`; three planes: leading product at column 0, small at 256
-          const uint32_t d_main = tmem_base + (P == 1 ? (uint32_t)buf * kTmemBuf : 0u);
-          const uint32_t d_small = tmem_base + kTmemBuf;
-          for (int kb = c0; kb < c1 && ok; ++kb, ++it) {
-            const int s = it % STAGES;
-            ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, g.status, g.wait_limit_ns);
+          const uint32_t d_main = tmem_base + (uint32_t)buf * kTmemBuf;
+          const uint32_t d_small = d_main + g.small_off;
+          for (int kb = c0; kb < c1 && ok; ++kb, ring.next(stages)) {
+            const int s = ring.s;
+            ok = mbar_wait(&full[s], ring.phase, abort_flag, g.status, g.wait_limit_ns);
             if (!ok) break;
             tcgen05_fence_after();
-            const uint32_t sa = smem_u32(smem + (size_t)s * L::kStage);
-            const uint32_t sb = sa + P * L::kATile;
+            const uint32_t sa = smem_u32(smem + (size_t)s * g.stage_bytes);
+            const uint32_t sb = sa + P * kATile;
 #pragma unroll
             for (int ks = 0; ks < BK / 16; ++ks) {
 #pragma unroll
               for (int q = 0; q < Pairs<P>::n; ++q) {
-                const uint32_t ta = sa + Pairs<P>::a(q) * L::kATile;
-                const uint32_t tb = sb + Pairs<P>::b(q) * L::kBTile;
+                const uint32_t ta = sa + Pairs<P>::a(q) * kATile;
+                const uint32_t tb = sb + Pairs<P>::b(q) * b_tile;
                 // K-major: 32 bytes along the swizzled row per k-step of 16
                 // MN-major: 16 k-rows of 128 bytes per k-step
                 const uint64_t da = p.a_mn ? make_desc(ta + ks * 2048, BK * 128, 1024, 2u)
@@ -733,17 +771,16 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
     // registers and releases TMEM, so the next tile's MMAs start while it scales and stores.
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
-    uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes;
+    uint8_t *epi_stage = smem + kEpiOffset + (warp - 2) * kEpiBlockBytes;
     uint32_t unit = 0;
     bool ok = true;
     float slope_max = 0.f;
     MaxTracker maxima;
-    const int col_lo = half * 128;
-    for (int w = blockIdx.x; w < num_work && ok; w += gridDim.x) {
-      const Work x = decode_work<BM>(g, w);
+    for (Walk walk(g, blockIdx.x); ok && walk.next(g);) {
+      const Work x = walk.tile<BM>(g);
       const GemmProb &p = g.p[x.prob];
       const int row0 = x.m0 + q * 32;
-      const int col_hi = min(p.BN, col_lo + 128);
+      const int hc = half_columns(p.BN), col_lo = half * hc, col_hi = half ? p.BN : hc;
       const float *bias = x.split == 0 ? p.bias : nullptr;
       const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
       maxima.follow(p.absmax_out, lane);
@@ -764,10 +801,10 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
       }
       // wait for accumulation unit `unit`; where its columns stand
       auto finished = [&](int buf) {
-        ok = mbar_wait(&tmem_full[buf], (unit / kAccBufs) & 1, abort_flag, g.status, g.wait_limit_ns);
+        ok = mbar_wait(&tmem_full[buf], AccUnit(unit, two_accs).parity, abort_flag, g.status, g.wait_limit_ns);
         ok = __all_sync(0xffffffffu, ok);
         tcgen05_fence_after();
-        return tmem_base + ((uint32_t)(q * 32) << 16) + (P == 1 ? (uint32_t)buf * kTmemBuf : 0u);
+        return tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * kTmemBuf;
       };
       auto release = [&](int buf) {
         tcgen05_fence_before();
@@ -781,13 +818,13 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
         // bounds the short contractions (256 x 256 tiles of K = 1024: 9.0 us, of them 5.8 MMAs; 10.2
         // with the whole slice read first and every column checked against N).
         if (x.kb1 - x.kb0 <= p.kc) {
-          const int buf = unit % kAccBufs;
+          const int buf = AccUnit(unit, two_accs).buf;
           const uint32_t t_row = finished(buf);
           if (!ok) break;
 #pragma unroll
           for (int b = 0; b < 4; ++b) {
             const int cc = col_lo + 32 * b;
-            if (cc < col_hi) read_block<P>(v[0], t_row + cc, out_scale);
+            if (cc < col_hi) read_block<P>(v[0], t_row + cc, 0, out_scale);
             if (b == 3) release(buf);
             if (cc < col_hi)
               store_block(p, v[0], epi_stage, lane, row0, x.n0 + cc, x.split, bias != nullptr, bias_l[b],
@@ -797,11 +834,11 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
         }
       }
       for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc) {
-        const int buf = unit % kAccBufs;
+        const int buf = AccUnit(unit, two_accs).buf;
         const uint32_t t_row = finished(buf);
         if (!ok) break;
-        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
-        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        if (c0 == x.kb0) read_accumulator<P>(v, t_row, g.small_off, col_lo, col_hi, out_scale);
+        else add_accumulator<P>(v, t_row, g.small_off, col_lo, col_hi, out_scale);
         release(buf);                       // the slice is in registers now
       }
       if (!ok) break;
@@ -834,16 +871,14 @@ __device__ __forceinline__ void gemm_tc_body(const GemmGroup &g) {
   }
 }
 
-template <int P, int BK, int STAGES, int BN_CAP>
+template <int P, int BK>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const __grid_constant__ GemmGroup g) {
-  zp_after_previous();
-  gemm_tc_body<P, BK, STAGES, BN_CAP, ZP_EPI_NONE>(g);
+  gemm_tc_body<P, BK, ZP_EPI_NONE>(g);
 }
 // the same contraction with a fused epilogue (the epilogue warps hold more live values)
-template <int P, int BK, int STAGES, int BN_CAP, int EPI>
+template <int P, int BK, int EPI>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_fused_kernel(const __grid_constant__ GemmGroup g) {
-  zp_after_previous();
-  gemm_tc_body<P, BK, STAGES, BN_CAP, EPI>(g);
+  gemm_tc_body<P, BK, EPI>(g);
 }
 
 // ---- short contractions -------------------------------------------------------------------
@@ -874,7 +909,6 @@ struct ShortLayout {
 template <int P>
 __global__ void __launch_bounds__(kShortThreads, 1)
 gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
-  zp_after_previous();
   using L = ShortLayout<P>;
   constexpr int STAGES = L::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -920,6 +954,7 @@ gemm_tc_short_kernel(const __grid_constant__ GemmGroup g) {
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  zp_after_previous();                  // all of the above ran beside the kernel before
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
@@ -1126,40 +1161,27 @@ __device__ __forceinline__ void umma_pair(uint32_t tmem_d, uint64_t desc_a, uint
 
 constexpr int BM2 = 256;               // rows of a pair's tile
 
-template <int P, int BK, int STAGES>
-struct SmemLayoutPair {
-  static constexpr int kATile = BM * BK * 2;          // this CTA's 128 rows
-  static constexpr int kBTile = 128 * BK * 2;         // this CTA's half of a <= 256-wide B tile
-  static constexpr int kStage = P * (kATile + kBTile);
-  static constexpr int kTiles = STAGES * kStage;
-  static constexpr int kBars = 8 * (2 * STAGES + 4);
-  static_assert(kBars + 16 <= 1024, "control words fit in one KB");
-  static constexpr int kEpiOffset = kTiles + 1024;
-  static constexpr int kTotal = kTiles + 1024 + kEpiBytes + 1024;
-};
-
-template <int P, int BK, int STAGES, int EPI>
+template <int P, int BK, int EPI>
 __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
-  using L = SmemLayoutPair<P, BK, STAGES>;
+  constexpr int kATile = BM * BK * 2;                 // this CTA's 128 rows
   extern __shared__ uint8_t smem_raw[];
   // the dynamic shared window starts at the same offset in both CTAs, so does everything below
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                               ~(uintptr_t)1023);
-  uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::kTiles);
-  uint64_t *empty = full + STAGES;
-  uint64_t *tmem_full = empty + STAGES;
+  uint64_t *full = reinterpret_cast<uint64_t *>(smem + kTileBytes);
+  uint64_t *empty = full + kMaxStages;
+  uint64_t *tmem_full = empty + kMaxStages;
   uint64_t *tmem_empty = tmem_full + 2;
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tmem_empty + 2);
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const uint32_t rank = cluster_ctarank();          // 0 = leader
-  const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const int num_work = g.total;
+  const int pair = blockIdx.x >> 1;
 
   if (threadIdx.x == 0) {
     prefetch_maps(g);
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int s = 0; s < g.stages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 16); }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1179,31 +1201,32 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
   cluster_sync_all();                   // both allocations exist before the leader's first MMA
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-
-  const uint32_t a_bytes = BM * BK * 2;
+  zp_after_previous();                  // all of the above ran beside the kernel before
+  const int stages = g.stages;
+  const bool two_accs = P == 1 || g.acc_bufs == 2;
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer (both CTAs)
     if (!g.unarmed && elect_one()) {
-      uint32_t it = 0;
+      Ring ring;
       bool ok = true;
-      for (int w = pair; w < num_work && ok; w += num_pairs) {
-        const Work x = decode_work<BM2>(g, w);
+      for (Walk walk(g, pair); ok && walk.next(g);) {
+        const Work x = walk.tile<BM2>(g);
         const GemmProb &p = g.p[x.prob];
         const int half_n = p.BN >> 1;
         const uint32_t b_bytes = (uint32_t)half_n * BK * 2;
         const int m0 = x.m0 + (int)rank * BM, n0 = x.n0 + (int)rank * half_n;
-        for (int kb = x.kb0; kb < x.kb1 && ok; ++kb, ++it) {
-          const int s = it % STAGES;
-          ok = mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+        for (int kb = x.kb0; kb < x.kb1 && ok; ++kb, ring.next(stages)) {
+          const int s = ring.s;
+          ok = mbar_wait(&empty[s], ring.phase ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
-          uint8_t *st = smem + (size_t)s * L::kStage;
-          if (rank == 0) mbar_expect_tx(&full[s], 2 * P * (a_bytes + b_bytes));
+          uint8_t *st = smem + (size_t)s * g.stage_bytes;
+          if (rank == 0) mbar_expect_tx(&full[s], 2 * P * (kATile + b_bytes));
           const uint32_t bar = map_to_cta(smem_u32(&full[s]), 0);
           const int k0 = kb * BK;
 #pragma unroll
           for (int pl = 0; pl < P; ++pl) {
-            uint8_t *ta = st + pl * L::kATile, *tb = st + P * L::kATile + pl * L::kBTile;
+            uint8_t *ta = st + pl * kATile, *tb = st + P * kATile + pl * g.b_tile;
             if (!p.a_mn) {
               tma_load_3d_pair(ta, &p.map_a, bar, k0, m0, pl);
             } else {
@@ -1220,43 +1243,43 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
         }
       }
       // the leader's last stage releases must have landed here before this CTA may exit
-      for (int j = 0; j < STAGES && ok; ++j, ++it)
-        ok = mbar_wait(&empty[it % STAGES], ((it / STAGES) & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+      for (int j = 0; j < stages && ok; ++j, ring.next(stages))
+        ok = mbar_wait(&empty[ring.s], ring.phase ^ 1, abort_flag, g.status, g.wait_limit_ns);
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer (leader only)
     if (rank == 0 && elect_one()) {
       constexpr uint32_t kLayout = BK == 64 ? 2u : 4u;
-      uint32_t it = 0, unit = 0;
+      const int b_tile = g.b_tile;
+      uint32_t unit = 0;
+      Ring ring;
       bool ok = true;
-      for (int w = pair; w < num_work && ok; w += num_pairs) {
-        const Work x = decode_work<BM2>(g, w);
+      for (Walk walk(g, pair); ok && walk.next(g);) {
+        const Work x = walk.tile<BM2>(g);
         const GemmProb &p = g.p[x.prob];
         const uint32_t idesc = instr_desc(g, p, BM2);
         for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc, ++unit) {
           const int c1 = min(x.kb1, c0 + p.kc);
-          // one plane: the two accumulator buffers alternate, so the next tile's MMAs run
-          // while the epilogue drains this one
-          const int buf = P == 1 ? (int)(unit & 1) : 0;
-          const uint32_t round = P == 1 ? (unit >> 1) : unit;
-          ok = mbar_wait(&tmem_empty[buf], (round & 1) ^ 1, abort_flag, g.status, g.wait_limit_ns);
+          const AccUnit acc(unit, two_accs);
+          const int buf = acc.buf;
+          ok = mbar_wait(&tmem_empty[buf], acc.parity ^ 1, abort_flag, g.status, g.wait_limit_ns);
           if (!ok) break;
           tcgen05_fence_after();
           const uint32_t d_main = tmem_base + (uint32_t)buf * kTmemBuf;
-          const uint32_t d_small = tmem_base + kTmemBuf;
-          for (int kb = c0; kb < c1 && ok; ++kb, ++it) {
-            const int s = it % STAGES;
-            ok = mbar_wait(&full[s], (it / STAGES) & 1, abort_flag, g.status, g.wait_limit_ns);
+          const uint32_t d_small = d_main + g.small_off;
+          for (int kb = c0; kb < c1 && ok; ++kb, ring.next(stages)) {
+            const int s = ring.s;
+            ok = mbar_wait(&full[s], ring.phase, abort_flag, g.status, g.wait_limit_ns);
             if (!ok) break;
             tcgen05_fence_after();
-            const uint32_t sa = smem_u32(smem + (size_t)s * L::kStage);
-            const uint32_t sb = sa + P * L::kATile;
+            const uint32_t sa = smem_u32(smem + (size_t)s * g.stage_bytes);
+            const uint32_t sb = sa + P * kATile;
 #pragma unroll
             for (int ks = 0; ks < BK / 16; ++ks) {
 #pragma unroll
               for (int q = 0; q < Pairs<P>::n; ++q) {
-                const uint32_t ta = sa + Pairs<P>::a(q) * L::kATile;
-                const uint32_t tb = sb + Pairs<P>::b(q) * L::kBTile;
+                const uint32_t ta = sa + Pairs<P>::a(q) * kATile;
+                const uint32_t tb = sb + Pairs<P>::b(q) * b_tile;
                 const uint64_t da = p.a_mn ? make_desc(ta + ks * 2048, BK * 128, 1024, 2u)
                                            : make_desc(ta + ks * 32, 16, 8 * BK * 2, kLayout);
                 const uint64_t db = p.b_mn ? make_desc(tb + ks * 2048, BK * 128, 1024, 2u)
@@ -1276,19 +1299,18 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
     // ---------------------------------------------------------------- epilogue (both CTAs)
     const int q = warp & 3;
     const int half = (warp - 2) >> 2;
-    uint8_t *epi_stage = smem + L::kEpiOffset + (warp - 2) * kEpiBlockBytes;
+    uint8_t *epi_stage = smem + kEpiOffset + (warp - 2) * kEpiBlockBytes;
     uint32_t unit = 0;
     bool ok = true;
     float slope_max = 0.f;
     MaxTracker maxima;
-    const int col_lo = half * 128;
     const uint32_t release_bar0 = map_to_cta(smem_u32(&tmem_empty[0]), 0);
     const uint32_t release_bar1 = map_to_cta(smem_u32(&tmem_empty[1]), 0);
-    for (int w = pair; w < num_work && ok; w += num_pairs) {
-      const Work x = decode_work<BM2>(g, w);
+    for (Walk walk(g, pair); ok && walk.next(g);) {
+      const Work x = walk.tile<BM2>(g);
       const GemmProb &p = g.p[x.prob];
       const int row0 = x.m0 + (int)rank * BM + q * 32;
-      const int col_hi = min(p.BN, col_lo + 128);
+      const int hc = half_columns(p.BN), col_lo = half * hc, col_hi = half ? p.BN : hc;
       const float *bias = x.split == 0 ? p.bias : nullptr;
       const float out_scale = (p.scale_a ? *p.scale_a : 1.f) * (p.scale_b ? *p.scale_b : 1.f);
       maxima.follow(p.absmax_out, lane);
@@ -1309,7 +1331,7 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
       }
       // wait for accumulation unit `unit`; where its columns stand
       auto finished = [&](int buf) {
-        ok = mbar_wait(&tmem_full[buf], (P == 1 ? unit >> 1 : unit) & 1, abort_flag, g.status, g.wait_limit_ns);
+        ok = mbar_wait(&tmem_full[buf], AccUnit(unit, two_accs).parity, abort_flag, g.status, g.wait_limit_ns);
         ok = __all_sync(0xffffffffu, ok);
         tcgen05_fence_after();
         return tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)buf * kTmemBuf;
@@ -1326,13 +1348,13 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
         // bounds the short contractions (256 x 256 tiles of K = 1024: 9.0 us, of them 5.8 MMAs; 10.2
         // with the whole slice read first and every column checked against N).
         if (x.kb1 - x.kb0 <= p.kc) {
-          const int buf = (int)(unit & 1);
+          const int buf = AccUnit(unit, two_accs).buf;
           const uint32_t t_row = finished(buf);
           if (!ok) break;
 #pragma unroll
           for (int b = 0; b < 4; ++b) {
             const int cc = col_lo + 32 * b;
-            if (cc < col_hi) read_block<P>(v[0], t_row + cc, out_scale);
+            if (cc < col_hi) read_block<P>(v[0], t_row + cc, 0, out_scale);
             if (b == 3) release(buf);
             if (cc < col_hi)
               store_block(p, v[0], epi_stage, lane, row0, x.n0 + cc, x.split, bias != nullptr, bias_l[b],
@@ -1342,11 +1364,11 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
         }
       }
       for (int c0 = x.kb0; c0 < x.kb1 && ok; c0 += p.kc) {
-        const int buf = P == 1 ? (int)(unit & 1) : 0;
+        const int buf = AccUnit(unit, two_accs).buf;
         const uint32_t t_row = finished(buf);
         if (!ok) break;
-        if (c0 == x.kb0) read_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
-        else add_accumulator<P>(v, t_row, col_lo, col_hi, out_scale);
+        if (c0 == x.kb0) read_accumulator<P>(v, t_row, g.small_off, col_lo, col_hi, out_scale);
+        else add_accumulator<P>(v, t_row, g.small_off, col_lo, col_hi, out_scale);
         release(buf);                       // the slice is in registers now
       }
       if (!ok) break;
@@ -1381,16 +1403,14 @@ __device__ __forceinline__ void gemm_tc_pair_body(const GemmGroup &g) {
   }
 }
 
-template <int P, int BK, int STAGES>
+template <int P, int BK>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_pair_kernel(const __grid_constant__ GemmGroup g) {
-  zp_after_previous();
-  gemm_tc_pair_body<P, BK, STAGES, ZP_EPI_NONE>(g);
+  gemm_tc_pair_body<P, BK, ZP_EPI_NONE>(g);
 }
-template <int P, int BK, int STAGES, int EPI>
+template <int P, int BK, int EPI>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_pair_fused_kernel(const __grid_constant__ GemmGroup g) {
-  zp_after_previous();
-  gemm_tc_pair_body<P, BK, STAGES, EPI>(g);
+  gemm_tc_pair_body<P, BK, EPI>(g);
 }
 
 // block_node[b] = the last node n with row_ptr[n] <= 32 b: the node of the first edge of 32-edge
@@ -1519,7 +1539,7 @@ double launch_score(const ZpGemmTc &g, bool pair, int splits) {
   return pad * wave * feed * (1.0 - 0.004 * splits);
 }
 bool use_pair(const ZpGemmTc &g) {
-  if (g.planes != 2 && g.planes != 1) return false;
+  if (g.planes == 3 && g.variant == 1) return false;
   if (g.variant == 2) return false;
   if (g.variant == 3) return true;
   if (!pair_enabled()) return false;
@@ -1529,9 +1549,10 @@ bool use_pair(const ZpGemmTc &g) {
   return launch_score(g, true, s) >= launch_score(g, false, s);
 }
 
+int pair_block_k(int planes) { return planes == 3 ? 32 : 64; }
+int single_block_k(int planes, int variant) { return ((planes == 3 && variant != 1) || planes == 2) ? 32 : 64; }
 int block_k(const ZpGemmTc &g) {
-  if (use_pair(g)) return 64;
-  return ((g.planes == 3 && g.variant != 1) || g.planes == 2) ? 32 : 64;
+  return use_pair(g) ? pair_block_k(g.planes) : single_block_k(g.planes, g.variant);
 }
 
 // Split of the contraction in whole 64-deep steps, so that it does not depend on the kernel's k-block
@@ -1566,12 +1587,76 @@ bool fused_mode_ok(const ZpGemmTc &g, int bk) {
   return ksplit == 1 && kbs <= kc && (g.epi->width % 4) == 0;
 }
 
-// Describes the products of one launch: tile shapes, work items, tensor maps.  Products whose items
-// take longest come first, so that what is left for the last round is short.
-// tile_m: rows of a tile; box_m: rows of A one CTA loads; halves: CTAs that share a B tile
-int fill_group(GemmGroup &grp, const ZpGemmTc *const *g, int n, int P, int bk, int tile_m, int halves,
-               int bn_cap) {
-  if (n < 1 || n > ZP_GEMM_GROUP) return ZP_ERR_INVALID_ARG;
+// Time of a tile: its MMAs or its operands' way from L2 (38 bytes per clock and SM), whichever is longer, and what
+// its epilogue adds.  It only has to rank shapes: 60 000 x 1280 -> 1152 in two planes takes 422 us in the pair
+// kernel and 453 in the single one, in one plane 157 and 174.
+double tile_cost(int planes, int halves, int bn, int steps, bool two_accs) {
+  const int passes = planes == 1 ? 1 : planes == 2 ? 3 : 6;
+  const double mma = 2.5 * passes * bn, feed = planes * 128.0 * (BM + bn / halves) / 38.0;
+  const double main = steps * std::max(mma, feed), drain = 24.0 * bn;
+  return (two_accs ? std::max(main, drain) + 0.1 * drain : main + 0.35 * drain) + (halves == 2 ? 900.0 : 600.0);
+}
+
+// bk: depth of a k-block; cap: widest tile
+void plan_group(GroupPlan &pl, const ZpGemmTc *const *g, int n, bool pair, int bk, int cap, int units) {
+  Shape shape[ZP_GEMM_GROUP];
+  const int P = g[0]->planes, halves = pair ? 2 : 1, tile_m = pair ? 256 : BM;
+  pl.pair = pair;
+  pl.bk = bk;
+  pl.halves = halves;
+  pl.max_bn = 0;
+  for (int i = 0; i < n; ++i) {
+    const int step = bn_step(*g[i], halves);
+    shape[i].bn = pick_bn(g[i]->N, std::max(cap / step, 1) * step, step);
+    pl.max_bn = std::max(pl.max_bn, shape[i].bn);
+  }
+  const bool two_accs = P == 1 || pl.max_bn <= kTmemBuf / 2;
+  for (int i = 0; i < n; ++i) {
+    Shape &s = shape[i];
+    split_plan(*g[i], bk, &s.ksplit, &s.kbs, &s.num_k);
+    s.num_n = (int)zp_ceil_div(g[i]->N, s.bn);
+    s.tiles = zp_ceil_div(g[i]->M, tile_m) * s.num_n * s.ksplit;
+    s.cost = tile_cost(P, halves, s.bn, s.kbs * bk / 64, two_accs);
+    int k = i;
+    for (; k > 0 && shape[pl.order[k - 1]].cost < s.cost; --k) pl.order[k] = pl.order[k - 1];
+    pl.order[k] = i;
+  }
+  for (int k = 0; k < n; ++k) pl.shape[k] = shape[pl.order[k]];
+  share_out(pl, n, units);
+}
+
+// The plan of a launch.  `kernel`: 0 the single-CTA kernel, 1 the pair kernel, 2 whichever gets done first.
+// Wide tiles live on fewer operand bytes and are taken wherever they go round: whole passes of 6 000 to 18 000
+// edges took 4 to 7 % longer with tiles of at most 192 columns and 3 to 7 % with 128.  Where there are fewer tiles
+// than units, narrower ones share the work out.
+void plan_launch(GroupPlan &pl, const ZpGemmTc *const *g, int n, int kernel) {
+  const int P = g[0]->planes, sms = device_sms();
+  const bool narrow = P == 3 && g[0]->variant == 1;
+  const int bk = single_block_k(P, g[0]->variant), widest = narrow ? 128 : 256;
+  if (kernel == 1) {
+    plan_group(pl, g, n, true, pair_block_k(P), widest, sms / 2);
+  } else {
+    plan_group(pl, g, n, false, bk, widest, sms);
+    if (kernel == 2) {
+      GroupPlan other;
+      plan_group(other, g, n, true, pair_block_k(P), widest, sms / 2);
+      if (other.makespan <= pl.makespan) pl = other;
+    }
+  }
+  int64_t tiles = 0;
+  for (int k = 0; k < n; ++k) tiles += pl.shape[k].tiles;
+  const int units = pl.pair ? sms / 2 : sms;
+  if (narrow || tiles >= units) return;
+  for (int cap : {192, 128, 64}) {
+    GroupPlan other;
+    plan_group(other, g, n, pl.pair, pl.bk, cap, units);
+    if (other.makespan < 0.97 * pl.makespan) pl = other;
+  }
+}
+
+// Describes a launch to the kernel.
+int fill_group(GemmGroup &grp, const GroupPlan &pl, const ZpGemmTc *const *g, int n) {
+  const int P = g[0]->planes, bk = pl.bk, halves = pl.halves;
   grp.n = n;
   grp.fp16 = g[0]->fp16;
   grp.status = g[0]->status;
@@ -1580,31 +1665,34 @@ int fill_group(GemmGroup &grp, const ZpGemmTc *const *g, int n, int P, int bk, i
   const ZpEpilogue *epi = g[0]->epi;
   if (epi) grp.epi = *epi;
   else grp.epi.mode = ZP_EPI_NONE;
-  int order[ZP_GEMM_GROUP];
-  int64_t cost[ZP_GEMM_GROUP];
-  for (int i = 0; i < n; ++i) {
-    int ksplit, kbs, num_k;
-    split_plan(*g[i], bk, &ksplit, &kbs, &num_k);
-    cost[i] = (int64_t)kbs * pick_bn(g[i]->N, bn_cap, bn_step(*g[i], halves));
-    int k = i;
-    for (; k > 0 && cost[order[k - 1]] < cost[i]; --k) order[k] = order[k - 1];
-    order[k] = i;
+  grp.classes = pl.classes;
+  std::copy(pl.unit0, pl.unit0 + pl.classes + 1, grp.unit0);
+  for (int c = 0; c < pl.classes; ++c) {
+    std::copy(pl.first[c], pl.first[c] + n, grp.first[c]);
+    std::copy(pl.count[c], pl.count[c] + n, grp.count[c]);
   }
+  grp.b_tile = pl.max_bn / halves * bk * 2;
+  grp.stage_bytes = P * (BM * bk * 2 + grp.b_tile);
+  grp.stages = std::min(kMaxStages, kTileBytes / grp.stage_bytes);
+  // one plane: one accumulator, alternating between two of 256 columns; two or three: the leading product's
+  // and the small ones', twice side by side where both fit 256 columns
+  grp.acc_bufs = P == 1 || pl.max_bn <= kTmemBuf / 2 ? 2 : 1;
+  grp.small_off = pl.max_bn <= kTmemBuf / 2 ? kTmemBuf / 2 : kTmemBuf;
   const CUtensorMapSwizzle kswz = bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
   grp.total = 0;
   for (int k = 0; k < n; ++k) {
-    const ZpGemmTc &q = *g[order[k]];
+    const ZpGemmTc &q = *g[pl.order[k]];
+    const Shape &s = pl.shape[k];
     GemmProb &p = grp.p[k];
     p.M = (int)q.M; p.N = (int)q.N;
-    split_plan(q, bk, &p.ksplit, &p.kb_per_split, &p.num_k);
+    p.ksplit = s.ksplit; p.kb_per_split = s.kbs; p.num_k = s.num_k;
     const int kc_elems = q.kc_elems > 0 ? q.kc_elems : 2048;
     p.kc = kc_elems / bk < 1 ? 1 : kc_elems / bk;
     p.a_mn = q.a_mn; p.b_mn = q.b_mn;
     p.scale_a = q.scale_a; p.scale_b = q.scale_b; p.absmax_out = q.absmax_out; p.bias = q.bias;
-    p.BN = pick_bn(q.N, bn_cap, bn_step(q, halves));
-    p.num_n = (int)zp_ceil_div(q.N, p.BN);
-    p.start = grp.total;
-    grp.total += (int)zp_ceil_div(q.M, tile_m) * p.num_n * p.ksplit;
+    p.BN = s.bn;
+    p.num_n = s.num_n;
+    grp.total += (int)s.tiles;
     int rc;
     if (!q.a_mn) rc = make_map(&p.map_a, q.A, q.K, q.M, P, q.lda, q.a_plane, bk, BM, kswz, q.fp16);
     else rc = make_map(&p.map_a, q.A, q.M, q.K, P, q.lda, q.a_plane, 64, bk, CU_TENSOR_MAP_SWIZZLE_128B, q.fp16);
@@ -1618,21 +1706,18 @@ int fill_group(GemmGroup &grp, const ZpGemmTc *const *g, int n, int P, int bk, i
   return ZP_OK;
 }
 
-template <int P, int BK, int STAGES, int BN_CAP, int EPI>
-int launch_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
-  using L = SmemLayout<P, BK, STAGES, BN_CAP>;
-  static_assert(L::kTotal <= 232448, "shared memory budget of one CTA");
+template <int P, int BK, int EPI>
+int launch_e(const ZpGemmTc *const *g, int n, const GroupPlan &pl, cudaStream_t st) {
   auto kernel = [] {
-    if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_kernel<P, BK, STAGES, BN_CAP>;
-    else return gemm_tc_fused_kernel<P, BK, STAGES, BN_CAP, EPI>;
+    if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_kernel<P, BK>;
+    else return gemm_tc_fused_kernel<P, BK, EPI>;
   }();
   static ZpSmemOptIn opt_in;
   int rc;
-  if ((rc = zp_ensure_smem(kernel, (size_t)L::kTotal, opt_in))) return rc;
+  if ((rc = zp_ensure_smem(kernel, (size_t)kSmemTotal, opt_in))) return rc;
   GemmGroup grp;
-  if ((rc = fill_group(grp, g, n, P, BK, BM, 1, BN_CAP))) return rc;
-  const int sms = device_sms(), grid = grp.total < sms ? grp.total : sms;
-  zp_launch(kernel, grid, kThreads, L::kTotal, st, grp);
+  if ((rc = fill_group(grp, pl, g, n))) return rc;
+  zp_launch(kernel, (unsigned)pl.units, kThreads, kSmemTotal, st, grp);
   ZP_LAUNCH_CHECK("gemm_tc_kernel");
   return ZP_OK;
 }
@@ -1645,9 +1730,12 @@ int launch_short(const ZpGemmTc &g, cudaStream_t st) {
   int rc;
   if ((rc = zp_ensure_smem(gemm_tc_short_kernel<P>, (size_t)L::kTotal, opt_in))) return rc;
   GemmGroup grp;
+  GroupPlan pl;
   const ZpGemmTc *one = &g;
-  if ((rc = fill_group(grp, &one, 1, P, kShortBK, BM, 1, kShortBN))) return rc;
-  const int sms = device_sms(), columns = grp.p[0].num_n, rows = grp.total / columns;
+  const int sms = device_sms();
+  plan_group(pl, &one, 1, false, kShortBK, kShortBN, sms);
+  if ((rc = fill_group(grp, pl, &one, 1))) return rc;
+  const int columns = grp.p[0].num_n, rows = grp.total / columns;
   grp.rows_apart = columns <= sms ? std::min(sms / columns, rows) : 0;
   if (grp.rows_apart < rows && columns * grp.rows_apart * 10 < sms * 9) grp.rows_apart = 0;
   const int grid = grp.rows_apart ? columns * grp.rows_apart : std::min(grp.total, sms);
@@ -1656,67 +1744,77 @@ int launch_short(const ZpGemmTc &g, cudaStream_t st) {
   return ZP_OK;
 }
 
-template <int P, int BK, int STAGES, int BN_CAP>
-int launch(const ZpGemmTc *const *g, int n, cudaStream_t st) {
+template <int P, int BK>
+int launch(const ZpGemmTc *const *g, int n, const GroupPlan &pl, cudaStream_t st) {
   const int mode = g[0]->epi ? g[0]->epi->mode : ZP_EPI_NONE;
   if constexpr (P == 1 || P == 2) {
-    if (mode == ZP_EPI_GATE) return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_GATE>(g, n, st);
-    if (mode == ZP_EPI_ROTATE_BACK) return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_ROTATE_BACK>(g, n, st);
+    if (mode == ZP_EPI_GATE) return launch_e<P, BK, ZP_EPI_GATE>(g, n, pl, st);
+    if (mode == ZP_EPI_ROTATE_BACK) return launch_e<P, BK, ZP_EPI_ROTATE_BACK>(g, n, pl, st);
   }
   if (mode != ZP_EPI_NONE) return ZP_ERR_UNSUPPORTED;
-  return launch_e<P, BK, STAGES, BN_CAP, ZP_EPI_NONE>(g, n, st);
+  return launch_e<P, BK, ZP_EPI_NONE>(g, n, pl, st);
 }
 
-template <int P, int BK, int STAGES, int EPI>
-int launch_pair_e(const ZpGemmTc *const *g, int n, cudaStream_t st) {
-  using L = SmemLayoutPair<P, BK, STAGES>;
-  static_assert(L::kTotal <= 232448, "shared memory budget of one CTA");
-  auto kernel = [] {
-    if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_pair_kernel<P, BK, STAGES>;
-    else return gemm_tc_pair_fused_kernel<P, BK, STAGES, EPI>;
-  }();
-  cudaLaunchAttribute attr[2];
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = L::kTotal; cfg.stream = st;
-  cfg.attrs = attr; cfg.numAttrs = 1;
+// CTA pairs of a kernel that the device holds at a time
+template <typename Kernel>
+int resident_pairs(Kernel *kernel, PerDevice &pairs, int *count) {
   int dev = 0;
   ZP_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) return ZP_ERR_UNSUPPORTED;
-  static PerDevice pairs;               // co-resident CTA pairs of this kernel, per device
-  int max_pairs;
-  {
-    std::lock_guard<std::mutex> hold(pairs.lock);
-    if (!pairs.done[dev]) {
-      ZP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-      const int sms = device_sms();
-      int fit = 0;
-      cfg.gridDim = dim3((unsigned)(sms / 2 * 2));
-      ZP_CUDA(cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg));
-      pairs.value[dev] = fit < sms / 2 ? fit : sms / 2;
-      pairs.done[dev] = true;
-    }
-    max_pairs = pairs.value[dev];
+  std::lock_guard<std::mutex> hold(pairs.lock);
+  if (!pairs.done[dev]) {
+    ZP_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemTotal));
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    const int sms = device_sms();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sms / 2 * 2)); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = kSmemTotal;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    int fit = 0;
+    ZP_CUDA(cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg));
+    pairs.value[dev] = fit < sms / 2 ? fit : sms / 2;
+    pairs.done[dev] = true;
   }
-  if (max_pairs < 1) return ZP_ERR_UNSUPPORTED;
+  *count = pairs.value[dev];
+  return *count < 1 ? ZP_ERR_UNSUPPORTED : ZP_OK;
+}
+
+template <int P, int BK, int EPI>
+int launch_pair_e(const ZpGemmTc *const *g, int n, const GroupPlan &planned, cudaStream_t st) {
+  auto kernel = [] {
+    if constexpr (EPI == ZP_EPI_NONE) return gemm_tc_pair_kernel<P, BK>;
+    else return gemm_tc_pair_fused_kernel<P, BK, EPI>;
+  }();
+  static PerDevice pairs;
+  int rc, units;
+  if ((rc = resident_pairs(kernel, pairs, &units))) return rc;
+  GroupPlan pl = planned;
+  if (pl.units > units) plan_group(pl, g, n, true, BK, 256, units);     // fewer than half the SMs
   GemmGroup grp;
-  if (const int rc = fill_group(grp, g, n, P, BK, BM2, 2, 256)) return rc;
-  cfg.gridDim = dim3((unsigned)(2 * (grp.total < max_pairs ? grp.total : max_pairs)));
-  cfg.numAttrs = 2;
+  if ((rc = fill_group(grp, pl, g, n))) return rc;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * pl.units)); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = kSmemTotal;
+  cfg.stream = st; cfg.attrs = attr; cfg.numAttrs = 2;
   ZP_CUDA(cudaLaunchKernelEx(&cfg, kernel, grp));
   ZP_LAUNCH_CHECK("gemm_tc_pair_kernel");
   return ZP_OK;
 }
 
-template <int P, int BK, int STAGES>
-int launch_pair(const ZpGemmTc *const *g, int n, cudaStream_t st) {
+template <int P, int BK>
+int launch_pair(const ZpGemmTc *const *g, int n, const GroupPlan &pl, cudaStream_t st) {
   const int mode = g[0]->epi ? g[0]->epi->mode : ZP_EPI_NONE;
-  if (mode == ZP_EPI_GATE) return launch_pair_e<P, BK, STAGES, ZP_EPI_GATE>(g, n, st);
-  if (mode == ZP_EPI_ROTATE_BACK) return launch_pair_e<P, BK, STAGES, ZP_EPI_ROTATE_BACK>(g, n, st);
-  return launch_pair_e<P, BK, STAGES, ZP_EPI_NONE>(g, n, st);
+  if constexpr (P == 1 || P == 2) {
+    if (mode == ZP_EPI_GATE) return launch_pair_e<P, BK, ZP_EPI_GATE>(g, n, pl, st);
+    if (mode == ZP_EPI_ROTATE_BACK) return launch_pair_e<P, BK, ZP_EPI_ROTATE_BACK>(g, n, pl, st);
+  }
+  if (mode != ZP_EPI_NONE) return ZP_ERR_UNSUPPORTED;
+  return launch_pair_e<P, BK, ZP_EPI_NONE>(g, n, pl, st);
 }
 
 int check_product(const ZpGemmTc &g) {
@@ -1732,18 +1830,33 @@ int check_product(const ZpGemmTc &g) {
   return ZP_OK;
 }
 
-// the launch for products of one format that all go the same way
-int dispatch(const ZpGemmTc *const *g, int n, bool pair, cudaStream_t st) {
+// Whether a group may go to the pair kernel: not where most of the work has short contractions, which leave its
+// cross-SM hand-offs exposed on every tile
+bool group_may_pair(const ZpGemmTc *const *g, int n) {
+  double work = 0.0, deep = 0.0;
+  for (int i = 0; i < n; ++i) {
+    const double w = (double)g[i]->M * (double)g[i]->N * (double)g[i]->K;
+    work += w;
+    if (g[i]->K >= 512) deep += w;
+  }
+  return pair_enabled() && deep > 0.5 * work;
+}
+
+// the launch for products of one format; `kernel` as for plan_launch
+int dispatch(const ZpGemmTc *const *g, int n, int kernel, cudaStream_t st) {
   const int planes = g[0]->planes;
-  if (pair) return planes == 2 ? launch_pair<2, 64, 3>(g, n, st) : launch_pair<1, 64, 6>(g, n, st);
-  const bool is_short = n == 1 && !g[0]->a_mn && !g[0]->b_mn && !(g[0]->epi && g[0]->epi->mode) &&
+  if (planes < 1 || planes > 3) return ZP_ERR_UNSUPPORTED;
+  const bool is_short = kernel == 0 && n == 1 && !g[0]->a_mn && !g[0]->b_mn && !(g[0]->epi && g[0]->epi->mode) &&
                         g[0]->ksplit <= 1 && g[0]->variant == 0 && g[0]->K * planes <= 256;
-  if (planes == 2) return is_short ? launch_short<2>(*g[0], st) : launch<2, 32, 4, 256>(g, n, st);
-  if (planes == 1) return is_short ? launch_short<1>(*g[0], st) : launch<1, 64, 4, 256>(g, n, st);
-  // three planes: two stages of six MMA passes each leave room for the store blocks
-  if (planes == 3)
-    return g[0]->variant == 1 ? launch<3, 64, 2, 128>(g, n, st) : launch<3, 32, 2, 256>(g, n, st);
-  return ZP_ERR_UNSUPPORTED;
+  if (is_short && planes <= 2) return planes == 2 ? launch_short<2>(*g[0], st) : launch_short<1>(*g[0], st);
+  GroupPlan pl;
+  plan_launch(pl, g, n, kernel);
+  if (pl.pair)
+    return planes == 2 ? launch_pair<2, 64>(g, n, pl, st) : planes == 1 ? launch_pair<1, 64>(g, n, pl, st)
+                                                                        : launch_pair<3, 32>(g, n, pl, st);
+  if (planes == 2) return launch<2, 32>(g, n, pl, st);
+  if (planes == 1) return launch<1, 64>(g, n, pl, st);
+  return pl.bk == 64 ? launch<3, 64>(g, n, pl, st) : launch<3, 32>(g, n, pl, st);
 }
 
 }  // namespace
@@ -1767,21 +1880,24 @@ int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits) {
   return best;
 }
 
-// One K split for all products of a group (their contraction is the same): the one whose rounds of
-// work items leave the least of the device idle.
-void zp_gemm_group_splits(ZpGemmTc *g, int n, int max_splits) {
-  const bool pair = use_pair(g[0]);
-  const int64_t units = pair ? device_sms() / 2 : device_sms();
-  int64_t tiles = 0;
-  for (int i = 0; i < n; ++i)
-    tiles += zp_ceil_div(g[i].M, pair ? BM2 : BM) * zp_ceil_div(g[i].N, pick_bn(g[i].N, 256, bn_step(g[i], pair ? 2 : 1)));
+// The K split of a group's products whose contraction runs over the edges (the last `nw` of n): the one
+// with which the launch gets done first, but no more partial results than that takes.
+void zp_gemm_group_splits(ZpGemmTc *g, int n, int nw, int max_splits) {
+  const ZpGemmTc *all[ZP_GEMM_GROUP];
+  if (n > ZP_GEMM_GROUP) n = ZP_GEMM_GROUP;
+  for (int i = 0; i < n; ++i) all[i] = &g[i];
+  const bool pair = group_may_pair(all, n);
   int best = 1;
-  double best_cost = 1e30;
+  double best_cost = 1e300;
   for (int s = 1; s <= max_splits; ++s) {
-    const double cost = (double)zp_ceil_div(tiles * s, units) / s + 0.004 * s;
+    for (int i = n - nw; i < n; ++i) g[i].ksplit = s;
+    GroupPlan pl;
+    plan_group(pl, all, n, pair, pair ? pair_block_k(all[0]->planes) : single_block_k(all[0]->planes, 0), 256,
+               pair ? device_sms() / 2 : device_sms());
+    const double cost = pl.makespan * (1.0 + 0.004 * s);
     if (cost < best_cost) { best_cost = cost; best = s; }
   }
-  for (int i = 0; i < n; ++i) g[i].ksplit = best;
+  for (int i = n - nw; i < n; ++i) g[i].ksplit = best;
 }
 
 int zp_launch_block_nodes(int64_t E, int64_t N, const int32_t *row_ptr, int32_t *block_node,
@@ -1803,23 +1919,18 @@ int zp_launch_gemm_tc(const ZpGemmTc &g, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0) return ZP_OK;
   if (const int rc = check_product(g)) return rc;
   const ZpGemmTc *one = &g;
-  return dispatch(&one, 1, use_pair(g), st);
+  return dispatch(&one, 1, use_pair(g) ? 1 : 0, st);
 }
 
-// Several independent products of one format in one launch.  The CTA-pair kernel takes them when
-// it would take most of the work on its own.
+// Several independent products of one format in one launch.
 int zp_launch_gemm_group(const ZpGemmTc *g, int n, cudaStream_t st) {
   const ZpGemmTc *live[ZP_GEMM_GROUP];
   int k = 0;
-  double pair_work = 0.0, work = 0.0;
   for (int i = 0; i < n; ++i) {
     if (g[i].M <= 0 || g[i].N <= 0) continue;
     if (const int rc = check_product(g[i])) return rc;
     if (k == ZP_GEMM_GROUP || (g[i].epi && g[i].epi->mode) || g[i].planes != g[0].planes) return ZP_ERR_INVALID_ARG;
-    const double w = (double)g[i].M * (double)g[i].N * (double)g[i].K;
-    work += w;
-    if (use_pair(g[i])) pair_work += w;
     live[k++] = &g[i];
   }
-  return k ? dispatch(live, k, pair_work > 0.5 * work, st) : ZP_OK;
+  return k ? dispatch(live, k, group_may_pair(live, k) ? 2 : 0, st) : ZP_OK;
 }
