@@ -71,9 +71,11 @@ def gemm_macs_per_edge(cfg) -> int:
     return total
 
 
-def hbm_bytes_per_step(block, n: int, e: int) -> dict:
+def hbm_bytes_per_step(block, n: int, e: int, by_node: bool = False) -> dict:
     """Algorithmic bytes one step moves in each HBM-bound kernel class (timing class names of the
-    library): fp32 arrays 4 bytes per value, 16-bit operand planes 2 bytes per value and plane."""
+    library): fp32 arrays 4 bytes per value, 16-bit operand planes 2 bytes per value and plane.
+    ``by_node``: the gradient of the embeddings is summed node by node within rotate_in_bwd instead of from
+    contributions written per edge."""
     c = block.cfg
     lay = block.layout
     K, Km = (c.lmax + 1) ** 2, lay.m_size[0] + 2 * sum(lay.m_size[1:])
@@ -96,6 +98,9 @@ def hbm_bytes_per_step(block, n: int, e: int) -> dict:
     }
     per_node = {"rotate_back_scatter": K * C * 4 + (nnz * C * 4 if fused else 0),
                 "src_reduce": K * C * 4}
+    if by_node:
+        per_edge["rotate_in_bwd"] -= per_edge.pop("src_reduce")
+        per_node["rotate_in_bwd"] = per_node.pop("src_reduce")
     return {k: int(e * v + n * per_node.get(k, 0)) for k, v in per_edge.items()}
 
 
@@ -508,7 +513,7 @@ def run_ours(args) -> dict | None:
     launches = sum(v[1] for v in timing.values()) / args.steps
     # HBM-side kernel classes: algorithmic bytes per step (each operand once; gathered node rows
     # come from L2 and are not counted) against the measured copy bandwidth
-    for k, nbytes in hbm_bytes_per_step(block, n, e).items():
+    for k, nbytes in hbm_bytes_per_step(block, n, e, by_node="src_reduce" not in kernels).items():
         if k in kernels and kernels[k]["ms_per_step"] > 0:
             gbs = nbytes / (kernels[k]["ms_per_step"] * 1e-3) / 1e9
             kernels[k]["hbm"] = {"algorithmic_bytes": nbytes, "gbs": gbs,

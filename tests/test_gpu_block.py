@@ -407,3 +407,30 @@ def test_weights_of_the_edge_convolution_by_size():
         assert torch.equal(want, eso2.EdgeConvFunction.apply(plan, graph, *ins, *flat))
         with pytest.raises(AssertionError):
             eso2.EdgeConvFunction.apply(plan, graph, *ins, w[0][:-1], *w[1:])
+
+
+@pytest.mark.parametrize("lmax,mmax,c,precision", [(4, 2, 128, "fp32"), (2, 2, 16, "fp32_bf16x3"), (3, 1, 40, "fp32"),
+                                                   (1, 1, 72, "fp32"), (4, 4, 160, "fp32"), (5, 2, 136, "fp32"),
+                                                   (6, 2, 24, "fp32_bf16x3"), (2, 0, 256, "fp32"), (1, 0, 8, "fp32")])
+def test_rotations_by_node_of_uneven_degrees(lmax, mmax, c, precision, jd64):
+    """Nodes of no edge, of one, of fewer than a block has workers, and a hub each way; with and without a
+    gradient of x_node."""
+    cfg = dict(lmax=lmax, mmax=mmax, sphere_channels=c, hidden_channels=16, edge_channels=8,
+               num_distance_basis=6, cutoff=5.0)
+    params = orc.init_params(cfg, seed=71)
+    case = random_case(cfg, 30, 260, seed=72)
+    ei = case["edge_index"]
+    ei[1, :90] = 4                                     # into one
+    ei[0, 90:150] = 7                                  # out of one
+    ei[:, 150:] = torch.where((ei[:, 150:] == 9) | (ei[:, 150:] == 0), 11, ei[:, 150:])
+    ei[0] = torch.where(ei[0] == ei[1], (ei[0] + 1) % 29 + 1, ei[0])
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    block = make_block(cfg, params, precision=precision)
+    got = gpu_node_out_and_vjp(block, case, case["upstream"])
+    check_against(*got, *want)
+    block.requires_grad_(False)
+    pos = case["pos"].cuda().float().requires_grad_(True)
+    out = block.node_output(pos, case["atomic_numbers"].cuda(), case["x_node"].cuda().float(), ei.cuda(),
+                            *(case[k].cuda().float() for k in ("shifts", "cos_gamma_k", "sin_gamma_k")))
+    (gpos,) = torch.autograd.grad(out, pos, case["upstream"].cuda().float())
+    assert rel_l2(gpos, want[2]) < 1e-5

@@ -121,8 +121,7 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
     w.dht = c.floats(e * t.Km * t.H);
     w.dh1 = c.planes(E, t.w1_cols, f, w.scales + kScDh1);
     w.da1 = c.floats(e * t.Km * 2 * t.C);
-    w.du_src = c.floats(e * 2 * t.K * t.C);
-    w.torque = c.floats(e * 4);
+    w.torque = c.floats(e * 4 * (size_t)zp_torque_slots(t));
     w.rot_grad = t.Km * t.H >= t.nnz_pad ? w.dht : c.floats(e * t.nnz_pad);
     w.wgrad = c.floats((size_t)kZpWgradSplits * p->g_elems);
     auto column_parts = [&](int64_t cols) { return c.floats((size_t)(zp_colsum_parts(E, cols) * cols)); };
@@ -452,7 +451,7 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
   const bool lean = !keep && fuse1 && fuse2;          // h1 rows and y are never written
   // |rot row . x| <= sqrt(2l+1) max|x|, over the rows the edges name
   ZP_TIMED(ZP_K_ROTATE_IN,
-           zp_launch_rotate_in(plan, c.E, c.x_node, c.src, c.dst, ws.rot, c.radial, ws.a1,
+           zp_launch_rotate_in(plan, c.E, c.x_node, c.src, c.dst, c.view, ws.rot, c.radial, ws.a1,
                                zp_scale_of(3.7f, ws.scales + kScX, ws.scales + kScA1, ws.scales + kScRad),
                                st));
   const int64_t N = c.N, E = c.E;
@@ -680,9 +679,6 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   // gw == NULL: the parameters are frozen (an MD / inference force evaluation): no weight-gradient
   // product, no bias column sum, no unfolding
   const bool want_w = gw != nullptr;
-  // grad_x_node == NULL: the embeddings are an input without a gradient (E and dE/dpos of one
-  // block): the per-edge contributions are neither written nor summed
-  float *du_out = grad_x_node ? ws.du_src : nullptr;
   const ZpTables &t = plan->t;
   const int P = plan->planes;
   const int64_t lda = (int64_t)t.Km * 2 * t.C, ldh = (int64_t)t.Km * t.H;
@@ -699,7 +695,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                         ws.scales + kScG, st));
   }
   ZP_TIMED(ZP_K_ROTATE_GRAD_OUT,
-           zp_launch_rotate_grad_out(plan, E, grad_node_out, ws.y, c.env, ws.rot, c.dst, ws.dy,
+           zp_launch_rotate_grad_out(plan, N, E, grad_node_out, ws.y, c.env, ws.rot, c.dst, c.row_ptr, ws.dy,
                                      zp_scale_of(3.7f, ws.scales + kScG, ws.scales + kScDy), grad_env,
                                      ws.torque, st));
   // One conv at a time: input gradient dX = dY W_fold (K-major against the transposed planes),
@@ -778,15 +774,15 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   // With the layer inside the call grad_radial leaves the kernel as operand planes for the layer's
   // VJP; their scale comes from |grad_radial| <= 2 max|da1| max|rot . x| <= 2 * 3.7 max|da1| max|x|
   ZP_TIMED(ZP_K_ROTATE_IN_BWD,
-           zp_launch_rotate_in_bwd(plan, E, ws.da1, radial, c.x_node, c.src, c.dst, ws.rot,
-                                   rl ? nullptr : grad_radial, du_out, ws.torque, st,
-                                   rl ? &ws.gr : nullptr,
+           zp_launch_rotate_in_bwd(plan, N, E, ws.da1, radial, c.x_node, c.row_ptr, c.perm_src,
+                                   c.row_ptr_src, ws.rot, rl ? nullptr : grad_radial, grad_x_node, ws.torque,
+                                   st, rl ? &ws.gr : nullptr,
                                    zp_scale_of(7.4f, ws.scales + kScDa1, ws.scales + kScGrScale,
                                                ws.scales + kScX)));
   // What is left are short kernels, most of them waiting on one another.  On the caller's stream
   // the way to the positions, first of all its product: a product takes whole SMs and waits for all
   // that was there before it.  On the second side stream the radial layer's parameter gradients,
-  // on the first the last sums of the convolutions' and the node sums.
+  // on the first the last sums of the convolutions'.
   if ((rc = lanes.fork())) return rc;
   if (rl && E > 0) {
     ZpFinalList radial_list;
@@ -804,12 +800,9 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
     zp_add_so2_grads(plan, ws.wgrad, plan->g_elems, splits_c1, splits_c2, gw, list);
     ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(list, lanes.pick(1)));
   }
-  if (grad_x_node)
-    ZP_TIMED(ZP_K_SRC_REDUCE,
-             zp_launch_node_reduce(plan, N, ws.du_src, c.row_ptr, c.perm_src, c.row_ptr_src,
-                                   grad_x_node, lanes.pick(1)));
   ZP_TIMED(ZP_K_WIGNER_BWD,
            zp_launch_edge_vec_grad(plan, E, c.edge_vec, c.cos_g, c.sin_g, ws.torque,
+                                   zp_torque_slots(t),
                                    ZpTorqueArgs{ws.da1, radial, c.x_node, ws.y, grad_node_out, c.env,
                                                 c.src, c.dst, ws.rot_grad},
                                    grad_edge_vec, st));

@@ -242,8 +242,10 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
       ZP_TIMED(ZP_K_FOLD, zp_launch_max_list(x_max, st));
     }
   }
-  const ZpConv c{N, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
-                 call->dst, call->row_ptr + call->first_node, nullptr, nullptr, &params->so2};
+  ZpConv c{N, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
+           call->dst, call->row_ptr + call->first_node, nullptr, nullptr, &params->so2};
+  if (call->perm_src && call->row_ptr_src)
+    c.view = ZpNodeView{call->n_rows, call->row_ptr, call->perm_src, call->row_ptr_src};
   return zp_core_forward(plan, ws, c, node_out, keep_for_backward, lanes);
 }
 

@@ -235,7 +235,7 @@ int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const flo
                          const float *sg, const float *grot, float *gev, cudaStream_t st);
 
 // The arrays of one edge convolution's VJP that an edge's rotation gradient comes from.
-// torque [E, 4]: for each edge the derivative of the loss under a rotation of the edge frame about
+// torque [slots][E, 4], to be summed over the slots: for each edge the derivative of the loss under a rotation of the edge frame about
 // its own axis (entry 0) and the two axes perpendicular to it (1, 2).
 struct ZpTorqueArgs {
   const float *da1, *radial, *x, *y, *g_out, *env;
@@ -244,33 +244,37 @@ struct ZpTorqueArgs {
 };
 // torque -> gradient of the edge vectors
 int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const float *cg,
-                            const float *sg, const float *torque, const ZpTorqueArgs &a, float *gev,
+                            const float *sg, const float *torque, int slots, const ZpTorqueArgs &a, float *gev,
                             cudaStream_t st);
 
+// All nodes that the edges name, with the edges into and out of each; perm_src null: the caller has no view by source
+struct ZpNodeView {
+  int64_t nodes;
+  const int32_t *row_ptr, *perm_src, *row_ptr_src;
+};
 int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32_t *src,
-                        const int32_t *dst, const float *rot, const float *radial,
+                        const int32_t *dst, const ZpNodeView &view, const float *rot, const float *radial,
                         const ZpPlanes &a1, const ZpScale &scale, cudaStream_t st);
 int zp_launch_rotate_back_scatter(const zp_plan *p, int64_t N, const float *y, const float *env,
                                   const float *rot, const int32_t *row_ptr, float *node_out,
                                   cudaStream_t st);
-int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const float *y,
-                              const float *env, const float *rot, const int32_t *dst,
+int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const float *g, const float *y,
+                              const float *env, const float *rot, const int32_t *dst, const int32_t *row_ptr,
                               const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
                               float *torque, cudaStream_t st);
-// du_both [E][2][K][C]: per-edge contributions to grad_x of the source (0) and destination (1)
-// grad_radial goes out as fp32 rows [E, R], or (grad_radial_planes given) as operand planes
-int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const float *radial,
-                            const float *x, const int32_t *src, const int32_t *dst,
-                            const float *rot, float *grad_radial, float *du_both, float *torque,
-                            cudaStream_t st, const ZpPlanes *grad_radial_planes,
-                            const ZpScale &scale);
+// grad_radial goes out as fp32 rows [E, R], or (grad_radial_planes given) as operand planes.  grad_x null:
+// nobody wants the gradient of x_node.  Slot 0 of torque holds what rotate_grad_out has left; as many slots are
+// written or added to as zp_torque_slots says.
+int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float *da1, const float *radial,
+                            const float *x, const int32_t *row_ptr, const int32_t *perm_src,
+                            const int32_t *row_ptr_src, const float *rot, float *grad_radial, float *grad_x,
+                            float *torque, cudaStream_t st,
+                            const ZpPlanes *grad_radial_planes, const ZpScale &scale);
+int zp_torque_slots(const ZpTables &t);
 // node_out[n, l^2 + j, c] = sum over the m' rows r of degree l, in table order, of
 //   head[n][rot_off[r] + j][c] + the continuation partials of the 32-edge blocks n's edges reach
 int zp_launch_node_sum(const zp_plan *p, int64_t N, const float *head, const float *cont,
                        const int32_t *row_ptr, float *node_out, cudaStream_t st);
-int zp_launch_node_reduce(const zp_plan *p, int64_t N, const float *du_both,
-                          const int32_t *row_ptr, const int32_t *perm_src,
-                          const int32_t *row_ptr_src, float *grad_x, cudaStream_t st);
 
 int zp_launch_gate_fwd(const zp_plan *p, int64_t E, const float *h1, const ZpPlanes &ht,
                        const ZpScale &scale, float *gate_max, cudaStream_t st);

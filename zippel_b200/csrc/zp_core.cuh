@@ -101,11 +101,11 @@ inline int zp_radial_splits(int64_t N, int64_t K) {
 }
 
 //   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials
-//   backward: dy planes | dht | dh1 planes | da1 | du_src | torque | wgrad partials | scratch
+//   backward: dy planes | dht | dh1 planes | da1 | torque | wgrad partials | scratch
 // mode 0 / 1: forward that keeps what a backward reads (1: plus the backward's own regions);
 // mode 2: forward alone with fused epilogues -- of h1 only the gate scalars exist, y does not.
 struct ZpWorkspace {
-  float *rot, *h1, *y, *dht, *da1, *du_src, *torque, *wgrad, *scales, *head, *cont;
+  float *rot, *h1, *y, *dht, *da1, *torque, *wgrad, *scales, *head, *cont;
   float *rot_grad;                       // [E, nnz_pad], in dht's place where it fits: that is read by then
   float *col1, *col2, *col_rad;          // partial column sums: bias gradients of conv1, conv2, radial
   float *radial, *rad_partials;          // radial layer inside the call: its output, dW partials
@@ -179,6 +179,7 @@ struct ZpConv {
   const float *x_node, *edge_vec, *cos_g, *sin_g, *radial, *env;
   const int32_t *src, *dst, *row_ptr, *perm_src, *row_ptr_src;
   const zp_weights *w;
+  ZpNodeView view{0, nullptr, nullptr, nullptr};     // forward: all nodes, where the caller has the view by source
 };
 // The last dense layer of the radial MLP (blocks/eso2_ref.py:169-182, rad_func[6]), when the call
 // runs it itself: radial[E, R] = h[E, ec] w[R, ec]^T + b.

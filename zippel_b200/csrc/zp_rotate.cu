@@ -2,7 +2,6 @@
 //
 //   rotate_in            a[e, r, c2] = radial[e, .] * sum_j rot[e, r, j] * [x_src ; x_dst][l_r^2 + j, c2]
 //   rotate_back_scatter  node_out[n, l^2 + j, c] = sum_{e -> n} env_e * sum_r rot[e, r, j] * y[e, r, c]
-//   node_reduce          fixed-order sums of those contributions per destination / source node
 //
 // They take over blocks/eso2_ref.py:334-335 (gather + rotate in, with the radial gain of
 // :269-271, :284-285 applied while the row is in registers) and :343-349 (envelope, rotate
@@ -101,6 +100,97 @@ rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
   RotIn<LMAX, LMAX, FMT>::run(t, xrow, rot_s + le * t.rot_ld, rad_s, ls,
                               static_cast<uint16_t *>(a1.base) + e * a1.ld + c2, 2 * a1.plane_stride,
                               pack2(inv, inv));
+}
+
+// The same by node (zp_rotate.cuh), for callers with a source view.  Four channels a lane.  60 000 edges at lmax 4 /
+// C 128 in two planes 454 -> 354 us, 384 000 in one 2.22 -> 1.42 ms, 240 000 at lmax 6 4.7 -> 2.3 ms.
+template <int L, int LMAX, int FMT>
+struct RotInN {
+  static __device__ __forceinline__ void run(const ZpTables &t, const float *x_s, const float *rot, float *rad_s, int ls,
+                                             uint16_t *out, int64_t plane_bytes, u64 inv, bool live, const float *next,
+                                             bool more) {
+    if constexpr (L > 0) RotInN<L - 1, LMAX, FMT>::run(t, x_s, rot, rad_s, ls, out, plane_bytes, inv, live, next, more);
+    constexpr int n = 2 * L + 1;
+    const int C2 = 2 * t.C;
+    const int mm = t.mmax < L ? t.mmax : L;
+    if (L > 0) cp_async_wait<LMAX>();    // (degree 0: the caller)
+    if (live) {
+      F4 u[n];
+#pragma unroll
+      for (int j = 0; j < n; ++j) u[j] = load4(x_s + (L * L + j) * ls);
+      const float *w = rot + t.deg_rot[L];
+      const float *g = rad_s + t.deg_rad[L] * ls;
+      uint16_t *o = out + L * C2;
+      {
+        F4 acc = zero4();
+        for_row_plain<n>(w, [&](int j, u64 c) { axpy4(acc, c, u[j]); });
+        put4<FMT>(o, plane_bytes, mul4(acc, load4(g)), inv);
+      }
+#pragma unroll 1
+      for (int am = 1; am <= mm; ++am) {
+        const int km = LMAX + 1 - am;
+        w += 2 * (n + 1);
+        g += ls;
+        o += ((am == 1 ? 1 : 2) * (km + 1) - 1) * C2;
+        const F4 gain = load4(g);
+        F4 ap = zero4(), an = zero4();
+        for_row_plain<n>(w - (n + 1), [&](int j, u64 c) { axpy4(ap, c, u[j]); });
+        for_row_plain<n>(w, [&](int j, u64 c) { axpy4(an, c, u[j]); });
+        put4<FMT>(o, plane_bytes, mul4(ap, gain), inv);
+        put4<FMT>(o + km * C2, plane_bytes, mul4(an, gain), inv);
+      }
+    }
+    if (more) stage_degree<L, LMAX, F4, false, true>(t, nullptr, 0, next, nullptr, rad_s, ls);
+    cp_async_commit();                   // (with degree 0 goes the rotation, requested before)
+  }
+};
+
+// shared memory: x [K][G] vectors | per worker: radial gains [rad_rows][G] | per worker: two rotations [rot_ld]
+template <int LMAX, int FMT>
+__global__ void __launch_bounds__(32 * kNodeMaxWarps, 2)
+node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, int G, int quads,
+                      const float *__restrict__ x, const int32_t *__restrict__ row_ptr,
+                      const int32_t *__restrict__ perm_src, const int32_t *__restrict__ row_ptr_src,
+                      const float *__restrict__ rot, const float *__restrict__ radial, const ZpPlanes a1,
+                      const ZpScale scale) {
+  zp_after_previous();
+  constexpr int K = (LMAX + 1) * (LMAX + 1);
+  extern __shared__ __align__(16) float node_s[];
+  const int64_t n = blockIdx.x;
+  const int workers = blockDim.x / G, w = threadIdx.x / G, li = threadIdx.x % G, ls = 4 * G;
+  const int c0 = blockIdx.y * quads * 4, mine = min(quads, (t.C - c0) / 4);
+  const bool active = li < mine;
+  const int c = c0 + 4 * li;
+  float *x_s = node_s, *stage = node_s + (size_t)K * ls, *rad_s = stage + (size_t)w * t.rad_rows * ls + 4 * li;
+  float *rot_s = stage + (size_t)workers * t.rad_rows * ls + (size_t)w * 2 * t.rot_ld;
+  const float inv = zp_publish_scale(a1, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
+  const u64 inv2 = pack2(inv, inv);
+  const NodeEdges edges(n, N, E, row_ptr, perm_src, row_ptr_src, blockIdx.z, gridDim.z);
+  if (edges.first == edges.last) return;
+  auto column = [&](int i) { return (i < edges.into ? t.C : 0) + c; };
+  auto gains = [&](int e, int i) { return radial + (size_t)(e < 0 ? 0 : e) * t.R + column(i); };
+  auto rotation = [&](int64_t e, int buffer) {
+    stage_rot(rot + (size_t)e * t.rot_ld, rot_s + buffer * t.rot_ld, t.rot_ld, li, G);
+  };
+  const int i0 = edges.first + w;
+  int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
+  if (e >= 0) rotation(e, 0);
+  StageAll<LMAX, LMAX, F4, false, true>::run(t, nullptr, 0, gains(e, i0), nullptr, rad_s, ls, e >= 0 && active);
+  stage_node<F4>(x + (size_t)n * t.K * t.C + c0, t.C, K, mine, x_s, ls);
+  __syncthreads();
+  for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
+    const int e_after = edges.edge(i + 2 * workers);
+    cp_async_wait<LMAX>();               // degree 0 and the rotation have landed
+    __syncwarp();                        // ... the other lanes' part of it, and all are done with the last
+    if (e_next >= 0) rotation(e_next, buffer ^ 1);
+    RotInN<LMAX, LMAX, FMT>::run(t, x_s + 4 * li, rot_s + buffer * t.rot_ld, rad_s, ls,
+                                 static_cast<uint16_t *>(a1.base) + (e < 0 ? 0 : e) * a1.ld + column(i),
+                                 2 * a1.plane_stride, inv2, e >= 0 && active, gains(e_next, i + workers),
+                                 e_next >= 0 && active);
+    e = e_next;
+    e_next = e_after;
+  }
+  cp_async_wait<0>();
 }
 
 // ------------------------------------------------------------------------------------------
@@ -238,37 +328,6 @@ rotate_back_scatter_kernel(const __grid_constant__ ZpTables t, int64_t N,
   }
 }
 
-constexpr int kReduceBatch = 8;
-// grad_x[n] = sum over edges INTO n of du_both[e][1]  +  sum over edges OUT OF n of du_both[e][0],
-// both in fixed (sorted) order.  Bound by the contributions it reads, once each: a thread keeps
-// kReduceBatch of them on their way (one at a time in a loop over channels left 216 nodes at 1.3 TB/s).
-__global__ void __launch_bounds__(128)
-node_reduce_kernel(int64_t N, int KC4, const float4 *__restrict__ du_both,
-                   const int32_t *__restrict__ row_ptr, const int32_t *__restrict__ perm_src,
-                   const int32_t *__restrict__ row_ptr_src, float4 *__restrict__ grad_x) {
-  zp_after_previous();
-  const int64_t n = blockIdx.x;
-  const int i = blockIdx.y * blockDim.x + threadIdx.x;
-  if (n >= N || i >= KC4) return;
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto add = [&](int beg, int end, auto slot) {
-    for (int k = beg; k < end; k += kReduceBatch) {
-      float4 v[kReduceBatch];
-#pragma unroll
-      for (int u = 0; u < kReduceBatch; ++u)
-        if (k + u < end) v[u] = __ldcs(&du_both[(size_t)slot(k + u) * KC4 + i]);
-#pragma unroll
-      for (int u = 0; u < kReduceBatch; ++u)
-        if (k + u < end) {
-          acc.x += v[u].x; acc.y += v[u].y; acc.z += v[u].z; acc.w += v[u].w;
-        }
-    }
-  };
-  add(row_ptr[n], row_ptr[n + 1], [](int k) { return 2 * (int64_t)k + 1; });
-  add(row_ptr_src[n], row_ptr_src[n + 1], [&](int k) { return 2 * (int64_t)perm_src[k]; });
-  grad_x[(size_t)n * KC4 + i] = acc;
-}
-
 // Final sums after the rotate-back epilogue of conv2.  The epilogue leaves, per m' row r, the
 // partial sums of a node's edges: head[n] for the run that starts at the node's first edge and
 // cont[b] for the run that enters 32-edge block b from the block before.  One block per node adds,
@@ -318,12 +377,39 @@ int zp_launch_node_sum(const zp_plan *p, int64_t N, const float *head, const flo
 }
 
 int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32_t *src,
-                        const int32_t *dst, const float *rot, const float *radial,
+                        const int32_t *dst, const ZpNodeView &view, const float *rot, const float *radial,
                         const ZpPlanes &a1, const ZpScale &scale, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const ZpTables &t = p->t;
   const int Q = t.C / 2;
   if (Q < 1 || Q > kRotInThreads) return ZP_ERR_UNSUPPORTED;
+  // by node where at least seven lanes of ten have channels (72 of them leave 14 of 32 lanes idle: 17 900 edges
+  // 173 us, 74 by edge)
+  const NodeShape ns = zp_node_shape(t.C, 4);
+  if (view.perm_src && 10 * ns.quads >= 7 * ns.G) {
+    const int64_t N = view.nodes;
+    const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t, t.rad_rows, 16, 4);
+    const dim3 grid((unsigned)N, (unsigned)ns.groups, (unsigned)nl.parts);
+#define CALL_FMT(LM, FMT)                                                                         \
+  {                                                                                               \
+    static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
+    if (int rc_ = zp_ensure_smem(node_rotate_in_kernel<LM, FMT>, nl.smem, opt_in)) return rc_;    \
+    zp_launch(node_rotate_in_kernel<LM, FMT>, grid, 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, x, \
+              view.row_ptr, view.perm_src, view.row_ptr_src, rot, radial, a1, scale);             \
+    break;                                                                                        \
+  }
+#define CALL(LM)                                               \
+  switch (zp_plane_format(a1)) {                               \
+    case kFmtBf16: CALL_FMT(LM, kFmtBf16)                      \
+    case kFmtFp16x2: CALL_FMT(LM, kFmtFp16x2)                  \
+    default: CALL_FMT(LM, kFmtBf16x3)                          \
+  }
+    ZP_DISPATCH_LMAX(t.lmax, CALL)
+#undef CALL
+#undef CALL_FMT
+    ZP_LAUNCH_CHECK("node_rotate_in_kernel");
+    return ZP_OK;
+  }
   int epb = kRotInThreads / Q;
   if (epb > kRotInMaxEdges) epb = kRotInMaxEdges;
   const dim3 grid((unsigned)zp_ceil_div(E, epb)), block(epb * Q);
@@ -368,17 +454,5 @@ int zp_launch_rotate_back_scatter(const zp_plan *p, int64_t N, const float *y, c
   ZP_DISPATCH_LMAX(t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("rotate_back_scatter_kernel");
-  return ZP_OK;
-}
-
-int zp_launch_node_reduce(const zp_plan *p, int64_t N, const float *du_both,
-                          const int32_t *row_ptr, const int32_t *perm_src,
-                          const int32_t *row_ptr_src, float *grad_x, cudaStream_t st) {
-  if (N == 0) return ZP_OK;
-  const int KC4 = p->t.K * p->t.C / 4;
-  const dim3 grid((unsigned)N, (unsigned)zp_ceil_div(KC4, 128));
-  zp_launch(node_reduce_kernel, grid, 128, 0, st, N, KC4, (const float4 *)du_both, row_ptr, perm_src,
-            row_ptr_src, (float4 *)grad_x);
-  ZP_LAUNCH_CHECK("node_reduce_kernel");
   return ZP_OK;
 }

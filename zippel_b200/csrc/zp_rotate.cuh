@@ -52,6 +52,29 @@ __device__ __forceinline__ F4 mul4(const F4 &x, const F4 &y) { return F4{mul2(x.
 __device__ __forceinline__ u64 dot4(u64 acc, const F4 &x, const F4 &y) {
   return fma2(x.a, y.a, fma2(x.b, y.b, acc));
 }
+// Two channels, for the degrees whose rows would not fit the registers four at a time
+struct __align__(8) F2 {
+  u64 a;
+};
+template <typename V> struct VecOf;
+template <> struct VecOf<F4> { static constexpr int n = 4; };
+template <> struct VecOf<F2> { static constexpr int n = 2; };
+template <typename V>
+__device__ __forceinline__ V load_vec(const float *p) { return *reinterpret_cast<const V *>(p); }
+template <typename V>
+__device__ __forceinline__ void store_vec(float *p, const V &v) { *reinterpret_cast<V *>(p) = v; }
+template <typename V>
+__device__ __forceinline__ V zero_vec() { return V{}; }
+__device__ __forceinline__ void axpy4(F2 &acc, u64 w, const F2 &v) { acc.a = fma2(w, v.a, acc.a); }
+__device__ __forceinline__ F2 mul4(const F2 &x, const F2 &y) { return F2{mul2(x.a, y.a)}; }
+__device__ __forceinline__ u64 dot4(u64 acc, const F2 &x, const F2 &y) { return fma2(x.a, y.a, acc); }
+// x y + z w
+__device__ __forceinline__ F4 mul_add4(const F4 &x, const F4 &y, const F4 &z, const F4 &w) {
+  return F4{fma2(x.a, y.a, mul2(z.a, w.a)), fma2(x.b, y.b, mul2(z.b, w.b))};
+}
+__device__ __forceinline__ F2 mul_add4(const F2 &x, const F2 &y, const F2 &z, const F2 &w) {
+  return F2{fma2(x.a, y.a, mul2(z.a, w.a))};
+}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -92,6 +115,32 @@ __device__ __forceinline__ void put4(void *at, int64_t plane_bytes, const F4 &v,
       const float2 f0 = __bfloat1622float2(h0), f1 = __bfloat1622float2(h1);
       xa = sub2(xa, pack2(f0.x, f0.y));
       xb = sub2(xb, pack2(f1.x, f1.y));
+    }
+  }
+}
+
+// ... and one pair
+template <int FMT>
+__device__ __forceinline__ void put4(void *at, int64_t plane_bytes, const F2 &v, u64 inv) {
+  char *dst = static_cast<char *>(at);
+  if constexpr (FMT == kFmtFp32) {
+    *reinterpret_cast<F2 *>(dst) = v;
+  } else if constexpr (FMT == kFmtFp16x2) {
+    const u64 x = mul2(v.a, inv);
+    const float2 f = unpack2(x);
+    const __half2 h = __floats2half2_rn(f.x, f.y);
+    const float2 b = __half22float2(h), r = unpack2(sub2(x, pack2(b.x, b.y)));
+    *reinterpret_cast<__half2 *>(dst) = h;
+    *reinterpret_cast<__half2 *>(dst + plane_bytes) = __floats2half2_rn(r.x, r.y);
+  } else {
+    u64 x = v.a;
+#pragma unroll
+    for (int pl = 0; pl < (FMT == kFmtBf16 ? 1 : 3); ++pl) {
+      const float2 f = unpack2(x);
+      const __nv_bfloat162 h = __floats2bfloat162_rn(f.x, f.y);
+      *reinterpret_cast<__nv_bfloat162 *>(dst + pl * plane_bytes) = h;
+      const float2 b = __bfloat1622float2(h);
+      x = sub2(x, pack2(b.x, b.y));
     }
   }
 }
@@ -160,10 +209,158 @@ __device__ __forceinline__ void for_row(const float2 *row, F f) {
     if (j + 1 < N) f(j + 1, w.y);
   }
 }
+// ... of a row as it stands in global memory (row start 8-byte aligned)
+template <int N, typename F>
+__device__ __forceinline__ void for_row_plain(const float *row, F f) {
+#pragma unroll
+  for (int j = 0; j < N; j += 2) {
+    const float2 w = *reinterpret_cast<const float2 *>(row + j);
+    f(j, pack2(w.x, w.x));
+    if (j + 1 < N) f(j + 1, pack2(w.y, w.y));
+  }
+}
 // rotation entries of `edges` consecutive edges duplicated into shared memory
 __device__ __forceinline__ void stage_dup(const float *__restrict__ rot, float2 *rot_s, int ld, int edges) {
   for (int i = threadIdx.x; i < ld * edges; i += blockDim.x) {
     const float v = rot[i];
     rot_s[i] = make_float2(v, v);
+  }
+}
+
+// ---- kernels by node ---------------------------------------------------------------------------
+// A block owns one node, whose rows of x (or of the upstream gradient) stand in shared memory, and goes through
+// the node's edges: by edge, a thread fetches them from L2 again and again, and those fetches were between a
+// third and a half of all that L2 has to deliver, which is what bounds these kernels (60 000 edges at lmax 4 / C 128:
+// 57 KB an edge in 450 us going in, 95 KB in 920 coming back, 7.6 and 6.2 TB/s).  G lanes are a worker, which has
+// an edge to itself, each lane one vector of channels; the node's edges are dealt to the workers in turn.
+// A degree's rows of the worker's next edge are requested as soon as those of the current one have been used,
+// so that one edge is always on its way.  All copies into a worker's rows are its lanes' own, but the rotation's.
+struct NodeShape {
+  int vec, groups, quads, G;             // channels a lane; blocks per node; lanes with channels, lanes of a worker
+};
+inline NodeShape zp_node_shape(int channels, int vec) {
+  NodeShape s;
+  s.vec = vec;
+  const int lanes = channels / vec;
+  s.groups = (lanes + 31) / 32;
+  s.quads = (lanes + s.groups - 1) / s.groups;
+  s.G = s.quads <= 4 ? 4 : s.quads <= 8 ? 8 : s.quads <= 16 ? 16 : 32;
+  return s;
+}
+// How a kernel by node is launched: a block for each of `parts` stretches of a node's edges, of four or eight warps
+// (less only where they do not fit).  What decides is how often the SMs have to take a new set of blocks, times
+// how long a block takes: its edges, and the start (row offsets, first rotation, first rows, one after the other,
+// as long as some three edges).  From 2 000 nodes on four warps and eight, whole nodes and halves are within 5 % of each
+// other and two warps 5 to 20 % behind; 216 nodes of 90 edges took 739 us a training step with eight warps, 799 with
+// four and 952 with two.
+constexpr int kNodeMaxWarps = 8;
+struct NodeLaunch {
+  int warps, parts;
+  size_t smem;
+};
+// blocks: nodes times channel groups; items: edges of a node on average; rows: vectors a lane holds of an edge;
+// sm_warps: warps of the kernel that an SM's registers hold; max_parts: 1 where a node's edges belong together
+inline NodeLaunch zp_node_launch(int64_t blocks, double items, const NodeShape &s, const ZpTables &t, int rows,
+                                 int sm_warps, int max_parts) {
+  NodeLaunch best{1, 1, 0};
+  double best_cost = 1e300;
+  for (int warps = 1; warps <= kNodeMaxWarps; warps *= 2) {
+    const size_t workers = 32 * warps / s.G;
+    const size_t smem = sizeof(float) * ((size_t)s.G * s.vec * (t.K + workers * rows) + workers * 2 * t.rot_ld);
+    if (warps > 1 && smem > 220 * 1024) break;
+    if (warps == 4) best_cost = 1e300;   // one and two were for rows too many for four
+    const int64_t resident = 148 * std::max<int64_t>(1, std::min<int64_t>(sm_warps / warps, (int64_t)(225 * 1024 / (smem + 1024))));
+    for (int parts = 1; parts <= max_parts; parts *= 2) {
+      const double rounds = std::max(1.0, (double)(blocks * parts) / (double)resident + 0.5);
+      const double cost = rounds * (items / (double)(parts * workers) + 3.0);
+      if (cost < 0.98 * best_cost) {
+        best_cost = cost;
+        best = NodeLaunch{warps, parts, smem};
+      }
+    }
+  }
+  return best;
+}
+
+// The node's edges, numbered: those into it, then (with a source view) those out of it.  Slots that the sort has
+// left out (edges of indices out of range) stand behind all others and count as edges into node 0.
+struct NodeEdges {
+  int beg, own, into, sbeg, total, rest;
+  const int32_t *perm_src;
+  int first, last;                       // this block's stretch of them
+  __device__ __forceinline__ NodeEdges(int64_t n, int64_t N, int64_t E, const int32_t *row_ptr, const int32_t *view,
+                                       const int32_t *row_ptr_src, int part, int parts) {
+    beg = row_ptr[n];
+    own = into = row_ptr[n + 1] - beg;
+    rest = sbeg = 0;
+    if (n == 0) {
+      rest = row_ptr[N];
+      into += (int)E - rest;
+    }
+    total = into;
+    perm_src = view;
+    if (view) {
+      sbeg = row_ptr_src[n];
+      total += row_ptr_src[n + 1] - sbeg;
+    }
+    first = (int)((int64_t)total * part / parts);
+    last = (int)((int64_t)total * (part + 1) / parts);
+  }
+  // -1: past this block's
+  __device__ __forceinline__ int edge(int i) const {
+    if (i >= last) return -1;
+    return i < own ? beg + i : i < into ? rest + i - own : perm_src[sbeg + i - into];
+  }
+};
+
+// Puts one degree's rows of an edge on their way: ROWS |m| <= mmax (m'-major, `stride` floats apart), RAD its
+// radial gains (2C floats apart); in shared memory as StageEdge.
+template <int L, int LMAX, typename V, bool ROWS, bool RAD>
+__device__ __forceinline__ void stage_degree(const ZpTables &t, const float *rows, int stride, const float *rad,
+                                             float *row_s, float *rad_s, int ls) {
+  constexpr int B = 4 * VecOf<V>::n;
+  const int mm = t.mmax < L ? t.mmax : L, C2 = 2 * t.C;
+  float *rs = row_s + (ROWS ? t.deg_row[L] * ls : 0), *gs = rad_s + (RAD ? t.deg_rad[L] * ls : 0);
+  int r = L, k = L;                              // row m = 0, gain |m| = 0 of this degree
+  if (ROWS) cp_async<B>(rs, rows + r * stride);
+  if (RAD) cp_async<B>(gs, rad + k * C2);
+#pragma unroll 1
+  for (int am = 1; am <= mm; ++am) {
+    const int km = LMAX + 1 - am;                // rows of +am
+    r += (am == 1 ? 1 : 2) * (km + 1) - 1;
+    k += km;
+    if (ROWS) {
+      rs += 2 * ls;
+      cp_async<B>(rs - ls, rows + r * stride);
+      cp_async<B>(rs, rows + (r + km) * stride);
+    }
+    if (RAD) {
+      gs += ls;
+      cp_async<B>(gs, rad + k * C2);
+    }
+  }
+}
+// all degrees of a first edge, a commit group each; what the caller has requested goes with the first
+template <int L, int LMAX, typename V, bool ROWS, bool RAD>
+struct StageAll {
+  static __device__ __forceinline__ void run(const ZpTables &t, const float *rows, int stride, const float *rad,
+                                             float *row_s, float *rad_s, int ls, bool live) {
+    if constexpr (L > 0) StageAll<L - 1, LMAX, V, ROWS, RAD>::run(t, rows, stride, rad, row_s, rad_s, ls, live);
+    if (live) stage_degree<L, LMAX, V, ROWS, RAD>(t, rows, stride, rad, row_s, rad_s, ls);
+    cp_async_commit();
+  }
+};
+// A worker's lanes request an edge's rotation.  Its entries are made into pairs where they are used, 300
+// instructions of 2400 an edge; copied into pairs, four bytes at a time, they took longer (rotate_in 354 -> 390 us at
+// lmax 4, 2.3 -> 3.8 ms for 240 000 edges at lmax 6, where their room costs blocks too).
+__device__ __forceinline__ void stage_rot(const float *rot, float *rot_s, int ld, int li, int G) {
+  for (int i = 4 * li; i < ld; i += 4 * G) cp_async<16>(rot_s + i, rot + i);
+}
+// `mine` vectors of each of the node's K rows into shared memory, ls floats a row
+template <typename V>
+__device__ __forceinline__ void stage_node(const float *x, int C, int K, int mine, float *x_s, int ls) {
+  for (int i = threadIdx.x; i < K * mine; i += blockDim.x) {
+    const int k = i / mine, q = i - k * mine;
+    store_vec<V>(x_s + k * ls + q * VecOf<V>::n, load_vec<V>(x + (size_t)k * C + q * VecOf<V>::n));
   }
 }

@@ -31,19 +31,22 @@ constexpr int kEdgesPerBlock = 16;       // narrow rows: bounds the rotations he
 
 struct Torque {
   u64 t0, t1, t2;
-  __device__ __forceinline__ void own(int m, const F4 &pp, const F4 &pm, const F4 &bp, const F4 &bm) {
+  template <typename V>
+  __device__ __forceinline__ void own(int m, const V &pp, const V &pm, const V &bp, const V &bm) {
     const u64 f = pack2((float)m, (float)m);
     t0 = fma2(f, sub2(dot4(0ull, pp, bm), dot4(0ull, pm, bp)), t0);
   }
   // (m, m + 1): q, s = p and b of m; y, t = those of m + 1
-  __device__ __forceinline__ void pair(float c, const F4 &qp, const F4 &qm, const F4 &sp, const F4 &sm,
-                                       const F4 &yp, const F4 &ym, const F4 &tp, const F4 &tm) {
+  template <typename V>
+  __device__ __forceinline__ void pair(float c, const V &qp, const V &qm, const V &sp, const V &sm,
+                                       const V &yp, const V &ym, const V &tp, const V &tm) {
     const u64 cc = pack2(c, c);
     t1 = fma2(cc, sub2(dot4(dot4(0ull, qp, tp), qm, tm), dot4(dot4(0ull, yp, sp), ym, sm)), t1);
     t2 = fma2(cc, sub2(dot4(dot4(0ull, ym, sp), qm, tp), dot4(dot4(0ull, qp, tm), yp, sm)), t2);
   }
   // (mmax, mmax + 1): p of the outer row is zero
-  __device__ __forceinline__ void outer(float c, const F4 &qp, const F4 &qm, const F4 &tp, const F4 &tm) {
+  template <typename V>
+  __device__ __forceinline__ void outer(float c, const V &qp, const V &qm, const V &tp, const V &tm) {
     const u64 cc = pack2(c, c);
     t1 = fma2(cc, dot4(dot4(0ull, qp, tp), qm, tm), t1);
     t2 = fma2(cc, sub2(dot4(0ull, qm, tp), dot4(0ull, qp, tm)), t2);
@@ -167,151 +170,336 @@ rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
   });
 }
 
+// The same by node (zp_rotate.cuh): a block for the edges into one node, whose rows of g are read once.  60 000
+// edges at lmax 4 / mmax 2 / C 128: 32 KB an edge from L2 by edge, 19 here.
+template <int L, int LMAX, int FMT>
+struct GradOutN {
+  static __device__ __forceinline__ void run(const ZpTables &t, const float *g_s, float *y_s, int ls, uint16_t *out,
+                                             int64_t plane_bytes, u64 inv, const float *rot, u64 env, bool live,
+                                             const float *next, bool more, u64 &genv, Torque &T) {
+    if constexpr (L > 0)
+      GradOutN<L - 1, LMAX, FMT>::run(t, g_s, y_s, ls, out, plane_bytes, inv, rot, env, live, next, more, genv, T);
+    constexpr int n = 2 * L + 1;
+    const int mm = t.mmax < L ? t.mmax : L;
+    if (L > 0) cp_async_wait<LMAX>();    // (degree 0: the caller)
+    if (live) {
+      F4 g[n];
+#pragma unroll
+      for (int j = 0; j < n; ++j) g[j] = load4(g_s + (L * L + j) * ls);
+      const float *w = rot + t.deg_rot[L];
+      const float *yr = y_s + t.deg_row[L] * ls;
+      uint16_t *o = out + L * t.C;
+      F4 qp = load4(yr), qm = zero4(), sp = zero4(), sm = zero4();          // row m = 0
+      for_row_plain<n>(w, [&](int j, u64 c) { axpy4(sp, c, g[j]); });
+      genv = dot4(genv, qp, sp);
+      put4<FMT>(o, plane_bytes, F4{mul2(sp.a, env), mul2(sp.b, env)}, inv);
+#pragma unroll 1
+      for (int am = 1; am <= mm; ++am) {
+        const int km = LMAX + 1 - am;
+        w += 2 * (n + 1);
+        yr += 2 * ls;
+        o += ((am == 1 ? 1 : 2) * (km + 1) - 1) * t.C;
+        const F4 yp = load4(yr - ls), ym = load4(yr);
+        F4 tp = zero4(), tm = zero4();
+        for_row_plain<n>(w - (n + 1), [&](int j, u64 c) { axpy4(tp, c, g[j]); });
+        for_row_plain<n>(w, [&](int j, u64 c) { axpy4(tm, c, g[j]); });
+        genv = dot4(dot4(genv, yp, tp), ym, tm);
+        put4<FMT>(o, plane_bytes, F4{mul2(tp.a, env), mul2(tp.b, env)}, inv);
+        put4<FMT>(o + km * t.C, plane_bytes, F4{mul2(tm.a, env), mul2(tm.b, env)}, inv);
+        T.own(am, yp, ym, tp, tm);
+        T.pair(t.couple[L][am - 1], qp, qm, sp, sm, yp, ym, tp, tm);
+        qp = yp; qm = ym; sp = tp; sm = tm;
+      }
+      if (L > t.mmax) {
+        w += 2 * (n + 1);
+        F4 tp = zero4(), tm = zero4();
+        for_row_plain<n>(w - (n + 1), [&](int j, u64 c) { axpy4(tp, c, g[j]); });
+        for_row_plain<n>(w, [&](int j, u64 c) { axpy4(tm, c, g[j]); });
+        T.outer(t.couple[L][mm], qp, qm, tp, tm);
+      }
+    }
+    if (more) stage_degree<L, LMAX, F4, true, false>(t, next, t.C, nullptr, y_s, nullptr, ls);
+    cp_async_commit();                   // (with degree 0 goes the rotation, requested before)
+  }
+};
+
+// shared memory: g [K][G] vectors | per worker: rows of y [Km][G] | per worker: two rotations [rot_ld]
+template <int LMAX, int FMT>
+__global__ void __launch_bounds__(32 * kNodeMaxWarps, 2)
+node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, int G, int quads,
+                            const float *__restrict__ g_out, const float *__restrict__ y,
+                            const float *__restrict__ env, const float *__restrict__ rot,
+                            const int32_t *__restrict__ row_ptr, const ZpPlanes dy, const ZpScale scale,
+                            float *__restrict__ grad_env, float4 *__restrict__ torque) {
+  zp_after_previous();
+  constexpr int K = (LMAX + 1) * (LMAX + 1);
+  extern __shared__ __align__(16) float node_s[];
+  const int64_t n = blockIdx.x;
+  const int workers = blockDim.x / G, w = threadIdx.x / G, li = threadIdx.x % G, ls = 4 * G;
+  const bool active = li < quads;
+  const int c = 4 * li;
+  float *g_s = node_s, *stage = node_s + (size_t)K * ls, *y_s = stage + (size_t)w * t.Km * ls + c;
+  float *rot_s = stage + (size_t)workers * t.Km * ls + (size_t)w * 2 * t.rot_ld;
+  const float inv = zp_publish_scale(dy, scale, blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0);
+  const u64 inv2 = pack2(inv, inv);
+  const NodeEdges edges(n, N, E, row_ptr, nullptr, nullptr, blockIdx.z, gridDim.z);
+  if (edges.first == edges.last) return;
+  auto rows = [&](int e) { return y + (size_t)(e < 0 ? 0 : e) * t.Km * t.C + c; };
+  auto rotation = [&](int64_t e, int buffer) {
+    stage_rot(rot + (size_t)e * t.rot_ld, rot_s + buffer * t.rot_ld, t.rot_ld, li, G);
+  };
+  const int i0 = edges.first + w;
+  int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
+  if (e >= 0) rotation(e, 0);
+  StageAll<LMAX, LMAX, F4, true, false>::run(t, rows(e), t.C, nullptr, y_s, nullptr, ls, e >= 0 && active);
+  stage_node<F4>(g_out + (size_t)n * t.K * t.C, t.C, K, quads, g_s, ls);
+  __syncthreads();
+  for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
+    const int e_after = edges.edge(i + 2 * workers);
+    const float env_e = e >= 0 ? env[e] : 0.f;
+    Torque T{0ull, 0ull, 0ull};
+    u64 genv = 0ull;
+    cp_async_wait<LMAX>();               // degree 0 and the rotation have landed
+    __syncwarp();                        // ... the other lanes' part of it, and all are done with the last
+    if (e_next >= 0) rotation(e_next, buffer ^ 1);
+    GradOutN<LMAX, LMAX, FMT>::run(t, g_s + c, y_s, ls, static_cast<uint16_t *>(dy.base) + (e < 0 ? 0 : e) * dy.ld + c,
+                                   2 * dy.plane_stride, inv2, rot_s + buffer * t.rot_ld, pack2(env_e, env_e),
+                                   e >= 0 && active, rows(e_next), e_next >= 0 && active, genv, T);
+    float t0 = sum2(T.t0), t1 = sum2(T.t1), t2 = sum2(T.t2), ge = sum2(genv);
+    for (int o = G / 2; o > 0; o >>= 1) {
+      t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+      ge += __shfl_xor_sync(0xffffffffu, ge, o);
+    }
+    if (li == 0 && e >= 0) {
+      torque[e] = make_float4(t0 * env_e, t1 * env_e, t2 * env_e, 0.f);
+      grad_env[e] = ge;
+    }
+    e = e_next;
+    e_next = e_after;
+  }
+  cp_async_wait<0>();
+}
+
 // ---- VJP of rotate_in over the 2C message channels -----------------------------------------------
 //   a[r]   = sum_j rot[r, j] u[l^2 + j]            (formed again; u = x_src | x_dst half)
 //   ga[r]  = da[e, r] * radial
 //   grad_radial[e, col] = sum over the +m / -m rows sharing the column of  da[r] * a[r]
 //                         (fp32 rows, or operand planes of the radial layer's VJP)
-//   du[e, half, l^2 + j] = sum_r rot[r, j] ga[r]   (summed per node afterwards)
 //   torque[e] += sums above with p = ga, b = a
+//   grad_x[node, l^2 + j] = sum over the node's edges and their rows  rot[r, j] ga[r]
 template <int FMT> struct Elem { using type = uint16_t; };
 template <> struct Elem<kFmtFp32> { using type = float; };
 
-template <int L, int LMAX, int FMT>
-struct RotInBwdE {
+// By node (zp_rotate.cuh).  What an edge adds to the node's gradient stays in registers: written per
+// edge and summed afterwards it was half of all bytes (2 x 25.6 KB of 95 KB an edge at lmax 4, C 128).  Four
+// channels a lane, two from lmax 5 on: 36 rows of four do not fit the registers.
+// SUMS: the gradient of x_node is wanted (not in a force evaluation; the others are the same to the last bit).
+// what a lane needs of an edge
+template <typename T_>
+struct EdgeAt {
+  const float *da, *rad;                 // its channels in row 0 of da1, in column 0 of radial
+  T_ *out;                               // ... of grad_radial
+};
+template <int L, int LMAX, int FMT, typename V, bool SUMS>
+struct NodeRot {
   using T_ = typename Elem<FMT>::type;
-  // da_s, rad_s: this thread's channels of the edge's gradient rows and radial gains; out: its quad
-  // in column 0 of grad_radial
-  static __device__ __forceinline__ void run(const ZpTables &t, const float *xrow, const float *da_s,
-                                             const float *rad_s, int ls, T_ *out, int64_t plane_bytes,
-                                             u64 inv, const float2 *rot_s, float *du_row, Torque &T) {
-    RotInBwdE<L - 1, LMAX, FMT>::run(t, xrow, da_s, rad_s, ls, out, plane_bytes, inv, rot_s, du_row, T);
+  // rot: the current edge's rotation; next: the worker's next edge, staged as this one is used up
+  static __device__ __forceinline__ void run(const ZpTables &t, const float *x_s, float *da_s, float *rad_s, int ls,
+                                             T_ *out, int64_t plane_bytes, u64 inv, const float *rot, bool live,
+                                             const EdgeAt<T_> &next, bool more,
+                                             V (&acc)[SUMS ? (LMAX + 1) * (LMAX + 1) : 1], Torque &T) {
+    if constexpr (L > 0)
+      NodeRot<L - 1, LMAX, FMT, V, SUMS>::run(t, x_s, da_s, rad_s, ls, out, plane_bytes, inv, rot, live, next, more, acc, T);
     constexpr int n = 2 * L + 1;
     const int C2 = 2 * t.C;
     const int mm = t.mmax < L ? t.mmax : L;
-    F4 u[n], du[n];
-    const float *xl = xrow + L * L * t.C;
+    if (L > 0) cp_async_wait<LMAX>();    // (degree 0: the caller)
+    if (live) {
+      V u[n];
 #pragma unroll
-    for (int j = 0; j < n; ++j) u[j] = load4(xl + j * t.C);
-    const float2 *w = rot_s + t.deg_rot[L];
-    const float *dr = da_s + t.deg_row[L] * ls, *gr = rad_s + t.deg_rad[L] * ls;
-    T_ *o = out + L * C2;
-    cp_async_wait<LMAX - L>();             // what degrees 0..L need has landed
-    F4 qp, qm = zero4(), sp = zero4(), sm = zero4();
-    {
-      const F4 da = load4(dr);
-      qp = mul4(da, load4(gr));
-      for_row<n>(w, [&](int j, u64 c) {
-        axpy4(sp, c, u[j]);
-        du[j] = F4{mul2(c, qp.a), mul2(c, qp.b)};
-      });
-      put4<FMT>(o, plane_bytes, mul4(da, sp), inv);
-    }
-    // a real loop over |m| (one copy of the body per degree keeps the code in the instruction cache)
+      for (int j = 0; j < n; ++j) u[j] = load_vec<V>(x_s + (L * L + j) * ls);
+      const float *w = rot + t.deg_rot[L];
+      const float *dr = da_s + t.deg_row[L] * ls, *gr = rad_s + t.deg_rad[L] * ls;
+      T_ *o = out + L * C2;
+      V qp, qm = zero_vec<V>(), sp = zero_vec<V>(), sm = zero_vec<V>();
+      {
+        const V da = load_vec<V>(dr);
+        qp = mul4(da, load_vec<V>(gr));
+        for_row_plain<n>(w, [&](int j, u64 c) {
+          axpy4(sp, c, u[j]);
+          if constexpr (SUMS) axpy4(acc[L * L + j], c, qp);
+        });
+        put4<FMT>(o, plane_bytes, mul4(da, sp), inv);
+      }
 #pragma unroll 1
-    for (int am = 1; am <= mm; ++am) {
-      w += 2 * (n + 1);
-      dr += 2 * ls;
-      gr += ls;
-      o += (LMAX + 1 - am) * C2;
-      const F4 rad = load4(gr), dp = load4(dr - ls), dm = load4(dr);
-      const F4 yp = mul4(dp, rad), ym = mul4(dm, rad);
-      F4 ap = zero4(), an = zero4();
-      for_row<n>(w - (n + 1), [&](int j, u64 c) {
-        axpy4(ap, c, u[j]);
-        axpy4(du[j], c, yp);
-      });
-      for_row<n>(w, [&](int j, u64 c) {
-        axpy4(an, c, u[j]);
-        axpy4(du[j], c, ym);
-      });
-      put4<FMT>(o, plane_bytes, F4{fma2(dp.a, ap.a, mul2(dm.a, an.a)), fma2(dp.b, ap.b, mul2(dm.b, an.b))}, inv);
-      T.own(am, yp, ym, ap, an);
-      T.pair(t.couple[L][am - 1], qp, qm, sp, sm, yp, ym, ap, an);
-      qp = yp; qm = ym; sp = ap; sm = an;
+      for (int am = 1; am <= mm; ++am) {
+        w += 2 * (n + 1);
+        dr += 2 * ls;
+        gr += ls;
+        o += (LMAX + 1 - am) * C2;
+        const V rad = load_vec<V>(gr), dp = load_vec<V>(dr - ls), dm = load_vec<V>(dr);
+        const V yp = mul4(dp, rad), ym = mul4(dm, rad);
+        V ap = zero_vec<V>(), an = zero_vec<V>();
+        for_row_plain<n>(w - (n + 1), [&](int j, u64 c) {
+          axpy4(ap, c, u[j]);
+          if constexpr (SUMS) axpy4(acc[L * L + j], c, yp);
+        });
+        for_row_plain<n>(w, [&](int j, u64 c) {
+          axpy4(an, c, u[j]);
+          if constexpr (SUMS) axpy4(acc[L * L + j], c, ym);
+        });
+        put4<FMT>(o, plane_bytes, mul_add4(dp, ap, dm, an), inv);
+        T.own(am, yp, ym, ap, an);
+        T.pair(t.couple[L][am - 1], qp, qm, sp, sm, yp, ym, ap, an);
+        qp = yp; qm = ym; sp = ap; sm = an;
+      }
+      if (L > t.mmax) {
+        w += 2 * (n + 1);
+        V ap = zero_vec<V>(), an = zero_vec<V>();
+        for_row_plain<n>(w - (n + 1), [&](int j, u64 c) { axpy4(ap, c, u[j]); });
+        for_row_plain<n>(w, [&](int j, u64 c) { axpy4(an, c, u[j]); });
+        T.outer(t.couple[L][mm], qp, qm, ap, an);
+      }
     }
-    if (du_row) {                        // no du_both: the caller wants no gradient of x_node
-      float *dl = du_row + L * L * t.C;
-#pragma unroll
-      for (int j = 0; j < n; ++j) store4(dl + j * t.C, du[j]);
-    }
-    if (L > t.mmax) {
-      w += 2 * (n + 1);
-      F4 ap = zero4(), an = zero4();
-      for_row<n>(w - (n + 1), [&](int j, u64 c) { axpy4(ap, c, u[j]); });
-      for_row<n>(w, [&](int j, u64 c) { axpy4(an, c, u[j]); });
-      T.outer(t.couple[L][mm], qp, qm, ap, an);
-    }
+    if (more) stage_degree<L, LMAX, V, true, true>(t, next.da, C2, next.rad, da_s, rad_s, ls);
+    cp_async_commit();                   // (with degree 0 goes the rotation, requested before)
   }
-};
-template <int LMAX, int FMT>
-struct RotInBwdE<-1, LMAX, FMT> {
-  static __device__ __forceinline__ void run(const ZpTables &, const float *, const float *,
-                                             const float *, int, typename Elem<FMT>::type *, int64_t,
-                                             u64, const float2 *, float *, Torque &) {}
 };
 
-// du_both [E][2][K][C]: half 0 = contribution to the source node, half 1 = to the destination.
-// shared memory: partial sums [blockDim] float4 | da [Km][blockDim] float4 | radial
-// [rad_rows][blockDim] float4 | rot [epb][rot_ld] dup.
-template <int LMAX, int FMT>
-__global__ void __launch_bounds__(kEdgeThreads, (LMAX <= 2 ? 4 : LMAX <= 4 ? 3 : 2))
-rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
-                     const float *__restrict__ da1, const float *__restrict__ radial,
-                     const float *__restrict__ x, const int32_t *__restrict__ src,
-                     const int32_t *__restrict__ dst, const float *__restrict__ rot,
-                     float *__restrict__ grad_radial, const ZpPlanes grad_radial_planes,
-                     const ZpScale scale, float *__restrict__ du_both, float4 *__restrict__ torque) {
+struct NodeArgs {
+  const float *da1, *radial, *x, *rot;
+  const int32_t *row_ptr, *perm_src, *row_ptr_src;
+  float *grad_radial, *grad_x;
+  float4 *torque;                        // [slots][E]; slot 1 + 2 group + half is written here
+};
+constexpr int kNodeQuadMaxL = 4;         // four channels a lane up to here
+template <bool PAIR> struct NodeVecOf { using type = F4; };
+template <> struct NodeVecOf<true> { using type = F2; };
+template <int LMAX> using NodeVec = typename NodeVecOf<(LMAX > kNodeQuadMaxL)>::type;
+inline NodeShape node_shape(const ZpTables &t) { return zp_node_shape(t.C, t.lmax <= kNodeQuadMaxL ? 4 : 2); }
+// shared memory: x [K][G] vectors | per worker: staged rows [Km + rad_rows][G] vectors, later its sums [K][G] |
+// per worker: two rotations [rot_ld]
+template <int LMAX, int FMT, bool SUMS>
+__global__ void __launch_bounds__(32 * kNodeMaxWarps, (SUMS && LMAX > 2 ? 1 : 2))
+node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, int G, int quads, const NodeArgs a,
+                          const ZpPlanes grad_radial_planes, const ZpScale scale) {
   zp_after_previous();
-  extern __shared__ __align__(16) float4 edge_s[];
-  const int ls = 4 * blockDim.x;
-  float *da_s = reinterpret_cast<float *>(edge_s + blockDim.x) + 4 * threadIdx.x;
+  using T_ = typename Elem<FMT>::type;
+  using V = NodeVec<LMAX>;
+  constexpr int K = (LMAX + 1) * (LMAX + 1), VN = VecOf<V>::n;
+  extern __shared__ __align__(16) float node_s[];
+  const int64_t n = blockIdx.x;
+  const int workers = blockDim.x / G, w = threadIdx.x / G, li = threadIdx.x % G;
+  const int ls = G * VN;                                    // floats between two rows
+  const int rows = SUMS ? max(t.Km + t.rad_rows, K) : t.Km + t.rad_rows;
+  const int c0 = blockIdx.y * quads * VN, mine = min(quads, (t.C - c0) / VN);
+  const bool active = li < mine;
+  const int c = c0 + li * VN;
+  float *x_s = node_s, *stage = node_s + (size_t)K * ls, *da_s = stage + (size_t)w * rows * ls + li * VN;
   float *rad_s = da_s + t.Km * ls;
-  float2 *rot_s = reinterpret_cast<float2 *>(edge_s + (size_t)blockDim.x * (1 + t.Km + t.rad_rows));
-  const int Q = t.C / 2;
-  const int64_t e0 = (int64_t)blockIdx.x * epb;
-  const int n_e = (int)min((int64_t)epb, E - e0);
-  const int le = threadIdx.x / Q, c2 = 4 * (threadIdx.x - le * Q);
-  const int64_t e = e0 + le;
-  if (le < n_e)
-    StageEdge<LMAX, LMAX, true, true>::run(t, da1 + (size_t)e * t.Km * 2 * t.C + c2, 2 * t.C, da_s,
-                                           radial + (size_t)e * t.R + c2, rad_s, ls);
-  stage_dup(rot + e0 * t.rot_ld, rot_s, t.rot_ld, n_e);
+  float *rot_s = stage + (size_t)workers * rows * ls + (size_t)w * 2 * t.rot_ld;
+  const float *xn = a.x + (size_t)n * t.K * t.C + c0;
+  const NodeEdges edges(n, N, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
   float inv = 1.f;
   if constexpr (FMT == kFmtFp16x2)
-    inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && threadIdx.x == 0);
+    inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
+  const u64 inv2 = pack2(inv, inv);
+  const int64_t plane_bytes = 2 * grad_radial_planes.plane_stride;
+  V acc[SUMS ? K : 1];
+#pragma unroll
+  for (int k = 0; k < (SUMS ? K : 1); ++k) acc[k] = zero_vec<V>();
+  if (!SUMS && edges.first == edges.last) return;
+
+  auto at = [&](int64_t e, int i) {
+    const int col = (i < edges.into ? t.C : 0) + c;
+    EdgeAt<T_> p;
+    p.da = a.da1 + (size_t)e * t.Km * 2 * t.C + col;
+    p.rad = a.radial + (size_t)e * t.R + col;
+    if constexpr (FMT == kFmtFp32) p.out = a.grad_radial + (size_t)e * t.R + col;
+    else p.out = static_cast<uint16_t *>(grad_radial_planes.base) + e * grad_radial_planes.ld + col;
+    return p;
+  };
+  auto rotation = [&](int64_t e, int buffer) {
+    stage_rot(a.rot + (size_t)e * t.rot_ld, rot_s + buffer * t.rot_ld, t.rot_ld, li, G);
+  };
+  const int i0 = edges.first + w;
+  int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
+  EdgeAt<T_> cur = at(e < 0 ? 0 : e, i0);
+  if (e >= 0) rotation(e, 0);
+  StageAll<LMAX, LMAX, V, true, true>::run(t, cur.da, 2 * t.C, cur.rad, da_s, rad_s, ls, e >= 0 && active);
+  if (edges.total > 0) stage_node<V>(xn, t.C, K, mine, x_s, ls);
   __syncthreads();
-  float4 sums = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (le < n_e) {
-    const int half = c2 >= t.C ? 1 : 0;
-    const int c = c2 - half * t.C;
-    const int64_t node = half ? dst[e] : src[e];
-    typename Elem<FMT>::type *out;
-    if constexpr (FMT == kFmtFp32) out = grad_radial + (size_t)e * t.R + c2;
-    else out = static_cast<uint16_t *>(grad_radial_planes.base) + e * grad_radial_planes.ld + c2;
+  for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
+    const int e_after = edges.edge(i + 2 * workers);
+    const EdgeAt<T_> next = at(e_next < 0 ? 0 : e_next, i + workers);
     Torque T{0ull, 0ull, 0ull};
-    RotInBwdE<LMAX, LMAX, FMT>::run(t, x + (size_t)node * t.K * t.C + c, da_s, rad_s, ls, out,
-                                    2 * grad_radial_planes.plane_stride, pack2(inv, inv),
-                                    rot_s + le * t.rot_ld,
-                                    du_both ? du_both + ((size_t)e * 2 + half) * t.K * t.C + c : nullptr, T);
-    sums = make_float4(sum2(T.t0), sum2(T.t1), sum2(T.t2), 0.f);
+    cp_async_wait<LMAX>();               // degree 0 and the rotation have landed
+    __syncwarp();                        // ... the other lanes' part of it, and all are done with the last
+    if (e_next >= 0) rotation(e_next, buffer ^ 1);
+    NodeRot<LMAX, LMAX, FMT, V, SUMS>::run(t, x_s + li * VN, da_s, rad_s, ls, cur.out, plane_bytes, inv2,
+                                     rot_s + buffer * t.rot_ld, e >= 0 && active, next, e_next >= 0 && active,
+                                     acc, T);
+    float t0 = sum2(T.t0), t1 = sum2(T.t1), t2 = sum2(T.t2);
+    for (int o = G / 2; o > 0; o >>= 1) {
+      t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+    }
+    if (li == 0 && e >= 0)
+      a.torque[(size_t)(1 + 2 * blockIdx.y + (i < edges.into ? 1 : 0)) * E + e] = make_float4(t0, t1, t2, 0.f);
+    e = e_next;
+    e_next = e_after;
+    cur = next;
   }
   cp_async_wait<0>();
-  reduce_edges(edge_s, sums, Q, n_e, [&](int s, const float4 &v) {
-    float4 o = torque[e0 + s];
-    o.x += v.x; o.y += v.y; o.z += v.z;
-    torque[e0 + s] = o;
-  });
+  if constexpr (!SUMS) return;
+  __syncthreads();                       // all are done with their rows: the sums take their place
+  float *sums = stage + (size_t)w * rows * ls + li * VN;
+#pragma unroll
+  for (int k = 0; k < K; ++k) store_vec<V>(sums + k * ls, acc[SUMS ? k : 0]);
+  __syncthreads();
+  float *gx = a.grad_x + (size_t)n * t.K * t.C + c0;
+  for (int i = threadIdx.x; i < K * mine * VN; i += blockDim.x) {
+    const int k = i / (mine * VN), q = i - k * mine * VN;
+    float s = 0.f;
+    for (int v = 0; v < workers; ++v) s += stage[((size_t)v * rows + k) * ls + q];
+    gx[(size_t)k * t.C + q] = s;
+  }
 }
 
 }  // namespace
 
-int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const float *y,
-                              const float *env, const float *rot, const int32_t *dst,
+int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const float *g, const float *y,
+                              const float *env, const float *rot, const int32_t *dst, const int32_t *row_ptr,
                               const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
                               float *torque, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const ZpTables &t = p->t;
+  const NodeShape ns = zp_node_shape(t.C, 4);
+  if (ns.groups == 1) {                  // the sums over an edge's channels are one worker's
+    const NodeLaunch nl = zp_node_launch(N, (double)E / (double)N, ns, t, t.Km, 16, 4);
+#define CALL_FMT(LM, FMT)                                                                         \
+  {                                                                                               \
+    static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
+    if (int rc_ = zp_ensure_smem(node_rotate_grad_out_kernel<LM, FMT>, nl.smem, opt_in)) return rc_; \
+    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3((unsigned)N, 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, \
+              g, y, env, rot, row_ptr, dy, scale, grad_env, reinterpret_cast<float4 *>(torque));  \
+    break;                                                                                        \
+  }
+#define CALL(LM)                                               \
+  switch (zp_plane_format(dy)) {                               \
+    case kFmtBf16: CALL_FMT(LM, kFmtBf16)                      \
+    case kFmtFp16x2: CALL_FMT(LM, kFmtFp16x2)                  \
+    default: CALL_FMT(LM, kFmtBf16x3)                          \
+  }
+    ZP_DISPATCH_LMAX(t.lmax, CALL)
+#undef CALL
+#undef CALL_FMT
+    ZP_LAUNCH_CHECK("node_rotate_grad_out_kernel");
+    return ZP_OK;
+  }
   const int Q = t.C / 4;
   if (Q < 1 || Q > kEdgeThreads) return ZP_ERR_UNSUPPORTED;
   const int epb = std::min(kEdgeThreads / Q, kEdgesPerBlock), threads = (epb * Q + 31) / 32 * 32;
@@ -338,28 +526,39 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t E, const float *g, const
   return ZP_OK;
 }
 
-int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const float *radial,
-                            const float *x, const int32_t *src, const int32_t *dst,
-                            const float *rot, float *grad_radial, float *du_both, float *torque,
-                            cudaStream_t st, const ZpPlanes *grad_radial_planes,
-                            const ZpScale &scale) {
+int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float *da1, const float *radial,
+                            const float *x, const int32_t *row_ptr, const int32_t *perm_src,
+                            const int32_t *row_ptr_src, const float *rot, float *grad_radial, float *grad_x,
+                            float *torque, cudaStream_t st,
+                            const ZpPlanes *grad_radial_planes, const ZpScale &scale) {
   const ZpPlanes gp = grad_radial_planes ? *grad_radial_planes : ZpPlanes{nullptr, 0, 0, 0, 0, nullptr};
-  if (E == 0) return ZP_OK;
   const ZpTables &t = p->t;
-  const int Q = t.C / 2;
-  if (Q < 1 || Q > kEdgeThreads) return ZP_ERR_UNSUPPORTED;
-  const int epb = std::min(kEdgeThreads / Q, kEdgesPerBlock), threads = (epb * Q + 31) / 32 * 32;
-  const unsigned grid = (unsigned)zp_ceil_div(E, epb);
-  const size_t smem = (size_t)threads * (1 + t.Km + t.rad_rows) * sizeof(float4) +
-                      (size_t)epb * t.rot_ld * sizeof(float2);
-#define CALL_FMT(LM, FMT)                                                                         \
+  if (grad_x ? N == 0 : E == 0) return ZP_OK;
+  if (t.C > 256) {
+    if (E) return ZP_ERR_UNSUPPORTED;
+    ZP_CUDA(cudaMemsetAsync(grad_x, 0, sizeof(float) * (size_t)N * t.K * t.C, st));
+    return ZP_OK;
+  }
+  const bool sums = grad_x != nullptr;
+  const NodeShape ns = node_shape(t);
+  const int rows = t.Km + t.rad_rows;
+  const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t,
+                                       sums ? std::max(rows, t.K) : rows, sums && t.lmax > 2 ? 8 : 16, sums ? 1 : 4);
+  const NodeArgs a{da1, radial, x, rot, row_ptr, perm_src, row_ptr_src, grad_radial, grad_x,
+                   reinterpret_cast<float4 *>(torque)};
+  const dim3 grid((unsigned)N, (unsigned)ns.groups, (unsigned)nl.parts);
+#define CALL_S(LM, FMT, S)                                                                        \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
-    if (int rc_ = zp_ensure_smem(rotate_in_bwd_kernel<LM, FMT>, smem, opt_in)) return rc_;        \
-    zp_launch(rotate_in_bwd_kernel<LM, FMT>, grid, threads, smem, st,                             \
-        t, E, epb, da1, radial, x, src, dst, rot, grad_radial, gp, scale, du_both,                \
-        reinterpret_cast<float4 *>(torque));                                                      \
-    break;                                                                                        \
+    if (int rc_ = zp_ensure_smem(node_rotate_in_bwd_kernel<LM, FMT, S>, nl.smem, opt_in)) return rc_; \
+    zp_launch(node_rotate_in_bwd_kernel<LM, FMT, S>, grid, 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, a, \
+              gp, scale);                                                                         \
+  }
+#define CALL_FMT(LM, FMT)                        \
+  {                                              \
+    if (sums) CALL_S(LM, FMT, true)              \
+    else CALL_S(LM, FMT, false)                  \
+    break;                                       \
   }
 #define CALL(LM)                                               \
   switch (zp_plane_format(gp)) {                               \
@@ -371,6 +570,9 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t E, const float *da1, const
   ZP_DISPATCH_LMAX(t.lmax, CALL)
 #undef CALL
 #undef CALL_FMT
-  ZP_LAUNCH_CHECK("rotate_in_bwd_kernel");
+#undef CALL_S
+  ZP_LAUNCH_CHECK("node_rotate_in_bwd_kernel");
   return ZP_OK;
 }
+
+int zp_torque_slots(const ZpTables &t) { return 1 + 2 * node_shape(t).groups; }

@@ -467,7 +467,7 @@ template <int LMAX>
 __global__ void __launch_bounds__(128)
 edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restrict__ J, int64_t E,
                      const float *__restrict__ ev, const float *__restrict__ cgam,
-                     const float *__restrict__ sgam, const float4 *__restrict__ torque,
+                     const float *__restrict__ sgam, const float4 *__restrict__ torque, int slots,
                      const ZpTorqueArgs a, float *__restrict__ gev) {
   zp_after_previous();
   __shared__ int steps[128], found[4];
@@ -485,7 +485,11 @@ edge_vec_grad_kernel(const __grid_constant__ ZpTables t, const double *__restric
     if (!step) {
       double gx = 0.0, gy = 0.0, gz = 0.0;
       if constexpr (LMAX >= 1) {
-        const float4 T = torque[e];
+        float4 T = torque[e];
+        for (int s = 1; s < slots; ++s) {
+          const float4 more = torque[s * E + e];
+          T.x += more.x; T.y += more.y; T.z += more.z;
+        }
         const double inv_r = rsqrt(s2), r = s2 * inv_r, ca = zh * inv_r, sa = xh * inv_r;
         const double c1 = cgam[e * (LMAX + 1) + 1], s1 = sgam[e * (LMAX + 1) + 1];
         const double gb = c1 * T.y + s1 * T.z, ga = s1 * T.y - c1 * T.z + yh * inv_r * T.x;
@@ -566,13 +570,13 @@ int zp_launch_wigner_bwd(const zp_plan *p, int64_t E, const float *ev, const flo
 }
 
 int zp_launch_edge_vec_grad(const zp_plan *p, int64_t E, const float *ev, const float *cg,
-                            const float *sg, const float *torque, const ZpTorqueArgs &a, float *gev,
+                            const float *sg, const float *torque, int slots, const ZpTorqueArgs &a, float *gev,
                             cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const dim3 grid((unsigned)zp_ceil_div(E, 128)), block(128);
 #define CALL(LM)                                                                                  \
   zp_launch(edge_vec_grad_kernel<LM>, grid, block, 0, st, p->t, p->jd_dev, E, ev, cg, sg,             \
-                                                      reinterpret_cast<const float4 *>(torque), a, gev)
+                                                      reinterpret_cast<const float4 *>(torque), slots, a, gev)
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
   ZP_LAUNCH_CHECK("edge_vec_grad_kernel");
