@@ -14,7 +14,7 @@
 
 #include <algorithm>
 
-#include "zp_common.cuh"
+#include "zp_rotate.cuh"
 
 namespace {
 
@@ -87,62 +87,87 @@ __global__ void absmax_row_range_kernel(const float *__restrict__ in, int64_t co
 // ------------------------------------------------------------------------------------------
 __device__ __forceinline__ float sigmoidf(float x) { return 1.f / (1.f + __expf(-x)); }
 
-// One thread per (edge, pair of rows, hidden-channel quad): both rows' loads are issued before
-// either is used, which doubles the bytes a thread keeps in flight.  With `gate_max` set it also records the largest
-// sigmoid'(gate) it sees: max|dht| * rows(l) * max|h1| * that value bounds the gate part of the
-// backward's dh1, which fixes the scale of its fp16 planes before they are written (the bound
-// follows the gates into saturation, where a constant 1/4 would be orders of magnitude loose).
-constexpr int kGateEdges = 8;
-constexpr int kGateSub = 4;            // groups of kGateEdges edges per block of gate_fwd
-__global__ void gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
-                                const float *__restrict__ h1, const ZpPlanes ht,
-                                const ZpScale scale, float *gate_max) {
-  zp_after_previous();
-  // blockIdx.x counts groups of kGateEdges edges; the items of a group are indexed with 32-bit
-  // arithmetic (a 64-bit division per thread would cost more than the rest of the kernel)
-  const int H4 = t.H / 4;
-  const int per_edge = ((t.Km + 1) / 2) * H4;
-  const int item = blockIdx.y * blockDim.x + threadIdx.x;            // within the group
-  const int le = item / per_edge, rem = item - le * per_edge;
-  const int rp = rem / H4;
-  const int h = (rem - rp * H4) * 4;
-  float seen = 0.f;
-  bool probe = false;
-  const float inv = zp_publish_scale(
-      ht, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
-  // a block walks kGateSub groups of kGateEdges edges: fewer, longer-lived blocks
-#pragma unroll 2
-  for (int sub = 0; sub < kGateSub; ++sub) {
-    const int64_t e0 = ((int64_t)blockIdx.x * kGateSub + sub) * kGateEdges + le;
-    const bool in_range = le < kGateEdges && e0 < E;
-    const int64_t e = in_range ? e0 : 0;            // out-of-range threads recompute edge 0
-    const float *row = h1 + (size_t)e * t.w1_cols;
-    float4 x[2], g[2];
-    int rk[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int r = 2 * rp + k;
-      rk[k] = r < t.Km ? r : -1;
-      const int rr = r < t.Km ? r : 0;               // a missing second row re-reads row 0
-      x[k] = *reinterpret_cast<const float4 *>(row + t.n_gate + rr * t.H + h);
-      g[k] = rr == 0 ? x[k] : *reinterpret_cast<const float4 *>(row + (t.row_l[rr] - 1) * t.H + h);
+// Both directions: one thread per (edge, hidden-channel quad) goes through the degrees.  A degree's gate is read
+// and its sigmoid formed once for its 2 mmax + 1 rows, and the rows of up to |m| = 2 are requested before any is
+// used.  Bound by HBM (forward 21.5 KB, backward 31 KB an edge at lmax 4 / mmax 2 / H 128 in two planes).
+//
+// With `gate_max` set the forward also records the largest sigmoid'(gate) it sees: max|dht| * rows(l) * max|h1| *
+// that value bounds the gate part of the backward's dh1, which fixes the scale of its fp16 planes before they
+// are written (the bound follows the gates into saturation, where a constant 1/4 would be orders of magnitude
+// loose).
+constexpr int kGateThreads = 128;
+struct GateItem {
+  int64_t e;
+  int h;
+  bool live;
+  // 32-bit arithmetic within a block: a 64-bit division per thread would cost more than the rest
+  __device__ __forceinline__ GateItem(int64_t E, int H4, int per_block) {
+    const int le = threadIdx.x / H4;
+    e = (int64_t)blockIdx.x * per_block + le;
+    h = ((int)threadIdx.x - le * H4 + (int)blockIdx.y * (int)blockDim.x) * 4;
+    live = le < per_block && e < E && h < 4 * H4;
+    if (gridDim.y > 1) {                 // rows wider than a block: a block per part of one edge
+      e = blockIdx.x;
+      h = ((int)blockIdx.y * (int)blockDim.x + (int)threadIdx.x) * 4;
+      live = h < 4 * H4;
     }
+    if (!live) { e = 0; h = 0; }         // recomputes edge 0
+  }
+};
+__device__ __forceinline__ F4 sigmoid4(const F4 &x) {
+  const float2 a = unpack2(x.a), b = unpack2(x.b);
+  return F4{pack2(sigmoidf(a.x), sigmoidf(a.y)), pack2(sigmoidf(b.x), sigmoidf(b.y))};
+}
+// s (1 - s)
+__device__ __forceinline__ F4 slope4(const F4 &s) {
+  const u64 one = pack2(1.f, 1.f);
+  return F4{mul2(s.a, sub2(one, s.a)), mul2(s.b, sub2(one, s.b))};
+}
+__device__ __forceinline__ float most4(const F4 &v) {
+  const float2 a = unpack2(v.a), b = unpack2(v.b);
+  return fmaxf(fmaxf(a.x, a.y), fmaxf(b.x, b.y));
+}
+
+template <int LM, int FMT>
+__global__ void __launch_bounds__(kGateThreads)
+gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int per_block, const float *__restrict__ h1,
+                const ZpPlanes ht, const ZpScale scale, float *gate_max) {
+  zp_after_previous();
+  const GateItem it(E, t.H / 4, per_block);
+  const float inv = zp_publish_scale(ht, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
+  const float *gates = h1 + (size_t)it.e * t.w1_cols + it.h, *x = gates + t.n_gate;
+  uint16_t *const out = static_cast<uint16_t *>(ht.base) + it.e * ht.ld + it.h;
+  const int64_t plane_bytes = 2 * ht.plane_stride;
+  const u64 inv2 = pack2(inv, inv);
+  const int H = t.H;
+  float seen = 0.f;
+  auto row = [&](int r, const F4 &v, const F4 &s) {
+    if (it.live) put4<FMT>(out + r * H, plane_bytes, mul4(v, s), inv2);
+  };
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int r = rk[k];
-      // row 0: x * sigmoid(x) (g holds x there); other rows: x * sigmoid(gate of the row's degree)
-      const float s0 = sigmoidf(g[k].x), s1 = sigmoidf(g[k].y), s2 = sigmoidf(g[k].z), s3 = sigmoidf(g[k].w);
-      const float o[4] = {x[k].x * s0, x[k].y * s1, x[k].z * s2, x[k].w * s3};
-      // every gate l is used by the m = 0 row r = l: those rows alone probe sigmoid'
-      if (gate_max != nullptr && r >= 1 && r <= t.lmax) {
-        probe = true;
-        seen = fmaxf(seen, fmaxf(fmaxf(s0 * (1.f - s0), s1 * (1.f - s1)),
-                                 fmaxf(s2 * (1.f - s2), s3 * (1.f - s3))));
-      }
-      if (in_range && r >= 0) zp_store_planes<4>(ht, e * ht.ld + (int64_t)r * t.H + h, o, inv);
+  for (int l = 0; l <= LM; ++l) {
+    const int mm = t.mmax < l ? t.mmax : l;
+    // rows of the degree in the m'-major order: l, then +m and -m, LM + 1 - m rows apart
+    const int p1 = l + LM, m1 = p1 + LM, p2 = p1 + 2 * LM - 1, m2 = p2 + LM - 1;
+    const F4 x0 = load4(x + l * H);
+    F4 g, a1, b1, a2, b2;
+    if (l > 0) g = load4(gates + (l - 1) * H);
+    if (mm >= 1) { a1 = load4(x + p1 * H); b1 = load4(x + m1 * H); }
+    if (mm >= 2) { a2 = load4(x + p2 * H); b2 = load4(x + m2 * H); }
+    const F4 s = sigmoid4(l > 0 ? g : x0);      // l = 0: x sigmoid(x)
+    if (l > 0) seen = fmaxf(seen, most4(slope4(s)));
+    row(l, x0, s);
+    if (mm >= 1) { row(p1, a1, s); row(m1, b1, s); }
+    if (mm >= 2) { row(p2, a2, s); row(m2, b2, s); }
+    for (int m = 3, p = p2; m <= mm; ++m) {
+      const int km = LM + 1 - m;
+      p += 2 * (km + 1) - 1;
+      const F4 a = load4(x + p * H), b = load4(x + (p + km) * H);
+      row(p, a, s);
+      row(p + km, b, s);
     }
   }
-  if (__any_sync(0xffffffffu, probe)) {
+  if (gate_max) {
 #pragma unroll
     for (int k = 16; k > 0; k >>= 1) seen = fmaxf(seen, __shfl_xor_sync(0xffffffffu, seen, k));
     // one address for the whole grid: only warps that would raise the maximum touch it atomically
@@ -151,74 +176,56 @@ __global__ void gate_fwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
   }
 }
 
-// one thread per (edge, hidden-channel quad): walks the Km rows, accumulates the lmax gate grads.
-// The scale of the fp16 planes is fixed beforehand from max |dht| and the forward's gate bound:
+// Also sums the lmax gate gradients.  The scale of the fp16 planes is fixed beforehand from max |dht| and the
+// forward's gate bound:
 //   |dh1 row| <= 1.1 max|dht|  (sigmoid <= 1, silu' <= 1.1),
 //   |dh1 gate_l| = sigmoid'(g_l) |sum_rows dht h1| <= max|dht| * rows(l) * max|h1| * max sigmoid'.
-template <int LM>
-__global__ void __launch_bounds__(128, 6) gate_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E,
-                                const float *__restrict__ h1, const float *__restrict__ dht,
-                                const ZpPlanes dh1, const ZpScale scale) {
+template <int LM, int FMT>
+__global__ void __launch_bounds__(kGateThreads)
+gate_bwd_kernel(const __grid_constant__ ZpTables t, int64_t E, int per_block, const float *__restrict__ h1,
+                const float *__restrict__ dht, const ZpPlanes dh1, const ZpScale scale) {
   zp_after_previous();
-  const int H4 = t.H / 4;
-  const int item = blockIdx.y * blockDim.x + threadIdx.x;            // within a group of edges
-  const int le = item / H4;
-  const int64_t e0 = (int64_t)blockIdx.x * kGateEdges + le;
-  const bool in_range = le < kGateEdges && e0 < E;
-  const int64_t e = in_range ? e0 : 0;            // out-of-range threads recompute edge 0
-  const int h = (item - le * H4) * 4;
-  const float *row = h1 + (size_t)e * t.w1_cols;
-  const int64_t drow = e * dh1.ld;
-  const float inv = zp_publish_scale(
-      dh1, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
-  const float *dt = dht + (size_t)e * t.Km * t.H;
-  constexpr int NL = LM > 0 ? LM : 1;        // gates: one per degree 1..lmax
-  float sg[NL][4], dg[NL][4];
+  const GateItem it(E, t.H / 4, per_block);
+  const float inv = zp_publish_scale(dh1, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
+  const float *gates = h1 + (size_t)it.e * t.w1_cols + it.h, *x = gates + t.n_gate;
+  const float *d = dht + (size_t)it.e * t.Km * t.H + it.h;
+  uint16_t *const out = static_cast<uint16_t *>(dh1.base) + it.e * dh1.ld + it.h;
+  const int64_t plane_bytes = 2 * dh1.plane_stride;
+  const u64 inv2 = pack2(inv, inv);
+  const int H = t.H;
+  auto put = [&](int column, const F4 &v) {
+    if (it.live) put4<FMT>(out + column, plane_bytes, v, inv2);
+  };
 #pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    if (l < LM) {
-      const float4 g = *reinterpret_cast<const float4 *>(row + l * t.H + h);
-      sg[l][0] = sigmoidf(g.x); sg[l][1] = sigmoidf(g.y);
-      sg[l][2] = sigmoidf(g.z); sg[l][3] = sigmoidf(g.w);
+  for (int l = 0; l <= LM; ++l) {
+    const int mm = t.mmax < l ? t.mmax : l;
+    const int p1 = l + LM, m1 = p1 + LM, p2 = p1 + 2 * LM - 1, m2 = p2 + LM - 1;
+    const F4 x0 = load4(x + l * H), d0 = load4(d + l * H);
+    F4 g, a1, b1, a2, b2, c1, e1, c2, e2;
+    if (l > 0) g = load4(gates + (l - 1) * H);
+    if (mm >= 1) { a1 = load4(x + p1 * H); b1 = load4(x + m1 * H); c1 = load4(d + p1 * H); e1 = load4(d + m1 * H); }
+    if (mm >= 2) { a2 = load4(x + p2 * H); b2 = load4(x + m2 * H); c2 = load4(d + p2 * H); e2 = load4(d + m2 * H); }
+    const F4 s = sigmoid4(l > 0 ? g : x0), slope = slope4(s);
+    if (l == 0) {                        // d (s + x s (1 - s))
+      put(t.n_gate, mul4(d0, F4{fma2(x0.a, slope.a, s.a), fma2(x0.b, slope.b, s.b)}));
+      continue;
     }
-#pragma unroll
-    for (int v = 0; v < 4; ++v) dg[l][v] = 0.f;
-  }
-#pragma unroll 4
-  for (int r = 0; r < t.Km; ++r) {
-    const float4 x4 = *reinterpret_cast<const float4 *>(row + t.n_gate + r * t.H + h);
-    const float4 d4 = *reinterpret_cast<const float4 *>(dt + r * t.H + h);
-    const float x[4] = {x4.x, x4.y, x4.z, x4.w}, d[4] = {d4.x, d4.y, d4.z, d4.w};
-    float o[4];
-    if (r == 0) {
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const float s = sigmoidf(x[v]);
-        o[v] = d[v] * (s + x[v] * s * (1.f - s));
-      }
-    } else {
-      const int l = t.row_l[r] - 1;
-#pragma unroll
-      for (int ll = 0; ll < NL; ++ll) {
-        if (ll == l) {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            o[v] = d[v] * sg[ll][v];
-            dg[ll][v] = fmaf(d[v], x[v], dg[ll][v]);
-          }
-        }
-      }
+    F4 dg = zero4();
+    auto row = [&](int r, const F4 &xv, const F4 &dv) {
+      put(t.n_gate + r * H, mul4(dv, s));
+      dg.a = fma2(dv.a, xv.a, dg.a);
+      dg.b = fma2(dv.b, xv.b, dg.b);
+    };
+    row(l, x0, d0);
+    if (mm >= 1) { row(p1, a1, c1); row(m1, b1, e1); }
+    if (mm >= 2) { row(p2, a2, c2); row(m2, b2, e2); }
+    for (int m = 3, p = p2; m <= mm; ++m) {
+      const int km = LM + 1 - m;
+      p += 2 * (km + 1) - 1;
+      row(p, load4(x + p * H), load4(d + p * H));
+      row(p + km, load4(x + (p + km) * H), load4(d + (p + km) * H));
     }
-    if (in_range) zp_store_planes<4>(dh1, drow + t.n_gate + r * t.H + h, o, inv);
-  }
-#pragma unroll
-  for (int l = 0; l < NL; ++l) {
-    if (l < LM) {
-      float o[4];
-#pragma unroll
-      for (int v = 0; v < 4; ++v) o[v] = dg[l][v] * sg[l][v] * (1.f - sg[l][v]);
-      if (in_range) zp_store_planes<4>(dh1, drow + l * t.H + h, o, inv);
-    }
+    put((l - 1) * H, mul4(dg, slope));
   }
 }
 
@@ -633,13 +640,28 @@ int zp_launch_absmax_row_range(const float *in, int64_t cols, const int32_t *fir
   return ZP_OK;
 }
 
+// blocks of whole edges; of parts of one edge where its row is wider than a block
+static dim3 gate_grid(int64_t E, int H4, int *per_block, int *threads) {
+  *per_block = H4 <= kGateThreads ? kGateThreads / H4 : 1;
+  *threads = H4 <= kGateThreads ? (*per_block * H4 + 31) / 32 * 32 : kGateThreads;
+  return dim3((unsigned)zp_ceil_div(E, *per_block), (unsigned)zp_ceil_div(H4, H4 <= kGateThreads ? H4 : kGateThreads));
+}
+
 int zp_launch_gate_fwd(const zp_plan *p, int64_t E, const float *h1, const ZpPlanes &ht,
                        const ZpScale &scale, float *gate_max, cudaStream_t st) {
   if (E == 0) return ZP_OK;
-  const int per_group = kGateEdges * ((p->t.Km + 1) / 2) * (p->t.H / 4);
-  const dim3 grid((unsigned)zp_ceil_div(E, kGateEdges * kGateSub),
-                  (unsigned)zp_ceil_div(per_group, 256));
-  zp_launch(gate_fwd_kernel, grid, 256, 0, st, p->t, E, h1, ht, scale, gate_max);
+  int per_block, threads;
+  const dim3 grid = gate_grid(E, p->t.H / 4, &per_block, &threads);
+#define CALL_FMT(LM, FMT) zp_launch(gate_fwd_kernel<LM, FMT>, grid, threads, 0, st, p->t, E, per_block, h1, ht, scale, gate_max)
+#define CALL(LM)                                               \
+  switch (zp_plane_format(ht)) {                               \
+    case kFmtBf16: CALL_FMT(LM, kFmtBf16); break;              \
+    case kFmtFp16x2: CALL_FMT(LM, kFmtFp16x2); break;          \
+    default: CALL_FMT(LM, kFmtBf16x3); break;                  \
+  }
+  ZP_DISPATCH_LMAX(p->t.lmax, CALL)
+#undef CALL
+#undef CALL_FMT
   ZP_LAUNCH_CHECK("gate_fwd_kernel");
   return ZP_OK;
 }
@@ -647,11 +669,18 @@ int zp_launch_gate_fwd(const zp_plan *p, int64_t E, const float *h1, const ZpPla
 int zp_launch_gate_bwd(const zp_plan *p, int64_t E, const float *h1, const float *dht,
                        const ZpPlanes &dh1, const ZpScale &scale, cudaStream_t st) {
   if (E == 0) return ZP_OK;
-  const int per_group = kGateEdges * (p->t.H / 4);
-  const dim3 grid((unsigned)zp_ceil_div(E, kGateEdges), (unsigned)zp_ceil_div(per_group, 128));
-#define CALL(LM) zp_launch(gate_bwd_kernel<LM>, grid, 128, 0, st, p->t, E, h1, dht, dh1, scale)
+  int per_block, threads;
+  const dim3 grid = gate_grid(E, p->t.H / 4, &per_block, &threads);
+#define CALL_FMT(LM, FMT) zp_launch(gate_bwd_kernel<LM, FMT>, grid, threads, 0, st, p->t, E, per_block, h1, dht, dh1, scale)
+#define CALL(LM)                                               \
+  switch (zp_plane_format(dh1)) {                               \
+    case kFmtBf16: CALL_FMT(LM, kFmtBf16); break;              \
+    case kFmtFp16x2: CALL_FMT(LM, kFmtFp16x2); break;          \
+    default: CALL_FMT(LM, kFmtBf16x3); break;                  \
+  }
   ZP_DISPATCH_LMAX(p->t.lmax, CALL)
 #undef CALL
+#undef CALL_FMT
   ZP_LAUNCH_CHECK("gate_bwd_kernel");
   return ZP_OK;
 }
