@@ -137,3 +137,17 @@ def test_long_lists(atoms, cap, outside):
     from oracle import neighbors_oracle as no
     for a, b in zip(run(pos, 20.0, 6.0, cap), no.neighbor_list(pos, 20.0, 6.0, cap)):
         assert a.shape == b.shape and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("n,box,cap", [(700, 17.0, 30), (900, 16.0, 8), (900, 16.0, 60), (400, 9.0, 30)])
+def test_cap_reached_near_by_and_not(n, box, cap):
+    """Two thirds of the atoms in a third of the box: some find the cap within the radius that is tried first, some
+    only within the cutoff, some not at all."""
+    from oracle import neighbors_oracle as no
+    rng = np.random.default_rng(n + cap)
+    pos = rng.random((n, 3)) * box
+    pos[:2 * n // 3, 0] /= 3.0
+    pos[:20] = np.round(pos[:20])                      # equal distances
+    want = no.neighbor_list(pos, box, 6.0, cap)
+    for g, w in zip(run(pos, box, 6.0, cap), want):
+        assert g.shape == w.shape and np.array_equal(g, w)

@@ -41,11 +41,15 @@ constexpr int kKept = 128;                         // edges per destination kept
 constexpr int kScanBlock = 1024;
 
 struct Grid {
-  double box, per_cell, cutoff2;   // per_cell: cells per unit of length
+  double box, per_cell;            // per_cell: cells per unit of length
   int nc;          // cells per dimension
   int w;           // search half-width in cells
   int reach;       // largest |image| component that can occur
-  float reach2;    // (cutoff / cell)^2 and a margin for working in fp32
+  struct Sphere {
+    double r2;     // pairs closer than its root
+    float reach2;  // (radius / cell)^2 and a margin for working in fp32
+    int w;         // half-width in cells
+  } all, near;     // the cutoff; where a cap binds, what most probably holds that many (else all again)
 };
 
 // words of the workspace's head: error bits, whether an atom lies outside the box, crowded atoms
@@ -175,12 +179,13 @@ int exclusive_scan(int64_t n, const int32_t *in, int32_t *out, int32_t *block_su
 
 // Calls f(hit, src, image code, d2) on all 32 lanes together for every batch of candidate
 // (source, image) pairs around destination j; `hit` marks the lanes whose candidate lies within
-// the cutoff.  The walk goes on while f returns true (the same on all lanes).  Bound by instruction
+// the sphere.  The walk goes on while f returns true (the same on all lanes).  Bound by instruction
 // issue: what hangs on images alone is formed once per column, and the conversions and products
 // of a shift are left out where it is zero (in a large cell, for most atoms).
 constexpr int kNoImage = 512 | 512 << 10 | 512 << 20;
 template <typename F>
-__device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__restrict__ cell_start,
+__device__ __forceinline__ void for_each_hit(const Grid &g, const Grid::Sphere &ball,
+                                             const int32_t *__restrict__ cell_start,
                                              const Sorted &atoms, int64_t at, int lane, F &&f) {
   const double xj = atoms.x[at], yj = atoms.y[at], zj = atoms.z[at];
   const int4 own = atoms.who[at];
@@ -189,21 +194,21 @@ __device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__res
                wz = (zj - own.z * g.box) * g.per_cell;
   const int cx = clamp_cell(wx, g), cy = clamp_cell(wy, g), cz = clamp_cell(wz, g);
   const float fx = (float)(wx - cx), fy = (float)(wy - cy), fz = (float)(wz - cz);
-  const int side = 2 * g.w + 1, columns = side * side;
-  const int kz1 = cell_image(cz + g.w, g);
+  const int w = ball.w, side = 2 * w + 1, columns = side * side;
+  const int kz1 = cell_image(cz + w, g);
   for (int q0 = 0; q0 < columns; q0 += 32) {
     // a lane per column of cells along z, cut to what the cutoff can reach
     const int q = q0 + lane;
-    const int ox = q / side - g.w, oy = q % side - g.w;
+    const int ox = q / side - w, oy = q % side - w;
     const float ax = ox > 0 ? ox - fx : ox < 0 ? fx - (ox + 1) : 0.f;
     const float ay = oy > 0 ? oy - fy : oy < 0 ? fy - (oy + 1) : 0.f;
-    const float r2 = g.reach2 - (ax * ax + ay * ay);
+    const float r2 = ball.reach2 - (ax * ax + ay * ay);
     const bool in = q < columns && r2 > 0.f;
     const float r = in ? sqrtf(r2) : 0.f;
-    const int u0 = max(cz - g.w, cz + (int)floorf(fz - r)), u1 = min(cz + g.w, cz + (int)floorf(fz + r));
+    const int u0 = max(cz - w, cz + (int)floorf(fz - r)), u1 = min(cz + w, cz + (int)floorf(fz + r));
     const int kx = cell_image(cx + ox, g), ky = cell_image(cy + oy, g);
     const int column = ((cx + ox - kx * g.nc) * g.nc + (cy + oy - ky * g.nc)) * g.nc;
-    for (int kz = cell_image(cz - g.w, g); kz <= kz1; ++kz) {
+    for (int kz = cell_image(cz - w, g); kz <= kz1; ++kz) {
       const int z0 = max(u0 - kz * g.nc, 0), z1 = min(u1 - kz * g.nc, g.nc - 1);
       int off = 0, len = 0;
       const int image = (512 - kx) | (512 - ky) << 10 | (512 - kz) << 20;
@@ -253,7 +258,7 @@ __device__ __forceinline__ void for_each_hit(const Grid &g, const int32_t *__res
             self = self && mx == 0 && my == 0 && mz == 0;
           }
           d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-          hit = d2 < g.cutoff2 && !self;
+          hit = d2 < ball.r2 && !self;
         }
         if (!f(hit, i, code, d2)) return;
       }
@@ -316,12 +321,12 @@ struct Writer {
 
 // Moves the ties of the `cap` nearest of the n <= 32 R hits to the front, n > cap > 0.
 template <int R>
-__device__ __forceinline__ void keep_nearest(Hit *h, int n, int cap, float cutoff2, int lane) {
+__device__ __forceinline__ void keep_nearest(Hit *h, int n, int cap, float radius2, int lane) {
       float near[R];                // rounding to fp32 keeps the order, or makes equals
 #pragma unroll
       for (int k = 0; k < R; ++k) near[k] = lane + 32 * k < n ? (float)h[lane + 32 * k].d2 : INFINITY;
       // close in on a distance that exactly `cap` hits do not exceed: by interpolation and by halves
-      float lo = 0.f, hi = cutoff2;
+      float lo = 0.f, hi = radius2;
       int below_lo = 0, below_hi = n;
       unsigned alive[R];            // survivors, a bit per lane
       bool found = false;
@@ -387,17 +392,24 @@ select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const S
   const int64_t j = atoms.who[at].w;           // in cell order: neighbours read the same cells
   Hit *h = hits[warp];
   int n = 0;                      // hits seen (warp-uniform)
-  for_each_hit(g, cell_start, atoms, at, lane,
-               [&](bool hit, int i, unsigned code, double d2) {
-                 const unsigned m = __ballot_sync(0xffffffffu, hit);
-                 const int slot = n + __popc(m & ((1u << lane) - 1u));
-                 if (hit && slot < kFewHits) {
-                   h[slot].d2 = d2;
-                   h[slot].tie = ((unsigned long long)(unsigned)i << 32) | code;
-                 }
-                 n += __popc(m);
-                 return n <= kFewHits || cap <= 0 || n < cap;    // past both the count is known
-               });
+  bool everything = g.near.r2 == g.all.r2;
+  for (;;) {
+    for_each_hit(g, everything ? g.all : g.near, cell_start, atoms, at, lane,
+                 [&](bool hit, int i, unsigned code, double d2) {
+                   const unsigned m = __ballot_sync(0xffffffffu, hit);
+                   const int slot = n + __popc(m & ((1u << lane) - 1u));
+                   if (hit && slot < kFewHits) {
+                     h[slot].d2 = d2;
+                     h[slot].tie = ((unsigned long long)(unsigned)i << 32) | code;
+                   }
+                   n += __popc(m);
+                   return n <= kFewHits || cap <= 0 || n < cap;    // past both the count is known
+                 });
+    if (everything || n >= cap) break;
+    everything = true;            // fewer than the cap so near: all within the cutoff
+    n = 0;
+    __syncwarp();
+  }
   kept += j * stride;
   if (n > kFewHits || (n > kKept && (cap <= 0 || cap > kKept))) {             // left to fill_many_kernel
     if (lane == 0) {
@@ -410,10 +422,12 @@ select_kernel(int64_t N, Grid g, const int32_t *__restrict__ cell_start, const S
   }
   __syncwarp();
   if (cap > 0 && n > cap) {
-    if (n <= 128)
-      keep_nearest<4>(h, n, cap, (float)g.cutoff2, lane);
+    if (n <= 64)
+      keep_nearest<2>(h, n, cap, (float)(everything ? g.all : g.near).r2, lane);
+    else if (n <= 128)
+      keep_nearest<4>(h, n, cap, (float)(everything ? g.all : g.near).r2, lane);
     else
-      keep_nearest<kFewHits / 32>(h, n, cap, (float)g.cutoff2, lane);
+      keep_nearest<kFewHits / 32>(h, n, cap, (float)(everything ? g.all : g.near).r2, lane);
     n = cap;
   }
   if (lane == 0) counts[j] = n;
@@ -467,7 +481,7 @@ fill_many_kernel(const int32_t *__restrict__ crowded, const int4 *__restrict__ o
     const Hit inf{INFINITY, ~0ull};
     int n = 0;                      // hits held (warp-uniform)
     bool overflow = false;
-    for_each_hit(g, cell_start, atoms, at, lane,
+    for_each_hit(g, g.all, cell_start, atoms, at, lane,
                  [&](bool hit, int i, unsigned code, double d2) {
                    const unsigned m = __ballot_sync(0xffffffffu, hit);
                    const int add = __popc(m);
@@ -530,26 +544,51 @@ struct NbWork {
   size_t bytes;
 };
 
-int make_grid(int64_t N, double box, double cutoff, Grid *g) {
+// Radius that the `cap` nearest of an atom most probably lie within: a uniform gas has that many 3.5
+// standard deviations below its mean there (one atom in 4 000 has not, and is walked again).  The cutoff, if that
+// leaves less than a fifth of the sphere out.  100 000 atoms of 90 hits, cap 30: a sphere of 56.
+double near_radius(int64_t N, double box, double cutoff, int cap) {
+  if (cap <= 0) return cutoff;
+  const double held = (double)N / (box * box * box) * (4.0 / 3.0 * 3.14159265358979) * cutoff * cutoff * cutoff;
+  const double want = cap + 4.0 * std::sqrt((double)cap) + 4.0;
+  return want < 0.8 * held ? cutoff * std::cbrt(want / held) : cutoff;
+}
+
+constexpr int kMaxCells = 256;           // per dimension
+
+int make_grid(int64_t N, double box, double cutoff, int cap, Grid *g) {
   if (!(box > 0.0) || !(cutoff > 0.0) || !std::isfinite(box) || !std::isfinite(cutoff))
     return ZP_ERR_INVALID_ARG;
-  // Cells a hair wider than the cutoff, so that a last-bit rounding of a cell coordinate can
-  // never put a pair within the cutoff more than w cells apart.  Half-cutoff cells leave 2.4 times
+  // Cells a hair wider than the radius, so that a last-bit rounding of a cell coordinate can
+  // never put a pair within it more than w cells apart.  Half-radius cells leave 2.4 times
   // as few candidates outside the sphere and still give a warp one column per lane (25); they
   // are taken when they are no more than the atoms, so that clearing and scanning them is cheap.
-  const double wide = cutoff * (1.0 + 1e-9);
-  int nc = (int)std::floor(box / (0.5 * wide));
-  if (nc < 1 || nc > 256 || (int64_t)nc * nc * nc > N) nc = (int)std::floor(box / wide);
-  if (nc < 1) nc = 1;
-  if (nc > 256) nc = 256;
+  constexpr double kHair = 1.0 + 1e-9;
+  const double wide = cutoff * kHair;
+  auto halves = [&](double radius) {
+    const double cells = std::floor(box / (0.5 * radius * kHair));
+    const bool fit = cells >= 1 && cells <= kMaxCells && cells * cells * cells <= (double)N;
+    return fit ? (int)cells : 0;
+  };
+  double near = near_radius(N, box, cutoff, cap);
+  int nc = halves(near);
+  if (nc == 0 && near < cutoff) nc = halves(near = cutoff);
+  if (nc == 0) {
+    near = cutoff;
+    const double cells = std::floor(box / wide);
+    nc = cells < 1 ? 1 : cells > kMaxCells ? kMaxCells : (int)cells;
+  }
   g->box = box;
   g->nc = nc;
   const double cell = box / nc;
   g->per_cell = nc / box;
-  g->cutoff2 = cutoff * cutoff;
-  g->reach2 = (float)(1.0001 * (cutoff / cell) * (cutoff / cell));
-  g->w = (int)std::ceil(wide / cell);
-  if (g->w < 1) g->w = 1;
+  auto sphere = [&](double radius) {
+    const int w = (int)std::ceil(radius * kHair / cell);
+    return Grid::Sphere{radius * radius, (float)(1.0001 * (radius / cell) * (radius / cell)), w < 1 ? 1 : w};
+  };
+  g->all = sphere(cutoff);
+  g->near = sphere(near);
+  g->w = g->all.w;
   g->reach = (int)std::ceil(cutoff / box);
   if (g->reach < 1) g->reach = 1;
   if (g->reach > 8) return ZP_ERR_UNSUPPORTED;         // box far smaller than the cutoff
@@ -559,7 +598,8 @@ int make_grid(int64_t N, double box, double cutoff, Grid *g) {
 // edges per destination kept from pass 1 to pass 2
 int kept_stride(int cap) { return cap > 0 && cap < kKept ? cap : kKept; }
 
-NbWork carve_nb(int64_t N, const Grid &g, int cap, void *base) {
+// most: room for the grid of any cap
+NbWork carve_nb(int64_t N, const Grid &g, int cap, void *base, bool most = false) {
   NbWork w;
   size_t off = 0;
   auto take = [&](size_t n) {
@@ -568,7 +608,8 @@ NbWork carve_nb(int64_t N, const Grid &g, int cap, void *base) {
     off += zp_align_up(n * sizeof(int32_t), 256);
     return p;
   };
-  const size_t cells = (size_t)g.nc * g.nc * g.nc;
+  size_t cells = (size_t)g.nc * g.nc * g.nc;
+  if (most) cells = std::max(cells, std::min<size_t>((size_t)N, (size_t)kMaxCells * kMaxCells * kMaxCells));
   w.flags = take((size_t)N + 4);
   w.crowded = w.flags + kCrowdedList;      // how many, then which
   w.cell_count = take(cells + 1);
@@ -592,12 +633,14 @@ NbWork carve_nb(int64_t N, const Grid &g, int cap, void *base) {
 extern "C" {
 
 size_t zp_neighbors_work_bytes(int64_t n_atoms, double box, double cutoff) {
-  return zp_neighbors_work_bytes_capped(n_atoms, box, cutoff, 0);
+  Grid g;
+  if (n_atoms < 0 || make_grid(n_atoms, box, cutoff, 0, &g)) return 0;
+  return carve_nb(n_atoms, g, 0, nullptr, true).bytes;
 }
 
 size_t zp_neighbors_work_bytes_capped(int64_t n_atoms, double box, double cutoff, int max_neighbors) {
   Grid g;
-  if (n_atoms < 0 || make_grid(n_atoms, box, cutoff, &g)) return 0;
+  if (n_atoms < 0 || make_grid(n_atoms, box, cutoff, max_neighbors, &g)) return 0;
   return carve_nb(n_atoms, g, max_neighbors, nullptr).bytes;
 }
 
@@ -605,7 +648,7 @@ int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, 
                        int32_t *row_ptr, int32_t *flags_out, void *work, size_t work_bytes,
                        void *stream) {
   Grid g;
-  int rc = make_grid(N, box, cutoff, &g);
+  int rc = make_grid(N, box, cutoff, max_neighbors, &g);
   if (rc) return rc;
   if (N < 0 || N > 2000000000ll || !row_ptr || !flags_out || !work || (N && !pos))
     return ZP_ERR_INVALID_ARG;
@@ -640,7 +683,7 @@ int zp_neighbors_fill(const double *pos, int64_t N, double box, double cutoff, i
                       const int32_t *row_ptr, int64_t E, int64_t *edge_index, double *shifts,
                       int32_t *flags_out, void *work, size_t work_bytes, void *stream) {
   Grid g;
-  int rc = make_grid(N, box, cutoff, &g);
+  int rc = make_grid(N, box, cutoff, max_neighbors, &g);
   if (rc) return rc;
   if (N < 0 || E < 0 || !row_ptr || !flags_out || !work || (N && !pos) ||
       (E && (!edge_index || !shifts)))
