@@ -24,7 +24,6 @@ thread_local int64_t g_launches = 0;
 // training step, apart / together: lmax 4, C 128 within 2 % of each other from 12 000 to 84 000 edges, fp32
 // and bf16; lmax 2, C 128 at 24 000 / 60 000 / 84 000 edges 1.79 / 3.93 / 5.38 ms against 1.64 / 3.71 /
 // 5.16; lmax 2, C 64 1.14 / 2.10 / 2.75 against 1.04 / 1.95 / 2.57: narrow ones would gain from a higher one.
-constexpr int64_t kTogetherEdges = 24000;
 constexpr int kChunkK = 2048;          // contraction length of one TMEM accumulation chunk
 
 // The fused epilogues (gate activation in conv1, rotation back + segmented sums in conv2) need
@@ -784,14 +783,17 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   // that was there before it.  On the second side stream the radial layer's parameter gradients,
   // on the first the last sums of the convolutions'.
   if ((rc = lanes.fork())) return rc;
+  const bool together = E <= kTogetherEdges;
   if (rl && E > 0) {
-    ZpFinalList radial_list;
+    ZpFinalList own;
+    ZpFinalList &radial_list = together && rl->later ? *rl->later : own;
+    const cudaStream_t side = together && !rl->later ? st : lanes.pick(2);
     ZP_TIMED(ZP_K_GEMM_WGRAD,
              zp_linear_backward_planes(plan, E, rl->ec, t.R, ws.hr, ws.rw, ws.gr, rl->grad_h,
                                        rl->grad_w, rl->grad_b, ws.rad_partials,
                                        zp_radial_splits(t.R, rl->ec), ws.col_rad, radial_list, st,
-                                       lanes.pick(2), rl->grad_h_max));
-    ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(radial_list, lanes.pick(2)));
+                                       side, rl->grad_h_max));
+    ZP_TIMED(ZP_K_FOLD, zp_launch_finalize(own, side));
   } else if (rl && rl->grad_w) {
     ZP_CUDA(cudaMemsetAsync(rl->grad_w, 0, sizeof(float) * (size_t)t.R * rl->ec, st));
     ZP_CUDA(cudaMemsetAsync(rl->grad_b, 0, sizeof(float) * (size_t)t.R, st));
@@ -805,7 +807,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                    zp_torque_slots(t),
                                    ZpTorqueArgs{ws.da1, radial, c.x_node, ws.y, grad_node_out, c.env,
                                                 c.src, c.dst, ws.rot_grad},
-                                   grad_edge_vec, st));
+                                   grad_edge_vec, together ? lanes.pick(2) : st));
   return ZP_OK;
 }
 
@@ -882,7 +884,7 @@ int zp_eso2_forward_radial(const zp_plan *plan, int64_t N, int64_t E, const floa
                            const int32_t *dst, const int32_t *row_ptr, const zp_weights *w,
                            float *node_out, void *workspace, size_t workspace_bytes,
                            int keep_for_backward, void *stream) {
-  const ZpRadialLayer rl{h_rad, rad_w, rad_b, edge_channels, nullptr, nullptr, nullptr, nullptr};
+  const ZpRadialLayer rl{h_rad, rad_w, rad_b, edge_channels, nullptr, nullptr, nullptr, nullptr, nullptr};
   return eso2_forward(plan, N, E, x_node, edge_vec, cos_g, sin_g, nullptr, env, src, dst, row_ptr,
                       w, node_out, workspace, workspace_bytes, stream, keep_for_backward, &rl);
 }
@@ -898,7 +900,7 @@ int zp_eso2_backward_radial(const zp_plan *plan, int64_t N, int64_t E, const flo
                             float *grad_env, const zp_weight_grads *gw, void *workspace,
                             size_t workspace_bytes, void *stream) {
   const ZpRadialLayer rl{h_rad, rad_w, rad_b, edge_channels, grad_h_rad, grad_rad_w, grad_rad_b,
-                         nullptr};
+                         nullptr, nullptr};
   return eso2_backward(plan, N, E, grad_node_out, x_node, edge_vec, cos_g, sin_g, nullptr, env, src,
                        dst, row_ptr, perm_src, row_ptr_src, w, grad_x_node, grad_edge_vec, nullptr,
                        grad_env, gw, workspace, workspace_bytes, stream, &rl);

@@ -285,7 +285,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
   // what the gradients of positions, embedding table and radial parameters all go through
   const bool chain = grad_pos || want_rad || grads->emb;
   ZpRadialLayer rl{nullptr, nullptr, nullptr, ec, chain && E > 0 ? b.g_hid1 : nullptr,
-                   grads->rad_w[2], grads->rad_b[2], fm.f1.fp16 ? sc + kScGHid1 : nullptr};
+                   grads->rad_w[2], grads->rad_b[2], fm.f1.fp16 ? sc + kScGHid1 : nullptr, &list};
   const ZpConv c{rows, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
                  call->dst, call->row_ptr, call->perm_src, call->row_ptr_src, &params->so2};
   ZpLanes lanes(plan, E, st);
@@ -316,7 +316,9 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                                                   sc + kScDz1),
                                     grads->ln_gamma[1], grads->ln_beta[1], grads->rad_b[1], ln1, list, st)))
       return rc;
-    if (want_rad && (rc = lanes.fork(2))) return rc;       // their weight gradients on the side
+    // their weight gradients on the side, where they are launches of their own
+    const bool apart = want_rad && E > kTogetherEdges;
+    if (apart && (rc = lanes.fork(2))) return rc;
     if ((rc = zp_linear_backward_planes(plan, E, ec, ec, b.hid0, b.w1, b.dz1, b.g_hid0,
                                         grads->rad_w[1], nullptr, b.part1, zp_radial_splits(ec, ec), nullptr,
                                         list, st, lanes.pick(2), fm.f0.fp16 ? sc + kScGHid0 : nullptr)))
@@ -330,11 +332,12 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
     // without an embedding gradient only the distance basis' columns of the input gradient are used
     const int64_t cols = grads->emb ? w0 : front->num_basis;
     const bool want_in = grad_pos || grads->emb;
-    if (want_rad && (rc = lanes.fork(2))) return rc;
+    if (apart && (rc = lanes.fork(2))) return rc;
     if ((rc = zp_linear_backward_planes(plan, E, w0, ec, b.xe, b.w0, b.dz0, want_in ? b.g_xe : nullptr,
                                         grads->rad_w[0], nullptr, b.part0, zp_radial_splits(ec, w0), nullptr,
                                         list, st, lanes.pick(2), nullptr, cols)))
       return rc;
+    if (!apart && (rc = lanes.join(2))) return rc;         // the rotation's part of the edge vectors' gradient
     if (want_in &&
         (rc = zp_launch_edge_features_bwd(*front, rows, E, b.edge_vec, b.dist, params->gauss_offsets,
                                           call->atomic_numbers, b.g_vec_rot, b.g_xe, round4(cols),

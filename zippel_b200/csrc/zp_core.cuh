@@ -91,6 +91,9 @@ enum { kScX = 0, kScRad, kScH1, kScA1, kScHt, kScDy, kScDh1, kScGate, kScMaxNode
        kScRstd1, kScW0, kScW0Scale, kScW1, kScW1Scale, kScXe, kScHid0, kScDz1, kScDz0,
        kScCount };
 
+// Up to this many edges the products of a step share one launch (zp_api.cu has the reasons).
+constexpr int64_t kTogetherEdges = 24000;
+
 constexpr int kZpWgradSplits = 8;
 // K splits of a radial layer's weight gradient [N, K], whose contraction runs over the edges: as many
 // as it takes to give every SM a share of the few tiles (eight left 140 SMs idle for 100 us at
@@ -188,6 +191,8 @@ struct ZpRadialLayer {
   int ec;
   float *grad_h, *grad_w, *grad_b;       // backward only
   float *grad_h_max;                     // device scalar updated with max |grad_h|, or null
+  ZpFinalList *later;                    // takes the last sums of the layer's parameter gradients where
+                                         // its products share a launch (null: they are formed at once)
 };
 
 int zp_check_weights(const zp_plan *p, const zp_weights *w);

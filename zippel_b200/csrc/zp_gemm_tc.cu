@@ -1880,22 +1880,34 @@ int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits) {
   return best;
 }
 
-// The K split of a group's products whose contraction runs over the edges (the last `nw` of n): the one
-// with which the launch gets done first, but no more partial results than that takes.
+// The K split of a group's products whose contraction runs over the edges (the last `nw` of n): of a few
+// that cut their tiles to between a whole and a third of the launch's time, the one with which it gets done
+// first, but no more partial results than that takes.
 void zp_gemm_group_splits(ZpGemmTc *g, int n, int nw, int max_splits) {
   const ZpGemmTc *all[ZP_GEMM_GROUP];
   if (n > ZP_GEMM_GROUP) n = ZP_GEMM_GROUP;
   for (int i = 0; i < n; ++i) all[i] = &g[i];
   const bool pair = group_may_pair(all, n);
-  int best = 1;
-  double best_cost = 1e300;
-  for (int s = 1; s <= max_splits; ++s) {
+  const int units = pair ? device_sms() / 2 : device_sms();
+  const int bk = pair ? pair_block_k(g[0].planes) : single_block_k(g[0].planes, 0);
+  GroupPlan pl;
+  auto split = [&](int s) {
     for (int i = n - nw; i < n; ++i) g[i].ksplit = s;
-    GroupPlan pl;
-    plan_group(pl, all, n, pair, pair ? pair_block_k(all[0]->planes) : single_block_k(all[0]->planes, 0), 256,
-               pair ? device_sms() / 2 : device_sms());
+    plan_group(pl, all, n, pair, bk, 256, units);
+  };
+  split(1);
+  double work = 0.0;
+  for (int k = 0; k < n; ++k) work += pl.shape[k].cost * (double)pl.shape[k].tiles;
+  const int whole = (int)std::ceil(pl.shape[0].cost / (work / units));     // the longest tile is one of theirs
+  int best = 1;
+  double best_cost = pl.makespan;
+  for (int thirds = 2; thirds <= 9; thirds += thirds < 4 ? 1 : 2) {
+    const int s = std::min(max_splits, (int)zp_ceil_div((int64_t)whole * thirds, 3));
+    if (s <= 1) continue;
+    split(s);
     const double cost = pl.makespan * (1.0 + 0.004 * s);
     if (cost < best_cost) { best_cost = cost; best = s; }
+    if (s == max_splits) break;
   }
   for (int i = n - nw; i < n; ++i) g[i].ksplit = best;
 }

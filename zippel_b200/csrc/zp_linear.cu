@@ -6,7 +6,7 @@
 // No transposed copies are made: W [N, K] as stored is the K-major B operand of the forward, the
 // MN-major B operand of the input gradient (contraction over N), and x / dy as stored are the
 // MN-major operands of the weight gradient (contraction over the M rows).
-#include "zp_common.cuh"
+#include "zp_core.cuh"
 
 namespace {
 
@@ -85,24 +85,31 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
                               float *dw, float *db, float *partials, int max_splits,
                               float *colsum_scratch, ZpFinalList &list, cudaStream_t st,
                               cudaStream_t side, float *dx_absmax, int64_t dx_cols) {
-  int rc;
+  int rc, n = 0;
   const int P = dy.planes, fp16 = dy.fp16;
+  const bool together = dx && dw && M <= kTogetherEdges;
+  ZpGemmTc g[2];
   if (dx) {
     const int64_t cols = dx_cols > 0 ? dx_cols : K;
-    const ZpGemmTc g{M, cols, N, P, dy.base, dy.ld, dy.plane_stride, 0,
-                     w.base, w.ld, w.plane_stride, 1, nullptr, dx, (cols + 3) / 4 * 4,
-                     plan->status_dev, 0, 1, 0, 0, fp16, dy.scale, w.scale, dx_absmax};
-    if ((rc = zp_launch_gemm_tc(g, st))) return rc;
+    g[n++] = ZpGemmTc{M, cols, N, P, dy.base, dy.ld, dy.plane_stride, 0,
+                      w.base, w.ld, w.plane_stride, 1, nullptr, dx, (cols + 3) / 4 * 4,
+                      plan->status_dev, 0, 1, 0, 0, fp16, dy.scale, w.scale, dx_absmax};
+    if (!together && (rc = zp_launch_gemm_tc(g[0], st))) return rc;
   }
   if (dw) {
     const int64_t ldk = (K + 3) / 4 * 4;         // rows of the partial sums start 16-byte aligned
-    ZpGemmTc g{N, K, M, P, dy.base, dy.ld, dy.plane_stride, 1,
-               x.base, x.ld, x.plane_stride, 1, nullptr, partials, ldk, plan->status_dev,
-               0, 1, N * ldk, 0, fp16, dy.scale, x.scale, nullptr};
-    g.ksplit = zp_gemm_tc_pick_splits(g, max_splits);
-    const int splits = zp_gemm_tc_splits(g);
-    if ((rc = zp_launch_gemm_tc(g, side))) return rc;
-    list.add(partials, dw, N * ldk, (int)N, (int)K, splits, ZP_FIN_SUM, (int)ldk);
+    ZpGemmTc &wg = g[n++];
+    wg = ZpGemmTc{N, K, M, P, dy.base, dy.ld, dy.plane_stride, 1,
+                  x.base, x.ld, x.plane_stride, 1, nullptr, partials, ldk, plan->status_dev,
+                  0, 1, N * ldk, 0, fp16, dy.scale, x.scale, nullptr};
+    if (together) {
+      zp_gemm_group_splits(g, n, 1, max_splits);
+      if ((rc = zp_launch_gemm_group(g, n, st))) return rc;
+    } else {
+      wg.ksplit = zp_gemm_tc_pick_splits(wg, max_splits);
+      if ((rc = zp_launch_gemm_tc(wg, side))) return rc;
+    }
+    list.add(partials, dw, N * ldk, (int)N, (int)K, zp_gemm_tc_splits(wg), ZP_FIN_SUM, (int)ldk);
   }
   if (db) return zp_launch_colsum(M, N, dy, db, colsum_scratch, list, side);
   return ZP_OK;
