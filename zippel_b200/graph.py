@@ -13,6 +13,7 @@ and applies no neighbour cap (fixtures/make_fixtures.py:13-15); both are defined
 
 from __future__ import annotations
 
+import ctypes
 import dataclasses
 
 import numpy as np
@@ -100,21 +101,18 @@ class EdgeGraph:
         the reference.  Skipped while the stream is being captured into a CUDA graph (no
         synchronisation is possible there; the kernels leave such edges out either way)."""
         lib, ei, e, dev = EdgeGraph._open(edge_index)
-        perm, src, dst, perm_src, row_ptr, row_ptr_src, work = EdgeGraph._arrays(lib, e, n_nodes, dev)
-        nbytes = work.numel()
-        with torch.cuda.device(dev):
-            st = torch.cuda.current_stream().cuda_stream
-            _lib.check(lib.zp_csr_build(ei.data_ptr(), e, n_nodes, perm.data_ptr(), src.data_ptr(),
-                                        dst.data_ptr(), row_ptr.data_ptr(), perm_src.data_ptr(),
-                                        row_ptr_src.data_ptr(), work.data_ptr(), nbytes, st),
-                       "zp_csr_build")
-            if validate and e and not torch.cuda.is_current_stream_capturing():
-                import ctypes
-                flag = ctypes.c_int(0)
-                _lib.check(lib.zp_csr_status(work.data_ptr(), st, ctypes.byref(flag)), "zp_csr_status")
-                if flag.value:
-                    raise IndexError(f"edge_index names a node outside [0, {n_nodes})")
-        return EdgeGraph(n_nodes, e, perm[:e], src[:e], dst[:e], row_ptr, perm_src[:e], row_ptr_src)
+        graph = EdgeGraph(n_nodes, e, *EdgeGraph._arrays(e, n_nodes, dev))
+        work = torch.empty(lib.zp_csr_work_bytes(e, n_nodes), dtype=torch.uint8, device=dev)
+        _lib.run(dev, "zp_csr_build", ei.data_ptr(), e, n_nodes, *graph.addresses(), work.data_ptr(), work.numel())
+        if validate and e:
+            with torch.cuda.device(dev):
+                if not torch.cuda.is_current_stream_capturing():
+                    flag = ctypes.c_int(0)
+                    _lib.check(lib.zp_csr_status(work.data_ptr(), torch.cuda.current_stream().cuda_stream,
+                                                 ctypes.byref(flag)), "zp_csr_status")
+                    if flag.value:
+                        raise IndexError(f"edge_index names a node outside [0, {n_nodes})")
+        return graph
 
     @staticmethod
     def _open(edge_index: torch.Tensor):
@@ -124,11 +122,12 @@ class EdgeGraph:
         return _lib.load(), ei, ei.shape[1], ei.device
 
     @staticmethod
-    def _arrays(lib, e: int, n_nodes: int, dev):
-        i32 = dict(dtype=torch.int32, device=dev)
-        edges = [torch.empty(max(e, 1), **i32) for _ in range(4)]
-        work = torch.empty(lib.zp_csr_work_bytes(e, n_nodes), dtype=torch.uint8, device=dev)
-        return (*edges, torch.empty(n_nodes + 1, **i32), torch.empty(n_nodes + 1, **i32), work)
+    def _arrays(e: int, n_nodes: int, dev) -> tuple:
+        """perm, src, dst, row_ptr, perm_src, row_ptr_src as parts of one allocation, each from a 256-byte boundary
+        on: an allocation for each cost the host as much as eight launches."""
+        sizes = (e, e, e, n_nodes + 1, e, n_nodes + 1)
+        steps = [n for size in sizes for n in (size, 64 - size % 64)]
+        return torch.empty(sum(steps), dtype=torch.int32, device=dev).split(steps)[::2]
 
     @staticmethod
     def build_checked(edge_index: torch.Tensor, atomic_numbers: torch.Tensor, n_elements: int):
@@ -289,23 +288,18 @@ def neighbor_list(pos: torch.Tensor, box: float, cutoff: float,
     work = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     out = torch.empty(n + 2, dtype=torch.int32, device=dev)       # row_ptr and, read with its end, flags
     row_ptr, flags = out[:n + 1], out[n + 1:]
-    with torch.cuda.device(dev):
-        st = torch.cuda.current_stream().cuda_stream
-        _lib.check(lib.zp_neighbors_count(p.data_ptr(), n, float(box), float(cutoff), cap,
-                                          row_ptr.data_ptr(), flags.data_ptr(), work.data_ptr(),
-                                          nbytes, st), "zp_neighbors_count")
-        e, fl = out[n:].tolist()
-        if fl & 1:
-            raise ValueError("neighbor_list: positions must be finite")
-        if fl & 2:
-            raise _lib.ZpError(7, "zp_neighbors_count (more neighbours per atom than an uncapped "
-                                  "list can hold)")
-        edge_index = torch.empty(2, e, dtype=torch.int64, device=dev)
-        shifts = torch.empty(e, 3, dtype=torch.float64, device=dev)
-        _lib.check(lib.zp_neighbors_fill(p.data_ptr(), n, float(box), float(cutoff), cap,
-                                         row_ptr.data_ptr(), e, edge_index.data_ptr(),
-                                         shifts.data_ptr(), flags.data_ptr(), work.data_ptr(),
-                                         nbytes, st), "zp_neighbors_fill")
+    args = (p.data_ptr(), n, float(box), float(cutoff), cap, row_ptr.data_ptr())
+    rest = (flags.data_ptr(), work.data_ptr(), nbytes)
+    _lib.run(dev, "zp_neighbors_count", *args, *rest)
+    e, fl = out[n:].tolist()
+    if fl & 1:
+        raise ValueError("neighbor_list: positions must be finite")
+    if fl & 2:
+        raise _lib.ZpError(7, "zp_neighbors_count (more neighbours per atom than an uncapped "
+                              "list can hold)")
+    edge_index = torch.empty(2, e, dtype=torch.int64, device=dev)
+    shifts = torch.empty(e, 3, dtype=torch.float64, device=dev)
+    _lib.run(dev, "zp_neighbors_fill", *args, e, edge_index.data_ptr(), shifts.data_ptr(), *rest)
     return edge_index, shifts, row_ptr
 
 
