@@ -231,7 +231,7 @@ __device__ __forceinline__ void stage_dup(const float *__restrict__ rot, float2 
 // A block owns one node, whose rows of x (or of the upstream gradient) stand in shared memory, and goes through
 // the node's edges: by edge, a thread fetches them from L2 again and again, and those fetches were between a
 // third and a half of all that L2 has to deliver, which is what bounds these kernels (60 000 edges at lmax 4 / C 128:
-// 57 KB an edge in 450 us going in, 95 KB in 920 coming back, 7.6 and 6.2 TB/s).  G lanes are a worker, which has
+// 57 KB an edge in 389 us going in, 95 KB in 810 coming back, 8.9 and 7.0 TB/s).  G lanes are a worker, which has
 // an edge to itself, each lane one vector of channels; the node's edges are dealt to the workers in turn.
 // A degree's rows of the worker's next edge are requested as soon as those of the current one have been used,
 // so that one edge is always on its way.  All copies into a worker's rows are its lanes' own, but the rotation's.
@@ -351,8 +351,8 @@ struct StageAll {
   }
 };
 // A worker's lanes request an edge's rotation.  Its entries are made into pairs where they are used, 300
-// instructions of 2400 an edge; copied into pairs, four bytes at a time, they took longer (rotate_in 354 -> 390 us at
-// lmax 4, 2.3 -> 3.8 ms for 240 000 edges at lmax 6, where their room costs blocks too).
+// instructions of 2400 an edge; copied into pairs, four bytes at a time, they took a tenth longer at lmax 4 and half
+// as long again at lmax 6, where their room costs blocks too.
 __device__ __forceinline__ void stage_rot(const float *rot, float *rot_s, int ld, int li, int G) {
   for (int i = 4 * li; i < ld; i += 4 * G) cp_async<16>(rot_s + i, rot + i);
 }
