@@ -16,14 +16,6 @@ namespace {
 thread_local char g_cuda_error[512] = "";
 thread_local int64_t g_launches = 0;
 
-// Up to this many edges the products of a step share one launch.  Beyond it each is a launch of its
-// own on the plan's streams: the fixed walk through one long list leaves CTAs idle at its end (3 % of the
-// products at lmax 4, C 128 and 60 000 edges), while the CTAs of a next launch start wherever an SM becomes
-// free; below it the set-up and the draining of each launch cost more (conv1 of 6 000 edges in bf16: 82 us
-// apart, 70 together).  What decides is tiles per SM, and the line is drawn for wide blocks.  A whole
-// training step, apart / together: lmax 4, C 128 within 2 % of each other from 12 000 to 84 000 edges, fp32
-// and bf16; lmax 2, C 128 at 24 000 / 60 000 / 84 000 edges 1.79 / 3.93 / 5.38 ms against 1.64 / 3.71 /
-// 5.16; lmax 2, C 64 1.14 / 2.10 / 2.75 against 1.04 / 1.95 / 2.57: narrow ones would gain from a higher one.
 constexpr int kChunkK = 2048;          // contraction length of one TMEM accumulation chunk
 
 // The fused epilogues (gate activation in conv1, rotation back + segmented sums in conv2) need
@@ -53,10 +45,11 @@ const float *wscale(const zp_plan *p, const ZpWorkspace &w, int conv, int m) {
 }
 
 // Independent products, in one launch or side by side (between fork and join).
-int run_products(const zp_plan *plan, ZpLanes &lanes, const ZpGemmTc *g, int n, int cls, cudaStream_t st) {
+int run_products(const zp_plan *plan, ZpLanes &lanes, const ZpGemmTc *g, int n, bool together, int cls,
+                 cudaStream_t st) {
   int rc;
   if (n == 0) return ZP_OK;
-  if (n <= ZP_GEMM_GROUP && (g[0].a_mn ? g[0].K : g[0].M) <= kTogetherEdges) {
+  if (together) {
     ZP_TIMED(cls, zp_launch_gemm_group(g, n, st));
     return ZP_OK;
   }
@@ -522,7 +515,7 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
     }
     const bool apart = E > kTogetherEdges;
     if (apart && (rc = lanes.fork())) return rc;
-    if ((rc = run_products(plan, lanes, products, plan->n_blocks, ZP_K_GEMM_FWD, st))) return rc;
+    if ((rc = run_products(plan, lanes, products, plan->n_blocks, !apart, ZP_K_GEMM_FWD, st))) return rc;
     if (apart && (rc = lanes.join())) return rc;
     // |gate(h1)| <= |h1|
     ZP_TIMED(ZP_K_GATE_FWD,
@@ -561,7 +554,7 @@ int zp_core_forward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c,
                            fuse2 ? &epi : nullptr};
     if (fuse2) ZP_TIMED(ZP_K_GEMM_FWD, zp_launch_gemm_tc(products[m], lanes.pick(m)));
   }
-  if (!fuse2 && E > 0 && (rc = run_products(plan, lanes, products, plan->n_blocks, ZP_K_GEMM_FWD, st)))
+  if (!fuse2 && E > 0 && (rc = run_products(plan, lanes, products, plan->n_blocks, !apart, ZP_K_GEMM_FWD, st)))
     return rc;
   if (apart && (rc = lanes.join())) return rc;
   if (fuse2)
@@ -748,7 +741,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                 plan->status_dev, 0, 1, plan->g_elems, 0, plan->fp16, dYm.scale,
                                 Xm.scale, nullptr, nullptr};
     }
-    const bool together = E <= kTogetherEdges && nd + nw <= ZP_GEMM_GROUP;
+    const bool together = E <= kTogetherBackward && nd + nw <= ZP_GEMM_GROUP;
     if (nw && together) zp_gemm_group_splits(products, nd + nw, nw, kZpWgradSplits);
     for (int m = 0; m < nw; ++m) {
       if (!together) wgrads[m].ksplit = zp_gemm_tc_pick_splits(wgrads[m], kZpWgradSplits);
@@ -756,7 +749,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
     }
     if ((rc = lanes.fork())) return rc;
     if (together) {
-      if ((rc = run_products(plan, lanes, products, nd + nw, ZP_K_GEMM_DGRAD, st))) return rc;
+      if ((rc = run_products(plan, lanes, products, nd + nw, true, ZP_K_GEMM_DGRAD, st))) return rc;
     } else {
       for (int m = 0; m < nd; ++m) {
         ZP_TIMED(ZP_K_GEMM_DGRAD, zp_launch_gemm_tc(products[m], lanes.pick(want_w ? 2 * m : m)));
@@ -783,7 +776,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   // that was there before it.  On the second side stream the radial layer's parameter gradients,
   // on the first the last sums of the convolutions'.
   if ((rc = lanes.fork())) return rc;
-  const bool together = E <= kTogetherEdges;
+  const bool together = E <= kTogetherBackward;
   if (rl && E > 0) {
     ZpFinalList own;
     ZpFinalList &radial_list = together && rl->later ? *rl->later : own;

@@ -317,7 +317,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                                     grads->ln_gamma[1], grads->ln_beta[1], grads->rad_b[1], ln1, list, st)))
       return rc;
     // their weight gradients on the side, where they are launches of their own
-    const bool apart = want_rad && E > kTogetherEdges;
+    const bool apart = want_rad && E > kTogetherBackward;
     if (apart && (rc = lanes.fork(2))) return rc;
     if ((rc = zp_linear_backward_planes(plan, E, ec, ec, b.hid0, b.w1, b.dz1, b.g_hid0,
                                         grads->rad_w[1], nullptr, b.part1, zp_radial_splits(ec, ec), nullptr,

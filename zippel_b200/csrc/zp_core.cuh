@@ -91,8 +91,15 @@ enum { kScX = 0, kScRad, kScH1, kScA1, kScHt, kScDy, kScDh1, kScGate, kScMaxNode
        kScRstd1, kScW0, kScW0Scale, kScW1, kScW1Scale, kScXe, kScHid0, kScDz1, kScDz0,
        kScCount };
 
-// Up to this many edges the products of a step share one launch (zp_api.cu has the reasons).
-constexpr int64_t kTogetherEdges = 24000;
+// Up to this many edges the products of a convolution share one launch, those of the forward and those of the
+// backward with the radial layers'.  Beyond it each is a launch of its own on the plan's streams: the
+// CTAs of a next launch start wherever an SM becomes free, and the tiles of one product keep to one operand in L2;
+// below it the set-up and the draining of each launch cost more.  Whole passes at lmax 4 / C 128, apart and together:
+// inference of 30 000 edges in fp32 1.70 / 1.67 ms, in bf16 0.93 / 0.91, of 60 000 3.19 / 3.20 to 3.23, of 105 000
+// 5.48 / 5.46 to 5.60; a training step of 30 000 4.98 / 4.73 and 2.61 / 2.44, of 60 000 9.56 / 9.19 and 4.85 / 4.66, of
+// 105 000 16.5 / 16.2 and 8.29 / 8.08, of 180 000 28.0 / 28.1.  lmax 2, 158 000 edges: 8.80 / 8.53; lmax 6, 60 000:
+// 19.45 / 19.3, 120 000: 39.1 / 39.7.
+constexpr int64_t kTogetherEdges = 40000, kTogetherBackward = 110000;
 
 constexpr int kZpWgradSplits = 8;
 // K splits of a radial layer's weight gradient [N, K], whose contraction runs over the edges: as many

@@ -1647,11 +1647,10 @@ void plan_launch(GroupPlan &pl, const ZpGemmTc *const *g, int n, int kernel) {
   for (int k = 0; k < n; ++k) tiles += pl.shape[k].tiles;
   const int units = pl.pair ? sms / 2 : sms;
   if (narrow || tiles >= units) return;
-  for (int cap : {192, 128, 64}) {
-    GroupPlan other;
-    plan_group(other, g, n, pl.pair, pl.bk, cap, units);
-    if (other.makespan < 0.97 * pl.makespan) pl = other;
-  }
+  const int cap = 4 * tiles <= units ? 64 : 2 * tiles <= units ? 128 : 192;
+  GroupPlan other;
+  plan_group(other, g, n, pl.pair, pl.bk, cap, units);
+  if (other.makespan < 0.97 * pl.makespan) pl = other;
 }
 
 // Describes a launch to the kernel.

@@ -87,7 +87,7 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
                               cudaStream_t side, float *dx_absmax, int64_t dx_cols) {
   int rc, n = 0;
   const int P = dy.planes, fp16 = dy.fp16;
-  const bool together = dx && dw && M <= kTogetherEdges;
+  const bool together = dx && dw && M <= kTogetherBackward;
   ZpGemmTc g[2];
   if (dx) {
     const int64_t cols = dx_cols > 0 ? dx_cols : K;
