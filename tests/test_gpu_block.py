@@ -409,6 +409,28 @@ def test_weights_of_the_edge_convolution_by_size():
             eso2.EdgeConvFunction.apply(plan, graph, *ins, w[0][:-1], *w[1:])
 
 
+@pytest.mark.parametrize("n,e", [(128, 4096), (129, 4096), (128, 4097), (3, 400), (1, 300), (2, 4096), (100, 7)])
+@pytest.mark.parametrize("order", ["any", "rising", "sorted"])
+def test_sort_by_one_block(n, e, order):
+    """At the line between the sort of one block and the general one, and buckets beyond what registers hold."""
+    import numpy as np
+
+    from zippel_b200.graph import EdgeGraph, csr_reference
+    g = torch.Generator("cpu").manual_seed(n + e)
+    ei = torch.randint(0, n, (2, e), generator=g)
+    if order == "sorted":
+        ei = ei[:, torch.argsort(ei[0], stable=True)]
+    if order != "any":
+        ei = ei[:, torch.argsort(ei[1], stable=True)]
+    want = csr_reference(ei.numpy(), n)
+    got = EdgeGraph.build(ei.cuda(), n)
+    for key in ("perm", "src", "dst", "row_ptr", "perm_src", "row_ptr_src"):
+        assert np.array_equal(getattr(got, key).cpu().numpy(), want[key]), key
+    ei[0, e // 2] = n
+    with pytest.raises(IndexError):
+        EdgeGraph.build(ei.cuda(), n)
+
+
 @pytest.mark.parametrize("lmax,mmax,c,precision", [(4, 2, 128, "fp32"), (2, 2, 16, "fp32_bf16x3"), (3, 1, 40, "fp32"),
                                                    (1, 1, 72, "fp32"), (4, 4, 160, "fp32"), (5, 2, 136, "fp32"),
                                                    (6, 2, 24, "fp32_bf16x3"), (2, 0, 256, "fp32"), (1, 0, 8, "fp32")])

@@ -8,7 +8,7 @@
 // operand planes, by the kernel that forms it (scaled from an a-priori bound instead of a scan),
 // the maxima and the planes of all weights are one launch each, and all parameter gradients share
 // one last launch.  A block of 2 000 edges is bound by its launches: 110 for an energy and its
-// forces when every piece was a call of its own, 42 here with its edge sort and head.
+// forces when every piece was a call of its own, 37 here with its edge sort and head.
 #include <cmath>
 
 #include "zp_core.cuh"

@@ -9,7 +9,7 @@
 // neighbour lists do, are in their buckets already: their first bucketing is skipped.  3 M edges of
 // 100 000 nodes take 110 us, in any other order 252 (295 for both with every edge counted and bucketed
 // twice); 2.7 M edges of 30 000 nodes, 90 each way, 121 and 367 (510).  What is left are the atomics and
-// scattered words of the source view.
+// scattered words of the source view.  Up to 4 096 edges of 128 nodes are sorted by one block.
 #include <algorithm>
 #include <mutex>
 
@@ -264,11 +264,12 @@ __global__ void rank_dst_kernel(int64_t N, int64_t E, const int64_t *__restrict_
 // One warp per source node: order the sorted-edge ids of its outgoing edges increasingly, in place:
 // up to 128 of them in registers, more with `tmp` holding the bucket as it was.
 template <int R>
-__device__ __forceinline__ void sort_src_bucket(int beg, int end, int lane, int32_t *perm_src) {
+__device__ __forceinline__ void sort_src_bucket(int beg, int end, int lane, const int32_t *bucket,
+                                                int32_t *perm_src) {
   uint32_t key[R];
 #pragma unroll
   for (int r = 0; r < R; ++r)
-    key[r] = beg + 32 * r + lane < end ? (uint32_t)perm_src[beg + 32 * r + lane] : ~0u;
+    key[r] = beg + 32 * r + lane < end ? (uint32_t)bucket[beg + 32 * r + lane] : ~0u;
   warp_sort(key, lane);
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -283,9 +284,9 @@ __global__ void rank_src_kernel(int64_t N, int64_t E, const int32_t *__restrict_
   const int lane = threadIdx.x % 32;
   if (n >= N) return;
   const int beg = row_ptr_src[n], end = row_ptr_src[n + 1];
-  if (end - beg <= 32) return sort_src_bucket<1>(beg, end, lane, perm_src);
-  if (end - beg <= 64) return sort_src_bucket<2>(beg, end, lane, perm_src);
-  if (end - beg <= 128) return sort_src_bucket<4>(beg, end, lane, perm_src);
+  if (end - beg <= 32) return sort_src_bucket<1>(beg, end, lane, perm_src, perm_src);
+  if (end - beg <= 64) return sort_src_bucket<2>(beg, end, lane, perm_src, perm_src);
+  if (end - beg <= 128) return sort_src_bucket<4>(beg, end, lane, perm_src, perm_src);
   for (int i = beg + lane; i < end; i += 32) tmp[i] = perm_src[i];
   __syncwarp();
   for (int i = beg + lane; i < end; i += 32) {
@@ -293,6 +294,141 @@ __global__ void rank_src_kernel(int64_t N, int64_t E, const int32_t *__restrict_
     int rank = 0;
     for (int j = beg; j < end; ++j) rank += tmp[j] < id;
     perm_src[beg + rank] = id;          // ids are positions 0 .. E-1 written by rank_dst_kernel
+  }
+}
+
+// The whole sort of a small graph by one block, everything between its arrays in shared memory: one launch for
+// six.  Calls of this size are the host's to bound: EdgeGraph.build of 64 to 128 nodes and 500 to 4 096 edges in the
+// order of a neighbour list 58-61 -> 44-51 us, in any other 60-72 -> 54-64; inference of 64 atoms (1 920 edges)
+// 199 -> 195, forces of 100 at lmax 4 613 -> 607.  One SM takes 17 to 22 us on the device for 6 000 to 10 000 edges, where the
+// five kernels take 13 once they are queued, and no pass of that size got faster; a thousand nodes are 31 buckets
+// for each warp, and their 4 000 edges in any order took 159 us for 65.
+constexpr int kSmallThreads = 1024, kSmallEdges = 4096, kSmallNodes = 128;
+struct SmallSort {
+  const int64_t *src, *dst, *z;
+  int n_elements;
+  int32_t *perm, *src_sorted, *dst_sorted, *row_ptr, *perm_src, *row_ptr_src, *flag;
+};
+// words of shared memory: offsets and cursors of both views, the buckets of both, the sources
+constexpr size_t small_sort_bytes(int64_t E, int64_t N) { return sizeof(int32_t) * (4 * (size_t)(N + 1) + 3 * (size_t)E); }
+
+__global__ void __launch_bounds__(kSmallThreads)
+small_sort_kernel(int E, int N, const SmallSort a) {
+  zp_after_previous();
+  extern __shared__ int32_t small_s[];
+  __shared__ int32_t sums[32], bits, falling;
+  int32_t *const row[2] = {small_s, small_s + N + 1};
+  int32_t *const cursor[2] = {row[1] + N + 1, row[1] + 2 * (N + 1)};
+  int32_t *const tmp = row[1] + 3 * (N + 1), *const out = tmp + E, *const source = out + E;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = kSmallThreads / 32;
+  if (threadIdx.x == 0) bits = falling = 0;
+  for (int i = threadIdx.x; i < 2 * (N + 1); i += kSmallThreads) cursor[0][i] = 0;
+  __syncthreads();
+  // counts, as count_kernel
+  for (int i0 = 0; i0 < E; i0 += kSmallThreads) {
+    const int i = i0 + threadIdx.x;
+    const int64_t d = i < E ? a.dst[i] : -1, s = i < E ? a.src[i] : -1;
+    const bool valid = (uint64_t)d < (uint64_t)N && (uint64_t)s < (uint64_t)N;
+    if (i < E && !valid) {
+      atomicOr(&bits, kFlagEdges);
+      if (N > 0) atomicAdd(&cursor[1][0], 1);
+    }
+    if (valid) {
+      atomicAdd(&cursor[0][d], 1);
+      atomicAdd(&cursor[1][s], 1);
+    }
+    if (i < E) source[i] = valid ? (int32_t)s : -1;
+    const int64_t before = __shfl_up_sync(0xffffffffu, d, 1);
+    if (i < E && (!valid || (lane ? before > d : i > 0 && a.dst[i - 1] > d))) falling = 1;
+  }
+  if (a.z)
+    for (int i = threadIdx.x; i < N; i += kSmallThreads)
+      if ((uint64_t)a.z[i] >= (uint64_t)a.n_elements) atomicOr(&bits, kFlagElements);
+  __syncthreads();
+  // offsets: every thread takes a stretch of the counters
+  const int per = (N + kSmallThreads - 1) / kSmallThreads;
+  for (int v = 0; v < 2; ++v) {
+    const int lo = min(N, (int)threadIdx.x * per), hi = min(N, lo + per);
+    int32_t sum = 0, total;
+    for (int i = lo; i < hi; ++i) sum += cursor[v][i];
+    int32_t run = block_exclusive_scan(sum, sums, total);
+    int32_t *const ptr = v ? a.row_ptr_src : a.row_ptr;
+    for (int i = lo; i < hi; ++i) {
+      const int32_t n = cursor[v][i];
+      ptr[i] = row[v][i] = cursor[v][i] = run;
+      run += n;
+    }
+    if (threadIdx.x == 0) ptr[N] = row[v][N] = total;      // edges counted
+  }
+  if (threadIdx.x == 0) {
+    a.flag[0] = bits;
+    a.flag[1] = falling;
+  }
+  __syncthreads();
+  const bool bucketed = falling != 0;
+  if (bucketed) {
+    for (int i = threadIdx.x; i < E; i += kSmallThreads) {
+      if (source[i] >= 0) tmp[atomicAdd(&cursor[0][a.dst[i]], 1)] = i;
+    }
+    __syncthreads();
+  }
+  // destinations, as rank_dst_kernel
+  for (int i = row[0][N] + threadIdx.x; i < E; i += kSmallThreads) {
+    a.perm[i] = a.src_sorted[i] = a.dst_sorted[i] = 0;
+    if (N > 0) out[atomicAdd(&cursor[1][0], 1)] = i;
+  }
+  for (int n = warp; n < N; n += warps) {
+    const int beg = row[0][n], end = row[0][n + 1];
+    auto load = [&](int i) -> unsigned long long {
+      const int32_t id = bucketed ? tmp[i] : i;
+      return ((unsigned long long)(uint32_t)source[id] << 32) | (uint32_t)id;
+    };
+    auto put = [&](unsigned long long key, int at) {
+      const int32_t s = (int32_t)(key >> 32);
+      a.perm[at] = (int32_t)(uint32_t)key;
+      a.src_sorted[at] = s;
+      a.dst_sorted[at] = n;
+      out[atomicAdd(&cursor[1][s], 1)] = at;
+    };
+    if (end - beg <= 64) {
+      constexpr int R = 2;
+      unsigned long long key[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) key[r] = beg + 32 * r + lane < end ? load(beg + 32 * r + lane) : ~0ull;
+      if (!bucket_rises(end - beg, lane, key)) warp_sort(key, lane);
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (beg + 32 * r + lane < end) put(key[r], beg + 32 * r + lane);
+    } else {
+      bool rising = true;
+      for (int i = beg + lane; i < end; i += 32) rising = rising && (i + 1 >= end || load(i) < load(i + 1));
+      rising = __all_sync(0xffffffffu, rising);
+      for (int i = beg + lane; i < end; i += 32) {
+        const unsigned long long key = load(i);
+        int at = i;
+        if (!rising) {
+          at = beg;
+          for (int j = beg; j < end; ++j) at += load(j) < key;
+        }
+        put(key, at);
+      }
+    }
+  }
+  __syncthreads();
+  // sources, as rank_src_kernel
+  for (int i = row[1][N] + threadIdx.x; i < E; i += kSmallThreads) a.perm_src[i] = 0;
+  for (int n = warp; n < N; n += warps) {
+    const int beg = row[1][n], end = row[1][n + 1];
+    if (end - beg <= 32) sort_src_bucket<1>(beg, end, lane, out, a.perm_src);
+    else if (end - beg <= 64) sort_src_bucket<2>(beg, end, lane, out, a.perm_src);
+    else if (end - beg <= 128) sort_src_bucket<4>(beg, end, lane, out, a.perm_src);
+    else
+      for (int i = beg + lane; i < end; i += 32) {
+        const int32_t id = out[i];
+        int rank = 0;
+        for (int j = beg; j < end; ++j) rank += out[j] < id;
+        a.perm_src[beg + rank] = id;
+      }
   }
 }
 
@@ -338,6 +474,16 @@ static int csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *p
   const CsrWork w = carve_csr(E, N, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
   const int64_t *src64 = edge_index, *dst64 = edge_index + E;
+  if (E > 0 && E <= kSmallEdges && N > 0 && N <= kSmallNodes) {
+    static ZpSmemOptIn opt_in;
+    const size_t smem = small_sort_bytes(E, N);
+    if (int rc = zp_ensure_smem(small_sort_kernel, small_sort_bytes(kSmallEdges, kSmallNodes), opt_in)) return rc;
+    zp_launch(small_sort_kernel, 1, kSmallThreads, smem, st, (int)E, (int)N,
+              SmallSort{src64, dst64, atomic_numbers, n_elements, perm, src_sorted, dst_sorted, row_ptr,
+                        perm_src, row_ptr_src, w.flag});
+    ZP_LAUNCH_CHECK("small_sort_kernel");
+    return ZP_OK;
+  }
   // one wave: on edges that need no bucketing it only looks at the flag
   const unsigned eb = (unsigned)std::min<int64_t>(zp_ceil_div(E > 0 ? E : 1, 256), 148 * 8);
   const unsigned nbw = (unsigned)zp_ceil_div((N > 0 ? N : 1) * 32, 256);
