@@ -52,6 +52,39 @@ def test_frozen_groups_leave_the_other_gradients_alone(frozen):
         assert (g is None) == (full[n] is None) and (g is None or rel_l2(g, full[n]) < 1e-6), n
 
 
+@pytest.mark.parametrize("precision,tol", [("fp32", 1.5e-5), ("fp32_bf16x3", 1.5e-5), ("bf16", 1e-4)])
+@pytest.mark.parametrize("edges", [6000, 60000, 120000])
+def test_every_choice_of_wanted_gradients(edges, precision, tol):
+    """With side streams (from 4 096 edges on) and on both sides of the line up to which products share a launch,
+    every choice of what wants a gradient forks and joins another way; each gradient is that of the call in which
+    all are wanted, but for other splits of the sums over the edges: an accumulator adds 2 048 of them in 128 steps,
+    each off by up to 2^-23 of the sum, 1.5e-5 at most.  (In bf16 such a difference may turn the rounding of an
+    operand: 2^-9 of one value in a thousand.)"""
+    cfg = dict(lmax=1, mmax=1, sphere_channels=16, hidden_channels=16, edge_channels=64,
+               num_distance_basis=16, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1), precision=precision)
+    case = {k: v.cuda().float() if v.is_floating_point() else v.cuda()
+            for k, v in random_case(cfg, edges // 20, edges, seed=2).items()}
+    groups = {"emb": ("elem_emb",), "rad": ("rad_func",), "so2": ("c1_", "c2_")}
+
+    def grads(wanted):
+        pos, x = (case[k].clone().requires_grad_(w in wanted) for k, w in (("pos", "pos"), ("x_node", "x")))
+        for n, p in block.named_parameters():
+            p.requires_grad_(any(n.startswith(groups[w]) for w in wanted if w in groups))
+        wrt = {"pos": pos, "x": x, **dict(block.named_parameters())}
+        wrt = {n: t for n, t in wrt.items() if t.requires_grad}
+        out = block.node_output(pos, case["atomic_numbers"], x, case["edge_index"], case["shifts"],
+                                case["cos_gamma_k"], case["sin_gamma_k"])
+        return dict(zip(wrt, torch.autograd.grad(out, list(wrt.values()), case["upstream"])))
+
+    everything = ("pos", "x", "emb", "rad", "so2")
+    full = grads(everything)
+    for choice in range(1, 31):
+        wanted = [w for i, w in enumerate(everything) if choice >> i & 1]
+        for n, g in grads(wanted).items():
+            assert rel_l2(g, full[n]) < tol, (wanted, n)
+
+
 @pytest.mark.parametrize("n,degree", [(3, 31), (3, 33), (2, 64), (2, 65), (16385, 2), (40000, 3)])
 def test_sort_at_its_bucket_and_scan_edges(n, degree):
     import numpy as np

@@ -316,12 +316,14 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
                                                   sc + kScDz1),
                                     grads->ln_gamma[1], grads->ln_beta[1], grads->rad_b[1], ln1, list, st)))
       return rc;
-    // their weight gradients on the side, where they are launches of their own
+    // their weight gradients on the side stream, if at all behind a fork after what they read: up to that line on
+    // the caller's, in the input gradient's launch or (nobody wants the input's) one of their own
     const bool apart = want_rad && E > kTogetherBackward;
+    const cudaStream_t side = apart ? lanes.pick(2) : st;
     if (apart && (rc = lanes.fork(2))) return rc;
     if ((rc = zp_linear_backward_planes(plan, E, ec, ec, b.hid0, b.w1, b.dz1, b.g_hid0,
                                         grads->rad_w[1], nullptr, b.part1, zp_radial_splits(ec, ec), nullptr,
-                                        list, st, lanes.pick(2), fm.f0.fp16 ? sc + kScGHid0 : nullptr)))
+                                        list, st, side, fm.f0.fp16 ? sc + kScGHid0 : nullptr)))
       return rc;
     if ((rc = zp_launch_ln_silu_bwd(E, ec, b.h0, params->ln_gamma[0], params->ln_beta[0], mean0, rstd0,
                                     b.g_hid0, nullptr, &b.dz0,
@@ -335,7 +337,7 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
     if (apart && (rc = lanes.fork(2))) return rc;
     if ((rc = zp_linear_backward_planes(plan, E, w0, ec, b.xe, b.w0, b.dz0, want_in ? b.g_xe : nullptr,
                                         grads->rad_w[0], nullptr, b.part0, zp_radial_splits(ec, w0), nullptr,
-                                        list, st, lanes.pick(2), nullptr, cols)))
+                                        list, st, side, nullptr, cols)))
       return rc;
     if (!apart && (rc = lanes.join(2))) return rc;         // the rotation's part of the edge vectors' gradient
     if (want_in &&
