@@ -10,6 +10,7 @@ import torch
 from oracle import eso2_oracle as orc
 from tests.helpers import (check_against, gpu_node_out_and_vjp, make_block, oracle_node_out_and_vjp,
                            random_case, rel_l2)
+from zippel_b200.graph import EdgeGraph
 
 pytestmark = pytest.mark.gpu
 
@@ -97,6 +98,40 @@ def test_sort_at_its_bucket_and_scan_edges(n, degree):
     check()
     for key, val in want.items():
         assert np.array_equal(getattr(got, key).cpu().numpy(), val), key
+
+
+def test_left_out_slots_are_edges_into_no_node():
+    """A slot that an unvalidated sort has left out reads as an edge 0 -> 0 that counts for source 0 alone: an edge
+    from a node at the same place with the same embedding.  (Sums in another order: 1e-5.)"""
+    cfg = dict(lmax=3, mmax=2, sphere_channels=16, hidden_channels=16, edge_channels=16,
+               num_distance_basis=8, cutoff=5.0)
+    block = make_block(cfg, orc.init_params(cfg, seed=1))
+    n, e = 12, 90
+    case = {k: v.cuda().float() if v.is_floating_point() else v.cuda()
+            for k, v in random_case(cfg, n + 1, e, seed=2).items()}
+    case["edge_index"] %= n
+    for k in ("pos", "x_node", "atomic_numbers"):
+        case[k][n] = case[k][0]
+    case["shifts"][0] = 0.5                    # the slots take those of edge 0
+    bad = torch.tensor([7, 31, 32, 60], device="cuda")
+
+    def grad_x(nodes, edge_index, edges):
+        x = case["x_node"][:nodes].clone().requires_grad_(True)
+        graph = EdgeGraph.build(edge_index, nodes, validate=False)
+        out = block.node_output(case["pos"][:nodes], case["atomic_numbers"][:nodes], x, edge_index,
+                                *[case[k][edges] for k in ("shifts", "cos_gamma_k", "sin_gamma_k")], graph=graph)
+        return torch.autograd.grad(out, x, case["upstream"][:nodes])[0]
+
+    broken = case["edge_index"].clone()
+    broken[1, bad] = n + 5
+    every = torch.arange(e, device="cuda")
+    valid = every[~torch.isin(every, bad)]
+    alone = grad_x(n, case["edge_index"][:, valid], valid)
+    twin = grad_x(n + 1, torch.cat([case["edge_index"][:, valid], torch.tensor([[n], [0]], device="cuda").repeat(1, len(bad))], 1),
+                  torch.cat([valid, torch.zeros_like(bad)]))
+    want = alone.clone()
+    want[0] += twin[n]
+    assert rel_l2(grad_x(n, broken, every), want) < 1e-5
 
 
 @pytest.mark.parametrize("what", ["edge", "element"])

@@ -156,7 +156,6 @@ node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, 
   zp_after_previous();
   constexpr int K = (LMAX + 1) * (LMAX + 1);
   extern __shared__ __align__(16) float node_s[];
-  const int64_t n = blockIdx.x;
   const int workers = blockDim.x / G, w = threadIdx.x / G, li = threadIdx.x % G, ls = 4 * G;
   const int c0 = blockIdx.y * quads * 4, mine = min(quads, (t.C - c0) / 4);
   const bool active = li < mine;
@@ -165,9 +164,9 @@ node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, 
   float *rot_s = stage + (size_t)workers * t.rad_rows * ls + (size_t)w * 2 * t.rot_ld;
   const float inv = zp_publish_scale(a1, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
-  const NodeEdges edges(n, N, E, row_ptr, perm_src, row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges edges(N, E, row_ptr, perm_src, row_ptr_src, blockIdx.z, gridDim.z);
   if (edges.first == edges.last) return;
-  auto column = [&](int i) { return (i < edges.into ? t.C : 0) + c; };
+  auto column = [&](int i) { return (i < edges.own ? t.C : 0) + c; };
   auto gains = [&](int e, int i) { return radial + (size_t)(e < 0 ? 0 : e) * t.R + column(i); };
   auto rotation = [&](int64_t e, int buffer) {
     stage_rot(rot + (size_t)e * t.rot_ld, rot_s + buffer * t.rot_ld, t.rot_ld, li, G);
@@ -176,7 +175,7 @@ node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, 
   int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, F4, false, true>::run(t, nullptr, 0, gains(e, i0), nullptr, rad_s, ls, e >= 0 && active);
-  stage_node<F4>(x + (size_t)n * t.K * t.C + c0, t.C, K, mine, x_s, ls);
+  stage_node<F4>(x + (size_t)edges.row(N) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -389,7 +388,7 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
   if (view.perm_src && 10 * ns.quads >= 7 * ns.G) {
     const int64_t N = view.nodes;
     const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t, t.rad_rows, 16, 4);
-    const dim3 grid((unsigned)N, (unsigned)ns.groups, (unsigned)nl.parts);
+    const dim3 grid((unsigned)(N + 1), (unsigned)ns.groups, (unsigned)nl.parts);
 #define CALL_FMT(LM, FMT)                                                                         \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \

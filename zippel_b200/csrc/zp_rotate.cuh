@@ -282,34 +282,33 @@ inline NodeLaunch zp_node_launch(int64_t blocks, double items, const NodeShape &
   return best;
 }
 
-// The node's edges, numbered: those into it, then (with a source view) those out of it.  Slots that the sort has
-// left out (edges of indices out of range) stand behind all others and count as edges into node 0.
+// The node's edges, numbered: those into it, then (with a source view) those out of it.  Block N of a launch
+// has the slots that the sort has left out (edges of indices out of range): they stand behind all others and read
+// as edges 0 -> 0, but are edges into no node.
 struct NodeEdges {
-  int beg, own, into, sbeg, total, rest;
+  int n, beg, own, sbeg, total;          // node; first and number of the edges into it; first edge out; of both
   const int32_t *perm_src;
   int first, last;                       // this block's stretch of them
-  __device__ __forceinline__ NodeEdges(int64_t n, int64_t N, int64_t E, const int32_t *row_ptr, const int32_t *view,
+  __device__ __forceinline__ NodeEdges(int64_t N, int64_t E, const int32_t *row_ptr, const int32_t *view,
                                        const int32_t *row_ptr_src, int part, int parts) {
+    n = blockIdx.x;
     beg = row_ptr[n];
-    own = into = row_ptr[n + 1] - beg;
-    rest = sbeg = 0;
-    if (n == 0) {
-      rest = row_ptr[N];
-      into += (int)E - rest;
-    }
-    total = into;
+    total = own = (n < N ? row_ptr[n + 1] : (int)E) - beg;
+    sbeg = 0;
     perm_src = view;
-    if (view) {
+    if (view && n < N) {
       sbeg = row_ptr_src[n];
       total += row_ptr_src[n + 1] - sbeg;
     }
     first = (int)((int64_t)total * part / parts);
     last = (int)((int64_t)total * (part + 1) / parts);
   }
+  __device__ __forceinline__ bool left_out(int64_t N) const { return n == N; }
+  __device__ __forceinline__ int64_t row(int64_t N) const { return n < N ? n : 0; }
   // -1: past this block's
   __device__ __forceinline__ int edge(int i) const {
     if (i >= last) return -1;
-    return i < own ? beg + i : i < into ? rest + i - own : perm_src[sbeg + i - into];
+    return i < own ? beg + i : perm_src[sbeg + i - own];
   }
 };
 

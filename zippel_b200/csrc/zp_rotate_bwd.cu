@@ -235,7 +235,6 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64
   zp_after_previous();
   constexpr int K = (LMAX + 1) * (LMAX + 1);
   extern __shared__ __align__(16) float node_s[];
-  const int64_t n = blockIdx.x;
   const int workers = blockDim.x / G, w = threadIdx.x / G, li = threadIdx.x % G, ls = 4 * G;
   const bool active = li < quads;
   const int c = 4 * li;
@@ -243,7 +242,7 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64
   float *rot_s = stage + (size_t)workers * t.Km * ls + (size_t)w * 2 * t.rot_ld;
   const float inv = zp_publish_scale(dy, scale, blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
-  const NodeEdges edges(n, N, E, row_ptr, nullptr, nullptr, blockIdx.z, gridDim.z);
+  const NodeEdges edges(N, E, row_ptr, nullptr, nullptr, blockIdx.z, gridDim.z);
   if (edges.first == edges.last) return;
   auto rows = [&](int e) { return y + (size_t)(e < 0 ? 0 : e) * t.Km * t.C + c; };
   auto rotation = [&](int64_t e, int buffer) {
@@ -253,7 +252,7 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64
   int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, F4, true, false>::run(t, rows(e), t.C, nullptr, y_s, nullptr, ls, e >= 0 && active);
-  stage_node<F4>(g_out + (size_t)n * t.K * t.C, t.C, K, quads, g_s, ls);
+  stage_node<F4>(g_out + (size_t)edges.row(N) * t.K * t.C, t.C, K, quads, g_s, ls);
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -393,7 +392,6 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   using V = NodeVec<LMAX>;
   constexpr int K = (LMAX + 1) * (LMAX + 1), VN = VecOf<V>::n;
   extern __shared__ __align__(16) float node_s[];
-  const int64_t n = blockIdx.x;
   const int workers = blockDim.x / G, w = threadIdx.x / G, li = threadIdx.x % G;
   const int ls = G * VN;                                    // floats between two rows
   const int rows = SUMS ? max(t.Km + t.rad_rows, K) : t.Km + t.rad_rows;
@@ -403,8 +401,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   float *x_s = node_s, *stage = node_s + (size_t)K * ls, *da_s = stage + (size_t)w * rows * ls + li * VN;
   float *rad_s = da_s + t.Km * ls;
   float *rot_s = stage + (size_t)workers * rows * ls + (size_t)w * 2 * t.rot_ld;
-  const float *xn = a.x + (size_t)n * t.K * t.C + c0;
-  const NodeEdges edges(n, N, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges edges(N, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
   float inv = 1.f;
   if constexpr (FMT == kFmtFp16x2)
     inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
@@ -416,7 +413,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   if (!SUMS && edges.first == edges.last) return;
 
   auto at = [&](int64_t e, int i) {
-    const int col = (i < edges.into ? t.C : 0) + c;
+    const int col = (i < edges.own ? t.C : 0) + c;
     EdgeAt<T_> p;
     p.da = a.da1 + (size_t)e * t.Km * 2 * t.C + col;
     p.rad = a.radial + (size_t)e * t.R + col;
@@ -432,7 +429,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   EdgeAt<T_> cur = at(e < 0 ? 0 : e, i0);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, V, true, true>::run(t, cur.da, 2 * t.C, cur.rad, da_s, rad_s, ls, e >= 0 && active);
-  if (edges.total > 0) stage_node<V>(xn, t.C, K, mine, x_s, ls);
+  if (edges.total > 0) stage_node<V>(a.x + (size_t)edges.row(N) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -451,19 +448,19 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
       t2 += __shfl_xor_sync(0xffffffffu, t2, o);
     }
     if (li == 0 && e >= 0)
-      a.torque[(size_t)(1 + 2 * blockIdx.y + (i < edges.into ? 1 : 0)) * E + e] = make_float4(t0, t1, t2, 0.f);
+      a.torque[(size_t)(1 + 2 * blockIdx.y + (i < edges.own ? 1 : 0)) * E + e] = make_float4(t0, t1, t2, 0.f);
     e = e_next;
     e_next = e_after;
     cur = next;
   }
   cp_async_wait<0>();
-  if constexpr (!SUMS) return;
+  if (!SUMS || edges.left_out(N)) return;
   __syncthreads();                       // all are done with their rows: the sums take their place
   float *sums = stage + (size_t)w * rows * ls + li * VN;
 #pragma unroll
   for (int k = 0; k < K; ++k) store_vec<V>(sums + k * ls, acc[SUMS ? k : 0]);
   __syncthreads();
-  float *gx = a.grad_x + (size_t)n * t.K * t.C + c0;
+  float *gx = a.grad_x + (size_t)edges.n * t.K * t.C + c0;
   for (int i = threadIdx.x; i < K * mine * VN; i += blockDim.x) {
     const int k = i / (mine * VN), q = i - k * mine * VN;
     float s = 0.f;
@@ -487,7 +484,7 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const floa
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(node_rotate_grad_out_kernel<LM, FMT>, nl.smem, opt_in)) return rc_; \
-    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3((unsigned)N, 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, \
+    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3((unsigned)(N + 1), 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, \
               g, y, env, rot, row_ptr, dy, scale, grad_env, reinterpret_cast<float4 *>(torque));  \
     break;                                                                                        \
   }
@@ -549,7 +546,7 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float 
                                        sums ? std::max(rows, t.K) : rows, sums && t.lmax > 2 ? 8 : 16, sums ? 1 : 4);
   const NodeArgs a{da1, radial, x, rot, row_ptr, perm_src, row_ptr_src, grad_radial, grad_x,
                    reinterpret_cast<float4 *>(torque)};
-  const dim3 grid((unsigned)N, (unsigned)ns.groups, (unsigned)nl.parts);
+  const dim3 grid((unsigned)(N + 1), (unsigned)ns.groups, (unsigned)nl.parts);
 #define CALL_S(LM, FMT, S)                                                                        \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
