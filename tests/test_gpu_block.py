@@ -161,6 +161,28 @@ def test_rotations_over_degrees_orders_and_widths(lmax, mmax, c, h, jd64):
     check_against(*gpu_node_out_and_vjp(make_block(cfg, params), case, case["upstream"]), *want)
 
 
+@pytest.mark.parametrize("lmax,mmax,c,precision", [(2, 2, 16, "fp32"), (3, 1, 24, "fp32_bf16x3"), (4, 2, 136, "fp32"),
+                                                   (5, 2, 72, "fp32")])
+def test_nodes_of_many_edges_are_cut(lmax, mmax, c, precision, jd64):
+    """A node with most of the edges, each way, among nodes of two: its edges are several blocks', whose sums are
+    added at the end."""
+    cfg = dict(lmax=lmax, mmax=mmax, sphere_channels=c, hidden_channels=8, edge_channels=8,
+               num_distance_basis=6, cutoff=5.0)
+    params = orc.init_params(cfg, seed=lmax)
+    n, e = 300, 2100
+    case = random_case(cfg, n, e, seed=mmax)
+    hub = 211
+    case["edge_index"][0, 600:1300] = hub
+    case["edge_index"][1, 1300:] = hub
+    case["shifts"] += 0.25                     # no edge of a node with itself has length zero
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    block = make_block(cfg, params, precision=precision)
+    got = gpu_node_out_and_vjp(block, case, case["upstream"])
+    check_against(*got, *want)
+    again = gpu_node_out_and_vjp(block, case, case["upstream"])
+    assert torch.equal(got[1], again[1])       # added in one order whoever comes last
+
+
 def test_edges_along_the_polar_axis(jd64):
     """An edge whose direction is the polar axis has no proper rotation; its gradient follows the
     construction of the matrices (clamped, large) and must not disturb the other edges."""

@@ -85,7 +85,9 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
   ZpCarver c(base);
   const size_t e = (size_t)E;
   const bool lean = mode == 2 && can_fuse(p, 0) && can_fuse(p, 1);
-  w.scales = c.floats(kScCount);
+  w.arrived_words = (size_t)kZpNodeCuts * zp_node_groups(t);
+  w.scales = c.floats(kScCount + w.arrived_words);
+  w.arrived = reinterpret_cast<int *>(w.scales + kScCount);
   w.rot = c.floats(e * t.rot_ld);
   w.a1 = c.planes(E, (int64_t)t.Km * 2 * t.C, f, w.scales + kScA1);
   w.ld_h1 = lean ? t.n_gate : t.w1_cols;
@@ -114,6 +116,7 @@ ZpWorkspace zp_carve(const zp_plan *p, int64_t N, int64_t E, int mode, void *bas
     w.dh1 = c.planes(E, t.w1_cols, f, w.scales + kScDh1);
     w.da1 = c.floats(e * t.Km * 2 * t.C);
     w.torque = c.floats(e * 4 * (size_t)zp_torque_slots(t));
+    w.cuts = c.floats((size_t)zp_node_cuts_most(E) * t.K * t.C);
     w.rot_grad = t.Km * t.H >= t.nnz_pad ? w.dht : c.floats(e * t.nnz_pad);
     w.wgrad = c.floats((size_t)kZpWgradSplits * p->g_elems);
     auto column_parts = [&](int64_t cols) { return c.floats((size_t)(zp_colsum_parts(E, cols) * cols)); };
@@ -678,7 +681,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   const float *radial = rl ? ws.radial : c.radial;      // rl: left there by the forward
 
   const bool scaled_gr = rl && ws.gr.fp16;               // the planes of grad_radial have a scale
-  ZP_CUDA(cudaMemsetAsync(ws.scales + kScBwd, 0, sizeof(float) * (kScBwdEnd - kScBwd), st));
+  ZP_CUDA(cudaMemsetAsync(ws.scales + kScBwd, 0, sizeof(float) * (kScCount - kScBwd + ws.arrived_words), st));
   if (plan->fp16 && E > 0) {
     // only rows dst[0] .. dst[E-1] (the edges are destination-sorted): the rows the kernels read,
     // and the only ones a caller that holds a node range's rows alone has
@@ -768,7 +771,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
   ZP_TIMED(ZP_K_ROTATE_IN_BWD,
            zp_launch_rotate_in_bwd(plan, N, E, ws.da1, radial, c.x_node, c.row_ptr, c.perm_src,
                                    c.row_ptr_src, ws.rot, rl ? nullptr : grad_radial, grad_x_node, ws.torque,
-                                   st, rl ? &ws.gr : nullptr,
+                                   ws.cuts, ws.arrived, st, rl ? &ws.gr : nullptr,
                                    zp_scale_of(7.4f, ws.scales + kScDa1, ws.scales + kScGrScale,
                                                ws.scales + kScX)));
   // What is left are short kernels, most of them waiting on one another.  On the caller's stream

@@ -268,9 +268,15 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const floa
 int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float *da1, const float *radial,
                             const float *x, const int32_t *row_ptr, const int32_t *perm_src,
                             const int32_t *row_ptr_src, const float *rot, float *grad_radial, float *grad_x,
-                            float *torque, cudaStream_t st,
+                            float *torque, float *cuts, int *arrived, cudaStream_t st,
                             const ZpPlanes *grad_radial_planes, const ZpScale &scale);
 int zp_torque_slots(const ZpTables &t);
+// Nodes of many edges are cut into stretches (zp_rotate.cuh), at this many places at most.  A cut's part of the
+// gradient of x_node stands in `cuts` [kZpNodeCuts][K][C] until the last stretch of its node to get done adds them up:
+// `arrived`, zero before the launch, counts them, kZpNodeCuts words for each group of channels.
+constexpr int kZpNodeCuts = 296;
+int64_t zp_node_cuts_most(int64_t E);              // no more than this many of E edges
+int zp_node_groups(const ZpTables &t);
 // node_out[n, l^2 + j, c] = sum over the m' rows r of degree l, in table order, of
 //   head[n][rot_off[r] + j][c] + the continuation partials of the 32-edge blocks n's edges reach
 int zp_launch_node_sum(const zp_plan *p, int64_t N, const float *head, const float *cont,

@@ -75,20 +75,20 @@ struct ZpCarver {
 
 // Device-side scale array (fp16 planes): raw maxima, derived scales, and per weight block
 // {max |W|, scale} from kScWeights on.  One memset at the start of a forward clears it; a backward
-// clears the maxima it accumulates itself, kScBwd .. kScBwdEnd.
+// clears the words from kScBwd on itself.
 enum { kScX = 0, kScRad, kScH1, kScA1, kScHt, kScDy, kScDh1, kScGate, kScMaxNode /* an int */,
        // the radial layer run inside the call: {max, scale} of its input and of its weight, scale
        // of the planes of grad_radial
        kScHr, kScHrScale, kScRw, kScRwScale, kScGrScale,
-       // maxima a backward accumulates: upstream gradient, conv2's and conv1's input gradient,
-       // gradients of the radial MLP's two hidden activations
-       kScBwd, kScG = kScBwd, kScDht, kScDa1, kScGHid1, kScGHid0, kScBwdEnd,
        kScWeights = 24,
        // the rest of the radial MLP (whole-block calls): maxima of the embedding table, of the
        // LayerNorm parameters and of 1/std, {max, scale} of the two weights, scales of activations
        // and gradients
        kScEmb = kScWeights + 4 * (ZP_MAX_L + 1), kScGamma0, kScBeta0, kScGamma1, kScBeta1, kScRstd0,
        kScRstd1, kScW0, kScW0Scale, kScW1, kScW1Scale, kScXe, kScHid0, kScDz1, kScDz0,
+       // what a backward clears at its start: maxima it accumulates (upstream gradient, conv2's and conv1's
+       // input gradient, gradients of the radial MLP's two hidden activations); its counters follow
+       kScBwd, kScG = kScBwd, kScDht, kScDa1, kScGHid1, kScGHid0,
        kScCount };
 
 // Up to this many edges the products of a convolution share one launch, those of the forward and those of the
@@ -111,11 +111,13 @@ inline int zp_radial_splits(int64_t N, int64_t K) {
 }
 
 //   forward:  rot | a1 planes | h1 | ht planes | y | folded weight planes | head, cont partials
-//   backward: dy planes | dht | dh1 planes | da1 | torque | wgrad partials | scratch
+//   backward: dy planes | dht | dh1 planes | da1 | torque | cut nodes' sums | wgrad partials | scratch
 // mode 0 / 1: forward that keeps what a backward reads (1: plus the backward's own regions);
 // mode 2: forward alone with fused epilogues -- of h1 only the gate scalars exist, y does not.
 struct ZpWorkspace {
-  float *rot, *h1, *y, *dht, *da1, *torque, *wgrad, *scales, *head, *cont;
+  float *rot, *h1, *y, *dht, *da1, *torque, *cuts, *wgrad, *scales, *head, *cont;
+  int *arrived;                          // behind the scales
+  size_t arrived_words;
   float *rot_grad;                       // [E, nnz_pad], in dht's place where it fits: that is read by then
   float *col1, *col2, *col_rad;          // partial column sums: bias gradients of conv1, conv2, radial
   float *radial, *rad_partials;          // radial layer inside the call: its output, dW partials

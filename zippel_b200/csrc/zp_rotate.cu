@@ -148,7 +148,7 @@ struct RotInN {
 // shared memory: x [K][G] vectors | per worker: radial gains [rad_rows][G] | per worker: two rotations [rot_ld]
 template <int LMAX, int FMT>
 __global__ void __launch_bounds__(32 * kNodeMaxWarps, 2)
-node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, int G, int quads,
+node_rotate_in_kernel(const __grid_constant__ ZpTables t, const NodeCut cut, int64_t E, int G, int quads,
                       const float *__restrict__ x, const int32_t *__restrict__ row_ptr,
                       const int32_t *__restrict__ perm_src, const int32_t *__restrict__ row_ptr_src,
                       const float *__restrict__ rot, const float *__restrict__ radial, const ZpPlanes a1,
@@ -164,7 +164,7 @@ node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, 
   float *rot_s = stage + (size_t)workers * t.rad_rows * ls + (size_t)w * 2 * t.rot_ld;
   const float inv = zp_publish_scale(a1, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
-  const NodeEdges edges(N, E, row_ptr, perm_src, row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges edges(blockIdx.x, cut, E, row_ptr, perm_src, row_ptr_src, blockIdx.z, gridDim.z);
   if (edges.first == edges.last) return;
   auto column = [&](int i) { return (i < edges.own ? t.C : 0) + c; };
   auto gains = [&](int e, int i) { return radial + (size_t)(e < 0 ? 0 : e) * t.R + column(i); };
@@ -175,7 +175,7 @@ node_rotate_in_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, 
   int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, F4, false, true>::run(t, nullptr, 0, gains(e, i0), nullptr, rad_s, ls, e >= 0 && active);
-  stage_node<F4>(x + (size_t)edges.row(N) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
+  stage_node<F4>(x + (size_t)edges.row(cut) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -388,12 +388,13 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
   if (view.perm_src && 10 * ns.quads >= 7 * ns.G) {
     const int64_t N = view.nodes;
     const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t, t.rad_rows, 16, 4);
-    const dim3 grid((unsigned)(N + 1), (unsigned)ns.groups, (unsigned)nl.parts);
+    const NodeCut cut = zp_node_cut(N, E, true, nl.parts);
+    const dim3 grid(cut.blocks(), (unsigned)ns.groups, (unsigned)nl.parts);
 #define CALL_FMT(LM, FMT)                                                                         \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(node_rotate_in_kernel<LM, FMT>, nl.smem, opt_in)) return rc_;    \
-    zp_launch(node_rotate_in_kernel<LM, FMT>, grid, 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, x, \
+    zp_launch(node_rotate_in_kernel<LM, FMT>, grid, 32 * nl.warps, nl.smem, st, t, cut, E, ns.G, ns.quads, x, \
               view.row_ptr, view.perm_src, view.row_ptr_src, rot, radial, a1, scale);             \
     break;                                                                                        \
   }

@@ -227,7 +227,7 @@ struct GradOutN {
 // shared memory: g [K][G] vectors | per worker: rows of y [Km][G] | per worker: two rotations [rot_ld]
 template <int LMAX, int FMT>
 __global__ void __launch_bounds__(32 * kNodeMaxWarps, 2)
-node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, int G, int quads,
+node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, const NodeCut cut, int64_t E, int G, int quads,
                             const float *__restrict__ g_out, const float *__restrict__ y,
                             const float *__restrict__ env, const float *__restrict__ rot,
                             const int32_t *__restrict__ row_ptr, const ZpPlanes dy, const ZpScale scale,
@@ -242,7 +242,7 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64
   float *rot_s = stage + (size_t)workers * t.Km * ls + (size_t)w * 2 * t.rot_ld;
   const float inv = zp_publish_scale(dy, scale, blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
-  const NodeEdges edges(N, E, row_ptr, nullptr, nullptr, blockIdx.z, gridDim.z);
+  const NodeEdges edges(blockIdx.x, cut, E, row_ptr, nullptr, nullptr, blockIdx.z, gridDim.z);
   if (edges.first == edges.last) return;
   auto rows = [&](int e) { return y + (size_t)(e < 0 ? 0 : e) * t.Km * t.C + c; };
   auto rotation = [&](int64_t e, int buffer) {
@@ -252,7 +252,7 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t N, int64
   int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, F4, true, false>::run(t, rows(e), t.C, nullptr, y_s, nullptr, ls, e >= 0 && active);
-  stage_node<F4>(g_out + (size_t)edges.row(N) * t.K * t.C, t.C, K, quads, g_s, ls);
+  stage_node<F4>(g_out + (size_t)edges.row(cut) * t.K * t.C, t.C, K, quads, g_s, ls);
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -375,6 +375,8 @@ struct NodeArgs {
   const int32_t *row_ptr, *perm_src, *row_ptr_src;
   float *grad_radial, *grad_x;
   float4 *torque;                        // [slots][E]; slot 1 + 2 group + half is written here
+  float *cuts;                           // [cut][K][C]: sums of what follows a cut
+  int *arrived;
 };
 constexpr int kNodeQuadMaxL = 4;         // four channels a lane up to here
 template <bool PAIR> struct NodeVecOf { using type = F4; };
@@ -385,7 +387,7 @@ inline NodeShape node_shape(const ZpTables &t) { return zp_node_shape(t.C, t.lma
 // per worker: two rotations [rot_ld]
 template <int LMAX, int FMT, bool SUMS>
 __global__ void __launch_bounds__(32 * kNodeMaxWarps, (SUMS && LMAX > 2 ? 1 : 2))
-node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t E, int G, int quads, const NodeArgs a,
+node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, const NodeCut cut, int64_t E, int G, int quads, const NodeArgs a,
                           const ZpPlanes grad_radial_planes, const ZpScale scale) {
   zp_after_previous();
   using T_ = typename Elem<FMT>::type;
@@ -401,7 +403,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   float *x_s = node_s, *stage = node_s + (size_t)K * ls, *da_s = stage + (size_t)w * rows * ls + li * VN;
   float *rad_s = da_s + t.Km * ls;
   float *rot_s = stage + (size_t)workers * rows * ls + (size_t)w * 2 * t.rot_ld;
-  const NodeEdges edges(N, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges edges(blockIdx.x, cut, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
   float inv = 1.f;
   if constexpr (FMT == kFmtFp16x2)
     inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
@@ -410,7 +412,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   V acc[SUMS ? K : 1];
 #pragma unroll
   for (int k = 0; k < (SUMS ? K : 1); ++k) acc[k] = zero_vec<V>();
-  if (!SUMS && edges.first == edges.last) return;
+  if (edges.first == edges.last && (!SUMS || blockIdx.x >= cut.nodes)) return;
 
   auto at = [&](int64_t e, int i) {
     const int col = (i < edges.own ? t.C : 0) + c;
@@ -429,7 +431,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
   EdgeAt<T_> cur = at(e < 0 ? 0 : e, i0);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, V, true, true>::run(t, cur.da, 2 * t.C, cur.rad, da_s, rad_s, ls, e >= 0 && active);
-  if (edges.total > 0) stage_node<V>(a.x + (size_t)edges.row(N) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
+  if (edges.total > 0) stage_node<V>(a.x + (size_t)edges.row(cut) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -454,18 +456,37 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, int64_t N, int64_t
     cur = next;
   }
   cp_async_wait<0>();
-  if (!SUMS || edges.left_out(N)) return;
+  if (!SUMS || edges.n == cut.nodes) return;
   __syncthreads();                       // all are done with their rows: the sums take their place
   float *sums = stage + (size_t)w * rows * ls + li * VN;
 #pragma unroll
   for (int k = 0; k < K; ++k) store_vec<V>(sums + k * ls, acc[SUMS ? k : 0]);
   __syncthreads();
-  float *gx = a.grad_x + (size_t)edges.n * t.K * t.C + c0;
+  const bool tail = blockIdx.x > cut.nodes;                 // what follows a cut
+  float *const gx = a.grad_x + (size_t)edges.n * t.K * t.C + c0;
+  float *const to = tail ? a.cuts + (size_t)(blockIdx.x - cut.nodes - 1) * t.K * t.C + c0 : gx;
   for (int i = threadIdx.x; i < K * mine * VN; i += blockDim.x) {
     const int k = i / (mine * VN), q = i - k * mine * VN;
     float s = 0.f;
     for (int v = 0; v < workers; ++v) s += stage[((size_t)v * rows + k) * ls + q];
-    gx[(size_t)k * t.C + q] = s;
+    to[(size_t)k * t.C + q] = s;
+  }
+  if (edges.cut0 > edges.cut1) return;
+  // a cut node: whoever gets done last adds up, in the order of the stretches
+  __shared__ int all_here;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0)
+    all_here = atomicAdd(a.arrived + blockIdx.y * kZpNodeCuts + edges.cut0, 1) == (int)(edges.cut1 - edges.cut0) + 1;
+  __syncthreads();
+  if (!all_here) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < K * mine * VN; i += blockDim.x) {
+    const int k = i / (mine * VN), q = i - k * mine * VN;
+    const size_t at = (size_t)k * t.C + q;
+    float s = __ldcg(gx + at);
+    for (uint32_t c1 = edges.cut0; c1 <= edges.cut1; ++c1) s += __ldcg(a.cuts + (size_t)(c1 - 1) * t.K * t.C + c0 + at);
+    gx[at] = s;
   }
 }
 
@@ -480,11 +501,12 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const floa
   const NodeShape ns = zp_node_shape(t.C, 4);
   if (ns.groups == 1) {                  // the sums over an edge's channels are one worker's
     const NodeLaunch nl = zp_node_launch(N, (double)E / (double)N, ns, t, t.Km, 16, 4);
+    const NodeCut cut = zp_node_cut(N, E, false, nl.parts);
 #define CALL_FMT(LM, FMT)                                                                         \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(node_rotate_grad_out_kernel<LM, FMT>, nl.smem, opt_in)) return rc_; \
-    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3((unsigned)(N + 1), 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, \
+    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3(cut.blocks(), 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, cut, E, ns.G, ns.quads, \
               g, y, env, rot, row_ptr, dy, scale, grad_env, reinterpret_cast<float4 *>(torque));  \
     break;                                                                                        \
   }
@@ -529,7 +551,7 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const floa
 int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float *da1, const float *radial,
                             const float *x, const int32_t *row_ptr, const int32_t *perm_src,
                             const int32_t *row_ptr_src, const float *rot, float *grad_radial, float *grad_x,
-                            float *torque, cudaStream_t st,
+                            float *torque, float *cuts, int *arrived, cudaStream_t st,
                             const ZpPlanes *grad_radial_planes, const ZpScale &scale) {
   const ZpPlanes gp = grad_radial_planes ? *grad_radial_planes : ZpPlanes{nullptr, 0, 0, 0, 0, nullptr};
   const ZpTables &t = p->t;
@@ -545,13 +567,14 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float 
   const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t,
                                        sums ? std::max(rows, t.K) : rows, sums && t.lmax > 2 ? 8 : 16, sums ? 1 : 4);
   const NodeArgs a{da1, radial, x, rot, row_ptr, perm_src, row_ptr_src, grad_radial, grad_x,
-                   reinterpret_cast<float4 *>(torque)};
-  const dim3 grid((unsigned)(N + 1), (unsigned)ns.groups, (unsigned)nl.parts);
+                   reinterpret_cast<float4 *>(torque), cuts, arrived};
+  const NodeCut cut = zp_node_cut(N, E, true, nl.parts);
+  const dim3 grid(cut.blocks(), (unsigned)ns.groups, (unsigned)nl.parts);
 #define CALL_S(LM, FMT, S)                                                                        \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(node_rotate_in_bwd_kernel<LM, FMT, S>, nl.smem, opt_in)) return rc_; \
-    zp_launch(node_rotate_in_bwd_kernel<LM, FMT, S>, grid, 32 * nl.warps, nl.smem, st, t, N, E, ns.G, ns.quads, a, \
+    zp_launch(node_rotate_in_bwd_kernel<LM, FMT, S>, grid, 32 * nl.warps, nl.smem, st, t, cut, E, ns.G, ns.quads, a, \
               gp, scale);                                                                         \
   }
 #define CALL_FMT(LM, FMT)                        \
@@ -575,4 +598,6 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float 
   return ZP_OK;
 }
 
-int zp_torque_slots(const ZpTables &t) { return 1 + 2 * node_shape(t).groups; }
+int zp_node_groups(const ZpTables &t) { return node_shape(t).groups; }
+int zp_torque_slots(const ZpTables &t) { return 1 + 2 * zp_node_groups(t); }
+int64_t zp_node_cuts_most(int64_t E) { return zp_node_cut(2 * E, E, true, 1).cuts; }
