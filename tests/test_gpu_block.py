@@ -183,6 +183,26 @@ def test_nodes_of_many_edges_are_cut(lmax, mmax, c, precision, jd64):
     assert torch.equal(got[1], again[1])       # added in one order whoever comes last
 
 
+@pytest.mark.parametrize("n,e", [(200, 199), (200, 200), (200, 599), (200, 600), (9, 160)])
+@pytest.mark.parametrize("lmax,c", [(2, 64), (4, 16), (5, 32)])
+def test_nodes_of_few_edges_whole_and_in_pieces(n, e, lmax, c, jd64, monkeypatch):
+    """On either side of the lines between kernels by edge and by node, and with a piece's edges at few of the rows."""
+    cfg = dict(lmax=lmax, mmax=2, sphere_channels=c, hidden_channels=8, edge_channels=8,
+               num_distance_basis=6, cutoff=5.0)
+    params = orc.init_params(cfg, seed=lmax)
+    case = random_case(cfg, n, e, seed=n + e)
+    want = oracle_node_out_and_vjp(cfg, params, case, case["upstream"], jd64)
+    block = make_block(cfg, params)
+    check_against(*gpu_node_out_and_vjp(block, case, case["upstream"]), *want)
+    monkeypatch.setattr("zippel_b200.blocks.eso2.MAX_EDGES_PER_CALL", 64)
+    dev = {k: v.cuda().float() if v.is_floating_point() else v.cuda() for k, v in case.items()}
+    out, gx, gpos, gparams = block.node_output_vjp(
+        *[dev[k] for k in ("pos", "atomic_numbers", "x_node", "edge_index", "shifts", "cos_gamma_k", "sin_gamma_k",
+                           "upstream")])
+    names = [name for name, _ in block.named_parameters()]
+    check_against(out, gx, gpos, dict(zip(names, gparams)), *want)
+
+
 def test_edges_along_the_polar_axis(jd64):
     """An edge whose direction is the polar axis has no proper rotation; its gradient follows the
     construction of the matrices (clamped, large) and must not disturb the other edges."""

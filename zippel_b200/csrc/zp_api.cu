@@ -690,7 +690,7 @@ int zp_core_backward(const zp_plan *plan, const ZpWorkspace &ws, const ZpConv &c
                                         ws.scales + kScG, st));
   }
   ZP_TIMED(ZP_K_ROTATE_GRAD_OUT,
-           zp_launch_rotate_grad_out(plan, N, E, grad_node_out, ws.y, c.env, ws.rot, c.dst, c.row_ptr, ws.dy,
+           zp_launch_rotate_grad_out(plan, c.first, c.into, E, grad_node_out, ws.y, c.env, ws.rot, c.dst, c.row_ptr, ws.dy,
                                      zp_scale_of(3.7f, ws.scales + kScG, ws.scales + kScDy), grad_env,
                                      ws.torque, st));
   // One conv at a time: input gradient dX = dY W_fold (K-major against the transposed planes),
@@ -842,7 +842,7 @@ static int eso2_backward(const zp_plan *plan, int64_t N, int64_t E, const float 
   if (workspace_bytes < ws.bytes) return ZP_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const ZpConv c{N, E, x_node, edge_vec, cos_g, sin_g, radial, env, src, dst, row_ptr, perm_src,
-                 row_ptr_src, w};
+                 row_ptr_src, w, {0, nullptr, nullptr, nullptr}, 0, N};
   ZpLanes lanes(plan, E, st);
   if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, grad_edge_vec, grad_radial,
                              grad_env, gw, rl, lanes)))

@@ -244,7 +244,9 @@ int zp_block_forward(const zp_plan *plan, const zp_front_config *front, const zp
   }
   ZpConv c{N, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
            call->dst, call->row_ptr + call->first_node, nullptr, nullptr, &params->so2};
-  if (call->perm_src && call->row_ptr_src)
+  // (a piece of a graph has most of its edges at few of the nodes: 100 000 in pieces of 30 000 edges took 51 ms of
+  // rotate_in by node, lmax 2 and 64 channels, 8.5 by edge)
+  if (N == call->n_rows && call->perm_src && call->row_ptr_src)
     c.view = ZpNodeView{call->n_rows, call->row_ptr, call->perm_src, call->row_ptr_src};
   return zp_core_forward(plan, ws, c, node_out, keep_for_backward, lanes);
 }
@@ -287,7 +289,8 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
   ZpRadialLayer rl{nullptr, nullptr, nullptr, ec, chain && E > 0 ? b.g_hid1 : nullptr,
                    grads->rad_w[2], grads->rad_b[2], fm.f1.fp16 ? sc + kScGHid1 : nullptr, &list};
   const ZpConv c{rows, E, call->x_node, b.edge_vec, b.cos_s, b.sin_s, ws.radial, b.env, call->src,
-                 call->dst, call->row_ptr, call->perm_src, call->row_ptr_src, &params->so2};
+                 call->dst, call->row_ptr, call->perm_src, call->row_ptr_src, &params->so2,
+                 {0, nullptr, nullptr, nullptr}, call->first_node, N};
   ZpLanes lanes(plan, E, st);
   if ((rc = zp_core_backward(plan, ws, c, grad_node_out, grad_x_node, b.g_vec_rot, nullptr, b.g_env,
                              want_so2 ? &grads->so2 : nullptr, &rl, lanes)))

@@ -258,7 +258,8 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
 int zp_launch_rotate_back_scatter(const zp_plan *p, int64_t N, const float *y, const float *env,
                                   const float *rot, const int32_t *row_ptr, float *node_out,
                                   cudaStream_t st);
-int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const float *g, const float *y,
+// N nodes from `first` on hold all edges' destinations
+int zp_launch_rotate_grad_out(const zp_plan *p, int64_t first, int64_t N, int64_t E, const float *g, const float *y,
                               const float *env, const float *rot, const int32_t *dst, const int32_t *row_ptr,
                               const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
                               float *torque, cudaStream_t st);

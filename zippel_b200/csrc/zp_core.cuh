@@ -192,6 +192,7 @@ struct ZpConv {
   const int32_t *src, *dst, *row_ptr, *perm_src, *row_ptr_src;
   const zp_weights *w;
   ZpNodeView view{0, nullptr, nullptr, nullptr};     // forward: all nodes, where the caller has the view by source
+  int64_t first = 0, into = 0;                       // backward: all edges end in these `into` nodes from `first` on
 };
 // The last dense layer of the radial MLP (blocks/eso2_ref.py:169-182, rad_func[6]), when the call
 // runs it itself: radial[E, R] = h[E, ec] w[R, ec]^T + b.

@@ -67,6 +67,13 @@ template <typename V>
 __device__ __forceinline__ void store_vec(float *p, const V &v) { *reinterpret_cast<V *>(p) = v; }
 template <typename V>
 __device__ __forceinline__ V zero_vec() { return V{}; }
+__device__ __forceinline__ u64 add2(u64 x, u64 y) {
+  u64 d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  return d;
+}
+__device__ __forceinline__ F4 add4(const F4 &x, const F4 &y) { return F4{add2(x.a, y.a), add2(x.b, y.b)}; }
+__device__ __forceinline__ F2 add4(const F2 &x, const F2 &y) { return F2{add2(x.a, y.a)}; }
 __device__ __forceinline__ void axpy4(F2 &acc, u64 w, const F2 &v) { acc.a = fma2(w, v.a, acc.a); }
 __device__ __forceinline__ F2 mul4(const F2 &x, const F2 &y) { return F2{mul2(x.a, y.a)}; }
 __device__ __forceinline__ u64 dot4(u64 acc, const F2 &x, const F2 &y) { return fma2(x.a, y.a, acc); }
@@ -249,12 +256,15 @@ inline NodeShape zp_node_shape(int channels, int vec) {
   s.G = s.quads <= 4 ? 4 : s.quads <= 8 ? 8 : s.quads <= 16 ? 16 : 32;
   return s;
 }
-// How a kernel by node is launched: a block for each of `parts` stretches of a node's edges, of four or eight warps
-// (less only where they do not fit).  What decides is how often the SMs have to take a new set of blocks, times
-// how long a block takes: its edges, and the start (row offsets, first rotation, first rows, one after the other,
-// as long as some three edges).  From 2 000 nodes on four warps and eight, whole nodes and halves are within 5 % of each
-// other and two warps 5 to 20 % behind; 216 nodes of 90 edges took 739 us a training step with eight warps, 799 with
-// four and 952 with two.
+// How a kernel by node is launched: a block for each of `parts` stretches of a node's edges.  What decides is how
+// often the SMs have to take a new set of blocks, times how long a block takes: its edges, and the start (row
+// offsets, first rotation, first rows, one after the other, as long as some three edges).  From 12 edges a node on four
+// warps and eight, whole nodes and halves are within 5 % of each other and two warps up to 10 % behind; 216 nodes of 90
+// edges took 739 us a training step with eight warps, 799 with four and 952 with two.  Nodes of few edges leave wide
+// blocks idle: the VJP of rotate_in over 60 000 edges (lmax 4, C 128) of nodes that have 1, 2, 4 and 8 each way took
+// 2.95, 1.72, 1.12 and 0.79 ms with four warps and the node's rows loaded before the first edge's were asked for; 0.90,
+// 0.74, 0.66 and 0.63 with one or two and all of them asked for at once (edge by edge 1.79, 1.38, 1.23 and 1.18).  One
+// or two are taken only where they promise a fifth: they lose that where a few nodes have most of the edges.
 constexpr int kNodeMaxWarps = 8;
 struct NodeLaunch {
   int warps, parts;
@@ -264,13 +274,17 @@ struct NodeLaunch {
 // sm_warps: warps of the kernel that an SM's registers hold; max_parts: 1 where a node's edges belong together
 inline NodeLaunch zp_node_launch(int64_t blocks, double items, const NodeShape &s, const ZpTables &t, int rows,
                                  int sm_warps, int max_parts) {
-  NodeLaunch best{1, 1, 0};
-  double best_cost = 1e300;
+  NodeLaunch best{1, 1, 0}, few{1, 1, 0};
+  double best_cost = 1e300, few_cost = 1e300;
   for (int warps = 1; warps <= kNodeMaxWarps; warps *= 2) {
     const size_t workers = 32 * warps / s.G;
     const size_t smem = sizeof(float) * ((size_t)s.G * s.vec * (t.K + workers * rows) + workers * 2 * t.rot_ld);
     if (warps > 1 && smem > 220 * 1024) break;
-    if (warps == 4) best_cost = 1e300;   // one and two were for rows too many for four
+    if (warps == 4) {
+      few = best;
+      few_cost = best_cost;
+      best_cost = 1e300;
+    }
     const int64_t resident = 148 * std::max<int64_t>(1, std::min<int64_t>(sm_warps / warps, (int64_t)(225 * 1024 / (smem + 1024))));
     for (int parts = 1; parts <= max_parts; parts *= 2) {
       const double rounds = std::max(1.0, (double)(blocks * parts) / (double)resident + 0.5);
@@ -281,7 +295,7 @@ inline NodeLaunch zp_node_launch(int64_t blocks, double items, const NodeShape &
       }
     }
   }
-  return best;
+  return few_cost < 0.8 * best_cost ? few : best;
 }
 
 // The node's edges, numbered: those into it, then (with a source view) those out of it.  Block N of a launch
@@ -416,11 +430,9 @@ struct StageAll {
 __device__ __forceinline__ void stage_rot(const float *rot, float *rot_s, int ld, int li, int G) {
   for (int i = 4 * li; i < ld; i += 4 * G) cp_async<16>(rot_s + i, rot + i);
 }
-// `mine` vectors of each of the node's K rows into shared memory, ls floats a row
+// Puts the node's K rows on their way into shared memory, ls floats a row: every lane its channels (at x, x_s) of
+// its worker's share of the rows.  For all workers, so a block meets once they have landed.
 template <typename V>
-__device__ __forceinline__ void stage_node(const float *x, int C, int K, int mine, float *x_s, int ls) {
-  for (int i = threadIdx.x; i < K * mine; i += blockDim.x) {
-    const int k = i / mine, q = i - k * mine;
-    store_vec<V>(x_s + k * ls + q * VecOf<V>::n, load_vec<V>(x + (size_t)k * C + q * VecOf<V>::n));
-  }
+__device__ __forceinline__ void stage_node(const float *x, int C, int K, int w, int workers, float *x_s, int ls) {
+  for (int k = w; k < K; k += workers) cp_async<4 * VecOf<V>::n>(x_s + k * ls, x + (size_t)k * C);
 }

@@ -249,10 +249,11 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, const NodeCut cu
     stage_rot(rot + (size_t)e * t.rot_ld, rot_s + buffer * t.rot_ld, t.rot_ld, li, G);
   };
   const int i0 = edges.first + w;
+  if (active) stage_node<F4>(g_out + (size_t)edges.row(cut) * t.K * t.C + c, t.C, K, w, workers, g_s + c, ls);
   int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
   if (e >= 0) rotation(e, 0);
   StageAll<LMAX, LMAX, F4, true, false>::run(t, rows(e), t.C, nullptr, y_s, nullptr, ls, e >= 0 && active);
-  stage_node<F4>(g_out + (size_t)edges.row(cut) * t.K * t.C, t.C, K, quads, g_s, ls);
+  cp_async_wait<LMAX>();                 // the node's rows went with degree 0
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
@@ -298,11 +299,9 @@ template <> struct Elem<kFmtFp32> { using type = float; };
 // and 231 of the sums -> 531, 384 000 in one 4.56 and 1.45 ms -> 2.90; bound by instruction issue (2 400 a worker and
 // edge half, eight warps to an SM at 252 registers), HBM at half its rate.
 // SUMS: the gradient of x_node is wanted (not in a force evaluation; the others are the same to the last bit).
-// what a lane needs of an edge
-template <typename T_>
+// what a lane needs of an edge: its channels in row 0 of da1, in column 0 of radial
 struct EdgeAt {
-  const float *da, *rad;                 // its channels in row 0 of da1, in column 0 of radial
-  T_ *out;                               // ... of grad_radial
+  const float *da, *rad;
 };
 template <int L, int LMAX, int FMT, typename V, bool SUMS>
 struct NodeRot {
@@ -310,7 +309,7 @@ struct NodeRot {
   // rot: the current edge's rotation; next: the worker's next edge, staged as this one is used up
   static __device__ __forceinline__ void run(const ZpTables &t, const float *x_s, float *da_s, float *rad_s, int ls,
                                              T_ *out, int64_t plane_bytes, u64 inv, const float *rot, bool live,
-                                             const EdgeAt<T_> &next, bool more,
+                                             const EdgeAt &next, bool more,
                                              V (&acc)[SUMS ? (LMAX + 1) * (LMAX + 1) : 1], Torque &T) {
     if constexpr (L > 0)
       NodeRot<L - 1, LMAX, FMT, V, SUMS>::run(t, x_s, da_s, rad_s, ls, out, plane_bytes, inv, rot, live, next, more, acc, T);
@@ -403,7 +402,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, const NodeCut cut,
   float *x_s = node_s, *stage = node_s + (size_t)K * ls, *da_s = stage + (size_t)w * rows * ls + li * VN;
   float *rad_s = da_s + t.Km * ls;
   float *rot_s = stage + (size_t)workers * rows * ls + (size_t)w * 2 * t.rot_ld;
-  const NodeEdges edges(blockIdx.x, cut, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges node(blockIdx.x, cut, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
   float inv = 1.f;
   if constexpr (FMT == kFmtFp16x2)
     inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
@@ -412,35 +411,46 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, const NodeCut cut,
   V acc[SUMS ? K : 1];
 #pragma unroll
   for (int k = 0; k < (SUMS ? K : 1); ++k) acc[k] = zero_vec<V>();
-  if (edges.first == edges.last && (!SUMS || blockIdx.x >= cut.nodes)) return;
+  if (node.first == node.last) {
+    if (SUMS && blockIdx.x < cut.nodes && active)
+      for (int k = w; k < K; k += workers) store_vec<V>(a.grad_x + ((size_t)blockIdx.x * K + k) * t.C + c, zero_vec<V>());
+    return;
+  }
+  // with sums the loop has every register in use
+  __shared__ __align__(16) unsigned char edges_s[sizeof(NodeEdges)];
+  if (SUMS && threadIdx.x == 0) *reinterpret_cast<NodeEdges *>(edges_s) = node;
+  if (SUMS) __syncthreads();
+  const NodeEdges &edges = SUMS ? *reinterpret_cast<NodeEdges *>(edges_s) : node;
 
-  auto at = [&](int64_t e, int i) {
-    const int col = (i < edges.own ? t.C : 0) + c;
-    EdgeAt<T_> p;
-    p.da = a.da1 + (size_t)e * t.Km * 2 * t.C + col;
-    p.rad = a.radial + (size_t)e * t.R + col;
-    if constexpr (FMT == kFmtFp32) p.out = a.grad_radial + (size_t)e * t.R + col;
-    else p.out = static_cast<uint16_t *>(grad_radial_planes.base) + e * grad_radial_planes.ld + col;
-    return p;
+  // (edge -1 reads as edge 0)
+  auto column = [&](int i) { return (i < edges.own ? t.C : 0) + c; };
+  auto at = [&](int e, int i) {
+    const size_t row = max(e, 0);
+    return EdgeAt{a.da1 + row * t.Km * 2 * t.C + column(i), a.radial + row * t.R + column(i)};
+  };
+  auto out_at = [&](int e, int i) {
+    const size_t row = max(e, 0);
+    if constexpr (FMT == kFmtFp32) return a.grad_radial + row * t.R + column(i);
+    else return static_cast<uint16_t *>(grad_radial_planes.base) + row * grad_radial_planes.ld + column(i);
   };
   auto rotation = [&](int64_t e, int buffer) {
     stage_rot(a.rot + (size_t)e * t.rot_ld, rot_s + buffer * t.rot_ld, t.rot_ld, li, G);
   };
   const int i0 = edges.first + w;
+  if (active) stage_node<V>(a.x + (size_t)edges.row(cut) * t.K * t.C + c, t.C, K, w, workers, x_s + li * VN, ls);
   int e = edges.edge(i0), e_next = edges.edge(i0 + workers);
-  EdgeAt<T_> cur = at(e < 0 ? 0 : e, i0);
   if (e >= 0) rotation(e, 0);
-  StageAll<LMAX, LMAX, V, true, true>::run(t, cur.da, 2 * t.C, cur.rad, da_s, rad_s, ls, e >= 0 && active);
-  if (edges.total > 0) stage_node<V>(a.x + (size_t)edges.row(cut) * t.K * t.C + c0, t.C, K, mine, x_s, ls);
+  StageAll<LMAX, LMAX, V, true, true>::run(t, at(e, i0).da, 2 * t.C, at(e, i0).rad, da_s, rad_s, ls, e >= 0 && active);
+  cp_async_wait<LMAX>();                 // the node's rows went with degree 0
   __syncthreads();
   for (int i = i0, buffer = 0; i - w < edges.last; i += workers, buffer ^= 1) {      // as often on all lanes
     const int e_after = edges.edge(i + 2 * workers);
-    const EdgeAt<T_> next = at(e_next < 0 ? 0 : e_next, i + workers);
+    const EdgeAt next = at(e_next, i + workers);
     Torque T{0ull, 0ull, 0ull};
     cp_async_wait<LMAX>();               // degree 0 and the rotation have landed
     __syncwarp();                        // ... the other lanes' part of it, and all are done with the last
     if (e_next >= 0) rotation(e_next, buffer ^ 1);
-    NodeRot<LMAX, LMAX, FMT, V, SUMS>::run(t, x_s + li * VN, da_s, rad_s, ls, cur.out, plane_bytes, inv2,
+    NodeRot<LMAX, LMAX, FMT, V, SUMS>::run(t, x_s + li * VN, da_s, rad_s, ls, out_at(e, i), plane_bytes, inv2,
                                      rot_s + buffer * t.rot_ld, e >= 0 && active, next, e_next >= 0 && active,
                                      acc, T);
     float t0 = sum2(T.t0), t1 = sum2(T.t1), t2 = sum2(T.t2);
@@ -453,53 +463,60 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, const NodeCut cut,
       a.torque[(size_t)(1 + 2 * blockIdx.y + (i < edges.own ? 1 : 0)) * E + e] = make_float4(t0, t1, t2, 0.f);
     e = e_next;
     e_next = e_after;
-    cur = next;
   }
   cp_async_wait<0>();
-  if (!SUMS || edges.n == cut.nodes) return;
+  if (!SUMS) return;
+  const int n = edges.n;
+  if (n == cut.nodes) return;            // left-out slots
+  // this lane's place in the rows that the sums go to
+  float *const to = (blockIdx.x > cut.nodes ? a.cuts + (size_t)(blockIdx.x - cut.nodes - 1) * K * t.C
+                                            : a.grad_x + (size_t)n * K * t.C) + c0 + li * VN;
   __syncthreads();                       // all are done with their rows: the sums take their place
-  float *sums = stage + (size_t)w * rows * ls + li * VN;
+  float *const sums = stage + li * VN;
 #pragma unroll
-  for (int k = 0; k < K; ++k) store_vec<V>(sums + k * ls, acc[SUMS ? k : 0]);
+  for (int k = 0; k < K; ++k) store_vec<V>(sums + ((size_t)w * rows + k) * ls, acc[SUMS ? k : 0]);
   __syncthreads();
-  const bool tail = blockIdx.x > cut.nodes;                 // what follows a cut
-  float *const gx = a.grad_x + (size_t)edges.n * t.K * t.C + c0;
-  float *const to = tail ? a.cuts + (size_t)(blockIdx.x - cut.nodes - 1) * t.K * t.C + c0 : gx;
-  for (int i = threadIdx.x; i < K * mine * VN; i += blockDim.x) {
-    const int k = i / (mine * VN), q = i - k * mine * VN;
-    float s = 0.f;
-    for (int v = 0; v < workers; ++v) s += stage[((size_t)v * rows + k) * ls + q];
-    to[(size_t)k * t.C + q] = s;
-  }
-  if (edges.cut0 > edges.cut1) return;
+  if (active)
+    for (int k = w; k < K; k += workers) {
+      V s = load_vec<V>(sums + k * ls);
+      for (int v = 1; v < workers; ++v) s = add4(s, load_vec<V>(sums + ((size_t)v * rows + k) * ls));
+      store_vec<V>(to + (size_t)k * t.C, s);
+    }
+  const int cut0 = edges.cut0, cut1 = edges.cut1;
+  if (cut0 > cut1) return;
   // a cut node: whoever gets done last adds up, in the order of the stretches
   __shared__ int all_here;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0)
-    all_here = atomicAdd(a.arrived + blockIdx.y * kZpNodeCuts + edges.cut0, 1) == (int)(edges.cut1 - edges.cut0) + 1;
+    all_here = atomicAdd(a.arrived + blockIdx.y * kZpNodeCuts + cut0, 1) == cut1 - cut0 + 1;
   __syncthreads();
-  if (!all_here) return;
+  if (!all_here || !active) return;
   __threadfence();
-  for (int i = threadIdx.x; i < K * mine * VN; i += blockDim.x) {
-    const int k = i / (mine * VN), q = i - k * mine * VN;
-    const size_t at = (size_t)k * t.C + q;
-    float s = __ldcg(gx + at);
-    for (uint32_t c1 = edges.cut0; c1 <= edges.cut1; ++c1) s += __ldcg(a.cuts + (size_t)(c1 - 1) * t.K * t.C + c0 + at);
-    gx[at] = s;
+  for (int k = w; k < K; k += workers) {
+    const size_t at = (size_t)k * t.C + c0 + li * VN;
+    float *const gx = a.grad_x + (size_t)n * K * t.C + at;
+    for (int v = 0; v < VN; ++v) {
+      float s = __ldcg(gx + v);
+      for (int i = cut0; i <= cut1; ++i) s += __ldcg(a.cuts + (size_t)(i - 1) * K * t.C + at + v);
+      gx[v] = s;
+    }
   }
 }
 
 }  // namespace
 
-int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const float *g, const float *y,
+int zp_launch_rotate_grad_out(const zp_plan *p, int64_t first, int64_t N, int64_t E, const float *g, const float *y,
                               const float *env, const float *rot, const int32_t *dst, const int32_t *row_ptr,
                               const ZpPlanes &dy, const ZpScale &scale, float *grad_env,
                               float *torque, cudaStream_t st) {
   if (E == 0) return ZP_OK;
   const ZpTables &t = p->t;
   const NodeShape ns = zp_node_shape(t.C, 4);
-  if (ns.groups == 1) {                  // the sums over an edge's channels are one worker's
+  // By node the sums over an edge's channels are one worker's; nodes of fewer than three edges are over before
+  // they have paid for their start.  By edge / by node at one, two and three edges a node: lmax 4, C 128, 60 000 edges
+  // 363 / 370, 346 / 298 and 336 / 265 us; lmax 6, 20 000 edges 255 / 298, 222 / 225; lmax 2, C 32, 20 000 21 / 42, 20 / 30.
+  if (ns.groups == 1 && E >= 3 * N) {
     const NodeLaunch nl = zp_node_launch(N, (double)E / (double)N, ns, t, t.Km, 16, 4);
     const NodeCut cut = zp_node_cut(N, E, false, nl.parts);
 #define CALL_FMT(LM, FMT)                                                                         \
@@ -507,7 +524,7 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t N, int64_t E, const floa
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(node_rotate_grad_out_kernel<LM, FMT>, nl.smem, opt_in)) return rc_; \
     zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3(cut.blocks(), 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, cut, E, ns.G, ns.quads, \
-              g, y, env, rot, row_ptr, dy, scale, grad_env, reinterpret_cast<float4 *>(torque));  \
+              g + (size_t)first * t.K * t.C, y, env, rot, row_ptr + first, dy, scale, grad_env, reinterpret_cast<float4 *>(torque));  \
     break;                                                                                        \
   }
 #define CALL(LM)                                               \
