@@ -383,10 +383,15 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
   const ZpTables &t = p->t;
   const int Q = t.C / 2;
   if (Q < 1 || Q > kRotInThreads) return ZP_ERR_UNSUPPORTED;
-  // by node where at least seven lanes of ten have channels (72 of them leave 14 of 32 lanes idle: 17 900 edges
-  // 173 us, 74 by edge), and not where most nodes have no edge (60 000 among 2 000 nodes of 100 000: 2 % of an inference)
+  // By node where it is the faster one.  Lanes without channels: 30 000 edges, by edge / by node, lmax 4, 64, 72,
+  // 96, 112 and 128 channels 152 / 135, 175 / 263, 212 / 220, 250 / 265 and 262 / 244 us, lmax 6, 72, 96, 112 and 128 347 / 431,
+  // 425 / 367, 411 / 355 and 520 / 392.  Half rows of other than whole 32-byte sectors are written twice: 56 and
+  // 104 channels 144 / 222 and 202 / 289 at lmax 4, 290 / 360 and 390 / 464 at lmax 6.  Narrow rows at low degrees: lmax 2,
+  // 257 000 edges of 32, 64 and 128 channels 287 / 378, 522 / 505 and 1 063 / 945.  And not where most nodes have
+  // no edge (60 000 among 2 000 nodes of 100 000: 2 % of an inference).
   const NodeShape ns = zp_node_shape(t.C, 4);
-  if (view.perm_src && 10 * ns.quads >= 7 * ns.G && E >= view.nodes) {
+  const bool full = t.lmax >= 5 ? t.C % 16 == 0 && 10 * ns.quads >= 7 * ns.G : ns.quads == ns.G;
+  if (view.perm_src && full && (t.lmax >= 3 || t.C >= 64) && E >= view.nodes) {
     const int64_t N = view.nodes;
     const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t, t.rad_rows, 16, 4);
     const NodeCut cut = zp_node_cut(N, E, true, nl.parts);

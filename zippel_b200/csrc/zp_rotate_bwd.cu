@@ -516,7 +516,8 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t first, int64_t N, int64_
   // By node the sums over an edge's channels are one worker's; nodes of fewer than three edges are over before
   // they have paid for their start.  By edge / by node at one, two and three edges a node: lmax 4, C 128, 60 000 edges
   // 363 / 370, 346 / 298 and 336 / 265 us; lmax 6, 20 000 edges 255 / 298, 222 / 225; lmax 2, C 32, 20 000 21 / 42, 20 / 30.
-  if (ns.groups == 1 && E >= 3 * N) {
+  // At lmax 1 a worker's idle lanes weigh more than the rows of g: 72 of 128 channels, 30 000 edges 19 / 24 us.
+  if (ns.groups == 1 && E >= 3 * N && (t.lmax >= 2 || 10 * ns.quads >= 7 * ns.G)) {
     const NodeLaunch nl = zp_node_launch(N, (double)E / (double)N, ns, t, t.Km, 16, 4);
     const NodeCut cut = zp_node_cut(N, E, false, nl.parts);
 #define CALL_FMT(LM, FMT)                                                                         \
