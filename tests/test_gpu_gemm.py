@@ -137,6 +137,12 @@ def test_tensor_core_linear_and_vjp(M, K, N, precision):
     assert plan.device_status() == 0
 
 
+@pytest.mark.parametrize("M,K,N", [(20000, 128, 128), (20001, 128, 128), (20001, 64, 64), (20001, 256, 256), (40000, 96, 96)])
+def test_tensor_core_linear_apart_and_together(M, K, N):
+    """On either side of the line between one launch for both products of the VJP and one for each."""
+    test_tensor_core_linear_and_vjp(M, K, N, 2)
+
+
 def test_bounded_wait_runs_out_and_the_library_keeps_working():
     """A wait that nothing will ever satisfy: the kernel must give up after its time limit, record
     ZP_ERR_DEVICE_TIMEOUT in the plan's status word and return with every warp (no trap, no hang);

@@ -363,6 +363,8 @@ bool zp_gemm_tc_fusable(const ZpGemmTc &g);
 int zp_gemm_tc_splits(const ZpGemmTc &g);
 // K split (<= max_splits) that fills the device's CTAs (or CTA pairs) most evenly for this problem
 int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits);
+// whether a launch of the product alone goes to the CTA-pair kernel
+bool zp_gemm_tc_pairs(const ZpGemmTc &g);
 // fp32 [rows, cols] (row stride ld_in) -> planes [rows, out.ld], zero padded
 int zp_launch_split_list(const ZpSplitList &list, cudaStream_t st);
 int zp_launch_split_planes(int64_t rows, int64_t cols, const float *in, int64_t ld_in,

@@ -1879,6 +1879,8 @@ int zp_gemm_tc_pick_splits(const ZpGemmTc &g, int max_splits) {
   return best;
 }
 
+bool zp_gemm_tc_pairs(const ZpGemmTc &g) { return use_pair(g); }
+
 // The K split of a group's products whose contraction runs over the edges (the last `nw` of n): of a few
 // that cut their tiles to between a whole and a third of the launch's time, the one with which it gets done
 // first, but no more partial results than that takes.

@@ -87,30 +87,37 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
                               cudaStream_t side, float *dx_absmax, int64_t dx_cols) {
   int rc, n = 0;
   const int P = dy.planes, fp16 = dy.fp16;
-  const bool together = dx && dw && M <= kTogetherBackward;
   ZpGemmTc g[2];
   if (dx) {
     const int64_t cols = dx_cols > 0 ? dx_cols : K;
     g[n++] = ZpGemmTc{M, cols, N, P, dy.base, dy.ld, dy.plane_stride, 0,
                       w.base, w.ld, w.plane_stride, 1, nullptr, dx, (cols + 3) / 4 * 4,
                       plan->status_dev, 0, 1, 0, 0, fp16, dy.scale, w.scale, dx_absmax};
-    if (!together && (rc = zp_launch_gemm_tc(g[0], st))) return rc;
   }
+  const int64_t ldk = (K + 3) / 4 * 4;           // rows of the partial sums start 16-byte aligned
+  ZpGemmTc &wg = g[n];
   if (dw) {
-    const int64_t ldk = (K + 3) / 4 * 4;         // rows of the partial sums start 16-byte aligned
-    ZpGemmTc &wg = g[n++];
     wg = ZpGemmTc{N, K, M, P, dy.base, dy.ld, dy.plane_stride, 1,
                   x.base, x.ld, x.plane_stride, 1, nullptr, partials, ldk, plan->status_dev,
                   0, 1, N * ldk, 0, fp16, dy.scale, x.scale, nullptr};
-    if (together) {
-      zp_gemm_group_splits(g, n, 1, max_splits);
-      if ((rc = zp_launch_gemm_group(g, n, st))) return rc;
-    } else {
-      wg.ksplit = zp_gemm_tc_pick_splits(wg, max_splits);
-      if ((rc = zp_launch_gemm_tc(wg, side))) return rc;
-    }
-    list.add(partials, dw, N * ldk, (int)N, (int)K, zp_gemm_tc_splits(wg), ZP_FIN_SUM, (int)ldk);
+    wg.ksplit = zp_gemm_tc_pick_splits(wg, max_splits);
+    ++n;
   }
+  // One launch for both, but not where the weight gradient would leave the CTA pairs for it: with two planes
+  // the other kernel takes its operands in k-blocks of half the depth, and they are all it has.  A call of the layer
+  // and its VJP, apart / together, two planes: 128 x 128 at 25 000, 40 000 and 100 000 rows 188 / 202, 212 / 248 and
+  // 332 / 387 us, 256 x 256 at 25 000 and 100 000 218 / 242 and 416 / 511 (15 000 rows of either the same within 5 %);
+  // same kernel either way: 64 x 64 at 100 000 384 / 357, 128 x 1536 at 25 000 357 / 334.
+  const bool together = dx && dw && M <= kTogetherBackward &&
+                        !(P == 2 && M > 20000 && zp_gemm_tc_pairs(wg) && !zp_gemm_tc_pairs(g[0]));
+  if (together) {
+    zp_gemm_group_splits(g, n, 1, max_splits);
+    if ((rc = zp_launch_gemm_group(g, n, st))) return rc;
+  } else {
+    if (dx && (rc = zp_launch_gemm_tc(g[0], st))) return rc;
+    if (dw && (rc = zp_launch_gemm_tc(wg, side))) return rc;
+  }
+  if (dw) list.add(partials, dw, N * ldk, (int)N, (int)K, zp_gemm_tc_splits(wg), ZP_FIN_SUM, (int)ldk);
   if (db) return zp_launch_colsum(M, N, dy, db, colsum_scratch, list, side);
   return ZP_OK;
 }
