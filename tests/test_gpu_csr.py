@@ -33,3 +33,20 @@ def test_bucket_sizes_and_input_orders(degree, order):
     g = EdgeGraph.build(torch.from_numpy(ei).cuda(), n)
     for key, value in want.items():
         assert np.array_equal(getattr(g, key).cpu().numpy(), value), key
+
+
+@pytest.mark.parametrize("n,degree", [(64, 64), (65, 63), (128, 32)])
+def test_recorded_sorts_on_either_side_of_the_one_block_line(n, degree):
+    from zippel_b200.graph import EdgeGraph, csr_reference
+    rng = np.random.default_rng(n)
+    edges = [rng.integers(0, n, (2, n * degree)) for _ in range(2)]
+    ei = torch.from_numpy(edges[0]).cuda()
+    EdgeGraph.build(ei, n)
+    recorded = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(recorded):
+        g = EdgeGraph.build(ei, n, validate=False)
+    for e in edges:
+        ei.copy_(torch.from_numpy(e))
+        recorded.replay()
+        for key, value in csr_reference(e, n).items():
+            assert np.array_equal(getattr(g, key).cpu().numpy(), value), key

@@ -303,7 +303,7 @@ __global__ void rank_src_kernel(int64_t N, int64_t E, const int32_t *__restrict_
 // 199 -> 195, forces of 100 at lmax 4 613 -> 607.  One SM takes 17 to 22 us on the device for 6 000 to 10 000 edges, where the
 // five kernels take 13 once they are queued, and no pass of that size got faster; a thousand nodes are 31 buckets
 // for each warp, and their 4 000 edges in any order took 159 us for 65.
-constexpr int kSmallThreads = 1024, kSmallEdges = 4096, kSmallNodes = 128;
+constexpr int kSmallThreads = 1024, kSmallEdges = 4096, kSmallNodes = 128, kSmallReplayed = 64;
 struct SmallSort {
   const int64_t *src, *dst, *z;
   int n_elements;
@@ -474,7 +474,16 @@ static int csr_build(const int64_t *edge_index, int64_t E, int64_t N, int32_t *p
   const CsrWork w = carve_csr(E, N, work);
   if (work_bytes < w.bytes) return ZP_ERR_WORKSPACE;
   const int64_t *src64 = edge_index, *dst64 = edge_index + E;
-  if (E > 0 && E <= kSmallEdges && N > 0 && N <= kSmallNodes) {
+  // (in a recorded graph launches cost the host nothing, and above 64 nodes one SM is no longer the faster: 100 to 128
+  // nodes, 1 000 to 4 096 edges in any order 19 to 24 us a replay, 14 to 15 with the five kernels; 64 nodes 13 to 17 and
+  // 14 to 16, 32 and fewer 5 to 13 and 12 to 25)
+  int64_t most = kSmallNodes;
+  if (E > 0 && E <= kSmallEdges && N > kSmallReplayed && N <= most) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) cudaGetLastError();
+    if (capture != cudaStreamCaptureStatusNone) most = kSmallReplayed;
+  }
+  if (E > 0 && E <= kSmallEdges && N > 0 && N <= most) {
     static ZpSmemOptIn opt_in;
     const size_t smem = small_sort_bytes(E, N);
     if (int rc = zp_ensure_smem(small_sort_kernel, small_sort_bytes(kSmallEdges, kSmallNodes), opt_in)) return rc;
