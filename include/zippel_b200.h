@@ -441,8 +441,8 @@ int zp_block_backward(const zp_plan *plan, const zp_front_config *front, const z
  * call found another number of edges than the first (not seen: both read the same copies).       */
 #define ZP_NEIGHBORS_MAX_HITS 1024
 #define ZP_NEIGHBORS_MAX_CAP 256
-/* Work for any max_neighbors, and for one (less where it is below 128): the first call keeps each
- * atom's edges there for the second.  */
+/* Work for any max_neighbors, and for one and all smaller ones (less where it is below 128): the first
+ * call keeps each atom's edges there for the second.  */
 size_t zp_neighbors_work_bytes(int64_t n_atoms, double box, double cutoff);
 size_t zp_neighbors_work_bytes_capped(int64_t n_atoms, double box, double cutoff, int max_neighbors);
 int zp_neighbors_count(const double *pos, int64_t n_atoms, double box, double cutoff,

@@ -151,3 +151,18 @@ def test_cap_reached_near_by_and_not(n, box, cap):
     want = no.neighbor_list(pos, box, 6.0, cap)
     for g, w in zip(run(pos, box, 6.0, cap), want):
         assert g.shape == w.shape and np.array_equal(g, w)
+
+
+@pytest.mark.parametrize("asked,cap", [(200, 130), (100, 5), (30, 30)])
+def test_work_of_a_cap_is_enough_for_smaller_ones(asked, cap):
+    """A smaller cap may be looked for in finer cells."""
+    from zippel_b200 import _lib
+    from zippel_b200.graph import neighbor_list
+    n, box, cutoff = 4000, 30.0, 9.0
+    pos = torch.rand(n, 3, dtype=torch.float64, generator=torch.Generator().manual_seed(cap)).cuda() * box
+    nbytes = _lib.load().zp_neighbors_work_bytes_capped(n, box, cutoff, asked)
+    work = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    out = torch.empty(n + 2, dtype=torch.int32, device="cuda")
+    _lib.run(pos.device, "zp_neighbors_count", pos.data_ptr(), n, box, cutoff, cap, out.data_ptr(),
+             out[n + 1:].data_ptr(), work.data_ptr(), nbytes)
+    assert torch.equal(out[:n + 1], neighbor_list(pos, box, cutoff, cap)[2]) and out[n + 1].item() == 0

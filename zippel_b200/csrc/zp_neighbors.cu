@@ -641,7 +641,7 @@ size_t zp_neighbors_work_bytes(int64_t n_atoms, double box, double cutoff) {
 size_t zp_neighbors_work_bytes_capped(int64_t n_atoms, double box, double cutoff, int max_neighbors) {
   Grid g;
   if (n_atoms < 0 || make_grid(n_atoms, box, cutoff, max_neighbors, &g)) return 0;
-  return carve_nb(n_atoms, g, max_neighbors, nullptr).bytes;
+  return carve_nb(n_atoms, g, max_neighbors, nullptr, true).bytes;      // a smaller cap may have finer cells
 }
 
 int zp_neighbors_count(const double *pos, int64_t N, double box, double cutoff, int max_neighbors,
