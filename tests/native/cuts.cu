@@ -36,33 +36,30 @@ int main(int argc, char **argv) {
     for (int both = 0; both < 2; ++both) {
       const int parts = 1 << pick(0, 2);
       const NodeCut cut = zp_node_cut(N, E, both, parts);
-      if (cut.cuts >= kZpNodeCuts || (int64_t)cut.cuts > zp_node_cut(2 * (int64_t)E, E, true, 1).cuts) return std::puts("cuts"), 1;
+      if (cut.cuts >= kZpNodeCuts || (int64_t)cut.cuts > zp_node_cut(1, E, true, 1).cuts) return std::puts("cuts"), 1;
       std::vector<int> into(E, 0), from(E, 0);
       std::map<int, int> stretches;
       std::map<int, std::pair<uint32_t, uint32_t>> said;
-      for (int b = 0; b < (int)cut.blocks(); ++b)
-        for (int part = 0; part < parts; ++part) {
-          const NodeEdges s(b, cut, E, row_ptr.data(), both ? view.data() : nullptr, row_ptr_src.data(), part, parts);
-          if (s.first > s.last || s.first < 0 || s.last > s.total || s.last - s.first > 2 * (int)cut.step) return std::puts("stretch"), 1;
-          if (s.n < 0 || s.n > N || s.row(cut) >= N || (b <= N && s.n != b)) return std::puts("node"), 1;
-          if (s.edge(s.last) != -1) return std::puts("end"), 1;
-          for (int i = s.first; i < s.last; ++i) {
-            const int e = s.edge(i);
-            if (e < 0 || e >= E) return std::puts("edge"), 1;
-            if (i < s.own ? into[e]++ || (s.n < N ? e < row_ptr[s.n] || e >= row_ptr[s.n + 1] : e < row_ptr[N])
-                          : from[e]++ != 0)
-              return std::puts("twice"), 1;
-          }
-          if (s.cut0 > s.cut1 || part) continue;
-          if (b <= N || s.first < s.last || s.last > 0) {
-            if (s.first == s.last && parts == 1 && b > N) continue;
-            said[s.n] = {s.cut0, s.cut1};
-          }
-          // as the kernel numbers what follows a cut
-          const bool mine = b <= N || ((uint32_t)(b - N) >= s.cut0 && (uint32_t)(b - N) <= s.cut1);
-          if (!mine && s.last > s.first) return std::puts("number"), 1;
-          if (mine) ++stretches[s.n];
+      for (int b = 0; b < (int)cut.blocks(); ++b) {
+        const NodeEdges s(b, cut, E, row_ptr.data(), both ? view.data() : nullptr, row_ptr_src.data());
+        const bool tail = b >= cut.ends();
+        if (s.first > s.last || s.first < 0 || s.last > s.total || s.last - s.first > 2 * (int)cut.step) return std::puts("stretch"), 1;
+        if (s.n < 0 || s.n > N || s.row(cut) >= N || (!tail && s.n != b / parts)) return std::puts("node"), 1;
+        if (s.edge(s.last) != -1) return std::puts("end"), 1;
+        for (int i = s.first; i < s.last; ++i) {
+          const int e = s.edge(i);
+          if (e < 0 || e >= E) return std::puts("edge"), 1;
+          if (i < s.own ? into[e]++ || (s.n < N ? e < row_ptr[s.n] || e >= row_ptr[s.n + 1] : e < row_ptr[N])
+                        : from[e]++ != 0)
+            return std::puts("twice"), 1;
         }
+        if (s.cut0 > s.cut1) continue;
+        said[s.n] = {s.cut0, s.cut1};
+        // as the kernel numbers what follows a cut
+        const uint32_t k = (uint32_t)(b - cut.ends() + 1);
+        if (tail && s.last > s.first && (k < s.cut0 || k > s.cut1)) return std::puts("number"), 1;
+        if (tail ? s.last > s.first : b % parts == 0) ++stretches[s.n];
+      }
       for (int e = 0; e < E; ++e)
         if (into[e] != 1 || from[e] != (both ? 1 : 0)) return std::puts("left out"), 1;
       for (auto &[n, cuts] : said) {

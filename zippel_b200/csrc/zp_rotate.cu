@@ -162,9 +162,9 @@ node_rotate_in_kernel(const __grid_constant__ ZpTables t, const NodeCut cut, int
   const int c = c0 + 4 * li;
   float *x_s = node_s, *stage = node_s + (size_t)K * ls, *rad_s = stage + (size_t)w * t.rad_rows * ls + 4 * li;
   float *rot_s = stage + (size_t)workers * t.rad_rows * ls + (size_t)w * 2 * t.rot_ld;
-  const float inv = zp_publish_scale(a1, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
+  const float inv = zp_publish_scale(a1, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
-  const NodeEdges edges(blockIdx.x, cut, E, row_ptr, perm_src, row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges edges(blockIdx.x, cut, E, row_ptr, perm_src, row_ptr_src);
   if (edges.first == edges.last) return;
   auto column = [&](int i) { return (i < edges.own ? t.C : 0) + c; };
   auto gains = [&](int e, int i) { return radial + (size_t)(e < 0 ? 0 : e) * t.R + column(i); };
@@ -395,7 +395,7 @@ int zp_launch_rotate_in(const zp_plan *p, int64_t E, const float *x, const int32
     const int64_t N = view.nodes;
     const NodeLaunch nl = zp_node_launch(N * ns.groups, 2.0 * (double)E / (double)N, ns, t, t.rad_rows, 16, 4);
     const NodeCut cut = zp_node_cut(N, E, true, nl.parts);
-    const dim3 grid(cut.blocks(), (unsigned)ns.groups, (unsigned)nl.parts);
+    const dim3 grid(cut.blocks(), (unsigned)ns.groups);
 #define CALL_FMT(LM, FMT)                                                                         \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \

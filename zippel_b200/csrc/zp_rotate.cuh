@@ -302,25 +302,25 @@ inline NodeLaunch zp_node_launch(int64_t blocks, double items, const NodeShape &
 // has the slots that the sort has left out (edges of indices out of range): they stand behind all others and read
 // as edges 0 -> 0, but are edges into no node.
 //
-// A node of more than two steps' edges is cut: all nodes' edges stand in one row, and it has a cut wherever
-// that row reaches a multiple of `step`.  Block n has what comes before the first cut, block N + k what
-// follows cut k (in `parts` parts like all others); of the blocks behind N those whose cut falls into no such
-// node, in most graphs all of them, end where they begin.  A part of a step is half of an SM's share of the
-// edges, so a node by itself keeps its block busy as long as the others take at most; but no less than twice a
-// node's mean, or graphs of even nodes would be cut (those of up to 74 nodes are: one and two of 90 edges took
-// 10 and 7 % longer a training step than edge by edge).  2 000 nodes of 30 edges and one of 20 000 more, lmax 4 /
-// C 128: a training step of 22.4 ms edge by edge took 52.5 with every node one block's, and takes 21.6; inference
-// 12.1, 20.7 and 12.2.
+// A node of very many edges is cut: all nodes' edges stand in one row, and it has a cut wherever that row reaches a
+// multiple of `step`.  The blocks of node n have what comes before the first cut, block k behind all nodes' what
+// follows cut k; those whose cut falls into no such node, in most graphs all of them, end where they begin.  A
+// step is half of an SM's share of the edges, and a node is left whole whose blocks have no more than that each, or
+// two; but no less than twice a node's mean, or graphs of even nodes would be cut (those of up to 74 nodes
+// are: one and two of 90 edges took 10 and 7 % longer a training step than edge by edge).  2 000 nodes of 30 edges
+// and one of 20 000 more, lmax 4 / C 128: a training step of 22.4 ms edge by edge took 52.5 with every node one
+// block's, and takes 21.6; inference 12.1, 20.7 and 12.2.
 struct NodeCut {
-  int nodes;                             // N
-  uint32_t step, cuts;
-  unsigned blocks() const { return (unsigned)nodes + 1 + cuts; }
+  int nodes, parts;                      // N; blocks of a node
+  uint32_t step, cuts, whole;            // whole: edges of a node that is not cut, at most
+  __host__ __device__ __forceinline__ int ends() const { return (nodes + 1) * parts; }    // blocks before the cuts'
+  unsigned blocks() const { return (unsigned)ends() + cuts; }
 };
 inline NodeCut zp_node_cut(int64_t N, int64_t E, bool both, int parts) {
-  const int64_t total = both ? 2 * E : E;
-  int64_t step = std::max<int64_t>(zp_ceil_div(parts * total, kZpNodeCuts), 64);
-  if (N > kZpNodeCuts / 4) step = std::max<int64_t>(step, 2 * zp_ceil_div(total, N));
-  return NodeCut{(int)N, (uint32_t)step, total ? (uint32_t)((total - 1) / step) : 0u};
+  const int64_t total = both ? 2 * E : E, pieces = std::max(parts, 2);
+  int64_t step = std::max<int64_t>(zp_ceil_div(total, kZpNodeCuts), 64);
+  if (N > kZpNodeCuts / 4) step = std::max<int64_t>(step, zp_ceil_div(4 * zp_ceil_div(total, N), pieces));
+  return NodeCut{(int)N, parts, (uint32_t)step, total ? (uint32_t)((total - 1) / step) : 0u, (uint32_t)(pieces * step)};
 }
 struct NodeEdges {
   int n, beg, own, sbeg, total;          // node; first and number of the edges into it; first edge out; of both
@@ -328,13 +328,18 @@ struct NodeEdges {
   int first, last;                       // this block's stretch of them
   uint32_t cut0, cut1;                   // first and last cut of the node (a cut node: cut0 <= cut1)
   __host__ __device__ __forceinline__ NodeEdges(int block, const NodeCut &cut, int64_t E, const int32_t *row_ptr,
-                                                const int32_t *view, const int32_t *row_ptr_src, int part, int parts) {
+                                                const int32_t *view, const int32_t *row_ptr_src) {
     const int N = cut.nodes;
     auto before = [&](int k) { return (uint32_t)row_ptr[k] + (view ? (uint32_t)row_ptr_src[k] : 0u); };
-    n = block;
+    const bool tail = block >= cut.ends();
     uint32_t at = 0;
-    if (n > N) {                         // the node that the cut falls into: the last that begins at it or before
-      at = (uint32_t)(n - N) * cut.step;
+    int part = 0, parts = 1;
+    if (!tail) {
+      parts = cut.parts;
+      n = block / parts;
+      part = block - n * parts;
+    } else {                             // the node that the cut falls into: the last that begins at it or before
+      at = (uint32_t)(block - cut.ends() + 1) * cut.step;
       int lo = 0, hi = N;                // before(lo) <= at; by halves it took 3 us of a block with nothing to do
       while (lo < hi) {
 #ifdef __CUDA_ARCH__
@@ -361,11 +366,11 @@ struct NodeEdges {
     int lo = 0, hi = total;
     cut0 = 1;
     cut1 = 0;
-    if ((uint32_t)total > 2 * cut.step) {
+    if ((uint32_t)total > cut.whole) {
       const uint32_t begin = before(n);
       cut0 = begin / cut.step + 1;
       cut1 = (begin + (uint32_t)total - 1) / cut.step;
-      if (block <= N) {
+      if (!tail) {
         hi = (int)(cut0 * cut.step - begin);
       } else if (at > begin && at - begin < (uint32_t)total) {
         lo = (int)(at - begin);
@@ -373,7 +378,7 @@ struct NodeEdges {
       } else {
         hi = 0;
       }
-    } else if (block > N) {
+    } else if (tail) {
       hi = 0;
     }
     first = lo + (int)((int64_t)(hi - lo) * part / parts);

@@ -240,9 +240,9 @@ node_rotate_grad_out_kernel(const __grid_constant__ ZpTables t, const NodeCut cu
   const int c = 4 * li;
   float *g_s = node_s, *stage = node_s + (size_t)K * ls, *y_s = stage + (size_t)w * t.Km * ls + c;
   float *rot_s = stage + (size_t)workers * t.Km * ls + (size_t)w * 2 * t.rot_ld;
-  const float inv = zp_publish_scale(dy, scale, blockIdx.x == 0 && blockIdx.z == 0 && threadIdx.x == 0);
+  const float inv = zp_publish_scale(dy, scale, blockIdx.x == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
-  const NodeEdges edges(blockIdx.x, cut, E, row_ptr, nullptr, nullptr, blockIdx.z, gridDim.z);
+  const NodeEdges edges(blockIdx.x, cut, E, row_ptr, nullptr, nullptr);
   if (edges.first == edges.last) return;
   auto rows = [&](int e) { return y + (size_t)(e < 0 ? 0 : e) * t.Km * t.C + c; };
   auto rotation = [&](int64_t e, int buffer) {
@@ -402,10 +402,10 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, const NodeCut cut,
   float *x_s = node_s, *stage = node_s + (size_t)K * ls, *da_s = stage + (size_t)w * rows * ls + li * VN;
   float *rad_s = da_s + t.Km * ls;
   float *rot_s = stage + (size_t)workers * rows * ls + (size_t)w * 2 * t.rot_ld;
-  const NodeEdges node(blockIdx.x, cut, E, a.row_ptr, a.perm_src, a.row_ptr_src, blockIdx.z, gridDim.z);
+  const NodeEdges node(blockIdx.x, cut, E, a.row_ptr, a.perm_src, a.row_ptr_src);
   float inv = 1.f;
   if constexpr (FMT == kFmtFp16x2)
-    inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0);
+    inv = zp_publish_scale(grad_radial_planes, scale, blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0);
   const u64 inv2 = pack2(inv, inv);
   const int64_t plane_bytes = 2 * grad_radial_planes.plane_stride;
   V acc[SUMS ? K : 1];
@@ -469,7 +469,7 @@ node_rotate_in_bwd_kernel(const __grid_constant__ ZpTables t, const NodeCut cut,
   const int n = edges.n;
   if (n == cut.nodes) return;            // left-out slots
   // this lane's place in the rows that the sums go to
-  float *const to = (blockIdx.x > cut.nodes ? a.cuts + (size_t)(blockIdx.x - cut.nodes - 1) * K * t.C
+  float *const to = (blockIdx.x >= cut.ends() ? a.cuts + (size_t)(blockIdx.x - cut.ends()) * K * t.C
                                             : a.grad_x + (size_t)n * K * t.C) + c0 + li * VN;
   __syncthreads();                       // all are done with their rows: the sums take their place
   float *const sums = stage + li * VN;
@@ -524,7 +524,7 @@ int zp_launch_rotate_grad_out(const zp_plan *p, int64_t first, int64_t N, int64_
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
     if (int rc_ = zp_ensure_smem(node_rotate_grad_out_kernel<LM, FMT>, nl.smem, opt_in)) return rc_; \
-    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3(cut.blocks(), 1, (unsigned)nl.parts), 32 * nl.warps, nl.smem, st, t, cut, E, ns.G, ns.quads, \
+    zp_launch(node_rotate_grad_out_kernel<LM, FMT>, dim3(cut.blocks()), 32 * nl.warps, nl.smem, st, t, cut, E, ns.G, ns.quads, \
               g + (size_t)first * t.K * t.C, y, env, rot, row_ptr + first, dy, scale, grad_env, reinterpret_cast<float4 *>(torque));  \
     break;                                                                                        \
   }
@@ -587,7 +587,7 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float 
   const NodeArgs a{da1, radial, x, rot, row_ptr, perm_src, row_ptr_src, grad_radial, grad_x,
                    reinterpret_cast<float4 *>(torque), cuts, arrived};
   const NodeCut cut = zp_node_cut(N, E, true, nl.parts);
-  const dim3 grid(cut.blocks(), (unsigned)ns.groups, (unsigned)nl.parts);
+  const dim3 grid(cut.blocks(), (unsigned)ns.groups);
 #define CALL_S(LM, FMT, S)                                                                        \
   {                                                                                               \
     static ZpSmemOptIn opt_in;               /* per instantiation and device */                   \
@@ -618,4 +618,4 @@ int zp_launch_rotate_in_bwd(const zp_plan *p, int64_t N, int64_t E, const float 
 
 int zp_node_groups(const ZpTables &t) { return node_shape(t).groups; }
 int zp_torque_slots(const ZpTables &t) { return 1 + 2 * zp_node_groups(t); }
-int64_t zp_node_cuts_most(int64_t E) { return zp_node_cut(2 * E, E, true, 1).cuts; }
+int64_t zp_node_cuts_most(int64_t E) { return zp_node_cut(1, E, true, 1).cuts; }
