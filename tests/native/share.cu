@@ -49,5 +49,15 @@ int main(int argc, char **argv) {
     for (; !one_by_one.empty(); one_by_one.pop()) best = one_by_one.top();
     if (std::abs(most - pl.makespan) > 1e-9 * best || most > best * (1.0 + 1e-9)) return std::printf("load %g %g\n", most, best), 1;
   }
+  // the most rows of a launch: no unit's count leaves 16 bits
+  for (int trial = 0; trial < 200; ++trial) {
+    const int64_t columns = pick(0, 1) ? pick(1, 4096) : pick(1, 64), rows = zp_rows_per_launch(columns);
+    GroupPlan pl;
+    pl.shape[0].tiles = zp_ceil_div(rows, 128) * zp_ceil_div(columns, 64);
+    pl.shape[0].cost = 4000;
+    share_out(pl, 1, pick(64, 148));
+    for (int c = 0; c < pl.classes; ++c)
+      if (pl.count[c][0] > INT16_MAX) return std::puts("count"), 1;
+  }
   std::puts("ok");
 }

@@ -1667,6 +1667,7 @@ int fill_group(GemmGroup &grp, const GroupPlan &pl, const ZpGemmTc *const *g, in
   grp.classes = pl.classes;
   std::copy(pl.unit0, pl.unit0 + pl.classes + 1, grp.unit0);
   for (int c = 0; c < pl.classes; ++c) {
+    if (*std::max_element(pl.count[c], pl.count[c] + n) > INT16_MAX) return ZP_ERR_TOO_LARGE;
     std::copy(pl.first[c], pl.first[c] + n, grp.first[c]);
     std::copy(pl.count[c], pl.count[c] + n, grp.count[c]);
   }
@@ -1931,6 +1932,15 @@ bool zp_gemm_tc_fusable(const ZpGemmTc &g) {
 int zp_launch_gemm_tc(const ZpGemmTc &g, cudaStream_t st) {
   if (g.M <= 0 || g.N <= 0) return ZP_OK;
   if (const int rc = check_product(g)) return rc;
+  if (g.M > zp_rows_per_launch(g.N) && !g.a_mn && !(g.epi && g.epi->mode)) {      // in halves
+    ZpGemmTc half[2] = {g, g};
+    half[0].M = zp_ceil_div(g.M / 2, 256) * 256;
+    half[1].M = g.M - half[0].M;
+    half[1].A = static_cast<const uint16_t *>(g.A) + half[0].M * g.lda;
+    half[1].C = g.C + half[0].M * g.ldc;
+    const int rc = zp_launch_gemm_tc(half[0], st);
+    return rc ? rc : zp_launch_gemm_tc(half[1], st);
+  }
   const ZpGemmTc *one = &g;
   return dispatch(&one, 1, use_pair(g) ? 1 : 0, st);
 }

@@ -26,6 +26,12 @@ struct GroupPlan {
   double makespan;
 };
 
+// A unit's tiles of a product are counted in 16 bits (a launch's parameters in 32 cost every small launch 0.2 us):
+// so many rows of tiles of at least 64 columns, on 64 units or more, one launch takes.
+inline int64_t zp_rows_per_launch(int64_t columns) {
+  return std::max<int64_t>(INT16_MAX / zp_ceil_div(columns, 64), 1) * 64 * 128;
+}
+
 // Shares the tiles out: products in turn, longest tiles first, every tile to a unit that has least so far.
 // Units that stand alike are a class and treated as one, so this takes a microsecond and not one per tile.
 // A fixed stride through the list gave the same units the longest tiles of every round.  With this, and the
