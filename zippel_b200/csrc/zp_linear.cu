@@ -100,7 +100,6 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
     wg = ZpGemmTc{N, K, M, P, dy.base, dy.ld, dy.plane_stride, 1,
                   x.base, x.ld, x.plane_stride, 1, nullptr, partials, ldk, plan->status_dev,
                   0, 1, N * ldk, 0, fp16, dy.scale, x.scale, nullptr};
-    wg.ksplit = zp_gemm_tc_pick_splits(wg, max_splits);
     ++n;
   }
   // One launch for both, but not where the weight gradient would leave the CTA pairs for it: with two planes
@@ -108,8 +107,11 @@ int zp_linear_backward_planes(const zp_plan *plan, int64_t M, int64_t K, int64_t
   // and its VJP, apart / together, two planes: 128 x 128 at 25 000, 40 000 and 100 000 rows 188 / 202, 212 / 248 and
   // 332 / 387 us, 256 x 256 at 25 000 and 100 000 218 / 242 and 416 / 511 (15 000 rows of either the same within 5 %);
   // same kernel either way: 64 x 64 at 100 000 384 / 357, 128 x 1536 at 25 000 357 / 334.
-  const bool together = dx && dw && M <= kTogetherBackward &&
-                        !(P == 2 && M > 20000 && zp_gemm_tc_pairs(wg) && !zp_gemm_tc_pairs(g[0]));
+  bool together = dx && dw && M <= kTogetherBackward;
+  if (dw && (!together || (P == 2 && M > 20000))) {
+    wg.ksplit = zp_gemm_tc_pick_splits(wg, max_splits);
+    if (together) together = !zp_gemm_tc_pairs(wg) || zp_gemm_tc_pairs(g[0]);
+  }
   if (together) {
     zp_gemm_group_splits(g, n, 1, max_splits);
     if ((rc = zp_launch_gemm_group(g, n, st))) return rc;
