@@ -225,7 +225,9 @@ int zp_eso2_forward_inference(const zp_plan *plan, int64_t n_nodes, int64_t n_ed
  * requires_grad = False on the weights): the weight-gradient products, the bias column sums and
  * the unfolding are not run, everything else is unchanged.  grad_x_node == NULL: the embeddings
  * are an input without a gradient (E and dE/dpos of one block, the reference's build_force,
- * blocks/eso2_ir.py:579-590): the per-edge contributions are neither written nor summed.       */
+ * blocks/eso2_ir.py:579-590): nothing is summed per node.  row_ptr, perm_src and row_ptr_src are read
+ * in that case too: an edge's rows of grad_radial and its torques are formed where its two nodes are, so
+ * both views have to name every edge.                                                            */
 int zp_eso2_backward(const zp_plan *plan, int64_t n_nodes, int64_t n_edges,
                      const float *grad_node_out, const float *x_node, const float *edge_vec,
                      const float *cos_g, const float *sin_g, const float *radial,
@@ -380,7 +382,8 @@ int zp_edge_features_backward(const zp_front_config *cfg, int64_t n_nodes, int64
  * Node ranges as zp_eso2_forward: node_out holds rows first_node .. first_node + n_nodes of the
  * n_rows nodes and the edges are those into them; row_ptr and row_ptr_src cover all n_rows nodes.
  * Per-edge inputs (shifts, cos_g, sin_g) are in the caller's order, `perm` names the position of a
- * sorted edge in them; perm .. row_ptr_src from zp_csr_build.                                    */
+ * sorted edge in them; perm .. row_ptr_src from zp_csr_build.  A forward may leave perm_src and
+ * row_ptr_src null; where both are given it reads them.                                          */
 typedef struct zp_block_call {
   int64_t n_nodes, n_edges, n_rows, first_node;
   const float *pos;                /* [n_rows, 3]                                               */
@@ -486,7 +489,7 @@ typedef enum zp_kernel_class {
   ZP_K_BIAS_GRAD = 9,
   ZP_K_GATE_BWD = 10,
   ZP_K_ROTATE_IN_BWD = 11,
-  ZP_K_SRC_REDUCE = 12,
+  ZP_K_SRC_REDUCE = 12,   /* (no launches: the node sums are part of ZP_K_ROTATE_IN_BWD)       */
   ZP_K_WIGNER_BWD = 13,
   ZP_N_KERNEL_CLASSES = 14
 } zp_kernel_class;

@@ -49,6 +49,13 @@ def test_hbm_bytes_per_step(bench, monkeypatch):
     assert bench.hbm_bytes_per_step(one_plane, n, e)["rotate_in"] == e * (r * 4 + km * 2 * c * 2)
 
 
+def test_hbm_bytes_per_step_by_node(bench):
+    """The gradient of the embeddings summed within rotate_in_bwd: as the library launches it."""
+    got = bench.hbm_bytes_per_step(ESO2Block(BlockConfig(**bench.CFG)), 2000, 60000, by_node=True)
+    assert "src_reduce" not in got
+    assert got["rotate_in_bwd"] == 60000 * (19 * 2 * 128 * 4 + 2 * 3072 * 4) + 2000 * 25 * 128 * 4
+
+
 def test_chunk_budget_quantisation():
     """The per-call edge budget keeps four significant bits: stable under small drifts of the
     free memory, never above the raw budget, never less than 7/8 of it."""

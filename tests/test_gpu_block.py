@@ -151,8 +151,8 @@ def test_bad_input_raises(what):
 @pytest.mark.parametrize("lmax,mmax,c,h", [(6, 3, 8, 8), (6, 6, 16, 8), (5, 4, 40, 8), (1, 0, 136, 8),
                                            (4, 4, 256, 8)])
 def test_rotations_over_degrees_orders_and_widths(lmax, mmax, c, h, jd64):
-    """Row walks, packed sums and torques of the per-edge kernels from two degrees to seven, orders
-    up to the degree, and widths that leave a block's last warp partly idle."""
+    """Row walks, packed sums and torques of the rotate kernels from two degrees to seven, orders up to the
+    degree, and widths that leave a warp partly idle (by edge) or a worker's lanes (by node)."""
     cfg = dict(lmax=lmax, mmax=mmax, sphere_channels=c, hidden_channels=h, edge_channels=8,
                num_distance_basis=6, cutoff=5.0)
     params = orc.init_params(cfg, seed=lmax)

@@ -202,7 +202,7 @@ def _f32(t: torch.Tensor) -> torch.Tensor:
 
 
 #: Upper bound on the edges handed to one forward/backward call of the C ABI.  ``None`` sizes it
-#: from the device's free memory (the per-call workspace is ~123 KB per edge at lmax 4 / C 128).
+#: from the device's free memory (the per-call workspace is ~98 KB per edge at lmax 4 / C 128).
 #: Larger graphs are processed as destination-node chunks; the backward then recomputes each
 #: chunk's forward instead of keeping every chunk's activations.
 MAX_EDGES_PER_CALL: int | None = None

@@ -13,7 +13,7 @@ It plays the part of the reference back end's ``allocate`` + ``run_program``
 module call (blocks/eso2_ref.py:317-349 and autograd through it).
 
 The recording keeps every buffer of one step alive in the graph's private memory pool — inputs,
-radial features, the block's workspace (about 125 KB per edge at lmax 4 / C 128 in the fp32
+radial features, the block's workspace (about 98 KB per edge at lmax 4 / C 128 in the fp32
 operand format) and all gradients — so the edge list must fit one call; graphs that need the
 chunked path cannot be recorded.
 

@@ -1501,9 +1501,8 @@ int pick_bn(int64_t N, int cap, int step = 16) {
   return best;
 }
 
-// The CTA-pair kernel serves the two-plane (fp16) and one-plane (bf16) formats unless the caller
-// forces a kernel:
-// variant 2 = single-CTA kernel, variant 3 = pair kernel.
+// The CTA-pair kernel serves all three formats unless the caller forces a kernel: variant 2 = single-CTA kernel,
+// variant 3 = pair kernel, and of three planes variant 1, which only the single-CTA kernel has.
 bool pair_enabled() {
   static int on = -1;
   if (on < 0) {

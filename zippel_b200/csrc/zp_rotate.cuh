@@ -1,4 +1,5 @@
-// Shared pieces of the per-edge rotate kernels: packed arithmetic, staging, plane stores.
+// Shared pieces of the rotate kernels, by edge and by node: packed arithmetic, staging, plane stores, and how a
+// kernel by node deals a graph's edges out.
 #pragma once
 
 #include <algorithm>

@@ -1,10 +1,10 @@
-// The VJPs of the per-edge rotate kernels.
+// The VJPs of the rotate kernels.
 //
-//   rotate_grad_out      the VJP of rotate_back_scatter (needs y)
-//   rotate_in_bwd        the VJP of rotate_in, per-edge node contributions
+//   rotate_grad_out      the VJP of rotate_back_scatter (needs y), by edge or by node
+//   rotate_in_bwd        the VJP of rotate_in by node, with the gradient of x_node
 //
-// (autograd through blocks/eso2_ref.py:334-349).  One (edge, channel quad) per thread; see
-// zp_rotate.cu for the forward kernels.
+// (autograd through blocks/eso2_ref.py:334-349).  By edge, one (edge, channel quad) per thread; by node
+// see zp_rotate.cuh, for the forward kernels zp_rotate.cu.
 #include <algorithm>
 
 #include "zp_rotate.cuh"
@@ -12,7 +12,7 @@
 namespace {
 
 // ------------------------------------------------------------------------------------------
-// per-edge backward kernels: one (edge, channel quad) per thread
+// rotate_grad_out by edge: one (edge, channel quad) per thread
 // ------------------------------------------------------------------------------------------
 // Gradient of the rotation.  Both kernels hold, for every row (l, m) of an edge, its rotated value
 // b[m] (a in the edge frame, or the rotated upstream gradient) and the factor p[m] it is multiplied
@@ -171,8 +171,8 @@ rotate_grad_out_kernel(const __grid_constant__ ZpTables t, int64_t E, int epb,
 }
 
 // The same by node (zp_rotate.cuh): a block for the edges into one node, whose rows of g are read once.  60 000
-// edges at lmax 4 / mmax 2 / C 128: 32 KB an edge from L2 by edge, 19 here, 314 -> 214 us; 384 000 in one plane 1.78 ->
-// 1.08 ms.
+// edges at lmax 4 / mmax 2 / C 128: 32 KB an edge from L2 by edge, 19 here, 321 -> 207 us in a training step; 384 000
+// in one plane 1.98 -> 1.22 ms.
 template <int L, int LMAX, int FMT>
 struct GradOutN {
   static __device__ __forceinline__ void run(const ZpTables &t, const float *g_s, float *y_s, int ls, uint16_t *out,
@@ -295,9 +295,9 @@ template <> struct Elem<kFmtFp32> { using type = float; };
 
 // By node (zp_rotate.cuh).  What an edge adds to the node's gradient stays in registers: written per
 // edge and summed afterwards it was half of all bytes (2 x 25.6 KB of 95 KB an edge at lmax 4, C 128).  Four
-// channels a lane, two from lmax 5 on: 36 rows of four do not fit the registers.  60 000 edges in two planes 810 us
-// and 231 of the sums -> 531, 384 000 in one 4.56 and 1.45 ms -> 2.90; bound by instruction issue (2 400 a worker and
-// edge half, eight warps to an SM at 252 registers), HBM at half its rate.
+// channels a lane, two from lmax 5 on: 36 rows of four do not fit the registers.  In a training step 60 000 edges in
+// two planes, sums included, 1 121 -> 523 us, 384 000 in one 7.13 -> 3.43 ms; bound by fixed latencies and instruction
+// issue (2 330 a worker and edge half, eight warps to an SM at 240 registers), HBM at half its rate.
 // SUMS: the gradient of x_node is wanted (not in a force evaluation; the others are the same to the last bit).
 // what a lane needs of an edge: its channels in row 0 of da1, in column 0 of radial
 struct EdgeAt {
