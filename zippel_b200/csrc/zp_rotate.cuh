@@ -306,9 +306,11 @@ inline NodeLaunch zp_node_launch(int64_t blocks, double items, const NodeShape &
 // A node of very many edges is cut: all nodes' edges stand in one row, and it has a cut wherever that row reaches a
 // multiple of `step`.  The blocks of node n have what comes before the first cut, block k behind all nodes' what
 // follows cut k; those whose cut falls into no such node, in most graphs all of them, end where they begin.  A
-// step is half of an SM's share of the edges, and a node is left whole whose blocks have no more than that each, or
-// two; but no less than twice a node's mean, or graphs of even nodes would be cut (those of up to 74 nodes
-// are: one and two of 90 edges took 10 and 7 % longer a training step than edge by edge).  2 000 nodes of 30 edges
+// step is half of an SM's share of the edges, so that a node by itself keeps its blocks busy as long as the others
+// take at most, and a node is left whole whose blocks (two at least) have no more than that each.  Nodes of up to
+// four times the mean are whole, or graphs of even nodes would be cut (those of up to 74 nodes are: one and two of 90
+// edges took 10 and 7 % longer a training step than edge by edge).  Lines of eight times the mean cost 200 nodes
+// of 30 edges and one of 600 more 11 % of a force evaluation, and gain nothing elsewhere.  2 000 nodes of 30 edges
 // and one of 20 000 more, lmax 4 / C 128: a training step of 22.4 ms edge by edge took 52.5 with every node one
 // block's, and takes 21.6; inference 12.1, 20.7 and 12.2.
 struct NodeCut {
